@@ -111,6 +111,18 @@ int llsa_rms_norm_fwd(const LlsaTensor* x, const LlsaTensor* weight, float eps, 
 int llsa_rope_fwd(const LlsaTensor* x, const LlsaTensor* freq, const LlsaTensor* y, void* stream);
 int llsa_rope_bwd(const LlsaTensor* dy, const LlsaTensor* freq, const LlsaTensor* dx, void* stream);
 
+/* Backward of the q / k preparation in front of the operators, up to two tensors in one launch: dx[i] = d/dx of
+ * rope(rms_norm(x[i])) applied to dy[i].  freq NULL: no rotation; it may be F32 whatever the data's type (every product and sum of
+ * the rotation is rounded to the wider type, as llsa_rope_bwd does).  Tensors whose norm_mask bit is set went through
+ * llsa_rms_norm_fwd with norm_weight[i] (F32 [C], a NULL entry means ones) and eps; their x[i] is read and, where dw[i] is not
+ * NULL, the weight's gradient (F32 [C]) is written; dw_partial is then a 1-D F32 scratch of llsa_rms_rope_bwd_partial_elems()
+ * elements.  dx[i] may be dy[i] (same strides).  C = 64.  Replaces MyRopeFunction.backward (rope.py:126-146) on q and k and the
+ * RMSNorm backward autograd runs after it (rope_dit_transformer_2d.py:215-238). */
+int64_t llsa_rms_rope_bwd_partial_elems(int n_tensors);
+int llsa_rms_rope_bwd(int n_tensors, const LlsaTensor* dy, const LlsaTensor* x, const LlsaTensor* const* norm_weight, int norm_mask,
+                      float eps, const LlsaTensor* freq, const LlsaTensor* dx, const LlsaTensor* dw_partial,
+                      const LlsaTensor* const* dw, void* stream);
+
 /* ---- selection: src/llsa/kernel/triton/topk.py ----------------------------
  * Coarse: idx[b,h,i,:] = top-`topk` columns of round_dtype(pq[b,h,i,:] . pk[b,h,:,:]^T),
  * descending, ties -> smallest index.  idx is I32 or I64 [B,H,M,topk].  Replaces

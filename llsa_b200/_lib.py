@@ -43,6 +43,7 @@ class LlsaAttnArgs(C.Structure):
 EXPORTS = [
     "llsa_version", "llsa_last_error_string", "llsa_mean_pool_fwd", "llsa_mean_pool_bwd", "llsa_pool_pyramid_fwd",
     "llsa_rope_pool_pyramid_fwd", "llsa_rms_rope_pool_pyramid_fwd", "llsa_rms_norm_fwd",
+    "llsa_rms_rope_bwd", "llsa_rms_rope_bwd_partial_elems",
     "llsa_rope_fwd", "llsa_rope_bwd", "llsa_coarse_topk", "llsa_refine_topk", "llsa_select_two_level", "llsa_transpose_scratch_bytes",
     "llsa_transpose_indices", "llsa_transpose_indices_pairs", "llsa_transpose_range_entries", "llsa_transpose_indices_noalloc", "llsa_attn_fwd", "llsa_attn_bwd",
     "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems", "llsa_status_check",
@@ -62,6 +63,9 @@ def _declare(lib: C.CDLL) -> None:
     lib.llsa_rope_pool_pyramid_fwd.argtypes = [C.c_int, TP, TP, C.c_int, TP, TP, TP, C.c_int, C.c_void_p]
     lib.llsa_rms_rope_pool_pyramid_fwd.argtypes = [C.c_int, TP, C.POINTER(TP), C.c_int, C.c_float, TP, C.c_int, TP, TP, TP, C.c_int, C.c_void_p]
     lib.llsa_rms_norm_fwd.argtypes = [TP, TP, C.c_float, TP, C.c_void_p]
+    lib.llsa_rms_rope_bwd.argtypes = [C.c_int, TP, TP, C.POINTER(TP), C.c_int, C.c_float, TP, TP, TP, C.POINTER(TP), C.c_void_p]
+    lib.llsa_rms_rope_bwd_partial_elems.argtypes = [C.c_int]
+    lib.llsa_rms_rope_bwd_partial_elems.restype = C.c_int64
     lib.llsa_rope_fwd.argtypes = [TP, TP, TP, C.c_void_p]
     lib.llsa_rope_bwd.argtypes = [TP, TP, TP, C.c_void_p]
     lib.llsa_coarse_topk.argtypes = [TP, TP, TP, C.c_int, C.c_void_p]
@@ -82,7 +86,7 @@ def _declare(lib: C.CDLL) -> None:
     lib.llsa_attn_bwd.argtypes = [C.POINTER(LlsaAttnArgs), C.c_void_p]
     for name in EXPORTS:
         fn = getattr(lib, name)
-        if name not in ("llsa_last_error_string", "llsa_transpose_scratch_bytes", "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems"):
+        if name not in ("llsa_last_error_string", "llsa_transpose_scratch_bytes", "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems", "llsa_rms_rope_bwd_partial_elems"):
             fn.restype = C.c_int
 
 

@@ -1,0 +1,265 @@
+// Backward of what stands in front of the attention operators: the 2-D rotation of q and k and their RMSNorm
+// (models/rope_dit_transformer_2d.py:215-238 run backwards), both tensors in one launch.
+//
+//   g  = rotation^-1 (dy), every product and sum rounded to the element type as rope_kernel<..., BWD> does (rope.cu)
+//   dx = rstd * (g w - xh * mean(g w xh)),  dw = sum over rows of g xh,   xh = x rstd,  rstd = rsqrt(mean(x^2) + eps)
+//
+// HBM-bound: reads dy and x, writes dx (dx may be dy's own memory).  A CTA takes chunks of kRowsPerThread * (threads / lanes)
+// neighbouring tokens of one (b,h) slice, so the slice is found once per chunk and every thread has all its loads (row of dy, of x,
+// of the table) in flight before it uses one.  The weight gradient is kept in registers over all chunks of a CTA, reduced through
+// shared memory, and leaves as one [C] row per CTA; a one-CTA-per-tensor kernel adds the rows in order (bit-reproducible).
+// B=4 H=6 N=16384, [B,N,H,D] storage, both tensors: 151 MB read and written.  The rotation's two launches and the eager fp32
+// formula it replaces moved 14 times that (2.05 ms).
+#include <string.h>
+
+#include <type_traits>
+
+#include "common.cuh"
+
+namespace llsa {
+
+constexpr int kFbThreads = 256, kFbRows = 4, kFbC = 64;
+
+template <typename T>
+struct FrontBwdArgs {
+  View<const T> dy[2], x[2];
+  View<T> dx[2];
+  const float* w[2];       // fp32 [C] or nullptr (ones)
+  float* dw_partial;       // [tensor][gridDim.x][C] or nullptr
+  const void* freq;        // [S, C] (even columns sin, odd columns cos) or nullptr
+  int64_t fs;
+  float eps;
+  int norm_mask;
+  int H, chunks_per_head;
+  int S, n_chunks;
+};
+
+template <typename T>
+__device__ __forceinline__ void ld16(const T* p, float (&v)[16 / sizeof(T)]) {
+  const uint4 x = *reinterpret_cast<const uint4*>(p);
+  if constexpr (sizeof(T) == 4) {
+    v[0] = __uint_as_float(x.x); v[1] = __uint_as_float(x.y); v[2] = __uint_as_float(x.z); v[3] = __uint_as_float(x.w);
+  } else {
+    v[0] = bf16_lo(x.x); v[1] = bf16_hi(x.x); v[2] = bf16_lo(x.y); v[3] = bf16_hi(x.y);
+    v[4] = bf16_lo(x.z); v[5] = bf16_hi(x.z); v[6] = bf16_lo(x.w); v[7] = bf16_hi(x.w);
+  }
+}
+template <typename T>
+__device__ __forceinline__ void st16(T* p, const float (&v)[16 / sizeof(T)]) {
+  uint4 x;
+  if constexpr (sizeof(T) == 4) {
+    x = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+  } else {
+    x = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+  }
+  *reinterpret_cast<uint4*>(p) = x;
+}
+
+// T: element type of the data, TF: of the table (the wider of the two is the type products and sums are rounded to)
+template <typename T, typename TF, bool NORM>
+__global__ void __launch_bounds__(kFbThreads) front_bwd_kernel(FrontBwdArgs<T> a) {
+  constexpr int VEC = 16 / sizeof(T), LANES = kFbC / VEC, STEP = kFbThreads / LANES;
+  using P = typename std::conditional<(sizeof(TF) > sizeof(T)), TF, T>::type;
+  const int ti = blockIdx.y, r0 = threadIdx.x / LANES, c = (threadIdx.x % LANES) * VEC;
+  const bool norm = NORM && ((a.norm_mask >> ti) & 1);
+  const TF* freq = reinterpret_cast<const TF*>(a.freq);
+  float w[VEC], dw[VEC];
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) {
+    w[i] = norm && a.w[ti] ? a.w[ti][c + i] : 1.f;
+    dw[i] = 0.f;
+  }
+  for (int ch = blockIdx.x; ch < a.n_chunks; ch += gridDim.x) {
+    const int bh = ch / a.chunks_per_head, s0 = (ch - bh * a.chunks_per_head) * (STEP * kFbRows) + r0;
+    const int b = bh / a.H, h = bh - b * a.H;
+    const T* dyp = a.dy[ti].head(b, h) + c;
+    const T* xp = NORM ? a.x[ti].head(b, h) + c : nullptr;
+    T* dxp = a.dx[ti].head(b, h) + c;
+    float g[kFbRows][VEC], x[kFbRows][VEC];
+#pragma unroll
+    for (int u = 0; u < kFbRows; ++u) {     // rows past the end are computed on the last row (the reductions need every lane) and dropped
+      const int64_t s = min(s0 + u * STEP, a.S - 1);
+      ld16<T>(dyp + s * a.dy[ti].sn, g[u]);
+      if (NORM) if (norm) ld16<T>(xp + s * a.x[ti].sn, x[u]);
+    }
+    if (freq) {
+#pragma unroll
+      for (int u = 0; u < kFbRows; ++u) {
+        const TF* fp = freq + (int64_t) min(s0 + u * STEP, a.S - 1) * a.fs + c;
+        float f[VEC];
+        if constexpr (sizeof(TF) == sizeof(T)) ld16<TF>(fp, f);
+        else {
+          float f0[4], f1[4];
+          ld16<TF>(fp, f0);
+          ld16<TF>(fp + 4, f1);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { f[i] = f0[i]; f[4 + i] = f1[i]; }
+        }
+#pragma unroll
+        for (int j = 0; j < VEC; j += 2) {
+          const float sn = f[j], cs = f[j + 1], ge = g[u][j], go = g[u][j + 1];
+          g[u][j] = round_to<T>(round_to<P>(__fadd_rn(round_to<P>(__fmul_rn(cs, ge)), round_to<P>(__fmul_rn(sn, go)))));
+          g[u][j + 1] = round_to<T>(round_to<P>(__fadd_rn(round_to<P>(__fmul_rn(-sn, ge)), round_to<P>(__fmul_rn(cs, go)))));
+        }
+      }
+    }
+    if (NORM) {
+      if (norm) {
+#pragma unroll
+        for (int u = 0; u < kFbRows; ++u) {
+          float ss = 0.f, dot = 0.f;
+#pragma unroll
+          for (int i = 0; i < VEC; ++i) { ss = fmaf(x[u][i], x[u][i], ss); dot = fmaf(g[u][i] * w[i], x[u][i], dot); }
+#pragma unroll
+          for (int o = 1; o < LANES; o <<= 1) {
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            dot += __shfl_xor_sync(0xffffffffu, dot, o);
+          }
+          const float rstd = rsqrtf(ss / (float) kFbC + a.eps), k = dot * rstd / (float) kFbC;      // k = mean(g w xh)
+          const bool live = s0 + u * STEP < a.S;
+#pragma unroll
+          for (int i = 0; i < VEC; ++i) {
+            const float xh = x[u][i] * rstd;
+            if (live) dw[i] = fmaf(g[u][i], xh, dw[i]);
+            g[u][i] = rstd * (g[u][i] * w[i] - xh * k);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kFbRows; ++u) {
+      const int s = s0 + u * STEP;
+      if (s < a.S) st16<T>(dxp + (int64_t) s * a.dx[ti].sn, g[u]);
+    }
+  }
+  if (NORM && a.dw_partial) {
+    __shared__ float sw[kFbThreads / 32][kFbC];
+    const int warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i)
+#pragma unroll
+      for (int o = LANES; o < 32; o <<= 1) dw[i] += __shfl_xor_sync(0xffffffffu, dw[i], o);
+    if ((threadIdx.x & 31) < LANES)
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) sw[warp][c + i] = dw[i];
+    __syncthreads();
+    if (threadIdx.x < kFbC) {
+      float s = 0.f;
+#pragma unroll
+      for (int k = 0; k < kFbThreads / 32; ++k) s += sw[k][threadIdx.x];
+      a.dw_partial[((int64_t) ti * gridDim.x + blockIdx.x) * kFbC + threadIdx.x] = s;
+    }
+  }
+}
+
+// dw[ti][c] = sum over the CTAs' rows, 16 strided partial sums per channel added in order
+__global__ void __launch_bounds__(1024) front_dw_kernel(const float* __restrict__ partial, int rows, float* dw0, float* dw1) {
+  __shared__ float sm[16][kFbC];
+  const int c = threadIdx.x & 63, k = threadIdx.x >> 6;
+  const float* p = partial + (int64_t) blockIdx.x * rows * kFbC + c;
+  float s = 0.f;
+#pragma unroll 4
+  for (int r = k; r < rows; r += 16) s += p[(int64_t) r * kFbC];
+  sm[k][c] = s;
+  __syncthreads();
+  if (k == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) t += sm[i][c];
+    float* out = blockIdx.x == 0 ? dw0 : dw1;
+    if (out) out[c] = t;
+  }
+}
+
+constexpr int kFbMaxCtas = 148 * 4;
+
+template <typename T, typename TF>
+static int launch_front_bwd(int n, FrontBwdArgs<T>& a, int64_t BH, int grid, cudaStream_t st) {
+  const dim3 g((unsigned) grid, (unsigned) n);
+  if (a.norm_mask) front_bwd_kernel<T, TF, true><<<g, kFbThreads, 0, st>>>(a);
+  else front_bwd_kernel<T, TF, false><<<g, kFbThreads, 0, st>>>(a);
+  LLSA_LAUNCH_OK("front_bwd_kernel");
+  return LLSA_OK;
+}
+
+template <typename T>
+static int front_bwd_typed(int n, const LlsaTensor* dy, const LlsaTensor* x, const LlsaTensor* const* norm_weight, int norm_mask, float eps,
+                           const LlsaTensor* freq, const LlsaTensor* dx, const LlsaTensor* dw_partial, const LlsaTensor* const* dw,
+                           cudaStream_t st) {
+  FrontBwdArgs<T> a;
+  memset(&a, 0, sizeof(a));
+  for (int i = 0; i < n; ++i) {
+    a.dy[i] = make_view<const T>(&dy[i]);
+    a.dx[i] = make_view<T>(&dx[i]);
+    if (norm_mask) a.x[i] = make_view<const T>(&x[i]);
+    if (norm_weight && norm_weight[i]) a.w[i] = (const float*) norm_weight[i]->ptr;
+  }
+  a.freq = freq ? freq->ptr : nullptr;
+  a.fs = freq ? freq->stride[0] : 0;
+  a.eps = eps;
+  a.norm_mask = norm_mask;
+  a.H = (int) dy[0].shape[1];
+  a.S = (int) dy[0].shape[2];
+  const int64_t BH = dy[0].shape[0] * dy[0].shape[1];
+  const int rows = kFbRows * kFbThreads / (kFbC * (int) sizeof(T) / 16);
+  a.chunks_per_head = (a.S + rows - 1) / rows;
+  const int64_t chunks = BH * a.chunks_per_head;
+  LLSA_REQUIRE(chunks < (1ll << 31), LLSA_ERR_SHAPE, "rms_rope_bwd: too many rows");
+  a.n_chunks = (int) chunks;
+  const int grid = (int) (chunks < kFbMaxCtas ? chunks : kFbMaxCtas);
+  const bool want_dw = norm_mask && dw && (dw[0] || (n > 1 && dw[1]));
+  a.dw_partial = want_dw ? (float*) dw_partial->ptr : nullptr;
+  int rc;
+  if (freq && freq->dtype == LLSA_F32) rc = launch_front_bwd<T, float>(n, a, BH, grid, st);
+  else rc = launch_front_bwd<T, T>(n, a, BH, grid, st);
+  if (rc || !want_dw) return rc;
+  front_dw_kernel<<<n, 1024, 0, st>>>(a.dw_partial, grid, dw[0] ? (float*) dw[0]->ptr : nullptr, n > 1 && dw[1] ? (float*) dw[1]->ptr : nullptr);
+  LLSA_LAUNCH_OK("front_dw_kernel");
+  return LLSA_OK;
+}
+
+}  // namespace llsa
+
+using namespace llsa;
+
+extern "C" int64_t llsa_rms_rope_bwd_partial_elems(int n_tensors) { return n_tensors > 0 ? (int64_t) n_tensors * kFbMaxCtas * kFbC : 0; }
+
+extern "C" int llsa_rms_rope_bwd(int n_tensors, const LlsaTensor* dy, const LlsaTensor* x, const LlsaTensor* const* norm_weight, int norm_mask,
+                                 float eps, const LlsaTensor* freq, const LlsaTensor* dx, const LlsaTensor* dw_partial,
+                                 const LlsaTensor* const* dw, void* stream) {
+  LLSA_REQUIRE(dy && dx, LLSA_ERR_NULL, "rms_rope_bwd: null tensor list");
+  LLSA_REQUIRE(n_tensors >= 1 && n_tensors <= 2, LLSA_ERR_ARG, "rms_rope_bwd: n_tensors must be 1 or 2");
+  LLSA_REQUIRE(norm_mask >= 0 && norm_mask < (1 << n_tensors) && (!norm_mask || x), LLSA_ERR_ARG, "rms_rope_bwd: bad norm mask");
+  LLSA_REQUIRE(eps >= 0.f, LLSA_ERR_ARG, "rms_rope_bwd: eps must not be negative");
+  const int dt = dy[0].dtype;
+  LLSA_REQUIRE(is_float_dtype(dt), LLSA_ERR_DTYPE, "rms_rope_bwd: dtype must be f32 or bf16");
+  LLSA_REQUIRE(dy[0].ndim == 4 && dy[0].shape[3] == kFbC, LLSA_ERR_SHAPE, "rms_rope_bwd: tensors must be [B,H,S,64]");
+  const int64_t B = dy[0].shape[0], H = dy[0].shape[1], S = dy[0].shape[2], C = kFbC;
+  LLSA_REQUIRE(S < (1ll << 31) - 4096, LLSA_ERR_SHAPE, "rms_rope_bwd: S=%lld too long", (long long) S);
+  int rc;
+  for (int i = 0; i < n_tensors; ++i) {
+    if ((rc = check_bhnd(&dy[i], "dy", dt, B, H, S, C))) return rc;
+    if ((rc = check_bhnd(&dx[i], "dx", dt, B, H, S, C))) return rc;
+    if (!((norm_mask >> i) & 1)) continue;
+    if ((rc = check_bhnd(&x[i], "x", dt, B, H, S, C))) return rc;
+    const int64_t sw[1] = {C};
+    if (norm_weight && norm_weight[i] && (rc = check_contig(norm_weight[i], "norm weight", LLSA_F32, 1, sw))) return rc;
+    if (dw && dw[i]) {
+      if ((rc = check_contig(dw[i], "dw", LLSA_F32, 1, sw))) return rc;
+      LLSA_REQUIRE(dw_partial && dw_partial->ptr && dw_partial->dtype == LLSA_F32 && dw_partial->ndim == 1 && is_contiguous(dw_partial) &&
+                       dw_partial->shape[0] >= llsa_rms_rope_bwd_partial_elems(n_tensors),
+                   LLSA_ERR_WORKSPACE, "rms_rope_bwd: dw_partial scratch missing or too small");
+    }
+  }
+  if (freq) {
+    LLSA_REQUIRE(freq->ptr && freq->ndim == 2 && freq->shape[0] == S && freq->shape[1] == C && freq->stride[1] == 1, LLSA_ERR_SHAPE,
+                 "rms_rope_bwd: freq must be [S,64] with unit inner stride");
+    LLSA_REQUIRE(freq->dtype == dt || freq->dtype == LLSA_F32, LLSA_ERR_DTYPE, "rms_rope_bwd: the table must be f32 or have the dtype of the data");
+    LLSA_REQUIRE(((uintptr_t) freq->ptr % 16) == 0 && (freq->stride[0] * (int64_t) dtype_size(freq->dtype)) % 16 == 0, LLSA_ERR_STRIDE,
+                 "rms_rope_bwd: table rows must be 16-byte aligned");
+  }
+  if (B * H * S == 0) return LLSA_OK;
+  cudaStream_t st = (cudaStream_t) stream;
+  return dt == LLSA_F32 ? front_bwd_typed<float>(n_tensors, dy, x, norm_weight, norm_mask, eps, freq, dx, dw_partial, dw, st)
+                        : front_bwd_typed<__nv_bfloat16>(n_tensors, dy, x, norm_weight, norm_mask, eps, freq, dx, dw_partial, dw, st);
+}
