@@ -109,6 +109,20 @@ def lib() -> C.CDLL:
     return _lib
 
 
+def host():
+    """The native host path of the operators (_host.so, csrc/host.cpp); builds it first if it is missing."""
+    lib()
+    with _lock:
+        if not os.path.exists(os.path.join(_PKG, "_host.so")):
+            from . import build as _build
+            _build.build(force=True)
+        try:
+            from . import _host
+        except ImportError as e:   # pragma: no cover
+            raise RuntimeError("llsa_b200: cannot load _host.so (%s); run `python -m llsa_b200.build --force`" % e)
+    return _host
+
+
 def desc(t: Optional[torch.Tensor]) -> Optional[LlsaTensor]:
     if t is None:
         return None

@@ -13,20 +13,21 @@ unchanged:
     llsa_l1, llsa_l2                           torch_op/flash_sparse_attention_res_1.py:41, _res_2.py:48
 
 Every function enqueues CUDA work on the current stream through
-libllsa_b200.so; tensors must live on a CUDA device.  The differentiable
-entry points are torch.library custom ops with registered autograd.
+libllsa_b200.so; tensors must live on a CUDA device.  llsa_l1 / llsa_l2 and their
+fused forms are one dispatcher operator each way with C++ autograd
+(csrc/host.cpp); mean_pool1d and my_rope_fn are torch.library custom ops.
 """
 from __future__ import annotations
 
 import ctypes as C
-import math
 import os
+import threading
 from typing import List, Optional, Tuple
 
 import torch
 
 from . import _lib
-from ._lib import desc, ptr, ref
+from ._lib import desc, ref
 
 __all__ = [
     "mean_pool1d", "my_rope_fn", "gen_sparse_indices", "compute_topk_indices_sparse", "transpose_indices",
@@ -47,12 +48,10 @@ _exact_pooled_grad = os.environ.get("LLSA_B200_EXACT_POOLED_GRAD", "0") == "1"
 
 _stage_hook = None
 _overlap_transpose = os.environ.get("LLSA_B200_OVERLAP_TRANSPOSE", "1") != "0"
-_side_streams = {}
 # Cross-check switch: keep the pooled-key stages on the mma.sync kernels (the form other shapes use).
 _no_tcgen05 = False
 # Cross-check switch: False = long pooled key lists take two passes over the keys for every row (no `fwd_redo` scratch).
 _one_pass_pooled = True
-_last_fwd_redo = None        # the marks of the most recent forward (tests look at how many rows the second launch redid)
 # Test hook: polls after which a bounded wait inside the tcgen05 kernels gives up (0 = the kernels' default).
 _wait_limit = 0
 # Device-side checks.  The kernels OR bits into a status word when they meet an out-of-range block index or when a
@@ -66,6 +65,7 @@ def set_device_checks(flag: bool) -> None:
     met an out-of-range block index or gave up a bounded wait."""
     global _device_checks
     _device_checks = bool(flag)
+    _native()
 
 
 def _new_status(device):
@@ -77,19 +77,13 @@ def _check_status(status, what: str) -> None:
         _lib.check(_lib.lib().llsa_status_check(int(status.item())), what)
 
 
-def _side_stream(device) -> "torch.cuda.Stream":
-    key = (device.type, device.index if device.index is not None else torch.cuda.current_device())
-    if key not in _side_streams:
-        _side_streams[key] = torch.cuda.Stream(device)
-    return _side_streams[key]
-
-
 def set_stage_hook(fn) -> None:
     """fn(name) is called right before each kernel group is enqueued (and with
     "end" after the last one of an operator); None disables it.  Used by the
     benchmark to bracket kernels with CUDA events."""
     global _stage_hook
     _stage_hook = fn
+    _native().set_stage_hook(fn)
 
 
 def _mark(name: str) -> None:
@@ -102,6 +96,75 @@ def set_exact_pooled_grad(flag: bool) -> None:
     mathematically exact (True) pooled-key gradient of llsa_l1."""
     global _exact_pooled_grad
     _exact_pooled_grad = bool(flag)
+    _native()
+
+
+# ----------------------------------------------------------------------------- native host path
+_host = None
+_host_lock = threading.Lock()
+_configured = None
+
+
+def _native():
+    """The native host path (csrc/host.cpp), with this module's settings handed over if they changed since the last call."""
+    global _host, _configured
+    if _host is None:
+        with _host_lock:
+            if _host is None:
+                module = _lib.host()
+                _register_fakes()
+                _host = module
+    now = (_force_generic, _no_tcgen05, _exact_pooled_grad, _one_pass_pooled, _device_checks, _overlap_transpose, _wait_limit)
+    if now != _configured:
+        flags = ((1 if _force_generic else 0) | (2 if _no_tcgen05 else 0) | (4 if _exact_pooled_grad else 0) | (0 if _one_pass_pooled else 8) |
+                 (16 if _device_checks else 0) | (0 if _overlap_transpose else 32))
+        _host.configure(flags, int(_wait_limit))
+        _configured = now
+    return _host
+
+
+def __getattr__(name):
+    if name == "_last_fwd_redo":      # the marks of the most recent forward over a long pooled list: which rows its second launch redid
+        _native()
+        return torch.ops.llsa_b200.last_fwd_redo()
+    raise AttributeError("module %r has no attribute %r" % (__name__, name))
+
+
+def _saved_specs(B, H, N, D, dtype, topk1, topk2, block_size, levels):
+    """Layout of the buffer a layer's forward leaves for its backward (csrc/host.cpp: Saved): [(name, dtype, shape)]."""
+    n1 = N // block_size
+    n2 = n1 // block_size
+    i32 = torch.int32
+    specs = [("lse", torch.float32, (B, H, N)), ("indices", i32, (B, H, n1, min(topk1, n1) if levels == 1 else topk1))]
+    if levels == 2:
+        specs.append(("p_indices", i32, (B, H, n2, min(topk2, n2))))
+    specs += [("pk", dtype, (B, H, n1, D)), ("pv", dtype, (B, H, n1, D))]
+    if levels == 2:
+        specs += [("pk2", dtype, (B, H, n2, D)), ("pv2", dtype, (B, H, n2, D))]
+    return specs
+
+
+def _register_fakes() -> None:
+    """Shapes of the native operators for tracing."""
+    @torch.library.register_fake("llsa_b200::layer_fwd")
+    def _(q, k, v, freq, wq, wk, eps, topk1, topk2, block_size, levels):
+        specs = _saved_specs(*q.shape, q.dtype, topk1, topk2, block_size, levels)
+        out = [torch.empty_like(q), q.new_empty((_carve_bytes(specs),), dtype=torch.uint8)]
+        return out + ([torch.empty_like(q), torch.empty_like(k)] if freq is not None or wq is not None or wk is not None else [])
+
+    @torch.library.register_fake("llsa_b200::layer_bwd")
+    def _(d_o, q, k, v, o, saved, freq, xq, xk, wq, wk, eps, topk1, topk2, block_size, levels, want_dw):
+        out = [torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)]
+        return out + ([torch.empty_like(w) for w in (wq, wk) if w is not None] if want_dw else [])
+
+    @torch.library.register_fake("llsa_b200::attn_fwd")
+    def _(q, k, v, pk, pv, pk2, pv2, indices, p_indices, topk, topk_p, block_size, w1, w2):
+        return [torch.empty_like(q), q.new_empty(q.shape[:-1], dtype=torch.float32)]
+
+    @torch.library.register_fake("llsa_b200::attn_bwd")
+    def _(d_o, q, k, v, pk, pv, pk2, pv2, o, lse, indices, p_indices, topk, topk_p, block_size, w1, w2, kvw1, kvw2, fold):
+        pooled = [pk, pv] + ([pk2, pv2] if pk2 is not None else [])
+        return [torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)] + [p.new_empty(p.shape, dtype=torch.float32) for p in pooled]
 
 
 def _need_cuda(*ts: torch.Tensor) -> None:
@@ -299,17 +362,6 @@ def rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], eps: float = 1e-5)
     return y
 
 
-def _rms_norm_bwd(x: torch.Tensor, weight: Optional[torch.Tensor], eps: float, dy: torch.Tensor):
-    """Gradient of y = (x * rsqrt(mean(x^2) + eps)) * w with respect to x and w (fp32 arithmetic, eager)."""
-    xf, g = x.float(), dy.float()
-    rstd = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
-    xh = xf * rstd
-    gw = g * weight.float() if weight is not None else g
-    dx = rstd * (gw - xh * (gw * xh).mean(-1, keepdim=True))
-    dw = (g * xh).reshape(-1, x.shape[-1]).sum(0).to(weight.dtype) if weight is not None else None
-    return dx.to(x.dtype), dw
-
-
 # ----------------------------------------------------------------------------- RoPE
 def _rope_impl(x: torch.Tensor, freq: torch.Tensor, bwd: bool) -> torch.Tensor:
     _need_cuda(x, freq)
@@ -460,46 +512,10 @@ def transpose_indices(q_topk_indices: torch.Tensor, k_ntx: Optional[int] = None,
 
 
 # ----------------------------------------------------------------------------- attention core
-def _attn_args(q, k, v, pk, pv, pk2, pv2, indices, p_indices, o, lse, topk, topk_p, block_size, w1, w2):
-    keep = dict(q=desc(q), k=desc(k), v=desc(v), pk=desc(pk), pv=desc(pv), pk2=desc(pk2), pv2=desc(pv2),
-                indices=desc(indices), p_indices=desc(p_indices), o=desc(o), lse=desc(lse))
-    a = _lib.LlsaAttnArgs()
-    for name, d in keep.items():
-        setattr(a, name, ptr(d))
-    a.topk, a.topk_p, a.block_size = int(topk), int(topk_p), int(block_size)
-    a.token_weight, a.token_weight_2 = float(w1), float(w2)
-    a.force_generic = 1 if _force_generic else 0
-    a.no_tcgen05 = 1 if _no_tcgen05 else 0
-    a.wait_limit = int(_wait_limit)
-    return a, keep
-
-
 def _attn_fwd(q, k, v, pk, pv, pk2, pv2, indices, p_indices, topk, topk_p, block_size, w1, w2):
-    _need_cuda(q, k, v)
-    _check_float(q, k, v, pk, pv)
-    q, k, v = _prep(q), _prep(k), _prep(v)
-    pk, pv = pk.contiguous(), pv.contiguous()
-    if pk2 is not None:
-        pk2, pv2, p_indices = pk2.contiguous(), pv2.contiguous(), p_indices.contiguous()
-    indices = indices.contiguous()
-    o = torch.empty_like(q)
-    lse = torch.empty(q.shape[:-1], device=q.device, dtype=torch.float32)
-    a, keep = _attn_args(q, k, v, pk, pv, pk2, pv2, indices, p_indices, o, lse, topk, topk_p, block_size, w1, w2)
-    status = _new_status(q.device)
-    a.status = status.data_ptr() if status is not None else None
-    # one byte per query row for the one-pass form of the long pooled key lists (include/llsa_b200.h: fwd_redo)
-    one_pass = q.dtype == torch.bfloat16 and _one_pass_pooled
-    redo = torch.empty((q.shape[0] * q.shape[1] * q.shape[2] + 3) // 4, device=q.device, dtype=torch.int32) if one_pass else None
-    redo_d = desc(redo)
-    a.fwd_redo = ptr(redo_d)
-    _mark("attn_fwd")
-    with torch.cuda.device(q.device):
-        _lib.check(_lib.lib().llsa_attn_fwd(C.byref(a), _stream(q)), "attn_fwd")
-    _mark("end")
-    _check_status(status, "attn_fwd")
-    global _last_fwd_redo
-    _last_fwd_redo = redo
-    return o, lse
+    _native()
+    return tuple(torch.ops.llsa_b200.attn_fwd(q, k, v, pk, pv, pk2, pv2, indices, p_indices, int(topk), int(topk_p), int(block_size), float(w1),
+                                              float(w2)))
 
 
 def _rows_ok(t: torch.Tensor) -> bool:
@@ -527,76 +543,10 @@ def _carve_bytes(specs) -> int:
 
 
 def _attn_bwd(do, q, k, v, pk, pv, pk2, pv2, o, lse, indices, p_indices, topk, topk_p, block_size, w1, w2, kvw1, kvw2, fold):
-    _need_cuda(do, q, k, v)
-    q, k, v, o, do = _prep(q), _prep(k), _prep(v), _prep(o), _prep(do)
-    pk, pv = pk.contiguous(), pv.contiguous()
-    if pk2 is not None:
-        pk2, pv2, p_indices = pk2.contiguous(), pv2.contiguous(), p_indices.contiguous()
-    indices = indices.contiguous()
-    lse = lse.contiguous()
-    B, H, Nq, T = q.shape[0], q.shape[1], q.shape[2], indices.shape[3]
-    tensor_core = q.dtype == torch.bfloat16 and not _force_generic
-    # The index transpose (one CTA per (b,h): a latency-bound kernel that leaves most SMs idle) is needed only by the fine
-    # dK/dV stage, so it runs on a side stream next to the dQ and pooled stages.
-    cur = torch.cuda.current_stream(q.device)
-    side = _side_stream(q.device) if _overlap_transpose and _stage_hook is None else None     # a stage hook times every stage on ONE stream
-    n_kv = k.shape[2] // block_size                       # buckets = KEY blocks
-    if side is not None:
-        side.wait_stream(cur)
-        with torch.cuda.stream(side):
-            offsets, flat, (pairs, ranges), t_status = _transpose(indices, n_kv, torch.int32, tensor_core)
-    else:
-        offsets, flat, (pairs, ranges), t_status = _transpose(indices, n_kv, torch.int32, tensor_core)
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    # every scratch tensor of the call comes out of ONE allocation; the fp32 pooled-gradient accumulators sit back to back in
-    # it (the library clears them with one memset)
-    f32 = torch.float32
-    specs = [("delta", f32, lse.shape), ("dpk", f32, pk.shape), ("dpv", f32, pv.shape)]
-    if pk2 is not None:
-        specs += [("dpk2", f32, pk2.shape), ("dpv2", f32, pv2.shape)]
-    if tensor_core:     # window partials of the fine dK/dV kernel and the P / dS hand-over (csrc/attn_bwd_mma.cu)
-        L = _lib.lib()
-        specs += [("partial", f32, (B, H, L.llsa_attn_bwd_partial_elems(B, H, Nq, T) // (B * H * 4096), 4096)),
-                  ("pds", f32, (L.llsa_attn_bwd_pds_elems(B, H, Nq, T),))]
-    ws = _carve(torch.empty(_carve_bytes(specs), device=q.device, dtype=torch.uint8), specs)
-    delta, dpk, dpv = ws["delta"], ws["dpk"], ws["dpv"]
-    dpk2, dpv2 = ws.get("dpk2"), ws.get("dpv2")
-    a, keep = _attn_args(q, k, v, pk, pv, pk2, pv2, indices, p_indices, o, lse, topk, topk_p, block_size, w1, w2)
-    status = _new_status(q.device)
-    a.status = status.data_ptr() if status is not None else None
-    extra = dict(d_o=desc(do), dq=desc(dq), dk=desc(dk), dv=desc(dv), offsets=desc(offsets), flat=desc(flat), delta=desc(delta),
-                 dpk_acc=desc(dpk), dpv_acc=desc(dpv), dpk2_acc=desc(dpk2), dpv2_acc=desc(dpv2), dkv_partial=desc(ws.get("partial")),
-                 fine_pds=desc(ws.get("pds")), flat_pairs=desc(pairs), flat_ranges=desc(ranges))
-    for name, d in extra.items():
-        setattr(a, name, ptr(d))
-    a.fold_pool_bwd = 1 if fold else 0
-    a.kv_weight, a.kv_weight_2 = float(kvw1), float(kvw2)
-
-    def join_side():
-        cur.wait_stream(side)                 # the CSR is ready; its memory now also belongs to this stream
-        for t in (offsets, flat) + ((pairs, ranges) if pairs is not None else ()):
-            t.record_stream(cur)
-
-    with torch.cuda.device(q.device):
-        if _stage_hook is None and side is None:
-            _lib.check(_lib.lib().llsa_attn_bwd(C.byref(a), _stream(q)), "attn_bwd")
-        elif _stage_hook is None:             # dQ and pooled stages, then the CSR's stream joins, then dK/dV
-            a.stage_mask = 3
-            _lib.check(_lib.lib().llsa_attn_bwd(C.byref(a), _stream(q)), "attn_bwd")
-            join_side()
-            a.stage_mask = 4
-            _lib.check(_lib.lib().llsa_attn_bwd(C.byref(a), _stream(q)), "attn_bwd")
-        else:
-            for mask, name in ((1, "attn_bwd_dq"), (2, "attn_bwd_dkv_pooled"), (4, "attn_bwd_dkv_fine")):
-                if mask == 4 and side is not None:
-                    join_side()
-                _mark(name)
-                a.stage_mask = mask
-                _lib.check(_lib.lib().llsa_attn_bwd(C.byref(a), _stream(q)), name)
-            _mark("end")
-    _check_status(t_status, "transpose_indices")
-    _check_status(status, "attn_bwd")
-    return dq, dk, dv, dpk, dpv, dpk2, dpv2
+    _native()
+    g = torch.ops.llsa_b200.attn_bwd(do, q, k, v, pk, pv, pk2, pv2, o, lse, indices, p_indices, int(topk), int(topk_p), int(block_size), float(w1),
+                                     float(w2), float(kvw1), float(kvw2), bool(fold))
+    return tuple(g) + (None,) * (7 - len(g))
 
 
 def sparse_indices_attn_res_fwd(q, k, v, pk, pv, indices, topk, token_weight=1, down_scale=4):
@@ -675,242 +625,60 @@ flash_sparse_residual_attention_l2_op = _FlashSparseResidualAttentionL2.apply
 
 
 # ----------------------------------------------------------------------------- fused drop-in operators
-@torch.library.custom_op("llsa_b200::llsa_l1_fwd", mutates_args=())
-def _llsa_l1_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, topk: int, block_size: int) -> List[torch.Tensor]:
-    (pq, pk, pv), _ = pool_pyramid([q, k, v], block_size, 1)
-    indices = _coarse_topk(pq, pk, topk)
-    o, lse = _attn_fwd(q, k, v, pk, pv, None, None, indices, None, indices.shape[-1], 0, block_size, float(block_size), 1.0)
-    return [o, lse, indices, pk, pv]
-
-
-@_llsa_l1_fwd.register_fake
-def _(q, k, v, topk, block_size):
-    B, H, N, D = q.shape
-    n1 = N // block_size
-    return [torch.empty_like(q), q.new_empty((B, H, N), dtype=torch.float32), q.new_empty((B, H, n1, min(topk, n1)), dtype=torch.int32),
-            k.new_empty((B, H, n1, D)), v.new_empty((B, H, n1, D))]
-
-
-@torch.library.custom_op("llsa_b200::llsa_l1_bwd", mutates_args=())
-def _llsa_l1_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Tensor, lse: torch.Tensor,
-                 indices: torch.Tensor, pk: torch.Tensor, pv: torch.Tensor, block_size: int, exact: bool) -> List[torch.Tensor]:
-    w = float(block_size)
-    dq, dk, dv, _, _, _, _ = _attn_bwd(do, q, k, v, pk, pv, None, None, o, lse, indices, None, indices.shape[-1], 0, block_size,
-                                       w, 1.0, w if exact else 1.0, 1.0, True)
-    return [dq, dk, dv]
-
-
-@_llsa_l1_bwd.register_fake
-def _(do, q, k, v, o, lse, indices, pk, pv, block_size, exact):
-    return [torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)]
-
-
-def _l1_setup(ctx, inputs, output):
-    q, k, v, topk, block_size = inputs
-    o, lse, indices, pk, pv = output
-    ctx.save_for_backward(q, k, v, o, lse, indices, pk, pv)
-    ctx.block_size = block_size
-    ctx.set_materialize_grads(False)       # only o carries a gradient: no zero-filled stand-ins for the other outputs
-
-
-def _l1_backward(ctx, grads):
-    if grads[0] is None:
-        return None, None, None, None, None
-    q, k, v, o, lse, indices, pk, pv = ctx.saved_tensors
-    dq, dk, dv = _llsa_l1_bwd(grads[0], q, k, v, o, lse, indices, pk, pv, ctx.block_size, _exact_pooled_grad)
-    return dq, dk, dv, None, None
-
-
-_llsa_l1_fwd.register_autograd(_l1_backward, setup_context=_l1_setup)
-
-
-@torch.library.custom_op("llsa_b200::llsa_l2_fwd", mutates_args=())
-def _llsa_l2_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, topk1: int, topk2: int, block_size: int) -> List[torch.Tensor]:
-    (pq, pk, pv), (pq2, pk2, pv2) = pool_pyramid([q, k, v], block_size, 2)
-    indices, p_indices = _select_two_level(pq, pk, pq2, pk2, topk1, topk2, block_size)
-    o, lse = _attn_fwd(q, k, v, pk, pv, pk2, pv2, indices, p_indices, topk1, p_indices.shape[-1], block_size,
-                       float(block_size), float(block_size * block_size))
-    return [o, lse, indices, p_indices, pk, pv, pk2, pv2]
-
-
-@_llsa_l2_fwd.register_fake
-def _(q, k, v, topk1, topk2, block_size):
-    B, H, N, D = q.shape
-    n1 = N // block_size
-    n2 = n1 // block_size
-    return [torch.empty_like(q), q.new_empty((B, H, N), dtype=torch.float32), q.new_empty((B, H, n1, topk1), dtype=torch.int32),
-            q.new_empty((B, H, n2, min(topk2, n2)), dtype=torch.int32), k.new_empty((B, H, n1, D)), v.new_empty((B, H, n1, D)),
-            k.new_empty((B, H, n2, D)), v.new_empty((B, H, n2, D))]
-
-
-@torch.library.custom_op("llsa_b200::llsa_l2_bwd", mutates_args=())
-def _llsa_l2_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Tensor, lse: torch.Tensor,
-                 indices: torch.Tensor, p_indices: torch.Tensor, pk: torch.Tensor, pv: torch.Tensor, pk2: torch.Tensor,
-                 pv2: torch.Tensor, block_size: int) -> List[torch.Tensor]:
-    w1, w2 = float(block_size), float(block_size * block_size)
-    dq, dk, dv, _, _, _, _ = _attn_bwd(do, q, k, v, pk, pv, pk2, pv2, o, lse, indices, p_indices, indices.shape[-1],
-                                       p_indices.shape[-1], block_size, w1, w2, w1, w2, True)
-    return [dq, dk, dv]
-
-
-@_llsa_l2_bwd.register_fake
-def _(do, q, k, v, o, lse, indices, p_indices, pk, pv, pk2, pv2, block_size):
-    return [torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)]
-
-
-def _l2_setup(ctx, inputs, output):
-    q, k, v, topk1, topk2, block_size = inputs
-    o, lse, indices, p_indices, pk, pv, pk2, pv2 = output
-    ctx.save_for_backward(q, k, v, o, lse, indices, p_indices, pk, pv, pk2, pv2)
-    ctx.block_size = block_size
-    ctx.set_materialize_grads(False)
-
-
-def _l2_backward(ctx, grads):
-    if grads[0] is None:
-        return None, None, None, None, None, None
-    q, k, v, o, lse, indices, p_indices, pk, pv, pk2, pv2 = ctx.saved_tensors
-    dq, dk, dv = _llsa_l2_bwd(grads[0], q, k, v, o, lse, indices, p_indices, pk, pv, pk2, pv2, ctx.block_size)
-    return dq, dk, dv, None, None, None
-
-
-_llsa_l2_fwd.register_autograd(_l2_backward, setup_context=_l2_setup)
-
-
-# ----------------------------------------------------------------------------- RoPE fused in front of the operators
-@torch.library.custom_op("llsa_b200::llsa_rope_fwd", mutates_args=())
-def _llsa_rope_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, freq: torch.Tensor, topk1: int, topk2: int, block_size: int,
-                   levels: int) -> List[torch.Tensor]:
-    (qr, kr, _), l1, l2 = rope_pool_pyramid([q, k, v], freq, [True, True, False], block_size, levels)
-    pq, pk, pv = l1
-    bs = block_size
-    if levels == 2:
-        pq2, pk2, pv2 = l2
-        indices, p_indices = _select_two_level(pq, pk, pq2, pk2, topk1, topk2, bs)
-        o, lse = _attn_fwd(qr, kr, v, pk, pv, pk2, pv2, indices, p_indices, topk1, p_indices.shape[-1], bs, float(bs), float(bs * bs))
-        return [o, lse, qr, kr, indices, pk, pv, p_indices, pk2, pv2]
-    indices = _coarse_topk(pq, pk, topk1)
-    o, lse = _attn_fwd(qr, kr, v, pk, pv, None, None, indices, None, indices.shape[-1], 0, bs, float(bs), 1.0)
-    return [o, lse, qr, kr, indices, pk, pv]
-
-
-@_llsa_rope_fwd.register_fake
-def _(q, k, v, freq, topk1, topk2, block_size, levels):
-    B, H, N, D = q.shape
-    n1 = N // block_size
-    n2 = n1 // block_size
-    out = [torch.empty_like(q), q.new_empty((B, H, N), dtype=torch.float32), torch.empty_like(q), torch.empty_like(k),
-           q.new_empty((B, H, n1, min(topk1, n1) if levels == 1 else topk1), dtype=torch.int32), k.new_empty((B, H, n1, D)), v.new_empty((B, H, n1, D))]
-    if levels == 2:
-        out += [q.new_empty((B, H, n2, min(topk2, n2)), dtype=torch.int32), k.new_empty((B, H, n2, D)), v.new_empty((B, H, n2, D))]
-    return out
-
-
-def _rope_op_setup(ctx, inputs, output):
-    q, k, v, freq, topk1, topk2, block_size, levels = inputs
-    ctx.save_for_backward(v, freq, *output)
-    ctx.block_size, ctx.levels = block_size, levels
-    ctx.set_materialize_grads(False)
-
-
-def _rope_op_backward(ctx, grads):
-    if grads[0] is None:
-        return (None,) * 8
-    v, freq, o, lse, qr, kr, indices, pk, pv = ctx.saved_tensors[:9]
-    if ctx.levels == 2:
-        p_indices, pk2, pv2 = ctx.saved_tensors[9:]
-        dqr, dkr, dv = _llsa_l2_bwd(grads[0], qr, kr, v, o, lse, indices, p_indices, pk, pv, pk2, pv2, ctx.block_size)
-    else:
-        dqr, dkr, dv = _llsa_l1_bwd(grads[0], qr, kr, v, o, lse, indices, pk, pv, ctx.block_size, _exact_pooled_grad)
-    return _rope_bwd_op(dqr, freq), _rope_bwd_op(dkr, freq), dv, None, None, None, None, None
-
-
-_llsa_rope_fwd.register_autograd(_rope_op_backward, setup_context=_rope_op_setup)
+def _layer(q, k, v, freq, wq, wk, eps, topk1, topk2, block_size, levels):
+    _native()
+    return torch.ops.llsa_b200.layer_fwd(q, k, v, freq, wq, wk, eps, topk1, topk2, block_size, levels)
 
 
 def llsa_l1_rope(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, freq: torch.Tensor, topk: int = 8, block_size: int = 16) -> torch.Tensor:
     """llsa_l1(my_rope_fn(q, freq), my_rope_fn(k, freq), v, topk, block_size) -- what RopeAttnProcessor computes
     (models/rope_dit_transformer_2d.py:232-241) -- with the rotation fused into the pooling pass."""
-    return _llsa_rope_fwd(q, k, v, freq, topk, 0, block_size, 1)[0]
+    return _layer(q, k, v, freq, None, None, 0.0, topk, 0, block_size, 1)[0]
 
 
 def llsa_l2_rope(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, freq: torch.Tensor, topk1: int = 8, topk2: int = 8,
                  block_size: int = 16) -> torch.Tensor:
     """llsa_l2(my_rope_fn(q, freq), my_rope_fn(k, freq), v, topk1, topk2, block_size)
     (models/rope_dit_transformer_2d.py:232-251) with the rotation fused into the pooling pass."""
-    return _llsa_rope_fwd(q, k, v, freq, topk1, topk2, block_size, 2)[0]
-
-
-class _LlsaRmsRope(torch.autograd.Function):
-    """llsa_l1 / llsa_l2 on RMS-normalised, rotated q and k: normalisation, rotation and pooling in one pass forward; the
-    backward runs the operator's backward, then the rotation's and the normalisation's."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, wq, wk, freq, eps, topk1, topk2, block_size, levels):
-        bs = block_size
-        (qr, kr, _), l1, l2 = rms_rope_pool_pyramid([q.detach(), k.detach(), v.detach()], [wq, wk, None], eps, freq, [True, True, False], bs, levels)
-        pq, pk, pv = l1
-        vd = v.detach()
-        if levels == 2:
-            pq2, pk2, pv2 = l2
-            indices, p_indices = _select_two_level(pq, pk, pq2, pk2, topk1, topk2, bs)
-            o, lse = _attn_fwd(qr, kr, vd, pk, pv, pk2, pv2, indices, p_indices, topk1, p_indices.shape[-1], bs, float(bs), float(bs * bs))
-            extra = [p_indices, pk2, pv2]
-        else:
-            indices = _coarse_topk(pq, pk, topk1)
-            o, lse = _attn_fwd(qr, kr, vd, pk, pv, None, None, indices, None, indices.shape[-1], 0, bs, float(bs), 1.0)
-            extra = []
-        ctx.save_for_backward(q, k, v, wq, wk, freq, o, lse, qr, kr, indices, pk, pv, *extra)
-        ctx.cfg = (float(eps), bs, levels)
-        return o
-
-    @staticmethod
-    def backward(ctx, do):
-        eps, bs, levels = ctx.cfg
-        q, k, v, wq, wk, freq, o, lse, qr, kr, indices, pk, pv = ctx.saved_tensors[:13]
-        if levels == 2:
-            p_indices, pk2, pv2 = ctx.saved_tensors[13:]
-            dqr, dkr, dv = _llsa_l2_bwd(do, qr, kr, v, o, lse, indices, p_indices, pk, pv, pk2, pv2, bs)
-        else:
-            dqr, dkr, dv = _llsa_l1_bwd(do, qr, kr, v, o, lse, indices, pk, pv, bs, _exact_pooled_grad)
-        dq, dwq = _rms_norm_bwd(q, wq, eps, _rope_bwd_op(dqr, freq))
-        dk, dwk = _rms_norm_bwd(k, wk, eps, _rope_bwd_op(dkr, freq))
-        return dq, dk, dv, dwq, dwk, None, None, None, None, None, None
+    return _layer(q, k, v, freq, None, None, 0.0, topk1, topk2, block_size, 2)[0]
 
 
 def llsa_l1_rms_rope(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, freq: torch.Tensor,
                      eps: float = 1e-5, topk: int = 8, block_size: int = 16) -> torch.Tensor:
     """llsa_l1(my_rope_fn(norm_q(q)), my_rope_fn(norm_k(k)), v, topk, block_size): the whole q / k preparation of the attention
     block (models/rope_dit_transformer_2d.py:215-241) fused into the pooling pass.  wq, wk: RMSNorm weights [D]."""
-    return _LlsaRmsRope.apply(q, k, v, wq, wk, freq, eps, topk, 0, block_size, 1)
+    return _layer(q, k, v, freq, wq, wk, eps, topk, 0, block_size, 1)[0]
 
 
 def llsa_l2_rms_rope(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, freq: torch.Tensor,
                      eps: float = 1e-5, topk1: int = 8, topk2: int = 8, block_size: int = 16) -> torch.Tensor:
     """llsa_l2 on RMS-normalised, rotated q and k (models/rope_dit_transformer_2d.py:215-251), q / k read once."""
-    return _LlsaRmsRope.apply(q, k, v, wq, wk, freq, eps, topk1, topk2, block_size, 2)
+    return _layer(q, k, v, freq, wq, wk, eps, topk1, topk2, block_size, 2)[0]
 
 
 def llsa_l1(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, topk: int = 8, block_size: int = 16) -> torch.Tensor:
     """One-level log-linear sparse attention; q, k, v [B,H,N,D] (any batch/head/token
     strides), returns o like q; differentiable in q, k, v.  Drop-in for llsa_l1
     (torch_op/flash_sparse_attention_res_1.py:41-47)."""
-    return _llsa_l1_fwd(q, k, v, topk, block_size)[0]
+    return _layer(q, k, v, None, None, None, 0.0, topk, 0, block_size, 1)[0]
 
 
 def llsa_l2(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, topk1: int = 8, topk2: int = 8, block_size: int = 16) -> torch.Tensor:
     """Two-level log-linear sparse attention.  Drop-in for llsa_l2
     (torch_op/flash_sparse_attention_res_2.py:48-59)."""
-    return _llsa_l2_fwd(q, k, v, topk1, topk2, block_size)[0]
+    return _layer(q, k, v, None, None, None, 0.0, topk1, topk2, block_size, 2)[0]
+
+
+def _layer_debug(q, k, v, topk1, topk2, block_size, levels):
+    o, saved = _layer(q, k, v, None, None, None, 0.0, topk1, topk2, block_size, levels)
+    return dict(o=o, **_carve(saved, _saved_specs(*q.shape, q.dtype, topk1, topk2, block_size, levels)))
 
 
 def llsa_l1_debug(q, k, v, topk=8, block_size=16):
     """llsa_l1 returning its intermediates: dict(o, lse, indices, pk, pv)."""
-    o, lse, indices, pk, pv = _llsa_l1_fwd(q, k, v, topk, block_size)
-    return dict(o=o, lse=lse, indices=indices, pk=pk, pv=pv)
+    return _layer_debug(q, k, v, topk, 0, block_size, 1)
 
 
 def llsa_l2_debug(q, k, v, topk1=8, topk2=8, block_size=16):
     """llsa_l2 returning its intermediates: dict(o, lse, indices, p_indices, pk, pv, pk2, pv2)."""
-    o, lse, indices, p_indices, pk, pv, pk2, pv2 = _llsa_l2_fwd(q, k, v, topk1, topk2, block_size)
-    return dict(o=o, lse=lse, indices=indices, p_indices=p_indices, pk=pk, pv=pv, pk2=pk2, pv2=pv2)
+    return _layer_debug(q, k, v, topk1, topk2, block_size, 2)
