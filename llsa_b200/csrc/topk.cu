@@ -140,116 +140,299 @@ coarse_topk_kernel(const T* __restrict__ pq, const T* __restrict__ pk, void* __r
   }
 }
 
-// pq1: contiguous [B*H, M, D] (M query blocks); pk1: contiguous [B*H, Mk, D] (Mk key blocks, Mk != M when the
-// queries are a shard of the sequence); p_idx [B*H, M/bs, p_topk] with values in [0, Mk/bs); out [B*H, M, topk].
-// MMA = true (bf16, D = 64, bs = 16): the 16 x C score tile comes from mma.sync with fp32
-// accumulation of the exact bf16 products, as the reference's tl.dot does.
-
 // ---- coarse selection on the tensor cores (bf16, D = 64, top-k <= 8) ---------------------------
-// A CTA owns 64 query rows (16 per warp, the m16 of mma.sync.m16n8k16) and streams the keys through a
-// double-buffered shared-memory tile of 64 keys (cp.async).  Scores are rounded to bf16 as torch.matmul
-// would store them (topk.py:7); a lane sees columns 2t, 2t+1 (+8) of rows g and g+8 of every 16-key
-// block and keeps the best 8 of each of its two rows in sorted registers -- columns arrive in
-// increasing order and an equal score never displaces an earlier one, so ties go to the smallest index.
-// The four lanes of a quad cover a row between them; their 4 x 8 candidates are merged at the end by
-// the warp (two reductions per output, as in the refine kernel below).
-constexpr int kCmRows = 64, kCmKeys = 64, kCmTop = 8;
+// Scores are rounded to bf16 as torch.matmul would store them (topk.py:7), so a score and its column fit one 32-bit word:
+// the order-preserving image of the bf16 value above the complemented column (65535 - column).  Larger word = better candidate,
+// ties already decided in favour of the smaller column, and a candidate list is kept sorted with integer minima and maxima.
+//   * A warp owns ROWT * 16 query rows (the m16 of mma.sync.m16n8k16) and every KW-th 16-key block; its key fragments come straight
+//     from L1 / L2 (one 256-bit load per lane and eight keys), the next block's while this one is scored.
+//   * Lists of 1024 keys and more: pass 1 scores all keys and keeps the maximum of each lane's columns per row.  The top-k-th largest
+//     of a row's 4 KW group maxima bounds its top-k-th score from below (with 16 groups some eleven scores of a row reach it,
+//     whatever its length).  Pass 2 scores the keys again and looks only at what reaches the bound: a quarter of the instructions per
+//     score, and few insertions.  Without a bound the kernel spends its time inserting: until a lane has seen most of its columns, some
+//     lane of the warp has something to insert in almost every block (235 us below).  A bound from every fourth block leaves
+//     four times as many insertions (158 us); below 1024 keys the two barriers cost what the bound saves.
+//   * The row's 4 KW sorted lists meet in shared memory: lane l holds list l, a round takes the largest head, its owner moves on.
+// Large problems are bound by the latency of a warp's product and comparison chains (four warps per scheduler, tensor pipe 41 % busy);
+// keys through a cp.async ring or 24 warps per SM of one row tile each changed nothing.  n = M = 4096, 8 slices: 243 us with one pass
+// and lists of (value, column) pairs in four-warp CTAs of 64 rows, 139 now; n = M = 1024, 8 slices: 59 -> 20; n = M = 256, 24
+// slices: 24 -> 6.7; n = M = 64, 6 slices: 14.9 -> 3.7.
+constexpr int kCmTop = 8, kCmWarps = 8, kCmBoundFrom = 1024;
+
+__device__ __forceinline__ uint32_t umax(uint32_t a, uint32_t b) { return a > b ? a : b; }
+__device__ __forceinline__ uint32_t umin(uint32_t a, uint32_t b) { return a < b ? a : b; }
+
+template <uint32_t SEL>
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b) {      // selector bit 3 of a byte: its sign, replicated (__byte_perm drops that bit)
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "n"(SEL));
+  return d;
+}
+
+// Candidate words of two neighbouring columns: cinv holds 65535 - c (low half) and 65535 - (c + 1) (high half).
+// NaN (0x7FFF after the conversion) ranks above everything as in torch.topk, -0 ties with +0.
+__device__ __forceinline__ void candidate_words(float s0, float s1, uint32_t cinv, uint32_t& k0, uint32_t& k1) {
+  __nv_bfloat162 p = __hadd2(__floats2bfloat162_rn(s0, s1), __float2bfloat162_rn(0.f));      // -0 + 0 = +0
+  const uint32_t u = *reinterpret_cast<uint32_t*>(&p);
+  const uint32_t o = u ^ (prmt<0xBB99>(u, 0u) | 0x80008000u);      // negative: all bits flipped, else the sign bit set
+  k0 = prmt<0x1054>(o, cinv);
+  k1 = prmt<0x3276>(o, cinv);
+}
+
+__device__ __forceinline__ float max_nan(float a, float b) {      // NaN if either is
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+
+__device__ __forceinline__ void list_insert(uint32_t (&list)[kCmTop], uint32_t k) {
+  list[kCmTop - 1] = umax(list[kCmTop - 1], k);
+#pragma unroll
+  for (int u = kCmTop - 1; u > 0; --u) {
+    const uint32_t hi = umax(list[u - 1], list[u]), lo = umin(list[u - 1], list[u]);
+    list[u - 1] = hi;
+    list[u] = lo;
+  }
+}
+
+// ROWT row tiles per warp, KW warps share a CTA's keys, the other kCmWarps / KW are further row tiles.
+template <int ROWT, int KW>
+__global__ void __launch_bounds__(kCmWarps * 32)
+coarse_topk_mma_kernel(const bf16* __restrict__ pq, const bf16* __restrict__ pk, void* __restrict__ idx_out, int idx64, int64_t M, int64_t n,
+                       int topk) {
+  constexpr int RG = kCmWarps / KW, ROWS = RG * ROWT * 16;
+  __shared__ uint32_t lists[ROWS][KW * 4 * kCmTop + 4];      // + 4: rows shift by four banks.  Pass 1: the group maxima
+  __shared__ uint32_t bound[ROWS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int kw = warp % KW, wrow = (warp / KW) * ROWT * 16;
+  const int64_t bh = blockIdx.y, row0 = (int64_t) blockIdx.x * ROWS + wrow;
+  const bf16* k0 = pk + bh * n * 64;
+  const int n_blk = (int) (n / 16);
+  RowFrag q[ROWT][2];
+#pragma unroll
+  for (int r = 0; r < ROWT; ++r) {                            // rows past M are computed and dropped
+    load_rowfrag(q[r][0], pq + (bh * M + min(row0 + r * 16 + g, M - 1)) * 64, t);
+    load_rowfrag(q[r][1], pq + (bh * M + min(row0 + r * 16 + g + 8, M - 1)) * 64, t);
+  }
+  // scores of this warp's blocks, one after the other: visit(block number, scores)
+  auto walk = [&](auto&& visit) {
+    RowFrag ka, kb;
+    if (kw < n_blk) {
+      load_rowfrag(ka, k0 + (int64_t) (kw * 16 + g) * 64, t);
+      load_rowfrag(kb, k0 + (int64_t) (kw * 16 + 8 + g) * 64, t);
+    }
+    for (int blk = kw; blk < n_blk; blk += KW) {
+      float s[ROWT][2][4];
+#pragma unroll
+      for (int r = 0; r < ROWT; ++r) mma_rows_x_keys_z(s[r][0], s[r][1], q[r][0], q[r][1], ka, kb);
+      if (blk + KW < n_blk) {
+        const int c = (blk + KW) * 16;
+        load_rowfrag(ka, k0 + (int64_t) (c + g) * 64, t);
+        load_rowfrag(kb, k0 + (int64_t) (c + 8 + g) * 64, t);
+      }
+      visit(blk, s);
+    }
+  };
+  // ---- pass 1: group maxima -> bounds
+  const bool bounded = n >= kCmBoundFrom;
+  if (bounded) {
+    float m[ROWT][2];
+#pragma unroll
+    for (int r = 0; r < ROWT; ++r) m[r][0] = m[r][1] = -CUDART_INF_F;
+    walk([&](int, const float (&s)[ROWT][2][4]) {
+#pragma unroll
+      for (int r = 0; r < ROWT; ++r)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          m[r][e] = fmax3(fmax3(m[r][e], s[r][0][2 * e], s[r][0][2 * e + 1]), s[r][1][2 * e], s[r][1][2 * e + 1]);
+    });
+#pragma unroll
+    for (int r = 0; r < ROWT; ++r)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {                      // no column, or none but -inf and NaN: 0, no bound
+        uint32_t w, other;
+        candidate_words(m[r][e], 0.f, 0u, w, other);
+        lists[wrow + r * 16 + g + 8 * e][kw * 4 + t] = m[r][e] > -CUDART_INF_F ? w & 0xFFFF0000u : 0u;
+      }
+    __syncthreads();
+    for (int r = warp; r < ROWS; r += kCmWarps) {
+      uint32_t x = lane < KW * 4 ? lists[r][lane] : 0u, best = 0u;
+      for (int u = 0; u < topk; ++u) {
+        best = __reduce_max_sync(0xffffffffu, x);
+        const unsigned who = __ballot_sync(0xffffffffu, x == best);
+        if (lane == __ffs((int) who) - 1) x = 0u;
+      }
+      if (lane == 0) bound[r] = best;
+    }
+    __syncthreads();
+  }
+  // ---- pass 2: what reaches the bound
+  uint32_t list[ROWT][2][kCmTop], thr[ROWT][2];
+  float low[ROWT][2];          // a score below this rounds to less than the bound
+#pragma unroll
+  for (int r = 0; r < ROWT; ++r)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const uint32_t w = bounded ? bound[wrow + r * 16 + g + 8 * e] : 0u;
+      thr[r][e] = w > 0u ? w - 1u : 0u;
+      const uint32_t below = (w >> 16) - ((w >> 16) == 0x8000u ? 2u : 1u);            // image of the bf16 value one step down (-0 is no step)
+      low[r][e] = w > 0x00800000u ? __uint_as_float((below & 0x8000u ? below ^ 0x8000u : ~below & 0xFFFFu) << 16) : -CUDART_INF_F;
+#pragma unroll
+      for (int u = 0; u < kCmTop; ++u) list[r][e][u] = 0u;
+    }
+  walk([&](int blk, const float (&s)[ROWT][2][4]) {
+    const uint32_t c = (uint32_t) (blk * 16 + 2 * t), inv0 = (65535u - c) | ((65534u - c) << 16), inv1 = inv0 - 0x00080008u;
+#pragma unroll
+    for (int r = 0; r < ROWT; ++r)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (max_nan(max_nan(s[r][0][2 * e], s[r][0][2 * e + 1]), max_nan(s[r][1][2 * e], s[r][1][2 * e + 1])) < low[r][e]) continue;      // false for NaN
+        uint32_t k[4];
+        candidate_words(s[r][0][2 * e], s[r][0][2 * e + 1], inv0, k[0], k[1]);
+        candidate_words(s[r][1][2 * e], s[r][1][2 * e + 1], inv1, k[2], k[3]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (k[u] > thr[r][e]) {
+            list_insert(list[r][e], k[u]);
+            thr[r][e] = umax(thr[r][e], list[r][e][kCmTop - 1]);
+          }
+      }
+  });
+#pragma unroll
+  for (int r = 0; r < ROWT; ++r)
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int u = 0; u < kCmTop; ++u) lists[wrow + r * 16 + g + 8 * e][(kw * 4 + t) * kCmTop + u] = list[r][e][u];
+  __syncthreads();
+  for (int r = warp; r < ROWS; r += kCmWarps) {
+    const int64_t row = (int64_t) blockIdx.x * ROWS + r;
+    if (row >= M) continue;
+    const uint32_t* mine = &lists[r][lane * kCmTop];
+    uint32_t head = lane < KW * 4 ? mine[0] : 0u, won = 0u;
+    int at = 0;
+    for (int u = 0; u < topk; ++u) {
+      const uint32_t best = __reduce_max_sync(0xffffffffu, head);
+      if (lane == u) won = best;
+      if (head == best) { ++at; head = at < kCmTop ? mine[at] : 0u; }      // candidate words are distinct: one owner
+    }
+    if (lane < topk) {
+      const int64_t o = (bh * M + row) * topk + lane;
+      const uint32_t col = 65535u - (won & 0xFFFFu);
+      if (idx64) reinterpret_cast<int64_t*>(idx_out)[o] = (int64_t) col;
+      else reinterpret_cast<int32_t*>(idx_out)[o] = (int32_t) col;
+    }
+  }
+}
+
+// ---- coarse selection with scalar arithmetic, D = 64, top-k <= 32 (fp32, and the bf16 shapes below) ------------------------
+// A score is one fp32 chain over the channels in order, so fp32 and the bf16 shapes that were always scored this way (list
+// lengths that are no multiple of 64, top-k above 8) keep their scores bit for bit.  A CTA owns 16 query rows and walks the keys in
+// chunks of 256 through shared memory; a thread scores 8 rows x 2 keys (64 FMAs per sixteen 128-bit shared loads: FMA and shared
+// pipes are in balance).  A row's running list lives in a warp, sorted, one candidate per lane; only candidates above its
+// last entry cost more than a comparison.  One thread per key and eight rows one after the other, with a scan over all scores per
+// winner (coarse_topk_kernel below, kept for other D and longer lists), took 18 us at n = M = 64, B H = 2 (fp32), 32 us at
+// n = M = 160, top-16, B H = 5 and 4850 us at n = M = 4064, B H = 8; this form 10.5, 18 and 865.
+constexpr int kCtRows = 16, kCtKeys = 256, kCtPitch = 68, kCtScPitch = kCtKeys + 4;
+constexpr size_t kCtSmem = ((size_t) (kCtRows + kCtKeys) * kCtPitch + (size_t) kCtRows * kCtScPitch) * 4;
 
 __device__ __forceinline__ uint32_t orderable(float v);
 
-__device__ __forceinline__ void top8_insert(float (&val)[kCmTop], int (&idx)[kCmTop], float v, int i) {
-  // NaN ranks first (torch.topk); -inf is lifted above the lists' initial -inf so that every column can enter:
-  // a lane always ends with eight real columns, whatever the scores are
-  v = v != v ? CUDART_INF_F : fmaxf(v, -3.0e38f);
-  if (!(v > val[kCmTop - 1])) return;
-  val[kCmTop - 1] = v;
-  idx[kCmTop - 1] = i;
-#pragma unroll
-  for (int u = kCmTop - 1; u > 0; --u) {
-    const bool sw = val[u] > val[u - 1];
-    const float tv = val[u];
-    const int ti = idx[u];
-    val[u] = sw ? val[u - 1] : tv;  idx[u] = sw ? idx[u - 1] : ti;
-    val[u - 1] = sw ? tv : val[u - 1];  idx[u - 1] = sw ? ti : idx[u - 1];
+// Sorted list of the best `topk` 64-bit candidates (score image above the complemented column) spread over a warp, lane u holding
+// the u-th; `thr` is the last one.  Every lane brings one candidate (0: none).
+__device__ __forceinline__ void warp_list_insert(uint64_t& list, uint64_t& thr, uint64_t cand, int topk, int lane) {
+  unsigned todo = __ballot_sync(0xffffffffu, cand > thr);
+  while (todo) {
+    const uint64_t c = __shfl_sync(0xffffffffu, cand, __ffs((int) todo) - 1);
+    const int pos = __popc(__ballot_sync(0xffffffffu, list > c));
+    const uint64_t up = __shfl_up_sync(0xffffffffu, list, 1);
+    list = lane == pos ? c : (lane > pos ? up : list);
+    thr = __shfl_sync(0xffffffffu, list, topk - 1);
+    todo &= (todo - 1) & __ballot_sync(0xffffffffu, cand > thr);
   }
 }
 
-__global__ void __launch_bounds__(128)
-coarse_topk_mma_kernel(const bf16* __restrict__ pq, const bf16* __restrict__ pk, void* __restrict__ idx_out, int idx64, int64_t M, int64_t n,
-                       int topk) {
-  __shared__ __align__(16) bf16 sk[2][kCmKeys * kSmemPitch];
-  __shared__ float cand_v[4][16][32];
-  __shared__ int cand_i[4][16][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int64_t bh = blockIdx.y, row0 = (int64_t) blockIdx.x * kCmRows + warp * 16;
-  const bf16* k0 = pk + bh * n * 64;
-  auto stage = [&](int64_t kt, int buf) {               // 64 keys x 128 bytes: 4 chunks of 16 bytes per thread
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int ch = c * 128 + threadIdx.x, r = ch >> 3, col = (ch & 7) * 8;
-      cp_async16(&sk[buf][r * kSmemPitch + col], k0 + (kt * kCmKeys + r) * 64 + col);
-    }
-    cp_async_commit();
-  };
-  stage(0, 0);
-  RowFrag qlo, qhi;
+template <typename T>
+__device__ __forceinline__ float4 load4(const T* p) {
+  if constexpr (sizeof(T) == 2) {
+    const uint2 x = __ldg(reinterpret_cast<const uint2*>(p));
+    return make_float4(bf16_lo(x.x), bf16_hi(x.x), bf16_lo(x.y), bf16_hi(x.y));
+  } else {
+    return __ldg(reinterpret_cast<const float4*>(p));
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+coarse_topk_tile_kernel(const T* __restrict__ pq, const T* __restrict__ pk, void* __restrict__ idx_out, int idx64, int64_t M, int64_t n, int topk) {
+  extern __shared__ __align__(16) float sm[];
+  float* qs = sm;                                   // [16][kCtPitch]
+  float* ks = qs + kCtRows * kCtPitch;              // [256][kCtPitch]
+  uint32_t* sc = reinterpret_cast<uint32_t*>(ks + kCtKeys * kCtPitch);      // [16][kCtScPitch] score images
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t bh = blockIdx.y, row0 = (int64_t) blockIdx.x * kCtRows;
+  const T* k0 = pk + bh * n * 64;
   {
-    const int64_t ra = min(row0 + g, M - 1), rb = min(row0 + g + 8, M - 1);     // rows past M are computed and dropped
-    load_rowfrag(qlo, pq + (bh * M + ra) * 64, t);
-    load_rowfrag(qhi, pq + (bh * M + rb) * 64, t);
+    const int r = tid >> 4, d = (tid & 15) * 4;
+    *reinterpret_cast<float4*>(qs + r * kCtPitch + d) = load4<T>(pq + (bh * M + min(row0 + r, M - 1)) * 64 + d);
   }
-  float v0[kCmTop], v1[kCmTop];
-  int i0[kCmTop], i1[kCmTop];
-#pragma unroll
-  for (int u = 0; u < kCmTop; ++u) { v0[u] = v1[u] = -CUDART_INF_F; i0[u] = i1[u] = 0x7FFFFFFF; }
-  const int64_t n_tiles = n / kCmKeys;
-  for (int64_t kt = 0; kt < n_tiles; ++kt) {
-    if (kt + 1 < n_tiles) stage(kt + 1, (int) ((kt + 1) & 1));
-    else cp_async_commit();
-    cp_async_wait_group<1>();
-    __syncthreads();
-    const bf16* tile = sk[kt & 1];
-#pragma unroll
-    for (int blk = 0; blk < 4; ++blk) {
-      RowFrag ka, kb;
-      load_rowfrag_smem(ka, tile + (blk * 16 + g) * kSmemPitch, t);
-      load_rowfrag_smem(kb, tile + (blk * 16 + 8 + g) * kSmemPitch, t);
-      float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
-      mma_rows_x_keys(s0, s1, qlo, qhi, ka, kb);
-      const int c = (int) (kt * kCmKeys) + blk * 16 + 2 * t;
-      top8_insert(v0, i0, round_to<bf16>(s0[0]), c);     top8_insert(v0, i0, round_to<bf16>(s0[1]), c + 1);
-      top8_insert(v0, i0, round_to<bf16>(s1[0]), c + 8); top8_insert(v0, i0, round_to<bf16>(s1[1]), c + 9);
-      top8_insert(v1, i1, round_to<bf16>(s0[2]), c);     top8_insert(v1, i1, round_to<bf16>(s0[3]), c + 1);
-      top8_insert(v1, i1, round_to<bf16>(s1[2]), c + 8); top8_insert(v1, i1, round_to<bf16>(s1[3]), c + 9);
+  const int rw = (warp >> 2) * 8, kw = (warp & 3) * 64 + lane;      // this thread's rows and its first key
+  uint64_t list[2] = {0, 0}, thr[2] = {0, 0};
+  for (int64_t base = 0; base < n; base += kCtKeys) {
+    const int cn = (int) min((int64_t) kCtKeys, n - base);
+    for (int i = tid; i < cn * 16; i += 256) {
+      const int r = i >> 4, d = (i & 15) * 4;
+      *reinterpret_cast<float4*>(ks + r * kCtPitch + d) = load4<T>(k0 + (base + r) * 64 + d);
     }
-    __syncthreads();          // the buffer read here is refilled by the next iteration's stage()
-  }
+    __syncthreads();
+    if ((warp & 3) * 64 < cn) {                     // keys past the chunk's end read stale rows and are dropped by the selection
+      float acc[8][2];
 #pragma unroll
-  for (int u = 0; u < kCmTop; ++u) {
-    cand_v[warp][g][t * kCmTop + u] = v0[u];      cand_i[warp][g][t * kCmTop + u] = i0[u];
-    cand_v[warp][g + 8][t * kCmTop + u] = v1[u];  cand_i[warp][g + 8][t * kCmTop + u] = i1[u];
-  }
-  __syncwarp();
-  for (int r = 0; r < 16; ++r) {
-    if (row0 + r >= M) break;
-    uint32_t key = orderable(cand_v[warp][r][lane]);
-    uint32_t blk = (uint32_t) cand_i[warp][r][lane];
-    if (blk == 0x7FFFFFFFu) key = 0u;                    // unused slot
-    for (int tt = 0; tt < topk; ++tt) {
-      const uint32_t mk = __reduce_max_sync(0xffffffffu, key);
-      const uint32_t mb = __reduce_min_sync(0xffffffffu, key == mk ? blk : 0xFFFFFFFFu);
-      if (key == mk && blk == mb) { key = 0u; blk = 0xFFFFFFFFu; }
-      if (lane == 0) {
-        const int64_t o = (bh * M + row0 + r) * topk + tt;
-        if (idx64) reinterpret_cast<int64_t*>(idx_out)[o] = (int64_t) mb;
-        else reinterpret_cast<int32_t*>(idx_out)[o] = (int32_t) mb;
+      for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = 0.f;
+#pragma unroll 4
+      for (int d = 0; d < 64; d += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(ks + kw * kCtPitch + d), y = *reinterpret_cast<const float4*>(ks + (kw + 32) * kCtPitch + d);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const float4 q = *reinterpret_cast<const float4*>(qs + (rw + r) * kCtPitch + d);
+          acc[r][0] = fmaf(q.x, x.x, acc[r][0]); acc[r][0] = fmaf(q.y, x.y, acc[r][0]);
+          acc[r][0] = fmaf(q.z, x.z, acc[r][0]); acc[r][0] = fmaf(q.w, x.w, acc[r][0]);
+          acc[r][1] = fmaf(q.x, y.x, acc[r][1]); acc[r][1] = fmaf(q.y, y.y, acc[r][1]);
+          acc[r][1] = fmaf(q.z, y.z, acc[r][1]); acc[r][1] = fmaf(q.w, y.w, acc[r][1]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        sc[(rw + r) * kCtScPitch + kw] = orderable(nan_first(round_to<T>(acc[r][0])));
+        sc[(rw + r) * kCtScPitch + kw + 32] = orderable(nan_first(round_to<T>(acc[r][1])));
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const uint32_t* s = sc + (warp + 8 * e) * kCtScPitch;
+      for (int j = lane; j - lane < cn; j += 32) {
+        const uint64_t cand = j < cn ? ((uint64_t) s[j] << 32) | (0xFFFFFFFFu - (uint32_t) (base + j)) : 0;
+        warp_list_insert(list[e], thr[e], cand, topk, lane);
       }
     }
   }
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int64_t row = row0 + warp + 8 * e;
+    if (row < M && lane < topk) {
+      const int64_t o = (bh * M + row) * topk + lane;
+      const uint32_t col = 0xFFFFFFFFu - (uint32_t) list[e];
+      if (idx64) reinterpret_cast<int64_t*>(idx_out)[o] = (int64_t) col;
+      else reinterpret_cast<int32_t*>(idx_out)[o] = (int32_t) col;
+    }
+  }
 }
 
-constexpr int kRefineSlots = 8;        // register path of the refine selection: up to 256 candidates per row
-
+// Refine step.  pq1: contiguous [B*H, M, D] (M query blocks); pk1: contiguous [B*H, Mk, D] (Mk key blocks, Mk != M when the
+// queries are a shard of the sequence); p_idx [B*H, M/bs, p_topk] with values in [0, Mk/bs); out [B*H, M, topk].
+// MMA = true (bf16, D = 64, bs = 16): the 16 x C score tile comes from mma.sync with fp32
+// accumulation of the exact bf16 products, as the reference's tl.dot does.
 // Order-preserving map of a float onto uint32 (larger float <=> larger integer, -0 and +0 share one image so
 // that they tie like the float comparison does).
 __device__ __forceinline__ uint32_t orderable(float v) {
@@ -259,41 +442,75 @@ __device__ __forceinline__ uint32_t orderable(float v) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// Refine selection with the candidates of a row in registers: lane l keeps candidates l, l + 32, ... (SLOTS of them) as
-// order-preserving 32-bit images of the scores; a round is two warp reductions: the largest score, then the smallest
-// block index among its holders.
-template <int SLOTS>
-__device__ __forceinline__ void refine_select_regs(const float* sc, const int* cand, int C, int bs, int topk, void* idx_out, int idx64,
-                                                   int64_t out_row0, int warp, int lane, int nwarps) {
-  for (int r = warp; r < bs; r += nwarps) {
-    const float* s = sc + r * C;
-    uint32_t key[SLOTS], blk[SLOTS];
+// Refine selection with the candidates of a row in registers: lane l keeps candidates l, l + 32, ... (eight of them) as 64-bit words,
+// the order-preserving image of the score above the complemented block index, sorted once, so that its best is always slot 0.  A round is
+// one warp maximum over the score images and a ballot (a second maximum, over the complemented blocks, only where scores tie); the winner's
+// lane shifts its list up by one, and winner t stays in lane t until one store writes the row's list (top-k <= 32; a store by each winner
+// is 20 % slower).  A warp takes
+// two rows at a time: the rounds are chains of warp-wide instructions, and two chains hide each other's latency.
+__device__ __forceinline__ void refine_select_sorted8(const float* sc, const int* cand, int C, int bs, int topk, void* idx_out, int idx64,
+                                                      int64_t out_row0, int warp, int lane, int nwarps) {
+  constexpr int SLOTS = 8;
+  for (int r0 = warp; r0 < bs; r0 += 2 * nwarps) {
+    uint64_t w[2][SLOTS];
+    uint32_t mine[2] = {0u, 0u};
 #pragma unroll
-    for (int u = 0; u < SLOTS; ++u) {
-      const int j = lane + 32 * u;
-      key[u] = (j < C && cand[j] >= 0) ? orderable(s[j]) : 0u;            // 0 is below every real score's image
-      blk[u] = j < C ? (uint32_t) cand[j] : 0xFFFFFFFFu;
+    for (int e = 0; e < 2; ++e) {
+      const float* s = sc + min(r0 + e * nwarps, bs - 1) * C;      // past the last row: computed on it and dropped
+#pragma unroll
+      for (int u = 0; u < SLOTS; ++u) {
+        const int j = lane + 32 * u;
+        w[e][u] = (j < C && cand[j] >= 0) ? ((uint64_t) orderable(s[j]) << 32) | (0xFFFFFFFFu - (uint32_t) cand[j]) : 0;      // 0 is below every real candidate
+      }
+#pragma unroll
+      for (int k = 2; k <= SLOTS; k <<= 1)                          // bitonic, descending
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+          for (int i = 0; i < SLOTS; ++i)
+            if ((i ^ j) > i) {
+              const bool desc = (i & k) == 0;
+              const uint64_t x = w[e][i], y = w[e][i ^ j];
+              const bool sw = desc ? y > x : x > y;
+              w[e][i] = sw ? y : x;
+              w[e][i ^ j] = sw ? x : y;
+            }
     }
     for (int t = 0; t < topk; ++t) {
-      uint32_t bk = key[0], bb = blk[0];
 #pragma unroll
-      for (int u = 1; u < SLOTS; ++u)
-        if (key[u] > bk || (key[u] == bk && blk[u] < bb)) { bk = key[u]; bb = blk[u]; }
-      const uint32_t mk = __reduce_max_sync(0xffffffffu, bk);
-      const uint32_t mb = __reduce_min_sync(0xffffffffu, bk == mk ? bb : 0xFFFFFFFFu);
+      for (int e = 0; e < 2; ++e) {
+        const uint32_t hi = (uint32_t) (w[e][0] >> 32), lo = (uint32_t) w[e][0];
+        const uint32_t m = __reduce_max_sync(0xffffffffu, hi);
+        unsigned who = __ballot_sync(0xffffffffu, hi == m);
+        if (who & (who - 1)) {                                      // equal scores: the smallest block
+          const uint32_t ml = __reduce_max_sync(0xffffffffu, hi == m ? lo : 0u);
+          who = __ballot_sync(0xffffffffu, hi == m && lo == ml);
+        }
+        const int src = __ffs((int) who) - 1;
+        const uint32_t win = __shfl_sync(0xffffffffu, lo, src);
+        if (lane == t) mine[e] = win;
+        if (lane == src) {                                          // candidates are distinct blocks: one owner
 #pragma unroll
-      for (int u = 0; u < SLOTS; ++u)
-        if (key[u] == mk && blk[u] == mb) { key[u] = 0u; blk[u] = 0xFFFFFFFFu; }      // candidates are distinct blocks: one owner
-      if (lane == 0) {
-        const int64_t o = (out_row0 + r) * topk + t;
-        if (idx64) reinterpret_cast<int64_t*>(idx_out)[o] = (int64_t) mb;
-        else reinterpret_cast<int32_t*>(idx_out)[o] = (int32_t) mb;
+          for (int u = 0; u + 1 < SLOTS; ++u) w[e][u] = w[e][u + 1];
+          w[e][SLOTS - 1] = 0;
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int r = r0 + e * nwarps;
+      if (r < bs && lane < topk) {
+        const int64_t o = (out_row0 + r) * topk + lane;
+        const uint32_t blk = 0xFFFFFFFFu - mine[e];
+        if (idx64) reinterpret_cast<int64_t*>(idx_out)[o] = (int64_t) blk;
+        else reinterpret_cast<int32_t*>(idx_out)[o] = (int32_t) blk;
       }
     }
   }
 }
 
-// The same selection for at most 128 candidates and top-k <= 32 with fewer instructions per round: a lane sorts its four
+// The same for at most 128 candidates (four per lane) with 32-bit words, which is faster there (33.0 against 34.3 us at 48 slices of 64
+// parents): a lane sorts its four
 // candidates once (descending score image, ascending block index among equals), so its best is always slot 0; a round is two warp
 // reductions, the winner's lane shifts its list up by one, and winner t stays in lane t until one store writes the row's list.
 __device__ __forceinline__ void refine_select_sorted4(const float* sc, const int* cand, int C, int bs, int topk, void* idx_out, int idx64,
@@ -331,14 +548,14 @@ __device__ __forceinline__ void refine_select_sorted4(const float* sc, const int
   }
 }
 
-// Coarse selection of ONE level-2 query block against 64 level-2 keys, inside the refine kernel's CTA (four warps: 16 keys
+// Coarse selection of ONE level-2 query block inside the refine kernel's CTA: against 64 level-2 keys on the tensor cores (four warps: 16 keys
 // each).  The scores are the ones coarse_topk_mma_kernel computes -- the same mma.sync k-steps in the same order on the same
 // operands (all 16 A rows hold the query block's row, so every row of the result is that row's), rounded to bf16, NaN first --
 // and the winners come out in the same order (descending score, ties to the smaller key), so the fused form returns the
 // bits of the two-kernel form while saving its launch and its 64 x 64-score CTAs.
 struct FusedCoarse {
-  const bf16* pq2;     // [BH, M / bs, 64]
-  const bf16* pk2;     // [BH, 64, 64]
+  const void* pq2;     // [BH, M / bs, 64], the data's type
+  const void* pk2;     // [BH, n2, 64]
   void* pidx_out;      // [BH, M / bs, p_topk]
   int pidx64;
 };
@@ -346,8 +563,8 @@ struct FusedCoarse {
 __device__ __forceinline__ void coarse_row_64(const FusedCoarse& f, int64_t bh, int64_t P, int64_t n2q, int p_topk, float* sc2, int* s_pidx) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   RowFrag q2, ka, kb;
-  load_rowfrag(q2, f.pq2 + (bh * n2q + P) * 64, t);
-  const bf16* k0 = f.pk2 + bh * 64 * 64;
+  load_rowfrag(q2, reinterpret_cast<const bf16*>(f.pq2) + (bh * n2q + P) * 64, t);
+  const bf16* k0 = reinterpret_cast<const bf16*>(f.pk2) + bh * 64 * 64;
   load_rowfrag(ka, k0 + (warp * 16 + g) * 64, t);
   load_rowfrag(kb, k0 + (warp * 16 + 8 + g) * 64, t);
   float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
@@ -362,9 +579,7 @@ __device__ __forceinline__ void coarse_row_64(const FusedCoarse& f, int64_t bh, 
     uint32_t key[2], blk[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      float v = sc2[lane + 32 * u];
-      v = v != v ? CUDART_INF_F : fmaxf(v, -3.0e38f);       // as top8_insert orders them
-      key[u] = orderable(v);
+      key[u] = orderable(sc2[lane + 32 * u]);
       blk[u] = (uint32_t) (lane + 32 * u);
     }
     uint32_t mine = 0;
@@ -388,12 +603,49 @@ __device__ __forceinline__ void coarse_row_64(const FusedCoarse& f, int64_t bh, 
   __syncthreads();
 }
 
-template <typename T, bool MMA, bool FUSED = false>
+// The same with scalar arithmetic for the level-2 lists coarse_topk_tile_kernel would take (same channel order, same bits), up to
+// kFusedKeys keys, one thread per key.
+constexpr int kFusedKeys = 256;
+template <typename T>
+__device__ __forceinline__ void coarse_row_scalar(const FusedCoarse& f, int64_t bh, int64_t P, int64_t n2q, int n2, int p_topk, uint32_t* sc2,
+                                                  int* s_pidx) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const T* q = reinterpret_cast<const T*>(f.pq2) + (bh * n2q + P) * 64;
+  for (int j = threadIdx.x; j < n2; j += blockDim.x) {
+    const T* k = reinterpret_cast<const T*>(f.pk2) + (bh * n2 + j) * 64;
+    float acc = 0.f;
+#pragma unroll
+    for (int d = 0; d < 64; d += 4) {
+      const float4 a = load4<T>(q + d), x = load4<T>(k + d);
+      acc = fmaf(a.x, x.x, acc); acc = fmaf(a.y, x.y, acc); acc = fmaf(a.z, x.z, acc); acc = fmaf(a.w, x.w, acc);
+    }
+    sc2[j] = orderable(nan_first(round_to<T>(acc)));
+  }
+  __syncthreads();
+  if (warp == 0) {
+    uint64_t list = 0, thr = 0;
+    for (int j = lane; j - lane < n2; j += 32)
+      warp_list_insert(list, thr, j < n2 ? ((uint64_t) sc2[j] << 32) | (0xFFFFFFFFu - (uint32_t) j) : 0, p_topk, lane);
+    if (lane < p_topk) {
+      const uint32_t col = 0xFFFFFFFFu - (uint32_t) list;
+      s_pidx[lane] = (int) col;
+      const int64_t o = (bh * n2q + P) * p_topk + lane;
+      if (f.pidx64) reinterpret_cast<int64_t*>(f.pidx_out)[o] = (int64_t) col;
+      else reinterpret_cast<int32_t*>(f.pidx_out)[o] = (int32_t) col;
+    }
+  }
+  __syncthreads();
+}
+
+// FUSED: 0 parents given, 1 selected here by coarse_row_64, 2 by coarse_row_scalar
+template <typename T, bool MMA, int FUSED = 0>
 __global__ void __launch_bounds__(128)
 refine_topk_kernel(const T* __restrict__ pq1, const T* __restrict__ pk1, IdxView p_idx, void* __restrict__ idx_out, int idx64, int64_t M,
-                   int64_t Mk, int D, int topk, int p_topk, int bs, FusedCoarse fused) {
+                   int64_t Mk, int D_, int topk, int p_topk, int bs_, FusedCoarse fused) {
+  // constants where the dispatch fixes them: no division by a run-time block size per candidate
+  const int D = MMA || FUSED ? 64 : D_, bs = MMA || FUSED ? 16 : bs_;
   extern __shared__ float sm[];
-  __shared__ float s_sc2[64];
+  __shared__ float s_sc2[FUSED == 2 ? kFusedKeys : 64];
   __shared__ int s_pidx[kMaxTopk];
   const int C = p_topk * bs;
   float* qs = sm;                 // [bs][D]
@@ -404,7 +656,8 @@ refine_topk_kernel(const T* __restrict__ pq1, const T* __restrict__ pk1, IdxView
   const T* k0 = pk1 + bh * Mk * D;
   if constexpr (!MMA)                                    // the tensor-core path takes its query fragments straight from global memory
     for (int i = threadIdx.x; i < bs * D; i += blockDim.x) qs[i] = to_f32<T>(q0[i]);
-  if constexpr (FUSED) coarse_row_64(fused, bh, P, n2q, p_topk, s_sc2, s_pidx);
+  if constexpr (FUSED == 1) coarse_row_64(fused, bh, P, n2q, p_topk, s_sc2, s_pidx);
+  if constexpr (FUSED == 2) coarse_row_scalar<T>(fused, bh, P, n2q, (int) n2, p_topk, reinterpret_cast<uint32_t*>(s_sc2), s_pidx);
   for (int j = threadIdx.x; j < C; j += blockDim.x) {
     int64_t p = FUSED ? (int64_t) s_pidx[j / bs] : p_idx.at((bh * n2q + P) * p_topk + j / bs);
     p = p < 0 ? 0 : (p >= n2 ? n2 - 1 : p);      // never read outside the tensor
@@ -473,10 +726,9 @@ refine_topk_kernel(const T* __restrict__ pq1, const T* __restrict__ pk1, IdxView
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  if (C <= 32 * kRefineSlots) {
-    if (C <= 128 && topk <= 32) refine_select_sorted4(sc, cand, C, bs, topk, idx_out, idx64, bh * M + P * bs, warp, lane, nwarps);
-    else if (C <= 128) refine_select_regs<4>(sc, cand, C, bs, topk, idx_out, idx64, bh * M + P * bs, warp, lane, nwarps);
-    else refine_select_regs<kRefineSlots>(sc, cand, C, bs, topk, idx_out, idx64, bh * M + P * bs, warp, lane, nwarps);
+  if (C <= 256 && topk <= 32) {
+    if (C <= 128) refine_select_sorted4(sc, cand, C, bs, topk, idx_out, idx64, bh * M + P * bs, warp, lane, nwarps);
+    else refine_select_sorted8(sc, cand, C, bs, topk, idx_out, idx64, bh * M + P * bs, warp, lane, nwarps);
     return;
   }
   for (int r = warp; r < bs; r += nwarps) {
@@ -506,6 +758,14 @@ refine_topk_kernel(const T* __restrict__ pq1, const T* __restrict__ pk1, IdxView
 
 using namespace llsa;
 
+// The tensor-core kernel's range: its accumulation order differs from the scalar kernels' in the last bit of a score, so the line
+// between the two decides which bits a caller gets and stays where it was (whole 64-key tiles, top-k <= 8).
+static bool coarse_on_mma(const LlsaTensor* pq, const LlsaTensor* pk, int topk) {
+  const int64_t n = pk->shape[2];
+  return pq->dtype == LLSA_BF16 && pq->shape[3] == 64 && topk <= kCmTop && n % 64 == 0 && n <= 65536 && ((uintptr_t) pq->ptr % 32) == 0 &&
+         ((uintptr_t) pk->ptr % 32) == 0;
+}
+
 extern "C" int llsa_coarse_topk(const LlsaTensor* pq, const LlsaTensor* pk, const LlsaTensor* idx, int topk, void* stream) {
   LLSA_REQUIRE(pq && pk && idx && pq->ptr && pk->ptr && idx->ptr, LLSA_ERR_NULL, "coarse_topk: null tensor");
   LLSA_REQUIRE(pq->ndim == 4 && pk->ndim == 4, LLSA_ERR_SHAPE, "coarse_topk: pq, pk must be [B,H,M,D]");
@@ -520,21 +780,36 @@ extern "C" int llsa_coarse_topk(const LlsaTensor* pq, const LlsaTensor* pk, cons
   if ((rc = check_contig(pk, "pk", pq->dtype, 4, sk))) return rc;
   if ((rc = check_contig(idx, "idx", idx->dtype, 4, si))) return rc;
   if (B * H * M == 0) return LLSA_OK;
-  const size_t smem = (size_t) kCoarseRows * (D + kCoarseChunk) * 4 + (size_t) kCoarseRows * kMaxTopk * (4 + 8) * 2;
-  dim3 grid((unsigned) ((M + kCoarseRows - 1) / kCoarseRows), (unsigned) (B * H));
   cudaStream_t st = (cudaStream_t) stream;
-  if (pq->dtype == LLSA_F32) {
-    LLSA_SMEM_LIMIT((coarse_topk_kernel<float>), smem);
-    coarse_topk_kernel<float><<<grid, kCoarseThreads, smem, st>>>((const float*) pq->ptr, (const float*) pk->ptr, idx->ptr,
-                                                                   idx->dtype == LLSA_I64, M, n, (int) D, topk);
-  } else if (D == 64 && topk <= kCmTop && n % kCmKeys == 0 && n >= topk && ((uintptr_t) pq->ptr % 32) == 0 && ((uintptr_t) pk->ptr % 16) == 0 &&
-             n * 64 < (int64_t) 1 << 31) {
-    coarse_topk_mma_kernel<<<dim3((unsigned) ((M + kCmRows - 1) / kCmRows), (unsigned) (B * H)), 128, 0, st>>>(
-        (const __nv_bfloat16*) pq->ptr, (const __nv_bfloat16*) pk->ptr, idx->ptr, idx->dtype == LLSA_I64, M, n, topk);
+  const unsigned BH = (unsigned) (B * H);
+  const int idx64 = idx->dtype == LLSA_I64;
+  const bool bf = pq->dtype == LLSA_BF16;
+  auto blocks = [&](int rows) { return dim3((unsigned) ((M + rows - 1) / rows), BH); };
+  if (coarse_on_mma(pq, pk, topk)) {
+    const bf16 *q = (const bf16*) pq->ptr, *k = (const bf16*) pk->ptr;
+    // 64 rows per CTA (each key read from L2 once per 64 rows) where that still gives every SM two CTAs, else 16 rows, the keys
+    // split over all eight warps
+    if (B * H * ((M + 63) / 64) >= 2 * 148) coarse_topk_mma_kernel<2, 4><<<blocks(64), kCmWarps * 32, 0, st>>>(q, k, idx->ptr, idx64, M, n, topk);
+    else coarse_topk_mma_kernel<1, 8><<<blocks(16), kCmWarps * 32, 0, st>>>(q, k, idx->ptr, idx64, M, n, topk);
+  } else if (D == 64 && topk <= 32 && n < (1ll << 31)) {
+    if (bf) {
+      LLSA_SMEM_LIMIT((coarse_topk_tile_kernel<bf16>), kCtSmem);
+      coarse_topk_tile_kernel<bf16><<<blocks(kCtRows), 256, kCtSmem, st>>>((const bf16*) pq->ptr, (const bf16*) pk->ptr, idx->ptr, idx64, M, n, topk);
+    } else {
+      LLSA_SMEM_LIMIT((coarse_topk_tile_kernel<float>), kCtSmem);
+      coarse_topk_tile_kernel<float><<<blocks(kCtRows), 256, kCtSmem, st>>>((const float*) pq->ptr, (const float*) pk->ptr, idx->ptr, idx64, M, n, topk);
+    }
   } else {
-    LLSA_SMEM_LIMIT((coarse_topk_kernel<__nv_bfloat16>), smem);
-    coarse_topk_kernel<__nv_bfloat16><<<grid, kCoarseThreads, smem, st>>>((const __nv_bfloat16*) pq->ptr, (const __nv_bfloat16*) pk->ptr,
-                                                                           idx->ptr, idx->dtype == LLSA_I64, M, n, (int) D, topk);
+    const size_t smem = (size_t) kCoarseRows * (D + kCoarseChunk) * 4 + (size_t) kCoarseRows * kMaxTopk * (4 + 8) * 2;
+    if (!bf) {
+      LLSA_SMEM_LIMIT((coarse_topk_kernel<float>), smem);
+      coarse_topk_kernel<float><<<blocks(kCoarseRows), kCoarseThreads, smem, st>>>((const float*) pq->ptr, (const float*) pk->ptr, idx->ptr, idx64, M, n,
+                                                                                   (int) D, topk);
+    } else {
+      LLSA_SMEM_LIMIT((coarse_topk_kernel<bf16>), smem);
+      coarse_topk_kernel<bf16><<<blocks(kCoarseRows), kCoarseThreads, smem, st>>>((const bf16*) pq->ptr, (const bf16*) pk->ptr, idx->ptr, idx64, M, n,
+                                                                                  (int) D, topk);
+    }
   }
   LLSA_LAUNCH_OK("coarse_topk_kernel");
   return LLSA_OK;
@@ -583,42 +858,60 @@ extern "C" int llsa_refine_topk(const LlsaTensor* pq1, const LlsaTensor* pk1, co
 extern "C" int llsa_select_two_level(const LlsaTensor* pq1, const LlsaTensor* pk1, const LlsaTensor* pq2, const LlsaTensor* pk2,
                                      const LlsaTensor* p_idx, const LlsaTensor* idx, int topk, int p_topk, int block_size, void* stream) {
   LLSA_REQUIRE(pq1 && pk1 && pq2 && pk2 && p_idx && idx, LLSA_ERR_NULL, "select_two_level: null tensor");
-  // the fused form covers the benchmark class: bf16, D = 64, block 16, exactly 64 level-2 keys, at most 8 parents per row
-  const bool fusable = pq1->ptr && pk1->ptr && pq2->ptr && pk2->ptr && p_idx->ptr && idx->ptr && pq1->dtype == LLSA_BF16 && pq1->ndim == 4 &&
-                       pk2->ndim == 4 && pq1->shape[3] == 64 && block_size == 16 && pk2->shape[2] == 64 && p_topk >= 2 && p_topk <= kCmTop &&
-                       p_topk % 2 == 0 && ((uintptr_t) pq1->ptr % 32) == 0 && ((uintptr_t) pk1->ptr % 32) == 0 &&
-                       ((uintptr_t) pq2->ptr % 32) == 0 && ((uintptr_t) pk2->ptr % 32) == 0;
+  const int bs = block_size;
+  // One launch where the level-2 list is short: exactly 64 keys where the tensor-core coarse kernel would score them, or up to
+  // kFusedKeys keys where the scalar one would (a CTA then reads the whole level-2 list of its head: 32 KB at most, from L2).
+  bool fusable = pq1->ptr && pk1->ptr && pq2->ptr && pk2->ptr && p_idx->ptr && idx->ptr && is_float_dtype(pq1->dtype) && pk1->dtype == pq1->dtype &&
+                 pq2->dtype == pq1->dtype && pk2->dtype == pq1->dtype && pq1->ndim == 4 && pk1->ndim == 4 && pq2->ndim == 4 && pk2->ndim == 4 &&
+                 pq1->shape[3] == 64 && bs == 16 && p_topk >= 2 && p_topk % 2 == 0 && p_topk <= 16 && p_topk <= pk2->shape[2] &&
+                 ((uintptr_t) pq1->ptr % 32) == 0 && ((uintptr_t) pk1->ptr % 32) == 0 && ((uintptr_t) pq2->ptr % 32) == 0 &&
+                 ((uintptr_t) pk2->ptr % 32) == 0;
+  const bool on_mma = fusable && coarse_on_mma(pq2, pk2, p_topk);
+  if (fusable) fusable = on_mma ? pk2->shape[2] == 64 : pk2->shape[2] <= kFusedKeys;
   if (!fusable) {
     int rc = llsa_coarse_topk(pq2, pk2, p_idx, p_topk, stream);
     if (rc) return rc;
     return llsa_refine_topk(pq1, pk1, p_idx, idx, topk, p_topk, block_size, stream);
   }
-  const int64_t B = pq1->shape[0], H = pq1->shape[1], M = pq1->shape[2], D = 64, Mk = pk1->shape[2];
-  const int bs = block_size;
-  LLSA_REQUIRE(pk1->dtype == LLSA_BF16 && pq2->dtype == LLSA_BF16 && pk2->dtype == LLSA_BF16, LLSA_ERR_DTYPE, "select_two_level: all pooled tensors must be bf16");
+  const int64_t B = pq1->shape[0], H = pq1->shape[1], M = pq1->shape[2], D = 64, Mk = pk1->shape[2], n2 = pk2->shape[2];
+  const int dt = pq1->dtype;
   LLSA_REQUIRE(is_index_dtype(idx->dtype) && is_index_dtype(p_idx->dtype), LLSA_ERR_DTYPE, "select_two_level: index tensors must be i32 or i64");
-  LLSA_REQUIRE(M % bs == 0 && Mk == 64 * bs, LLSA_ERR_SHAPE, "select_two_level: M=%lld / Mk=%lld do not fit 64 level-2 keys", (long long) M, (long long) Mk);
-  LLSA_REQUIRE(topk >= 1 && topk <= p_topk * bs, LLSA_ERR_ARG, "select_two_level: bad topk=%d / p_topk=%d", topk, p_topk);
-  const int64_t sq[4] = {B, H, M, D}, sk[4] = {B, H, Mk, D}, sq2[4] = {B, H, M / bs, D}, sk2[4] = {B, H, 64, D}, sp[4] = {B, H, M / bs, p_topk},
+  LLSA_REQUIRE(M % bs == 0 && Mk == n2 * bs, LLSA_ERR_SHAPE, "select_two_level: M=%lld / Mk=%lld do not fit %lld level-2 keys", (long long) M, (long long) Mk,
+               (long long) n2);
+  LLSA_REQUIRE(topk >= 1 && topk <= kMaxTopk && topk <= p_topk * bs, LLSA_ERR_ARG, "select_two_level: bad topk=%d / p_topk=%d", topk, p_topk);
+  const int64_t sq[4] = {B, H, M, D}, sk[4] = {B, H, Mk, D}, sq2[4] = {B, H, M / bs, D}, sk2[4] = {B, H, n2, D}, sp[4] = {B, H, M / bs, p_topk},
                 si[4] = {B, H, M, topk};
   int rc;
-  if ((rc = check_contig(pq1, "pq1", LLSA_BF16, 4, sq))) return rc;
-  if ((rc = check_contig(pk1, "pk1", LLSA_BF16, 4, sk))) return rc;
-  if ((rc = check_contig(pq2, "pq2", LLSA_BF16, 4, sq2))) return rc;
-  if ((rc = check_contig(pk2, "pk2", LLSA_BF16, 4, sk2))) return rc;
+  if ((rc = check_contig(pq1, "pq1", dt, 4, sq))) return rc;
+  if ((rc = check_contig(pk1, "pk1", dt, 4, sk))) return rc;
+  if ((rc = check_contig(pq2, "pq2", dt, 4, sq2))) return rc;
+  if ((rc = check_contig(pk2, "pk2", dt, 4, sk2))) return rc;
   if ((rc = check_contig(p_idx, "p_idx", p_idx->dtype, 4, sp))) return rc;
   if ((rc = check_contig(idx, "idx", idx->dtype, 4, si))) return rc;
   if (B * H * M == 0) return LLSA_OK;
   const size_t smem = ((size_t) bs * D + (size_t) bs * p_topk * bs + (size_t) p_topk * bs) * 4;
   FusedCoarse f;
-  f.pq2 = (const __nv_bfloat16*) pq2->ptr;
-  f.pk2 = (const __nv_bfloat16*) pk2->ptr;
+  f.pq2 = pq2->ptr;
+  f.pk2 = pk2->ptr;
   f.pidx_out = p_idx->ptr;
   f.pidx64 = p_idx->dtype == LLSA_I64;
-  LLSA_SMEM_LIMIT((refine_topk_kernel<__nv_bfloat16, true, true>), smem);
-  refine_topk_kernel<__nv_bfloat16, true, true><<<dim3((unsigned) (M / bs), (unsigned) (B * H)), 128, smem, (cudaStream_t) stream>>>(
-      (const __nv_bfloat16*) pq1->ptr, (const __nv_bfloat16*) pk1->ptr, IdxView{nullptr, 0}, idx->ptr, idx->dtype == LLSA_I64, M, Mk, (int) D, topk,
-      p_topk, bs, f);
+  const dim3 grid((unsigned) (M / bs), (unsigned) (B * H));
+  cudaStream_t st = (cudaStream_t) stream;
+  const int idx64 = idx->dtype == LLSA_I64;
+  const IdxView none{nullptr, 0};
+  if (dt == LLSA_F32) {
+    LLSA_SMEM_LIMIT((refine_topk_kernel<float, false, 2>), smem);
+    refine_topk_kernel<float, false, 2><<<grid, 128, smem, st>>>((const float*) pq1->ptr, (const float*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D,
+                                                                 topk, p_topk, bs, f);
+  } else if (on_mma) {
+    LLSA_SMEM_LIMIT((refine_topk_kernel<bf16, true, 1>), smem);
+    refine_topk_kernel<bf16, true, 1><<<grid, 128, smem, st>>>((const bf16*) pq1->ptr, (const bf16*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D, topk,
+                                                               p_topk, bs, f);
+  } else {
+    LLSA_SMEM_LIMIT((refine_topk_kernel<bf16, true, 2>), smem);
+    refine_topk_kernel<bf16, true, 2><<<grid, 128, smem, st>>>((const bf16*) pq1->ptr, (const bf16*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D, topk,
+                                                               p_topk, bs, f);
+  }
   LLSA_LAUNCH_OK("refine_topk_kernel<fused>");
   return LLSA_OK;
 }

@@ -1,0 +1,58 @@
+"""Coarse selection over the list lengths where its kernels change, and the fused two-level selection against its two steps."""
+import pytest
+import torch
+
+from helpers import topk_mismatch_rows
+from llsa_b200 import ops, synth
+from oracle import llsa_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+# (BH, M, n): fewer keys than a 16-key block holds rows for, whole 64-key tiles (tensor cores: 16-row and, from 296 CTAs of 64 rows on,
+# 64-row CTAs), ragged lists (scalar: below, at and past a 256-key chunk), rows that do not fill a tile
+@pytest.mark.parametrize("BH,M,n", [(2, 64, 64), (3, 72, 128), (5, 4096, 320), (2, 40, 21), (3, 160, 160), (1, 300, 256 + 33), (2, 17, 1000)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("topk", [1, 8, 16])
+def test_coarse_topk_shapes(BH, M, n, dtype, topk):
+    gen = torch.Generator().manual_seed(1000 * n + M + topk)
+    pq, pk = (torch.randn(1, BH, M, 64, generator=gen) * 0.25).to(dtype), (torch.randn(1, BH, n, 64, generator=gen) * 0.25).to(dtype)
+    pk[:, :, n // 2] = pk[:, :, n // 3]                     # two equal columns: the smaller one first
+    got = ops._coarse_topk(pq.to(DEV), pk.to(DEV), topk).cpu()
+    want = O.gen_sparse_indices(pq, pk, topk)
+    scores = (pq.float() @ pk.float().transpose(-1, -2)).to(dtype).float()
+    # a bf16 score may round to the neighbouring value when its fp32 sum is taken in another order: one ulp of the largest scores (|s| < 4)
+    differ, bad = topk_mismatch_rows(got, want, scores, margin=2.0 ** -6 if dtype == torch.bfloat16 else 1e-6)
+    assert bad == 0 and differ <= max(2, 0.02 * BH * M)
+    assert int(got.min()) >= 0 and int(got.max()) < n
+    assert topk == 1 or (got.sort(-1).values.diff(dim=-1) > 0).all(), "duplicate block in a row"
+
+
+def test_coarse_topk_zero_and_negative_scores_tie_and_order():
+    """Scores of exactly zero of either sign tie, so the smaller column wins; all-negative rows come out in order."""
+    pq, pk = torch.zeros(1, 1, 64, 64, dtype=torch.bfloat16), torch.zeros(1, 1, 128, 64, dtype=torch.bfloat16)
+    pq[..., 0] = 1.0
+    pk[0, 0, :, 0] = -torch.arange(128).float().to(torch.bfloat16) - 1
+    pk[0, 0, 64:, 0] = -0.0
+    got = ops._coarse_topk(pq.to(DEV), pk.to(DEV), 8).cpu()
+    assert torch.equal(got, torch.arange(64, 72, dtype=torch.int32).expand(1, 1, 64, 8))
+    pk[0, 0, 64:, 0] = -1000.0
+    got = ops._coarse_topk(pq.to(DEV), pk.to(DEV), 8).cpu()
+    assert torch.equal(got, torch.arange(8, dtype=torch.int32).expand(1, 1, 64, 8))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("N,topk,p_topk", [(2048, 8, 8), (5376, 8, 8), (16384, 8, 8), (16384, 16, 16), (24576, 4, 4), (40960, 16, 16), (73728, 8, 8)])
+def test_select_two_level_is_its_two_steps(N, topk, p_topk, dtype):
+    """One launch (level-2 lists of 8, 21, 64, 96, 160 keys) or two (288 keys): the bits of the coarse step followed by the refine step."""
+    q, k = synth.gaussian_qkv(N + topk, 1, 2, N // 16, 64, n_tensors=2, dtype=dtype)
+    pq, pk = q.to(DEV), k.to(DEV)
+    pq2, pk2 = ops.mean_pool1d(pq, 16), ops.mean_pool1d(pk, 16)
+    idx, pidx = ops._select_two_level(pq, pk, pq2, pk2, topk, p_topk, 16)
+    assert torch.equal(pidx, ops._coarse_topk(pq2, pk2, p_topk))
+    assert torch.equal(idx, ops._refine_topk(pq, pk, pidx, topk, p_topk, 16))
+    want = O.compute_topk_indices_sparse(pq.cpu(), pk.cpu(), pidx.cpu().long(), topk, p_topk, 16)
+    scores = pq.cpu().float() @ pk.cpu().float().transpose(-1, -2)
+    differ, bad = topk_mismatch_rows(idx.cpu(), want, scores, margin=1e-5)       # fp32 sums of 64 products of size < 16 in another order
+    assert bad == 0
