@@ -4,12 +4,12 @@
 //   g  = rotation^-1 (dy), every product and sum rounded to the element type as rope_kernel<..., BWD> does (rope.cu)
 //   dx = rstd * (g w - xh * mean(g w xh)),  dw = sum over rows of g xh,   xh = x rstd,  rstd = rsqrt(mean(x^2) + eps)
 //
-// HBM-bound: reads dy and x, writes dx (dx may be dy's own memory).  A CTA takes chunks of kRowsPerThread * (threads / lanes)
+// HBM-bound: reads dy and x, writes dx (dx may be dy's own memory).  A CTA takes chunks of fb_rows * (threads / lanes)
 // neighbouring tokens of one (b,h) slice, so the slice is found once per chunk and every thread has all its loads (row of dy, of x,
 // of the table) in flight before it uses one.  The weight gradient is kept in registers over all chunks of a CTA, reduced through
 // shared memory, and leaves as one [C] row per CTA; a one-CTA-per-tensor kernel adds the rows in order (bit-reproducible).
-// B=4 H=6 N=16384, [B,N,H,D] storage, both tensors: 151 MB read and written.  The rotation's two launches and the eager fp32
-// formula it replaces moved 14 times that (2.05 ms).
+// B=4 H=6 N=16384, [B,N,H,D] storage, both tensors: 302 MB in 65 us = 4.6 TB/s; the rotation's two launches and the eager fp32 formula it
+// replaces took 2050 us.
 #include <string.h>
 
 #include <type_traits>
@@ -18,7 +18,7 @@
 
 namespace llsa {
 
-constexpr int kFbThreads = 256, kFbRows = 4, kFbC = 64;
+constexpr int kFbThreads = 256, kFbC = 64;
 
 template <typename T>
 struct FrontBwdArgs {
@@ -34,9 +34,12 @@ struct FrontBwdArgs {
   int S, n_chunks;
 };
 
+// Rows a thread takes at a time: with the norm two keep the registers at four CTAs per SM (four rows: 128 registers, two CTAs, 94 us
+// at the size above), without it four.
+constexpr int fb_rows(bool norm) { return norm ? 2 : 4; }
+
 template <typename T>
-__device__ __forceinline__ void ld16(const T* p, float (&v)[16 / sizeof(T)]) {
-  const uint4 x = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void unpack16(const uint4& x, float (&v)[16 / sizeof(T)]) {
   if constexpr (sizeof(T) == 4) {
     v[0] = __uint_as_float(x.x); v[1] = __uint_as_float(x.y); v[2] = __uint_as_float(x.z); v[3] = __uint_as_float(x.w);
   } else {
@@ -45,21 +48,51 @@ __device__ __forceinline__ void ld16(const T* p, float (&v)[16 / sizeof(T)]) {
   }
 }
 template <typename T>
-__device__ __forceinline__ void st16(T* p, const float (&v)[16 / sizeof(T)]) {
-  uint4 x;
-  if constexpr (sizeof(T) == 4) {
-    x = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
-  } else {
-    x = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-  }
-  *reinterpret_cast<uint4*>(p) = x;
+__device__ __forceinline__ uint4 pack16(const float (&v)[16 / sizeof(T)]) {
+  if constexpr (sizeof(T) == 4) return make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+  else return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
 }
 
-// T: element type of the data, TF: of the table (the wider of the two is the type products and sums are rounded to)
+// g of one 16-byte group after the inverse rotation by table entries f.  bf16 data with a bf16 table in packed arithmetic: the sum or
+// product of two bf16 values rounded to fp32 and then to bf16 is the value rounded once (24 >= 2 * 8 + 2 bits).
+__device__ __forceinline__ uint32_t unrotate_pair(uint32_t g, uint32_t f) {       // (cos ge + sin go, -sin ge + cos go)
+  const uint32_t cc = __byte_perm(f, 0u, 0x3232), ss = __byte_perm(f, 0u, 0x1010) ^ 0x80000000u, sw = __byte_perm(g, 0u, 0x1032);
+  const __nv_bfloat162 x = __hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&cc), *reinterpret_cast<const __nv_bfloat162*>(&g)),
+                       y = __hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&ss), *reinterpret_cast<const __nv_bfloat162*>(&sw));
+  const __nv_bfloat162 z = __hadd2_rn(x, y);
+  return *reinterpret_cast<const uint32_t*>(&z);
+}
+template <typename T, typename TF>
+__device__ __forceinline__ void unrotate(uint4& raw, const TF* fp) {
+  if constexpr (sizeof(T) == 2 && sizeof(TF) == 2) {
+    const uint4 f = *reinterpret_cast<const uint4*>(fp);
+    raw = make_uint4(unrotate_pair(raw.x, f.x), unrotate_pair(raw.y, f.y), unrotate_pair(raw.z, f.z), unrotate_pair(raw.w, f.w));
+  } else {
+    using P = typename std::conditional<(sizeof(TF) > sizeof(T)), TF, T>::type;      // products and sums are rounded to the wider type
+    constexpr int VEC = 16 / sizeof(T);
+    float g[VEC], f[VEC];
+    unpack16<T>(raw, g);
+#pragma unroll
+    for (int i = 0; i < VEC; i += 16 / (int) sizeof(TF)) {
+      float part[16 / sizeof(TF)];
+      unpack16<TF>(*reinterpret_cast<const uint4*>(fp + i), part);
+#pragma unroll
+      for (int j = 0; j < 16 / (int) sizeof(TF); ++j) f[i + j] = part[j];
+    }
+#pragma unroll
+    for (int j = 0; j < VEC; j += 2) {
+      const float sn = f[j], cs = f[j + 1], ge = g[j], go = g[j + 1];
+      g[j] = round_to<P>(__fadd_rn(round_to<P>(__fmul_rn(cs, ge)), round_to<P>(__fmul_rn(sn, go))));
+      g[j + 1] = round_to<P>(__fadd_rn(round_to<P>(__fmul_rn(-sn, ge)), round_to<P>(__fmul_rn(cs, go))));
+    }
+    raw = pack16<T>(g);
+  }
+}
+
+// T: element type of the data, TF: of the table
 template <typename T, typename TF, bool NORM>
-__global__ void __launch_bounds__(kFbThreads) front_bwd_kernel(FrontBwdArgs<T> a) {
-  constexpr int VEC = 16 / sizeof(T), LANES = kFbC / VEC, STEP = kFbThreads / LANES;
-  using P = typename std::conditional<(sizeof(TF) > sizeof(T)), TF, T>::type;
+__global__ void __launch_bounds__(kFbThreads, NORM ? 4 : 1) front_bwd_kernel(FrontBwdArgs<T> a) {
+  constexpr int VEC = 16 / sizeof(T), LANES = kFbC / VEC, STEP = kFbThreads / LANES, ROWS = fb_rows(NORM);
   const int ti = blockIdx.y, r0 = threadIdx.x / LANES, c = (threadIdx.x % LANES) * VEC;
   const bool norm = NORM && ((a.norm_mask >> ti) & 1);
   const TF* freq = reinterpret_cast<const TF*>(a.freq);
@@ -70,66 +103,47 @@ __global__ void __launch_bounds__(kFbThreads) front_bwd_kernel(FrontBwdArgs<T> a
     dw[i] = 0.f;
   }
   for (int ch = blockIdx.x; ch < a.n_chunks; ch += gridDim.x) {
-    const int bh = ch / a.chunks_per_head, s0 = (ch - bh * a.chunks_per_head) * (STEP * kFbRows) + r0;
+    const int bh = ch / a.chunks_per_head, s0 = (ch - bh * a.chunks_per_head) * (STEP * ROWS) + r0;
     const int b = bh / a.H, h = bh - b * a.H;
     const T* dyp = a.dy[ti].head(b, h) + c;
     const T* xp = NORM ? a.x[ti].head(b, h) + c : nullptr;
     T* dxp = a.dx[ti].head(b, h) + c;
-    float g[kFbRows][VEC], x[kFbRows][VEC];
+    uint4 g[ROWS], x[ROWS];
 #pragma unroll
-    for (int u = 0; u < kFbRows; ++u) {     // rows past the end are computed on the last row (the reductions need every lane) and dropped
+    for (int u = 0; u < ROWS; ++u) {     // rows past the end are computed on the last row (the reductions need every lane) and dropped
       const int64_t s = min(s0 + u * STEP, a.S - 1);
-      ld16<T>(dyp + s * a.dy[ti].sn, g[u]);
-      if (NORM) if (norm) ld16<T>(xp + s * a.x[ti].sn, x[u]);
+      g[u] = *reinterpret_cast<const uint4*>(dyp + s * a.dy[ti].sn);
+      if (NORM) if (norm) x[u] = *reinterpret_cast<const uint4*>(xp + s * a.x[ti].sn);
     }
-    if (freq) {
 #pragma unroll
-      for (int u = 0; u < kFbRows; ++u) {
-        const TF* fp = freq + (int64_t) min(s0 + u * STEP, a.S - 1) * a.fs + c;
-        float f[VEC];
-        if constexpr (sizeof(TF) == sizeof(T)) ld16<TF>(fp, f);
-        else {
-          float f0[4], f1[4];
-          ld16<TF>(fp, f0);
-          ld16<TF>(fp + 4, f1);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) { f[i] = f0[i]; f[4 + i] = f1[i]; }
-        }
-#pragma unroll
-        for (int j = 0; j < VEC; j += 2) {
-          const float sn = f[j], cs = f[j + 1], ge = g[u][j], go = g[u][j + 1];
-          g[u][j] = round_to<T>(round_to<P>(__fadd_rn(round_to<P>(__fmul_rn(cs, ge)), round_to<P>(__fmul_rn(sn, go)))));
-          g[u][j + 1] = round_to<T>(round_to<P>(__fadd_rn(round_to<P>(__fmul_rn(-sn, ge)), round_to<P>(__fmul_rn(cs, go)))));
-        }
-      }
-    }
-    if (NORM) {
-      if (norm) {
-#pragma unroll
-        for (int u = 0; u < kFbRows; ++u) {
+    for (int u = 0; u < ROWS; ++u) {
+      const int s = s0 + u * STEP;
+      if (freq) unrotate<T, TF>(g[u], freq + (int64_t) min(s, a.S - 1) * a.fs + c);
+      if (NORM) {
+        if (norm) {
+          float gv[VEC], xv[VEC];
+          unpack16<T>(g[u], gv);
+          unpack16<T>(x[u], xv);
           float ss = 0.f, dot = 0.f;
 #pragma unroll
-          for (int i = 0; i < VEC; ++i) { ss = fmaf(x[u][i], x[u][i], ss); dot = fmaf(g[u][i] * w[i], x[u][i], dot); }
+          for (int i = 0; i < VEC; ++i) { ss = fmaf(xv[i], xv[i], ss); dot = fmaf(gv[i] * w[i], xv[i], dot); }
 #pragma unroll
           for (int o = 1; o < LANES; o <<= 1) {
             ss += __shfl_xor_sync(0xffffffffu, ss, o);
             dot += __shfl_xor_sync(0xffffffffu, dot, o);
           }
           const float rstd = rsqrtf(ss / (float) kFbC + a.eps), k = dot * rstd / (float) kFbC;      // k = mean(g w xh)
-          const bool live = s0 + u * STEP < a.S;
+          const float live = s < a.S ? 1.f : 0.f;
 #pragma unroll
           for (int i = 0; i < VEC; ++i) {
-            const float xh = x[u][i] * rstd;
-            if (live) dw[i] = fmaf(g[u][i], xh, dw[i]);
-            g[u][i] = rstd * (g[u][i] * w[i] - xh * k);
+            const float xh = xv[i] * rstd;
+            dw[i] = fmaf(gv[i] * live, xh, dw[i]);
+            gv[i] = rstd * (gv[i] * w[i] - xh * k);
           }
+          g[u] = pack16<T>(gv);
         }
       }
-    }
-#pragma unroll
-    for (int u = 0; u < kFbRows; ++u) {
-      const int s = s0 + u * STEP;
-      if (s < a.S) st16<T>(dxp + (int64_t) s * a.dx[ti].sn, g[u]);
+      if (s < a.S) *reinterpret_cast<uint4*>(dxp + (int64_t) s * a.dx[ti].sn) = g[u];
     }
   }
   if (NORM && a.dw_partial) {
@@ -158,7 +172,7 @@ __global__ void __launch_bounds__(1024) front_dw_kernel(const float* __restrict_
   const int c = threadIdx.x & 63, k = threadIdx.x >> 6;
   const float* p = partial + (int64_t) blockIdx.x * rows * kFbC + c;
   float s = 0.f;
-#pragma unroll 4
+#pragma unroll 10
   for (int r = k; r < rows; r += 16) s += p[(int64_t) r * kFbC];
   sm[k][c] = s;
   __syncthreads();
@@ -201,7 +215,7 @@ static int front_bwd_typed(int n, const LlsaTensor* dy, const LlsaTensor* x, con
   a.H = (int) dy[0].shape[1];
   a.S = (int) dy[0].shape[2];
   const int64_t BH = dy[0].shape[0] * dy[0].shape[1];
-  const int rows = kFbRows * kFbThreads / (kFbC * (int) sizeof(T) / 16);
+  const int rows = fb_rows(norm_mask != 0) * kFbThreads / (kFbC * (int) sizeof(T) / 16);
   a.chunks_per_head = (a.S + rows - 1) / rows;
   const int64_t chunks = BH * a.chunks_per_head;
   LLSA_REQUIRE(chunks < (1ll << 31), LLSA_ERR_SHAPE, "rms_rope_bwd: too many rows");

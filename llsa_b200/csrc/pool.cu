@@ -6,7 +6,7 @@
 // accumulator in fp32 registers but round it to T after each add, which gives
 // the same bits.
 //
-// pool_pyramid_kernel writes every pyramid level of q, k and v in one pass over
+// pool_pyramid_kernel (any block size and channel count; pool_pyramid_bf16_kernel for the attention shapes in bf16) writes every pyramid level of q, k and v in one pass over
 // HBM: one CTA owns one level-2 row (bs level-1 rows x bs tokens), each thread
 // a 16-byte channel group of one level-1 row; the bs loads of a thread are
 // independent 128-bit loads, the level-2 row is reduced through shared memory.
@@ -68,15 +68,25 @@ struct PyramidArgs {
 // RMSNorm of one token row held by `lanes` neighbouring threads (VEC consecutive channels each; lanes a power of two, the
 // group aligned inside its warp): squares summed in channel order per thread, then a butterfly over the group.  The
 // stand-alone kernel and the fused pooling pass share this function, so their results are identical bit for bit.
-template <typename T, int VEC>
-__device__ __forceinline__ void rms_normalise(float (&v)[VEC], const float* w, int c, int lanes, int C, float eps) {
+// `w`: the VEC weights of this thread's channels.  The caller rounds.
+template <int VEC>
+__device__ __forceinline__ void rms_normalise_f32(float (&v)[VEC], const float (&w)[VEC], int lanes, int C, float eps) {
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < VEC; ++i) ss = __fmaf_rn(v[i], v[i], ss);
   for (int o = 1; o < lanes; o <<= 1) ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));
   const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(ss, (float) C), eps));
 #pragma unroll
-  for (int i = 0; i < VEC; ++i) v[i] = round_to<T>(__fmul_rn(__fmul_rn(v[i], rstd), w ? w[c + i] : 1.f));
+  for (int i = 0; i < VEC; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], rstd), w[i]);
+}
+template <typename T, int VEC>
+__device__ __forceinline__ void rms_normalise(float (&v)[VEC], const float* w, int c, int lanes, int C, float eps) {
+  float wv[VEC];
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) wv[i] = w ? w[c + i] : 1.f;
+  rms_normalise_f32<VEC>(v, wv, lanes, C, eps);
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) v[i] = round_to<T>(v[i]);
 }
 
 // Interleaved-pair rotation of VEC channels of one token, every product and sum rounded to T separately
@@ -174,6 +184,99 @@ __global__ void pool_pyramid_kernel(PyramidArgs<T> a, int rows_per_cta, int64_t 
       for (int rr = 0; rr < a.bs; ++rr) acc2 = round_to<T>(acc2 + smem[rr * a.C + ch]);
       acc2 = round_to<T>(__fdiv_rn(acc2, (float) a.bs));
       a.y2[ti][(bh * ctas_per_head + grp) * a.C + ch] = from_f32<T>(acc2);
+    }
+  }
+}
+
+// ---- bf16, 64 channels, blocks of 16 tokens: the shape of every attention call -------------------------------------------------
+// The contract of the kernel above in packed bf16 arithmetic: a sum or product of two bf16 values rounded to fp32 and then to bf16 is
+// the value rounded to bf16 once (24 >= 2 * 8 + 2 bits), so `add`, the rotation's products and sums and the division by 16 are one
+// bf16x2 instruction for two channels instead of six.  HBM-bound: a thread has its sixteen (transformed tensors: eight) 16-byte loads
+// in flight before it uses the first.  B=1 H=6 N=16384 with norm and rotation, [B,N,H,D] storage: 30.7 -> 14.9 us; B=4: 115 ->
+// 48.5 us (252 MB moved: 5.2 TB/s); B=8 H=6 N=16384 without: 67.7 -> 60.5 us (322 MB: 5.3 TB/s).
+using bf162 = __nv_bfloat162;
+__device__ __forceinline__ uint32_t as_u32(bf162 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ bf162 as_bf2(uint32_t v) { return *reinterpret_cast<bf162*>(&v); }
+__device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) { return as_u32(__hadd2_rn(as_bf2(a), as_bf2(b))); }
+__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) { return as_u32(__hmul2_rn(as_bf2(a), as_bf2(b))); }
+__device__ __forceinline__ uint4 ld_stream(const void* p) {      // volatile: the loads of a thread stay together in front of their uses
+  uint4 v;
+  asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+// one rotated pair: x = (xe, xo), f = (sin, cos) -> (cos xe - sin xo, sin xe + cos xo)
+__device__ __forceinline__ uint32_t rope_pair(uint32_t x, uint32_t f) {
+  const uint32_t cc = __byte_perm(f, 0u, 0x3232), ss = __byte_perm(f, 0u, 0x1010) ^ 0x00008000u, sw = __byte_perm(x, 0u, 0x1032);
+  return add2(mul2(cc, x), mul2(ss, sw));
+}
+
+template <int LEVELS, bool ROPE, bool NORM>
+__global__ void __launch_bounds__(128) pool_pyramid_bf16_kernel(PyramidArgs<__nv_bfloat16> a, int groups_per_head) {
+  constexpr int BS = 16, C = 64;
+  __shared__ __align__(16) uint4 s_row[LEVELS == 2 ? BS * 8 : 1];
+  const int ti = blockIdx.y, bh = blockIdx.x / groups_per_head, grp = blockIdx.x - bh * groups_per_head;
+  const int b = bh / a.H, h = bh - b * a.H, r = threadIdx.x >> 3, c = (threadIdx.x & 7) * 8;
+  const int row1 = grp * BS + r;                           // level-1 row inside (b,h)
+  const bool live = LEVELS == 2 || row1 < a.n1;            // past the last row: computed on it (the norm's reductions need every lane), dropped
+  const int64_t tok0 = (int64_t) (live ? row1 : (int) a.n1 - 1) * BS;
+  const __nv_bfloat16* xp = a.x[ti].row(b, h, tok0) + c;
+  const int64_t sn = a.x[ti].sn;
+  uint32_t acc[4] = {0u, 0u, 0u, 0u};
+  auto pool = [&](const uint4& v) {
+    acc[0] = add2(acc[0], v.x); acc[1] = add2(acc[1], v.y); acc[2] = add2(acc[2], v.z); acc[3] = add2(acc[3], v.w);
+  };
+  const bool rope = ROPE && ((a.rope_mask >> ti) & 1), norm = NORM && ((a.norm_mask >> ti) & 1);
+  if (!rope && !norm) {
+    uint4 v[BS];
+#pragma unroll
+    for (int t = 0; t < BS; ++t) v[t] = ld_stream(xp + t * sn);
+#pragma unroll
+    for (int t = 0; t < BS; ++t) pool(v[t]);
+  } else if constexpr (ROPE || NORM) {
+    __nv_bfloat16* rp = a.xr[ti].row(b, h, tok0) + c;
+    const int64_t rs = a.xr[ti].sn;
+    const __nv_bfloat16* fp = rope ? a.freq + tok0 * a.fs + c : nullptr;
+    float w[8];
+    if (NORM) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w[i] = norm && a.norm_w[ti] ? __ldg(a.norm_w[ti] + c + i) : 1.f;
+    }
+#pragma unroll 1
+    for (int t0 = 0; t0 < BS; t0 += 8) {
+      uint4 v[8], f[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) v[t] = ld_stream(xp + (t0 + t) * sn);
+      if (ROPE && rope) {
+#pragma unroll
+        for (int t = 0; t < 8; ++t) f[t] = ld_stream(fp + (t0 + t) * a.fs);
+      }
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        if (NORM && norm) {
+          float x[8] = {bf16_lo(v[t].x), bf16_hi(v[t].x), bf16_lo(v[t].y), bf16_hi(v[t].y), bf16_lo(v[t].z), bf16_hi(v[t].z), bf16_lo(v[t].w), bf16_hi(v[t].w)};
+          rms_normalise_f32<8>(x, w, 8, C, a.eps);
+          v[t] = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+        }
+        if (ROPE && rope)
+          v[t] = make_uint4(rope_pair(v[t].x, f[t].x), rope_pair(v[t].y, f[t].y), rope_pair(v[t].z, f[t].z), rope_pair(v[t].w, f[t].w));
+        if (live) *reinterpret_cast<uint4*>(rp + (t0 + t) * rs) = v[t];
+        pool(v[t]);
+      }
+    }
+  }
+  constexpr uint32_t kSixteenth = 0x3D803D80u;             // 1/16 twice
+  const uint4 y = make_uint4(mul2(acc[0], kSixteenth), mul2(acc[1], kSixteenth), mul2(acc[2], kSixteenth), mul2(acc[3], kSixteenth));
+  if (live) *reinterpret_cast<uint4*>(a.y1[ti] + ((int64_t) bh * a.n1 + row1) * C + c) = y;
+  if (LEVELS == 2) {
+    s_row[threadIdx.x] = y;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(s_row) + threadIdx.x;
+      uint32_t s = 0u;
+#pragma unroll
+      for (int i = 0; i < BS; ++i) s = add2(s, p[i * 32]);
+      reinterpret_cast<uint32_t*>(a.y2[ti] + ((int64_t) bh * groups_per_head + grp) * C)[threadIdx.x] = mul2(s, kSixteenth);
     }
   }
 }
@@ -300,6 +403,14 @@ struct NormSpec {
   float eps;
 };
 
+template <int LEVELS>
+static void launch_pyramid_bf16(const PyramidArgs<__nv_bfloat16>& a, dim3 grid, int groups, cudaStream_t st) {
+  if (a.rope_mask && a.norm_mask) pool_pyramid_bf16_kernel<LEVELS, true, true><<<grid, 128, 0, st>>>(a, groups);
+  else if (a.rope_mask) pool_pyramid_bf16_kernel<LEVELS, true, false><<<grid, 128, 0, st>>>(a, groups);
+  else if (a.norm_mask) pool_pyramid_bf16_kernel<LEVELS, false, true><<<grid, 128, 0, st>>>(a, groups);
+  else pool_pyramid_bf16_kernel<LEVELS, false, false><<<grid, 128, 0, st>>>(a, groups);
+}
+
 template <typename T, int LEVELS>
 static void launch_pyramid_variant(const PyramidArgs<T>& a, dim3 grid, int threads, size_t smem, int rows, int64_t per_head, cudaStream_t st) {
   if (a.rope_mask && a.norm_mask) pool_pyramid_kernel<T, LEVELS, true, true><<<grid, threads, smem, st>>>(a, rows, per_head);
@@ -335,6 +446,16 @@ static int launch_pyramid(int n, const LlsaTensor* x, const LlsaTensor* y1, cons
   }
   a.H = (int) H; a.C = (int) C; a.n1 = N / bs; a.bs = bs;
   const int lanes = (int) (C / VEC);
+  if constexpr (sizeof(T) == 2) {
+    if (C == 64 && bs == 16 && a.n1 < (1ll << 27)) {
+      const int64_t groups = (a.n1 + 15) / 16;
+      const dim3 grid((unsigned) (B * H * groups), n);
+      if (y2) launch_pyramid_bf16<2>(a, grid, (int) groups, st);
+      else launch_pyramid_bf16<1>(a, grid, (int) groups, st);
+      LLSA_LAUNCH_OK("pool_pyramid_bf16_kernel");
+      return LLSA_OK;
+    }
+  }
   if (y2) {
     const int64_t n2 = a.n1 / bs;
     dim3 grid((unsigned) (B * H * n2), n);
