@@ -147,9 +147,9 @@ int llsa_select_two_level(const LlsaTensor* pq1, const LlsaTensor* pk1, const Ll
 /* ---- index transpose: src/llsa/kernel/triton/indices_transpose.py ---------
  * Query-major lists idx [B,H,M,T] (I32/I64, values in [0,n_kv)) -> KV-major CSR:
  * offsets [B,H,n_kv+1] (I32 or I64) and flat [B,H,M*T] (I32), each bucket in
- * ascending query order (a stable counting sort without atomics).  `scratch`
- * is llsa_transpose_scratch_bytes() bytes of device memory (may be NULL when
- * that returns 0); `status` is one int32 on the device, set non-zero if an
+ * ascending query order (a stable counting sort).  `scratch` is
+ * llsa_transpose_scratch_bytes() bytes of device memory (may be NULL when that
+ * returns 0); it is checked, and no longer written (the count tables now fit in shared memory); `status` is one int32 on the device, set non-zero if an
  * index is out of range (may be NULL).  Replaces transpose_indices =
  * _count_k_major + torch.cumsum + _k_major_indices (indices_transpose.py:6-109). */
 size_t llsa_transpose_scratch_bytes(int64_t B, int64_t H, int64_t M, int64_t T, int64_t n_kv);

@@ -3,19 +3,25 @@
 //
 // The reference builds the CSR with a global-atomic histogram, a cumsum and a
 // second pass that claims slots with atomics, which leaves the order inside a
-// bucket to chance (indices_transpose.py:23-27, :70-78).  Here one CTA per (b,h)
-// runs a stable counting sort WITHOUT atomics:
-//   1. the E = M*T entries are cut into W contiguous segments, one per warp; a
-//      warp walks its segment 32 entries at a time, groups equal keys with
-//      __match_any_sync and lets the lowest lane of each group add the group size
-//      to the warp's own row of a [W][n_kv] count table;
-//   2. every key's column of the table is turned into exclusive prefixes over the
-//      segments and the column totals are scanned across keys -> offsets;
-//   3. the warps walk their segments again; an entry lands at
-//      offsets[key] + (count in earlier segments) + (count earlier in this segment)
-//      + (rank inside its match group).
-// Entries keep their original relative order, so every bucket lists its query
-// blocks in ascending order and the output is bit-reproducible.
+// bucket to chance (indices_transpose.py:23-27, :70-78).  Here it is a stable
+// counting sort WITHOUT atomics: entries keep their original relative order, so
+// every bucket lists its query blocks in ascending order and the output is
+// bit-reproducible.
+//
+// transpose_range_kernel: a CTA owns a RANGE OF KEYS of one (b,h) and scans all E = M*T entries of the head twice.
+//   1. the entries are cut into W contiguous segments, one per warp; a warp counts those inside the CTA's range in its own row of a
+//      [W][keys of the range] table (shared-memory atomics: a count has no order).  Entries with smaller keys are counted on
+//      the side: that count is the range's first position, so ranges need nothing from one another;
+//   2. every key's column of the table is turned into exclusive prefixes over the segments and the column totals are scanned
+//      across the range's keys -> offsets;
+//   3. the warps walk their segments again, 32 entries at a time; lanes with equal keys find one another by setting their bits in the
+//      key's mask word, and an entry lands at
+//      offsets[key] + (count in earlier segments) + (count earlier in this segment) + (equal keys in lower lanes).
+// The tables stay in shared memory whatever the number of keys, and a head occupies as many SMs as it has ranges: the scan of the
+// entries is repeated per range, but they come from L2 and most lanes have nothing to do.  One CTA per head with all keys and
+// __match_any_sync to group equal keys (transpose_kernel, kept for the entry point with the built-in table) took 28 us for 48 heads of
+// 8,192 entries, 128 us for 5 of 40,960 and 674 us for 6 of 131,072: match.any occupies an SM for about a hundred cycles a warp (key
+// ranges with it were slower still); this kernel 13, 36 and 107.
 #include <mutex>
 
 #include "common.cuh"
@@ -64,6 +70,145 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
   return excl;
 }
 
+// Work ranges of the dK/dV kernel: nominally S = range_entries entries each, but a bucket of at most S entries is never cut -- the range
+// that would begin inside it begins at the bucket's first entry instead (ranges then hold 1 .. 2 S - 1 entries); only longer buckets
+// are cut, at multiples of S.  The entry that lands on such a multiple knows its bucket [b0, b1).
+__device__ __forceinline__ void place_range(const TransposeArgs& a, int64_t bh, int pos, int b0, int b1, int key) {
+  const int S = a.range_entries;
+  a.ranges[bh * (((int) a.E + S - 1) / S) + pos / S] = make_int2(b1 - b0 <= S ? b0 : pos, key);
+}
+
+// ---- one CTA per (b,h) and key range ----------------------------------------------------------------
+template <int W>
+__global__ void __launch_bounds__(W * 32) transpose_range_kernel(TransposeArgs a, int keys_per_range, uint32_t t_magic) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ int warp_sums[32];
+  __shared__ int s_below[W], s_kept[W];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t bh = blockIdx.y;
+  const int E = (int) a.E, n = (int) a.n_kv, lo = (int) blockIdx.x * keys_per_range, K = min(keys_per_range, n - lo);
+  const bool last = (int) blockIdx.x + 1 == (int) gridDim.x;
+  int* base = reinterpret_cast<int*>(smraw);             // [K + 1]
+  int* tab = base + keys_per_range + 1;                  // [W][K] entries seen, then [W][K] lanes that hold the key right now
+  for (int i = threadIdx.x; i < 2 * W * K; i += blockDim.x) tab[i] = 0;
+  __syncthreads();
+
+  const int L = ((E + W - 1) / W + 31) / 32 * 32, seg0 = min(E, warp * L), seg1 = min(E, seg0 + L);
+  const int64_t* idx64 = reinterpret_cast<const int64_t*>(a.idx.p) + bh * E;
+  const int32_t* idx32 = reinterpret_cast<const int32_t*>(a.idx.p) + bh * E;
+  int32_t* flat = a.flat + bh * E;
+  int32_t* pairs = a.pairs ? a.pairs + bh * E : nullptr;
+  // a key outside [0, n) (whatever its upper half holds) comes back as -1
+  auto key_at = [&](int e) -> int {
+    if (!a.idx.is64) return idx32[e];
+    const int64_t k = idx64[e];
+    return k < 0 || k >= n ? -1 : (int) k;
+  };
+  int* mytab = tab + warp * K;
+  unsigned* mymask = reinterpret_cast<unsigned*>(tab + (W + warp) * K);
+  const unsigned lt_mask = (1u << lane) - 1u;
+  // walk(f): f(entry, key - lo, inside the range) for 32 entries at a time, four loads ahead
+  auto walk = [&](auto&& f) {
+    constexpr int AHEAD = 4;
+    int key[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int e = seg0 + u * 32 + lane;
+      key[u] = e < seg1 ? key_at(e) : -1;
+    }
+    for (int e0 = seg0; e0 < seg1; e0 += 32 * AHEAD) {
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        const int e = e0 + u * 32 + lane, en = e + 32 * AHEAD, k = key[u];
+        key[u] = en < seg1 ? key_at(en) : -1;
+        f(e, k, e < seg1);
+      }
+    }
+  };
+
+  // ---- 1: per-segment histograms of the range, entries below it
+  int below = 0, kept = 0;
+  walk([&](int e, int k, bool real) {
+    const bool valid = real && k >= 0 && k < n;
+    if (real && !valid && last && a.status) atomicOr(a.status, (int) LLSA_DEV_BAD_INDEX);
+    below += valid && k < lo;
+    kept += valid;
+    const int kk = k - lo;
+    if (valid && kk >= 0 && kk < K) atomicAdd(&mytab[kk], 1);
+  });
+  below = __reduce_add_sync(0xffffffffu, below);
+  kept = __reduce_add_sync(0xffffffffu, kept);
+  if (lane == 0) { s_below[warp] = below; s_kept[warp] = kept; }
+  __syncthreads();
+  int total_entries = 0, carry = 0;
+#pragma unroll
+  for (int w = 0; w < W; ++w) { carry += s_below[w]; total_entries += s_kept[w]; }
+
+  // ---- 2: per-key prefix over segments, then scan of the totals over the range's keys
+  for (int j0 = 0; j0 < K; j0 += blockDim.x) {
+    const int j = j0 + threadIdx.x;
+    int run = 0;
+    if (j < K) {
+#pragma unroll
+      for (int s = 0; s < W; ++s) {
+        const int c = tab[s * K + j];
+        tab[s * K + j] = run;
+        run += c;
+      }
+    }
+    int total;
+    const int excl = block_exclusive_scan(run, warp_sums, total);
+    if (j < K) {
+      base[j] = carry + excl;
+      if (a.off64) reinterpret_cast<int64_t*>(a.offsets)[bh * (n + 1) + lo + j] = carry + excl;
+      else reinterpret_cast<int32_t*>(a.offsets)[bh * (n + 1) + lo + j] = carry + excl;
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) {
+    base[K] = carry;
+    if (last) {
+      if (a.off64) reinterpret_cast<int64_t*>(a.offsets)[bh * (n + 1) + n] = carry;
+      else reinterpret_cast<int32_t*>(a.offsets)[bh * (n + 1) + n] = carry;
+    }
+  }
+  __syncthreads();
+  // work ranges that lie wholly behind the last entry (entries were dropped, or E is not a multiple of the range size) are empty
+  if (a.ranges && last) {
+    const int R = (E + a.range_entries - 1) / a.range_entries;
+    for (int r = total_entries / a.range_entries + threadIdx.x; r < R; r += blockDim.x)
+      if (r * a.range_entries >= total_entries) a.ranges[bh * R + r] = make_int2(total_entries, n - 1);
+  }
+
+  // ---- 3: stable fill
+  walk([&](int e, int k, bool real) {
+    const int kk = k - lo;
+    const bool in = real && k >= 0 && k < n && kk >= 0 && kk < K;
+    if (!__any_sync(0xffffffffu, in)) return;
+    if (in) atomicOr(&mymask[kk], 1u << lane);
+    __syncwarp();
+    unsigned peers = 0;
+    int seen = 0;
+    if (in) {
+      peers = mymask[kk];
+      seen = mytab[kk];
+      const int pos = base[kk] + seen + __popc(peers & lt_mask);
+      int m = t_magic == 0u ? e : (int) __umulhi((uint32_t) e, t_magic);      // e / T, or one more where e * T passes 2^32
+      m -= (int64_t) m * a.T > e;
+      flat[pos] = m;
+      if (pairs) pairs[pos] = e;
+      if (a.ranges && (pos & (a.range_entries - 1)) == 0) place_range(a, bh, pos, base[kk], base[kk + 1], k);
+    }
+    __syncwarp();
+    if (in && (peers & lt_mask) == 0) {
+      mytab[kk] = seen + __popc(peers);
+      mymask[kk] = 0u;
+    }
+    __syncwarp();
+  });
+}
+
+// ---- one CTA per (b,h), all keys, the count table in shared or global memory ------------------------
 __global__ void __launch_bounds__(1024) transpose_kernel(TransposeArgs a) {
   extern __shared__ unsigned char smraw[];
   __shared__ int warp_sums[32];
@@ -128,15 +273,7 @@ __global__ void __launch_bounds__(1024) transpose_kernel(TransposeArgs a) {
     else reinterpret_cast<int32_t*>(a.offsets)[bh * (n + 1) + n] = carry;
   }
   __syncthreads();
-  // ranges that lie wholly behind the last entry (entries were dropped, or E is not a multiple of the range size) are empty
-  if (a.ranges) {
-    const int64_t R = (E + a.range_entries - 1) / a.range_entries;
-    for (int64_t r = threadIdx.x; r < R; r += blockDim.x)
-      if (r * a.range_entries >= carry) a.ranges[bh * R + r] = make_int2(carry, (int) n - 1);
-  }
-
   // ---- 3: stable fill
-  const int total_entries = carry;          // every thread ran the same scan: entries that were kept
   for (int64_t e0 = seg0; e0 < seg1; e0 += 32) {
     const int64_t e = e0 + lane;
     bool valid = e < seg1;
@@ -151,15 +288,6 @@ __global__ void __launch_bounds__(1024) transpose_kernel(TransposeArgs a) {
       const int pos = base[key] + seen + __popc(peers & lt_mask);
       if (pos < E) {
         a.flat[bh * E + pos] = (int32_t) (e / a.T);
-        if (a.pairs) a.pairs[bh * E + pos] = (int32_t) e;
-        // Work ranges of the dK/dV kernel: nominally S = range_entries entries each, but a bucket of at most S entries is
-        // never cut -- the range that would begin inside it begins at the bucket's first entry instead (ranges then hold
-        // 1 .. 2 S - 1 entries); only longer buckets are cut, at multiples of S.  The entry that lands on such a multiple knows
-        // its bucket and that bucket's extent.
-        if (a.ranges && pos % a.range_entries == 0) {
-          const int S = a.range_entries, b0 = base[key], b1 = key + 1 < n ? base[key + 1] : total_entries;
-          a.ranges[bh * ((E + S - 1) / S) + pos / S] = make_int2(b1 - b0 <= S ? b0 : pos, (int) key);
-        }
       }
     }
     __syncwarp();
@@ -229,11 +357,10 @@ static int transpose_impl(const LlsaTensor* idx, const LlsaTensor* offsets, cons
   }
   // the per-key prefixes over the segments are 16-bit: with distinct keys inside a row a key occurs at most M times per head
   LLSA_REQUIRE(M <= 65535, LLSA_ERR_SHAPE, "transpose_indices: M=%lld query blocks per head exceed the supported 65535", (long long) M);
+  LLSA_REQUIRE((int64_t) n_kv * 4 <= 200 * 1024, LLSA_ERR_SHAPE, "transpose_indices: n_kv=%lld too large", (long long) n_kv);
+  const size_t need = llsa_transpose_scratch_bytes(B, H, M, T, n_kv);
+  LLSA_REQUIRE(need == 0 || (scratch && scratch_bytes >= need), LLSA_ERR_WORKSPACE, "transpose_indices: needs %zu bytes of scratch", need);
   if (B * H == 0) return LLSA_OK;
-  size_t smem;
-  bool global;
-  const int W = plan_transpose(n_kv, E, &smem, &global);
-  LLSA_REQUIRE(smem <= 200 * 1024, LLSA_ERR_SHAPE, "transpose_indices: n_kv=%lld too large", (long long) n_kv);
   TransposeArgs a;
   a.idx = make_idx(idx);
   a.offsets = offsets->ptr;
@@ -247,15 +374,30 @@ static int transpose_impl(const LlsaTensor* idx, const LlsaTensor* offsets, cons
   a.n_kv = n_kv;
   a.gtab = nullptr;
   a.status = status;
-  if (global) {
-    const size_t need = (size_t) B * H * 32 * n_kv * 2;
-    LLSA_REQUIRE(scratch && scratch_bytes >= need, LLSA_ERR_WORKSPACE, "transpose_indices: needs %zu bytes of scratch", need);
-    a.gtab = (uint16_t*) scratch;
+  // e / T from the high half of e * ceil(2^32 / T); T = 1 is marked by 0
+  const uint32_t t_magic = T == 1 ? 0u : (uint32_t) (((1ull << 32) + T - 1) / (uint64_t) T);
+  // Warps: a warp's walk is a chain of some 300 cycles per 32 entries, so long lists get 32 (5 heads of 40,960 entries: 36 us against 46
+  // with 16), short ones 16 (fewer rows to clear and to scan: 24 heads of 2,048 entries 5.5 us against 6.9).  Ranges: about 96 CTAs on the
+  // GPU, since every range scans the whole list (48 heads of 8,192 entries: 13 us with 2 ranges, 19 with 4), at least 128 keys each,
+  // the tables within shared memory.
+  const int warps = E > 16384 ? 32 : 16;
+  const int64_t most_keys = (196 * 1024 / 4 - 1) / (2 * warps + 1);
+  int64_t ranges_per_head = (96 + B * H - 1) / (B * H);
+  const int64_t most = (n_kv + 127) / 128, fewest = (n_kv + most_keys - 1) / most_keys;
+  ranges_per_head = ranges_per_head > most ? most : ranges_per_head;
+  ranges_per_head = ranges_per_head < fewest ? fewest : ranges_per_head;
+  const int keys = (int) ((n_kv + ranges_per_head - 1) / ranges_per_head);
+  const dim3 grid((unsigned) ((n_kv + keys - 1) / keys), (unsigned) (B * H));
+  const size_t smem = ((size_t) keys * (2 * warps + 1) + 1) * sizeof(int);
+  cudaStream_t st = (cudaStream_t) stream;
+  if (warps == 32) {
+    LLSA_SMEM_LIMIT((transpose_range_kernel<32>), smem);
+    transpose_range_kernel<32><<<grid, 32 * 32, smem, st>>>(a, keys, t_magic);
+  } else {
+    LLSA_SMEM_LIMIT((transpose_range_kernel<16>), smem);
+    transpose_range_kernel<16><<<grid, 16 * 32, smem, st>>>(a, keys, t_magic);
   }
-  // a segment holds at most 65535 entries, so the 16-bit counters cannot overflow
-  LLSA_SMEM_LIMIT((transpose_kernel), smem);
-  transpose_kernel<<<(unsigned) (B * H), W * 32, smem, (cudaStream_t) stream>>>(a);
-  LLSA_LAUNCH_OK("transpose_kernel");
+  LLSA_LAUNCH_OK("transpose_range_kernel");
   return LLSA_OK;
 }
 
@@ -348,9 +490,6 @@ extern "C" int llsa_transpose_indices_noalloc(const LlsaTensor* idx, const LlsaT
   a.offsets = offsets->ptr;
   a.off64 = offsets->dtype == LLSA_I64;
   a.flat = (int32_t*) flat->ptr;
-  a.pairs = nullptr;
-  a.ranges = nullptr;
-  a.range_entries = kRangeEntries;
   a.E = E;
   a.T = (int) T;
   a.n_kv = n_kv;

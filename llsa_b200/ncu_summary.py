@@ -23,7 +23,7 @@ GROUPS = {
     "pool_pyramid": ("pool_pyramid_kernel", "pool_pyramid_bf16_kernel"),
     "coarse_topk": ("coarse_topk_mma_kernel", "coarse_topk_kernel"),
     "refine_topk": ("refine_topk_kernel",),
-    "transpose_indices": ("transpose_kernel",),
+    "transpose_indices": ("transpose_range_kernel",),
 }
 UNIT = {"byte": 1.0, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9, "Tbyte": 1e12, "ns": 1e-3, "us": 1.0, "ms": 1e3, "s": 1e6}
 COLS = [("time us", "gpu__time_duration.sum"), ("dram rd MB", "dram__bytes_read.sum"), ("dram wr MB", "dram__bytes_write.sum"),

@@ -56,3 +56,31 @@ def test_select_two_level_is_its_two_steps(N, topk, p_topk, dtype):
     scores = pq.cpu().float() @ pk.cpu().float().transpose(-1, -2)
     differ, bad = topk_mismatch_rows(idx.cpu(), want, scores, margin=1e-5)       # fp32 sums of 64 products of size < 16 in another order
     assert bad == 0
+
+
+# lists with repeats inside a row, every entry in one bucket, keys outside their range; one and several key ranges, 16 and 32 warps, T = 1
+@pytest.mark.parametrize("BH,M,T,n,kind", [(1, 16, 8, 16, "uniform"), (3, 130, 6, 129, "uniform"), (2, 3000, 8, 3000, "one"), (1, 5000, 16, 5000, "hot"),
+                                           (2, 300, 1, 1000, "uniform"), (60, 64, 8, 64, "hot"), (1, 16384, 8, 16384, "hot")])
+def test_transpose_ranges(BH, M, T, n, kind):
+    gen = torch.Generator().manual_seed(M + T)
+    idx = torch.randint(0, n, (1, BH, M, T), generator=gen, dtype=torch.int32)
+    if kind == "one":
+        idx[:] = n - 1
+    elif kind == "hot":
+        idx[..., : T // 2] = torch.randint(0, 5, (1, BH, M, T // 2), generator=gen, dtype=torch.int32)
+    off, flat = ops.transpose_indices(idx.to(DEV), n)
+    e = torch.arange(M * T).expand(BH, -1)
+    key, order = idx.reshape(BH, -1).long().sort(dim=1, stable=True)
+    assert torch.equal(flat.cpu()[0].long(), e.gather(1, order) // T)
+    assert torch.equal(off.cpu()[0, :, 1:].long(), torch.searchsorted(key, torch.arange(n).expand(BH, -1).contiguous(), right=True))
+    assert int(off[..., 0].abs().max()) == 0
+    # the pairs list, and what lies behind the last kept entry when keys are dropped
+    bad = idx.clone()
+    bad[:, :, M // 2] = n
+    off, flat, (pairs, ranges), _ = ops._transpose(bad.to(DEV), n, torch.int32, True)
+    kept = (M - 1) * T
+    assert (off.cpu()[0, :, -1] == kept).all()
+    assert torch.equal(pairs.cpu()[0, :, :kept] // T, flat.cpu()[0, :, :kept])
+    assert (pairs.cpu()[0, :, :kept].sort(-1).values.diff(dim=-1) > 0).all()
+    cut = ranges.cpu()[0, ..., 0]
+    assert int(cut.min()) >= 0 and int(cut.max()) <= kept and (cut.diff(dim=-1) >= 0).all()
