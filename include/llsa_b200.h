@@ -255,8 +255,8 @@ typedef struct LlsaAttnArgs {
                                   caller zeroes it, and reads it back after synchronising */
   const LlsaTensor* fwd_redo;  /* forward, optional: I32 scratch of at least B*H*N/4 elements (one byte per
                                   query row; not read before it is written).  With it, a pooled stage
-                                  that walks a long pooled key list (more than 192 pooled keys per row)
-                                  makes ONE pass over the keys with the fine part's log-sum-exp as the
+                                  that walks the pooled key list chunk by chunk (any number of pooled keys
+                                  per row but 64, 128 and 192) makes ONE pass over the keys with the fine part's log-sum-exp as the
                                   reference of its exponentials, marks here the rows whose pooled keys
                                   outweigh the fine ones by more than 1e30, and a second launch redoes
                                   exactly those rows with the exact two-pass form.  NULL: two passes for

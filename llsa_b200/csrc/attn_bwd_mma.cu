@@ -907,7 +907,7 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
   // pooled keys on tcgen05 (attn_pooled_bwd_tc.cu): the dQ kernel then covers the fine blocks only and the
   // tensor-core kernel adds the pooled part of dq and produces the pooled-key gradients
   const bool tc = pooled_bwd_tc_ok(a) && !g->no_tcgen05;
-  // long pooled key lists: the pooled part of dQ on the key-loop tcgen05 kernel (the pooled dK/dV stay on mma.sync)
+  // other pooled key lists: the key-loop tcgen05 kernels (dQ, then the key-major dK/dV)
   const bool loop_dq = !tc && pooled_dq_loop_tc_keys(a) > 0 && !g->no_tcgen05;
   if (mask & 1) {
     int rc = zero_pooled_acc(g, st);
@@ -937,20 +937,14 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
       int rc = launch_attn_dq_pooled_loop_tc(g, a, BH, st);
       if (rc) return rc;
     }
-    // the keys every query attends to (level 1 of one level, level 2 of two levels) on the key-major tcgen05 kernel; what is
-    // left for the mma.sync kernel is the gathered level-1 part of the two-level form
-    const int dense_level = loop_dq ? pooled_dkv_loop_tc_level(a) : 0;
-    AttnP<bf16> ap = a;
-    if (dense_level) {
+    if (loop_dq) {
       int rc = launch_attn_dkv_pooled_loop_tc(g, a, BH, st);
       if (rc) return rc;
-      if (dense_level == 1) ap.p1_blocks = 0; else ap.p2_blocks = 0;
-    }
-    if (ap.p1_blocks + ap.p2_blocks > 0) {
+    } else {
       constexpr int NWP = 8;
       const size_t smem = (size_t) 2 * kBS * kBS * kSmemPitch * sizeof(bf16) + 2 * kBS * kBS * sizeof(float);
       LLSA_SMEM_LIMIT((attn_dkv_pooled_kernel<NWP>), smem);
-      attn_dkv_pooled_kernel<NWP><<<dim3((unsigned) (a.nq1 / kBS), BH), NWP * 32, smem, st>>>(ap);
+      attn_dkv_pooled_kernel<NWP><<<dim3((unsigned) (a.nq1 / kBS), BH), NWP * 32, smem, st>>>(a);
       LLSA_LAUNCH_OK("attn_dkv_pooled_kernel");
     }
   }

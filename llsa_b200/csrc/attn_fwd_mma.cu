@@ -424,7 +424,8 @@ int launch_attn_fwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
   AttnP<bf16> a = build_attn_params<bf16>(g, false);
   constexpr int NW = 8;
   const int64_t BH = g->q->shape[0] * a.H;
-  const bool loop_tc = pooled_loop_tc_keys(a) > 0;
+  // all pooled keys of a row at once where they fit (64, 128, 192 keys), else chunk by chunk
+  const bool loop_tc = !pooled_tc_keys(a) && pooled_loop_tc_keys(a) > 0;
   if ((pooled_tc_keys(a) || loop_tc) && !g->no_tcgen05) {
     // fine blocks on mma.sync (o and lse of the fine part alone), pooled keys on tcgen05, merged there
     if (a.topk == 8) {

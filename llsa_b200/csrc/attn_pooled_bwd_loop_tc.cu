@@ -7,6 +7,8 @@
 //     dP = dO . V_c^T   [128 x 64]
 //     dS = exp2(S*scale*log2e + log2 w - lse) * (dP - delta) * scale      softmax warps, thread = query row
 //     dQ += dS . K_c    [128 x 64]  (K = 64 keys)             dS read from TENSOR MEMORY (packed bf16 over S), K_c MN-major
+// Two levels: first the gathered level-1 blocks (four to a chunk), then the level-2 keys.  Either list may end inside a chunk (at 32 keys):
+// what is loaded behind its end is neither exponentiated nor multiplied.
 // The final log-sum-exp is known in the backward, so one pass over the chunks suffices.  dQ accumulates in TMEM over
 // all chunks of the tile and is then added to the fine part already in dq.
 // TMEM columns: three buffers, chunk number n of the CTA (counted over all its tiles) uses buffer n mod 3: S at 128 b,
@@ -51,8 +53,8 @@ struct DqBars {
   uint64_t sdp_ready[kBufs], ds_ready[kBufs], buf_free[kBufs], dq_ready, dq_free;
 };
 
-// jobs: 64-key chunks per tile (even); gathered: number of leading chunks that are gathered level-1 blocks (0 or 2);
-// n_c: rows per head of the contiguous pooled tensor.
+// jobs: 64-key chunks per tile; gathered: number of leading chunks that are gathered level-1 blocks; n_c: rows per head of the
+// contiguous pooled tensor.
 __global__ void __launch_bounds__(kThreads, 1)
 attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps, int jobs, int gathered, int64_t n_c, int n_tiles,
                               int tiles_per_head) {
@@ -94,49 +96,46 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
   tc::fence_after_sync();
   const uint32_t tmem = s_tmem;
   const int n_my = (n_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x;
+  // keys of chunk j that belong to its list (a multiple of 32)
+  auto keys_of = [&](int j) {
+    const int left = j < gathered ? a.p1_blocks * kBS - j * kCk : (int) n_c - (j - gathered) * kCk;
+    return left < kCk ? left : kCk;
+  };
 
   if (warp == 8) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      int cj = 0;                                   // chunks loaded so far
-      for (int i = 0; i < n_my; ++i) {
-        const int tile = blockIdx.x + i * gridDim.x, qs = i & 1;
-        const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
-        if (!tc::bounded_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag)) break;
+    // lane 0 waits and issues; the blocks of a gathered chunk are issued by the lanes that hold their row (lane j: gathered block j)
+    int cj = 0;                                     // chunks loaded so far
+    for (int i = 0; i < n_my; ++i) {
+      const int tile = blockIdx.x + i * gridDim.x, qs = i & 1;
+      const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
+      int ok = 1, krow = 0;
+      if (lane == 0 && (ok = tc::bounded_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag))) {
         tma::expect_tx(&bars.q_full[qs], 2 * kTile * 2);
         tma::load_4d(sQ + qs * kTile, &maps.q, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
         tma::load_4d(sDO + qs * kTile, &maps.d_o, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
-        int krow[8];
-        if (gathered) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) krow[j] = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, j) * kBS);
-        }
-        bool ok = true;
-        for (int j = 0; ok && j < jobs; ++j, ++cj) {
-          const int st = cj % kStages;
-          const uint32_t par = ((cj / kStages) & 1) ^ 1;
-          const int crow = (int) ((int64_t) bh * n_c + (int64_t) (j - gathered) * kCk);
-          if (!(ok = tc::bounded_wait(&bars.k_empty[st], par, abort_flag))) break;
-          tma::expect_tx(&bars.k_full[st], kChunkElems * 2);
-          if (j < gathered) {
-#pragma unroll
-            for (int b4 = 0; b4 < 4; ++b4)
-              tma::load_2d(sK + st * kChunkElems + b4 * kBS * 64, &maps.kg, &bars.k_full[st], 0, j == 0 ? krow[b4] : krow[4 + b4]);
-          } else {
-            tma::load_2d(sK + st * kChunkElems, &maps.kc, &bars.k_full[st], 0, crow);
-          }
-          if (!(ok = tc::bounded_wait(&bars.v_empty[st], par, abort_flag))) break;
-          tma::expect_tx(&bars.v_full[st], kChunkElems * 2);
-          if (j < gathered) {
-#pragma unroll
-            for (int b4 = 0; b4 < 4; ++b4)
-              tma::load_2d(sV + st * kChunkElems + b4 * kBS * 64, &maps.vg, &bars.v_full[st], 0, j == 0 ? krow[b4] : krow[4 + b4]);
-          } else {
-            tma::load_2d(sV + st * kChunkElems, &maps.vc, &bars.v_full[st], 0, crow);
-          }
-        }
-        if (!ok) break;
       }
+      if (gathered) krow = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, min(lane, a.p1_blocks - 1)) * kBS);
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      for (int j = 0; ok && j < jobs; ++j, ++cj) {
+        const int st = cj % kStages;
+        const uint32_t par = ((cj / kStages) & 1) ^ 1;
+        const int crow = (int) ((int64_t) bh * n_c + (int64_t) (j - gathered) * kCk);
+        const bool mine = j < gathered && (lane >> 2) == j;
+        if (lane == 0 && (ok = tc::bounded_wait(&bars.k_empty[st], par, abort_flag))) {
+          tma::expect_tx(&bars.k_full[st], kChunkElems * 2);
+          if (j >= gathered) tma::load_2d(sK + st * kChunkElems, &maps.kc, &bars.k_full[st], 0, crow);
+        }
+        if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
+        if (mine) tma::load_2d(sK + st * kChunkElems + (lane & 3) * kBS * 64, &maps.kg, &bars.k_full[st], 0, krow);
+        if (lane == 0 && (ok = tc::bounded_wait(&bars.v_empty[st], par, abort_flag))) {
+          tma::expect_tx(&bars.v_full[st], kChunkElems * 2);
+          if (j >= gathered) tma::load_2d(sV + st * kChunkElems, &maps.vc, &bars.v_full[st], 0, crow);
+        }
+        if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
+        if (mine) tma::load_2d(sV + st * kChunkElems + (lane & 3) * kBS * 64, &maps.vg, &bars.v_full[st], 0, krow);
+      }
+      if (!ok) break;
     }
   } else if (warp == 9) {
     // ---------------------------------------------------------------- MMA issuer 1: S and dP
@@ -194,9 +193,12 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
           if (j == 0 && i > 0 && !(ok = tc::bounded_wait(&bars.dq_free, (i - 1) & 1, abort_flag))) break;     // previous tile's dQ has been read
           tc::fence_after_sync();
           const uint64_t kdesc = ((uint64_t) hi << 32) | (uint64_t) (lKm + st * kCStage);       // 16 key rows = 2048 bytes per k-step
-#pragma unroll
-          for (int s4 = 0; s4 < 4; ++s4)
-            tc::umma_ts(tmem + kColDQ, tmem + buf * 128 + s4 * 8, kdesc + 128 * s4, id_dq, (j > 0 || s4 > 0) ? 1u : 0u);
+          tc::umma_ts(tmem + kColDQ, tmem + buf * 128, kdesc, id_dq, j > 0 ? 1u : 0u);
+          tc::umma_ts(tmem + kColDQ, tmem + buf * 128 + 8, kdesc + 128, id_dq, 1u);
+          if (keys_of(j) == kCk) {
+            tc::umma_ts(tmem + kColDQ, tmem + buf * 128 + 16, kdesc + 256, id_dq, 1u);
+            tc::umma_ts(tmem + kColDQ, tmem + buf * 128 + 24, kdesc + 384, id_dq, 1u);
+          }
           tc::umma_commit(&bars.k_empty[st]);
           tc::umma_commit(&bars.buf_free[buf]);
           if (++st == kStages) st = 0;
@@ -226,14 +228,16 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
 #pragma unroll
       for (int q4 = 0; q4 < 4; ++q4) old[q4] = *reinterpret_cast<const uint4*>(dqrow + 8 * q4);
       bool ok = true;
-      for (int j = wg; j < jobs; j += 2) {
-        const float off = ((gathered ? (j < gathered) : !a.two_level) ? lw1 : lw2) - L;
+      for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
+        const float off = ((j < gathered || !a.two_level) ? lw1 : lw2) - L;
+        const int halves = keys_of(j) / 32;
         ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.sdp_ready[buf], bph, abort_flag));
         tc::fence_after_sync();
         if (!ok) break;
         const uint32_t t_b = t_lane + buf * 128;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
+          if (half == halves) break;
           tc::tmem_ld32_async(t_b + 32 * half, vs);
           tc::tmem_ld32_async(t_b + 64 + 32 * half, vd);
           tc::tmem_ld_wait(vs);
@@ -283,29 +287,25 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
 
 }  // namespace
 
-// Pooled keys per row if the key-loop dQ kernel applies (a multiple of 128 beyond what the single-shot backward takes).
-int pooled_dq_loop_tc_keys(const AttnP<bf16>& a) {
-  const int64_t np = (int64_t) (a.p1_blocks + a.p2_blocks) * kBS;
-  if (np <= 192 || np % 128 || a.Nq % kRows) return 0;
-  if (a.two_level && (a.p1_blocks != 8 || a.p2_blocks == 0)) return 0;
-  return (int) np;
-}
+// Pooled keys per row if the key-loop dQ kernel applies, else 0: the key-loop forward's range.
+int pooled_dq_loop_tc_keys(const AttnP<bf16>& a) { return pooled_loop_tc_keys(a); }
 
 int launch_attn_dq_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, int64_t BH, cudaStream_t st) {
-  const int np = pooled_dq_loop_tc_keys(a);
   DqMaps maps;
   memset(&maps, 0, sizeof(maps));
   int rc;
   if ((rc = tma::make_map_bhnd(&maps.q, g->q, kRows))) return rc;
   if ((rc = tma::make_map_bhnd(&maps.d_o, g->d_o, kRows))) return rc;
-  const int gathered = a.two_level ? 2 : 0;
-  const int64_t n_c = a.two_level ? a.n2 : a.n1;
+  const int64_t n_c = a.two_level ? (int64_t) a.p2_blocks * kBS : a.n1;
+  const int gathered = a.two_level ? (a.p1_blocks + 3) / 4 : 0, jobs = gathered + (int) ((n_c + kCk - 1) / kCk);
   if (gathered) {
     if ((rc = tma::make_map_rows(&maps.kg, a.pk, (uint64_t) BH * a.n1, kBS))) return rc;
     if ((rc = tma::make_map_rows(&maps.vg, a.pv, (uint64_t) BH * a.n1, kBS))) return rc;
   }
-  if ((rc = tma::make_map_rows(&maps.kc, a.two_level ? a.pk2 : a.pk, (uint64_t) BH * n_c, kCk))) return rc;
-  if ((rc = tma::make_map_rows(&maps.vc, a.two_level ? a.pv2 : a.pv, (uint64_t) BH * n_c, kCk))) return rc;
+  if (n_c) {
+    if ((rc = tma::make_map_rows(&maps.kc, a.two_level ? a.pk2 : a.pk, (uint64_t) BH * n_c, kCk))) return rc;
+    if ((rc = tma::make_map_rows(&maps.vc, a.two_level ? a.pv2 : a.pv, (uint64_t) BH * n_c, kCk))) return rc;
+  }
   const int tiles_per_head = (int) (a.Nq / kRows), n_tiles = (int) (BH * tiles_per_head);
   int dev = 0, sms = 148;
   LLSA_CUDA_OK(cudaGetDevice(&dev));
@@ -313,7 +313,7 @@ int launch_attn_dq_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, i
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) (4 * kTile + 2 * kStages * kChunkElems) * sizeof(bf16);
   LLSA_SMEM_LIMIT((attn_dq_pooled_loop_tc_kernel), smem);
-  attn_dq_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, np / kCk, gathered, n_c, n_tiles, tiles_per_head);
+  attn_dq_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, jobs, gathered, n_c, n_tiles, tiles_per_head);
   LLSA_LAUNCH_OK("attn_dq_pooled_loop_tc_kernel");
   return LLSA_OK;
 }

@@ -1,9 +1,11 @@
-// Pooled-key gradients on tcgen05 for the keys that EVERY query attends to: all level-1 pooled keys of the
-// one-level form (sparse_attention_res_1.py:362-400) and all level-2 keys of the two-level form
-// (_attn_bwd_res_dpkv2, sparse_attention_res_2.py:418-489) -- the key-major half of the pooled backward, with a
-// loop over the queries.
+// Pooled-key gradients on tcgen05, the key-major half of the pooled backward, with a loop over the queries.  Two forms:
+//   dense    the keys that EVERY query attends to: all level-1 pooled keys of the one-level form (sparse_attention_res_1.py:362-400),
+//            all level-2 keys of the two-level form (_attn_bwd_res_dpkv2, sparse_attention_res_2.py:418-489);
+//   gathered the level-1 keys of the two-level form: the children of the level-2 blocks a parent selected, met by the parent's 256
+//            query rows only (_attn_bwd_res_dpkv1_sparse, sparse_attention_res_2.py:491-575).
 //
-// A work unit is (head, chunk of 128 pooled keys) and a range of the head's query rows, walked 64 at a time (a job):
+// A work unit is (head, chunk of 128 pooled keys) -- gathered: (parent, eight of its blocks) -- and a range of the query rows that
+// meet it, walked 64 at a time (a job):
 //     S^T  = K_c . Q_t^T   [128 keys x 64 queries]  (K = 64 channels)   shared-memory operands
 //     dP^T = V_c . dO_t^T  [128 x 64]
 //     P^T  = exp2(S^T*scale*log2e + log2 w - lse[q]),  dS^T = P^T * (dP^T - delta[q]) * scale     thread = key row;
@@ -12,12 +14,13 @@
 //     dK_c += dS^T . Q_t                                   S^T / dP^T), dO_t / Q_t as MN-major operands (the same tiles)
 // dK_c, dV_c accumulate in TMEM over the unit's query range and are then written to the fp32 pooled-gradient
 // accumulators (scaled by kv_weight / token_weight, the reference's weighting of the pooled dK/dV side): plain stores if
-// the unit covers all queries of its head, reductions otherwise.
+// the unit covers all queries of its head, reductions otherwise.  Rows of a chunk behind the end of its list (which may end at any
+// multiple of 32 keys) hold a repeated block or the rows that follow in memory; their results stay in their own rows and are dropped.
 // Work split: all (head, chunk, job) triples in that order form one flat list that is cut into gridDim.x equal pieces,
 // one per CTA; a piece is one to a few units (it changes unit where it crosses a chunk boundary).
 // TMEM columns: three buffers, job number n of the CTA uses buffer n mod 3: S^T at 128 b, dP^T at 128 b + 64; dV at
 // [384,448), dK at [448,512).
-// Roles (one persistent CTA per SM, 11 warps): warp 8 lane 0 = TMA producer (K_c, V_c per unit; Q_t, dO_t, lse, delta per
+// Roles (one persistent CTA per SM, 11 warps): warp 8 lane 0 = TMA producer (K_c, V_c per unit in two stages; Q_t, dO_t, lse, delta per
 // job in a ring of 8), warp 9 lane 0 issues S^T and dP^T, warp 10 lane 0 issues dV and dK (one issuing thread, with its
 // waits, commits and fences, is slower than the tensor pipe), warps 0-3 / 4-7 = two softmax warpgroups on alternating
 // jobs; at the end of a unit group 0 writes dV, group 1 writes dK.  Every mbarrier wait is bounded (abort flag, TMEM freed).
@@ -44,11 +47,11 @@ constexpr uint32_t kColDV = 384, kColDK = 448;
 
 struct KvMaps {
   CUtensorMap q, d_o;         // [B,H,Nq,64] 4-D, box 64 rows
-  CUtensorMap k, v;           // contiguous pooled keys / values [BH*n, 64], box 128 rows
+  CUtensorMap k, v;           // contiguous pooled keys / values [BH*n, 64], box 128 rows (gathered: 16 rows)
 };
 
 struct KvBars {
-  uint64_t kv_full, kv_empty, q_full[kStages], q_empty[kStages], sdp_ready[kBufs], pds_ready[kBufs], buf_free[kBufs], acc_ready, acc_free;
+  uint64_t kv_full[2], kv_empty[2], q_full[kStages], q_empty[kStages], sdp_ready[kBufs], pds_ready[kBufs], buf_free[kBufs], acc_ready, acc_free;
 };
 
 // A CTA's piece of the flat job list, walked unit by unit.
@@ -71,19 +74,21 @@ struct Piece {
   }
 };
 
-// n_keys: pooled keys per head (a multiple of 128); jobs_all: 64-row query jobs per head; n_base: heads x key chunks.
+// n_keys: rows per head of the pooled tensor; jobs_all: 64-row query jobs per unit; n_base: units; chunks: chunks per head, gathered: per
+// parent.
+template <bool GATHER>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps maps, float* __restrict__ dpk, float* __restrict__ dpv,
-                               int64_t n_keys, int jobs_all, int n_base, float lw_log2, float out_mul) {
+                               int64_t n_keys, int jobs_all, int n_base, int chunks, float lw_log2, float out_mul) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ KvBars bars;
   __shared__ uint32_t s_tmem;
   __shared__ tc::WaitCtl s_ctl;
   __shared__ __align__(16) float s_lse[kStages][kQ], s_delta[kStages][kQ];
   bf16* base = reinterpret_cast<bf16*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-  bf16* sK = base;                           // [128][64]
-  bf16* sV = sK + kKeyTile;                  // [128][64]
-  bf16* sQ = sV + kKeyTile;                  // [kStages][64][64]
+  bf16* sK = base;                           // [2][128][64]
+  bf16* sV = sK + 2 * kKeyTile;              // [2][128][64]
+  bf16* sQ = sV + 2 * kKeyTile;              // [kStages][64][64]
   bf16* sDO = sQ + kStages * kQTile;         // [kStages][64][64]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile tc::WaitCtl* abort_flag = &s_ctl;
@@ -91,8 +96,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
   if (tid == 0) {
     s_ctl.abort = 0;
     s_ctl.limit = a.wait_limit > 0 ? a.wait_limit : tc::kWaitPolls;
-    tc::mbar_init(&bars.kv_full, 1);
-    tc::mbar_init(&bars.kv_empty, 1);
+    for (int i = 0; i < 2; ++i) { tc::mbar_init(&bars.kv_full[i], 1); tc::mbar_init(&bars.kv_empty[i], 1); }
     for (int i = 0; i < kStages; ++i) { tc::mbar_init(&bars.q_full[i], 1); tc::mbar_init(&bars.q_empty[i], 1); }
     for (int i = 0; i < kBufs; ++i) {
       tc::mbar_init(&bars.sdp_ready[i], 1);
@@ -108,31 +112,46 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = s_tmem;
-  const int chunks_per_head = (int) (n_keys / kKeys);
+  const int units_per_head = GATHER ? chunks * (int) a.nq2 : chunks;
   Piece pc((int64_t) n_base * jobs_all, jobs_all);
 
   if (warp == 8) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      int cj = 0;
-      bool ok = true;
-      for (int i = 0; ok && pc.next(); ++i) {
-        const int bh = pc.unit / chunks_per_head, c = pc.unit % chunks_per_head;
-        if (!tc::bounded_wait(&bars.kv_empty, (i & 1) ^ 1, abort_flag)) break;
-        tma::expect_tx(&bars.kv_full, 2 * kKeyTile * 2);
-        tma::load_2d(sK, &maps.k, &bars.kv_full, 0, (int) ((int64_t) bh * n_keys + (int64_t) c * kKeys));
-        tma::load_2d(sV, &maps.v, &bars.kv_full, 0, (int) ((int64_t) bh * n_keys + (int64_t) c * kKeys));
-        for (int j = 0; j < pc.n; ++j, ++cj) {
+    // lane 0 waits and issues; gathered: lane j < 8 fetches and issues block j of the unit's keys
+    int cj = 0, ok = 1;
+    for (int i = 0; ok && pc.next(); ++i) {
+      const int bh = pc.unit / units_per_head, u = pc.unit - bh * units_per_head, ks = i & 1;
+      const int c = GATHER ? u % chunks : u, q0 = GATHER ? u / chunks * (kBS * kBS) : 0;      // chunk; first query row of the parent
+      int krow = 0;
+      if (GATHER) krow = (int) ((int64_t) bh * n_keys + p1_block(a, bh, q0 / kBS, min(c * 8 + (lane & 7), a.p1_blocks - 1)) * kBS);
+      if (lane == 0 && (ok = tc::bounded_wait(&bars.kv_empty[ks], ((i >> 1) & 1) ^ 1, abort_flag))) {
+        tma::expect_tx(&bars.kv_full[ks], 2 * kKeyTile * 2);
+        if (!GATHER) {
+          const int krow0 = (int) ((int64_t) bh * n_keys + (int64_t) c * kKeys);
+          tma::load_2d(sK + ks * kKeyTile, &maps.k, &bars.kv_full[ks], 0, krow0);
+          tma::load_2d(sV + ks * kKeyTile, &maps.v, &bars.kv_full[ks], 0, krow0);
+        }
+      }
+      if (GATHER) {
+        if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
+        if (lane < 8) {
+          tma::load_2d(sK + ks * kKeyTile + lane * kBS * 64, &maps.k, &bars.kv_full[ks], 0, krow);
+          tma::load_2d(sV + ks * kKeyTile + lane * kBS * 64, &maps.v, &bars.kv_full[ks], 0, krow);
+        }
+      }
+      if (lane == 0) {
+        for (int j = 0; ok && j < pc.n; ++j, ++cj) {
           const int st = cj & (kStages - 1);
           if (!(ok = tc::bounded_wait(&bars.q_empty[st], ((cj / kStages) & 1) ^ 1, abort_flag))) break;
           tma::expect_tx(&bars.q_full[st], 2 * kQTile * 2 + 2 * kQ * 4);
-          const int qrow = (pc.job0 + j) * kQ;
+          const int qrow = q0 + (pc.job0 + j) * kQ;
           tma::load_4d(sQ + st * kQTile, &maps.q, &bars.q_full[st], 0, qrow, bh % a.H, bh / a.H);
           tma::load_4d(sDO + st * kQTile, &maps.d_o, &bars.q_full[st], 0, qrow, bh % a.H, bh / a.H);
           tma::load_bulk(s_lse[st], a.lse + (int64_t) bh * a.Nq + qrow, kQ * 4, &bars.q_full[st]);
           tma::load_bulk(s_delta[st], a.delta + (int64_t) bh * a.Nq + qrow, kQ * 4, &bars.q_full[st]);
         }
       }
+      ok = __shfl_sync(0xffffffffu, ok, 0);
     }
   } else if (warp == 9) {
     // ---------------------------------------------------------------- MMA issuer 1: S^T and dP^T of every job
@@ -140,13 +159,15 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       const uint32_t id_s = tc::instr_desc(kKeys, kQ, 0, 0);
       const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
       auto lo = [](const void* p, uint32_t lbo_bytes) { return ((tc::smem_u32(p) >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16); };
-      constexpr uint32_t kQStage = (uint32_t) (kQTile * 2) >> 4;
+      constexpr uint32_t kQStage = (uint32_t) (kQTile * 2) >> 4, kKeyStage = (uint32_t) (kKeyTile * 2) >> 4;
       const uint32_t lK = lo(sK, 16), lV = lo(sV, 16), lQ = lo(sQ, 16), lDO = lo(sDO, 16);
       int cj = 0, buf = 0;                          // jobs issued so far by this CTA; buffer of the next one
       uint32_t bph = 0;                             // phase parity of that buffer's barriers
       bool ok = true;
       for (int i = 0; ok && pc.next(); ++i) {
-        if (!(ok = tc::bounded_wait(&bars.kv_full, i & 1, abort_flag))) break;
+        const int ks = i & 1;
+        if (!(ok = tc::bounded_wait(&bars.kv_full[ks], (i >> 1) & 1, abort_flag))) break;
+        const uint32_t k_ = lK + ks * kKeyStage, v_ = lV + ks * kKeyStage;
         for (int j = 0; j < pc.n; ++j, ++cj) {
           const int st = cj & (kStages - 1);
           // the buffer's previous job (three back): the dV / dK instructions that read its P^T / dS^T have completed
@@ -154,18 +175,18 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
           if (!(ok = tc::bounded_wait(&bars.q_full[st], (cj / kStages) & 1, abort_flag))) break;
           tc::fence_after_sync();
           const uint32_t d = tmem + buf * 128, q_ = lQ + st * kQStage, o_ = lDO + st * kQStage;
-          tc::umma_ss_lh<0>(d, lK, hi, q_, hi, id_s);
-          tc::umma_ss_lh<0>(d + 64, lV, hi, o_, hi, id_s);
+          tc::umma_ss_lh<0>(d, k_, hi, q_, hi, id_s);
+          tc::umma_ss_lh<0>(d + 64, v_, hi, o_, hi, id_s);
 #pragma unroll
           for (int s4 = 1; s4 < 4; ++s4) {
-            tc::umma_ss_lh<1>(d, lK + 2 * s4, hi, q_ + 2 * s4, hi, id_s);
-            tc::umma_ss_lh<1>(d + 64, lV + 2 * s4, hi, o_ + 2 * s4, hi, id_s);
+            tc::umma_ss_lh<1>(d, k_ + 2 * s4, hi, q_ + 2 * s4, hi, id_s);
+            tc::umma_ss_lh<1>(d + 64, v_ + 2 * s4, hi, o_ + 2 * s4, hi, id_s);
           }
           tc::umma_commit(&bars.sdp_ready[buf]);
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
         }
         if (!ok) break;
-        tc::umma_commit(&bars.kv_empty);             // the key chunk is only read by these products
+        tc::umma_commit(&bars.kv_empty[ks]);         // the key chunk is only read by these products
       }
     }
   } else if (warp == 10) {
@@ -214,7 +235,17 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
     float vs[32], vd[32];
     bool ok = true;
     for (int i = 0; ok && pc.next(); ++i) {
-      const int bh = pc.unit / chunks_per_head, c = pc.unit % chunks_per_head;
+      const int bh = pc.unit / units_per_head, u = pc.unit - bh * units_per_head, c = GATHER ? u % chunks : u;
+      // this thread's key: its row in the pooled tensor (gathered: fetched now, used at the end of the unit), or none
+      bool live = true;
+      int64_t key = (int64_t) c * kKeys + r;
+      if (GATHER) {
+        const int blk = c * 8 + (r >> 4);
+        live = blk < a.p1_blocks;
+        key = p1_block(a, bh, u / chunks * kBS, live ? blk : 0) * kBS + (r & 15);
+      } else {
+        live = key < n_keys;
+      }
       for (; jn < jc + pc.n; jn += 2) {
         const int st = jn & (kStages - 1);
         ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.sdp_ready[buf], bph, abort_flag));
@@ -256,13 +287,14 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.acc_ready, (uint32_t) (i & 1), abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
-      float* dst = (wg == 0 ? dpv : dpk) + ((int64_t) bh * n_keys + (int64_t) c * kKeys + r) * kD;
-      const bool whole = pc.n == jobs_all;           // the unit saw every query of its head: nobody else adds to these rows
+      float* dst = (wg == 0 ? dpv : dpk) + ((int64_t) bh * n_keys + key) * kD;
+      const bool whole = !GATHER && pc.n == jobs_all;           // the unit saw every query of its head: nobody else adds to these rows
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         tc::tmem_ld32_async(t_acc + 32 * half, vs);
         tc::tmem_ld_wait(vs);
-        if (whole) {
+        if (!live) {
+        } else if (whole) {
 #pragma unroll
           for (int q4 = 0; q4 < 8; ++q4)
             *reinterpret_cast<float4*>(dst + 32 * half + 4 * q4) = make_float4(vs[4 * q4] * out_mul, vs[4 * q4 + 1] * out_mul, vs[4 * q4 + 2] * out_mul, vs[4 * q4 + 3] * out_mul);
@@ -286,41 +318,40 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
 
 }  // namespace
 
-// The pooled keys that every query attends to -- all level-1 keys of the one-level form, all level-2 keys of the two-level
-// form: the key-major tcgen05 kernel applies when their count is a multiple of 128 and the query rows come in pairs of
-// 64-row jobs.  Returns the pooling level it would handle (1 or 2), else 0.
-int pooled_dkv_loop_tc_level(const AttnP<bf16>& a) {
-  if (a.Nq % (2 * kQ)) return 0;
-  if (!a.two_level) return (a.p1_blocks > 0 && a.n1 % kKeys == 0) ? 1 : 0;
-  return (a.p2_blocks > 0 && a.n2 % kKeys == 0) ? 2 : 0;
-}
-
+// Launches the dense form (level 1 of one level, level 2 of two levels) and, with two levels, the gathered form: all pooled dK/dV of a
+// problem the key-loop dQ kernel takes.
 int launch_attn_dkv_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, int64_t BH, cudaStream_t st) {
-  const int level = pooled_dkv_loop_tc_level(a);
   KvMaps maps;
   memset(&maps, 0, sizeof(maps));
   int rc;
   if ((rc = tma::make_map_bhnd(&maps.q, g->q, kQ))) return rc;
   if ((rc = tma::make_map_bhnd(&maps.d_o, g->d_o, kQ))) return rc;
-  const int64_t n_keys = level == 1 ? a.n1 : a.n2;
-  if ((rc = tma::make_map_rows(&maps.k, level == 1 ? a.pk : a.pk2, (uint64_t) BH * n_keys, kKeys))) return rc;
-  if ((rc = tma::make_map_rows(&maps.v, level == 1 ? a.pv : a.pv2, (uint64_t) BH * n_keys, kKeys))) return rc;
   int dev = 0, sms = 148;
   LLSA_CUDA_OK(cudaGetDevice(&dev));
   LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // one CTA per SM, each with an equal piece of the flat (head, chunk, job) list
-  const int jobs_all = (int) (a.Nq / kQ), n_base = (int) (BH * (n_keys / kKeys));
-  const int64_t total = (int64_t) n_base * jobs_all;
-  const int grid = total < sms ? (int) total : sms;
-  const size_t smem = 1024 + (size_t) (2 * kKeyTile + 2 * kStages * kQTile) * sizeof(bf16);
-  LLSA_SMEM_LIMIT((attn_dkv_pooled_loop_tc_kernel), smem);
-  if (level == 1)
-    attn_dkv_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, a.dpk, a.dpv, n_keys, jobs_all, n_base, log2f(a.w1),
-                                                                 a.kvw1 / a.w1);
-  else
-    attn_dkv_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, a.dpk2, a.dpv2, n_keys, jobs_all, n_base, log2f(a.w2),
-                                                                 a.kvw2 / a.w2);
-  LLSA_LAUNCH_OK("attn_dkv_pooled_loop_tc_kernel");
+  const size_t smem = 1024 + (size_t) (4 * kKeyTile + 2 * kStages * kQTile) * sizeof(bf16);
+  // one CTA per SM, each with an equal piece of the flat (unit, job) list
+  auto grid_of = [&](int64_t total) { return total < sms ? (int) total : sms; };
+  const int64_t n_dense = a.two_level ? (int64_t) a.p2_blocks * kBS : a.n1;
+  if (n_dense) {
+    if ((rc = tma::make_map_rows(&maps.k, a.two_level ? a.pk2 : a.pk, (uint64_t) BH * n_dense, kKeys))) return rc;
+    if ((rc = tma::make_map_rows(&maps.v, a.two_level ? a.pv2 : a.pv, (uint64_t) BH * n_dense, kKeys))) return rc;
+    const int chunks = (int) ((n_dense + kKeys - 1) / kKeys), jobs = (int) (a.Nq / kQ), units = (int) BH * chunks;
+    const float w = a.two_level ? a.w2 : a.w1, kvw = a.two_level ? a.kvw2 : a.kvw1;
+    LLSA_SMEM_LIMIT((attn_dkv_pooled_loop_tc_kernel<false>), smem);
+    attn_dkv_pooled_loop_tc_kernel<false><<<grid_of((int64_t) units * jobs), kThreads, smem, st>>>(
+        a, maps, a.two_level ? a.dpk2 : a.dpk, a.two_level ? a.dpv2 : a.dpv, n_dense, jobs, units, chunks, log2f(w), kvw / w);
+    LLSA_LAUNCH_OK("attn_dkv_pooled_loop_tc_kernel");
+  }
+  if (a.two_level) {
+    if ((rc = tma::make_map_rows(&maps.k, a.pk, (uint64_t) BH * a.n1, kBS))) return rc;
+    if ((rc = tma::make_map_rows(&maps.v, a.pv, (uint64_t) BH * a.n1, kBS))) return rc;
+    const int chunks = (a.p1_blocks + 7) / 8, jobs = kBS * kBS / kQ, units = (int) (BH * a.nq2) * chunks;
+    LLSA_SMEM_LIMIT((attn_dkv_pooled_loop_tc_kernel<true>), smem);
+    attn_dkv_pooled_loop_tc_kernel<true><<<grid_of((int64_t) units * jobs), kThreads, smem, st>>>(a, maps, a.dpk, a.dpv, a.n1, jobs, units, chunks,
+                                                                                                 log2f(a.w1), a.kvw1 / a.w1);
+    LLSA_LAUNCH_OK("attn_dkv_pooled_loop_tc_kernel<gathered>");
+  }
   return LLSA_OK;
 }
 

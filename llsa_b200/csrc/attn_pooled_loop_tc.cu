@@ -3,8 +3,10 @@
 // attn_pooled_tc.cu keeps all pooled keys of a tile in tensor memory at once and therefore stops at 192 keys.
 // Here a tile of 128 query rows walks its pooled keys chunk by chunk:
 //   one level  (sparse_attention_res_1.py:85-106): ALL N/16 level-1 pooled keys, weight token_weight;
-//   two levels (sparse_attention_res_2.py:94-149): chunk 0 = the 128 level-1 children of the parent's selected
-//              level-2 blocks (gathered, weight token_weight), then ALL N/256 level-2 keys (weight token_weight_2).
+//   two levels (sparse_attention_res_2.py:94-149): first the level-1 children of the parent's selected level-2 blocks (gathered,
+//              eight blocks to a chunk, weight token_weight), then ALL N/256 level-2 keys (weight token_weight_2).
+// Both lists may end inside a chunk (at a multiple of 32 keys): what lies behind the end is loaded (a repeated block, or the rows
+// that follow in memory) and neither exponentiated nor multiplied: the softmax warps and the P.V steps stop at the list's end.
 // Two passes over the chunks make the softmax exact without rescaling an accumulator that lives in TMEM:
 //   pass 1: S = Q.K_c^T per chunk, row maxima only;
 //   pass 2: S again, P = exp2(S*scale*log2e + log2 w - max) written back into TMEM over S (packed bf16) and used as
@@ -60,8 +62,8 @@ struct LoopBars {
   uint64_t s_ready[kBufs], wg_done[kBufs], buf_free[kBufs], o_ready, o_free, xchg;
 };
 
-// n_chunks: chunks per tile; gathered: chunk 0 is the gathered level-1 set (two levels); n_c: rows per head of the
-// contiguous pooled tensor.
+// n_chunks: chunks per tile; gathered: how many of them, the first ones, are gathered level-1 blocks (two levels); n_c: rows per
+// head of the contiguous pooled tensor.
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps maps, int n_chunks, int gathered, int64_t n_c, int n_tiles,
                                int tiles_per_head, int n_pass, unsigned char* redo) {
@@ -112,51 +114,50 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   // jobs per tile; job j of tile i has the CTA-wide number i * jobs + j, which picks the S buffer (mod 3) and the softmax
   // group (mod 2; with one pass and an odd chunk count the parity of a tile's first job alternates)
   const int jobs = n_pass * n_chunks, first_p2 = jobs - n_chunks;
+  // keys of chunk c that belong to its list (a multiple of 32)
+  auto keys_of = [&](int c) {
+    const int left = c < gathered ? a.p1_blocks * kBS - c * kChunk : (int) n_c - (c - gathered) * kChunk;
+    return left < kChunk ? left : kChunk;
+  };
 
   if (warp == 8) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      int kjob = 0, vjob = 0;
-      for (int i = 0; i < n_my; ++i) {
-        const int tile = blockIdx.x + i * gridDim.x, qs = i & 1;
-        const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
-        if (!tc::bounded_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag)) break;
+    // lane 0 waits and issues; the blocks of a gathered chunk are issued by the lanes that hold their row (lane j: gathered block j)
+    int kjob = 0, vjob = 0;
+    for (int i = 0; i < n_my; ++i) {
+      const int tile = blockIdx.x + i * gridDim.x, qs = i & 1;
+      const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
+      int ok = 1, krow = 0;
+      if (lane == 0 && (ok = tc::bounded_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag))) {
         tma::expect_tx(&bars.q_full[qs], kTile * 2);
         tma::load_4d(sQ + qs * kTile, &maps.q, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
-        int krow[8];
-        if (gathered) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) krow[j] = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, j) * kBS);
-        }
-        bool ok = true;
-        for (int j = 0; ok && j < jobs; ++j) {
-          const int c = j % n_chunks, pass = j >= first_p2;
-          const int crow = (int) ((int64_t) bh * n_c + (int64_t) (c - gathered) * kChunk);      // contiguous chunk
-          const int ks = kjob % kKStages;
-          if (!(ok = tc::bounded_wait(&bars.k_empty[ks], ((kjob / kKStages) & 1) ^ 1, abort_flag))) break;
-          tma::expect_tx(&bars.k_full[ks], kTile * 2);
-          if (gathered && c == 0) {
-#pragma unroll
-            for (int b8 = 0; b8 < 8; ++b8) tma::load_2d(sK + ks * kTile + b8 * kBS * 64, &maps.kg, &bars.k_full[ks], 0, krow[b8]);
-          } else {
-            tma::load_2d(sK + ks * kTile, &maps.kc, &bars.k_full[ks], 0, crow);
-          }
-          ++kjob;
-          if (pass == 1) {
-            const int vs = vjob % kVStages;
-            if (!(ok = tc::bounded_wait(&bars.v_empty[vs], ((vjob / kVStages) & 1) ^ 1, abort_flag))) break;
-            tma::expect_tx(&bars.v_full[vs], kTile * 2);
-            if (gathered && c == 0) {
-#pragma unroll
-              for (int b8 = 0; b8 < 8; ++b8) tma::load_2d(sV + vs * kTile + b8 * kBS * 64, &maps.vg, &bars.v_full[vs], 0, krow[b8]);
-            } else {
-              tma::load_2d(sV + vs * kTile, &maps.vc, &bars.v_full[vs], 0, crow);
-            }
-            ++vjob;
-          }
-        }
-        if (!ok) break;
       }
+      if (gathered) krow = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, min(lane, a.p1_blocks - 1)) * kBS);
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      for (int j = 0; ok && j < jobs; ++j) {
+        const int c = j % n_chunks, pass = j >= first_p2;
+        const int crow = (int) ((int64_t) bh * n_c + (int64_t) (c - gathered) * kChunk);      // contiguous chunk
+        const bool mine = (lane >> 3) == c;                                                   // a lane of this gathered chunk
+        const int ks = kjob % kKStages;
+        if (lane == 0 && (ok = tc::bounded_wait(&bars.k_empty[ks], ((kjob / kKStages) & 1) ^ 1, abort_flag))) {
+          tma::expect_tx(&bars.k_full[ks], kTile * 2);
+          if (c >= gathered) tma::load_2d(sK + ks * kTile, &maps.kc, &bars.k_full[ks], 0, crow);
+        }
+        if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
+        if (c < gathered && mine) tma::load_2d(sK + ks * kTile + (lane & 7) * kBS * 64, &maps.kg, &bars.k_full[ks], 0, krow);
+        ++kjob;
+        if (pass == 1) {
+          const int vs = vjob % kVStages;
+          if (lane == 0 && (ok = tc::bounded_wait(&bars.v_empty[vs], ((vjob / kVStages) & 1) ^ 1, abort_flag))) {
+            tma::expect_tx(&bars.v_full[vs], kTile * 2);
+            if (c >= gathered) tma::load_2d(sV + vs * kTile, &maps.vc, &bars.v_full[vs], 0, crow);
+          }
+          if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
+          if (c < gathered && mine) tma::load_2d(sV + vs * kTile + (lane & 7) * kBS * 64, &maps.vg, &bars.v_full[vs], 0, krow);
+          ++vjob;
+        }
+      }
+      if (!ok) break;
     }
   } else if (warp == 9) {
     // ---------------------------------------------------------------- MMA issuer 1: S of every job
@@ -210,9 +211,16 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
             if (c == 0 && i > 0 && !(ok = tc::bounded_wait(&bars.o_free, (i - 1) & 1, abort_flag))) break;      // previous tile's O has been read
             tc::fence_after_sync();
             const uint64_t vdesc = ((uint64_t) hi << 32) | (uint64_t) (lV + vs * kStage);
+            // P: 16 keys = 8 packed columns per k-step; V: 16 key rows = 2048 bytes
+            const int ksteps = keys_of(c) / 16;
+            if (ksteps == 8) {
 #pragma unroll
-            for (int s8 = 0; s8 < 8; ++s8)       // P: 16 keys = 8 packed columns per k-step; V: 16 key rows = 2048 bytes
-              tc::umma_ts(tmem + kColO, tmem + buf * kChunk + s8 * 8, vdesc + 128 * s8, id_o, (c > 0 || s8 > 0) ? 1u : 0u);
+              for (int s8 = 0; s8 < 8; ++s8)
+                tc::umma_ts(tmem + kColO, tmem + buf * kChunk + s8 * 8, vdesc + 128 * s8, id_o, (c > 0 || s8 > 0) ? 1u : 0u);
+            } else {
+              for (int s8 = 0; s8 < ksteps; ++s8)
+                tc::umma_ts(tmem + kColO, tmem + buf * kChunk + s8 * 8, vdesc + 128 * s8, id_o, (c > 0 || s8 > 0) ? 1u : 0u);
+            }
             tc::umma_commit(&bars.v_empty[vs]);
             if (++vs == kVStages) { vs = 0; vph ^= 1; }
           }
@@ -256,24 +264,27 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       const float lse_f = a.lse[(int64_t) bh * a.Nq + row];
       // one pass: the fine part's log-sum-exp is the reference of the exponentials
       float mx = n_pass == 1 ? lse_f * kLog2eF : -INFINITY, lsum = 0.f;
-      bool ok = true;
+      bool ok = true, exchanged = n_pass == 1;
+      // two passes: the groups exchange their row maxima once per tile, before their first pass-2 job (a group may have none)
+      auto exchange_max = [&]() -> bool {
+        float other;
+        exchanged = true;
+        if (!exchange(mx, other)) return false;
+        mx = fmaxf(mx, other);
+        return true;
+      };
       for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
         const int c = j % n_chunks, pass = j >= first_p2;
-        const float lw = (gathered ? (c == 0) : !a.two_level) ? lw1 : lw2;
-        if (n_pass == 2 && pass == 1 && j - 2 < first_p2) {
-          // first pass-2 job of this group: exchange the row maxima of the two groups
-          float other;
-          if (!(ok = exchange(mx, other))) break;
-          mx = fmaxf(mx, other);
-        }
+        const float lw = (c < gathered || !a.two_level) ? lw1 : lw2;
+        const int nq = keys_of(c) / 32;
+        if (pass == 1 && !exchanged && !(ok = exchange_max())) break;
         ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.s_ready[buf], bph, abort_flag));
         tc::fence_after_sync();
         if (!ok) break;
         const uint32_t t_s = t_lane + buf * kChunk;
         if (pass == 0) {
           float m = -INFINITY;
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
+          for (int q4 = 0; q4 < nq; ++q4) {
             tc::tmem_ld32_async(t_s + 32 * q4, va);
             tc::tmem_ld_wait(va);
 #pragma unroll
@@ -283,7 +294,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         } else {
           const float off = lw - mx;
 #pragma unroll 1          // unrolled, the four quarters' registers overlap and 18 of them spill (to L2: L1 is 28 KB here)
-          for (int q4 = 0; q4 < 4; ++q4) {
+          for (int q4 = 0; q4 < nq; ++q4) {
             tc::tmem_ld32_async(t_s + 32 * q4, va);
             tc::tmem_ld_wait(va);
             uint32_t pk[16];
@@ -303,6 +314,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         buf += 2;
         if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
       }
+      if (ok && !exchanged) ok = exchange_max();
       float lse_out = __int_as_float(0x7fc00000);               // NaN unless everything completed
       if (ok) {
         float other;
@@ -362,30 +374,31 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
 
 }  // namespace
 
-// Pooled keys per row if the key-loop kernel applies (a multiple of 128, more than the 192 the single-shot kernel
-// holds), else 0.
+// Pooled keys per row if the key-loop kernel applies, else 0.  Up to 32 gathered blocks (one per lane of the producer warp); both lists
+// end at multiples of 32 keys (an even top-k; N/16 or N/256 a multiple of 32 where that list is attended to).
 int pooled_loop_tc_keys(const AttnP<bf16>& a) {
   const int64_t np = (int64_t) (a.p1_blocks + a.p2_blocks) * kBS;
-  if (np <= 192 || np % kChunk || a.Nq % kRows) return 0;
-  if (a.two_level && a.p1_blocks != 8) return 0;         // the gathered chunk is exactly 8 blocks
-  if (a.two_level && a.p2_blocks == 0) return 0;
+  if (np == 0 || a.Nq % kRows || (a.p1_blocks * kBS) % 32 || (a.p2_blocks * kBS) % 32) return 0;
+  if (a.two_level && a.p1_blocks > 32) return 0;
   return (int) np;
 }
 
 int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, int64_t BH, cudaStream_t st) {
-  const int np = pooled_loop_tc_keys(a);
   LoopMaps maps;
   memset(&maps, 0, sizeof(maps));
   int rc;
   if ((rc = tma::make_map_bhnd(&maps.q, g->q, kRows))) return rc;
-  const int gathered = a.two_level ? 1 : 0;
-  const int64_t n_c = a.two_level ? a.n2 : a.n1;
+  // chunks of the gathered list (two levels), then of the list every row attends to
+  const int64_t n_c = a.two_level ? (int64_t) a.p2_blocks * kBS : a.n1;
+  const int gathered = a.two_level ? (a.p1_blocks + 7) / 8 : 0, n_chunks = gathered + (int) ((n_c + kChunk - 1) / kChunk);
   if (gathered) {
     if ((rc = tma::make_map_rows(&maps.kg, a.pk, (uint64_t) BH * a.n1, kBS))) return rc;
     if ((rc = tma::make_map_rows(&maps.vg, a.pv, (uint64_t) BH * a.n1, kBS))) return rc;
   }
-  if ((rc = tma::make_map_rows(&maps.kc, a.two_level ? a.pk2 : a.pk, (uint64_t) BH * n_c, kChunk))) return rc;
-  if ((rc = tma::make_map_rows(&maps.vc, a.two_level ? a.pv2 : a.pv, (uint64_t) BH * n_c, kChunk))) return rc;
+  if (n_c) {
+    if ((rc = tma::make_map_rows(&maps.kc, a.two_level ? a.pk2 : a.pk, (uint64_t) BH * n_c, kChunk))) return rc;
+    if ((rc = tma::make_map_rows(&maps.vc, a.two_level ? a.pv2 : a.pv, (uint64_t) BH * n_c, kChunk))) return rc;
+  }
   const int tiles_per_head = (int) (a.Nq / kRows), n_tiles = (int) (BH * tiles_per_head);
   int dev = 0, sms = 148;
   LLSA_CUDA_OK(cudaGetDevice(&dev));
@@ -395,10 +408,10 @@ int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
   LLSA_SMEM_LIMIT((attn_fwd_pooled_loop_tc_kernel), smem);
   unsigned char* redo = g->fwd_redo ? reinterpret_cast<unsigned char*>(g->fwd_redo->ptr) : nullptr;
   if (redo) {        // one pass with the fine part's log-sum-exp as reference, then the two-pass form for the rows it marked
-    attn_fwd_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, np / kChunk, gathered, n_c, n_tiles, tiles_per_head, 1, redo);
+    attn_fwd_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, 1, redo);
     LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");
   }
-  attn_fwd_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, np / kChunk, gathered, n_c, n_tiles, tiles_per_head, 2, redo);
+  attn_fwd_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, 2, redo);
   LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");
   return LLSA_OK;
 }

@@ -304,11 +304,11 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
   status.check("attn_bwd");
 }
 
-// Marks of the one-pass form of the long pooled lists (include/llsa_b200.h: fwd_redo): one byte per query row, wanted where a row
-// attends to more pooled keys than the single-shot kernel holds (192).
+// Marks of the one-pass form of the pooled lists that are walked chunk by chunk (include/llsa_b200.h: fwd_redo): one byte per query
+// row, wanted where a row's pooled keys are not the 64, 128 or 192 the single-shot kernel holds.
 int64_t redo_elems(const Dims& d, bool bf16, bool two, int64_t topk_p) {
-  const int64_t pooled = two ? topk_p * d.bs + (d.n2 >= 64 ? d.n2 : 0) : d.n1;
-  return bf16 && !flag(kTwoPass) && pooled > 192 ? (d.B * d.H * d.Nq + 3) / 4 : 0;
+  const int64_t pooled = two ? topk_p * d.bs + (d.n2 >= 64 ? d.n2 : 0) : (d.n1 >= 64 ? d.n1 : 0);
+  return bf16 && !flag(kTwoPass) && (pooled > 192 || pooled % 64) ? (d.B * d.H * d.Nq + 3) / 4 : 0;
 }
 void keep_redo(const Tensor& t) {
   std::lock_guard<std::mutex> lock(g_redo_mutex);

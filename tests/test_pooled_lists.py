@@ -1,0 +1,54 @@
+"""The key-loop tcgen05 kernels (forward, pooled dQ, pooled dK/dV) over pooled lists that end inside a chunk, against the oracle."""
+import pytest
+import torch
+
+import llsa_b200
+from llsa_b200 import ops, synth
+from oracle import llsa_oracle as O
+from test_gpu_parity import _oracle_l2_check, assert_bf16_close
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+# gathered keys alone (fewer than 64 level-2 keys): a quarter, half, three quarters of a chunk, one, two, four chunks; level-2 tails of 32, 96 and
+# 64 + 32 keys behind them
+@pytest.mark.parametrize("B,H,N,topk,topk2", [(2, 3, 5376, 8, 8), (1, 2, 4096, 8, 2), (1, 2, 4096, 8, 4), (1, 1, 4096, 8, 6), (1, 2, 5120, 16, 16),
+                                              (1, 1, 8192, 8, 32), (1, 2, 24576, 8, 8), (1, 1, 24576, 4, 4), (1, 1, 40960, 16, 16)])
+def test_two_level_lists_vs_oracle(B, H, N, topk, topk2):
+    q, k, v, do = synth.gaussian_qkv(N + topk2, B, H, N, 64, dtype=torch.bfloat16)
+    _oracle_l2_check(llsa_b200, q, k, v, do, topk1=topk, topk2=topk2, label="N=%d top-%d/%d" % (N, topk, topk2))
+
+
+@pytest.mark.parametrize("one_pass", [True, False])
+@pytest.mark.parametrize("B,H,N", [(2, 3, 1536), (1, 2, 2560), (1, 2, 5632), (3, 1, 8704)])      # 96, 160, 352, 544 pooled keys
+def test_one_level_lists_vs_oracle(B, H, N, one_pass, monkeypatch):
+    monkeypatch.setattr(ops, "_one_pass_pooled", one_pass)
+    q, k, v, do = synth.gaussian_qkv(N, B, H, N, 64, dtype=torch.bfloat16)
+    qg, kg, vg = [t.to(DEV).requires_grad_(True) for t in (q, k, v)]
+    dbg = llsa_b200.llsa_l1_debug(qg, kg, vg, 8, 16)
+    idx, pk, pv = dbg["indices"].cpu(), dbg["pk"].cpu(), dbg["pv"].cpu()
+    o_ref, lse_ref = O.attn_fwd_l1(q, k, v, pk, pv, idx, faithful=False)
+    assert_bf16_close(dbg["o"].detach(), o_ref, "o")
+    assert float((dbg["lse"].cpu() - lse_ref).abs().max()) < 2e-2
+    dbg["o"].backward(do.to(DEV))
+    dq, dk, dv, dpk, dpv = O.attn_bwd_l1(do, q, k, v, pk, pv, o_ref.float(), lse_ref, idx, faithful=False)
+    assert_bf16_close(qg.grad, dq, "dq")
+    assert_bf16_close(kg.grad, dk + O.mean_pool1d_bwd(dpk, 16), "dk")
+    assert_bf16_close(vg.grad, dv + O.mean_pool1d_bwd(dpv, 16), "dv")
+
+
+def test_tail_keys_of_the_next_head_do_not_leak():
+    """A chunk's rows behind the end of a head's list belong to the next head: NaN and infinities there must stay there."""
+    q, k, v, do = [t.to(DEV) for t in synth.gaussian_qkv(5, 1, 2, 2560, 64, dtype=torch.bfloat16)]
+    want = [t.detach().clone().requires_grad_(True) for t in (q[:, :1], k[:, :1], v[:, :1])]
+    o_want = llsa_b200.llsa_l1(*want, 8, 16)
+    o_want.backward(do[:, :1])
+    k2, v2 = k.clone(), v.clone()
+    k2[:, 1], v2[:, 1] = float("inf"), float("nan")
+    got = [t.detach().clone().requires_grad_(True) for t in (q, k2, v2)]
+    o = llsa_b200.llsa_l1(*got, 8, 16)
+    o.backward(do)
+    assert torch.equal(o[:, :1], o_want) and torch.equal(got[0].grad[:, :1], want[0].grad)
+    for i in (1, 2):      # fp32 reductions: the order of the sums may differ
+        assert float((got[i].grad[:, :1].float() - want[i].grad.float()).norm() / want[i].grad.float().norm()) < 1e-3
