@@ -24,7 +24,7 @@
 //                          dV += P^T.dO, dK += dS^T.Q with P, dS read back; tiles of
 //                          buckets that straddle a range meet in shared memory / a
 //                          global partial tensor (no atomics), and
-//   attn_dkv_finish_ld_kernel sums the window partials; every store folds in the pooling
+//   attn_dkv_finish_kernel sums the window partials; every store folds in the pooling
 //                          backward (dk += (dpk[j] + dpk2[j/16]/16)/16), one bf16 store.
 // The reference multiplies k by scale into new tensors first (res_1.py:420-422);
 // here scale rides in the exp2 argument and in the epilogues.
@@ -443,19 +443,6 @@ __device__ __forceinline__ void tile_add_mem(const float* s, float (&dk)[8][4], 
     dv[u][0] += y.x; dv[u][1] += y.y; dv[u][2] += y.z; dv[u][3] += y.w;
   }
 }
-// The same from global memory with all 16 loads in flight before the first add: for the finish kernel, whose warps do
-// little else than wait for these loads.
-__device__ __forceinline__ void tile_add_mem_batched(const float* s, float (&dk)[8][4], float (&dv)[8][4], int lane) {
-  const float4* s4 = reinterpret_cast<const float4*>(s) + lane;
-  float4 x[8], y[8];
-#pragma unroll
-  for (int u = 0; u < 8; ++u) { x[u] = __ldcg(s4 + u * 32); y[u] = __ldcg(s4 + (8 + u) * 32); }
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    dk[u][0] += x[u].x; dk[u][1] += x[u].y; dk[u][2] += x[u].z; dk[u][3] += x[u].w;
-    dv[u][0] += y[u].x; dv[u][1] += y[u].y; dv[u][2] += y[u].z; dv[u][3] += y[u].w;
-  }
-}
 __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) {
 #pragma unroll
   for (int u = 0; u < 8; ++u) dk[u][0] = dk[u][1] = dk[u][2] = dk[u][3] = dv[u][0] = dv[u][1] = dv[u][2] = dv[u][3] = 0.f;
@@ -475,7 +462,7 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 //     bucket, so a warp starts without a search.  A longer bucket is cut at multiples of kRangeEntries: a warp parks
 //     the tile of a bucket it shares with EARLIER warps in its shared-memory slot; the tile it shares with later warps
 //     stays in its accumulators until the CTA has synchronised and is then completed from their slots; pieces of
-//     buckets that straddle windows go to the `partial` scratch and attn_dkv_finish_ld_kernel adds them in window order.
+//     buckets that straddle windows go to the `partial` scratch and attn_dkv_finish_kernel adds them in window order.
 //   * The pooled-gradient rows a finished tile folds in (the pooling backward) are requested into registers when
 //     the bucket begins and parked in shared memory right before the store.
 // Accumulator layout (ldmatrix): tile u holds channels 8u + 2t, 8u + 2t + 1 of keys g (c0, c1) and g + 8 (c2, c3).
@@ -485,45 +472,7 @@ constexpr int kRingFineStageBytes = 2 * kRingTileElems * (int) sizeof(bf16);    
 constexpr int kRingFoldBytes = 4 * 64 * (int) sizeof(float);                           // per warp: dpk, dpv, dpk2, dpv2 rows of the bucket
 
 // Pooling-backward fold and scale for the ldmatrix accumulator layout: afterwards dk / dv hold the final fp32 values.
-// The four gradient rows of KV block j (64 fp32 each) arrive with two 128-bit loads per lane -- lanes 0..15 the 16 quads
-// of the key rows, lanes 16..31 of the value rows, level 1 and level 2 -- so that a warp can have the next block's rows
-// under way (8 registers) while it finishes this one.
-struct FoldRows { float4 e, f; };
-__device__ __forceinline__ FoldRows dkv_fold_rows_load(const AttnP<bf16>& a, int64_t bh, int64_t j, int lane) {
-  FoldRows r;
-  r.e = r.f = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (a.fold) {
-    const int half = lane >> 4, q = lane & 15;
-    r.e = __ldcg(reinterpret_cast<const float4*>((half ? a.dpv : a.dpk) + (bh * a.n1 + j) * kD + 4 * q));
-    if (a.two_level) r.f = __ldcg(reinterpret_cast<const float4*>((half ? a.dpv2 : a.dpk2) + (bh * a.n2 + j / kBS) * kD + 4 * q));
-  }
-  return r;
-}
-__device__ __forceinline__ void dkv_fine_fold_apply(const AttnP<bf16>& a, const FoldRows& r, float (&dk)[8][4], float (&dv)[8][4], int lane) {
-  if (a.fold) {
-    const int t = lane & 3;
-    float4 e = r.e;
-    if (a.two_level) { e.x += r.f.x * (1.f / kBS); e.y += r.f.y * (1.f / kBS); e.z += r.f.z * (1.f / kBS); e.w += r.f.w * (1.f / kBS); }
-    const bool hi = (t & 1) != 0;                 // channels 8u + 2t, 8u + 2t + 1: quad 2u + t/2, its first or second pair
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int src = 2 * u + (t >> 1);
-      const float kx0 = __shfl_sync(0xffffffffu, e.x, src), ky0 = __shfl_sync(0xffffffffu, e.y, src);
-      const float kx1 = __shfl_sync(0xffffffffu, e.z, src), ky1 = __shfl_sync(0xffffffffu, e.w, src);
-      const float vx0 = __shfl_sync(0xffffffffu, e.x, 16 + src), vy0 = __shfl_sync(0xffffffffu, e.y, 16 + src);
-      const float vx1 = __shfl_sync(0xffffffffu, e.z, 16 + src), vy1 = __shfl_sync(0xffffffffu, e.w, 16 + src);
-      const float2 ek = make_float2(hi ? kx1 : kx0, hi ? ky1 : ky0), ev = make_float2(hi ? vx1 : vx0, hi ? vy1 : vy0);
-      dk[u][0] = dk[u][0] * a.scale + ek.x * (1.f / kBS); dk[u][1] = dk[u][1] * a.scale + ek.y * (1.f / kBS);
-      dk[u][2] = dk[u][2] * a.scale + ek.x * (1.f / kBS); dk[u][3] = dk[u][3] * a.scale + ek.y * (1.f / kBS);
-      dv[u][0] += ev.x * (1.f / kBS); dv[u][1] += ev.y * (1.f / kBS); dv[u][2] += ev.x * (1.f / kBS); dv[u][3] += ev.y * (1.f / kBS);
-    }
-  } else {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) { dk[u][0] *= a.scale; dk[u][1] *= a.scale; dk[u][2] *= a.scale; dk[u][3] *= a.scale; }
-  }
-}
-
-// The same from this warp's copy of the four gradient rows in shared memory ([dpk | dpv | dpk2 | dpv2] x 64 fp32, fetched with
+// The four gradient rows of KV block j come from this warp's copy in shared memory ([dpk | dpv | dpk2 | dpv2] x 64 fp32, fetched with
 // cp.async when the bucket began); sa_fold already includes the lane's 8t bytes.
 __device__ __forceinline__ void dkv_fine_fold_smem(const AttnP<bf16>& a, uint32_t sa_fold, float (&dk)[8][4], float (&dv)[8][4]) {
   if (a.fold) {
@@ -831,66 +780,110 @@ __global__ void __launch_bounds__(kRingWarps * 32, 2) attn_dkv_fine_ring_kernel(
   }
 }
 
-constexpr int kFinishPerWarp = 8;
-// One warp per eight KV blocks: blocks nobody selected get their pooling-backward term alone, blocks whose bucket was cut
-// across windows of the main kernel get the sum of their pieces, in window order.
-__global__ void __launch_bounds__(128) attn_dkv_finish_ld_kernel(AttnP<bf16> a, const float* __restrict__ partial, int n_windows) {
-  __shared__ __align__(1024) unsigned char s_stage[4][2 * kRingTileElems * sizeof(bf16)];      // per warp: a dK and a dV tile on their way out
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
-  const int64_t j0 = ((int64_t) blockIdx.x * 4 + warp) * kFinishPerWarp, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
-  if (j0 >= a.n1) return;
-  // a warp looks at eight consecutive buckets at once (lane i: offsets of bucket j0 + i) and works only on those that need it:
-  // most buckets were finished by one warp of the main kernel
-  const int64_t jl = j0 + lane < a.n1 ? j0 + lane : a.n1 - 1;
-  // offsets are clamped to [0, E] and to each other: a malformed CSR cannot send the range arithmetic below outside `partial`
-  const int64_t E = a.nq1 * a.topk;
-  const int my_bo = lane < kFinishPerWarp ? (int) min(E, max((int64_t) 0, csr_off(a, bh, jl))) : 0;
-  const int my_be = lane < kFinishPerWarp ? (int) min(E, max((int64_t) my_bo, csr_off(a, bh, jl + 1))) : 1;
-  const int range = a.range_entries, window = kRingWarps * range;       // nominal entries per warp / per CTA of the main kernel
-  const bool need = lane < kFinishPerWarp && j0 + lane < a.n1 && (my_be == my_bo || (my_be - my_bo > range && my_bo / window != (my_be - 1) / window));
-  unsigned todo = __ballot_sync(0xffffffffu, need);
-  if (!todo) return;
-  const uint32_t st_sa = (uint32_t) __cvta_generic_to_shared(s_stage[warp]);
-  const uint32_t sa_cp0 = st_sa + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4), sa_cp1 = sa_cp0 ^ 64;
-  uint32_t sa_m[4];
-  {
-    const uint32_t base = st_sa + ((lane & 7) + ((lane >> 3) & 1) * 8) * 128 + (((lane >> 4) ^ (lane & 7)) << 4);
+// KV blocks nobody selected: their dk / dv are the pooling-backward term alone, one row sixteen times.  A warp looks at four blocks, one per
+// lane, and writes the empty ones two at a time: lane (tensor, row parity, 16-byte chunk) has both blocks' gradient rows in flight.
+constexpr int kPlainPerWarp = 4;
+__device__ __forceinline__ void dkv_store_unselected(const AttnP<bf16>& a, int64_t b, int64_t h, int64_t bh, int first, int lane) {
+  const int n1 = (int) a.n1, jl = min(first + lane, n1 - 1);
+  unsigned todo = __ballot_sync(0xffffffffu, lane < kPlainPerWarp && first + lane < n1 && csr_off(a, bh, jl + 1) <= csr_off(a, bh, jl));
+  const int ten = lane >> 4, rr = (lane >> 3) & 1, c = (lane & 7) * 8;
+  const View<bf16> out = ten ? a.dv : a.dk;
+  const float *g1 = ten ? a.dpv : a.dpk, *g2 = ten ? a.dpv2 : a.dpk2;
+  while (todo) {
+    float4 e[2][2], f[2][2];
+    int j[2];
+    unsigned m = todo;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) sa_m[c] = base ^ (c << 5);
-  }
-  // pieces of the split buckets: towards L2 now (two of a piece's 64 lines per lane), they are read a few microseconds later
-  for (unsigned m = todo; m; m &= m - 1) {
-    const int l = __ffs((int) m) - 1;
-    const int bo = __shfl_sync(0xffffffffu, my_bo, l), be = __shfl_sync(0xffffffffu, my_be, l);
-    if (be > bo) {
-      const int c_first = bo / window, c_last = min((be - 1) / window, n_windows - 1);
-      for (int c = c_first; c <= c_last; ++c) {
-        const char* pf = reinterpret_cast<const char*>(partial + ((bh * n_windows + c) * 2 + (c == c_first ? 1 : 0)) * (int64_t) kTileFloats);
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(pf + 128 * lane));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(pf + 128 * (32 + lane)));
+    for (int u = 0; u < 2; ++u) {
+      j[u] = m ? first + __ffs((int) m) - 1 : -1;
+      m &= m - 1;
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        e[u][v] = f[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j[u] >= 0 && a.fold) {
+          e[u][v] = __ldcg(reinterpret_cast<const float4*>(g1 + (bh * a.n1 + j[u]) * kD + c + 4 * v));
+          if (a.two_level) f[u][v] = __ldcg(reinterpret_cast<const float4*>(g2 + (bh * a.n2 + j[u] / kBS) * kD + c + 4 * v));
+        }
       }
     }
-  }
-  // the gradient rows of the next bucket are requested before this one is finished
-  FoldRows rows = dkv_fold_rows_load(a, bh, j0 + __ffs((int) todo) - 1, lane);
-  while (todo) {
-    const int l = __ffs((int) todo) - 1;
-    todo &= todo - 1;
-    const FoldRows mine = rows;
-    if (todo) rows = dkv_fold_rows_load(a, bh, j0 + __ffs((int) todo) - 1, lane);
-    const int bo = __shfl_sync(0xffffffffu, my_bo, l), be = __shfl_sync(0xffffffffu, my_be, l);
-    const int64_t j = j0 + l;
-    float dk[8][4], dv[8][4];
-    tile_zero(dk, dv);
-    if (be > bo) {
-      // a bucket of more than `range` entries is cut at multiples of `range` only, so its pieces by windows lie
-      // between multiples of `window`: the first is the tail of the window that holds entry bo, every later one a head
-      const int c_first = bo / window, c_last = min((be - 1) / window, n_windows - 1);
-      for (int c = c_first; c <= c_last; ++c)
-        tile_add_mem_batched(partial + ((bh * n_windows + c) * 2 + (c == c_first ? 1 : 0)) * (int64_t) kTileFloats, dk, dv, lane);
+    todo = m;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (j[u] < 0) break;
+      uint32_t w[4];
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const float4 x = e[u][v], y = f[u][v];
+        const float s = 1.f / kBS;
+        w[2 * v] = pack_bf16((x.x + y.x * s) * s, (x.y + y.y * s) * s);
+        w[2 * v + 1] = pack_bf16((x.z + y.z * s) * s, (x.w + y.w * s) * s);
+      }
+      bf16* p = out.row(b, h, (int64_t) j[u] * kBS + rr) + c;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(p + 2 * i * out.sn) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    dkv_fine_fold_apply(a, mine, dk, dv, lane);
-    dkv_tile_store_staged<0>(a, b, h, j, dk, dv, sa_m, sa_cp0, sa_cp1, lane);
+  }
+}
+
+// Buckets whose pieces lie in several windows of the kernel above.  Each of them crosses a window boundary, and a boundary lies in one
+// bucket: one CTA per boundary looks up that bucket (the transpose kernel left it beside the range that starts there), leaves unless
+// this is the first boundary the bucket crosses, and adds the pieces in window order: the tail of the window the bucket begins in, then
+// the heads.  A warp owns 32 channels of one tensor, so a piece is four 128-bit loads per lane, four pieces in flight.
+// blockIdx.x >= n_windows - 1: the unselected blocks, 16 per CTA -- stores at the memory's rate next to the latency of the lookups (as extra
+// CTAs or extra work of the kernel above they cost twice as much: two CTAs of it fill an SM).
+// One warp for eight buckets, looking for both kinds, took 46 us at 48 slices of 16384 tokens and 160 us at 6 of 262144; this kernel FIN_A
+// and FIN_B.
+__global__ void __launch_bounds__(128) attn_dkv_finish_kernel(AttnP<bf16> a, const float* __restrict__ partial, int n_windows) {
+  if ((int) blockIdx.x >= n_windows - 1) {
+    const int first = (((int) blockIdx.x - (n_windows - 1)) * 4 + (int) (threadIdx.x >> 5)) * kPlainPerWarp;
+    dkv_store_unselected(a, blockIdx.y / a.H, blockIdx.y % a.H, blockIdx.y, first, threadIdx.x & 31);
+    return;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n1 = (int) a.n1;
+  const int64_t bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
+  const int E = (int) (a.nq1 * a.topk), range = a.range_entries, window = kRingWarps * range;       // nominal entries per warp / per CTA of the main kernel
+  const int R = (E + range - 1) / range, edge = ((int) blockIdx.x + 1) * window;
+  // offsets are clamped to [0, E] and to each other: a malformed CSR cannot send the arithmetic below outside `partial`
+  const int j = min(max(__ldcg(&a.ranges[bh * R + edge / range].y), 0), n1 - 1);
+  const int bo = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, j))), be = (int) min((int64_t) E, max((int64_t) bo, csr_off(a, bh, j + 1)));
+  if (be - bo <= range || bo >= edge || be <= edge || bo / window != (int) blockIdx.x) return;
+  const int c_first = bo / window, c_last = min((be - 1) / window, n_windows - 1);
+  const int ten = warp >> 1, u0 = (warp & 1) * 4;                      // tiles u0 .. u0 + 3 of dk / dv: tile u holds channels 8u + 2t, +1 of rows g, g + 8
+  float acc[4][4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.f;
+  for (int c0 = c_first; c0 <= c_last; c0 += 4) {
+    float4 x[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = min(c0 + i, c_last);
+      const float4* p = reinterpret_cast<const float4*>(partial + ((bh * n_windows + c) * 2 + (c == c_first ? 1 : 0)) * (int64_t) kTileFloats) + (8 * ten + u0) * 32 + lane;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[i][u] = __ldcg(p + u * 32);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (c0 + i > c_last) break;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { acc[u][0] += x[i][u].x; acc[u][1] += x[i][u].y; acc[u][2] += x[i][u].z; acc[u][3] += x[i][u].w; }
+    }
+  }
+  const float *g1 = (ten ? a.dpv : a.dpk) + (bh * a.n1 + j) * kD, *g2 = a.two_level ? (ten ? a.dpv2 : a.dpk2) + (bh * a.n2 + j / kBS) * kD : nullptr;
+  const View<bf16> out = ten ? a.dv : a.dk;
+  const float mul = ten ? 1.f : a.scale;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int c = 8 * (u0 + u) + 2 * t;
+    float2 e = make_float2(0.f, 0.f);
+    if (a.fold) {
+      e = __ldcg(reinterpret_cast<const float2*>(g1 + c));
+      if (a.two_level) {
+        const float2 f = __ldcg(reinterpret_cast<const float2*>(g2 + c));
+        e.x += f.x * (1.f / kBS); e.y += f.y * (1.f / kBS);
+      }
+    }
+    *reinterpret_cast<uint32_t*>(out.row(b, h, (int64_t) j * kBS + g) + c) = pack_bf16(acc[u][0] * mul + e.x * (1.f / kBS), acc[u][1] * mul + e.y * (1.f / kBS));
+    *reinterpret_cast<uint32_t*>(out.row(b, h, (int64_t) j * kBS + g + 8) + c) = pack_bf16(acc[u][2] * mul + e.x * (1.f / kBS), acc[u][3] * mul + e.y * (1.f / kBS));
   }
 }
 
@@ -956,8 +949,9 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel), smem);
     attn_dkv_fine_ring_kernel<<<dim3((unsigned) n_windows, BH), kRingWarps * 32, smem, st>>>(a, partial);
     LLSA_LAUNCH_OK("attn_dkv_fine_ring_kernel");
-    attn_dkv_finish_ld_kernel<<<dim3((unsigned) ((a.n1 + 4 * kFinishPerWarp - 1) / (4 * kFinishPerWarp)), BH), 128, 0, st>>>(a, partial, n_windows);
-    LLSA_LAUNCH_OK("attn_dkv_finish_ld_kernel");
+    const int n_plain = (int) ((a.n1 + 4 * kPlainPerWarp - 1) / (4 * kPlainPerWarp));
+    attn_dkv_finish_kernel<<<dim3((unsigned) (n_windows - 1 + n_plain), BH), 128, 0, st>>>(a, partial, n_windows);
+    LLSA_LAUNCH_OK("attn_dkv_finish_kernel");
   }
   return LLSA_OK;
 }
