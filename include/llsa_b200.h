@@ -227,7 +227,8 @@ typedef struct LlsaAttnArgs {
                                   one-level backward uses 1 here (sparse_attention_res_1.py:389) */
   int32_t force_generic;       /* 1: use the plain FFMA kernels for any dtype   */
   int32_t stage_mask;          /* backward only; 0 = everything.  Otherwise a bit set of
-                                  1: zero the *_acc tensors + delta + dq,  2: pooled-key
+                                  1: zero the *_acc tensors (not with 8: the caller has cleared
+                                  them, on another stream for instance) + delta + dq,  2: pooled-key
                                   gradients (and the pooled part of dq where the tcgen05
                                   kernels apply),  4: dk, dv -- to be issued in this order
                                   (lets a caller time the kernels separately, or build the CSR

@@ -237,6 +237,8 @@ constexpr int kDqStages = 3;
 
 template <int NW>
 __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   bf16* ring = reinterpret_cast<bf16*>(smem_raw) + warp * (kDqStages * 2 * kRingTileElems);
@@ -549,6 +551,8 @@ __device__ __forceinline__ void dkv_fine_store_staged(const AttnP<bf16>& a, int6
   dkv_tile_store_staged<SB>(a, b, h, j, dk, dv, sa_m, sa_cp0, sa_cp1, lane);
 }
 __global__ void __launch_bounds__(kRingWarps * 32, 2) attn_dkv_fine_ring_kernel(AttnP<bf16> a, float* __restrict__ partial) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // the swizzle arithmetic below works on absolute shared addresses: start at a 128-byte boundary (the launch adds 128 bytes)
   unsigned char* smem = smem_raw + ((128u - ((uint32_t) __cvta_generic_to_shared(smem_raw) & 127u)) & 127u);
@@ -903,8 +907,10 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
   // other pooled key lists: the key-loop tcgen05 kernels (dQ, then the key-major dK/dV)
   const bool loop_dq = !tc && pooled_dq_loop_tc_keys(a) > 0 && !g->no_tcgen05;
   if (mask & 1) {
-    int rc = zero_pooled_acc(g, st);
-    if (rc) return rc;
+    if (!(g->stage_mask & 8)) {
+      int rc = zero_pooled_acc(g, st);
+      if (rc) return rc;
+    }
     constexpr int NWQ = 4;
     AttnP<bf16> aq = a;
     if (tc || loop_dq) aq.p1_blocks = aq.p2_blocks = 0;
@@ -914,7 +920,7 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     if (n_all == 0) {
       const size_t ring = (size_t) NWQ * kDqStages * 2 * kRingTileElems * sizeof(bf16);
       LLSA_SMEM_LIMIT((attn_dq_fine_kernel<NWQ>), ring);
-      attn_dq_fine_kernel<NWQ><<<dim3((unsigned) (a.nq1 / NWQ), BH), NWQ * 32, ring, st>>>(aq);
+      launch_pdl(attn_dq_fine_kernel<NWQ>, dim3((unsigned) (a.nq1 / NWQ), BH), NWQ * 32, ring, st, aq);
       LLSA_LAUNCH_OK("attn_dq_fine_kernel");
     } else {
       LLSA_SMEM_LIMIT((attn_dq_mma_kernel<NWQ>), smem);
@@ -947,7 +953,7 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     float* partial = (float*) g->dkv_partial->ptr;
     const size_t smem = (size_t) kRingWarps * (kTileFloats * sizeof(float) + kRingFineStages * kRingFineStageBytes + kRingFoldBytes) + 128;   // per warp: slot, ring, gradient rows
     LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel), smem);
-    attn_dkv_fine_ring_kernel<<<dim3((unsigned) n_windows, BH), kRingWarps * 32, smem, st>>>(a, partial);
+    launch_pdl(attn_dkv_fine_ring_kernel, dim3((unsigned) n_windows, BH), kRingWarps * 32, smem, st, a, partial);
     LLSA_LAUNCH_OK("attn_dkv_fine_ring_kernel");
     const int n_plain = (int) ((a.n1 + 4 * kPlainPerWarp - 1) / (4 * kPlainPerWarp));
     attn_dkv_finish_kernel<<<dim3((unsigned) (n_windows - 1 + n_plain), BH), 128, 0, st>>>(a, partial, n_windows);

@@ -181,6 +181,8 @@ constexpr int kFineStages = 3;
 
 template <int NW>
 __global__ void __launch_bounds__(NW * 32, 2) attn_fwd_fine_kernel(AttnP<bf16> a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   bf16* ring = reinterpret_cast<bf16*>(smem_raw) + warp * (kFineStages * 2 * kRingTileElems);
@@ -279,6 +281,8 @@ __device__ __forceinline__ void static_for(F&& f) {
 
 template <int NW>
 __global__ void __launch_bounds__(NW * 32, 2) attn_fwd_fine8_kernel(AttnP<bf16> a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // the swizzle arithmetic works on absolute shared addresses: start at a 128-byte boundary (the launch adds 128 bytes)
   const uint32_t smem_sa = ((uint32_t) __cvta_generic_to_shared(smem_raw) + 127u) & ~127u;
@@ -431,12 +435,12 @@ int launch_attn_fwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     if (a.topk == 8) {
       const size_t ring = (size_t) NW * kF8Stages * kF8TileBytes + 128;
       LLSA_SMEM_LIMIT((attn_fwd_fine8_kernel<NW>), ring);
-      attn_fwd_fine8_kernel<NW><<<dim3((unsigned) (a.nq1 / NW), (unsigned) BH), NW * 32, ring, st>>>(a);
+      launch_pdl(attn_fwd_fine8_kernel<NW>, dim3((unsigned) (a.nq1 / NW), (unsigned) BH), NW * 32, ring, st, a);
       LLSA_LAUNCH_OK("attn_fwd_fine8_kernel");
     } else {
       const size_t ring = (size_t) NW * kFineStages * 2 * kRingTileElems * sizeof(bf16);
       LLSA_SMEM_LIMIT((attn_fwd_fine_kernel<NW>), ring);
-      attn_fwd_fine_kernel<NW><<<dim3((unsigned) (a.nq1 / NW), (unsigned) BH), NW * 32, ring, st>>>(a);
+      launch_pdl(attn_fwd_fine_kernel<NW>, dim3((unsigned) (a.nq1 / NW), (unsigned) BH), NW * 32, ring, st, a);
       LLSA_LAUNCH_OK("attn_fwd_fine_kernel");
     }
     return loop_tc ? launch_attn_fwd_pooled_loop_tc(g, a, BH, st) : launch_attn_fwd_pooled_tc(g, a, BH, st);

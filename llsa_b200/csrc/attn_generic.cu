@@ -136,6 +136,8 @@ constexpr size_t kGenericSmem = (size_t) (2 + 2 * kGw) * kTileF * sizeof(float);
 
 template <typename T>
 __global__ void __launch_bounds__(kGw * 32) attn_fwd_generic(AttnP<T> a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   __shared__ float s_m[kGw][kBS], s_l[kGw][kBS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ra = lane >> 2, rb = lane & 3;
@@ -202,6 +204,8 @@ __global__ void __launch_bounds__(kGw * 32) attn_fwd_generic(AttnP<T> a) {
 
 template <typename T>
 __global__ void __launch_bounds__(kGw * 32) attn_dq_generic(AttnP<T> a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   __shared__ float s_delta[kBS], s_lse[kBS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ra = lane >> 2, rb = lane & 3;
@@ -269,6 +273,8 @@ __global__ void __launch_bounds__(kGw * 32) attn_dq_generic(AttnP<T> a) {
 // Lane rows are KEYS here (scores are S^T), the columns query rows.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kGw * 32) attn_dkv_generic(AttnP<T> a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ra = lane >> 2, rb = lane & 3;
   const int64_t bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
@@ -383,7 +389,7 @@ static int fwd_generic_t(const LlsaAttnArgs* g, cudaStream_t st) {
   AttnP<T> a = build_attn_params<T>(g, false);
   dim3 grid((unsigned) a.nq1, (unsigned) (g->q->shape[0] * a.H));
   LLSA_SMEM_LIMIT((attn_fwd_generic<T>), kGenericSmem);
-  attn_fwd_generic<T><<<grid, kGw * 32, kGenericSmem, st>>>(a);
+  launch_pdl(attn_fwd_generic<T>, grid, kGw * 32, kGenericSmem, st, a);
   LLSA_LAUNCH_OK("attn_fwd_generic");
   return LLSA_OK;
 }
@@ -411,21 +417,23 @@ static int bwd_generic_t(const LlsaAttnArgs* g, cudaStream_t st) {
   const unsigned BH = (unsigned) (g->q->shape[0] * a.H);
   const int mask = g->stage_mask ? g->stage_mask : 7;
   if (mask & 1) {
-    int rc = zero_pooled_acc(g, st);
-    if (rc) return rc;
+    if (!(g->stage_mask & 8)) {
+      int rc = zero_pooled_acc(g, st);
+      if (rc) return rc;
+    }
     LLSA_SMEM_LIMIT((attn_dq_generic<T>), kGenericSmem);
-    attn_dq_generic<T><<<dim3((unsigned) a.nq1, BH), kGw * 32, kGenericSmem, st>>>(a);
+    launch_pdl(attn_dq_generic<T>, dim3((unsigned) a.nq1, BH), kGw * 32, kGenericSmem, st, a);
     LLSA_LAUNCH_OK("attn_dq_generic");
   }
   const int ptiles = a.p1_blocks + a.p2_blocks;
   if ((mask & 2) && ptiles > 0) {
     LLSA_SMEM_LIMIT((attn_dkv_generic<T, 1>), kGenericSmem);
-    attn_dkv_generic<T, 1><<<dim3((unsigned) ptiles, BH, (unsigned) (a.nq1 / kBS)), kGw * 32, kGenericSmem, st>>>(a);
+    launch_pdl(attn_dkv_generic<T, 1>, dim3((unsigned) ptiles, BH, (unsigned) (a.nq1 / kBS)), kGw * 32, kGenericSmem, st, a);
     LLSA_LAUNCH_OK("attn_dkv_generic<pooled>");
   }
   if (mask & 4) {
     LLSA_SMEM_LIMIT((attn_dkv_generic<T, 0>), kGenericSmem);
-    attn_dkv_generic<T, 0><<<dim3((unsigned) a.n1, BH), kGw * 32, kGenericSmem, st>>>(a);
+    launch_pdl(attn_dkv_generic<T, 0>, dim3((unsigned) a.n1, BH), kGw * 32, kGenericSmem, st, a);
     LLSA_LAUNCH_OK("attn_dkv_generic<fine>");
   }
   return LLSA_OK;

@@ -90,10 +90,12 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
     tc::mbar_init(&bars.dq_free, 8);
     tc::fence_mbar_init();
   }
+  pdl_wait();
   if (warp == 0) tc::tmem_alloc(&s_tmem, 512);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  pdl_trigger();
   const uint32_t tmem = s_tmem;
   const int n_my = (n_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x;
   // keys of chunk j that belong to its list (a multiple of 32)
@@ -313,7 +315,7 @@ int launch_attn_dq_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, i
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) (4 * kTile + 2 * kStages * kChunkElems) * sizeof(bf16);
   LLSA_SMEM_LIMIT((attn_dq_pooled_loop_tc_kernel), smem);
-  attn_dq_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, jobs, gathered, n_c, n_tiles, tiles_per_head);
+  launch_pdl(attn_dq_pooled_loop_tc_kernel, grid, kThreads, smem, st, a, maps, jobs, gathered, n_c, n_tiles, tiles_per_head);
   LLSA_LAUNCH_OK("attn_dq_pooled_loop_tc_kernel");
   return LLSA_OK;
 }

@@ -103,10 +103,12 @@ attn_bwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ BwdMaps maps, i
     tc::mbar_init(&bars.acc_free, 4);
     tc::fence_mbar_init();
   }
+  pdl_wait();
   if (warp == 0) tc::tmem_alloc(&s_tmem, 512);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  pdl_trigger();
   const uint32_t tmem = s_tmem;
   // contiguous tile range of this CTA
   const int t_begin = (int) ((int64_t) n_tiles * blockIdx.x / gridDim.x), t_end = (int) ((int64_t) n_tiles * (blockIdx.x + 1) / gridDim.x);
@@ -440,7 +442,7 @@ int launch_attn_bwd_pooled_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, int64
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) 14 * kTile * sizeof(bf16);     // Q, dO x 2, K1 x 2, V1, K2 + V2, P x 3, dS x 3
   LLSA_SMEM_LIMIT((attn_bwd_pooled_tc_kernel), smem);
-  attn_bwd_pooled_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, n_tiles, tiles_per_head);
+  launch_pdl(attn_bwd_pooled_tc_kernel, grid, kThreads, smem, st, a, maps, n_tiles, tiles_per_head);
   LLSA_LAUNCH_OK("attn_bwd_pooled_tc_kernel");
   return LLSA_OK;
 }

@@ -107,10 +107,12 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
     tc::mbar_init(&bars.acc_free, 8);
     tc::fence_mbar_init();
   }
+  pdl_wait();
   if (warp == 0) tc::tmem_alloc(&s_tmem, 512);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  pdl_trigger();
   const uint32_t tmem = s_tmem;
   const int units_per_head = GATHER ? chunks * (int) a.nq2 : chunks;
   Piece pc((int64_t) n_base * jobs_all, jobs_all);
@@ -339,7 +341,7 @@ int launch_attn_dkv_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
     const int chunks = (int) ((n_dense + kKeys - 1) / kKeys), jobs = (int) (a.Nq / kQ), units = (int) BH * chunks;
     const float w = a.two_level ? a.w2 : a.w1, kvw = a.two_level ? a.kvw2 : a.kvw1;
     LLSA_SMEM_LIMIT((attn_dkv_pooled_loop_tc_kernel<false>), smem);
-    attn_dkv_pooled_loop_tc_kernel<false><<<grid_of((int64_t) units * jobs), kThreads, smem, st>>>(
+    launch_pdl(attn_dkv_pooled_loop_tc_kernel<false>, grid_of((int64_t) units * jobs), kThreads, smem, st, 
         a, maps, a.two_level ? a.dpk2 : a.dpk, a.two_level ? a.dpv2 : a.dpv, n_dense, jobs, units, chunks, log2f(w), kvw / w);
     LLSA_LAUNCH_OK("attn_dkv_pooled_loop_tc_kernel");
   }
@@ -348,7 +350,7 @@ int launch_attn_dkv_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
     if ((rc = tma::make_map_rows(&maps.v, a.pv, (uint64_t) BH * a.n1, kBS))) return rc;
     const int chunks = (a.p1_blocks + 7) / 8, jobs = kBS * kBS / kQ, units = (int) (BH * a.nq2) * chunks;
     LLSA_SMEM_LIMIT((attn_dkv_pooled_loop_tc_kernel<true>), smem);
-    attn_dkv_pooled_loop_tc_kernel<true><<<grid_of((int64_t) units * jobs), kThreads, smem, st>>>(a, maps, a.dpk, a.dpv, a.n1, jobs, units, chunks,
+    launch_pdl(attn_dkv_pooled_loop_tc_kernel<true>, grid_of((int64_t) units * jobs), kThreads, smem, st, a, maps, a.dpk, a.dpv, a.n1, jobs, units, chunks,
                                                                                                  log2f(a.w1), a.kvw1 / a.w1);
     LLSA_LAUNCH_OK("attn_dkv_pooled_loop_tc_kernel<gathered>");
   }

@@ -80,6 +80,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   volatile tc::WaitCtl* abort_flag = &s_ctl;
   const int n_my = (n_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x;
   if (n_pass == 2 && redo) {
+    pdl_wait();
     // the second launch: anything to redo in this CTA's tiles?  (a tile's 128 marks are 32 words)
     int any = 0;
     if (warp == 0)
@@ -106,10 +107,12 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
     tc::mbar_init(&bars.xchg, 8);
     tc::fence_mbar_init();
   }
+  pdl_wait();
   if (warp == 0) tc::tmem_alloc(&s_tmem, 512);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  pdl_trigger();
   const uint32_t tmem = s_tmem;
   // jobs per tile; job j of tile i has the CTA-wide number i * jobs + j, which picks the S buffer (mod 3) and the softmax
   // group (mod 2; with one pass and an odd chunk count the parity of a tile's first job alternates)
@@ -408,10 +411,10 @@ int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
   LLSA_SMEM_LIMIT((attn_fwd_pooled_loop_tc_kernel), smem);
   unsigned char* redo = g->fwd_redo ? reinterpret_cast<unsigned char*>(g->fwd_redo->ptr) : nullptr;
   if (redo) {        // one pass with the fine part's log-sum-exp as reference, then the two-pass form for the rows it marked
-    attn_fwd_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, 1, redo);
+    launch_pdl(attn_fwd_pooled_loop_tc_kernel, grid, kThreads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, 1, redo);
     LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");
   }
-  attn_fwd_pooled_loop_tc_kernel<<<grid, kThreads, smem, st>>>(a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, 2, redo);
+  launch_pdl(attn_fwd_pooled_loop_tc_kernel, grid, kThreads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, 2, redo);
   LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");
   return LLSA_OK;
 }

@@ -82,10 +82,12 @@ attn_fwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ TcMaps maps, in
     }
     tc::fence_mbar_init();
   }
+  pdl_wait();
   if (warp == 0) tc::tmem_alloc(&s_tmem, 512);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  pdl_trigger();
   const uint32_t tmem = s_tmem;
   const int n_my = (n_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x;
 
@@ -299,7 +301,7 @@ int launch_attn_fwd_pooled_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, int64
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) kTcStages * (kTcRows * 64 + 2 * np * 64) * sizeof(bf16);
   LLSA_SMEM_LIMIT((attn_fwd_pooled_tc_kernel), smem);
-  attn_fwd_pooled_tc_kernel<<<grid, kTcThreads, smem, st>>>(a, maps, p1_keys, np, n_tiles, tiles_per_head);
+  launch_pdl(attn_fwd_pooled_tc_kernel, grid, kTcThreads, smem, st, a, maps, p1_keys, np, n_tiles, tiles_per_head);
   LLSA_LAUNCH_OK("attn_fwd_pooled_tc_kernel");
   return LLSA_OK;
 }

@@ -168,6 +168,8 @@ __global__ void __launch_bounds__(kFbThreads, NORM ? 4 : 1) front_bwd_kernel(Fro
 
 // dw[ti][c] = sum over the CTAs' rows, 16 strided partial sums per channel added in order
 __global__ void __launch_bounds__(1024) front_dw_kernel(const float* __restrict__ partial, int rows, float* dw0, float* dw1) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float sm[16][kFbC];
   const int c = threadIdx.x & 63, k = threadIdx.x >> 6;
   const float* p = partial + (int64_t) blockIdx.x * rows * kFbC + c;
@@ -227,7 +229,7 @@ static int front_bwd_typed(int n, const LlsaTensor* dy, const LlsaTensor* x, con
   if (freq && freq->dtype == LLSA_F32) rc = launch_front_bwd<T, float>(n, a, BH, grid, st);
   else rc = launch_front_bwd<T, T>(n, a, BH, grid, st);
   if (rc || !want_dw) return rc;
-  front_dw_kernel<<<n, 1024, 0, st>>>(a.dw_partial, grid, dw[0] ? (float*) dw[0]->ptr : nullptr, n > 1 && dw[1] ? (float*) dw[1]->ptr : nullptr);
+  launch_pdl(front_dw_kernel, n, 1024, 0, st, a.dw_partial, grid, dw[0] ? (float*) dw[0]->ptr : nullptr, n > 1 && dw[1] ? (float*) dw[1]->ptr : nullptr);
   LLSA_LAUNCH_OK("front_dw_kernel");
   return LLSA_OK;
 }

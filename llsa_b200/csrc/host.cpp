@@ -281,12 +281,14 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
     at::cuda::CUDAEvent fork, join;
     fork.record(cur);
     fork.block(side);
+    // the accumulators are cleared and the lists transposed next to the dQ stage, which needs neither
+    if (acc1) C10_CUDA_CHECK(cudaMemsetAsync(acc, 0, (2 * acc1 + 2 * acc2) * 4, side));
     transpose(side);
     join.record(side);
-    a.stage_mask = 3;
+    a.stage_mask = 1 | 8;
     ok(llsa_attn_bwd(&a, cur), "attn_bwd");
     join.block(cur);
-    a.stage_mask = 4;
+    a.stage_mask = 2 | 4;
     ok(llsa_attn_bwd(&a, cur), "attn_bwd");
   } else {
     transpose(cur);

@@ -200,6 +200,8 @@ template <int ROWT, int KW>
 __global__ void __launch_bounds__(kCmWarps * 32)
 coarse_topk_mma_kernel(const bf16* __restrict__ pq, const bf16* __restrict__ pk, void* __restrict__ idx_out, int idx64, int64_t M, int64_t n,
                        int topk) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int RG = kCmWarps / KW, ROWS = RG * ROWT * 16;
   __shared__ uint32_t lists[ROWS][KW * 4 * kCmTop + 4];      // + 4: rows shift by four banks.  Pass 1: the group maxima
   __shared__ uint32_t bound[ROWS];
@@ -365,6 +367,8 @@ __device__ __forceinline__ float4 load4(const T* p) {
 template <typename T>
 __global__ void __launch_bounds__(256)
 coarse_topk_tile_kernel(const T* __restrict__ pq, const T* __restrict__ pk, void* __restrict__ idx_out, int idx64, int64_t M, int64_t n, int topk) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   float* qs = sm;                                   // [16][kCtPitch]
   float* ks = qs + kCtRows * kCtPitch;              // [256][kCtPitch]
@@ -642,6 +646,8 @@ template <typename T, bool MMA, int FUSED = 0>
 __global__ void __launch_bounds__(128)
 refine_topk_kernel(const T* __restrict__ pq1, const T* __restrict__ pk1, IdxView p_idx, void* __restrict__ idx_out, int idx64, int64_t M,
                    int64_t Mk, int D_, int topk, int p_topk, int bs_, FusedCoarse fused) {
+  pdl_trigger();
+  pdl_wait();
   // constants where the dispatch fixes them: no division by a run-time block size per candidate
   const int D = MMA || FUSED ? 64 : D_, bs = MMA || FUSED ? 16 : bs_;
   extern __shared__ float sm[];
@@ -789,15 +795,15 @@ extern "C" int llsa_coarse_topk(const LlsaTensor* pq, const LlsaTensor* pk, cons
     const bf16 *q = (const bf16*) pq->ptr, *k = (const bf16*) pk->ptr;
     // 64 rows per CTA (each key read from L2 once per 64 rows) where that still gives every SM two CTAs, else 16 rows, the keys
     // split over all eight warps
-    if (B * H * ((M + 63) / 64) >= 2 * 148) coarse_topk_mma_kernel<2, 4><<<blocks(64), kCmWarps * 32, 0, st>>>(q, k, idx->ptr, idx64, M, n, topk);
-    else coarse_topk_mma_kernel<1, 8><<<blocks(16), kCmWarps * 32, 0, st>>>(q, k, idx->ptr, idx64, M, n, topk);
+    if (B * H * ((M + 63) / 64) >= 2 * 148) launch_pdl(coarse_topk_mma_kernel<2, 4>, blocks(64), kCmWarps * 32, 0, st, q, k, idx->ptr, idx64, M, n, topk);
+    else launch_pdl(coarse_topk_mma_kernel<1, 8>, blocks(16), kCmWarps * 32, 0, st, q, k, idx->ptr, idx64, M, n, topk);
   } else if (D == 64 && topk <= 32 && n < (1ll << 31)) {
     if (bf) {
       LLSA_SMEM_LIMIT((coarse_topk_tile_kernel<bf16>), kCtSmem);
-      coarse_topk_tile_kernel<bf16><<<blocks(kCtRows), 256, kCtSmem, st>>>((const bf16*) pq->ptr, (const bf16*) pk->ptr, idx->ptr, idx64, M, n, topk);
+      launch_pdl(coarse_topk_tile_kernel<bf16>, blocks(kCtRows), 256, kCtSmem, st, (const bf16*) pq->ptr, (const bf16*) pk->ptr, idx->ptr, idx64, M, n, topk);
     } else {
       LLSA_SMEM_LIMIT((coarse_topk_tile_kernel<float>), kCtSmem);
-      coarse_topk_tile_kernel<float><<<blocks(kCtRows), 256, kCtSmem, st>>>((const float*) pq->ptr, (const float*) pk->ptr, idx->ptr, idx64, M, n, topk);
+      launch_pdl(coarse_topk_tile_kernel<float>, blocks(kCtRows), 256, kCtSmem, st, (const float*) pq->ptr, (const float*) pk->ptr, idx->ptr, idx64, M, n, topk);
     }
   } else {
     const size_t smem = (size_t) kCoarseRows * (D + kCoarseChunk) * 4 + (size_t) kCoarseRows * kMaxTopk * (4 + 8) * 2;
@@ -840,15 +846,15 @@ extern "C" int llsa_refine_topk(const LlsaTensor* pq1, const LlsaTensor* pk1, co
   cudaStream_t st = (cudaStream_t) stream;
   if (pq1->dtype == LLSA_F32) {
     LLSA_SMEM_LIMIT((refine_topk_kernel<float, false>), smem);
-    refine_topk_kernel<float, false><<<grid, 128, smem, st>>>((const float*) pq1->ptr, (const float*) pk1->ptr, make_idx(p_idx), idx->ptr,
+    launch_pdl(refine_topk_kernel<float, false>, grid, 128, smem, st, (const float*) pq1->ptr, (const float*) pk1->ptr, make_idx(p_idx), idx->ptr,
                                                               idx->dtype == LLSA_I64, M, Mk, (int) D, topk, p_topk, bs, FusedCoarse{});
   } else if (D == 64 && bs == 16 && p_topk % 2 == 0 && ((uintptr_t) pq1->ptr % 32) == 0 && ((uintptr_t) pk1->ptr % 32) == 0) {
     LLSA_SMEM_LIMIT((refine_topk_kernel<__nv_bfloat16, true>), smem);
-    refine_topk_kernel<__nv_bfloat16, true><<<grid, 128, smem, st>>>((const __nv_bfloat16*) pq1->ptr, (const __nv_bfloat16*) pk1->ptr,
+    launch_pdl(refine_topk_kernel<__nv_bfloat16, true>, grid, 128, smem, st, (const __nv_bfloat16*) pq1->ptr, (const __nv_bfloat16*) pk1->ptr,
                                                                      make_idx(p_idx), idx->ptr, idx->dtype == LLSA_I64, M, Mk, (int) D, topk, p_topk, bs, FusedCoarse{});
   } else {
     LLSA_SMEM_LIMIT((refine_topk_kernel<__nv_bfloat16, false>), smem);
-    refine_topk_kernel<__nv_bfloat16, false><<<grid, 128, smem, st>>>((const __nv_bfloat16*) pq1->ptr, (const __nv_bfloat16*) pk1->ptr,
+    launch_pdl(refine_topk_kernel<__nv_bfloat16, false>, grid, 128, smem, st, (const __nv_bfloat16*) pq1->ptr, (const __nv_bfloat16*) pk1->ptr,
                                                                       make_idx(p_idx), idx->ptr, idx->dtype == LLSA_I64, M, Mk, (int) D, topk, p_topk, bs, FusedCoarse{});
   }
   LLSA_LAUNCH_OK("refine_topk_kernel");
@@ -901,15 +907,15 @@ extern "C" int llsa_select_two_level(const LlsaTensor* pq1, const LlsaTensor* pk
   const IdxView none{nullptr, 0};
   if (dt == LLSA_F32) {
     LLSA_SMEM_LIMIT((refine_topk_kernel<float, false, 2>), smem);
-    refine_topk_kernel<float, false, 2><<<grid, 128, smem, st>>>((const float*) pq1->ptr, (const float*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D,
+    launch_pdl(refine_topk_kernel<float, false, 2>, grid, 128, smem, st, (const float*) pq1->ptr, (const float*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D,
                                                                  topk, p_topk, bs, f);
   } else if (on_mma) {
     LLSA_SMEM_LIMIT((refine_topk_kernel<bf16, true, 1>), smem);
-    refine_topk_kernel<bf16, true, 1><<<grid, 128, smem, st>>>((const bf16*) pq1->ptr, (const bf16*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D, topk,
+    launch_pdl(refine_topk_kernel<bf16, true, 1>, grid, 128, smem, st, (const bf16*) pq1->ptr, (const bf16*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D, topk,
                                                                p_topk, bs, f);
   } else {
     LLSA_SMEM_LIMIT((refine_topk_kernel<bf16, true, 2>), smem);
-    refine_topk_kernel<bf16, true, 2><<<grid, 128, smem, st>>>((const bf16*) pq1->ptr, (const bf16*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D, topk,
+    launch_pdl(refine_topk_kernel<bf16, true, 2>, grid, 128, smem, st, (const bf16*) pq1->ptr, (const bf16*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D, topk,
                                                                p_topk, bs, f);
   }
   LLSA_LAUNCH_OK("refine_topk_kernel<fused>");

@@ -81,6 +81,8 @@ __device__ __forceinline__ void place_range(const TransposeArgs& a, int64_t bh, 
 // ---- one CTA per (b,h) and key range ----------------------------------------------------------------
 template <int W>
 __global__ void __launch_bounds__(W * 32) transpose_range_kernel(TransposeArgs a, int keys_per_range, uint32_t t_magic) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int warp_sums[32];
   __shared__ int s_below[W], s_kept[W];
@@ -392,10 +394,10 @@ static int transpose_impl(const LlsaTensor* idx, const LlsaTensor* offsets, cons
   cudaStream_t st = (cudaStream_t) stream;
   if (warps == 32) {
     LLSA_SMEM_LIMIT((transpose_range_kernel<32>), smem);
-    transpose_range_kernel<32><<<grid, 32 * 32, smem, st>>>(a, keys, t_magic);
+    launch_pdl(transpose_range_kernel<32>, grid, 32 * 32, smem, st, a, keys, t_magic);
   } else {
     LLSA_SMEM_LIMIT((transpose_range_kernel<16>), smem);
-    transpose_range_kernel<16><<<grid, 16 * 32, smem, st>>>(a, keys, t_magic);
+    launch_pdl(transpose_range_kernel<16>, grid, 16 * 32, smem, st, a, keys, t_magic);
   }
   LLSA_LAUNCH_OK("transpose_range_kernel");
   return LLSA_OK;
