@@ -835,8 +835,8 @@ __device__ __forceinline__ void dkv_store_unselected(const AttnP<bf16>& a, int64
 // the heads.  A warp owns 32 channels of one tensor, so a piece is four 128-bit loads per lane, four pieces in flight.
 // blockIdx.x >= n_windows - 1: the unselected blocks, 16 per CTA -- stores at the memory's rate next to the latency of the lookups (as extra
 // CTAs or extra work of the kernel above they cost twice as much: two CTAs of it fill an SM).
-// One warp for eight buckets, looking for both kinds, took 46 us at 48 slices of 16384 tokens and 160 us at 6 of 262144; this kernel FIN_A
-// and FIN_B.
+// One warp for eight buckets, looking for both kinds, took 46 us at 48 slices of 16384 tokens and 160 us at 6 of 262144; this kernel 31
+// and 81.
 __global__ void __launch_bounds__(128) attn_dkv_finish_kernel(AttnP<bf16> a, const float* __restrict__ partial, int n_windows) {
   if ((int) blockIdx.x >= n_windows - 1) {
     const int first = (((int) blockIdx.x - (n_windows - 1)) * 4 + (int) (threadIdx.x >> 5)) * kPlainPerWarp;
