@@ -12,14 +12,16 @@
 // The final log-sum-exp is known in the backward, so one pass over the chunks suffices.  dQ accumulates in TMEM over
 // all chunks of the tile and is then added to the fine part already in dq.
 // TMEM columns: three buffers, chunk number n of the CTA (counted over all its tiles) uses buffer n mod 3: S at 128 b,
-// dP at 128 b + 64; dQ at [384, 448).
-// Roles (one persistent CTA per SM, 11 warps): warp 8 lane 0 = TMA producer (Q, dO per tile, 2 stages; K and V
-// chunks in rings of 8: a stage is refilled four chunks before it is needed), warp 9 lane 0 issues S and dP, warp 10 lane 0 issues dQ, warps 0-3 / 4-7 = two softmax
-// warpgroups on alternating chunks; in the epilogue group w handles dQ columns [32 w, 32 w + 32).
-// Two issuing threads because one is the pace of the kernel: with the waits, commits and fences around twelve
-// instructions per chunk a single thread needed 1,400 cycles per chunk against 576 of tensor-pipe time.  The two run
+// dP at 128 b + 64.
+// TMEM columns: dQ of tile i at [384 + 64 (i mod 2), + 64).
+// Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64): warps 8 and 11 = TMA producers (Q, dO per
+// tile, 2 stages, and K chunks; V chunks; one ring of 8 pairs), warp 9 issues S and dP, warp 10 dQ, warps 0-3 / 4-7 = two softmax
+// warpgroups on alternating chunks, warps 12-15 = epilogue, thread = row: adds dQ to the row.  The two issuing warps run
 // independently (S / dP of the next tile start while dQ of this one is still being issued); a buffer goes back to the
-// S / dP thread through buf_free, committed behind the dQ instructions that read its dS.
+// S / dP warp through buf_free, committed behind the dQ instructions that read its dS.
+// A clock trace of the form with one producer lane, the epilogue in the softmax groups and one dQ accumulator (1,050 us at two levels,
+// B=1 H=6 N=262144: 1,350 cycles a chunk, tensor pipe 576) showed the producer needing 1,130 cycles a chunk for two waits and two copies
+// and an idle tensor pipe at every tile boundary; this form DQ_T.
 // Every mbarrier wait is bounded (abort flag; the kernel then ends early and frees its TMEM; dq is left partial).
 #include <string.h>
 
@@ -37,7 +39,7 @@ constexpr int kCk = 64;                      // keys per chunk
 constexpr int kTile = kRows * 64;            // elements of a [128 x 64] bf16 tile (16 KB)
 constexpr int kChunkElems = kCk * 64;        // elements of a key chunk (8 KB)
 constexpr int kStages = 8;
-constexpr int kThreads = 352;
+constexpr int kThreads = 512;
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr int kBufs = 3;
 constexpr uint32_t kColDQ = 384;
@@ -49,8 +51,8 @@ struct DqMaps {
 };
 
 struct DqBars {
-  uint64_t q_full[2], q_empty[2], k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages];
-  uint64_t sdp_ready[kBufs], ds_ready[kBufs], buf_free[kBufs], dq_ready, dq_free;
+  uint64_t q_full[2], q_empty[2], kv_full[kStages], kv_empty[kStages];
+  uint64_t sdp_ready[kBufs], ds_ready[kBufs], buf_free[kBufs], dq_ready[2], dq_free[2];
 };
 
 // jobs: 64-key chunks per tile; gathered: number of leading chunks that are gathered level-1 blocks; n_c: rows per head of the
@@ -83,11 +85,13 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
       tc::mbar_init(&bars.buf_free[i], 1);
     }
     for (int i = 0; i < kStages; ++i) {
-      tc::mbar_init(&bars.k_full[i], 1); tc::mbar_init(&bars.k_empty[i], 1);
-      tc::mbar_init(&bars.v_full[i], 1); tc::mbar_init(&bars.v_empty[i], 1);
+      tc::mbar_init(&bars.kv_full[i], 2);         // both producers
+      tc::mbar_init(&bars.kv_empty[i], 1);
     }
-    tc::mbar_init(&bars.dq_ready, 1);
-    tc::mbar_init(&bars.dq_free, 8);
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&bars.dq_ready[i], 1);
+      tc::mbar_init(&bars.dq_free[i], 4);
+    }
     tc::fence_mbar_init();
   }
   pdl_wait();
@@ -104,44 +108,43 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
     return left < kCk ? left : kCk;
   };
 
-  if (warp == 8) {
-    // ---------------------------------------------------------------- TMA producer
-    // lane 0 waits and issues; the blocks of a gathered chunk are issued by the lanes that hold their row (lane j: gathered block j)
-    int cj = 0;                                     // chunks loaded so far
-    for (int i = 0; i < n_my; ++i) {
+  if (warp == 8 || warp == 11) {
+    // ---------------------------------------------------------------- TMA producers: warp 8 Q, dO and keys, warp 11 values
+    const bool vals = warp == 11;
+    const CUtensorMap *mg = vals ? &maps.vg : &maps.kg, *mc = vals ? &maps.vc : &maps.kc;
+    bf16* ring = vals ? sV : sK;
+    int st = 0;
+    uint32_t ph = 1;
+    bool ok = true;
+    for (int i = 0; ok && i < n_my; ++i) {
       const int tile = blockIdx.x + i * gridDim.x, qs = i & 1;
       const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
-      int ok = 1, krow = 0;
-      if (lane == 0 && (ok = tc::bounded_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag))) {
-        tma::expect_tx(&bars.q_full[qs], 2 * kTile * 2);
-        tma::load_4d(sQ + qs * kTile, &maps.q, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
-        tma::load_4d(sDO + qs * kTile, &maps.d_o, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
+      if (!vals) {
+        if (!(ok = tc::warp_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag))) break;
+        tma::expect_tx_w(&bars.q_full[qs], 2 * kTile * 2);
+        tma::load_4d_w(sQ + qs * kTile, &maps.q, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
+        tma::load_4d_w(sDO + qs * kTile, &maps.d_o, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
       }
+      int krow = 0;                                           // lane j: first row of gathered block j
       if (gathered) krow = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, min(lane, a.p1_blocks - 1)) * kBS);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      for (int j = 0; ok && j < jobs; ++j, ++cj) {
-        const int st = cj % kStages;
-        const uint32_t par = ((cj / kStages) & 1) ^ 1;
-        const int crow = (int) ((int64_t) bh * n_c + (int64_t) (j - gathered) * kCk);
-        const bool mine = j < gathered && (lane >> 2) == j;
-        if (lane == 0 && (ok = tc::bounded_wait(&bars.k_empty[st], par, abort_flag))) {
-          tma::expect_tx(&bars.k_full[st], kChunkElems * 2);
-          if (j >= gathered) tma::load_2d(sK + st * kChunkElems, &maps.kc, &bars.k_full[st], 0, crow);
+      int crow = (int) ((int64_t) bh * n_c);                  // next contiguous chunk
+      for (int j = 0; j < jobs; ++j) {
+        if (!(ok = tc::warp_wait(&bars.kv_empty[st], ph, abort_flag))) break;
+        tma::expect_tx_w(&bars.kv_full[st], kChunkElems * 2);
+        if (j < gathered) {
+#pragma unroll
+          for (int b4 = 0; b4 < 4; ++b4)
+            tma::load_2d_w(ring + st * kChunkElems + b4 * kBS * 64, mg, &bars.kv_full[st], 0, __shfl_sync(0xffffffffu, krow, (j * 4 + b4) & 31));
+        } else {
+          tma::load_2d_w(ring + st * kChunkElems, mc, &bars.kv_full[st], 0, crow);
+          crow += kCk;
         }
-        if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
-        if (mine) tma::load_2d(sK + st * kChunkElems + (lane & 3) * kBS * 64, &maps.kg, &bars.k_full[st], 0, krow);
-        if (lane == 0 && (ok = tc::bounded_wait(&bars.v_empty[st], par, abort_flag))) {
-          tma::expect_tx(&bars.v_full[st], kChunkElems * 2);
-          if (j >= gathered) tma::load_2d(sV + st * kChunkElems, &maps.vc, &bars.v_full[st], 0, crow);
-        }
-        if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
-        if (mine) tma::load_2d(sV + st * kChunkElems + (lane & 3) * kBS * 64, &maps.vg, &bars.v_full[st], 0, krow);
+        if (++st == kStages) { st = 0; ph ^= 1; }
       }
-      if (!ok) break;
     }
   } else if (warp == 9) {
     // ---------------------------------------------------------------- MMA issuer 1: S and dP
-    if (lane == 0) {
+    {
       const uint32_t id_s = tc::instr_desc(kRows, kCk, 0, 0);
       const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
       auto lo = [](const void* p, uint32_t lbo_bytes) { return ((tc::smem_u32(p) >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16); };
@@ -152,36 +155,29 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
       bool ok = true;
       for (int i = 0; ok && i < n_my; ++i) {
         const int qs = i & 1;
-        if (!(ok = tc::bounded_wait(&bars.q_full[qs], (i >> 1) & 1, abort_flag))) break;
+        if (!(ok = tc::warp_wait(&bars.q_full[qs], (i >> 1) & 1, abort_flag))) break;
         const uint32_t q_ = lQ + qs * kQStage, o_ = lDO + qs * kQStage;
         for (int j = 0; j < jobs; ++j) {
-          // the buffer's previous chunk (three back): its dQ instructions have read dS
-          if (cj >= kBufs && !(ok = tc::bounded_wait(&bars.buf_free[buf], bph ^ 1, abort_flag))) break;
-          if (!(ok = tc::bounded_wait(&bars.k_full[st], par, abort_flag))) break;
-          if (!(ok = tc::bounded_wait(&bars.v_full[st], par, abort_flag))) break;
+          // even lanes: the chunk; odd lanes: the buffer's previous chunk (three back), whose dQ instructions have read dS
+          const bool b = (lane & 1) && cj >= kBufs;
+          if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : &bars.kv_full[st], b ? bph ^ 1 : par, abort_flag))) break;
           tc::fence_after_sync();
           const uint32_t d = tmem + buf * 128;
           const uint32_t k_ = lK + st * kCStage, v_ = lV + st * kCStage;
-          tc::umma_ss_lh<0>(d, q_, hi, k_, hi, id_s);
-          tc::umma_ss_lh<0>(d + 64, o_, hi, v_, hi, id_s);
-#pragma unroll
-          for (int s4 = 1; s4 < 4; ++s4) {
-            tc::umma_ss_lh<1>(d, q_ + 2 * s4, hi, k_ + 2 * s4, hi, id_s);
-            tc::umma_ss_lh<1>(d + 64, o_ + 2 * s4, hi, v_ + 2 * s4, hi, id_s);
-          }
-          tc::umma_commit(&bars.sdp_ready[buf]);
-          tc::umma_commit(&bars.v_empty[st]);        // the values are not needed again
+          tc::umma_ss_k64(d, q_, hi, k_, hi, id_s);
+          tc::umma_ss_k64(d + 64, o_, hi, v_, hi, id_s);
+          tc::umma_commit_w(&bars.sdp_ready[buf]);
           ++cj;
           if (++st == kStages) { st = 0; par ^= 1; }
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
         }
         if (!ok) break;
-        tc::umma_commit(&bars.q_empty[qs]);
+        tc::umma_commit_w(&bars.q_empty[qs]);
       }
     }
   } else if (warp == 10) {
     // ---------------------------------------------------------------- MMA issuer 2: dQ (+)= dS(chunk, TMEM) . K chunk
-    if (lane == 0) {
+    {
       const uint32_t id_dq = tc::instr_desc(kRows, 64, 0, 1);
       const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
       constexpr uint32_t kCStage = (uint32_t) (kChunkElems * 2) >> 4;
@@ -191,45 +187,43 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
       bool ok = true;
       for (int i = 0; ok && i < n_my; ++i) {
         for (int j = 0; j < jobs; ++j) {
-          if (!(ok = tc::bounded_wait(&bars.ds_ready[buf], bph, abort_flag))) break;
-          if (j == 0 && i > 0 && !(ok = tc::bounded_wait(&bars.dq_free, (i - 1) & 1, abort_flag))) break;     // previous tile's dQ has been read
+          // odd lanes, first chunk of a tile: dQ of the tile before the last has been read
+          const bool f = (lane & 1) && j == 0 && i > 1;
+          if (!(ok = tc::warp_wait(f ? &bars.dq_free[i & 1] : &bars.ds_ready[buf], f ? ((uint32_t) (i - 2) >> 1) & 1 : bph, abort_flag))) break;
           tc::fence_after_sync();
-          const uint64_t kdesc = ((uint64_t) hi << 32) | (uint64_t) (lKm + st * kCStage);       // 16 key rows = 2048 bytes per k-step
-          tc::umma_ts(tmem + kColDQ, tmem + buf * 128, kdesc, id_dq, j > 0 ? 1u : 0u);
-          tc::umma_ts(tmem + kColDQ, tmem + buf * 128 + 8, kdesc + 128, id_dq, 1u);
-          if (keys_of(j) == kCk) {
-            tc::umma_ts(tmem + kColDQ, tmem + buf * 128 + 16, kdesc + 256, id_dq, 1u);
-            tc::umma_ts(tmem + kColDQ, tmem + buf * 128 + 24, kdesc + 384, id_dq, 1u);
-          }
-          tc::umma_commit(&bars.k_empty[st]);
-          tc::umma_commit(&bars.buf_free[buf]);
+          const uint32_t k_ = lKm + st * kCStage, d_ = tmem + buf * 128;       // 16 key rows = 2048 bytes per k-step
+          if (keys_of(j) == kCk) tc::umma_ts_k64(tmem + kColDQ + (i & 1) * 64, d_, k_, hi, id_dq, j > 0 ? 1u : 0u);
+          else tc::umma_ts_k32(tmem + kColDQ + (i & 1) * 64, d_, k_, hi, id_dq, j > 0 ? 1u : 0u);
+          tc::umma_commit_w(&bars.kv_empty[st]);
+          tc::umma_commit_w(&bars.buf_free[buf]);
           if (++st == kStages) st = 0;
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
         }
         if (!ok) break;
-        tc::umma_commit(&bars.dq_ready);
+        tc::umma_commit_w(&bars.dq_ready[i & 1]);
       }
     }
-  } else {
-    // ---------------------------------------------------------------- dS, then the dq update; thread = query row
+  } else if (warp < 8) {
+    // ---------------------------------------------------------------- dS; thread = query row
     const int wg = warp >> 2, qd = warp & 3, r = qd * 32 + lane;
     const float sl2 = a.scale * kLog2eF;
     const float lw1 = log2f(a.w1), lw2 = log2f(a.w2);
     const uint32_t t_lane = tmem + ((uint32_t) (qd * 32) << 16);
     int buf = wg;                          // this group takes every other chunk: buffer and phase parity of its next one
     uint32_t bph = 0;
-    const uint32_t t_dq = tmem + kColDQ + wg * 32 + ((uint32_t) (qd * 32) << 16);
     float vs[32], vd[32];
-    for (int i = 0; i < n_my; ++i) {
+    float lse_next = 0.f, delta_next = 0.f;
+    auto fetch = [&](int i) {              // this thread's row of tile i
       const int tile = blockIdx.x + i * gridDim.x;
-      const int bh = tile / tiles_per_head, row = (tile % tiles_per_head) * kRows + r;
-      const float L = a.lse[(int64_t) bh * a.Nq + row] * kLog2eF;
-      const float dls = a.delta[(int64_t) bh * a.Nq + row] * a.scale;
-      bf16* dqrow = a.dq.row(bh / a.H, bh % a.H, row) + wg * 32;
-      uint4 old[4];
-#pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) old[q4] = *reinterpret_cast<const uint4*>(dqrow + 8 * q4);
-      bool ok = true;
+      const int64_t at = (int64_t) (tile / tiles_per_head) * a.Nq + (tile % tiles_per_head) * kRows + r;
+      lse_next = a.lse[at];
+      delta_next = a.delta[at];
+    };
+    if (n_my > 0) fetch(0);
+    bool ok = true;
+    for (int i = 0; ok && i < n_my; ++i) {
+      const float L = lse_next * kLog2eF, dls = delta_next * a.scale;
+      if (i + 1 < n_my) fetch(i + 1);
       for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
         const float off = ((j < gathered || !a.two_level) ? lw1 : lw2) - L;
         const int halves = keys_of(j) / 32;
@@ -259,25 +253,42 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
         buf += 2;
         if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
       }
-      if (!ok) break;
-      ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.dq_ready, (uint32_t) (i & 1), abort_flag));
+    }
+  } else {
+    // ---------------------------------------------------------------- dq += dQ; thread = query row
+    const int qd = warp & 3, r = qd * 32 + lane;
+    bool ok = true;
+    for (int i = 0; ok && i < n_my; ++i) {
+      const int tile = blockIdx.x + i * gridDim.x;
+      const int bh = tile / tiles_per_head, row = (tile % tiles_per_head) * kRows + r;
+      bf16* dqrow = a.dq.row(bh / a.H, bh % a.H, row);
+      uint4 old[8];                        // the fine part: requested before the wait
+#pragma unroll
+      for (int q8 = 0; q8 < 8; ++q8) old[q8] = *reinterpret_cast<const uint4*>(dqrow + 8 * q8);
+      ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.dq_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
-      tc::tmem_ld32_async(t_dq, vs);
-      tc::tmem_ld_wait(vs);
 #pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) {
-        const uint4 f = old[q4];
-        uint4 w;
-        w.x = pack_bf16(bf16_lo(f.x) + vs[8 * q4], bf16_hi(f.x) + vs[8 * q4 + 1]);
-        w.y = pack_bf16(bf16_lo(f.y) + vs[8 * q4 + 2], bf16_hi(f.y) + vs[8 * q4 + 3]);
-        w.z = pack_bf16(bf16_lo(f.z) + vs[8 * q4 + 4], bf16_hi(f.z) + vs[8 * q4 + 5]);
-        w.w = pack_bf16(bf16_lo(f.w) + vs[8 * q4 + 6], bf16_hi(f.w) + vs[8 * q4 + 7]);
-        *reinterpret_cast<uint4*>(dqrow + 8 * q4) = w;
+      for (int half = 0; half < 2; ++half) {
+        float v[32];
+        tc::tmem_ld32_async(tmem + kColDQ + (i & 1) * 64 + half * 32 + ((uint32_t) (qd * 32) << 16), v);
+        tc::tmem_ld_wait(v);
+        if (half == 1) {
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tma::mbar_arrive(&bars.dq_free[i & 1]);
+        }
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4) {
+          const uint4 f = old[half * 4 + q4];
+          uint4 w;
+          w.x = pack_bf16(bf16_lo(f.x) + v[8 * q4], bf16_hi(f.x) + v[8 * q4 + 1]);
+          w.y = pack_bf16(bf16_lo(f.y) + v[8 * q4 + 2], bf16_hi(f.y) + v[8 * q4 + 3]);
+          w.z = pack_bf16(bf16_lo(f.z) + v[8 * q4 + 4], bf16_hi(f.z) + v[8 * q4 + 5]);
+          w.w = pack_bf16(bf16_lo(f.w) + v[8 * q4 + 6], bf16_hi(f.w) + v[8 * q4 + 7]);
+          *reinterpret_cast<uint4*>(dqrow + half * 32 + 8 * q4) = w;
+        }
       }
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) tma::mbar_arrive(&bars.dq_free);
     }
   }
   if (abort_flag->abort) tc::abort_drain();

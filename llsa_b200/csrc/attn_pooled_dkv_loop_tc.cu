@@ -18,12 +18,15 @@
 // multiple of 32 keys) hold a repeated block or the rows that follow in memory; their results stay in their own rows and are dropped.
 // Work split: all (head, chunk, job) triples in that order form one flat list that is cut into gridDim.x equal pieces,
 // one per CTA; a piece is one to a few units (it changes unit where it crosses a chunk boundary).
-// TMEM columns: three buffers, job number n of the CTA uses buffer n mod 3: S^T at 128 b, dP^T at 128 b + 64; dV at
-// [384,448), dK at [448,512).
-// Roles (one persistent CTA per SM, 11 warps): warp 8 lane 0 = TMA producer (K_c, V_c per unit in two stages; Q_t, dO_t, lse, delta per
-// job in a ring of 8), warp 9 lane 0 issues S^T and dP^T, warp 10 lane 0 issues dV and dK (one issuing thread, with its
-// waits, commits and fences, is slower than the tensor pipe), warps 0-3 / 4-7 = two softmax warpgroups on alternating
-// jobs; at the end of a unit group 0 writes dV, group 1 writes dK.  Every mbarrier wait is bounded (abort flag, TMEM freed).
+// TMEM columns: NB buffers, job number n of the CTA uses buffer n mod NB: S^T at 128 b, dP^T at 128 b + 64; then NA accumulators, unit number
+// i of the CTA uses i mod NA: dV, dK (64 columns each).  Dense units are hundreds of jobs long: NB = 3, NA = 1.  Gathered units are
+// four jobs long: NB = 2, NA = 2, so that a unit's first products do not wait for the last one's results to be read.
+// Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64): warps 8 and 11 = TMA producers (K_c, V_c
+// per unit in two stages, Q_t per job; dO_t, lse, delta per job; a ring of 8), warp 9 issues S^T and dP^T, warp 10 dV and dK,
+// warps 0-3 / 4-7 = two softmax warpgroups on alternating jobs, warps 12-15 write a unit's dV and dK, thread = key row.  Every mbarrier
+// wait is bounded (abort flag, TMEM freed).
+// Two levels, B=1 H=6 N=262144 (tensor pipe 768 cycles a job): with one producer lane and results written by the softmax groups 1,010 us
+// dense, 315 gathered; this form DKV_T.
 #include <string.h>
 
 #include "attn.cuh"
@@ -40,10 +43,8 @@ constexpr int kQ = 64;                       // query rows per job (MMA N)
 constexpr int kKeyTile = kKeys * 64;         // elements of the K / V chunk (16 KB)
 constexpr int kQTile = kQ * 64;              // elements of a Q / dO job tile (8 KB)
 constexpr int kStages = 8;
-constexpr int kThreads = 352;
-constexpr int kBufs = 3;
+constexpr int kThreads = 512;
 constexpr float kLog2eF = 1.4426950408889634f;
-constexpr uint32_t kColDV = 384, kColDK = 448;
 
 struct KvMaps {
   CUtensorMap q, d_o;         // [B,H,Nq,64] 4-D, box 64 rows
@@ -51,7 +52,7 @@ struct KvMaps {
 };
 
 struct KvBars {
-  uint64_t kv_full[2], kv_empty[2], q_full[kStages], q_empty[kStages], sdp_ready[kBufs], pds_ready[kBufs], buf_free[kBufs], acc_ready, acc_free;
+  uint64_t kv_full[2], kv_empty[2], q_full[kStages], q_empty[kStages], sdp_ready[3], pds_ready[3], buf_free[3], acc_ready[2], acc_free[2];
 };
 
 // A CTA's piece of the flat job list, walked unit by unit.
@@ -90,6 +91,8 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
   bf16* sV = sK + 2 * kKeyTile;              // [2][128][64]
   bf16* sQ = sV + 2 * kKeyTile;              // [kStages][64][64]
   bf16* sDO = sQ + kStages * kQTile;         // [kStages][64][64]
+  constexpr int kBufs = GATHER ? 2 : 3, kAccs = GATHER ? 2 : 1;
+  constexpr uint32_t kColAcc = kBufs * 128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile tc::WaitCtl* abort_flag = &s_ctl;
 
@@ -97,14 +100,13 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
     s_ctl.abort = 0;
     s_ctl.limit = a.wait_limit > 0 ? a.wait_limit : tc::kWaitPolls;
     for (int i = 0; i < 2; ++i) { tc::mbar_init(&bars.kv_full[i], 1); tc::mbar_init(&bars.kv_empty[i], 1); }
-    for (int i = 0; i < kStages; ++i) { tc::mbar_init(&bars.q_full[i], 1); tc::mbar_init(&bars.q_empty[i], 1); }
+    for (int i = 0; i < kStages; ++i) { tc::mbar_init(&bars.q_full[i], 2); tc::mbar_init(&bars.q_empty[i], 1); }
     for (int i = 0; i < kBufs; ++i) {
       tc::mbar_init(&bars.sdp_ready[i], 1);
       tc::mbar_init(&bars.pds_ready[i], 4);
       tc::mbar_init(&bars.buf_free[i], 1);
     }
-    tc::mbar_init(&bars.acc_ready, 1);
-    tc::mbar_init(&bars.acc_free, 8);
+    for (int i = 0; i < kAccs; ++i) { tc::mbar_init(&bars.acc_ready[i], 1); tc::mbar_init(&bars.acc_free[i], 4); }
     tc::fence_mbar_init();
   }
   pdl_wait();
@@ -117,47 +119,51 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
   const int units_per_head = GATHER ? chunks * (int) a.nq2 : chunks;
   Piece pc((int64_t) n_base * jobs_all, jobs_all);
 
-  if (warp == 8) {
-    // ---------------------------------------------------------------- TMA producer
-    // lane 0 waits and issues; gathered: lane j < 8 fetches and issues block j of the unit's keys
-    int cj = 0, ok = 1;
+  if (warp == 8 || warp == 11) {
+    // ---------------------------------------------------------------- TMA producers: warp 8 the unit's keys and Q, warp 11 dO, lse, delta
+    const bool second = warp == 11;
+    int st = 0;
+    uint32_t ph = 1;
+    bool ok = true;
     for (int i = 0; ok && pc.next(); ++i) {
       const int bh = pc.unit / units_per_head, u = pc.unit - bh * units_per_head, ks = i & 1;
       const int c = GATHER ? u % chunks : u, q0 = GATHER ? u / chunks * (kBS * kBS) : 0;      // chunk; first query row of the parent
-      int krow = 0;
-      if (GATHER) krow = (int) ((int64_t) bh * n_keys + p1_block(a, bh, q0 / kBS, min(c * 8 + (lane & 7), a.p1_blocks - 1)) * kBS);
-      if (lane == 0 && (ok = tc::bounded_wait(&bars.kv_empty[ks], ((i >> 1) & 1) ^ 1, abort_flag))) {
-        tma::expect_tx(&bars.kv_full[ks], 2 * kKeyTile * 2);
+      if (!second) {
+        int krow = (int) ((int64_t) bh * n_keys + (int64_t) c * kKeys);
+        if (GATHER) krow = (int) ((int64_t) bh * n_keys + p1_block(a, bh, q0 / kBS, min(c * 8 + (lane & 7), a.p1_blocks - 1)) * kBS);      // lane j: block j
+        if (!(ok = tc::warp_wait(&bars.kv_empty[ks], ((i >> 1) & 1) ^ 1, abort_flag))) break;
+        tma::expect_tx_w(&bars.kv_full[ks], 2 * kKeyTile * 2);
         if (!GATHER) {
-          const int krow0 = (int) ((int64_t) bh * n_keys + (int64_t) c * kKeys);
-          tma::load_2d(sK + ks * kKeyTile, &maps.k, &bars.kv_full[ks], 0, krow0);
-          tma::load_2d(sV + ks * kKeyTile, &maps.v, &bars.kv_full[ks], 0, krow0);
+          tma::load_2d_w(sK + ks * kKeyTile, &maps.k, &bars.kv_full[ks], 0, krow);
+          tma::load_2d_w(sV + ks * kKeyTile, &maps.v, &bars.kv_full[ks], 0, krow);
+        } else {
+#pragma unroll
+          for (int b8 = 0; b8 < 8; ++b8) {
+            const int row = __shfl_sync(0xffffffffu, krow, b8);
+            tma::load_2d_w(sK + ks * kKeyTile + b8 * kBS * 64, &maps.k, &bars.kv_full[ks], 0, row);
+            tma::load_2d_w(sV + ks * kKeyTile + b8 * kBS * 64, &maps.v, &bars.kv_full[ks], 0, row);
+          }
         }
       }
-      if (GATHER) {
-        if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
-        if (lane < 8) {
-          tma::load_2d(sK + ks * kKeyTile + lane * kBS * 64, &maps.k, &bars.kv_full[ks], 0, krow);
-          tma::load_2d(sV + ks * kKeyTile + lane * kBS * 64, &maps.v, &bars.kv_full[ks], 0, krow);
+      const int hd = bh % a.H, bt = bh / a.H;
+      int qrow = q0 + pc.job0 * kQ;
+      for (int j = 0; j < pc.n; ++j, qrow += kQ) {
+        if (!(ok = tc::warp_wait(&bars.q_empty[st], ph, abort_flag))) break;
+        if (!second) {
+          tma::expect_tx_w(&bars.q_full[st], kQTile * 2);
+          tma::load_4d_w(sQ + st * kQTile, &maps.q, &bars.q_full[st], 0, qrow, hd, bt);
+        } else {
+          tma::expect_tx_w(&bars.q_full[st], kQTile * 2 + 2 * kQ * 4);
+          tma::load_4d_w(sDO + st * kQTile, &maps.d_o, &bars.q_full[st], 0, qrow, hd, bt);
+          tma::load_bulk_w(s_lse[st], a.lse + (int64_t) bh * a.Nq + qrow, kQ * 4, &bars.q_full[st]);
+          tma::load_bulk_w(s_delta[st], a.delta + (int64_t) bh * a.Nq + qrow, kQ * 4, &bars.q_full[st]);
         }
+        if (++st == kStages) { st = 0; ph ^= 1; }
       }
-      if (lane == 0) {
-        for (int j = 0; ok && j < pc.n; ++j, ++cj) {
-          const int st = cj & (kStages - 1);
-          if (!(ok = tc::bounded_wait(&bars.q_empty[st], ((cj / kStages) & 1) ^ 1, abort_flag))) break;
-          tma::expect_tx(&bars.q_full[st], 2 * kQTile * 2 + 2 * kQ * 4);
-          const int qrow = q0 + (pc.job0 + j) * kQ;
-          tma::load_4d(sQ + st * kQTile, &maps.q, &bars.q_full[st], 0, qrow, bh % a.H, bh / a.H);
-          tma::load_4d(sDO + st * kQTile, &maps.d_o, &bars.q_full[st], 0, qrow, bh % a.H, bh / a.H);
-          tma::load_bulk(s_lse[st], a.lse + (int64_t) bh * a.Nq + qrow, kQ * 4, &bars.q_full[st]);
-          tma::load_bulk(s_delta[st], a.delta + (int64_t) bh * a.Nq + qrow, kQ * 4, &bars.q_full[st]);
-        }
-      }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
     }
   } else if (warp == 9) {
     // ---------------------------------------------------------------- MMA issuer 1: S^T and dP^T of every job
-    if (lane == 0) {
+    {
       const uint32_t id_s = tc::instr_desc(kKeys, kQ, 0, 0);
       const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
       auto lo = [](const void* p, uint32_t lbo_bytes) { return ((tc::smem_u32(p) >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16); };
@@ -168,32 +174,27 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       bool ok = true;
       for (int i = 0; ok && pc.next(); ++i) {
         const int ks = i & 1;
-        if (!(ok = tc::bounded_wait(&bars.kv_full[ks], (i >> 1) & 1, abort_flag))) break;
+        if (!(ok = tc::warp_wait(&bars.kv_full[ks], (i >> 1) & 1, abort_flag))) break;
         const uint32_t k_ = lK + ks * kKeyStage, v_ = lV + ks * kKeyStage;
         for (int j = 0; j < pc.n; ++j, ++cj) {
           const int st = cj & (kStages - 1);
-          // the buffer's previous job (three back): the dV / dK instructions that read its P^T / dS^T have completed
-          if (cj >= kBufs && !(ok = tc::bounded_wait(&bars.buf_free[buf], bph ^ 1, abort_flag))) break;
-          if (!(ok = tc::bounded_wait(&bars.q_full[st], (cj / kStages) & 1, abort_flag))) break;
+          // even lanes: the query tile; odd lanes: the buffer's previous job (kBufs back), whose P^T / dS^T have been read
+          const bool b = (lane & 1) && cj >= kBufs;
+          if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : &bars.q_full[st], b ? bph ^ 1 : (uint32_t) (cj / kStages) & 1, abort_flag))) break;
           tc::fence_after_sync();
           const uint32_t d = tmem + buf * 128, q_ = lQ + st * kQStage, o_ = lDO + st * kQStage;
-          tc::umma_ss_lh<0>(d, k_, hi, q_, hi, id_s);
-          tc::umma_ss_lh<0>(d + 64, v_, hi, o_, hi, id_s);
-#pragma unroll
-          for (int s4 = 1; s4 < 4; ++s4) {
-            tc::umma_ss_lh<1>(d, k_ + 2 * s4, hi, q_ + 2 * s4, hi, id_s);
-            tc::umma_ss_lh<1>(d + 64, v_ + 2 * s4, hi, o_ + 2 * s4, hi, id_s);
-          }
-          tc::umma_commit(&bars.sdp_ready[buf]);
+          tc::umma_ss_k64(d, k_, hi, q_, hi, id_s);
+          tc::umma_ss_k64(d + 64, v_, hi, o_, hi, id_s);
+          tc::umma_commit_w(&bars.sdp_ready[buf]);
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
         }
         if (!ok) break;
-        tc::umma_commit(&bars.kv_empty[ks]);         // the key chunk is only read by these products
+        tc::umma_commit_w(&bars.kv_empty[ks]);         // the key chunk is only read by these products
       }
     }
   } else if (warp == 10) {
     // ---------------------------------------------------------------- MMA issuer 2: dV (+)= P^T . dO_t, dK (+)= dS^T . Q_t
-    if (lane == 0) {
+    {
       const uint32_t id_o = tc::instr_desc(kKeys, 64, 0, 1);
       const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
       auto lo = [](const void* p, uint32_t lbo_bytes) { return ((tc::smem_u32(p) >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16); };
@@ -205,40 +206,77 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       for (int i = 0; ok && pc.next(); ++i) {
         for (int j = 0; j < pc.n; ++j, ++cj) {
           const int st = cj & (kStages - 1);
-          if (!(ok = tc::bounded_wait(&bars.pds_ready[buf], bph, abort_flag))) break;
-          if (j == 0 && i > 0 && !(ok = tc::bounded_wait(&bars.acc_free, (i - 1) & 1, abort_flag))) break;    // previous unit's results have been read
+          // odd lanes, first job of a unit: the results this accumulator held last have been read
+          const bool f = (lane & 1) && j == 0 && i >= kAccs;
+          if (!(ok = tc::warp_wait(f ? &bars.acc_free[i % kAccs] : &bars.pds_ready[buf], f ? (uint32_t) (i / kAccs - 1) & 1 : bph, abort_flag))) break;
           tc::fence_after_sync();
           // 4 k-steps of 16 query rows (2048 bytes of the MN-major dO / Q tile)
-          const uint64_t dodesc = ((uint64_t) hi << 32) | (uint64_t) (lDOm + st * kQStage), qdesc = ((uint64_t) hi << 32) | (uint64_t) (lQm + st * kQStage);
-          const uint32_t b = tmem + buf * 128;
-#pragma unroll
-          for (int s4 = 0; s4 < 4; ++s4) {
-            const uint32_t acc = (j > 0 || s4 > 0) ? 1u : 0u;
-            tc::umma_ts(tmem + kColDV, b + s4 * 8, dodesc + 128 * s4, id_o, acc);
-            tc::umma_ts(tmem + kColDK, b + 64 + s4 * 8, qdesc + 128 * s4, id_o, acc);
-          }
-          tc::umma_commit(&bars.q_empty[st]);
-          tc::umma_commit(&bars.buf_free[buf]);
+          const uint32_t o_ = lDOm + st * kQStage, q_ = lQm + st * kQStage, b = tmem + buf * 128, acc = tmem + kColAcc + (i % kAccs) * 128;
+          tc::umma_ts_k64(acc, b, o_, hi, id_o, j > 0 ? 1u : 0u);
+          tc::umma_ts_k64(acc + 64, b + 64, q_, hi, id_o, j > 0 ? 1u : 0u);
+          tc::umma_commit_w(&bars.q_empty[st]);
+          tc::umma_commit_w(&bars.buf_free[buf]);
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
         }
         if (!ok) break;
-        tc::umma_commit(&bars.acc_ready);
+        tc::umma_commit_w(&bars.acc_ready[i % kAccs]);
+      }
+    }
+  } else if (warp < 8) {
+    // ---------------------------------------------------------------- P^T / dS^T; thread = key row
+    const int wg = warp >> 2, qd = warp & 3;
+    const float sl2 = a.scale * kLog2eF;
+    const uint32_t t_lane = tmem + ((uint32_t) (qd * 32) << 16);
+    const int64_t total = pc.f_end - pc.f;         // jobs of this CTA
+    int buf = wg;                                  // buffer of this group's next job and the phase parity of its barriers
+    uint32_t bph = 0;
+    float vs[32], vd[32];
+    for (int64_t jn = wg; jn < total; jn += 2) {
+      const int st = (int) jn & (kStages - 1);
+      const bool ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.sdp_ready[buf], bph, abort_flag));
+      tc::fence_after_sync();
+      if (!ok) break;
+      const uint32_t t_b = t_lane + buf * 128;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        tc::tmem_ld32_async(t_b + 32 * half, vs);
+        tc::tmem_ld32_async(t_b + 64 + 32 * half, vd);
+        tc::tmem_ld_wait(vs);
+        tc::tmem_ld_wait(vd);
+        uint32_t pp[16], pd[16];
+#pragma unroll
+        for (int q4 = 0; q4 < 8; ++q4) {           // 4 query columns at a time: their lse / delta are broadcast reads
+          const float4 l4 = *reinterpret_cast<const float4*>(&s_lse[st][32 * half + 4 * q4]);
+          const float4 d4 = *reinterpret_cast<const float4*>(&s_delta[st][32 * half + 4 * q4]);
+          const float p0 = fast_exp2(fmaf(vs[4 * q4], sl2, fmaf(l4.x, -kLog2eF, lw_log2)));
+          const float p1 = fast_exp2(fmaf(vs[4 * q4 + 1], sl2, fmaf(l4.y, -kLog2eF, lw_log2)));
+          const float p2 = fast_exp2(fmaf(vs[4 * q4 + 2], sl2, fmaf(l4.z, -kLog2eF, lw_log2)));
+          const float p3 = fast_exp2(fmaf(vs[4 * q4 + 3], sl2, fmaf(l4.w, -kLog2eF, lw_log2)));
+          pp[2 * q4] = pack_bf16(p0, p1);
+          pp[2 * q4 + 1] = pack_bf16(p2, p3);
+          pd[2 * q4] = pack_bf16(p0 * ((vd[4 * q4] - d4.x) * a.scale), p1 * ((vd[4 * q4 + 1] - d4.y) * a.scale));
+          pd[2 * q4 + 1] = pack_bf16(p2 * ((vd[4 * q4 + 2] - d4.z) * a.scale), p3 * ((vd[4 * q4 + 3] - d4.w) * a.scale));
+        }
+        tc::tmem_st16(t_b + 16 * half, pp);            // P^T over S^T columns read before
+        tc::tmem_st16(t_b + 64 + 16 * half, pd);       // dS^T over dP^T columns read before
+      }
+      tc::tmem_st_wait();
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tma::mbar_arrive(&bars.pds_ready[buf]);
+      if (kBufs == 2) {                              // the group's own buffer again
+        bph ^= 1;
+      } else {
+        buf += 2;
+        if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
       }
     }
   } else {
-    // ---------------------------------------------------------------- P^T / dS^T, then the results; thread = key row
-    const int wg = warp >> 2, qd = warp & 3, r = qd * 32 + lane;
-    const float sl2 = a.scale * kLog2eF;
-    const uint32_t t_lane = tmem + ((uint32_t) (qd * 32) << 16);
-    const uint32_t t_acc = t_lane + (wg == 0 ? kColDV : kColDK);
-    int jn = wg, jc = 0;                          // this group's next job and the unit's first job, both numbered over the CTA
-    int buf = wg;                                 // buffer of job jn and the phase parity of its barriers
-    uint32_t bph = 0;
-    float vs[32], vd[32];
-    bool ok = true;
-    for (int i = 0; ok && pc.next(); ++i) {
+    // ---------------------------------------------------------------- results of a unit; thread = key row
+    const int qd = warp & 3, r = qd * 32 + lane;
+    for (int i = 0; pc.next(); ++i) {
       const int bh = pc.unit / units_per_head, u = pc.unit - bh * units_per_head, c = GATHER ? u % chunks : u;
-      // this thread's key: its row in the pooled tensor (gathered: fetched now, used at the end of the unit), or none
+      // this thread's key: its row in the pooled tensor, or none
       bool live = true;
       int64_t key = (int64_t) c * kKeys + r;
       if (GATHER) {
@@ -248,67 +286,31 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       } else {
         live = key < n_keys;
       }
-      for (; jn < jc + pc.n; jn += 2) {
-        const int st = jn & (kStages - 1);
-        ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.sdp_ready[buf], bph, abort_flag));
-        tc::fence_after_sync();
-        if (!ok) break;
-        const uint32_t t_b = t_lane + buf * 128;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          tc::tmem_ld32_async(t_b + 32 * half, vs);
-          tc::tmem_ld32_async(t_b + 64 + 32 * half, vd);
-          tc::tmem_ld_wait(vs);
-          tc::tmem_ld_wait(vd);
-          uint32_t pp[16], pd[16];
-#pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4) {           // 4 query columns at a time: their lse / delta are broadcast reads
-            const float4 l4 = *reinterpret_cast<const float4*>(&s_lse[st][32 * half + 4 * q4]);
-            const float4 d4 = *reinterpret_cast<const float4*>(&s_delta[st][32 * half + 4 * q4]);
-            const float p0 = fast_exp2(fmaf(vs[4 * q4], sl2, fmaf(l4.x, -kLog2eF, lw_log2)));
-            const float p1 = fast_exp2(fmaf(vs[4 * q4 + 1], sl2, fmaf(l4.y, -kLog2eF, lw_log2)));
-            const float p2 = fast_exp2(fmaf(vs[4 * q4 + 2], sl2, fmaf(l4.z, -kLog2eF, lw_log2)));
-            const float p3 = fast_exp2(fmaf(vs[4 * q4 + 3], sl2, fmaf(l4.w, -kLog2eF, lw_log2)));
-            pp[2 * q4] = pack_bf16(p0, p1);
-            pp[2 * q4 + 1] = pack_bf16(p2, p3);
-            pd[2 * q4] = pack_bf16(p0 * ((vd[4 * q4] - d4.x) * a.scale), p1 * ((vd[4 * q4 + 1] - d4.y) * a.scale));
-            pd[2 * q4 + 1] = pack_bf16(p2 * ((vd[4 * q4 + 2] - d4.z) * a.scale), p3 * ((vd[4 * q4 + 3] - d4.w) * a.scale));
-          }
-          tc::tmem_st16(t_b + 16 * half, pp);            // P^T over S^T columns read before
-          tc::tmem_st16(t_b + 64 + 16 * half, pd);       // dS^T over dP^T columns read before
-        }
-        tc::tmem_st_wait();
-        tc::fence_before_sync();
-        __syncwarp();
-        if (lane == 0) tma::mbar_arrive(&bars.pds_ready[buf]);
-        buf += 2;
-        if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
-      }
-      if (!ok) break;
-      jc += pc.n;
-      ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.acc_ready, (uint32_t) (i & 1), abort_flag));
+      const bool whole = !GATHER && pc.n == jobs_all;           // the unit saw every query of its head: nobody else adds to these rows
+      const bool ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.acc_ready[i % kAccs], (uint32_t) (i / kAccs) & 1, abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
-      float* dst = (wg == 0 ? dpv : dpk) + ((int64_t) bh * n_keys + key) * kD;
-      const bool whole = !GATHER && pc.n == jobs_all;           // the unit saw every query of its head: nobody else adds to these rows
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        tc::tmem_ld32_async(t_acc + 32 * half, vs);
-        tc::tmem_ld_wait(vs);
+      for (int part = 0; part < 4; ++part) {
+        float v[32];
+        tc::tmem_ld32_async(tmem + kColAcc + (i % kAccs) * 128 + part * 32 + ((uint32_t) (qd * 32) << 16), v);
+        tc::tmem_ld_wait(v);
+        if (part == 3) {
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tma::mbar_arrive(&bars.acc_free[i % kAccs]);
+        }
+        float* dst = (part < 2 ? dpv : dpk) + ((int64_t) bh * n_keys + key) * kD + (part & 1) * 32;
         if (!live) {
         } else if (whole) {
 #pragma unroll
           for (int q4 = 0; q4 < 8; ++q4)
-            *reinterpret_cast<float4*>(dst + 32 * half + 4 * q4) = make_float4(vs[4 * q4] * out_mul, vs[4 * q4 + 1] * out_mul, vs[4 * q4 + 2] * out_mul, vs[4 * q4 + 3] * out_mul);
+            *reinterpret_cast<float4*>(dst + 4 * q4) = make_float4(v[4 * q4] * out_mul, v[4 * q4 + 1] * out_mul, v[4 * q4 + 2] * out_mul, v[4 * q4 + 3] * out_mul);
         } else {
 #pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4)
-            red_add_v4(dst + 32 * half + 4 * q4, vs[4 * q4] * out_mul, vs[4 * q4 + 1] * out_mul, vs[4 * q4 + 2] * out_mul, vs[4 * q4 + 3] * out_mul);
+          for (int q4 = 0; q4 < 8; ++q4) red_add_v4(dst + 4 * q4, v[4 * q4] * out_mul, v[4 * q4 + 1] * out_mul, v[4 * q4 + 2] * out_mul, v[4 * q4 + 3] * out_mul);
         }
       }
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) tma::mbar_arrive(&bars.acc_free);
     }
   }
   if (abort_flag->abort) tc::abort_drain();

@@ -17,18 +17,20 @@
 // hold anything up to 2^127 times it; a row whose pooled keys outweigh its fine keys by more than that (its row sum
 // passes 1e30, or is NaN) is left untouched and marked in `redo`, and a second launch of the two-pass form redoes
 // exactly the marked rows (it scans its tiles' marks first and returns at once when there are none).
-// Roles (one persistent CTA per SM, 11 warps):
-//   warp 8, one lane : TMA producer: Q per tile (2 stages), K chunks (ring of 4; every chunk is loaded in both
-//                      passes), V chunks (ring of 4, pass 2 only)
-//   warp 9, one lane : issues S of every "job" (a chunk of a pass).  Job number n, counted over all tiles of the CTA,
-//                      uses S buffer n mod 3 (TMEM columns [128 b, 128 b + 128)); O lives in [384,448).
-//   warp 10, one lane: issues O += P.V of the pass-2 jobs and hands every job's buffer back to warp 9 (buf_free,
-//                      committed behind the instructions that read P).  Two issuing threads because one, with its waits,
-//                      commits and fences, was the pace of the kernel: 2,050 cycles per job against 780 of pipe time.
+// Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64):
+//   warp 8, warp 11  : TMA producers: Q per tile (2 stages) and K chunks (ring of 4; every chunk is loaded in both passes); V chunks (ring
+//                      of 4, pass 2 only)
+//   warp 9           : issues S of every "job" (a chunk of a pass).  Job number n, counted over all tiles of the CTA,
+//                      uses S buffer n mod 3 (TMEM columns [128 b, 128 b + 128)); O of tile i lives in [384 + 64 (i mod 2), + 64).
+//   warp 10          : issues O += P.V of the pass-2 jobs and hands every job's buffer back to warp 9 (buf_free,
+//                      committed behind the instructions that read P)
 //   warps 0-3 / 4-7  : two softmax warpgroups, group w owns the jobs n = w (mod 2); thread r owns query row r
-//                      (TMEM lane r).  Row maxima and row sums of the two groups meet in shared memory (an
-//                      mbarrier with one arrival per softmax warp, so that this wait is bounded too).  Epilogue: group w merges O columns [32w, 32w+32)
-//                      with the fine part (o, lse written by the fine kernel) and stores them.
+//                      (TMEM lane r).  They leave a row's sum (and reference) in shared memory and go on to the next tile.
+//   warps 12-15      : epilogue, thread = row: merges O with the fine part (o, lse written by the fine kernel) and stores both.
+// What bounds it: the 128 exponentials of a row and job on the SM's 16 MUFU lanes (1,024 cycles a job; tensor pipe 640).  A clock trace
+// of the form with one producer lane, the epilogue in the softmax groups and one O buffer (785 us at l1, B=2 H=4 N=65536: 1,630 cycles a
+// job) showed the producer needing 1,300 cycles a job for its two waits and two copies, and 5,900 idle cycles at every tile boundary;
+// this form FWD_T.
 // Every mbarrier wait is bounded; a wait that expires raises a CTA-wide abort flag, every role leaves its loops,
 // lse of the unfinished rows is poisoned with NaN and TMEM is freed.
 #include <string.h>
@@ -46,7 +48,7 @@ constexpr int kRows = 128;
 constexpr int kChunk = 128;                 // keys per chunk
 constexpr int kTile = kRows * 64;           // elements of a [128 x 64] bf16 tile (16 KB)
 constexpr int kKStages = 4, kVStages = 4;
-constexpr int kThreads = 352;
+constexpr int kThreads = 512;
 constexpr int kBufs = 3;
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr uint32_t kColO = 384;
@@ -59,7 +61,7 @@ struct LoopMaps {
 
 struct LoopBars {
   uint64_t q_full[2], q_empty[2], k_full[kKStages], k_empty[kKStages], v_full[kVStages], v_empty[kVStages];
-  uint64_t s_ready[kBufs], wg_done[kBufs], buf_free[kBufs], o_ready, o_free, xchg;
+  uint64_t s_ready[kBufs], wg_done[kBufs], buf_free[kBufs], o_ready[2], o_free[2], sum_ready[2], xchg;
 };
 
 // n_chunks: chunks per tile; gathered: how many of them, the first ones, are gathered level-1 blocks (two levels); n_c: rows per
@@ -71,7 +73,8 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   __shared__ LoopBars bars;
   __shared__ uint32_t s_tmem;
   __shared__ tc::WaitCtl s_ctl;
-  __shared__ float s_part[2][2][kRows];     // [exchange parity][group][row]: row maxima, then row sums
+  __shared__ float s_max[2][2][kRows];               // [tile parity][group][row]: row maxima after pass 1
+  __shared__ float s_sum[2][2][kRows], s_ref[2][kRows];      // [tile parity][group][row] row sums; [tile parity][row] their reference
   bf16* base = reinterpret_cast<bf16*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   bf16* sQ = base;                          // [2][128][64]
   bf16* sK = sQ + 2 * kTile;                // [kKStages][128][64]
@@ -83,8 +86,8 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
     pdl_wait();
     // the second launch: anything to redo in this CTA's tiles?  (a tile's 128 marks are 32 words)
     int any = 0;
-    if (warp == 0)
-      for (int i = 0; i < n_my; ++i) any |= (int) reinterpret_cast<const uint32_t*>(redo)[(int64_t) (blockIdx.x + i * gridDim.x) * (kRows / 4) + lane];
+    for (int i = warp; i < n_my; i += kThreads / 32)
+      any |= (int) reinterpret_cast<const uint32_t*>(redo)[(int64_t) (blockIdx.x + i * gridDim.x) * (kRows / 4) + lane];
     if (!__syncthreads_or(any)) return;
   }
 
@@ -102,8 +105,11 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
     }
     for (int i = 0; i < kKStages; ++i) { tc::mbar_init(&bars.k_full[i], 1); tc::mbar_init(&bars.k_empty[i], 1); }
     for (int i = 0; i < kVStages; ++i) { tc::mbar_init(&bars.v_full[i], 1); tc::mbar_init(&bars.v_empty[i], 1); }
-    tc::mbar_init(&bars.o_ready, 1);
-    tc::mbar_init(&bars.o_free, 8);
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&bars.o_ready[i], 1);
+      tc::mbar_init(&bars.o_free[i], 4);
+      tc::mbar_init(&bars.sum_ready[i], 8);
+    }
     tc::mbar_init(&bars.xchg, 8);
     tc::fence_mbar_init();
   }
@@ -123,48 +129,45 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
     return left < kChunk ? left : kChunk;
   };
 
-  if (warp == 8) {
-    // ---------------------------------------------------------------- TMA producer
-    // lane 0 waits and issues; the blocks of a gathered chunk are issued by the lanes that hold their row (lane j: gathered block j)
-    int kjob = 0, vjob = 0;
-    for (int i = 0; i < n_my; ++i) {
+  if (warp == 8 || warp == 11) {
+    // ---------------------------------------------------------------- TMA producers: warp 8 Q and keys, warp 11 values
+    const bool vals = warp == 11;
+    uint64_t *full = vals ? bars.v_full : bars.k_full, *empty = vals ? bars.v_empty : bars.k_empty;
+    const CUtensorMap *mg = vals ? &maps.vg : &maps.kg, *mc = vals ? &maps.vc : &maps.kc;
+    bf16* ring = vals ? sV : sK;
+    static_assert(kKStages == kVStages, "one loop for both rings");
+    int st = 0;
+    uint32_t ph = 1;
+    bool ok = true;
+    for (int i = 0; ok && i < n_my; ++i) {
       const int tile = blockIdx.x + i * gridDim.x, qs = i & 1;
       const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
-      int ok = 1, krow = 0;
-      if (lane == 0 && (ok = tc::bounded_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag))) {
-        tma::expect_tx(&bars.q_full[qs], kTile * 2);
-        tma::load_4d(sQ + qs * kTile, &maps.q, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
+      if (!vals) {
+        if (!(ok = tc::warp_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag))) break;
+        tma::expect_tx_w(&bars.q_full[qs], kTile * 2);
+        tma::load_4d_w(sQ + qs * kTile, &maps.q, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
       }
+      int krow = 0;                                           // lane j: first row of gathered block j
       if (gathered) krow = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, min(lane, a.p1_blocks - 1)) * kBS);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      for (int j = 0; ok && j < jobs; ++j) {
-        const int c = j % n_chunks, pass = j >= first_p2;
-        const int crow = (int) ((int64_t) bh * n_c + (int64_t) (c - gathered) * kChunk);      // contiguous chunk
-        const bool mine = (lane >> 3) == c;                                                   // a lane of this gathered chunk
-        const int ks = kjob % kKStages;
-        if (lane == 0 && (ok = tc::bounded_wait(&bars.k_empty[ks], ((kjob / kKStages) & 1) ^ 1, abort_flag))) {
-          tma::expect_tx(&bars.k_full[ks], kTile * 2);
-          if (c >= gathered) tma::load_2d(sK + ks * kTile, &maps.kc, &bars.k_full[ks], 0, crow);
+      int crow = (int) ((int64_t) bh * n_c);                  // next contiguous chunk
+      for (int j = vals ? first_p2 : 0; j < jobs; ++j) {
+        const int c = j >= n_chunks ? j - n_chunks : j;
+        if (!(ok = tc::warp_wait(&empty[st], ph, abort_flag))) break;
+        tma::expect_tx_w(&full[st], kTile * 2);
+        if (c < gathered) {
+#pragma unroll
+          for (int b8 = 0; b8 < 8; ++b8) tma::load_2d_w(ring + st * kTile + b8 * kBS * 64, mg, &full[st], 0, __shfl_sync(0xffffffffu, krow, (c * 8 + b8) & 31));
+        } else {
+          if (c == gathered) crow = (int) ((int64_t) bh * n_c);
+          tma::load_2d_w(ring + st * kTile, mc, &full[st], 0, crow);
+          crow += kChunk;
         }
-        if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
-        if (c < gathered && mine) tma::load_2d(sK + ks * kTile + (lane & 7) * kBS * 64, &maps.kg, &bars.k_full[ks], 0, krow);
-        ++kjob;
-        if (pass == 1) {
-          const int vs = vjob % kVStages;
-          if (lane == 0 && (ok = tc::bounded_wait(&bars.v_empty[vs], ((vjob / kVStages) & 1) ^ 1, abort_flag))) {
-            tma::expect_tx(&bars.v_full[vs], kTile * 2);
-            if (c >= gathered) tma::load_2d(sV + vs * kTile, &maps.vc, &bars.v_full[vs], 0, crow);
-          }
-          if (!(ok = __shfl_sync(0xffffffffu, ok, 0))) break;
-          if (c < gathered && mine) tma::load_2d(sV + vs * kTile + (lane & 7) * kBS * 64, &maps.vg, &bars.v_full[vs], 0, krow);
-          ++vjob;
-        }
+        if (++st == kKStages) { st = 0; ph ^= 1; }
       }
-      if (!ok) break;
     }
   } else if (warp == 9) {
     // ---------------------------------------------------------------- MMA issuer 1: S of every job
-    if (lane == 0) {
+    {
       const uint32_t id_s = tc::instr_desc(kRows, kChunk, 0, 0);
       const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
       auto lo = [](const void* p, uint32_t lbo_bytes) { return ((tc::smem_u32(p) >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16); };
@@ -175,29 +178,27 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       bool ok = true;
       for (int i = 0; ok && i < n_my; ++i) {
         const int qs = i & 1;
-        if (!(ok = tc::bounded_wait(&bars.q_full[qs], (i >> 1) & 1, abort_flag))) break;
+        if (!(ok = tc::warp_wait(&bars.q_full[qs], (i >> 1) & 1, abort_flag))) break;
         const uint32_t q_ = lQ + qs * kStage;
         for (int j = 0; j < jobs; ++j, ++n) {
-          // the buffer's previous job (three back): its group has read S and, in pass 2, P.V has read P
-          if (n >= kBufs && !(ok = tc::bounded_wait(&bars.buf_free[buf], bph ^ 1, abort_flag))) break;
-          if (!(ok = tc::bounded_wait(&bars.k_full[ks], kph, abort_flag))) break;
+          // even lanes: the key chunk; odd lanes: the buffer's previous job (three back), whose group has read S and, in pass 2, P.V P
+          const bool b = (lane & 1) && n >= kBufs;
+          if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : &bars.k_full[ks], b ? bph ^ 1 : kph, abort_flag))) break;
           tc::fence_after_sync();
           const uint32_t k_ = lK + ks * kStage, d = tmem + buf * kChunk;
-          tc::umma_ss_lh<0>(d, q_, hi, k_, hi, id_s);
-#pragma unroll
-          for (int s4 = 1; s4 < 4; ++s4) tc::umma_ss_lh<1>(d, q_ + 2 * s4, hi, k_ + 2 * s4, hi, id_s);
-          tc::umma_commit(&bars.s_ready[buf]);
-          tc::umma_commit(&bars.k_empty[ks]);
+          tc::umma_ss_k64(d, q_, hi, k_, hi, id_s);
+          tc::umma_commit_w(&bars.s_ready[buf]);
+          tc::umma_commit_w(&bars.k_empty[ks]);
           if (++ks == kKStages) { ks = 0; kph ^= 1; }
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
         }
         if (!ok) break;
-        tc::umma_commit(&bars.q_empty[qs]);
+        tc::umma_commit_w(&bars.q_empty[qs]);
       }
     }
   } else if (warp == 10) {
     // ---------------------------------------------------------------- MMA issuer 2: O (+)= P(job, TMEM) . V chunk
-    if (lane == 0) {
+    {
       const uint32_t id_o = tc::instr_desc(kRows, 64, 0, 1);
       const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
       constexpr uint32_t kStage = (uint32_t) (kTile * 2) >> 4;
@@ -207,85 +208,77 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       bool ok = true;
       for (int i = 0; ok && i < n_my; ++i) {
         for (int j = 0; j < jobs; ++j) {
-          if (!(ok = tc::bounded_wait(&bars.wg_done[buf], bph, abort_flag))) break;
-          if (j >= first_p2) {
-            const int c = j - first_p2;
-            if (!(ok = tc::bounded_wait(&bars.v_full[vs], vph, abort_flag))) break;
-            if (c == 0 && i > 0 && !(ok = tc::bounded_wait(&bars.o_free, (i - 1) & 1, abort_flag))) break;      // previous tile's O has been read
+          // even lanes: the group's job; odd lanes of a pass-2 job: the value chunk; lane 3: O of the tile before the last has been read
+          const bool pv = j >= first_p2;
+          const int c = j - first_p2;
+          uint64_t* bar = &bars.wg_done[buf];
+          uint32_t par = bph;
+          if (pv && lane == 3 && c == 0 && i > 1) { bar = &bars.o_free[i & 1]; par = ((i - 2) >> 1) & 1; }
+          else if (pv && (lane & 1)) { bar = &bars.v_full[vs]; par = vph; }
+          if (!(ok = tc::warp_wait(bar, par, abort_flag))) break;
+          if (pv) {
             tc::fence_after_sync();
-            const uint64_t vdesc = ((uint64_t) hi << 32) | (uint64_t) (lV + vs * kStage);
+            const uint32_t v_ = lV + vs * kStage, p_ = tmem + buf * kChunk, o_ = tmem + kColO + (i & 1) * 64;
             // P: 16 keys = 8 packed columns per k-step; V: 16 key rows = 2048 bytes
             const int ksteps = keys_of(c) / 16;
-            if (ksteps == 8) {
-#pragma unroll
-              for (int s8 = 0; s8 < 8; ++s8)
-                tc::umma_ts(tmem + kColO, tmem + buf * kChunk + s8 * 8, vdesc + 128 * s8, id_o, (c > 0 || s8 > 0) ? 1u : 0u);
-            } else {
-              for (int s8 = 0; s8 < ksteps; ++s8)
-                tc::umma_ts(tmem + kColO, tmem + buf * kChunk + s8 * 8, vdesc + 128 * s8, id_o, (c > 0 || s8 > 0) ? 1u : 0u);
+            const uint32_t acc = c > 0 ? 1u : 0u;
+            if (ksteps >= 4) {
+              if (ksteps == 8) tc::umma_ts_k128(o_, p_, v_, hi, id_o, acc);
+              else tc::umma_ts_k64(o_, p_, v_, hi, id_o, acc);
             }
-            tc::umma_commit(&bars.v_empty[vs]);
+            if (ksteps & 2) tc::umma_ts_k32(o_, p_ + (ksteps == 6 ? 32 : 0), v_ + (ksteps == 6 ? 512 : 0), hi, id_o, ksteps == 6 ? 1u : acc);
+            tc::umma_commit_w(&bars.v_empty[vs]);
             if (++vs == kVStages) { vs = 0; vph ^= 1; }
           }
-          tc::umma_commit(&bars.buf_free[buf]);
+          tc::umma_commit_w(&bars.buf_free[buf]);
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
         }
         if (!ok) break;
-        tc::umma_commit(&bars.o_ready);
+        tc::umma_commit_w(&bars.o_ready[i & 1]);
       }
     }
-  } else {
-    // ---------------------------------------------------------------- softmax + epilogue, thread = query row
+  } else if (warp < 8) {
+    // ---------------------------------------------------------------- softmax, thread = query row
     const int wg = warp >> 2, qd = warp & 3, r = qd * 32 + lane;
     const float sl2 = a.scale * kLog2eF;
     const float lw1 = log2f(a.w1), lw2 = log2f(a.w2);
     const uint32_t t_lane = tmem + ((uint32_t) (qd * 32) << 16);
-    const uint32_t t_o = t_lane + kColO + wg * 32;
     int buf = wg;                          // S buffer of this group's next job (it takes every other job of the CTA) and
     uint32_t bph = 0;                      // the phase parity of that buffer's barriers
-    uint32_t n_x = 0;                      // exchanges so far
     float va[32];
-    // Both groups publish a per-row value and read the other group's.  The buffer alternates with the exchange count:
-    // a buffer is rewritten two exchanges later, after every thread has passed the barrier in between.
-    auto exchange = [&](float mine, float& other) -> bool {
-      s_part[n_x & 1][wg][r] = mine;
-      __syncwarp();
-      if (lane == 0) tma::mbar_arrive(&bars.xchg);
-      const bool ok_ = __all_sync(0xffffffffu, tc::bounded_wait(&bars.xchg, n_x & 1, abort_flag));
-      other = s_part[n_x & 1][wg ^ 1][r];
-      ++n_x;
-      return ok_;
-    };
-    for (int i = 0; i < n_my; ++i) {
+    auto lse_of = [&](int i) {             // the fine part's log-sum-exp of this thread's row of tile i
       const int tile = blockIdx.x + i * gridDim.x;
-      const int bh = tile / tiles_per_head, row = (tile % tiles_per_head) * kRows + r;
-      bf16* orow = a.o.row(bh / a.H, bh % a.H, row) + wg * 32;
-      // the fine part of this row (this group's 32 channels): requested now, consumed in the epilogue
-      uint4 of[4];
-#pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) of[q4] = *reinterpret_cast<const uint4*>(orow + 8 * q4);
-      const float lse_f = a.lse[(int64_t) bh * a.Nq + row];
+      return a.lse[(int64_t) (tile / tiles_per_head) * a.Nq + (tile % tiles_per_head) * kRows + r];
+    };
+    float lse_next = n_pass == 1 && n_my > 0 ? lse_of(0) : 0.f;
+    bool ok = true;
+    for (int i = 0; ok && i < n_my; ++i) {
       // one pass: the fine part's log-sum-exp is the reference of the exponentials
-      float mx = n_pass == 1 ? lse_f * kLog2eF : -INFINITY, lsum = 0.f;
-      bool ok = true, exchanged = n_pass == 1;
-      // two passes: the groups exchange their row maxima once per tile, before their first pass-2 job (a group may have none)
+      float mx = n_pass == 1 ? lse_next * kLog2eF : -INFINITY, lsum = 0.f;
+      if (n_pass == 1 && i + 1 < n_my) lse_next = lse_of(i + 1);
+      bool exchanged = n_pass == 1;
+      // two passes: the groups exchange their row maxima once per tile, before their first pass-2 job (a group may have none); a copy is
+      // rewritten two exchanges later, after both groups have passed the barrier in between
       auto exchange_max = [&]() -> bool {
-        float other;
         exchanged = true;
-        if (!exchange(mx, other)) return false;
-        mx = fmaxf(mx, other);
-        return true;
+        s_max[i & 1][wg][r] = mx;
+        __syncwarp();
+        if (lane == 0) tma::mbar_arrive(&bars.xchg);
+        const bool ok_ = __all_sync(0xffffffffu, tc::bounded_wait(&bars.xchg, (uint32_t) i & 1, abort_flag));
+        mx = fmaxf(s_max[i & 1][0][r], s_max[i & 1][1][r]);
+        return ok_;
       };
       for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
-        const int c = j % n_chunks, pass = j >= first_p2;
+        const bool p2 = j >= first_p2;
+        const int c = j >= n_chunks ? j - n_chunks : j;
         const float lw = (c < gathered || !a.two_level) ? lw1 : lw2;
         const int nq = keys_of(c) / 32;
-        if (pass == 1 && !exchanged && !(ok = exchange_max())) break;
+        if (p2 && !exchanged && !(ok = exchange_max())) break;
         ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.s_ready[buf], bph, abort_flag));
         tc::fence_after_sync();
         if (!ok) break;
         const uint32_t t_s = t_lane + buf * kChunk;
-        if (pass == 0) {
+        if (!p2) {
           float m = -INFINITY;
           for (int q4 = 0; q4 < nq; ++q4) {
             tc::tmem_ld32_async(t_s + 32 * q4, va);
@@ -296,7 +289,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           mx = fmaxf(mx, fmaf(m, sl2, lw));
         } else {
           const float off = lw - mx;
-#pragma unroll 1          // unrolled, the four quarters' registers overlap and 18 of them spill (to L2: L1 is 28 KB here)
+#pragma unroll 1          // unrolled, the four quarters' registers overlap and spill (to L2: L1 is 28 KB here)
           for (int q4 = 0; q4 < nq; ++q4) {
             tc::tmem_ld32_async(t_s + 32 * q4, va);
             tc::tmem_ld_wait(va);
@@ -318,54 +311,71 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
       }
       if (ok && !exchanged) ok = exchange_max();
-      float lse_out = __int_as_float(0x7fc00000);               // NaN unless everything completed
-      if (ok) {
-        float other;
-        ok = exchange(lsum, other);
-        lsum = wg == 0 ? lsum + other : other + lsum;          // the same order in both groups: identical bits
-      }
-      // does this launch own the row?  One pass: unless its sum left the safe range (then the mark hands it to the
-      // second launch).  Second launch: only the marked rows.
+      // the sums of the tile before the last have been read
+      if (ok && i > 1) ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_free[i & 1], ((uint32_t) (i - 2) >> 1) & 1, abort_flag));
+      if (!ok) break;
+      s_sum[i & 1][wg][r] = lsum;
+      if (wg == 0) s_ref[i & 1][r] = mx;
+      __syncwarp();
+      if (lane == 0) tma::mbar_arrive(&bars.sum_ready[i & 1]);
+    }
+  } else {
+    // ---------------------------------------------------------------- epilogue, thread = query row
+    const int qd = warp & 3, r = qd * 32 + lane;
+    bool ok = true;
+    for (int i = 0; i < n_my; ++i) {
+      const int tile = blockIdx.x + i * gridDim.x;
+      const int bh = tile / tiles_per_head, row = (tile % tiles_per_head) * kRows + r;
+      bf16* orow = a.o.row(bh / a.H, bh % a.H, row);
+      float* lse_p = a.lse + (int64_t) bh * a.Nq + row;
+      // the fine part of this row, and whether the second launch owns it: requested before the waits
+      uint4 of[8];
+#pragma unroll
+      for (int q8 = 0; q8 < 8; ++q8) of[q8] = *reinterpret_cast<const uint4*>(orow + 8 * q8);
+      const float lse_f = *lse_p;
       bool mine = true;
-      if (redo) {
-        if (n_pass == 1) {
-          mine = lsum < 1e30f;                                  // false for NaN too
-          if (wg == 0 && ok) redo[(int64_t) bh * a.Nq + row] = mine ? 0 : 1;
-        } else {
-          mine = redo[(int64_t) bh * a.Nq + row] != 0;
-        }
+      if (redo && n_pass == 2) mine = redo[(int64_t) bh * a.Nq + row] != 0;
+      ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.sum_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
+      ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
+      tc::fence_after_sync();
+      if (!ok) {
+        if (mine) *lse_p = __int_as_float(0x7fc00000);             // NaN: not completed
+        break;
       }
-      if (ok) {
-        ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_ready, (uint32_t) (i & 1), abort_flag));
-        tc::fence_after_sync();
+      const float lsum = s_sum[i & 1][0][r] + s_sum[i & 1][1][r], mx = s_ref[i & 1][r];
+      // one pass: the row is this launch's unless its sum left the safe range (false for NaN too): the mark hands it to the second
+      if (redo && n_pass == 1) {
+        mine = lsum < 1e30f;
+        redo[(int64_t) bh * a.Nq + row] = mine ? 0 : 1;
       }
-      if (ok) {
-        tc::tmem_ld32_async(t_o, va);
-        const float Lf = lse_f * kLog2eF;                        // fine part, log2 domain
-        const float Lp = mx + log2f(lsum);
-        const float Lm = fmaxf(Lf, Lp);
-        const float ef = fast_exp2(Lf - Lm), ep = fast_exp2(Lp - Lm);
-        const float inv = 1.f / (ef + ep);
-        const float wf = ef * inv, wp = lsum > 0.f ? ep * inv / lsum : 0.f;      // every exponential may have underflowed
-        lse_out = (Lm + log2f(ef + ep)) * 0.6931471805599453f;
+      const float Lf = lse_f * kLog2eF;                        // fine part, log2 domain
+      const float Lp = mx + log2f(lsum);
+      const float Lm = fmaxf(Lf, Lp);
+      const float ef = fast_exp2(Lf - Lm), ep = fast_exp2(Lp - Lm);
+      const float inv = 1.f / (ef + ep);
+      const float wf = ef * inv, wp = lsum > 0.f ? ep * inv / lsum : 0.f;      // every exponential may have underflowed
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        float va[32];
+        tc::tmem_ld32_async(tmem + kColO + (i & 1) * 64 + half * 32 + ((uint32_t) (qd * 32) << 16), va);
         tc::tmem_ld_wait(va);
+        if (half == 1) {                                        // O and the sums are in registers
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tma::mbar_arrive(&bars.o_free[i & 1]);
+        }
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
-          const uint4 f = of[q4];
+          const uint4 f = of[half * 4 + q4];
           uint4 w;
           w.x = pack_bf16(bf16_lo(f.x) * wf + va[8 * q4] * wp, bf16_hi(f.x) * wf + va[8 * q4 + 1] * wp);
           w.y = pack_bf16(bf16_lo(f.y) * wf + va[8 * q4 + 2] * wp, bf16_hi(f.y) * wf + va[8 * q4 + 3] * wp);
           w.z = pack_bf16(bf16_lo(f.z) * wf + va[8 * q4 + 4] * wp, bf16_hi(f.z) * wf + va[8 * q4 + 5] * wp);
           w.w = pack_bf16(bf16_lo(f.w) * wf + va[8 * q4 + 6] * wp, bf16_hi(f.w) * wf + va[8 * q4 + 7] * wp);
-          if (mine) *reinterpret_cast<uint4*>(orow + 8 * q4) = w;
+          if (mine) *reinterpret_cast<uint4*>(orow + half * 32 + 8 * q4) = w;
         }
-        tc::fence_before_sync();
-        __syncwarp();
-        if (lane == 0) tma::mbar_arrive(&bars.o_free);
       }
-      // both groups read the fine lse above; group 0 replaces it only after both have (second exchange barrier)
-      if (wg == 0 && mine) a.lse[(int64_t) bh * a.Nq + row] = lse_out;
-      if (!ok) break;
+      if (mine) *lse_p = (Lm + log2f(ef + ep)) * 0.6931471805599453f;
     }
   }
   if (abort_flag->abort) tc::abort_drain();

@@ -65,6 +65,18 @@ __device__ __forceinline__ bool bounded_wait(uint64_t* bar, uint32_t parity, vol
   c->abort = 1;
   return false;
 }
+// The same by a whole warp in step: lane l waits for bars[l]'s phase (several barriers at the price of one: the test is one instruction
+// whatever addresses its lanes bring), and the answer is the same in every lane, which keeps the control flow around it uniform.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile WaitCtl* c) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const int limit = c->limit;
+  for (int i = 0; i < limit; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 1023) == 1023 && __any_sync(0xffffffffu, c->abort != 0)) return false;
+  }
+  c->abort = 1;
+  return false;
+}
 // After an abort: a fixed, bounded pause (about 60 microseconds) in which bulk copies and tensor-core instructions
 // this CTA has already issued complete, before its shared and tensor memory are given back.
 __device__ __forceinline__ void abort_drain() {
@@ -123,6 +135,112 @@ __device__ __forceinline__ void umma_ss_lh(uint32_t tmem_d, uint32_t a_lo, uint3
       :
       : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(ACC), "r"(0u)
       : "memory");
+}
+// ---- issue by a warp in step: every lane executes the statement, elect.sync picks the lane that issues.  tcgen05.mma takes its
+// descriptors from uniform registers and is issued once per executing thread; where the compiler sees an elected thread in uniform control
+// flow the descriptors stay there, where it sees `if (lane == 0)` every instruction costs some 98 cycles of moves, whatever its size, and
+// issuing, not the tensor pipe, is the pace of a kernel whose products have N = 64.
+// One statement issues all k-steps of a tile, 16 elements of K each.
+// A, B in shared memory, both K-major (32 bytes per k-step), K = 64: D = A . B
+__device__ __forceinline__ void umma_ss_k64(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred f, t, e;\n\t.reg .b32 al, bl;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 f, %6, 0; setp.eq.b32 t, %6, 0;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "add.u32 al, %1, 0; add.u32 bl, %3, 0;\n\t"
+      "mov.b64 da, {al, %2}; mov.b64 db, {bl, %4};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %6, %6, %6}, f;\n\t"
+      "add.u32 al, %1, 2; add.u32 bl, %3, 2;\n\t"
+      "mov.b64 da, {al, %2}; mov.b64 db, {bl, %4};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 4; add.u32 bl, %3, 4;\n\t"
+      "mov.b64 da, {al, %2}; mov.b64 db, {bl, %4};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 6; add.u32 bl, %3, 6;\n\t"
+      "mov.b64 da, {al, %2}; mov.b64 db, {bl, %4};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %6, %6, %6}, t;\n\t"
+      "}"
+      :
+      : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(0u)
+      : "memory");
+}
+// A in tensor memory (two K values per column), B in shared memory and MN-major (16 rows of 128 bytes per k-step): D (+)= A . B, K = 32, 64
+// or 128; `accumulate` is for the first k-step
+__device__ __forceinline__ void umma_ts_k32(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, t, e;\n\t.reg .b32 al, bl;\n\t.reg .b64 db;\n\t"
+      "setp.ne.b32 p, %5, 0; setp.eq.b32 t, %6, 0;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "add.u32 al, %1, 0; add.u32 bl, %2, 0;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, p;\n\t"
+      "add.u32 al, %1, 8; add.u32 bl, %2, 128;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "}"
+      :
+      : "r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts_k64(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, t, e;\n\t.reg .b32 al, bl;\n\t.reg .b64 db;\n\t"
+      "setp.ne.b32 p, %5, 0; setp.eq.b32 t, %6, 0;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "add.u32 al, %1, 0; add.u32 bl, %2, 0;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, p;\n\t"
+      "add.u32 al, %1, 8; add.u32 bl, %2, 128;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 16; add.u32 bl, %2, 256;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 24; add.u32 bl, %2, 384;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "}"
+      :
+      : "r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts_k128(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, t, e;\n\t.reg .b32 al, bl;\n\t.reg .b64 db;\n\t"
+      "setp.ne.b32 p, %5, 0; setp.eq.b32 t, %6, 0;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "add.u32 al, %1, 0; add.u32 bl, %2, 0;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, p;\n\t"
+      "add.u32 al, %1, 8; add.u32 bl, %2, 128;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 16; add.u32 bl, %2, 256;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 24; add.u32 bl, %2, 384;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 32; add.u32 bl, %2, 512;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 40; add.u32 bl, %2, 640;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 48; add.u32 bl, %2, 768;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "add.u32 al, %1, 56; add.u32 bl, %2, 896;\n\t"
+      "mov.b64 db, {bl, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [al], db, %4, {%6, %6, %6, %6}, t;\n\t"
+      "}"
+      :
+      : "r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_w(uint64_t* bar) {
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+               "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
 }
 // Runtime accumulate flag.
 __device__ __forceinline__ void umma_ss_lh(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
