@@ -5,7 +5,8 @@
 // Per tile of 128 query rows and per chunk c of its pooled keys:
 //     S  = Q  . K_c^T   [128 x 64]  (K = 64 channels)        shared-memory operands
 //     dP = dO . V_c^T   [128 x 64]
-//     dS = exp2(S*scale*log2e + log2 w - lse) * (dP - delta) * scale      softmax warps, thread = query row
+//     dS = exp2(S*scale*log2e + log2 w - lse) * (dP - delta)              softmax warps, thread = query row; the scale (a power of two)
+//                                                                         is applied to dQ
 //     dQ += dS . K_c    [128 x 64]  (K = 64 keys)             dS read from TENSOR MEMORY (packed bf16 over S), K_c MN-major
 // Two levels: first the gathered level-1 blocks (four to a chunk), then the level-2 keys.  Either list may end inside a chunk (at 32 keys):
 // what is loaded behind its end is neither exponentiated nor multiplied.
@@ -222,10 +223,12 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
     if (n_my > 0) fetch(0);
     bool ok = true;
     for (int i = 0; ok && i < n_my; ++i) {
-      const float L = lse_next * kLog2eF, dls = delta_next * a.scale;
+      const float L = lse_next * kLog2eF;
+      const F2 nd2 = f2(-delta_next, -delta_next), sl22 = f2(sl2, sl2);
       if (i + 1 < n_my) fetch(i + 1);
       for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
         const float off = ((j < gathered || !a.two_level) ? lw1 : lw2) - L;
+        const F2 off2 = f2(off, off);
         const int halves = keys_of(j) / 32;
         ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.sdp_ready[buf], bph, abort_flag));
         tc::fence_after_sync();
@@ -241,8 +244,10 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
           uint32_t pk[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            const float p0 = fast_exp2(fmaf(vs[2 * e], sl2, off)), p1 = fast_exp2(fmaf(vs[2 * e + 1], sl2, off));
-            pk[e] = pack_bf16(p0 * fmaf(vd[2 * e], a.scale, -dls), p1 * fmaf(vd[2 * e + 1], a.scale, -dls));
+            float x0, x1;
+            f2_get(f2_fma(f2(vs[2 * e], vs[2 * e + 1]), sl22, off2), x0, x1);
+            f2_get(f2_mul(f2(fast_exp2(x0), fast_exp2(x1)), f2_add(f2(vd[2 * e], vd[2 * e + 1]), nd2)), x0, x1);
+            pk[e] = pack_bf16(x0, x1);
           }
           tc::tmem_st16(t_b + 16 * half, pk);          // dS columns [16 half, 16 half + 16) over S columns read before
         }
@@ -282,10 +287,10 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
         for (int q4 = 0; q4 < 4; ++q4) {
           const uint4 f = old[half * 4 + q4];
           uint4 w;
-          w.x = pack_bf16(bf16_lo(f.x) + v[8 * q4], bf16_hi(f.x) + v[8 * q4 + 1]);
-          w.y = pack_bf16(bf16_lo(f.y) + v[8 * q4 + 2], bf16_hi(f.y) + v[8 * q4 + 3]);
-          w.z = pack_bf16(bf16_lo(f.z) + v[8 * q4 + 4], bf16_hi(f.z) + v[8 * q4 + 5]);
-          w.w = pack_bf16(bf16_lo(f.w) + v[8 * q4 + 6], bf16_hi(f.w) + v[8 * q4 + 7]);
+          w.x = pack_bf16(fmaf(v[8 * q4], a.scale, bf16_lo(f.x)), fmaf(v[8 * q4 + 1], a.scale, bf16_hi(f.x)));
+          w.y = pack_bf16(fmaf(v[8 * q4 + 2], a.scale, bf16_lo(f.y)), fmaf(v[8 * q4 + 3], a.scale, bf16_hi(f.y)));
+          w.z = pack_bf16(fmaf(v[8 * q4 + 4], a.scale, bf16_lo(f.z)), fmaf(v[8 * q4 + 5], a.scale, bf16_hi(f.z)));
+          w.w = pack_bf16(fmaf(v[8 * q4 + 6], a.scale, bf16_lo(f.w)), fmaf(v[8 * q4 + 7], a.scale, bf16_hi(f.w)));
           *reinterpret_cast<uint4*>(dqrow + half * 32 + 8 * q4) = w;
         }
       }

@@ -8,7 +8,8 @@
 // meet it, walked 64 at a time (a job):
 //     S^T  = K_c . Q_t^T   [128 keys x 64 queries]  (K = 64 channels)   shared-memory operands
 //     dP^T = V_c . dO_t^T  [128 x 64]
-//     P^T  = exp2(S^T*scale*log2e + log2 w - lse[q]),  dS^T = P^T * (dP^T - delta[q]) * scale     thread = key row;
+//     P^T  = exp2(S^T*scale*log2e + log2 w - lse[q]),  dS^T = P^T * (dP^T - delta[q])     thread = key row; the scale
+//            (a power of two) is applied to dK;
 //            lse and delta of the 64 query columns sit in shared memory next to the Q / dO tile
 //     dV_c += P^T  . dO_t  [128 x 64]  (K = 64 queries)   P^T, dS^T read from TENSOR MEMORY (packed bf16, written over
 //     dK_c += dS^T . Q_t                                   S^T / dP^T), dO_t / Q_t as MN-major operands (the same tiles)
@@ -231,6 +232,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
     int buf = wg;                                  // buffer of this group's next job and the phase parity of its barriers
     uint32_t bph = 0;
     float vs[32], vd[32];
+    const F2 sl22 = f2(sl2, sl2), nlog2e2 = f2(-kLog2eF, -kLog2eF), lw2 = f2(lw_log2, lw_log2), minus1 = f2(-1.f, -1.f);
     for (int64_t jn = wg; jn < total; jn += 2) {
       const int st = (int) jn & (kStages - 1);
       const bool ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.sdp_ready[buf], bph, abort_flag));
@@ -248,14 +250,18 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
         for (int q4 = 0; q4 < 8; ++q4) {           // 4 query columns at a time: their lse / delta are broadcast reads
           const float4 l4 = *reinterpret_cast<const float4*>(&s_lse[st][32 * half + 4 * q4]);
           const float4 d4 = *reinterpret_cast<const float4*>(&s_delta[st][32 * half + 4 * q4]);
-          const float p0 = fast_exp2(fmaf(vs[4 * q4], sl2, fmaf(l4.x, -kLog2eF, lw_log2)));
-          const float p1 = fast_exp2(fmaf(vs[4 * q4 + 1], sl2, fmaf(l4.y, -kLog2eF, lw_log2)));
-          const float p2 = fast_exp2(fmaf(vs[4 * q4 + 2], sl2, fmaf(l4.z, -kLog2eF, lw_log2)));
-          const float p3 = fast_exp2(fmaf(vs[4 * q4 + 3], sl2, fmaf(l4.w, -kLog2eF, lw_log2)));
-          pp[2 * q4] = pack_bf16(p0, p1);
-          pp[2 * q4 + 1] = pack_bf16(p2, p3);
-          pd[2 * q4] = pack_bf16(p0 * ((vd[4 * q4] - d4.x) * a.scale), p1 * ((vd[4 * q4 + 1] - d4.y) * a.scale));
-          pd[2 * q4 + 1] = pack_bf16(p2 * ((vd[4 * q4 + 2] - d4.z) * a.scale), p3 * ((vd[4 * q4 + 3] - d4.w) * a.scale));
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const F2 l2 = e ? f2(l4.z, l4.w) : f2(l4.x, l4.y), d2 = e ? f2(d4.z, d4.w) : f2(d4.x, d4.y);
+            const int k = 4 * q4 + 2 * e;
+            float x0, x1;
+            f2_get(f2_fma(f2(vs[k], vs[k + 1]), sl22, f2_fma(l2, nlog2e2, lw2)), x0, x1);
+            x0 = fast_exp2(x0);
+            x1 = fast_exp2(x1);
+            pp[2 * q4 + e] = pack_bf16(x0, x1);
+            f2_get(f2_mul(f2(x0, x1), f2_fma(d2, minus1, f2(vd[k], vd[k + 1]))), x0, x1);
+            pd[2 * q4 + e] = pack_bf16(x0, x1);
+          }
         }
         tc::tmem_st16(t_b + 16 * half, pp);            // P^T over S^T columns read before
         tc::tmem_st16(t_b + 64 + 16 * half, pd);       // dS^T over dP^T columns read before
@@ -300,15 +306,16 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
           __syncwarp();
           if (lane == 0) tma::mbar_arrive(&bars.acc_free[i % kAccs]);
         }
+        const float mul = part < 2 ? out_mul : out_mul * a.scale;
         float* dst = (part < 2 ? dpv : dpk) + ((int64_t) bh * n_keys + key) * kD + (part & 1) * 32;
         if (!live) {
         } else if (whole) {
 #pragma unroll
           for (int q4 = 0; q4 < 8; ++q4)
-            *reinterpret_cast<float4*>(dst + 4 * q4) = make_float4(v[4 * q4] * out_mul, v[4 * q4 + 1] * out_mul, v[4 * q4 + 2] * out_mul, v[4 * q4 + 3] * out_mul);
+            *reinterpret_cast<float4*>(dst + 4 * q4) = make_float4(v[4 * q4] * mul, v[4 * q4 + 1] * mul, v[4 * q4 + 2] * mul, v[4 * q4 + 3] * mul);
         } else {
 #pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4) red_add_v4(dst + 4 * q4, v[4 * q4] * out_mul, v[4 * q4 + 1] * out_mul, v[4 * q4 + 2] * out_mul, v[4 * q4 + 3] * out_mul);
+          for (int q4 = 0; q4 < 8; ++q4) red_add_v4(dst + 4 * q4, v[4 * q4] * mul, v[4 * q4 + 1] * mul, v[4 * q4 + 2] * mul, v[4 * q4 + 3] * mul);
         }
       }
     }

@@ -254,7 +254,8 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
     bool ok = true;
     for (int i = 0; ok && i < n_my; ++i) {
       // one pass: the fine part's log-sum-exp is the reference of the exponentials
-      float mx = n_pass == 1 ? lse_next * kLog2eF : -INFINITY, lsum = 0.f;
+      float mx = n_pass == 1 ? lse_next * kLog2eF : -INFINITY;
+      F2 sum[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};      // four running sums: a chain of adds per element is a third of a job
       if (n_pass == 1 && i + 1 < n_my) lse_next = lse_of(i + 1);
       bool exchanged = n_pass == 1;
       // two passes: the groups exchange their row maxima once per tile, before their first pass-2 job (a group may have none); a copy is
@@ -288,7 +289,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           }
           mx = fmaxf(mx, fmaf(m, sl2, lw));
         } else {
-          const float off = lw - mx;
+          const F2 sl22 = f2(sl2, sl2), off2 = f2(lw - mx, lw - mx);
 #pragma unroll 1          // unrolled, the four quarters' registers overlap and spill (to L2: L1 is 28 KB here)
           for (int q4 = 0; q4 < nq; ++q4) {
             tc::tmem_ld32_async(t_s + 32 * q4, va);
@@ -296,9 +297,12 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
             uint32_t pk[16];
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
-              const float e0 = fast_exp2(fmaf(va[2 * e], sl2, off)), e1 = fast_exp2(fmaf(va[2 * e + 1], sl2, off));
-              lsum += e0 + e1;
-              pk[e] = pack_bf16(e0, e1);
+              float x0, x1;
+              f2_get(f2_fma(f2(va[2 * e], va[2 * e + 1]), sl22, off2), x0, x1);
+              x0 = fast_exp2(x0);
+              x1 = fast_exp2(x1);
+              sum[e & 1] = f2_add(sum[e & 1], f2(x0, x1));
+              pk[e] = pack_bf16(x0, x1);
             }
             tc::tmem_st16(t_s + 16 * q4, pk);          // P columns [16 q4, 16 q4 + 16): scores read before
           }
@@ -314,7 +318,9 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       // the sums of the tile before the last have been read
       if (ok && i > 1) ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_free[i & 1], ((uint32_t) (i - 2) >> 1) & 1, abort_flag));
       if (!ok) break;
-      s_sum[i & 1][wg][r] = lsum;
+      float l0, l1;
+      f2_get(f2_add(sum[0], sum[1]), l0, l1);
+      s_sum[i & 1][wg][r] = l0 + l1;
       if (wg == 0) s_ref[i & 1][r] = mx;
       __syncwarp();
       if (lane == 0) tma::mbar_arrive(&bars.sum_ready[i & 1]);
