@@ -28,10 +28,14 @@
 //                          backward (dk += (dpk[j] + dpk2[j/16]/16)/16), one bf16 store.
 // The reference multiplies k by scale into new tensors first (res_1.py:420-422);
 // here scale rides in the exp2 argument and in the epilogues.
+#include <string.h>
+
 #include <type_traits>
 
 #include "attn.cuh"
 #include "mma_frag.cuh"
+#include "tc05.cuh"
+#include "tma.cuh"
 
 namespace llsa {
 
@@ -468,10 +472,30 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 //   * The pooled-gradient rows a finished tile folds in (the pooling backward) are requested into registers when
 //     the bucket begins and parked in shared memory right before the store.
 // Accumulator layout (ldmatrix): tile u holds channels 8u + 2t, 8u + 2t + 1 of keys g (c0, c1) and g + 8 (c2, c3).
-constexpr int kRingWarps = 4;                   // warps per CTA, each on its own range; two CTAs per SM
-constexpr int kRingFineStages = 4;
-constexpr int kRingFineStageBytes = 2 * kRingTileElems * (int) sizeof(bf16);           // Q tile, dO tile
+constexpr int kRingWarps = 4;                   // warps per CTA
+constexpr int kRingFineStages = 3;
+constexpr int kRingTileBytes = kRingTileElems * (int) sizeof(bf16);
+constexpr int kRingFineStageBytes = 2 * kRingTileBytes + 1024;                         // Q tile, dO tile, P^T and dS^T registers
 constexpr int kRingFoldBytes = 4 * 64 * (int) sizeof(float);                           // per warp: dpk, dpv, dpk2, dpv2 rows of the bucket
+constexpr int kRingWarpBytes = kRingFineStages * kRingFineStageBytes + kRingFoldBytes;
+constexpr int kRingWindow = 64;                 // nominal entries per window: the unit whose cut buckets meet in the `partial` scratch
+
+struct FineMaps {
+  CUtensorMap q, d_o;          // [B,H,Nq,64] 4-D, box 16 rows
+};
+// One lane requests an entry: Q tile, dO tile and the kilobyte of P^T / dS^T, all counted by one barrier.
+__device__ __forceinline__ void load_entry_w(uint32_t dst, const FineMaps& m, const uint4* pds, uint64_t* bar, int row, int h, int b) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t.reg .b32 d, p;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "add.u32 d, %0, 2048; add.u32 p, %0, 4096;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], 5120;\n\t"
+      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%8, %5, %6, %7}], [%4];\n\t"
+      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [d], [%2, {%8, %5, %6, %7}], [%4];\n\t"
+      "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [p], [%3], 1024, [%4];\n\t"
+      "}" ::"r"(dst), "l"(&m.q), "l"(&m.d_o), "l"(pds), "r"(tc::smem_u32(bar)), "r"(row), "r"(h), "r"(b), "r"(0)
+      : "memory");
+}
 
 // Pooling-backward fold and scale for the ldmatrix accumulator layout: afterwards dk / dv hold the final fp32 values.
 // The four gradient rows of KV block j come from this warp's copy in shared memory ([dpk | dpv | dpk2 | dpv2] x 64 fp32, fetched with
@@ -511,81 +535,72 @@ __device__ __forceinline__ void dkv_fine_fold_smem(const AttnP<bf16>& a, uint32_
   }
 }
 
-// The staging half of the store below: dk / dv already hold the final fp32 values.
-template <int SB>
-__device__ __forceinline__ void dkv_tile_store_staged(const AttnP<bf16>& a, int64_t b, int64_t h, int64_t j, float (&dk)[8][4], float (&dv)[8][4],
-                                                      const uint32_t (&sa_m)[4], uint32_t sa_cp0, uint32_t sa_cp1, int lane) {
-  constexpr int TB = kRingTileElems * (int) sizeof(bf16);
+// Store of a finished tile through a free ring stage (`so` bytes into the ring): stmatrix writes the bf16 tile in the ring's swizzled row
+// layout (the ldmatrix addresses sa_m), every lane reads back four 16-byte chunks per tensor (sa_cp: rows (lane/8) + {0, 4, 8, 12}) and
+// eight lanes write one whole 128-byte row: full sectors, 8 store instructions instead of 32.
+__device__ __forceinline__ void dkv_fine_store_staged(const AttnP<bf16>& a, int64_t b, int64_t h, int64_t j, float (&dk)[8][4],
+                                                      float (&dv)[8][4], const uint32_t (&sa_m)[4], uint32_t sa_cp, uint32_t so,
+                                                      uint32_t sa_fold, int lane) {
+  constexpr int TB = kRingTileBytes;
+  dkv_fine_fold_smem(a, sa_fold, dk, dv);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    stsm_x4<SB>(sa_m[c], pack_bf16(dk[2 * c][0], dk[2 * c][1]), pack_bf16(dk[2 * c][2], dk[2 * c][3]),
-                pack_bf16(dk[2 * c + 1][0], dk[2 * c + 1][1]), pack_bf16(dk[2 * c + 1][2], dk[2 * c + 1][3]));
-    stsm_x4<SB + TB>(sa_m[c], pack_bf16(dv[2 * c][0], dv[2 * c][1]), pack_bf16(dv[2 * c][2], dv[2 * c][3]),
-                     pack_bf16(dv[2 * c + 1][0], dv[2 * c + 1][1]), pack_bf16(dv[2 * c + 1][2], dv[2 * c + 1][3]));
+    stsm_x4<0>(sa_m[c] + so, pack_bf16(dk[2 * c][0], dk[2 * c][1]), pack_bf16(dk[2 * c][2], dk[2 * c][3]),
+               pack_bf16(dk[2 * c + 1][0], dk[2 * c + 1][1]), pack_bf16(dk[2 * c + 1][2], dk[2 * c + 1][3]));
+    stsm_x4<TB>(sa_m[c] + so, pack_bf16(dv[2 * c][0], dv[2 * c][1]), pack_bf16(dv[2 * c][2], dv[2 * c][3]),
+                pack_bf16(dv[2 * c + 1][0], dv[2 * c + 1][1]), pack_bf16(dv[2 * c + 1][2], dv[2 * c + 1][3]));
   }
   __syncwarp();
+  const uint32_t sa_cp0 = sa_cp + so, sa_cp1 = (sa_cp ^ 64) + so;
   bf16* kp = a.dk.row(b, h, j * kBS + (lane >> 3)) + (lane & 7) * 8;
   bf16* vp = a.dv.row(b, h, j * kBS + (lane >> 3)) + (lane & 7) * 8;
   const int64_t ks = 4 * a.dk.sn, vs = 4 * a.dv.sn;
   uint4 x;
-  lds128<SB>(x.x, x.y, x.z, x.w, sa_cp0);             *reinterpret_cast<uint4*>(kp) = x;
-  lds128<SB + 512>(x.x, x.y, x.z, x.w, sa_cp1);       *reinterpret_cast<uint4*>(kp + ks) = x;
-  lds128<SB + 1024>(x.x, x.y, x.z, x.w, sa_cp0);      *reinterpret_cast<uint4*>(kp + 2 * ks) = x;
-  lds128<SB + 1536>(x.x, x.y, x.z, x.w, sa_cp1);      *reinterpret_cast<uint4*>(kp + 3 * ks) = x;
-  lds128<SB + TB>(x.x, x.y, x.z, x.w, sa_cp0);        *reinterpret_cast<uint4*>(vp) = x;
-  lds128<SB + TB + 512>(x.x, x.y, x.z, x.w, sa_cp1);  *reinterpret_cast<uint4*>(vp + vs) = x;
-  lds128<SB + TB + 1024>(x.x, x.y, x.z, x.w, sa_cp0); *reinterpret_cast<uint4*>(vp + 2 * vs) = x;
-  lds128<SB + TB + 1536>(x.x, x.y, x.z, x.w, sa_cp1); *reinterpret_cast<uint4*>(vp + 3 * vs) = x;
+  lds128<0>(x.x, x.y, x.z, x.w, sa_cp0);         *reinterpret_cast<uint4*>(kp) = x;
+  lds128<512>(x.x, x.y, x.z, x.w, sa_cp1);       *reinterpret_cast<uint4*>(kp + ks) = x;
+  lds128<1024>(x.x, x.y, x.z, x.w, sa_cp0);      *reinterpret_cast<uint4*>(kp + 2 * ks) = x;
+  lds128<1536>(x.x, x.y, x.z, x.w, sa_cp1);      *reinterpret_cast<uint4*>(kp + 3 * ks) = x;
+  lds128<TB>(x.x, x.y, x.z, x.w, sa_cp0);        *reinterpret_cast<uint4*>(vp) = x;
+  lds128<TB + 512>(x.x, x.y, x.z, x.w, sa_cp1);  *reinterpret_cast<uint4*>(vp + vs) = x;
+  lds128<TB + 1024>(x.x, x.y, x.z, x.w, sa_cp0); *reinterpret_cast<uint4*>(vp + 2 * vs) = x;
+  lds128<TB + 1536>(x.x, x.y, x.z, x.w, sa_cp1); *reinterpret_cast<uint4*>(vp + 3 * vs) = x;
   __syncwarp();
+  tc::fence_async_smem();                 // the stage is refilled by the asynchronous proxy
 }
 
-
-// Store of a finished tile through a free ring stage at byte offset SB: stmatrix writes the bf16 tile in the ring's swizzled row
-// layout (the ldmatrix addresses sa_m), every lane reads back four 16-byte chunks per tensor (the cp.async addresses sa_cp0 /
-// sa_cp1) and eight lanes write one whole 128-byte row: full sectors, 8 store instructions instead of 32.
-template <int SB>
-__device__ __forceinline__ void dkv_fine_store_staged(const AttnP<bf16>& a, int64_t b, int64_t h, int64_t j, float (&dk)[8][4],
-                                                      float (&dv)[8][4], const uint32_t (&sa_m)[4], uint32_t sa_cp0, uint32_t sa_cp1,
-                                                      uint32_t sa_fold, int lane) {
-  dkv_fine_fold_smem(a, sa_fold, dk, dv);
-  dkv_tile_store_staged<SB>(a, b, h, j, dk, dv, sa_m, sa_cp0, sa_cp1, lane);
-}
-__global__ void __launch_bounds__(kRingWarps * 32, 2) attn_dkv_fine_ring_kernel(AttnP<bf16> a, float* __restrict__ partial) {
+template <bool PERSISTENT>
+__global__ void __launch_bounds__(kRingWarps * 32, PERSISTENT ? 3 : 2)
+attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, float* __restrict__ partial, int n_windows, int64_t n_total) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t s_full[kRingWarps][kRingFineStages];
+  __shared__ tc::WaitCtl s_ctl;
+  __shared__ int s_head_bucket[kRingWarps];
+  // swizzled tiles: 1024-byte aligned
+  unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
+  float* slots = reinterpret_cast<float*>(smem + kRingWarps * kRingWarpBytes);   // !PERSISTENT: [kRingWarps][kTileFloats], tile of the bucket a warp shares with earlier warps
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
+  volatile tc::WaitCtl* ctl = &s_ctl;
+  if (threadIdx.x == 0) {
+    s_ctl.abort = 0;
+    s_ctl.limit = a.wait_limit > 0 ? a.wait_limit : tc::kWaitPolls;
+  }
+  if (threadIdx.x < kRingWarps) s_head_bucket[threadIdx.x] = -1;
+  if (threadIdx.x < kRingWarps * kRingFineStages) tc::mbar_init(&s_full[0][0] + threadIdx.x, 1);
+  tc::fence_mbar_init();
   pdl_trigger();
   pdl_wait();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  // the swizzle arithmetic below works on absolute shared addresses: start at a 128-byte boundary (the launch adds 128 bytes)
-  unsigned char* smem = smem_raw + ((128u - ((uint32_t) __cvta_generic_to_shared(smem_raw) & 127u)) & 127u);
-  float* slots = reinterpret_cast<float*>(smem);            // [kRingWarps][kTileFloats]: tile of the bucket a warp shares with earlier warps
-  __shared__ int s_head_bucket[kRingWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
-  // per warp: the ring stages, then its copy of the pooled-gradient rows the current bucket folds in (4 rows x 256 bytes)
-  constexpr int kWarpBytes = kRingFineStages * kRingFineStageBytes + kRingFoldBytes;
-  constexpr int kFoldOff = kRingFineStages * kRingFineStageBytes;
-  unsigned char* ring = smem + kRingWarps * kTileFloats * sizeof(float) + warp * kWarpBytes;
-  const int64_t bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
-  const int E = (int) (a.nq1 * a.topk), n1 = (int) a.n1;
-  const int R = (E + a.range_entries - 1) / a.range_entries;
-  // entries the CSR really holds: fewer than E when the transpose dropped out-of-range indices; ranges and offsets handed in
-  // by a caller are not trusted further than these clamps and the bounds on the bucket walk below
-  const int E_used = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1)));
-  auto cut = [&](int r) { return r < R ? min(max(__ldcg(&a.ranges[bh * R + r].x), 0), E_used) : E_used; };
-  const int r = blockIdx.x * kRingWarps + warp;           // this warp's range; the CTA's window is its four ranges
-  const int cb = cut(blockIdx.x * kRingWarps), ce = max(cut((blockIdx.x + 1) * kRingWarps), cb);
-  const int rb = min(max(cut(r), cb), ce), re = min(max(cut(r + 1), rb), ce);
-  const int32_t* fl = a.flat + bh * (int64_t) E;
-  const int32_t* pr = a.pairs + bh * (int64_t) E;
-  if (threadIdx.x < kRingWarps) s_head_bucket[threadIdx.x] = -1;
   __syncthreads();
 
-  // Per-lane shared addresses, computed once (the ring is 128-byte aligned, so the chunk index of an address is its bits 4..6
-  // and a swizzle partner is one XOR away):
-  //   sa_cp0 / sa_cp1  where this lane's cp.async chunks of tile rows (lane/8) + {0, 8} / + {4, 12} land
-  //   sa_m[c]          ldmatrix.trans row address for output channels 16c..16c+15
-  const uint32_t ring_sa = (uint32_t) __cvta_generic_to_shared(ring);
-  const uint32_t sa_t8 = ring_sa + 8 * t, sa_l16 = ring_sa + lane * 16;      // + immediates: gradient rows
-  const uint32_t sa_fold = sa_t8 + kFoldOff;
-  const uint32_t sa_cp0 = ring_sa + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4), sa_cp1 = sa_cp0 ^ 64;
+  const int E = (int) (a.nq1 * a.topk), n1 = (int) a.n1;
+  const int R = (E + a.range_entries - 1) / a.range_entries;
+  // Per-lane shared addresses of stage 0, computed once (tiles are 1024-byte aligned, so the chunk index of an address is its bits
+  // 4..6 and a swizzle partner is one XOR away):
+  //   sa_cp    16-byte chunk lane % 8 of tile rows lane / 8 and lane / 8 + 8 (^ 64: + 4, + 12)
+  //   sa_m[c]  ldmatrix.trans row address for output channels 16c..16c+15
+  const uint32_t ring_sa = tc::smem_u32(smem + warp * kRingWarpBytes), sa_l16 = ring_sa + lane * 16;
+  constexpr int kFoldOff = kRingFineStages * kRingFineStageBytes;
+  const uint32_t sa_fold = ring_sa + 8 * t + kFoldOff;
+  const uint32_t sa_cp = ring_sa + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4);
   uint32_t sa_m[4];
   {
     const int lr = (lane & 7) + ((lane >> 3) & 1) * 8;
@@ -594,28 +609,52 @@ __global__ void __launch_bounds__(kRingWarps * 32, 2) attn_dkv_fine_ring_kernel(
     for (int c = 0; c < 4; ++c) sa_m[c] = base ^ (c << 5);
   }
   float dk[8][4], dv[8][4];
-  int tail_j = -1;                          // bucket whose tile is still in dk / dv after the loop
-  if (rb < re) {
-    const int n = min(re - rb, 4 * 32);     // entries of this warp: 1..127 for ranges cut by the transpose kernel
-    // lane i: query block and pair number of entries rb + i, rb + 32 + i, ... (clamped: nothing is read outside the tensors);
-    // requested first, they arrive while the bucket offsets below are being fetched
-    int my_qb[4] = {0, 0, 0, 0}, my_pair[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (lane + 32 * u < n) {
-        my_qb[u] = __ldcg(fl + rb + 32 * u + lane);
-        my_pair[u] = __ldcg(pr + rb + 32 * u + lane);
+  int tail_j = -1;                          // !PERSISTENT: bucket whose tile is still in dk / dv after the loop
+  int st = 0, ph = 0;                       // ring stage of the entry at hand, parity of its fill
+  int64_t bh = blockIdx.y;
+  int ce = 0;
+  // entries the CSR really holds: fewer than E when the transpose dropped out-of-range indices; ranges and offsets handed in
+  // by a caller are not trusted further than these clamps and the bounds on the bucket walk below
+  auto cut = [&](int r, int used) { return r < R ? min(max(__ldcg(&a.ranges[bh * R + r].x), 0), used) : used; };
+  // a span: PERSISTENT one window (two ranges) after another per warp, otherwise one range per warp and one window per CTA
+  bool ok = true;
+  for (int64_t w = PERSISTENT ? (int64_t) warp * gridDim.x + blockIdx.x : 0; ok && w < (PERSISTENT ? n_total : 1); w += PERSISTENT ? (int64_t) kRingWarps * gridDim.x : 1) {
+    int r0, rb, re;
+    if (PERSISTENT) bh = w / n_windows;
+    const int E_used = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1)));
+    const int win = PERSISTENT ? (int) (w % n_windows) : (int) blockIdx.x;
+    if (PERSISTENT) {
+      r0 = win * (kRingWindow / kRangeEntries);
+      rb = cut(r0, E_used);
+      re = max(cut(r0 + kRingWindow / kRangeEntries, E_used), rb);
+    } else {
+      r0 = win * kRingWarps + warp;
+      const int cb = cut(win * kRingWarps, E_used);
+      ce = max(cut((win + 1) * kRingWarps, E_used), cb);
+      rb = min(max(cut(r0, E_used), cb), ce);
+      re = min(max(cut(r0 + 1, E_used), rb), ce);
+    }
+    if (rb >= re) continue;
+    const int64_t b = bh / a.H, h = bh % a.H;
+    float* const pieces = partial + (bh * n_windows + win) * 2 * (int64_t) kTileFloats;     // the window's head and tail slots
+    const int32_t* fl = a.flat + bh * (int64_t) E;
+    const int32_t* pr = a.pairs + bh * (int64_t) E;
+    const int n = re - rb;
+    // lane i: query block and pair number of entry 32 c + i of the chunk c being requested and of the one after it (clamped: nothing is
+    // read outside the tensors)
+    int cur_qb = 0, cur_pair = 0, nx_qb = 0, nx_pair = 0;
+    auto fetch = [&](int i0) {
+      if (i0 + lane < n) {
+        nx_qb = min(max(__ldcg(fl + rb + i0 + lane), 0), (int) a.nq1 - 1);
+        nx_pair = min(max(__ldcg(pr + rb + i0 + lane), 0), E - 1);
       }
+    };
+    fetch(0);
     // first bucket of the range (handed over by the transpose kernel; clamped, and moved on if it does not hold rb)
-    int j = min(max(__ldcg(&a.ranges[bh * R + r].y), 0), n1 - 1);
+    int j = min(max(__ldcg(&a.ranges[bh * R + r0].y), 0), n1 - 1);
     int bo = (int) csr_off(a, bh, j), nxt = (int) csr_off(a, bh, j + 1);
     while (nxt <= rb && j + 1 < n1) { ++j; bo = nxt; nxt = (int) csr_off(a, bh, j + 1); }
     int nxt2 = j + 2 <= n1 ? (int) csr_off(a, bh, j + 2) : 0x7fffffff;      // one bucket ahead: no load to wait for at a switch
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      my_qb[u] = my_qb[u] < 0 ? 0 : (my_qb[u] >= (int) a.nq1 ? (int) a.nq1 - 1 : my_qb[u]);
-      my_pair[u] = my_pair[u] < 0 ? 0 : (my_pair[u] >= E ? E - 1 : my_pair[u]);
-    }
     // the pooled-gradient rows the bucket's store folds in: lanes 0..15 hold the dpk row, lanes 16..31 the dpv row (16 bytes each)
     uint4 f1 = make_uint4(0u, 0u, 0u, 0u), f2 = make_uint4(0u, 0u, 0u, 0u);
     auto load_fold = [&](int jj) {
@@ -631,80 +670,39 @@ __global__ void __launch_bounds__(kRingWarps * 32, 2) attn_dkv_fine_ring_kernel(
       }
       __syncwarp();
     };
-    // global side: row (lane/8), chunk (lane%8) of block 0; a block is qblk / dblk bytes further, four rows qstep / dstep bytes
-    const char* q_lane = reinterpret_cast<const char*>(a.q.row(b, h, lane >> 3) + (lane & 7) * 8);
-    const char* d_lane = reinterpret_cast<const char*>(a.d_o.row(b, h, lane >> 3) + (lane & 7) * 8);
-    const int qblk = (int) (kBS * a.q.sn * sizeof(bf16)), dblk = (int) (kBS * a.d_o.sn * sizeof(bf16));
-    const int qstep = (int) (4 * a.q.sn * sizeof(bf16)), dstep = (int) (4 * a.d_o.sn * sizeof(bf16));
-    // the P / dS registers of the whole range come from HBM (the hand-over does not fit the L2): every lane pulls its own
-    // entries' 1 KB towards L2 now, so that the loads three entries ahead find them there
+    const uint4* pds = a.pds + bh * (int64_t) E * 64;
+    int rst = st;                            // ring stage of the next request
+    auto request = [&](int i) {
+      if ((i & 31) == 0) {
+        cur_qb = nx_qb;
+        cur_pair = nx_pair;
+        // the hand-over does not fit the L2: every lane pulls its own entry's kilobyte there ahead of the copies
+        if (i + lane < n) {
+          const char* pf = reinterpret_cast<const char*>(pds + (int64_t) cur_pair * 64);
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (lane + 32 * u < n) {
-        const char* pf = reinterpret_cast<const char*>(a.pds + (bh * (int64_t) E + my_pair[u]) * 64);
-#pragma unroll
-        for (int l = 0; l < 8; ++l) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf + 128 * l));
+          for (int l = 0; l < 8; ++l) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf + 128 * l));
+        }
+        fetch(i + 32);
       }
-    const uint4* pds_lane = a.pds + bh * (int64_t) E * 64 + lane;
-    uint4 pP[kRingFineStages], pD[kRingFineStages];       // P^T / dS^T registers of the entries in flight
-    // The request for entry i goes out in four parts (PART 0..3) so that the entry loop can put a part between two groups of
-    // products: address arithmetic and copies of the entry three ahead then run while the tensor pipe works on this one.
-    const char* qp_i = q_lane;
-    const char* dp_i = d_lane;
-    auto issue_part = [&](auto stage_tag, auto part_tag, int i) {
-      constexpr int ST = decltype(stage_tag)::value, PART = decltype(part_tag)::value;
-      constexpr int SB = ST * kRingFineStageBytes, TB = kRingTileElems * (int) sizeof(bf16);
-      if (PART == 0) {
-        const int u = i >> 5;
-        const int qb = __shfl_sync(0xffffffffu, u == 0 ? my_qb[0] : (u == 1 ? my_qb[1] : (u == 2 ? my_qb[2] : my_qb[3])), i & 31);
-        const int pair = __shfl_sync(0xffffffffu, u == 0 ? my_pair[0] : (u == 1 ? my_pair[1] : (u == 2 ? my_pair[2] : my_pair[3])), i & 31);
-        qp_i = q_lane + (int64_t) qb * qblk;
-        dp_i = d_lane + (int64_t) qb * dblk;
-        const uint4* pp = pds_lane + (int64_t) pair * 64;
-        pP[ST] = __ldcg(pp);
-        pD[ST] = __ldcg(pp + 32);
-      } else if (PART == 1) {
-        cp_async16_sa<SB>(sa_cp0, qp_i);
-        cp_async16_sa<SB + 512>(sa_cp1, qp_i + qstep);
-        cp_async16_sa<SB + 1024>(sa_cp0, qp_i + 2 * qstep);
-        cp_async16_sa<SB + 1536>(sa_cp1, qp_i + 3 * qstep);
-      } else if (PART == 2) {
-        cp_async16_sa<SB + TB>(sa_cp0, dp_i);
-        cp_async16_sa<SB + TB + 512>(sa_cp1, dp_i + dstep);
-      } else {
-        cp_async16_sa<SB + TB + 1024>(sa_cp0, dp_i + 2 * dstep);
-        cp_async16_sa<SB + TB + 1536>(sa_cp1, dp_i + 3 * dstep);
-      }
+      const int qb = __shfl_sync(0xffffffffu, cur_qb, i & 31), pair = __shfl_sync(0xffffffffu, cur_pair, i & 31);
+      load_entry_w(ring_sa + rst * kRingFineStageBytes, maps, pds + (int64_t) pair * 64, &s_full[warp][rst], qb * kBS, (int) h, (int) b);
+      rst = rst == kRingFineStages - 1 ? 0 : rst + 1;
     };
-    auto issue = [&](auto stage_tag, int i) {
-      issue_part(stage_tag, std::integral_constant<int, 0>{}, i);
-      issue_part(stage_tag, std::integral_constant<int, 1>{}, i);
-      issue_part(stage_tag, std::integral_constant<int, 2>{}, i);
-      issue_part(stage_tag, std::integral_constant<int, 3>{}, i);
-    };
-    static_assert(kRingFineStages == 4, "the entry loop below is unrolled over four stages");
-    if (0 < n) issue(std::integral_constant<int, 0>{}, 0);
-    cp_async_commit();
-    if (1 < n) issue(std::integral_constant<int, 1>{}, 1);
-    cp_async_commit();
-    if (2 < n) issue(std::integral_constant<int, 2>{}, 2);
-    cp_async_commit();
+    request(0);
+    if (1 < n) request(1);
     load_fold(j);
     tile_zero(dk, dv);
-    // one entry; the ring stage is a template argument so that every shared-memory offset below is an immediate
-    auto entry = [&](auto stage_tag, int i) {
-      constexpr int S = decltype(stage_tag)::value, SF = (S + kRingFineStages - 1) % kRingFineStages;    // SF: the stage read an entry ago
-      constexpr int SB = S * kRingFineStageBytes, TB = kRingTileElems * (int) sizeof(bf16);
+    for (int i = 0; i < n; ++i) {
       const int e = rb + i;
-      cp_async_wait_group<kRingFineStages - 2>();     // entry i has landed (this lane's chunks) ...
-      __syncwarp();                                   // ... and everybody else's; stage SF is free
-      if (e >= nxt && j + 1 < n1) {                   // next non-empty bucket; stage SF stages the store before it is refilled
+      const uint32_t so = st * kRingFineStageBytes;
+      if (!(ok = tc::warp_wait(&s_full[warp][st], ph, ctl))) break;
+      if (e >= nxt && j + 1 < n1) {                   // next non-empty bucket; the stage read an entry ago stages the store
         if (bo >= rb) {
           park_fold();
-          dkv_fine_store_staged<SF * kRingFineStageBytes>(a, b, h, j, dk, dv, sa_m, sa_cp0, sa_cp1, sa_fold, lane);
-        } else {
-          tile_to_mem(slots + warp * kTileFloats, dk, dv, lane);   // began in an earlier warp's range
-          if (lane == 0) s_head_bucket[warp] = j;
+          dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, rst * kRingFineStageBytes, sa_fold, lane);
+        } else {                                      // began in an earlier span
+          tile_to_mem(PERSISTENT ? pieces : slots + warp * kTileFloats, dk, dv, lane);
+          if (!PERSISTENT && lane == 0) s_head_bucket[warp] = j;
         }
         ++j; bo = nxt; nxt = nxt2;
         while (nxt <= e && j + 1 < n1) { ++j; bo = nxt; nxt = (int) csr_off(a, bh, j + 1); }      // empty buckets
@@ -712,76 +710,67 @@ __global__ void __launch_bounds__(kRingWarps * 32, 2) attn_dkv_fine_ring_kernel(
         load_fold(j);
         tile_zero(dk, dv);
       }
-      const uint4 P = pP[S], D = pD[S];
-      const bool more = i + kRingFineStages - 1 < n;
-      constexpr auto sf_tag = std::integral_constant<int, SF>{};
-      // all eight operand loads first (a product issued right behind its own load would wait out the load's latency), then
-      // the sixteen products in four groups with a part of the next request between them
-      uint32_t bd[4][4], bq[4][4];
+      // the stage read an entry ago is free: its operands were consumed by products already issued
+      if (i + kRingFineStages - 1 < n) request(i + kRingFineStages - 1);
+      uint4 P, D;
+      lds128<2 * kRingTileBytes>(P.x, P.y, P.z, P.w, sa_l16 + so);
+      lds128<2 * kRingTileBytes + 512>(D.x, D.y, D.z, D.w, sa_l16 + so);
+      uint32_t bd[4][4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) ldsm_x4_trans<SB + TB>(bd[c][0], bd[c][1], bd[c][2], bd[c][3], sa_m[c]);
+      for (int c = 0; c < 4; ++c) ldsm_x4_trans<kRingTileBytes>(bd[c][0], bd[c][1], bd[c][2], bd[c][3], sa_m[c] + so);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) ldsm_x4_trans<SB>(bq[c][0], bq[c][1], bq[c][2], bq[c][3], sa_m[c]);
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < 4; ++c) {
+        uint32_t bq[4];
+        ldsm_x4_trans<0>(bq[0], bq[1], bq[2], bq[3], sa_m[c] + so);
         mma_bf16_16816(dv[2 * c], P.x, P.y, P.z, P.w, bd[c][0], bd[c][1]);
         mma_bf16_16816(dv[2 * c + 1], P.x, P.y, P.z, P.w, bd[c][2], bd[c][3]);
-      }
-      if (more) issue_part(sf_tag, std::integral_constant<int, 0>{}, i + kRingFineStages - 1);
 #pragma unroll
-      for (int c = 2; c < 4; ++c) {
-        mma_bf16_16816(dv[2 * c], P.x, P.y, P.z, P.w, bd[c][0], bd[c][1]);
-        mma_bf16_16816(dv[2 * c + 1], P.x, P.y, P.z, P.w, bd[c][2], bd[c][3]);
+        for (int x = 0; x < 4; ++x) bd[c][x] = bq[x];
       }
-      if (more) issue_part(sf_tag, std::integral_constant<int, 1>{}, i + kRingFineStages - 1);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        mma_bf16_16816(dk[2 * c], D.x, D.y, D.z, D.w, bq[c][0], bq[c][1]);
-        mma_bf16_16816(dk[2 * c + 1], D.x, D.y, D.z, D.w, bq[c][2], bq[c][3]);
+      for (int c = 0; c < 4; ++c) {
+        mma_bf16_16816(dk[2 * c], D.x, D.y, D.z, D.w, bd[c][0], bd[c][1]);
+        mma_bf16_16816(dk[2 * c + 1], D.x, D.y, D.z, D.w, bd[c][2], bd[c][3]);
       }
-      if (more) issue_part(sf_tag, std::integral_constant<int, 2>{}, i + kRingFineStages - 1);
-#pragma unroll
-      for (int c = 2; c < 4; ++c) {
-        mma_bf16_16816(dk[2 * c], D.x, D.y, D.z, D.w, bq[c][0], bq[c][1]);
-        mma_bf16_16816(dk[2 * c + 1], D.x, D.y, D.z, D.w, bq[c][2], bq[c][3]);
-      }
-      if (more) issue_part(sf_tag, std::integral_constant<int, 3>{}, i + kRingFineStages - 1);
-      cp_async_commit();
-    };
-    for (int i = 0; i < n; i += 4) {
-      entry(std::integral_constant<int, 0>{}, i);
-      if (i + 1 < n) entry(std::integral_constant<int, 1>{}, i + 1);
-      if (i + 2 < n) entry(std::integral_constant<int, 2>{}, i + 2);
-      if (i + 3 < n) entry(std::integral_constant<int, 3>{}, i + 3);
+      if (st == kRingFineStages - 1) { st = 0; ph ^= 1; } else { ++st; }
     }
-    cp_async_wait_all();
+    if (!ok) break;
     __syncwarp();
-    park_fold();                            // the last bucket's gradient rows, for whichever path below stores it
-    // the last bucket of the range (the ring is idle by now)
+    // the last bucket of the span; the ring is idle by now
     if (bo >= rb && nxt <= re) {
-      dkv_fine_store_staged<0>(a, b, h, j, dk, dv, sa_m, sa_cp0, sa_cp1, sa_fold, lane);
+      park_fold();
+      dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, 0, sa_fold, lane);
+    } else if (PERSISTENT) {
+      tile_to_mem(pieces + (bo >= rb ? kTileFloats : 0), dk, dv, lane);     // continues in the next window, or lies across the whole of this one
     } else if (bo < rb) {                   // the whole range lies inside one bucket that began earlier
       tile_to_mem(slots + warp * kTileFloats, dk, dv, lane);
       if (lane == 0) s_head_bucket[warp] = j;
     } else {
+      park_fold();
       tail_j = j;                           // continues in later warps (or windows): completed below
     }
   }
+  if (!ok) tc::abort_drain();
   __syncthreads();
-  if (tail_j >= 0) {
-    for (int w = warp + 1; w < kRingWarps && s_head_bucket[w] == tail_j; ++w) tile_add_mem(slots + w * kTileFloats, dk, dv, lane);
-    if ((int) csr_off(a, bh, tail_j + 1) <= ce) {
-      dkv_fine_store_staged<0>(a, b, h, tail_j, dk, dv, sa_m, sa_cp0, sa_cp1, sa_fold, lane);
-    } else {                                // runs on into the next window: this window's tail slot
-      tile_to_mem(partial + ((bh * gridDim.x + blockIdx.x) * 2 + 1) * (int64_t) kTileFloats, dk, dv, lane);
+  if (!PERSISTENT) {
+    const int64_t b = bh / a.H, h = bh % a.H;
+    float* const pieces = partial + (bh * n_windows + blockIdx.x) * 2 * (int64_t) kTileFloats;
+    if (tail_j >= 0) {
+      for (int w = warp + 1; w < kRingWarps && s_head_bucket[w] == tail_j; ++w) tile_add_mem(slots + w * kTileFloats, dk, dv, lane);
+      if ((int) csr_off(a, bh, tail_j + 1) <= ce) {
+        dkv_fine_store_staged(a, b, h, tail_j, dk, dv, sa_m, sa_cp, 0, sa_fold, lane);
+      } else {                                // runs on into the next window: this window's tail slot
+        tile_to_mem(pieces + kTileFloats, dk, dv, lane);
+      }
+    }
+    if (warp == 0 && s_head_bucket[0] >= 0) { // began in an earlier window: this window's head slot
+      const int j0 = s_head_bucket[0];
+      tile_zero(dk, dv);
+      for (int w = 0; w < kRingWarps && s_head_bucket[w] == j0; ++w) tile_add_mem(slots + w * kTileFloats, dk, dv, lane);
+      tile_to_mem(pieces, dk, dv, lane);
     }
   }
-  if (warp == 0 && s_head_bucket[0] >= 0) { // began in an earlier window: this window's head slot
-    const int j0 = s_head_bucket[0];
-    tile_zero(dk, dv);
-    for (int w = 0; w < kRingWarps && s_head_bucket[w] == j0; ++w) tile_add_mem(slots + w * kTileFloats, dk, dv, lane);
-    tile_to_mem(partial + ((bh * gridDim.x + blockIdx.x) * 2 + 0) * (int64_t) kTileFloats, dk, dv, lane);
-  }
+  if (threadIdx.x == 0 && s_ctl.abort && a.status) atomicOr(a.status, (int) LLSA_DEV_WAIT_EXPIRED);
 }
 
 // KV blocks nobody selected: their dk / dv are the pooling-backward term alone, one row sixteen times.  A warp looks at four blocks, one per
@@ -845,7 +834,7 @@ __global__ void __launch_bounds__(128) attn_dkv_finish_kernel(AttnP<bf16> a, con
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n1 = (int) a.n1;
   const int64_t bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
-  const int E = (int) (a.nq1 * a.topk), range = a.range_entries, window = kRingWarps * range;       // nominal entries per warp / per CTA of the main kernel
+  const int E = (int) (a.nq1 * a.topk), range = a.range_entries, window = kRingWindow;
   const int R = (E + range - 1) / range, edge = ((int) blockIdx.x + 1) * window;
   // offsets are clamped to [0, E] and to each other: a malformed CSR cannot send the arithmetic below outside `partial`
   const int j = min(max(__ldcg(&a.ranges[bh * R + edge / range].y), 0), n1 - 1);
@@ -949,11 +938,27 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
   }
   if (mask & 4) {
     const int64_t E = a.nq1 * a.topk;
-    const int n_ranges = (int) ((E + a.range_entries - 1) / a.range_entries), n_windows = (n_ranges + kRingWarps - 1) / kRingWarps;
+    const int n_windows = (int) ((E + kRingWindow - 1) / kRingWindow);
     float* partial = (float*) g->dkv_partial->ptr;
-    const size_t smem = (size_t) kRingWarps * (kTileFloats * sizeof(float) + kRingFineStages * kRingFineStageBytes + kRingFoldBytes) + 128;   // per warp: slot, ring, gradient rows
-    LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel), smem);
-    launch_pdl(attn_dkv_fine_ring_kernel, dim3((unsigned) n_windows, BH), kRingWarps * 32, smem, st, a, partial);
+    FineMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    int rc;
+    if ((rc = tma::make_map_bhnd(&maps.q, g->q, kBS))) return rc;
+    if ((rc = tma::make_map_bhnd(&maps.d_o, g->d_o, kBS))) return rc;
+    const size_t ring = (size_t) kRingWarps * kRingWarpBytes + 1024;
+    if (a.range_entries == kRangeEntries) {
+      int dev = 0, sms = 148;
+      LLSA_CUDA_OK(cudaGetDevice(&dev));
+      LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      const int64_t total = (int64_t) n_windows * BH, most = (total + kRingWarps - 1) / kRingWarps;
+      const unsigned grid = (unsigned) (most < 3 * sms ? most : 3 * sms);
+      LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel<true>), ring);
+      launch_pdl(attn_dkv_fine_ring_kernel<true>, dim3(grid), kRingWarps * 32, ring, st, a, maps, partial, n_windows, total);
+    } else {
+      const size_t smem = ring + (size_t) kRingWarps * kTileFloats * sizeof(float);
+      LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel<false>), smem);
+      launch_pdl(attn_dkv_fine_ring_kernel<false>, dim3((unsigned) n_windows, BH), kRingWarps * 32, smem, st, a, maps, partial, n_windows, (int64_t) 0);
+    }
     LLSA_LAUNCH_OK("attn_dkv_fine_ring_kernel");
     const int n_plain = (int) ((a.n1 + 4 * kPlainPerWarp - 1) / (4 * kPlainPerWarp));
     attn_dkv_finish_kernel<<<dim3((unsigned) (n_windows - 1 + n_plain), BH), 128, 0, st>>>(a, partial, n_windows);

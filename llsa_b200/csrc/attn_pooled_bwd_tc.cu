@@ -10,7 +10,7 @@
 //     dQ = dS . PK          [128 x 64],  K = 192     dS K-major, PK MN-major (the same copy of PK)
 //     dPV = P^T  . dO       [192 x 64],  K = 128     P MN-major (rows = queries), dO MN-major
 //     dPK = dS^T . Q        [192 x 64],  K = 128
-// with P = exp(S*scale + ln w - lse) and dS = P * (dP - delta) * scale computed by the softmax warps
+// with P = exp(S*scale + ln w - lse) and dS = P * (dP - delta) computed by the softmax warps
 // between the first two and the last three.  The 64 level-2 keys would need an M = 64 product; instead
 // P(tile 2) and dS(tile 2) are laid out next to each other and used as ONE M = 128 operand against
 // [Q | dO] (N = 128): the result holds dPK2 in TMEM lanes 64..127 of its first 64 columns and dPV2 in
@@ -30,11 +30,11 @@
 //   warps 12-15       : drain warpgroup: at the end of a parent adds dPV1 / dPK1 (TMEM lane = pooled
 //                       key) to the fp32 pooled-gradient accumulators with red.global.add.v4.f32, at
 //                       the end of a head the level-2 results.
-//   warp 16, one lane : TMA producer (Q, dO and the level-1 keys double-buffered; level-1 values
+//   warp 16           : TMA producer (Q, dO and the level-1 keys double-buffered; level-1 values
 //                       reloaded as soon as dP of the parent's last tile has read them)
-//   warp 17, one lane : tcgen05.mma issuer for S, dP and dQ.  Its operations execute in issue order, so S of
+//   warp 17           : tcgen05.mma issuer for S, dP and dQ.  Its operations execute in issue order, so S of
 //                       the next tile is issued as soon as dP of this tile has been read, ahead of dQ.
-//   warp 18, one lane : tcgen05.mma issuer for the three transposed products (accumulators and operands no
+//   warp 18           : tcgen05.mma issuer for the three transposed products (accumulators and operands no
 //                       instruction of warp 17 writes; ordered against it by the barriers only).
 // Every mbarrier wait is bounded; a wait that expires raises a CTA-wide abort flag, every role leaves
 // its loop, the host-visible status word is set and TMEM is freed.
@@ -115,163 +115,123 @@ attn_bwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ BwdMaps maps, i
   const int n_my = t_end - t_begin;
 
   if (warp == 16) {
-    // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      for (int i = 0; i < n_my; ++i) {
-        const int tile = t_begin + i, s = i & 1;
-        const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
-        const bool new_parent = i == 0 || (tile >> 1) != ((tile - 1) >> 1);
-        const bool new_head = i == 0 || bh != (tile - 1) / tiles_per_head;
-        int krow[8];                      // rows of the parent's 8 selected level-1 key blocks: independent loads, ahead of the waits
-        if (new_parent) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) krow[j] = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, j) * kBS);
-        }
-        // stage s (and the level-1 key buffer of the parent two back) is free once every product of tile i - 2 has completed
-        if (i >= 2 && !tc::bounded_wait(&bars.mma_done[s], ((i - 2) >> 1) & 1, abort_flag)) break;
-        // the level-2 buffers are free once every product of the previous tile has completed
-        if (i >= 1 && new_head && !tc::bounded_wait(&bars.mma_done[(i - 1) & 1], ((i - 1) >> 1) & 1, abort_flag)) break;
-        tma::expect_tx(&bars.full[s], 2u * kTile * 2 + (new_parent ? 2u * kTile * 2 : 0u) + (new_head ? (uint32_t) kTile * 2 : 0u));
-        tma::load_4d(sQ + s * kTile, &maps.q, &bars.full[s], 0, row0, bh % a.H, bh / a.H);
-        tma::load_4d(sDO + s * kTile, &maps.d_o, &bars.full[s], 0, row0, bh % a.H, bh / a.H);
-        if (new_head) {
-          tma::load_2d(sK2, &maps.pk2, &bars.full[s], 0, (int) ((int64_t) bh * a.n2));
-          tma::load_2d(sV2, &maps.pv2, &bars.full[s], 0, (int) ((int64_t) bh * a.n2));
-        }
-        if (new_parent) {
-          bf16* k1 = sK1 + ((tile >> 1) & 1) * kTile;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) tma::load_2d(k1 + j * kBS * 64, &maps.pk1, &bars.full[s], 0, krow[j]);
-          // the level-1 values are last read by dP of the previous tile.  New parents come every other tile, so one of
-          // the two v_free barriers is waited on at each of its phases and the other never.
-          if (i >= 1 && !tc::bounded_wait(&bars.v_free[(i - 1) & 1], ((i - 1) >> 1) & 1, abort_flag)) break;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) tma::load_2d(sV1 + j * kBS * 64, &maps.pv1, &bars.full[s], 0, krow[j]);
-        }
+    // ---------------------------------------------------------------- TMA producer (the warp in step: tc05.cuh, umma_ss_k64)
+    for (int i = 0; i < n_my; ++i) {
+      const int tile = t_begin + i, s = i & 1;
+      const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
+      const bool new_parent = i == 0 || (tile >> 1) != ((tile - 1) >> 1);
+      const bool new_head = i == 0 || bh != (tile - 1) / tiles_per_head;
+      int krow = 0;                       // lane j: row of the parent's j-th selected level-1 key block, loaded ahead of the waits
+      if (new_parent) krow = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, lane & 7) * kBS);
+      // stage s (and the level-1 key buffer of the parent two back) is free once every product of tile i - 2 has completed
+      if (i >= 2 && !tc::warp_wait(&bars.mma_done[s], ((i - 2) >> 1) & 1, abort_flag)) break;
+      // the level-2 buffers are free once every product of the previous tile has completed
+      if (i >= 1 && new_head && !tc::warp_wait(&bars.mma_done[(i - 1) & 1], ((i - 1) >> 1) & 1, abort_flag)) break;
+      tma::expect_tx_w(&bars.full[s], 2u * kTile * 2 + (new_parent ? 2u * kTile * 2 : 0u) + (new_head ? (uint32_t) kTile * 2 : 0u));
+      tma::load_4d_w(sQ + s * kTile, &maps.q, &bars.full[s], 0, row0, bh % a.H, bh / a.H);
+      tma::load_4d_w(sDO + s * kTile, &maps.d_o, &bars.full[s], 0, row0, bh % a.H, bh / a.H);
+      if (new_head) {
+        tma::load_2d_w(sK2, &maps.pk2, &bars.full[s], 0, (int) ((int64_t) bh * a.n2));
+        tma::load_2d_w(sV2, &maps.pv2, &bars.full[s], 0, (int) ((int64_t) bh * a.n2));
+      }
+      if (new_parent) {
+        bf16* k1 = sK1 + ((tile >> 1) & 1) * kTile;
+        for (int j = 0; j < 8; ++j) tma::load_2d_w(k1 + j * kBS * 64, &maps.pk1, &bars.full[s], 0, __shfl_sync(0xffffffffu, krow, j));
+        // the level-1 values are last read by dP of the previous tile.  New parents come every other tile, so one of
+        // the two v_free barriers is waited on at each of its phases and the other never.
+        if (i >= 1 && !tc::warp_wait(&bars.v_free[(i - 1) & 1], ((i - 1) >> 1) & 1, abort_flag)) break;
+        for (int j = 0; j < 8; ++j) tma::load_2d_w(sV1 + j * kBS * 64, &maps.pv1, &bars.full[s], 0, __shfl_sync(0xffffffffu, krow, j));
       }
     }
   } else if (warp == 17) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      const uint32_t id_s128 = tc::instr_desc(128, 128, 0, 0), id_s64 = tc::instr_desc(128, 64, 0, 0), id_s192 = tc::instr_desc(128, 192, 0, 0);
-      const uint32_t id_dq = tc::instr_desc(128, 64, 0, 1), id_kv = tc::instr_desc(128, 64, 1, 1), id_kv2 = tc::instr_desc(128, 128, 1, 1);
-      // Shared-memory descriptors as (low word, high word).  The high word (stride between 8-row groups = 1024 bytes,
-      // descriptor version, 128-byte swizzle) is the same for every operand here; the low word holds the address
-      // (>> 4, 14 bits: addresses stay below 2^18) and the leading-dimension byte offset, so a k-step is one 32-bit add:
-      // K-major operand: 32 bytes (2 units) per k-step of 16 channels inside the swizzled 128-byte row;
-      // MN-major operand: 16 rows = 2048 bytes (128 units) per k-step.
-      const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
-      // Every operand sits at a compile-time offset from the 1024-byte aligned base, and the address field counts 16-byte
-      // units below 2^14, so each low word is `sb` plus a constant: one live register instead of twenty.
-      const uint32_t sb = (tc::smem_u32(base) >> 4) & 0x3FFFu;
-      constexpr uint32_t kU = (uint32_t) (kTile * 2) >> 4;          // 16-byte units of one [128 x 64] tile
-      auto lo = [sb](uint32_t units, uint32_t lbo_bytes) { return sb + units + ((lbo_bytes >> 4) << 16); };
-      constexpr uint32_t kStage = kU;                                // one 16 KB buffer further
-      constexpr uint32_t kT = kTile * 2;                             // bytes of a tile
-      constexpr uint32_t uQ = 0, uDO = 2 * kU, uK1 = 4 * kU, uK2 = 6 * kU, uV1 = 6 * kU + kU / 2, uP = 8 * kU;
-      const uint32_t lK2_k = lo(uK2, 16), lK2_m = lo(uK2, 1024), lV_k = lo(uV1, 16);                // [V1;V2] as N = 192 rows
-      const uint32_t lDS_k0 = lo(uP + 4 * kU, 16), lDS_k1 = lo(uP + 5 * kU, 16), lDS_k2 = lo(uP + 3 * kU, 16);
-      const uint32_t lP1_m = lo(uP, kT), lDS1_m = lo(uP + 4 * kU, kT), lP2_m = lo(uP + 2 * kU, kT);   // M = 128 over two tiles
-      const uint32_t lQ_k0 = lo(uQ, 16), lDO_k0 = lo(uDO, 16), lQ_m0 = lo(uQ, 1024), lDO_m0 = lo(uDO, 1024);
-      const uint32_t lQDO_m0 = lo(uQ, 2 * kT);                       // N = 128: channels of Q, then of dO (32 KB further)
-      const uint32_t lK1_k0 = lo(uK1, 16), lK1_m0 = lo(uK1, 1024);
-      auto issue_s = [&](int i) -> bool {          // S(i) = Q . [PK1 ; PK2]^T into columns [0,192)
-        const int s = i & 1;
-        if (!tc::bounded_wait(&bars.full[s], (i >> 1) & 1, abort_flag)) return false;
-        tc::fence_after_sync();
-        const uint32_t q_ = lQ_k0 + s * kStage, k1_ = lK1_k0 + (((t_begin + i) >> 1) & 1) * kStage;
-        tc::umma_ss_lh<0>(tmem, q_, hi, k1_, hi, id_s128);
-        tc::umma_ss_lh<0>(tmem + 128, q_, hi, lK2_k, hi, id_s64);
-#pragma unroll
-        for (int ks = 1; ks < 4; ++ks) {
-          tc::umma_ss_lh<1>(tmem, q_ + 2 * ks, hi, k1_ + 2 * ks, hi, id_s128);
-          tc::umma_ss_lh<1>(tmem + 128, q_ + 2 * ks, hi, lK2_k + 2 * ks, hi, id_s64);
-        }
-        tc::umma_commit(&bars.s_ready);
-        return true;
-      };
-      bool ok = n_my > 0 && issue_s(0);
-      for (int i = 0; ok && i < n_my; ++i) {
-        const int s = i & 1, tile = t_begin + i;
-        // dP(i) = dO . [PV1 ; PV2]^T over the columns of S once every softmax warp has read S
-        if (!tc::bounded_wait(&bars.s_consumed, i & 1, abort_flag)) break;
-        tc::fence_after_sync();
-        {
-          const uint32_t d_ = lDO_k0 + s * kStage;
-          tc::umma_ss_lh<0>(tmem, d_, hi, lV_k, hi, id_s192);
-#pragma unroll
-          for (int ks = 1; ks < 4; ++ks) tc::umma_ss_lh<1>(tmem, d_ + 2 * ks, hi, lV_k + 2 * ks, hi, id_s192);
-        }
-        tc::umma_commit(&bars.dp_ready);
-        tc::umma_commit(&bars.v_free[s]);
-        if (!tc::bounded_wait(&bars.pds_ready, i & 1, abort_flag)) break;
-        tc::fence_after_sync();
-        // The next tile's S goes ahead of this tile's output products, unless it belongs to a new head: the level-2
-        // buffers are reloaded only after these products have completed.
-        const bool next_early = i + 1 < n_my && (tile + 1) % tiles_per_head != 0;
-        if (next_early && !issue_s(i + 1)) break;
-        // dQ = dS . [PK1 ; PK2]: 12 k-steps of 16 keys, dS tile ks / 4; its columns are free once the drain warps have read
-        // the previous tile's dQ
-        if (i > 0 && !tc::bounded_wait(&bars.dq_free, (i - 1) & 1, abort_flag)) break;
-        tc::fence_after_sync();
-        {
-          const uint32_t k1_ = lK1_m0 + ((tile >> 1) & 1) * kStage;
-          tc::umma_ss_lh<0>(tmem + kColDQ, lDS_k0, hi, k1_, hi, id_dq);
-#pragma unroll
-          for (int ks = 1; ks < 4; ++ks) tc::umma_ss_lh<1>(tmem + kColDQ, lDS_k0 + 2 * ks, hi, k1_ + 128 * ks, hi, id_dq);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks) tc::umma_ss_lh<1>(tmem + kColDQ, lDS_k1 + 2 * ks, hi, k1_ + 128 * (4 + ks), hi, id_dq);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks) tc::umma_ss_lh<1>(tmem + kColDQ, lDS_k2 + 2 * ks, hi, lK2_m + 128 * ks, hi, id_dq);
-        }
-        tc::umma_commit(&bars.out_ready);           // this thread's half: S, dP, dQ of the tile
-        tc::umma_commit(&bars.mma_done[s]);
-        if (!next_early && i + 1 < n_my && !issue_s(i + 1)) break;
-      }
+    const uint32_t id_s128 = tc::instr_desc(128, 128, 0, 0), id_s64 = tc::instr_desc(128, 64, 0, 0), id_s192 = tc::instr_desc(128, 192, 0, 0);
+    const uint32_t id_dq = tc::instr_desc(128, 64, 0, 1);
+    // Shared-memory descriptors as (low word, high word).  The high word (stride between 8-row groups = 1024 bytes,
+    // descriptor version, 128-byte swizzle) is the same for every operand here; the low word holds the address
+    // (>> 4, 14 bits: addresses stay below 2^18) and the leading-dimension byte offset, so a k-step is one 32-bit add.
+    const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
+    // Every operand sits at a compile-time offset from the 1024-byte aligned base, and the address field counts 16-byte
+    // units below 2^14, so each low word is `sb` plus a constant: one live register instead of twenty.
+    const uint32_t sb = (tc::smem_u32(base) >> 4) & 0x3FFFu;
+    constexpr uint32_t kU = (uint32_t) (kTile * 2) >> 4;          // 16-byte units of one [128 x 64] tile
+    auto lo = [sb](uint32_t units, uint32_t lbo_bytes) { return sb + units + ((lbo_bytes >> 4) << 16); };
+    constexpr uint32_t kStage = kU;                                // one 16 KB buffer further
+    constexpr uint32_t uQ = 0, uDO = 2 * kU, uK1 = 4 * kU, uK2 = 6 * kU, uV1 = 6 * kU + kU / 2, uP = 8 * kU;
+    const uint32_t lK2_k = lo(uK2, 16), lK2_m = lo(uK2, 1024), lV_k = lo(uV1, 16);                // [V1;V2] as N = 192 rows
+    const uint32_t lDS_k0 = lo(uP + 4 * kU, 16), lDS_k1 = lo(uP + 5 * kU, 16), lDS_k2 = lo(uP + 3 * kU, 16);
+    const uint32_t lQ_k0 = lo(uQ, 16), lDO_k0 = lo(uDO, 16), lK1_k0 = lo(uK1, 16), lK1_m0 = lo(uK1, 1024);
+    auto issue_s = [&](int i) -> bool {          // S(i) = Q . [PK1 ; PK2]^T into columns [0,192)
+      const int s = i & 1;
+      if (!tc::warp_wait(&bars.full[s], (i >> 1) & 1, abort_flag)) return false;
+      tc::fence_after_sync();
+      const uint32_t q_ = lQ_k0 + s * kStage, k1_ = lK1_k0 + (((t_begin + i) >> 1) & 1) * kStage;
+      tc::umma_ss_k64(tmem, q_, hi, k1_, hi, id_s128);
+      tc::umma_ss_k64(tmem + 128, q_, hi, lK2_k, hi, id_s64);
+      tc::umma_commit_w(&bars.s_ready);
+      return true;
+    };
+    bool ok = n_my > 0 && issue_s(0);
+    for (int i = 0; ok && i < n_my; ++i) {
+      const int s = i & 1, tile = t_begin + i;
+      // dP(i) = dO . [PV1 ; PV2]^T over the columns of S once every softmax warp has read S
+      if (!tc::warp_wait(&bars.s_consumed, i & 1, abort_flag)) break;
+      tc::fence_after_sync();
+      tc::umma_ss_k64(tmem, lDO_k0 + s * kStage, hi, lV_k, hi, id_s192);
+      tc::umma_commit_w(&bars.dp_ready);
+      tc::umma_commit_w(&bars.v_free[s]);
+      if (!tc::warp_wait(&bars.pds_ready, i & 1, abort_flag)) break;
+      tc::fence_after_sync();
+      // The next tile's S goes ahead of this tile's output products, unless it belongs to a new head: the level-2
+      // buffers are reloaded only after these products have completed.
+      const bool next_early = i + 1 < n_my && (tile + 1) % tiles_per_head != 0;
+      if (next_early && !issue_s(i + 1)) break;
+      // dQ = dS . [PK1 ; PK2]: 12 k-steps of 16 keys, dS tile ks / 4; its columns are free once the drain warps have read
+      // the previous tile's dQ
+      if (i > 0 && !tc::warp_wait(&bars.dq_free, (i - 1) & 1, abort_flag)) break;
+      tc::fence_after_sync();
+      const uint32_t k1_ = lK1_m0 + ((tile >> 1) & 1) * kStage;
+      tc::umma_ss_k64<2, 128>(tmem + kColDQ, lDS_k0, hi, k1_, hi, id_dq, 0);
+      tc::umma_ss_k64<2, 128>(tmem + kColDQ, lDS_k1, hi, k1_ + 128 * 4, hi, id_dq, 1);
+      tc::umma_ss_k64<2, 128>(tmem + kColDQ, lDS_k2, hi, lK2_m, hi, id_dq, 1);
+      tc::umma_commit_w(&bars.out_ready);           // this warp's half: S, dP, dQ of the tile
+      tc::umma_commit_w(&bars.mma_done[s]);
+      if (!next_early && i + 1 < n_my && !issue_s(i + 1)) break;
     }
   } else if (warp == 18) {
     // ---------------------------------------------------------------- second MMA issuer: the three transposed products
-    // One thread issues a tcgen05.mma of these shapes every 56-90 cycles here, the pipe takes one every 48-64: the tile's 48
-    // instructions are dealt to two threads in two warps.  This one's 24 write accumulators nobody else's instructions
-    // touch and read P / dS, Q and dO only, so nothing orders the two threads but the barriers: out_ready and mma_done
-    // count one commit of each.
-    if (lane == 0) {
-      const uint32_t id_kv = tc::instr_desc(128, 64, 1, 1), id_kv2 = tc::instr_desc(128, 128, 1, 1);
-      const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
-      const uint32_t sb = (tc::smem_u32(base) >> 4) & 0x3FFFu;
-      constexpr uint32_t kU = (uint32_t) (kTile * 2) >> 4, kStage = kU, kT = kTile * 2;
-      auto lo = [sb](uint32_t units, uint32_t lbo_bytes) { return sb + units + ((lbo_bytes >> 4) << 16); };
-      constexpr uint32_t uQ = 0, uDO = 2 * kU, uP = 8 * kU;
-      const uint32_t lP1_m = lo(uP, kT), lDS1_m = lo(uP + 4 * kU, kT), lP2_m = lo(uP + 2 * kU, kT);   // M = 128 over two tiles
-      const uint32_t lQ_m0 = lo(uQ, 1024), lDO_m0 = lo(uDO, 1024), lQDO_m0 = lo(uQ, 2 * kT);
-      int parents_done = 0;
-      for (int i = 0; i < n_my; ++i) {
-        const int s = i & 1, tile = t_begin + i;
-        if (!tc::bounded_wait(&bars.pds_ready, i & 1, abort_flag)) break;
-        tc::fence_after_sync();
-        // transposed products, K = 128 query rows in 8 k-steps.  Level-1 results accumulate over the tiles of a
-        // parent, level-2 results over the tiles of a head; a fresh start waits for the drain warps to have read
-        // the previous parent's results.
-        const uint32_t acc1 = (i > 0 && (tile & 1)) ? 1u : 0u;
-        const uint32_t acc2 = (i > 0 && (tile % tiles_per_head) != 0) ? 1u : 0u;
-        if (!acc1 && parents_done > 0 && !tc::bounded_wait(&bars.acc_free, (parents_done - 1) & 1, abort_flag)) break;
-        tc::fence_after_sync();
-        {
-          const uint32_t do_ = lDO_m0 + s * kStage, q_ = lQ_m0 + s * kStage, qdo_ = lQDO_m0 + s * kStage;
-          tc::umma_ss_lh(tmem + kColPV1, lP1_m, hi, do_, hi, id_kv, acc1);
-          tc::umma_ss_lh(tmem + kColPK1, lDS1_m, hi, q_, hi, id_kv, acc1);
-          tc::umma_ss_lh(tmem + kColYX, lP2_m, hi, qdo_, hi, id_kv2, acc2);
-#pragma unroll
-          for (int ks = 1; ks < 8; ++ks) {
-            tc::umma_ss_lh<1>(tmem + kColPV1, lP1_m + 128 * ks, hi, do_ + 128 * ks, hi, id_kv);
-            tc::umma_ss_lh<1>(tmem + kColPK1, lDS1_m + 128 * ks, hi, q_ + 128 * ks, hi, id_kv);
-            tc::umma_ss_lh<1>(tmem + kColYX, lP2_m + 128 * ks, hi, qdo_ + 128 * ks, hi, id_kv2);
-          }
-        }
-        tc::umma_commit(&bars.out_ready);
-        tc::umma_commit(&bars.mma_done[s]);
-        if ((tile & 1) || i == n_my - 1) ++parents_done;
-      }
+    // A warp of their own: its products write accumulators no other instruction touches and read P / dS, Q and dO only, so
+    // nothing orders the two issuers but the barriers; out_ready and mma_done count one commit of each.
+    const uint32_t id_kv = tc::instr_desc(128, 64, 1, 1), id_kv2 = tc::instr_desc(128, 128, 1, 1);
+    const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
+    const uint32_t sb = (tc::smem_u32(base) >> 4) & 0x3FFFu;
+    constexpr uint32_t kU = (uint32_t) (kTile * 2) >> 4, kStage = kU, kT = kTile * 2;
+    auto lo = [sb](uint32_t units, uint32_t lbo_bytes) { return sb + units + ((lbo_bytes >> 4) << 16); };
+    constexpr uint32_t uQ = 0, uDO = 2 * kU, uP = 8 * kU;
+    const uint32_t lP1_m = lo(uP, kT), lDS1_m = lo(uP + 4 * kU, kT), lP2_m = lo(uP + 2 * kU, kT);   // M = 128 over two tiles
+    const uint32_t lQ_m0 = lo(uQ, 1024), lDO_m0 = lo(uDO, 1024), lQDO_m0 = lo(uQ, 2 * kT);   // N = 128: channels of Q, then of dO (32 KB further)
+    int parents_done = 0;
+    for (int i = 0; i < n_my; ++i) {
+      const int s = i & 1, tile = t_begin + i;
+      if (!tc::warp_wait(&bars.pds_ready, i & 1, abort_flag)) break;
+      tc::fence_after_sync();
+      // transposed products, K = 128 query rows in 8 k-steps.  Level-1 results accumulate over the tiles of a
+      // parent, level-2 results over the tiles of a head; a fresh start waits for the drain warps to have read
+      // the previous parent's results.
+      const uint32_t acc1 = (i > 0 && (tile & 1)) ? 1u : 0u;
+      const uint32_t acc2 = (i > 0 && (tile % tiles_per_head) != 0) ? 1u : 0u;
+      if (!acc1 && parents_done > 0 && !tc::warp_wait(&bars.acc_free, (parents_done - 1) & 1, abort_flag)) break;
+      tc::fence_after_sync();
+      const uint32_t do_ = lDO_m0 + s * kStage, q_ = lQ_m0 + s * kStage, qdo_ = lQDO_m0 + s * kStage;
+      tc::umma_ss_k64<128, 128>(tmem + kColPV1, lP1_m, hi, do_, hi, id_kv, acc1);
+      tc::umma_ss_k64<128, 128>(tmem + kColPK1, lDS1_m, hi, q_, hi, id_kv, acc1);
+      tc::umma_ss_k64<128, 128>(tmem + kColYX, lP2_m, hi, qdo_, hi, id_kv2, acc2);
+      tc::umma_ss_k64<128, 128>(tmem + kColPV1, lP1_m + 512, hi, do_ + 512, hi, id_kv, 1);
+      tc::umma_ss_k64<128, 128>(tmem + kColPK1, lDS1_m + 512, hi, q_ + 512, hi, id_kv, 1);
+      tc::umma_ss_k64<128, 128>(tmem + kColYX, lP2_m + 512, hi, qdo_ + 512, hi, id_kv2, 1);
+      tc::umma_commit_w(&bars.out_ready);
+      tc::umma_commit_w(&bars.mma_done[s]);
+      if ((tile & 1) || i == n_my - 1) ++parents_done;
     }
   } else if (warp >= 12) {
     // ---------------------------------------------------------------- drain warpgroup
@@ -306,10 +266,10 @@ attn_bwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ BwdMaps maps, i
         for (int q = 0; q < 2; ++q) {
           const uint4 f = old[2 * c + q];
           uint4 w;
-          w.x = pack_bf16(bf16_lo(f.x) + va[8 * q], bf16_hi(f.x) + va[8 * q + 1]);
-          w.y = pack_bf16(bf16_lo(f.y) + va[8 * q + 2], bf16_hi(f.y) + va[8 * q + 3]);
-          w.z = pack_bf16(bf16_lo(f.z) + va[8 * q + 4], bf16_hi(f.z) + va[8 * q + 5]);
-          w.w = pack_bf16(bf16_lo(f.w) + va[8 * q + 6], bf16_hi(f.w) + va[8 * q + 7]);
+          w.x = pack_bf16(fmaf(va[8 * q], a.scale, bf16_lo(f.x)), fmaf(va[8 * q + 1], a.scale, bf16_hi(f.x)));
+          w.y = pack_bf16(fmaf(va[8 * q + 2], a.scale, bf16_lo(f.y)), fmaf(va[8 * q + 3], a.scale, bf16_hi(f.y)));
+          w.z = pack_bf16(fmaf(va[8 * q + 4], a.scale, bf16_lo(f.z)), fmaf(va[8 * q + 5], a.scale, bf16_hi(f.z)));
+          w.w = pack_bf16(fmaf(va[8 * q + 6], a.scale, bf16_lo(f.w)), fmaf(va[8 * q + 7], a.scale, bf16_hi(f.w)));
           *reinterpret_cast<uint4*>(dqrow + 16 * c + 8 * q) = w;
         }
       }
@@ -319,11 +279,11 @@ attn_bwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ BwdMaps maps, i
       if (!parent_end) continue;
       // end of a parent: TMEM lane r = level-1 pooled key r of the parent
       red_cols(a.dpv + ((int64_t) bh * a.n1 + key) * kD, kColPV1, a.kvw1 / a.w1);
-      red_cols(a.dpk + ((int64_t) bh * a.n1 + key) * kD, kColPK1, a.kvw1 / a.w1);
+      red_cols(a.dpk + ((int64_t) bh * a.n1 + key) * kD, kColPK1, a.kvw1 / a.w1 * a.scale);
       if (i == n_my - 1 || (tile + 1) % tiles_per_head == 0) {
         // level-2 keys: dPK2 of key r - 64 in lanes 64..127 of the first 64 columns, dPV2 of key r in lanes 0..63 of the last 64
         if (qd < 2) red_cols(a.dpv2 + ((int64_t) bh * a.n2 + r) * kD, kColX, a.kvw2 / a.w2);
-        else red_cols(a.dpk2 + ((int64_t) bh * a.n2 + (r - 64)) * kD, kColY, a.kvw2 / a.w2);
+        else red_cols(a.dpk2 + ((int64_t) bh * a.n2 + (r - 64)) * kD, kColY, a.kvw2 / a.w2 * a.scale);
       }
       tc::fence_before_sync();
       __syncwarp();
@@ -333,6 +293,7 @@ attn_bwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ BwdMaps maps, i
     // ---------------------------------------------------------------- softmax / dS; thread = query row
     const int wg = warp >> 2, qd = warp & 3, r = qd * 32 + lane;
     const float sl2 = a.scale * kLog2eF;
+    const F2 sl22 = f2(sl2, sl2);
     const float lw = log2f(wg < 2 ? a.w1 : a.w2);
     const uint32_t t_row = tmem + ((uint32_t) (qd * 32) << 16);
     // this thread's row in its P tile and its dS tile: start of the row with the swizzle of chunk 0 applied
@@ -348,7 +309,7 @@ attn_bwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ BwdMaps maps, i
     for (int i = 0; i < n_my; ++i) {
       const int tile = t_begin + i;
       const float off = lw - lse_n * kLog2eF;
-      const float dls = delta_n * a.scale;
+      const F2 off2 = f2(off, off), nd2 = f2(-delta_n, -delta_n);
       ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.s_ready, i & 1, abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
@@ -358,7 +319,11 @@ attn_bwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ BwdMaps maps, i
       for (int c = 0; c < 4; ++c) {
         tc::tmem_ld16(t_row + wg * 64 + 16 * c, vh);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) pk[8 * c + j] = pack_bf16(fast_exp2(fmaf(vh[2 * j], sl2, off)), fast_exp2(fmaf(vh[2 * j + 1], sl2, off)));
+        for (int j = 0; j < 8; ++j) {
+          float x0, x1;
+          f2_get(f2_fma(f2(vh[2 * j], vh[2 * j + 1]), sl22, off2), x0, x1);
+          pk[8 * c + j] = pack_bf16(fast_exp2(x0), fast_exp2(x1));
+        }
       }
       tc::fence_before_sync();
       __syncwarp();
@@ -391,7 +356,9 @@ attn_bwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ BwdMaps maps, i
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const uint32_t p2 = pk[8 * C + e];
-          w[e] = pack_bf16(bf16_lo(p2) * fmaf(vh[2 * e], a.scale, -dls), bf16_hi(p2) * fmaf(vh[2 * e + 1], a.scale, -dls));
+          float d0, d1;
+          f2_get(f2_mul(f2(bf16_lo(p2), bf16_hi(p2)), f2_add(f2(vh[2 * e], vh[2 * e + 1]), nd2)), d0, d1);
+          w[e] = pack_bf16(d0, d1);
         }
         tc::sts128_xor<32 * C>(myDS, w[0], w[1], w[2], w[3]);
         tc::sts128_xor<32 * C + 16>(myDS, w[4], w[5], w[6], w[7]);

@@ -45,6 +45,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// One look, no suspension
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // ---- bounded waits of the warp-specialised kernels -------------------------------------------------
 // One WaitCtl per CTA (shared memory).  A wait polls at most `limit` times; the first wait that runs out raises
 // `abort`, which every other wait of the CTA notices within a thousand polls, so all roles leave their loops, the
@@ -56,9 +68,9 @@ struct WaitCtl {
 };
 constexpr int kWaitPolls = 400000;
 __device__ __forceinline__ bool bounded_wait(uint64_t* bar, uint32_t parity, volatile WaitCtl* c) {
-  if (mbar_try_wait(bar, parity)) return true;        // already complete: the common case for the threads that issue MMAs and copies
+  if (mbar_test(bar, parity)) return true;            // the first of the `limit` polls: a try_wait may suspend the thread for a while
   const int limit = c->limit;
-  for (int i = 0; i < limit; ++i) {
+  for (int i = 1; i < limit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 1023) == 1023 && c->abort) return false;
   }
@@ -68,9 +80,9 @@ __device__ __forceinline__ bool bounded_wait(uint64_t* bar, uint32_t parity, vol
 // The same by a whole warp in step: lane l waits for bars[l]'s phase (several barriers at the price of one: the test is one instruction
 // whatever addresses its lanes bring), and the answer is the same in every lane, which keeps the control flow around it uniform.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile WaitCtl* c) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
   const int limit = c->limit;
-  for (int i = 0; i < limit; ++i) {
+  for (int i = 1; i < limit; ++i) {
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     if ((i & 1023) == 1023 && __any_sync(0xffffffffu, c->abort != 0)) return false;
   }
@@ -140,28 +152,32 @@ __device__ __forceinline__ void umma_ss_lh(uint32_t tmem_d, uint32_t a_lo, uint3
 // descriptors from uniform registers and is issued once per executing thread; where the compiler sees an elected thread in uniform control
 // flow the descriptors stay there, where it sees `if (lane == 0)` every instruction costs some 98 cycles of moves, whatever its size, and
 // issuing, not the tensor pipe, is the pace of a kernel whose products have N = 64.
-// One statement issues all k-steps of a tile, 16 elements of K each.
-// A, B in shared memory, both K-major (32 bytes per k-step), K = 64: D = A . B
-__device__ __forceinline__ void umma_ss_k64(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
+// One statement issues four k-steps, 16 elements of K each.
+// A, B in shared memory; AS / BS: descriptor units (16 bytes) per k-step, 2 for a K-major operand (32 bytes inside the swizzled row), 128
+// for an MN-major one (16 rows).  D (+)= A . B, K = 64; `accumulate` is for the first k-step
+template <int AS = 2, int BS = 2>
+__device__ __forceinline__ void umma_ss_k64(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                            uint32_t accumulate = 0) {
   asm volatile(
       "{\n\t.reg .pred f, t, e;\n\t.reg .b32 al, bl;\n\t.reg .b64 da, db;\n\t"
-      "setp.ne.b32 f, %6, 0; setp.eq.b32 t, %6, 0;\n\t"
+      "setp.ne.b32 f, %7, 0; setp.eq.b32 t, %6, 0;\n\t"
       "elect.sync _|e, 0xffffffff;\n\t"
       "add.u32 al, %1, 0; add.u32 bl, %3, 0;\n\t"
       "mov.b64 da, {al, %2}; mov.b64 db, {bl, %4};\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %6, %6, %6}, f;\n\t"
-      "add.u32 al, %1, 2; add.u32 bl, %3, 2;\n\t"
+      "add.u32 al, %1, %8; add.u32 bl, %3, %9;\n\t"
       "mov.b64 da, {al, %2}; mov.b64 db, {bl, %4};\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %6, %6, %6}, t;\n\t"
-      "add.u32 al, %1, 4; add.u32 bl, %3, 4;\n\t"
+      "add.u32 al, %1, %10; add.u32 bl, %3, %11;\n\t"
       "mov.b64 da, {al, %2}; mov.b64 db, {bl, %4};\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %6, %6, %6}, t;\n\t"
-      "add.u32 al, %1, 6; add.u32 bl, %3, 6;\n\t"
+      "add.u32 al, %1, %12; add.u32 bl, %3, %13;\n\t"
       "mov.b64 da, {al, %2}; mov.b64 db, {bl, %4};\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %6, %6, %6}, t;\n\t"
       "}"
       :
-      : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(0u)
+      : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(0u), "r"(accumulate), "n"(AS), "n"(BS), "n"(2 * AS),
+        "n"(2 * BS), "n"(3 * AS), "n"(3 * BS)
       : "memory");
 }
 // A in tensor memory (two K values per column), B in shared memory and MN-major (16 rows of 128 bytes per k-step): D (+)= A . B, K = 32, 64
