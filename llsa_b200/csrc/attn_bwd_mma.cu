@@ -472,7 +472,8 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 //   * The pooled-gradient rows a finished tile folds in (the pooling backward) are requested into registers when
 //     the bucket begins and parked in shared memory right before the store.
 // Accumulator layout (ldmatrix): tile u holds channels 8u + 2t, 8u + 2t + 1 of keys g (c0, c1) and g + 8 (c2, c3).
-constexpr int kRingWarps = 4;                   // warps per CTA
+constexpr int kRingWarps = 4;                   // warps per CTA, one window per CTA
+constexpr int kRingWarpsP = 12;                 // warps per CTA, one persistent CTA per SM
 constexpr int kRingFineStages = 3;
 constexpr int kRingTileBytes = kRingTileElems * (int) sizeof(bf16);
 constexpr int kRingFineStageBytes = 2 * kRingTileBytes + 1024;                         // Q tile, dO tile, P^T and dS^T registers
@@ -569,23 +570,26 @@ __device__ __forceinline__ void dkv_fine_store_staged(const AttnP<bf16>& a, int6
 }
 
 template <bool PERSISTENT>
-__global__ void __launch_bounds__(kRingWarps * 32, PERSISTENT ? 3 : 2)
+__global__ void __launch_bounds__((PERSISTENT ? kRingWarpsP : kRingWarps) * 32, PERSISTENT ? 1 : 2)
 attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, float* __restrict__ partial, int n_windows, int64_t n_total) {
+  constexpr int NW = PERSISTENT ? kRingWarpsP : kRingWarps;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t s_full[kRingWarps][kRingFineStages];
+  __shared__ uint64_t s_full[NW][kRingFineStages];
   __shared__ tc::WaitCtl s_ctl;
-  __shared__ int s_head_bucket[kRingWarps];
+  __shared__ int s_head_bucket[NW];
+  __shared__ int s_next;
   // swizzled tiles: 1024-byte aligned
   unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
-  float* slots = reinterpret_cast<float*>(smem + kRingWarps * kRingWarpBytes);   // !PERSISTENT: [kRingWarps][kTileFloats], tile of the bucket a warp shares with earlier warps
+  float* slots = reinterpret_cast<float*>(smem + NW * kRingWarpBytes);   // !PERSISTENT: [kRingWarps][kTileFloats], tile of the bucket a warp shares with earlier warps
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
   volatile tc::WaitCtl* ctl = &s_ctl;
   if (threadIdx.x == 0) {
     s_ctl.abort = 0;
     s_ctl.limit = a.wait_limit > 0 ? a.wait_limit : tc::kWaitPolls;
+    s_next = 0;
   }
-  if (threadIdx.x < kRingWarps) s_head_bucket[threadIdx.x] = -1;
-  if (threadIdx.x < kRingWarps * kRingFineStages) tc::mbar_init(&s_full[0][0] + threadIdx.x, 1);
+  if (threadIdx.x < NW) s_head_bucket[threadIdx.x] = -1;
+  if (threadIdx.x < NW * kRingFineStages) tc::mbar_init(&s_full[0][0] + threadIdx.x, 1);
   tc::fence_mbar_init();
   pdl_trigger();
   pdl_wait();
@@ -616,24 +620,40 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
   // entries the CSR really holds: fewer than E when the transpose dropped out-of-range indices; ranges and offsets handed in
   // by a caller are not trusted further than these clamps and the bounds on the bucket walk below
   auto cut = [&](int r, int used) { return r < R ? min(max(__ldcg(&a.ranges[bh * R + r].x), 0), used) : used; };
-  // a span: PERSISTENT one window (two ranges) after another per warp, otherwise one range per warp and one window per CTA
+  // A span of the entry list.  !PERSISTENT: one range per warp, one window per CTA.  PERSISTENT: the warps of a CTA draw one range after
+  // another; a range that begins inside a bucket is left to the warp that has the range in front of it, unless it opens a window.
   bool ok = true;
-  for (int64_t w = PERSISTENT ? (int64_t) warp * gridDim.x + blockIdx.x : 0; ok && w < (PERSISTENT ? n_total : 1); w += PERSISTENT ? (int64_t) kRingWarps * gridDim.x : 1) {
+  for (bool more = true; ok && more; more = PERSISTENT) {
     int r0, rb, re;
-    if (PERSISTENT) bh = w / n_windows;
-    const int E_used = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1)));
-    const int win = PERSISTENT ? (int) (w % n_windows) : (int) blockIdx.x;
     if (PERSISTENT) {
-      r0 = win * (kRingWindow / kRangeEntries);
-      rb = cut(r0, E_used);
-      re = max(cut(r0 + kRingWindow / kRangeEntries, E_used), rb);
+      int k = 0;
+      if (lane == 0) k = atomicAdd(&s_next, 1);
+      k = __shfl_sync(0xffffffffu, k, 0);
+      const int64_t u = blockIdx.x + (int64_t) (k >> 1) * gridDim.x;        // both ranges of a window: a left-over range is work for its neighbour
+      if (u >= n_total) break;
+      bh = u / n_windows;
+      r0 = (int) (u % n_windows) * 2 + (k & 1);
+      if (r0 >= R) continue;
     } else {
-      r0 = win * kRingWarps + warp;
-      const int cb = cut(win * kRingWarps, E_used);
-      ce = max(cut((win + 1) * kRingWarps, E_used), cb);
+      r0 = blockIdx.x * kRingWarps + warp;
+    }
+    const int E_used = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1)));
+    if (PERSISTENT) {
+      auto begins_inside = [&](int r) {
+        const int2 x = __ldcg(&a.ranges[bh * R + r]);
+        return (int) csr_off(a, bh, min(max(x.y, 0), n1 - 1)) < x.x;
+      };
+      const bool odd = r0 & 1, both = (odd || r0 + 1 < R) && begins_inside(r0 | 1);
+      if (odd && both) continue;
+      rb = cut(r0, E_used);
+      re = max(cut(r0 + (both ? 2 : 1), E_used), rb);
+    } else {
+      const int cb = cut(blockIdx.x * kRingWarps, E_used);
+      ce = max(cut((blockIdx.x + 1) * kRingWarps, E_used), cb);
       rb = min(max(cut(r0, E_used), cb), ce);
       re = min(max(cut(r0 + 1, E_used), rb), ce);
     }
+    const int win = PERSISTENT ? r0 / (kRingWindow / kRangeEntries) : (int) blockIdx.x;
     if (rb >= re) continue;
     const int64_t b = bh / a.H, h = bh % a.H;
     float* const pieces = partial + (bh * n_windows + win) * 2 * (int64_t) kTileFloats;     // the window's head and tail slots
@@ -945,17 +965,17 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     int rc;
     if ((rc = tma::make_map_bhnd(&maps.q, g->q, kBS))) return rc;
     if ((rc = tma::make_map_bhnd(&maps.d_o, g->d_o, kBS))) return rc;
-    const size_t ring = (size_t) kRingWarps * kRingWarpBytes + 1024;
     if (a.range_entries == kRangeEntries) {
       int dev = 0, sms = 148;
       LLSA_CUDA_OK(cudaGetDevice(&dev));
       LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      const int64_t total = (int64_t) n_windows * BH, most = (total + kRingWarps - 1) / kRingWarps;
-      const unsigned grid = (unsigned) (most < 3 * sms ? most : 3 * sms);
+      static_assert(kRingWindow == 2 * kRangeEntries, "a window of the persistent form is two ranges");
+      const int64_t total = (int64_t) n_windows * BH;
+      const size_t ring = (size_t) kRingWarpsP * kRingWarpBytes + 1024;
       LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel<true>), ring);
-      launch_pdl(attn_dkv_fine_ring_kernel<true>, dim3(grid), kRingWarps * 32, ring, st, a, maps, partial, n_windows, total);
+      launch_pdl(attn_dkv_fine_ring_kernel<true>, dim3((unsigned) (total < sms ? total : sms)), kRingWarpsP * 32, ring, st, a, maps, partial, n_windows, total);
     } else {
-      const size_t smem = ring + (size_t) kRingWarps * kTileFloats * sizeof(float);
+      const size_t smem = 1024 + (size_t) kRingWarps * (kRingWarpBytes + kTileFloats * sizeof(float));
       LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel<false>), smem);
       launch_pdl(attn_dkv_fine_ring_kernel<false>, dim3((unsigned) n_windows, BH), kRingWarps * 32, smem, st, a, maps, partial, n_windows, (int64_t) 0);
     }
