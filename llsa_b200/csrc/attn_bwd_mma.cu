@@ -40,6 +40,7 @@
 namespace llsa {
 
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kRingTileBytes = kRingTileElems * (int) sizeof(bf16);
 
 __device__ __forceinline__ float rowfrag_dot(const RowFrag& x, const RowFrag& y) {
   float acc = 0.f;
@@ -84,18 +85,21 @@ __device__ __forceinline__ void dq_p_ds(float (&s0)[4], float (&s1)[4], const fl
   da[3] = pack_bf16(s1[2] * (p1[2] - r.delta1), s1[3] * (p1[3] - r.delta1));
 }
 
-// Hands P and dS of a (query block, selected block) pair to the dK/dV stage.  That stage multiplies their transposes
-// (rows = keys) from the left: dV += P^T.dO, dK += dS^T.Q.  The A operand of those products holds, in lane (g,t),
-// (key g, queries 2t,2t+1), (key g+8, same), (key g, queries 8+2t,9+2t), (key g+8, same); the registers here hold
-// (query g, keys 2t,2t+1), (query g+8, ..), (query g, keys 8+2t,..), (query g+8, ..): each is an 8x8 matrix spread over
-// the warp, and transposing the four (movmatrix) and swapping the middle two gives exactly the A operand.  One uint4 per
-// lane and matrix: 1 KB per pair, written and later read in full 512-byte rows.
+// Hands P and dS of a (query block, selected block) pair to the dK/dV stage, 1 KB per pair: P, then dS, each as four 8x8 matrices of 128
+// contiguous bytes (rows = queries: queries 0..7 x keys 0..7, queries 8..15 x keys 0..7, then keys 8..15), so a register of all lanes is
+// one whole line and the reader's ldmatrix.trans delivers the transposes its products need (load_pds_t).
 __device__ __forceinline__ void store_pds(uint4* dst, const uint32_t (&pa)[4], const uint32_t (&da)[4], int lane) {
-  uint4 p, d;
-  p.x = movmatrix_trans(pa[0]); p.y = movmatrix_trans(pa[2]); p.z = movmatrix_trans(pa[1]); p.w = movmatrix_trans(pa[3]);
-  d.x = movmatrix_trans(da[0]); d.y = movmatrix_trans(da[2]); d.z = movmatrix_trans(da[1]); d.w = movmatrix_trans(da[3]);
-  dst[lane] = p;
-  dst[32 + lane] = d;
+  uint32_t* d = reinterpret_cast<uint32_t*>(dst) + lane;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) { d[m * 32] = pa[m]; d[128 + m * 32] = da[m]; }
+}
+// P^T or dS^T from the hand-over in shared memory as the A operand of dV += P^T.dO, dK += dS^T.Q: (key g, queries 2t, 2t+1),
+// (key g+8, same), (key g, queries 8+2t, 9+2t), (key g+8, same); sa: start of the matrix + 16 * lane
+template <int IMM>
+__device__ __forceinline__ uint4 load_pds_t(uint32_t sa) {
+  uint4 r;
+  ldsm_x4_trans<IMM>(r.x, r.z, r.y, r.w, sa);
+  return r;
 }
 
 struct GlobalKV {
@@ -235,95 +239,140 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_mma_kernel(AttnP<bf16> a, 
   store_acc_row_t<1>(a.dq.row(b, h, qb * kBS + g + 8), dq, t, a.scale);
 }
 
-// Fine blocks only (the pooled keys are on the tcgen05 kernel): the selected K / V blocks go through a per-warp
-// cp.async ring in shared memory, two blocks ahead, instead of being held in registers one block ahead.
+// Fine blocks only (the pooled keys are on the tcgen05 kernels): one warp per query block; the selected K / V blocks go through a per-warp
+// ring in shared memory, filled by TMA two blocks ahead.
 constexpr int kDqStages = 3;
+struct KvMaps {
+  CUtensorMap k, v;            // [B,H,N,64] 4-D, box 16 rows
+};
+// One lane requests a block: its K tile and its V tile, both counted by one barrier.
+__device__ __forceinline__ void load_kv_w(uint32_t dst, const KvMaps& m, uint64_t* bar, int row, int h, int b) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t.reg .b32 d;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "add.u32 d, %0, 2048;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], 4096;\n\t"
+      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%7, %4, %5, %6}], [%3];\n\t"
+      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [d], [%2, {%7, %4, %5, %6}], [%3];\n\t"
+      "}" ::"r"(dst), "l"(&m.k), "l"(&m.v), "r"(tc::smem_u32(bar)), "r"(row), "r"(h), "r"(b), "r"(0)
+      : "memory");
+}
 
 template <int NW>
-__global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a) {
+__global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps maps) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t s_full[NW][kDqStages];
+  __shared__ tc::WaitCtl s_ctl[NW];             // a warp's own: the warps of a CTA share nothing
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  constexpr int kStageBytes = 2 * kRingTileBytes;
+  const uint32_t ring_sa = ((tc::smem_u32(smem_raw) + 1023u) & ~1023u) + warp * kDqStages * kStageBytes;
+  volatile tc::WaitCtl* ctl = &s_ctl[warp];
+  if (lane < kDqStages) tc::mbar_init(&s_full[warp][lane], 1);
+  if (lane == 0) {
+    ctl->abort = 0;
+    ctl->limit = a.wait_limit > 0 ? a.wait_limit : tc::kWaitPolls;
+  }
+  tc::fence_mbar_init();
+  __syncwarp();
   pdl_trigger();
   pdl_wait();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  bf16* ring = reinterpret_cast<bf16*>(smem_raw) + warp * (kDqStages * 2 * kRingTileElems);
   const int64_t qb = (int64_t) blockIdx.x * NW + warp, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
   const int my_fine = lane < a.topk ? (int) fine_block(a, bh, qb, lane) : 0;
-  const float sl2 = a.scale * kLog2e;
   const int n_glob = a.topk;
-  // a lane copies the same four 16-byte chunks of every K tile and of every V tile: offsets computed once
-  int off_k[4], off_v[4], off_s[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = i * 4 + (lane >> 3), c = lane & 7;
-    off_k[i] = r * (int) a.k.sn + c * 8;
-    off_v[i] = r * (int) a.v.sn + c * 8;
-    off_s[i] = r * 64 + ((c ^ (r & 7)) << 3);
-  }
-  const bf16* kb0 = a.k.row(b, h, 0);
-  const bf16* vb0 = a.v.row(b, h, 0);
-  const int64_t kblk = (int64_t) kBS * a.k.sn, vblk = (int64_t) kBS * a.v.sn;
-  auto issue = [&](int i) {
-    const int64_t j = __shfl_sync(0xffffffffu, my_fine, i);
-    bf16* stage = ring + (i % kDqStages) * 2 * kRingTileElems;
-    const bf16* kp = kb0 + j * kblk;
-    const bf16* vp = vb0 + j * vblk;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      cp_async16(stage + off_s[u], kp + off_k[u]);
-      cp_async16(stage + kRingTileElems + off_s[u], vp + off_v[u]);
-    }
+  int rst = 0;
+  auto request = [&](int i) {
+    load_kv_w(ring_sa + rst * kStageBytes, maps, &s_full[warp][rst], __shfl_sync(0xffffffffu, my_fine, i) * kBS, (int) h, (int) b);
+    rst = rst == kDqStages - 1 ? 0 : rst + 1;
   };
 #pragma unroll
-  for (int s = 0; s < kDqStages - 1; ++s) {
-    if (s < n_glob) issue(s);
-    cp_async_commit();
-  }
+  for (int s = 0; s < kDqStages - 1; ++s)
+    if (s < n_glob) request(s);
+  // shared addresses of stage 0: chunks 2t, 2t + 1 of row g (sa_f, sa_f ^ 16; row g + 8 is 1024 bytes on), ldmatrix rows of channels 0..15
+  // (sa_m; ^ 32 c: channels 16c..)
+  const uint32_t sa_f = ring_sa + g * 128 + (((2 * t) ^ g) << 4);
+  const uint32_t sa_m = ring_sa + ((lane & 7) + ((lane >> 3) & 1) * 8) * 128 + (((lane >> 4) ^ (lane & 7)) << 4);
   RowFrag qlo, qhi, dlo, dhi;
   load_rowfrag(qlo, a.q.row(b, h, qb * kBS + g), t);
   load_rowfrag(qhi, a.q.row(b, h, qb * kBS + g + 8), t);
   load_rowfrag(dlo, a.d_o.row(b, h, qb * kBS + g), t);
   load_rowfrag(dhi, a.d_o.row(b, h, qb * kBS + g + 8), t);
-  DqRow row;
+  const int64_t rbase = bh * a.Nq + qb * kBS;
+  F2 nl0, nl1, nd0, nd1;                        // minus lse (log2 domain) and minus delta of rows g and g + 8, twice
   {
     RowFrag olo, ohi;
     load_rowfrag(olo, a.o_in.row(b, h, qb * kBS + g), t);
     load_rowfrag(ohi, a.o_in.row(b, h, qb * kBS + g + 8), t);
-    row.delta0 = quad_sum(rowfrag_dot(olo, dlo));
-    row.delta1 = quad_sum(rowfrag_dot(ohi, dhi));
+    const float l0 = -a.lse[rbase + g] * kLog2e, l1 = -a.lse[rbase + g + 8] * kLog2e;
+    const float d0 = quad_sum(rowfrag_dot(olo, dlo)), d1 = quad_sum(rowfrag_dot(ohi, dhi));
+    if (t == 0) { a.delta[rbase + g] = d0; a.delta[rbase + g + 8] = d1; }
+    nl0 = f2(l0, l0); nl1 = f2(l1, l1); nd0 = f2(-d0, -d0); nd1 = f2(-d1, -d1);
   }
-  const int64_t rbase = bh * a.Nq + qb * kBS;
-  if (t == 0) { a.delta[rbase + g] = row.delta0; a.delta[rbase + g + 8] = row.delta1; }
-  row.L0 = a.lse[rbase + g] * kLog2e;
-  row.L1 = a.lse[rbase + g + 8] * kLog2e;
+  const float sl2 = a.scale * kLog2e;
+  const F2 sl22 = f2(sl2, sl2);
   float dq[8][4];
 #pragma unroll
   for (int j = 0; j < 8; ++j) dq[j][0] = dq[j][1] = dq[j][2] = dq[j][3] = 0.f;
+  int st = 0, ph = 0;
+  bool ok = true;
+  uint4* pds = a.pds ? a.pds + (bh * a.nq1 + qb) * a.topk * 64 : nullptr;
   for (int gi = 0; gi < n_glob; ++gi) {
-    cp_async_wait_group<kDqStages - 2>();       // block gi has landed (this lane's chunks) ...
-    __syncwarp();                               // ... and everybody else's; the stage read last time is free
-    if (gi + kDqStages - 1 < n_glob) issue(gi + kDqStages - 1);
-    cp_async_commit();
-    const bf16* tk = ring + (gi % kDqStages) * 2 * kRingTileElems;
-    RowFrag k0, k1, v0, v1;
-    load_rowfrag_ring(k0, tk, g, t);
-    load_rowfrag_ring(k1, tk, g + 8, t);
-    load_rowfrag_ring(v0, tk + kRingTileElems, g, t);
-    load_rowfrag_ring(v1, tk + kRingTileElems, g + 8, t);
-    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, p0[4] = {0.f, 0.f, 0.f, 0.f}, p1[4] = {0.f, 0.f, 0.f, 0.f};
-    mma_rows_x_keys(s0, s1, qlo, qhi, k0, k1);
-    mma_rows_x_keys(p0, p1, dlo, dhi, v0, v1);
-    uint32_t da[4];
-    if (a.pds) {                            // P and dS also go to the dK/dV stage
-      uint32_t pa[4];
-      dq_p_ds(s0, s1, p0, p1, row, sl2, pa, da);
-      store_pds(a.pds + ((bh * a.nq1 + qb) * a.topk + gi) * 64, pa, da, lane);
-    } else {
-      dq_ds(s0, s1, p0, p1, row, sl2, 0.f, da);
+    if (!(ok = tc::warp_wait(&s_full[warp][st], ph, ctl))) break;
+    if (gi + kDqStages - 1 < n_glob) request(gi + kDqStages - 1);      // into the stage read last time: its operands were consumed by products already issued
+    const uint32_t so = st * kStageBytes, f0 = sa_f + so, f1 = (sa_f ^ 16) + so, m0 = sa_m + so;
+    float s0[4], s1[4], p0[4], p1[4];
+    half_rows_x_keys<0, true>(s0, s1, qlo, qhi, f0);
+    half_rows_x_keys<kRingTileBytes, true>(p0, p1, dlo, dhi, f0);
+    half_rows_x_keys<0, false>(s0, s1, qlo, qhi, f1);
+    half_rows_x_keys<kRingTileBytes, false>(p0, p1, dlo, dhi, f1);
+    // P = exp2(s * scale * log2(e) - lse), dS / scale = P * (dP - delta)
+    uint32_t pa[4], da[4];
+    auto half = [&](const float x0, const float x1, const float y0, const float y1, F2 nl, F2 nd, uint32_t& p, uint32_t& d) {
+      float e0, e1;
+      f2_get(f2_fma(f2(x0, x1), sl22, nl), e0, e1);
+      e0 = fast_exp2(e0);
+      e1 = fast_exp2(e1);
+      p = pack_bf16(e0, e1);
+      float w0, w1;
+      f2_get(f2_mul(f2(e0, e1), f2_add(f2(y0, y1), nd)), w0, w1);
+      d = pack_bf16(w0, w1);
+    };
+    half(s0[0], s0[1], p0[0], p0[1], nl0, nd0, pa[0], da[0]);
+    half(s0[2], s0[3], p0[2], p0[3], nl1, nd1, pa[1], da[1]);
+    half(s1[0], s1[1], p1[0], p1[1], nl0, nd0, pa[2], da[2]);
+    half(s1[2], s1[3], p1[2], p1[3], nl1, nd1, pa[3], da[3]);
+    if (pds) {                              // P and dS also go to the dK/dV stage
+      store_pds(pds, pa, da, lane);
+      pds += 64;
     }
-    mma_x_rowfrag_t(dq, da[0], da[1], da[2], da[3], k0, k1);      // K transposed in registers (movmatrix)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {           // dQ += dS.K: K read transposed, 16 channels at a time
+      uint32_t bk[4];
+      ldsm_x4_trans<0>(bk[0], bk[1], bk[2], bk[3], m0 ^ (c << 5));
+      mma_bf16_16816(dq[2 * c], da[0], da[1], da[2], da[3], bk[0], bk[1]);
+      mma_bf16_16816(dq[2 * c + 1], da[0], da[1], da[2], da[3], bk[2], bk[3]);
+    }
+    if (st == kDqStages - 1) { st = 0; ph ^= 1; } else { ++st; }
   }
-  store_acc_row_t<0>(a.dq.row(b, h, qb * kBS + g), dq, t, a.scale);
-  store_acc_row_t<1>(a.dq.row(b, h, qb * kBS + g + 8), dq, t, a.scale);
+  if (!ok) {
+    tc::abort_drain();
+    if (lane == 0 && a.status) atomicOr(a.status, (int) LLSA_DEV_WAIT_EXPIRED);
+    return;
+  }
+  // the tile leaves through the idle ring (stmatrix, then eight lanes write one whole row)
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    stsm_x4<0>(sa_m ^ (c << 5), pack_bf16(dq[2 * c][0] * a.scale, dq[2 * c][1] * a.scale), pack_bf16(dq[2 * c][2] * a.scale, dq[2 * c][3] * a.scale),
+               pack_bf16(dq[2 * c + 1][0] * a.scale, dq[2 * c + 1][1] * a.scale), pack_bf16(dq[2 * c + 1][2] * a.scale, dq[2 * c + 1][3] * a.scale));
+  __syncwarp();
+  const uint32_t sa_cp = ring_sa + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4);
+  bf16* out = a.dq.row(b, h, qb * kBS + (lane >> 3)) + (lane & 7) * 8;
+  const int64_t step = 4 * a.dq.sn;
+  uint4 x;
+  lds128<0>(x.x, x.y, x.z, x.w, sa_cp);         *reinterpret_cast<uint4*>(out) = x;
+  lds128<512>(x.x, x.y, x.z, x.w, sa_cp ^ 64);  *reinterpret_cast<uint4*>(out + step) = x;
+  lds128<1024>(x.x, x.y, x.z, x.w, sa_cp);      *reinterpret_cast<uint4*>(out + 2 * step) = x;
+  lds128<1536>(x.x, x.y, x.z, x.w, sa_cp ^ 64); *reinterpret_cast<uint4*>(out + 3 * step) = x;
 }
 
 // P^T and dS^T (bf16, as A registers) of one (key tile) x (query block) pair from the
@@ -475,8 +524,7 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 constexpr int kRingWarps = 4;                   // warps per CTA, one window per CTA
 constexpr int kRingWarpsP = 12;                 // warps per CTA, one persistent CTA per SM
 constexpr int kRingFineStages = 3;
-constexpr int kRingTileBytes = kRingTileElems * (int) sizeof(bf16);
-constexpr int kRingFineStageBytes = 2 * kRingTileBytes + 1024;                         // Q tile, dO tile, P^T and dS^T registers
+constexpr int kRingFineStageBytes = 2 * kRingTileBytes + 1024;                         // Q tile, dO tile, P and dS
 constexpr int kRingFoldBytes = 4 * 64 * (int) sizeof(float);                           // per warp: dpk, dpv, dpk2, dpv2 rows of the bucket
 constexpr int kRingWarpBytes = kRingFineStages * kRingFineStageBytes + kRingFoldBytes;
 constexpr int kRingWindow = 64;                 // nominal entries per window: the unit whose cut buckets meet in the `partial` scratch
@@ -732,9 +780,7 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
       }
       // the stage read an entry ago is free: its operands were consumed by products already issued
       if (i + kRingFineStages - 1 < n) request(i + kRingFineStages - 1);
-      uint4 P, D;
-      lds128<2 * kRingTileBytes>(P.x, P.y, P.z, P.w, sa_l16 + so);
-      lds128<2 * kRingTileBytes + 512>(D.x, D.y, D.z, D.w, sa_l16 + so);
+      const uint4 P = load_pds_t<2 * kRingTileBytes>(sa_l16 + so), D = load_pds_t<2 * kRingTileBytes + 512>(sa_l16 + so);
       uint32_t bd[4][4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) ldsm_x4_trans<kRingTileBytes>(bd[c][0], bd[c][1], bd[c][2], bd[c][3], sa_m[c] + so);
@@ -927,9 +973,14 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     const int n_smem = n_all < 12 ? n_all : 12;   // 12 tiles = 54 KB of K+V, three CTAs per SM
     const size_t smem = (size_t) n_smem * kBS * kSmemPitch * sizeof(bf16) * 2;
     if (n_all == 0) {
-      const size_t ring = (size_t) NWQ * kDqStages * 2 * kRingTileElems * sizeof(bf16);
+      KvMaps maps;
+      memset(&maps, 0, sizeof(maps));
+      int rc;
+      if ((rc = tma::make_map_bhnd(&maps.k, g->k, kBS))) return rc;
+      if ((rc = tma::make_map_bhnd(&maps.v, g->v, kBS))) return rc;
+      const size_t ring = (size_t) NWQ * kDqStages * 2 * kRingTileBytes + 1024;
       LLSA_SMEM_LIMIT((attn_dq_fine_kernel<NWQ>), ring);
-      launch_pdl(attn_dq_fine_kernel<NWQ>, dim3((unsigned) (a.nq1 / NWQ), BH), NWQ * 32, ring, st, aq);
+      launch_pdl(attn_dq_fine_kernel<NWQ>, dim3((unsigned) (a.nq1 / NWQ), BH), NWQ * 32, ring, st, aq, maps);
       LLSA_LAUNCH_OK("attn_dq_fine_kernel");
     } else {
       LLSA_SMEM_LIMIT((attn_dq_mma_kernel<NWQ>), smem);
