@@ -75,14 +75,6 @@ static int check_attn_args(const LlsaAttnArgs* g, bool bwd) {
                    LLSA_ERR_WORKSPACE, "attn_bwd: dkv_partial must be a contiguous F32 tensor of at least %lld elements", (long long) need);
     }
     if (dt == LLSA_BF16 && !g->force_generic) {
-      // P / dS hand-over between the dQ stage and the dK/dV stage of the tensor-core path
-      const int64_t need = B * H * nq1 * g->topk * 256;
-      LLSA_REQUIRE(g->fine_pds && g->fine_pds->ptr && g->fine_pds->dtype == LLSA_F32 && is_contiguous(g->fine_pds), LLSA_ERR_WORKSPACE,
-                   "attn_bwd: fine_pds scratch missing (a contiguous F32 tensor of llsa_attn_bwd_pds_elems() elements)");
-      int64_t have = 1;
-      for (int i = 0; i < g->fine_pds->ndim; ++i) have *= g->fine_pds->shape[i];
-      LLSA_REQUIRE(have >= need && ((uintptr_t) g->fine_pds->ptr % 16) == 0, LLSA_ERR_WORKSPACE,
-                   "attn_bwd: fine_pds holds %lld elements, %lld needed", (long long) have, (long long) need);
       LLSA_REQUIRE(g->flat_pairs && g->flat_ranges, LLSA_ERR_WORKSPACE, "attn_bwd: flat_pairs / flat_ranges missing (llsa_transpose_indices_pairs)");
       if ((rc = check_contig(g->flat_pairs, "flat_pairs", LLSA_I32, 3, sf))) return rc;
       LLSA_REQUIRE(g->flat_ranges->ndim == 4 && range_entries_of(nq1 * g->topk, g->flat_ranges->shape[2]) > 0, LLSA_ERR_SHAPE,

@@ -52,6 +52,29 @@ __device__ __forceinline__ float rowfrag_dot(const RowFrag& x, const RowFrag& y)
   return acc;
 }
 
+// One lane requests a row of 64 fp32 values.
+__device__ __forceinline__ void load_row_w(uint32_t dst, const float* src, uint64_t* bar) {
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+               "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 256, [%2];\n\t}" ::"r"(dst), "l"(src),
+               "r"(tc::smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void cp_async4_sa(uint32_t sa, const void* gsrc) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(gsrc) : "memory");
+}
+// One lane requests rows [row, row + 16) of two [B,H,N,64] tensors as neighbouring 2 KB tiles, counted by one barrier whose phase expects
+// `bytes` in all.
+__device__ __forceinline__ void load_tiles_w(uint32_t dst, const CUtensorMap* m0, const CUtensorMap* m1, uint64_t* bar, int bytes, int row, int h, int b) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t.reg .b32 d;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "add.u32 d, %0, 2048;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %8;\n\t"
+      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%7, %4, %5, %6}], [%3];\n\t"
+      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [d], [%2, {%7, %4, %5, %6}], [%3];\n\t"
+      "}" ::"r"(dst), "l"(m0), "l"(m1), "r"(tc::smem_u32(bar)), "r"(row), "r"(h), "r"(b), "r"(0), "r"(bytes)
+      : "memory");
+}
+
 struct DqRow {
   float L0, L1, delta0, delta1;   // lse (log2 domain) and delta of rows g and g+8
 };
@@ -69,37 +92,6 @@ __device__ __forceinline__ void dq_ds(float (&s0)[4], float (&s1)[4], const floa
   s1[2] = fast_exp2(fmaf(s1[2], sl2, lw - r.L1)) * (p1[2] - r.delta1);
   s1[3] = fast_exp2(fmaf(s1[3], sl2, lw - r.L1)) * (p1[3] - r.delta1);
   da[0] = pack_bf16(s0[0], s0[1]); da[1] = pack_bf16(s0[2], s0[3]); da[2] = pack_bf16(s1[0], s1[1]); da[3] = pack_bf16(s1[2], s1[3]);
-}
-
-// The same for a fine block (weight 1), returning P (bf16) as well: both go to the dK/dV stage.
-__device__ __forceinline__ void dq_p_ds(float (&s0)[4], float (&s1)[4], const float (&p0)[4], const float (&p1)[4], const DqRow& r, float sl2,
-                                        uint32_t (&pa)[4], uint32_t (&da)[4]) {
-  s0[0] = fast_exp2(fmaf(s0[0], sl2, -r.L0)); s0[1] = fast_exp2(fmaf(s0[1], sl2, -r.L0));
-  s0[2] = fast_exp2(fmaf(s0[2], sl2, -r.L1)); s0[3] = fast_exp2(fmaf(s0[3], sl2, -r.L1));
-  s1[0] = fast_exp2(fmaf(s1[0], sl2, -r.L0)); s1[1] = fast_exp2(fmaf(s1[1], sl2, -r.L0));
-  s1[2] = fast_exp2(fmaf(s1[2], sl2, -r.L1)); s1[3] = fast_exp2(fmaf(s1[3], sl2, -r.L1));
-  pa[0] = pack_bf16(s0[0], s0[1]); pa[1] = pack_bf16(s0[2], s0[3]); pa[2] = pack_bf16(s1[0], s1[1]); pa[3] = pack_bf16(s1[2], s1[3]);
-  da[0] = pack_bf16(s0[0] * (p0[0] - r.delta0), s0[1] * (p0[1] - r.delta0));
-  da[1] = pack_bf16(s0[2] * (p0[2] - r.delta1), s0[3] * (p0[3] - r.delta1));
-  da[2] = pack_bf16(s1[0] * (p1[0] - r.delta0), s1[1] * (p1[1] - r.delta0));
-  da[3] = pack_bf16(s1[2] * (p1[2] - r.delta1), s1[3] * (p1[3] - r.delta1));
-}
-
-// Hands P and dS of a (query block, selected block) pair to the dK/dV stage, 1 KB per pair: P, then dS, each as four 8x8 matrices of 128
-// contiguous bytes (rows = queries: queries 0..7 x keys 0..7, queries 8..15 x keys 0..7, then keys 8..15), so a register of all lanes is
-// one whole line and the reader's ldmatrix.trans delivers the transposes its products need (load_pds_t).
-__device__ __forceinline__ void store_pds(uint4* dst, const uint32_t (&pa)[4], const uint32_t (&da)[4], int lane) {
-  uint32_t* d = reinterpret_cast<uint32_t*>(dst) + lane;
-#pragma unroll
-  for (int m = 0; m < 4; ++m) { d[m * 32] = pa[m]; d[128 + m * 32] = da[m]; }
-}
-// P^T or dS^T from the hand-over in shared memory as the A operand of dV += P^T.dO, dK += dS^T.Q: (key g, queries 2t, 2t+1),
-// (key g+8, same), (key g, queries 8+2t, 9+2t), (key g+8, same); sa: start of the matrix + 16 * lane
-template <int IMM>
-__device__ __forceinline__ uint4 load_pds_t(uint32_t sa) {
-  uint4 r;
-  ldsm_x4_trans<IMM>(r.x, r.z, r.y, r.w, sa);
-  return r;
 }
 
 struct GlobalKV {
@@ -207,13 +199,7 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_mma_kernel(AttnP<bf16> a, 
         load_rowfrag(v1, r.v + (int64_t) (g + 8) * r.vs, t);
       }
       uint32_t da[4];
-      if (gi < a.topk && a.pds) {           // a fine block: P and dS also go to the dK/dV stage
-        uint32_t pa[4];
-        dq_p_ds(s0, s1, p0, p1, row, sl2, pa, da);
-        store_pds(a.pds + ((bh * a.nq1 + qb) * a.topk + gi) * 64, pa, da, lane);
-      } else {
-        dq_ds(s0, s1, p0, p1, row, sl2, lw, da);
-      }
+      dq_ds(s0, s1, p0, p1, row, sl2, lw, da);
 #pragma unroll
       for (int i = 0; i < 8; ++i) mma_bf16_16816(dq[i], da[0], da[1], da[2], da[3], tk0[i], tk1[i]);
     }
@@ -245,19 +231,6 @@ constexpr int kDqStages = 3;
 struct KvMaps {
   CUtensorMap k, v;            // [B,H,N,64] 4-D, box 16 rows
 };
-// One lane requests a block: its K tile and its V tile, both counted by one barrier.
-__device__ __forceinline__ void load_kv_w(uint32_t dst, const KvMaps& m, uint64_t* bar, int row, int h, int b) {
-  asm volatile(
-      "{\n\t.reg .pred e;\n\t.reg .b32 d;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "add.u32 d, %0, 2048;\n\t"
-      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], 4096;\n\t"
-      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%7, %4, %5, %6}], [%3];\n\t"
-      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [d], [%2, {%7, %4, %5, %6}], [%3];\n\t"
-      "}" ::"r"(dst), "l"(&m.k), "l"(&m.v), "r"(tc::smem_u32(bar)), "r"(row), "r"(h), "r"(b), "r"(0)
-      : "memory");
-}
-
 template <int NW>
 __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps maps) {
   extern __shared__ unsigned char smem_raw[];
@@ -281,7 +254,7 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a,
   const int n_glob = a.topk;
   int rst = 0;
   auto request = [&](int i) {
-    load_kv_w(ring_sa + rst * kStageBytes, maps, &s_full[warp][rst], __shfl_sync(0xffffffffu, my_fine, i) * kBS, (int) h, (int) b);
+    load_tiles_w(ring_sa + rst * kStageBytes, &maps.k, &maps.v, &s_full[warp][rst], 2 * kRingTileBytes, __shfl_sync(0xffffffffu, my_fine, i) * kBS, (int) h, (int) b);
     rst = rst == kDqStages - 1 ? 0 : rst + 1;
   };
 #pragma unroll
@@ -314,7 +287,6 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a,
   for (int j = 0; j < 8; ++j) dq[j][0] = dq[j][1] = dq[j][2] = dq[j][3] = 0.f;
   int st = 0, ph = 0;
   bool ok = true;
-  uint4* pds = a.pds ? a.pds + (bh * a.nq1 + qb) * a.topk * 64 : nullptr;
   for (int gi = 0; gi < n_glob; ++gi) {
     if (!(ok = tc::warp_wait(&s_full[warp][st], ph, ctl))) break;
     if (gi + kDqStages - 1 < n_glob) request(gi + kDqStages - 1);      // into the stage read last time: its operands were consumed by products already issued
@@ -325,25 +297,16 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a,
     half_rows_x_keys<0, false>(s0, s1, qlo, qhi, f1);
     half_rows_x_keys<kRingTileBytes, false>(p0, p1, dlo, dhi, f1);
     // P = exp2(s * scale * log2(e) - lse), dS / scale = P * (dP - delta)
-    uint32_t pa[4], da[4];
-    auto half = [&](const float x0, const float x1, const float y0, const float y1, F2 nl, F2 nd, uint32_t& p, uint32_t& d) {
-      float e0, e1;
-      f2_get(f2_fma(f2(x0, x1), sl22, nl), e0, e1);
-      e0 = fast_exp2(e0);
-      e1 = fast_exp2(e1);
-      p = pack_bf16(e0, e1);
-      float w0, w1;
-      f2_get(f2_mul(f2(e0, e1), f2_add(f2(y0, y1), nd)), w0, w1);
-      d = pack_bf16(w0, w1);
+    uint32_t da[4];
+    auto half = [&](float x0, float x1, float y0, float y1, F2 nl, F2 nd) {
+      f2_get(f2_fma(f2(x0, x1), sl22, nl), x0, x1);
+      f2_get(f2_mul(f2(fast_exp2(x0), fast_exp2(x1)), f2_add(f2(y0, y1), nd)), y0, y1);
+      return pack_bf16(y0, y1);
     };
-    half(s0[0], s0[1], p0[0], p0[1], nl0, nd0, pa[0], da[0]);
-    half(s0[2], s0[3], p0[2], p0[3], nl1, nd1, pa[1], da[1]);
-    half(s1[0], s1[1], p1[0], p1[1], nl0, nd0, pa[2], da[2]);
-    half(s1[2], s1[3], p1[2], p1[3], nl1, nd1, pa[3], da[3]);
-    if (pds) {                              // P and dS also go to the dK/dV stage
-      store_pds(pds, pa, da, lane);
-      pds += 64;
-    }
+    da[0] = half(s0[0], s0[1], p0[0], p0[1], nl0, nd0);
+    da[1] = half(s0[2], s0[3], p0[2], p0[3], nl1, nd1);
+    da[2] = half(s1[0], s1[1], p1[0], p1[1], nl0, nd0);
+    da[3] = half(s1[2], s1[3], p1[2], p1[3], nl1, nd1);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {           // dQ += dS.K: K read transposed, 16 channels at a time
       uint32_t bk[4];
@@ -524,27 +487,16 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 constexpr int kRingWarps = 4;                   // warps per CTA, one window per CTA
 constexpr int kRingWarpsP = 12;                 // warps per CTA, one persistent CTA per SM
 constexpr int kRingFineStages = 3;
-constexpr int kRingFineStageBytes = 2 * kRingTileBytes + 1024;                         // Q tile, dO tile, P and dS
-constexpr int kRingFoldBytes = 4 * 64 * (int) sizeof(float);                           // per warp: dpk, dpv, dpk2, dpv2 rows of the bucket
-constexpr int kRingWarpBytes = kRingFineStages * kRingFineStageBytes + kRingFoldBytes;
+constexpr int kRingFineStageBytes = 2 * kRingTileBytes;                                // Q tile, dO tile
+constexpr int kRingTilesBytes = (kRingFineStages + 1) * kRingFineStageBytes;           // per warp: the ring, then K and V tile of the next bucket
+constexpr int kRingFoldBytes = 4 * 64 * (int) sizeof(float);                           // dpk, dpv, dpk2, dpv2 rows of a bucket
+constexpr int kRingStatBytes = 2 * kBS * (int) sizeof(float);                          // lse, delta of a query block
+constexpr int kRingWarpBytes = kRingTilesBytes + 2 * kRingFoldBytes + kRingFineStages * kRingStatBytes;
 constexpr int kRingWindow = 64;                 // nominal entries per window: the unit whose cut buckets meet in the `partial` scratch
 
 struct FineMaps {
-  CUtensorMap q, d_o;          // [B,H,Nq,64] 4-D, box 16 rows
+  CUtensorMap q, d_o, k, v;    // [B,H,N,64] 4-D, box 16 rows
 };
-// One lane requests an entry: Q tile, dO tile and the kilobyte of P^T / dS^T, all counted by one barrier.
-__device__ __forceinline__ void load_entry_w(uint32_t dst, const FineMaps& m, const uint4* pds, uint64_t* bar, int row, int h, int b) {
-  asm volatile(
-      "{\n\t.reg .pred e;\n\t.reg .b32 d, p;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "add.u32 d, %0, 2048; add.u32 p, %0, 4096;\n\t"
-      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], 5120;\n\t"
-      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%8, %5, %6, %7}], [%4];\n\t"
-      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [d], [%2, {%8, %5, %6, %7}], [%4];\n\t"
-      "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [p], [%3], 1024, [%4];\n\t"
-      "}" ::"r"(dst), "l"(&m.q), "l"(&m.d_o), "l"(pds), "r"(tc::smem_u32(bar)), "r"(row), "r"(h), "r"(b), "r"(0)
-      : "memory");
-}
 
 // Pooling-backward fold and scale for the ldmatrix accumulator layout: afterwards dk / dv hold the final fp32 values.
 // The four gradient rows of KV block j come from this warp's copy in shared memory ([dpk | dpv | dpk2 | dpv2] x 64 fp32, fetched with
@@ -588,15 +540,15 @@ __device__ __forceinline__ void dkv_fine_fold_smem(const AttnP<bf16>& a, uint32_
 // layout (the ldmatrix addresses sa_m), every lane reads back four 16-byte chunks per tensor (sa_cp: rows (lane/8) + {0, 4, 8, 12}) and
 // eight lanes write one whole 128-byte row: full sectors, 8 store instructions instead of 32.
 __device__ __forceinline__ void dkv_fine_store_staged(const AttnP<bf16>& a, int64_t b, int64_t h, int64_t j, float (&dk)[8][4],
-                                                      float (&dv)[8][4], const uint32_t (&sa_m)[4], uint32_t sa_cp, uint32_t so,
+                                                      float (&dv)[8][4], uint32_t sa_m, uint32_t sa_cp, uint32_t so,
                                                       uint32_t sa_fold, int lane) {
   constexpr int TB = kRingTileBytes;
   dkv_fine_fold_smem(a, sa_fold, dk, dv);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    stsm_x4<0>(sa_m[c] + so, pack_bf16(dk[2 * c][0], dk[2 * c][1]), pack_bf16(dk[2 * c][2], dk[2 * c][3]),
+    stsm_x4<0>((sa_m ^ (c << 5)) + so, pack_bf16(dk[2 * c][0], dk[2 * c][1]), pack_bf16(dk[2 * c][2], dk[2 * c][3]),
                pack_bf16(dk[2 * c + 1][0], dk[2 * c + 1][1]), pack_bf16(dk[2 * c + 1][2], dk[2 * c + 1][3]));
-    stsm_x4<TB>(sa_m[c] + so, pack_bf16(dv[2 * c][0], dv[2 * c][1]), pack_bf16(dv[2 * c][2], dv[2 * c][3]),
+    stsm_x4<TB>((sa_m ^ (c << 5)) + so, pack_bf16(dv[2 * c][0], dv[2 * c][1]), pack_bf16(dv[2 * c][2], dv[2 * c][3]),
                 pack_bf16(dv[2 * c + 1][0], dv[2 * c + 1][1]), pack_bf16(dv[2 * c + 1][2], dv[2 * c + 1][3]));
   }
   __syncwarp();
@@ -622,14 +574,14 @@ __global__ void __launch_bounds__((PERSISTENT ? kRingWarpsP : kRingWarps) * 32, 
 attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, float* __restrict__ partial, int n_windows, int64_t n_total) {
   constexpr int NW = PERSISTENT ? kRingWarpsP : kRingWarps;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t s_full[NW][kRingFineStages];
+  __shared__ uint64_t s_full[NW][kRingFineStages + 1];       // the ring's stages, then the next bucket's K / V
   __shared__ tc::WaitCtl s_ctl;
   __shared__ int s_head_bucket[NW];
   __shared__ int s_next;
   // swizzled tiles: 1024-byte aligned
   unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   float* slots = reinterpret_cast<float*>(smem + NW * kRingWarpBytes);   // !PERSISTENT: [kRingWarps][kTileFloats], tile of the bucket a warp shares with earlier warps
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   volatile tc::WaitCtl* ctl = &s_ctl;
   if (threadIdx.x == 0) {
     s_ctl.abort = 0;
@@ -637,7 +589,7 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
     s_next = 0;
   }
   if (threadIdx.x < NW) s_head_bucket[threadIdx.x] = -1;
-  if (threadIdx.x < NW * kRingFineStages) tc::mbar_init(&s_full[0][0] + threadIdx.x, 1);
+  if (threadIdx.x < NW * (kRingFineStages + 1)) tc::mbar_init(&s_full[0][0] + threadIdx.x, 1);
   tc::fence_mbar_init();
   pdl_trigger();
   pdl_wait();
@@ -645,24 +597,23 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
 
   const int E = (int) (a.nq1 * a.topk), n1 = (int) a.n1;
   const int R = (E + a.range_entries - 1) / a.range_entries;
-  // Per-lane shared addresses of stage 0, computed once (tiles are 1024-byte aligned, so the chunk index of an address is its bits
-  // 4..6 and a swizzle partner is one XOR away):
-  //   sa_cp    16-byte chunk lane % 8 of tile rows lane / 8 and lane / 8 + 8 (^ 64: + 4, + 12)
-  //   sa_m[c]  ldmatrix.trans row address for output channels 16c..16c+15
-  const uint32_t ring_sa = tc::smem_u32(smem + warp * kRingWarpBytes), sa_l16 = ring_sa + lane * 16;
-  constexpr int kFoldOff = kRingFineStages * kRingFineStageBytes;
-  const uint32_t sa_fold = ring_sa + 8 * t + kFoldOff;
+  // Per-lane shared addresses of stage 0 (tiles are 1024-byte aligned, so the chunk index of an address is its bits 4..6 and a swizzle
+  // partner is one XOR away):
+  //   sa_cp  16-byte chunk lane % 8 of tile rows lane / 8 and lane / 8 + 8 (^ 64: + 4, + 12)
+  //   sa_f   chunk 2t of row g (^ 16: chunk 2t + 1; row g + 8 is 1024 bytes on)
+  //   sa_m   ldmatrix.trans row address for output channels 0..15 (^ 32 c: 16c..16c+15)
+  const uint32_t ring_sa = tc::smem_u32(smem + warp * kRingTilesBytes);
+  const uint32_t fold_sa = tc::smem_u32(smem + NW * kRingTilesBytes + warp * 2 * kRingFoldBytes);
+  const uint32_t stat_sa = tc::smem_u32(smem + NW * (kRingTilesBytes + 2 * kRingFoldBytes) + warp * kRingFineStages * kRingStatBytes);
   const uint32_t sa_cp = ring_sa + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4);
-  uint32_t sa_m[4];
-  {
-    const int lr = (lane & 7) + ((lane >> 3) & 1) * 8;
-    const uint32_t base = ring_sa + lr * 128 + (((lane >> 4) ^ (lane & 7)) << 4);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) sa_m[c] = base ^ (c << 5);
-  }
+  const uint32_t sa_f = ring_sa + g * 128 + (((2 * t) ^ g) << 4);
+  const uint32_t sa_m = ring_sa + ((lane & 7) + ((lane >> 3) & 1) * 8) * 128 + (((lane >> 4) ^ (lane & 7)) << 4);
+  const float sl2 = a.scale * kLog2e;
   float dk[8][4], dv[8][4];
+  RowFrag klo, khi, vlo, vhi;               // K and V of the bucket at hand, as A operands
   int tail_j = -1;                          // !PERSISTENT: bucket whose tile is still in dk / dv after the loop
   int st = 0, ph = 0;                       // ring stage of the entry at hand, parity of its fill
+  int kvph = 0, fold_buf = 0;               // parity of the next K / V fill, fold buffer of the bucket at hand
   int64_t bh = blockIdx.y;
   int ce = 0;
   // entries the CSR really holds: fewer than E when the transpose dropped out-of-range indices; ranges and offsets handed in
@@ -706,113 +657,152 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
     const int64_t b = bh / a.H, h = bh % a.H;
     float* const pieces = partial + (bh * n_windows + win) * 2 * (int64_t) kTileFloats;     // the window's head and tail slots
     const int32_t* fl = a.flat + bh * (int64_t) E;
-    const int32_t* pr = a.pairs + bh * (int64_t) E;
     const int n = re - rb;
-    // lane i: query block and pair number of entry 32 c + i of the chunk c being requested and of the one after it (clamped: nothing is
-    // read outside the tensors)
-    int cur_qb = 0, cur_pair = 0, nx_qb = 0, nx_pair = 0;
+    // lane i: query block of entry 32 c + i of the chunk c being requested and of the one after it (clamped: nothing is read outside the
+    // tensors)
+    int cur_qb = 0, nx_qb = 0;
     auto fetch = [&](int i0) {
-      if (i0 + lane < n) {
-        nx_qb = min(max(__ldcg(fl + rb + i0 + lane), 0), (int) a.nq1 - 1);
-        nx_pair = min(max(__ldcg(pr + rb + i0 + lane), 0), E - 1);
-      }
+      if (i0 + lane < n) nx_qb = min(max(__ldcg(fl + rb + i0 + lane), 0), (int) a.nq1 - 1);
     };
     fetch(0);
-    // first bucket of the range (handed over by the transpose kernel; clamped, and moved on if it does not hold rb)
-    int j = min(max(__ldcg(&a.ranges[bh * R + r0].y), 0), n1 - 1);
-    int bo = (int) csr_off(a, bh, j), nxt = (int) csr_off(a, bh, j + 1);
-    while (nxt <= rb && j + 1 < n1) { ++j; bo = nxt; nxt = (int) csr_off(a, bh, j + 1); }
-    int nxt2 = j + 2 <= n1 ? (int) csr_off(a, bh, j + 2) : 0x7fffffff;      // one bucket ahead: no load to wait for at a switch
-    // the pooled-gradient rows the bucket's store folds in: lanes 0..15 hold the dpk row, lanes 16..31 the dpv row (16 bytes each)
-    uint4 f1 = make_uint4(0u, 0u, 0u, 0u), f2 = make_uint4(0u, 0u, 0u, 0u);
-    auto load_fold = [&](int jj) {
-      if (a.fold) {
-        f1 = __ldcg(reinterpret_cast<const uint4*>((lane < 16 ? a.dpk : a.dpv) + (bh * a.n1 + jj) * kD + (lane & 15) * 4));
-        if (a.two_level) f2 = __ldcg(reinterpret_cast<const uint4*>((lane < 16 ? a.dpk2 : a.dpv2) + (bh * a.n2 + jj / kBS) * kD + (lane & 15) * 4));
-      }
-    };
-    auto park_fold = [&]() {
-      if (a.fold) {
-        sts128<kFoldOff>(sa_l16, f1);
-        if (a.two_level) sts128<kFoldOff + 512>(sa_l16, f2);
-      }
-      __syncwarp();
-    };
-    const uint4* pds = a.pds + bh * (int64_t) E * 64;
     int rst = st;                            // ring stage of the next request
-    auto request = [&](int i) {
-      if ((i & 31) == 0) {
-        cur_qb = nx_qb;
-        cur_pair = nx_pair;
-        // the hand-over does not fit the L2: every lane pulls its own entry's kilobyte there ahead of the copies
-        if (i + lane < n) {
-          const char* pf = reinterpret_cast<const char*>(pds + (int64_t) cur_pair * 64);
-#pragma unroll
-          for (int l = 0; l < 8; ++l) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf + 128 * l));
+    const float* stat = (lane < 16 ? a.lse : a.delta) + bh * a.Nq + (lane & 15);
+    auto request = [&](int i) {              // Q and dO tile by TMA, lse and delta by one 4-byte copy per lane
+      if (i < n) {
+        if ((i & 31) == 0) {
+          cur_qb = nx_qb;
+          fetch(i + 32);
         }
-        fetch(i + 32);
+        const int qb = __shfl_sync(0xffffffffu, cur_qb, i & 31);
+        load_tiles_w(ring_sa + rst * kRingFineStageBytes, &maps.q, &maps.d_o, &s_full[warp][rst], kRingFineStageBytes, qb * kBS, (int) h, (int) b);
+        cp_async4_sa(stat_sa + rst * kRingStatBytes + 4 * lane, stat + qb * kBS);
+        rst = rst == kRingFineStages - 1 ? 0 : rst + 1;
       }
-      const int qb = __shfl_sync(0xffffffffu, cur_qb, i & 31), pair = __shfl_sync(0xffffffffu, cur_pair, i & 31);
-      load_entry_w(ring_sa + rst * kRingFineStageBytes, maps, pds + (int64_t) pair * 64, &s_full[warp][rst], qb * kBS, (int) h, (int) b);
-      rst = rst == kRingFineStages - 1 ? 0 : rst + 1;
+      cp_async_commit();
     };
     request(0);
-    if (1 < n) request(1);
-    load_fold(j);
-    tile_zero(dk, dv);
+    request(1);
+    // Bucket walk: lane l holds the end of bucket jb + l, so the bucket of an entry is the number of ends at or below it, and the next
+    // non-empty bucket is known without a load while the one at hand is being worked on.
+    auto bucket_end = [&](int j0) { return j0 + 1 + lane <= n1 ? (int) csr_off(a, bh, j0 + 1 + lane) : 0x7fffffff; };
+    int jb = min(max(__ldcg(&a.ranges[bh * R + r0].y), 0), n1 - 1);
+    int ends = bucket_end(jb), ends2 = bucket_end(jb + 32);
+    int j = -1, nxt = rb, j2 = 0, nxt2 = 0;  // the bucket at hand and its end, the one after it and its end
+    auto find_bucket = [&](int e) {          // j2, nxt2: the bucket of entry e
+      int c = __popc(__ballot_sync(0xffffffffu, ends <= e));
+      while (c == 32) {
+        jb += 32;
+        ends = ends2;
+        ends2 = bucket_end(jb + 32);
+        c = __popc(__ballot_sync(0xffffffffu, ends <= e));
+      }
+      j2 = min(jb + c, n1 - 1);
+      nxt2 = max(__shfl_sync(0xffffffffu, ends, c), e + 1);      // whatever the offsets hold, the walk moves on
+    };
+    // K and V tile and the pooled-gradient rows the bucket's store folds in
+    auto request_bucket = [&]() {
+      uint64_t* bar = &s_full[warp][kRingFineStages];
+      const int rows = a.fold ? (a.two_level ? 4 : 2) : 0;
+      load_tiles_w(ring_sa + kRingFineStages * kRingFineStageBytes, &maps.k, &maps.v, bar, kRingFineStageBytes + rows * 256, j2 * kBS, (int) h, (int) b);
+      if (a.fold) {
+        const uint32_t dst = fold_sa + (fold_buf ^ 1) * kRingFoldBytes;
+        const int64_t o1 = (bh * a.n1 + j2) * kD, o2 = (bh * a.n2 + j2 / kBS) * kD;
+        load_row_w(dst, a.dpk + o1, bar);
+        load_row_w(dst + 256, a.dpv + o1, bar);
+        if (a.two_level) {
+          load_row_w(dst + 512, a.dpk2 + o2, bar);
+          load_row_w(dst + 768, a.dpv2 + o2, bar);
+        }
+      }
+    };
+    find_bucket(rb);
+    bool began_before = (int) csr_off(a, bh, j2) < rb;
+    request_bucket();
     for (int i = 0; i < n; ++i) {
       const int e = rb + i;
       const uint32_t so = st * kRingFineStageBytes;
       if (!(ok = tc::warp_wait(&s_full[warp][st], ph, ctl))) break;
-      if (e >= nxt && j + 1 < n1) {                   // next non-empty bucket; the stage read an entry ago stages the store
-        if (bo >= rb) {
-          park_fold();
-          dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, rst * kRingFineStageBytes, sa_fold, lane);
-        } else {                                      // began in an earlier span
-          tile_to_mem(PERSISTENT ? pieces : slots + warp * kTileFloats, dk, dv, lane);
-          if (!PERSISTENT && lane == 0) s_head_bucket[warp] = j;
+      cp_async_wait_group<1>();
+      __syncwarp();
+      const bool fresh = e >= nxt;
+      if (fresh) {                                    // next non-empty bucket; the stage read an entry ago stages the store
+        if (j >= 0) {
+          if (!began_before) {
+            dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, rst * kRingFineStageBytes, fold_sa + fold_buf * kRingFoldBytes + 8 * t, lane);
+          } else {                                    // began in an earlier span
+            tile_to_mem(PERSISTENT ? pieces : slots + warp * kTileFloats, dk, dv, lane);
+            if (!PERSISTENT && lane == 0) s_head_bucket[warp] = j;
+          }
+          began_before = false;
         }
-        ++j; bo = nxt; nxt = nxt2;
-        while (nxt <= e && j + 1 < n1) { ++j; bo = nxt; nxt = (int) csr_off(a, bh, j + 1); }      // empty buckets
-        nxt2 = j + 2 <= n1 ? (int) csr_off(a, bh, j + 2) : 0x7fffffff;
-        load_fold(j);
+        j = j2; nxt = nxt2;
+        fold_buf ^= 1;
+        if (!(ok = tc::warp_wait(&s_full[warp][kRingFineStages], kvph, ctl))) break;
+        kvph ^= 1;
+        constexpr int KV = kRingFineStages * kRingFineStageBytes, TB = kRingTileBytes;
+        rowfrag_sa<KV>(klo, sa_f, sa_f ^ 16);
+        rowfrag_sa<KV + 1024>(khi, sa_f, sa_f ^ 16);
+        rowfrag_sa<KV + TB>(vlo, sa_f, sa_f ^ 16);
+        rowfrag_sa<KV + TB + 1024>(vhi, sa_f, sa_f ^ 16);
         tile_zero(dk, dv);
       }
       // the stage read an entry ago is free: its operands were consumed by products already issued
-      if (i + kRingFineStages - 1 < n) request(i + kRingFineStages - 1);
-      const uint4 P = load_pds_t<2 * kRingTileBytes>(sa_l16 + so), D = load_pds_t<2 * kRingTileBytes + 512>(sa_l16 + so);
-      uint32_t bd[4][4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) ldsm_x4_trans<kRingTileBytes>(bd[c][0], bd[c][1], bd[c][2], bd[c][3], sa_m[c] + so);
+      request(i + kRingFineStages - 1);
+      // S^T = K.Q^T and dP^T = V.dO^T: rows = keys g, g + 8, columns = queries 2t, 2t + 1 (s0, e0) and 8 more (s1, e1)
+      float s0[4], s1[4], e0[4], e1[4];
+      const uint32_t f0 = sa_f + so, f1 = (sa_f ^ 16) + so;
+      half_rows_x_keys<0, true>(s0, s1, klo, khi, f0);
+      half_rows_x_keys<kRingTileBytes, true>(e0, e1, vlo, vhi, f0);
+      half_rows_x_keys<0, false>(s0, s1, klo, khi, f1);
+      half_rows_x_keys<kRingTileBytes, false>(e0, e1, vlo, vhi, f1);
+      const uint32_t sa_s = stat_sa + st * kRingStatBytes + 8 * t;
+      auto half = [&](const float2 l, const float2 d, const float (&s)[4], const float (&p)[4], uint32_t& P0, uint32_t& P1, uint32_t& D0, uint32_t& D1) {
+        const F2 nl = f2_mul(f2(l.x, l.y), f2(-kLog2e, -kLog2e)), nd = f2(-d.x, -d.y), sc = f2(sl2, sl2);
+        float x0, x1, y0, y1;
+        f2_get(f2_fma(f2(s[0], s[1]), sc, nl), x0, x1);
+        f2_get(f2_fma(f2(s[2], s[3]), sc, nl), y0, y1);
+        x0 = fast_exp2(x0); x1 = fast_exp2(x1); y0 = fast_exp2(y0); y1 = fast_exp2(y1);
+        P0 = pack_bf16(x0, x1);
+        P1 = pack_bf16(y0, y1);
+        f2_get(f2_mul(f2(x0, x1), f2_add(f2(p[0], p[1]), nd)), x0, x1);
+        f2_get(f2_mul(f2(y0, y1), f2_add(f2(p[2], p[3]), nd)), y0, y1);
+        D0 = pack_bf16(x0, x1);
+        D1 = pack_bf16(y0, y1);
+      };
+      uint4 P, D;                                     // P^T and dS^T / scale as A operands
+      half(lds64f<0>(sa_s), lds64f<64>(sa_s), s0, e0, P.x, P.y, D.x, D.y);
+      half(lds64f<32>(sa_s), lds64f<96>(sa_s), s1, e1, P.z, P.w, D.z, D.w);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        uint32_t bq[4];
-        ldsm_x4_trans<0>(bq[0], bq[1], bq[2], bq[3], sa_m[c] + so);
-        mma_bf16_16816(dv[2 * c], P.x, P.y, P.z, P.w, bd[c][0], bd[c][1]);
-        mma_bf16_16816(dv[2 * c + 1], P.x, P.y, P.z, P.w, bd[c][2], bd[c][3]);
-#pragma unroll
-        for (int x = 0; x < 4; ++x) bd[c][x] = bq[x];
+        uint32_t bd[4];
+        ldsm_x4_trans<kRingTileBytes>(bd[0], bd[1], bd[2], bd[3], (sa_m ^ (c << 5)) + so);
+        mma_bf16_16816(dv[2 * c], P.x, P.y, P.z, P.w, bd[0], bd[1]);
+        mma_bf16_16816(dv[2 * c + 1], P.x, P.y, P.z, P.w, bd[2], bd[3]);
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        mma_bf16_16816(dk[2 * c], D.x, D.y, D.z, D.w, bd[c][0], bd[c][1]);
-        mma_bf16_16816(dk[2 * c + 1], D.x, D.y, D.z, D.w, bd[c][2], bd[c][3]);
+        uint32_t bq[4];
+        ldsm_x4_trans<0>(bq[0], bq[1], bq[2], bq[3], (sa_m ^ (c << 5)) + so);
+        mma_bf16_16816(dk[2 * c], D.x, D.y, D.z, D.w, bq[0], bq[1]);
+        mma_bf16_16816(dk[2 * c + 1], D.x, D.y, D.z, D.w, bq[2], bq[3]);
+      }
+      if (fresh && nxt < re) {                        // K and V have been consumed: the next bucket's may overwrite them
+        find_bucket(nxt);
+        request_bucket();
       }
       if (st == kRingFineStages - 1) { st = 0; ph ^= 1; } else { ++st; }
     }
     if (!ok) break;
     __syncwarp();
     // the last bucket of the span; the ring is idle by now
-    if (bo >= rb && nxt <= re) {
-      park_fold();
-      dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, 0, sa_fold, lane);
+    if (!began_before && nxt <= re) {
+      dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, 0, fold_sa + fold_buf * kRingFoldBytes + 8 * t, lane);
     } else if (PERSISTENT) {
-      tile_to_mem(pieces + (bo >= rb ? kTileFloats : 0), dk, dv, lane);     // continues in the next window, or lies across the whole of this one
-    } else if (bo < rb) {                   // the whole range lies inside one bucket that began earlier
+      tile_to_mem(pieces + (began_before ? 0 : kTileFloats), dk, dv, lane);     // lies across the whole window or ends here, or continues in the next
+    } else if (began_before) {
       tile_to_mem(slots + warp * kTileFloats, dk, dv, lane);
       if (lane == 0) s_head_bucket[warp] = j;
     } else {
-      park_fold();
       tail_j = j;                           // continues in later warps (or windows): completed below
     }
   }
@@ -824,7 +814,7 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
     if (tail_j >= 0) {
       for (int w = warp + 1; w < kRingWarps && s_head_bucket[w] == tail_j; ++w) tile_add_mem(slots + w * kTileFloats, dk, dv, lane);
       if ((int) csr_off(a, bh, tail_j + 1) <= ce) {
-        dkv_fine_store_staged(a, b, h, tail_j, dk, dv, sa_m, sa_cp, 0, sa_fold, lane);
+        dkv_fine_store_staged(a, b, h, tail_j, dk, dv, sa_m, sa_cp, 0, fold_sa + fold_buf * kRingFoldBytes + 8 * t, lane);
       } else {                                // runs on into the next window: this window's tail slot
         tile_to_mem(pieces + kTileFloats, dk, dv, lane);
       }
@@ -1016,6 +1006,8 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     int rc;
     if ((rc = tma::make_map_bhnd(&maps.q, g->q, kBS))) return rc;
     if ((rc = tma::make_map_bhnd(&maps.d_o, g->d_o, kBS))) return rc;
+    if ((rc = tma::make_map_bhnd(&maps.k, g->k, kBS))) return rc;
+    if ((rc = tma::make_map_bhnd(&maps.v, g->v, kBS))) return rc;
     if (a.range_entries == kRangeEntries) {
       int dev = 0, sms = 148;
       LLSA_CUDA_OK(cudaGetDevice(&dev));

@@ -238,12 +238,11 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
   const int64_t R = (E + S - 1) / S;
   const size_t t_scratch = llsa_transpose_scratch_bytes(d.B, d.H, d.nq1, topk, d.n1);
   const int64_t n_partial = tensor_core ? llsa_attn_bwd_partial_elems(d.B, d.H, d.Nq, topk) : 0;
-  const int64_t n_pds = tensor_core ? llsa_attn_bwd_pds_elems(d.B, d.H, d.Nq, topk) : 0;
   const int64_t acc1 = BH * d.n1 * D, acc2 = c.two ? BH * d.n2 * D : 0;
   Carver cv;
   const int64_t o_off = cv.take(BH * (d.n1 + 1) * 4), o_flat = cv.take(BH * E * 4), o_pairs = cv.take(BH * E * 4), o_ranges = cv.take(BH * R * 8),
                 o_ts = cv.take((int64_t) t_scratch), o_delta = cv.take(BH * d.Nq * 4),
-                o_acc = cv.take(acc ? 0 : (2 * acc1 + 2 * acc2) * 4), o_partial = cv.take(n_partial * 4), o_pds = cv.take(n_pds * 4);
+                o_acc = cv.take(acc ? 0 : (2 * acc1 + 2 * acc2) * 4), o_partial = cv.take(n_partial * 4);
   const Tensor ws = byte_buffer(cv.off, like);
   char* p = (char*) ws.data_ptr();
   if (!acc) acc = (float*) (p + o_acc);
@@ -252,8 +251,7 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
                    delta = packed(p + o_delta, LLSA_F32, {d.B, d.H, d.Nq}), dpk = packed(acc, LLSA_F32, {d.B, d.H, d.n1, D}),
                    dpv = packed(acc + acc1, LLSA_F32, {d.B, d.H, d.n1, D}), dpk2 = packed(acc + 2 * acc1, LLSA_F32, {d.B, d.H, d.n2, D}),
                    dpv2 = packed(acc + 2 * acc1 + acc2, LLSA_F32, {d.B, d.H, d.n2, D}),
-                   partial = packed(p + o_partial, LLSA_F32, {d.B, d.H, BH ? n_partial / (BH * 4096) : 0, 4096}),
-                   pds = packed(p + o_pds, LLSA_F32, {n_pds});
+                   partial = packed(p + o_partial, LLSA_F32, {d.B, d.H, BH ? n_partial / (BH * 4096) : 0, 4096});
   const Status t_status(like), status(like);
 
   const at::cuda::CUDAStream cur = at::cuda::getCurrentCUDAStream(like.device().index());
@@ -271,7 +269,7 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
   a.offsets = &offsets; a.flat = &flat; a.delta = &delta;
   a.dpk_acc = &dpk; a.dpv_acc = &dpv;
   if (c.two) { a.dpk2_acc = &dpk2; a.dpv2_acc = &dpv2; }
-  if (tensor_core) { a.dkv_partial = &partial; a.fine_pds = &pds; a.flat_pairs = &pairs; a.flat_ranges = &ranges; }
+  if (tensor_core) { a.dkv_partial = &partial; a.flat_pairs = &pairs; a.flat_ranges = &ranges; }
   a.fold_pool_bwd = fold;
   a.kv_weight = (float) kvw1; a.kv_weight_2 = (float) kvw2;
   a.status = status.ptr();
