@@ -237,11 +237,7 @@ typedef struct LlsaAttnArgs {
                                   of llsa_attn_bwd_partial_elems() elements for dK/dV tiles of KV
                                   blocks whose list of query blocks is split over several CTAs (not
                                   read before it is written; may be NULL for f32 tensors) */
-  const LlsaTensor* fine_pds;  /* backward, bf16 tensors only: F32-typed scratch of
-                                  llsa_attn_bwd_pds_elems() elements.  The dQ stage (stage_mask 1)
-                                  leaves P and dS (bf16) of every (query block, selected block) pair
-                                  here and the dK/dV stage (stage_mask 4) reads them instead of
-                                  recomputing both from q, k, v, lse and delta */
+  const LlsaTensor* fine_pds;  /* not used any more (the dK/dV stage recomputes P and dS); may be NULL */
   const LlsaTensor* flat_pairs;/* backward, bf16 tensors only: I32 [B,H,N/16*topk], the `pairs` list of
                                   llsa_transpose_indices_pairs for the same CSR as offsets / flat */
   const LlsaTensor* flat_ranges;/* backward, bf16 tensors only: I32 [B,H,ceil(N/16*topk/S),2], the `ranges`
@@ -278,7 +274,8 @@ int llsa_attn_bwd(const LlsaAttnArgs* args, void* stream);
  * Nq query rows per (b,h) and `topk` selected blocks per query block (the caller allocates it; any 4-D contiguous
  * shape with at least this many elements is accepted).  The library itself never allocates device memory. */
 int64_t llsa_attn_bwd_partial_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk);
-/* Element count (4-byte elements) of LlsaAttnArgs.fine_pds: 1 KB per (query block, selected block) pair. */
+/* Element count (4-byte elements) LlsaAttnArgs.fine_pds used to need: 1 KB per (query block, selected block) pair.  No scratch of this
+ * size is needed any more. */
 int64_t llsa_attn_bwd_pds_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk);
 
 #ifdef __cplusplus

@@ -16,15 +16,13 @@
 //                          16 query blocks and add the 16x64 results into fp32
 //                          accumulators (one red.add per element and group).
 //   attn_dq_fine_kernel    the same for the fine blocks alone (the pooled keys then run on
-//                          tcgen05); both dQ kernels leave P and dS of every (query block,
-//                          selected block) pair in a scratch tensor for the next kernel.
-//   attn_dkv_fine_ring_kernel  the CSR of a head is cut into equal windows of 128 entries
-//                          (one CTA, 32 entries per warp) so every warp runs the same
-//                          number of steps however skewed the fan-in is; an entry is
-//                          dV += P^T.dO, dK += dS^T.Q with P, dS read back; tiles of
-//                          buckets that straddle a range meet in shared memory / a
-//                          global partial tensor (no atomics), and
-//   attn_dkv_finish_kernel sums the window partials; every store folds in the pooling
+//                          tcgen05)
+//   attn_dkv_fine_ring_kernel  the CSR of a head is cut into ranges of equal length (32
+//                          entries, buckets of up to that many kept whole), one warp each,
+//                          however skewed the fan-in is; an entry is S^T, dP^T, then
+//                          dV += P^T.dO, dK += dS^T.Q; pieces of longer buckets meet in
+//                          a global partial tensor (no atomics), and
+//   attn_dkv_finish_kernel sums the pieces; every store folds in the pooling
 //                          backward (dk += (dpk[j] + dpk2[j/16]/16)/16), one bf16 store.
 // The reference multiplies k by scale into new tensors first (res_1.py:420-422);
 // here scale rides in the exp2 argument and in the epilogues.
@@ -226,7 +224,9 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_mma_kernel(AttnP<bf16> a, 
 }
 
 // Fine blocks only (the pooled keys are on the tcgen05 kernels): one warp per query block; the selected K / V blocks go through a per-warp
-// ring in shared memory, filled by TMA two blocks ahead.
+// ring in shared memory, filled by TMA two blocks ahead, and K is read a second time, transposed, by ldmatrix.  Bound by the gather from
+// L2: 4 KB per (query block, selected block), 9.9 TB/s at 8 x 6 slices of 16384 tokens (158 us; 205 with P and dS, 1 KB per pair, written
+// out for the dK/dV stage).
 constexpr int kDqStages = 3;
 struct KvMaps {
   CUtensorMap k, v;            // [B,H,N,64] 4-D, box 16 rows
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a,
   for (int gi = 0; gi < n_glob; ++gi) {
     if (!(ok = tc::warp_wait(&s_full[warp][st], ph, ctl))) break;
     if (gi + kDqStages - 1 < n_glob) request(gi + kDqStages - 1);      // into the stage read last time: its operands were consumed by products already issued
-    const uint32_t so = st * kStageBytes, f0 = sa_f + so, f1 = (sa_f ^ 16) + so, m0 = sa_m + so;
+    const uint32_t so = st * kStageBytes, f0 = sa_f + so, f1 = f0 ^ 16, m0 = sa_m + so;
     float s0[4], s1[4], p0[4], p1[4];
     half_rows_x_keys<0, true>(s0, s1, qlo, qhi, f0);
     half_rows_x_keys<kRingTileBytes, true>(p0, p1, dlo, dhi, f0);
@@ -468,21 +468,23 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 
 // ---- fine dK/dV kernel ------------------------------------------------------------------------------
 // dV_j += P^T.dO and dK_j += dS^T.Q over the query blocks that selected KV block j (reference:
-// sparse_attention_res_2.py:371-415, the dK/dV half of _attn_bwd_res_dqkv).  P and dS are NOT recomputed here: the dQ
-// stage has left them, already transposed into A-operand registers, in `pds` (store_pds), so an entry costs two
-// 512-byte loads, the Q and dO tiles of its query block and 16 MMAs; K, V, lse and delta are not touched.
-//   * The Q / dO tiles come through a per-warp cp.async ring of kRingFineStages stages, three entries ahead, and are
-//     read with ldmatrix.trans (the B operand of a contraction over the tile's 16 rows).
-//   * The P^T / dS^T registers of the entry three ahead are requested with plain 128-bit loads into a rotating set
-//     of register buffers (two CTAs of four warps per SM leave 255 registers per thread).
-//   * A warp owns one range of the entry list, a CTA four consecutive ranges (its window).  The index transpose cuts
-//     the ranges so that a bucket of up to kRangeEntries entries is never split and hands over each range's first
-//     bucket, so a warp starts without a search.  A longer bucket is cut at multiples of kRangeEntries: a warp parks
-//     the tile of a bucket it shares with EARLIER warps in its shared-memory slot; the tile it shares with later warps
-//     stays in its accumulators until the CTA has synchronised and is then completed from their slots; pieces of
-//     buckets that straddle windows go to the `partial` scratch and attn_dkv_finish_kernel adds them in window order.
-//   * The pooled-gradient rows a finished tile folds in (the pooling backward) are requested into registers when
-//     the bucket begins and parked in shared memory right before the store.
+// sparse_attention_res_2.py:371-415, the dK/dV half of _attn_bwd_res_dqkv).
+//   * S^T = K.Q^T and dP^T = V.dO^T come out with rows = keys, which is the A operand of the two products that follow: nothing is
+//     transposed.  K and V of the bucket stay in registers as A operands.
+//   * The Q / dO tiles of an entry come through a per-warp ring of kRingFineStages stages, two entries ahead, as two TMA copies issued
+//     by one lane (plus one 4-byte copy per lane: lse and delta); K, V and the pooled-gradient rows of the next bucket through a buffer
+//     of their own, requested as soon as those of the bucket at hand sit in registers.
+//   * Two forms.  PERSISTENT (ranges of kRangeEntries, i.e. problems of some 4,700 ranges and more): one CTA of twelve warps per SM; a
+//     window is two ranges, a warp draws one range after another from a counter in shared memory, and where a long bucket crosses from
+//     the first range of a window into the second one warp takes both.  Otherwise (ranges of half that size): one CTA of four warps per
+//     window of four ranges, every range on a warp at once; a warp parks the tile of a bucket it shares with EARLIER warps in its
+//     shared-memory slot, the tile it shares with later ones stays in its accumulators until the CTA has synchronised.
+//     Pieces of buckets that straddle windows go to the `partial` scratch and attn_dkv_finish_kernel adds them in window order.
+// What bounds it: issue slots (0.42 instructions per scheduler and cycle with three warps on each; some 290 instructions per entry), then
+// the raggedness of the last ranges.  With P and dS handed over by the dQ stage instead of recomputed this kernel issued half as much,
+// but 1 KB per entry went out to HBM and came back: at 8 x 6 slices of 16384 tokens, top 8, dQ stage 205 -> 158 us and this one 192 -> 255
+// on random inputs, 207 -> 164 and 284 -> 255 on correlated ones; at 6 of 262144 421 -> 315 and 563 -> 460 (the first figures of the
+// correlated pairs with eight warps per SM in groups of four that waited for the longest of their ranges: 322 and 645 on random inputs).
 // Accumulator layout (ldmatrix): tile u holds channels 8u + 2t, 8u + 2t + 1 of keys g (c0, c1) and g + 8 (c2, c3).
 constexpr int kRingWarps = 4;                   // warps per CTA, one window per CTA
 constexpr int kRingWarpsP = 12;                 // warps per CTA, one persistent CTA per SM
@@ -498,38 +500,35 @@ struct FineMaps {
   CUtensorMap q, d_o, k, v;    // [B,H,N,64] 4-D, box 16 rows
 };
 
-// Pooling-backward fold and scale for the ldmatrix accumulator layout: afterwards dk / dv hold the final fp32 values.
-// The four gradient rows of KV block j come from this warp's copy in shared memory ([dpk | dpv | dpk2 | dpv2] x 64 fp32, fetched with
-// cp.async when the bucket began); sa_fold already includes the lane's 8t bytes.
-__device__ __forceinline__ void dkv_fine_fold_smem(const AttnP<bf16>& a, uint32_t sa_fold, float (&dk)[8][4], float (&dv)[8][4]) {
+// Pooling-backward fold and scale for the ldmatrix accumulator layout: afterwards dk / dv hold the final fp32 values.  The gradient rows
+// [dpk | dpv | dpk2 | dpv2] x 64 fp32 of the bucket lie at `fold`; a lane first combines four channels of one tensor in place.
+template <int U>
+__device__ __forceinline__ void fold_tile(const AttnP<bf16>& a, uint32_t sa, float (&dk)[8][4], float (&dv)[8][4]) {
+  if constexpr (U < 8) {
+    const float2 ek = lds64f<32 * U>(sa), ev = lds64f<32 * U + 256>(sa);
+    dk[U][0] = fmaf(dk[U][0], a.scale, ek.x); dk[U][1] = fmaf(dk[U][1], a.scale, ek.y);
+    dk[U][2] = fmaf(dk[U][2], a.scale, ek.x); dk[U][3] = fmaf(dk[U][3], a.scale, ek.y);
+    dv[U][0] += ev.x; dv[U][1] += ev.y; dv[U][2] += ev.x; dv[U][3] += ev.y;
+    fold_tile<U + 1>(a, sa, dk, dv);
+  }
+}
+__device__ __forceinline__ void dkv_fine_fold_smem(const AttnP<bf16>& a, uint32_t fold, float (&dk)[8][4], float (&dv)[8][4], int lane) {
   if (a.fold) {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      float2 ek, ev;
-      if (u == 0) { ek = lds64f<0>(sa_fold); ev = lds64f<256>(sa_fold); }
-      if (u == 1) { ek = lds64f<32>(sa_fold); ev = lds64f<256 + 32>(sa_fold); }
-      if (u == 2) { ek = lds64f<64>(sa_fold); ev = lds64f<256 + 64>(sa_fold); }
-      if (u == 3) { ek = lds64f<96>(sa_fold); ev = lds64f<256 + 96>(sa_fold); }
-      if (u == 4) { ek = lds64f<128>(sa_fold); ev = lds64f<256 + 128>(sa_fold); }
-      if (u == 5) { ek = lds64f<160>(sa_fold); ev = lds64f<256 + 160>(sa_fold); }
-      if (u == 6) { ek = lds64f<192>(sa_fold); ev = lds64f<256 + 192>(sa_fold); }
-      if (u == 7) { ek = lds64f<224>(sa_fold); ev = lds64f<256 + 224>(sa_fold); }
-      if (a.two_level) {
-        float2 fk, fv;
-        if (u == 0) { fk = lds64f<512>(sa_fold); fv = lds64f<768>(sa_fold); }
-        if (u == 1) { fk = lds64f<512 + 32>(sa_fold); fv = lds64f<768 + 32>(sa_fold); }
-        if (u == 2) { fk = lds64f<512 + 64>(sa_fold); fv = lds64f<768 + 64>(sa_fold); }
-        if (u == 3) { fk = lds64f<512 + 96>(sa_fold); fv = lds64f<768 + 96>(sa_fold); }
-        if (u == 4) { fk = lds64f<512 + 128>(sa_fold); fv = lds64f<768 + 128>(sa_fold); }
-        if (u == 5) { fk = lds64f<512 + 160>(sa_fold); fv = lds64f<768 + 160>(sa_fold); }
-        if (u == 6) { fk = lds64f<512 + 192>(sa_fold); fv = lds64f<768 + 192>(sa_fold); }
-        if (u == 7) { fk = lds64f<512 + 224>(sa_fold); fv = lds64f<768 + 224>(sa_fold); }
-        ek.x += fk.x * (1.f / kBS); ek.y += fk.y * (1.f / kBS); ev.x += fv.x * (1.f / kBS); ev.y += fv.y * (1.f / kBS);
-      }
-      dk[u][0] = dk[u][0] * a.scale + ek.x * (1.f / kBS); dk[u][1] = dk[u][1] * a.scale + ek.y * (1.f / kBS);
-      dk[u][2] = dk[u][2] * a.scale + ek.x * (1.f / kBS); dk[u][3] = dk[u][3] * a.scale + ek.y * (1.f / kBS);
-      dv[u][0] += ev.x * (1.f / kBS); dv[u][1] += ev.y * (1.f / kBS); dv[u][2] += ev.x * (1.f / kBS); dv[u][3] += ev.y * (1.f / kBS);
+    const uint32_t sa = fold + 16 * lane;
+    uint4 e;
+    lds128<0>(e.x, e.y, e.z, e.w, sa);
+    float x[4] = {__uint_as_float(e.x), __uint_as_float(e.y), __uint_as_float(e.z), __uint_as_float(e.w)};
+    if (a.two_level) {
+      uint4 f;
+      lds128<512>(f.x, f.y, f.z, f.w, sa);
+      x[0] += __uint_as_float(f.x) * (1.f / kBS); x[1] += __uint_as_float(f.y) * (1.f / kBS);
+      x[2] += __uint_as_float(f.z) * (1.f / kBS); x[3] += __uint_as_float(f.w) * (1.f / kBS);
     }
+    __syncwarp();
+    sts128<0>(sa, make_uint4(__float_as_uint(x[0] * (1.f / kBS)), __float_as_uint(x[1] * (1.f / kBS)), __float_as_uint(x[2] * (1.f / kBS)),
+                             __float_as_uint(x[3] * (1.f / kBS))));
+    __syncwarp();
+    fold_tile<0>(a, fold + 8 * (lane & 3), dk, dv);
   } else {
 #pragma unroll
     for (int u = 0; u < 8; ++u) { dk[u][0] *= a.scale; dk[u][1] *= a.scale; dk[u][2] *= a.scale; dk[u][3] *= a.scale; }
@@ -541,9 +540,9 @@ __device__ __forceinline__ void dkv_fine_fold_smem(const AttnP<bf16>& a, uint32_
 // eight lanes write one whole 128-byte row: full sectors, 8 store instructions instead of 32.
 __device__ __forceinline__ void dkv_fine_store_staged(const AttnP<bf16>& a, int64_t b, int64_t h, int64_t j, float (&dk)[8][4],
                                                       float (&dv)[8][4], uint32_t sa_m, uint32_t sa_cp, uint32_t so,
-                                                      uint32_t sa_fold, int lane) {
+                                                      uint32_t fold, int lane) {
   constexpr int TB = kRingTileBytes;
-  dkv_fine_fold_smem(a, sa_fold, dk, dv);
+  dkv_fine_fold_smem(a, fold, dk, dv, lane);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     stsm_x4<0>((sa_m ^ (c << 5)) + so, pack_bf16(dk[2 * c][0], dk[2 * c][1]), pack_bf16(dk[2 * c][2], dk[2 * c][3]),
@@ -728,7 +727,7 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
       if (fresh) {                                    // next non-empty bucket; the stage read an entry ago stages the store
         if (j >= 0) {
           if (!began_before) {
-            dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, rst * kRingFineStageBytes, fold_sa + fold_buf * kRingFoldBytes + 8 * t, lane);
+            dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, rst * kRingFineStageBytes, fold_sa + fold_buf * kRingFoldBytes, lane);
           } else {                                    // began in an earlier span
             tile_to_mem(PERSISTENT ? pieces : slots + warp * kTileFloats, dk, dv, lane);
             if (!PERSISTENT && lane == 0) s_head_bucket[warp] = j;
@@ -750,7 +749,7 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
       request(i + kRingFineStages - 1);
       // S^T = K.Q^T and dP^T = V.dO^T: rows = keys g, g + 8, columns = queries 2t, 2t + 1 (s0, e0) and 8 more (s1, e1)
       float s0[4], s1[4], e0[4], e1[4];
-      const uint32_t f0 = sa_f + so, f1 = (sa_f ^ 16) + so;
+      const uint32_t f0 = sa_f + so, f1 = f0 ^ 16, m0 = sa_m + so;
       half_rows_x_keys<0, true>(s0, s1, klo, khi, f0);
       half_rows_x_keys<kRingTileBytes, true>(e0, e1, vlo, vhi, f0);
       half_rows_x_keys<0, false>(s0, s1, klo, khi, f1);
@@ -775,14 +774,14 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t bd[4];
-        ldsm_x4_trans<kRingTileBytes>(bd[0], bd[1], bd[2], bd[3], (sa_m ^ (c << 5)) + so);
+        ldsm_x4_trans<kRingTileBytes>(bd[0], bd[1], bd[2], bd[3], m0 ^ (c << 5));
         mma_bf16_16816(dv[2 * c], P.x, P.y, P.z, P.w, bd[0], bd[1]);
         mma_bf16_16816(dv[2 * c + 1], P.x, P.y, P.z, P.w, bd[2], bd[3]);
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t bq[4];
-        ldsm_x4_trans<0>(bq[0], bq[1], bq[2], bq[3], (sa_m ^ (c << 5)) + so);
+        ldsm_x4_trans<0>(bq[0], bq[1], bq[2], bq[3], m0 ^ (c << 5));
         mma_bf16_16816(dk[2 * c], D.x, D.y, D.z, D.w, bq[0], bq[1]);
         mma_bf16_16816(dk[2 * c + 1], D.x, D.y, D.z, D.w, bq[2], bq[3]);
       }
@@ -796,7 +795,7 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
     __syncwarp();
     // the last bucket of the span; the ring is idle by now
     if (!began_before && nxt <= re) {
-      dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, 0, fold_sa + fold_buf * kRingFoldBytes + 8 * t, lane);
+      dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, 0, fold_sa + fold_buf * kRingFoldBytes, lane);
     } else if (PERSISTENT) {
       tile_to_mem(pieces + (began_before ? 0 : kTileFloats), dk, dv, lane);     // lies across the whole window or ends here, or continues in the next
     } else if (began_before) {
@@ -814,7 +813,7 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
     if (tail_j >= 0) {
       for (int w = warp + 1; w < kRingWarps && s_head_bucket[w] == tail_j; ++w) tile_add_mem(slots + w * kTileFloats, dk, dv, lane);
       if ((int) csr_off(a, bh, tail_j + 1) <= ce) {
-        dkv_fine_store_staged(a, b, h, tail_j, dk, dv, sa_m, sa_cp, 0, fold_sa + fold_buf * kRingFoldBytes + 8 * t, lane);
+        dkv_fine_store_staged(a, b, h, tail_j, dk, dv, sa_m, sa_cp, 0, fold_sa + fold_buf * kRingFoldBytes, lane);
       } else {                                // runs on into the next window: this window's tail slot
         tile_to_mem(pieces + kTileFloats, dk, dv, lane);
       }

@@ -1,0 +1,47 @@
+"""Fine dK/dV kernel in its persistent form (lists of 4,736 ranges and more) against the oracle."""
+import pytest
+import torch
+
+import llsa_b200
+from llsa_b200 import synth
+from oracle import llsa_oracle as O
+from test_gpu_parity import rel_l2
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _close(got, ref, name):
+    """bf16 operands (Q, K, V, P, dS) and a bf16 result: every rounding is relative, 2^-9 of the value or of a term of its sum, so the error
+    scales with the largest value of the tensor.  The sums have random signs: 5 x 2^-9 = 1e-2 covers five such roundings in the norm and
+    2e-2 of the largest value ten in one element."""
+    got, ref = got.detach().float().cpu(), ref.detach().float().cpu()
+    assert rel_l2(got, ref) <= 1e-2, name
+    assert float((got - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max())), name
+
+
+# 32 and 3 ranges per head (an odd number leaves a window of one range); hot: key blocks every query block selects, i.e. lists of N / 16
+# entries that are cut between windows and inside them, next to blocks nobody selects
+@pytest.mark.parametrize("B,H,N,topk,hot", [(37, 4, 2048, 8, ()), (37, 4, 2048, 8, (3,)), (37, 4, 2048, 8, (0, 1, 127)), (264, 6, 768, 2, ()),
+                                            (264, 6, 768, 2, (3,)), (264, 6, 768, 2, (0, 47))])
+def test_persistent_form_vs_oracle(B, H, N, topk, hot):
+    q, k, v, do = synth.gaussian_qkv(N + len(hot), 2, H, N, 64, dtype=torch.bfloat16)
+    u = torch.ones(64) * 0.35
+    if hot:
+        q = (q.float() + u).to(torch.bfloat16)
+        for j in hot:
+            k[:, :, 16 * j:16 * j + 16] = (k[:, :, 16 * j:16 * j + 16].float() + 4 * u).to(torch.bfloat16)
+    rep = (B + 1) // 2
+    Q, K, V, DO = [t.to(DEV).repeat(rep, 1, 1, 1)[:B].contiguous() for t in (q, k, v, do)]
+    Q, K, V = [t.requires_grad_(True) for t in (Q, K, V)]
+    dbg = llsa_b200.llsa_l1_debug(Q, K, V, topk, 16)
+    dbg["o"].backward(DO)
+    idx, pk, pv = [dbg[n][:2].cpu() for n in ("indices", "pk", "pv")]
+    assert all(bool((idx == j).any(-1).all()) for j in hot)
+    o_ref, lse_ref = O.attn_fwd_l1(q, k, v, pk, pv, idx, faithful=False)
+    dq, dk, dv, dpk, dpv = O.attn_bwd_l1(do, q, k, v, pk, pv, o_ref.float(), lse_ref, idx, faithful=False)
+    last = slice(2 * (rep - 1), B)                        # the same inputs again at the end of the batch
+    for sl, n in ((slice(0, 2), 2), (last, B - 2 * (rep - 1))):
+        _close(Q.grad[sl], dq[:n], "dq")
+        _close(K.grad[sl], (dk + O.mean_pool1d_bwd(dpk, 16))[:n], "dk")
+        _close(V.grad[sl], (dv + O.mean_pool1d_bwd(dpv, 16))[:n], "dv")
