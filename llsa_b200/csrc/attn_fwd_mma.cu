@@ -16,10 +16,14 @@
 // The softmax runs online, one 16-key block at a time, in the exp2 domain; a
 // pooled key's weight enters as +log2(weight) on its logit, which is what
 // `l += l_ij * W; acc += P.V * W` in the reference amounts to.
+#include <string.h>
+
 #include <type_traits>
 
 #include "attn.cuh"
 #include "mma_frag.cuh"
+#include "tc05.cuh"
+#include "tma.cuh"
 
 namespace llsa {
 
@@ -173,228 +177,170 @@ __global__ void __launch_bounds__(NW * 32, 2) attn_fwd_mma_kernel(AttnP<bf16> a,
   }
 }
 
-// Fine stage alone (the pooled stages then run on tcgen05, attn_pooled_tc.cu, and merge into the
-// o / lse written here).  Every selected K/V block costs a full L2/HBM round trip, far longer
-// than the 16 MMAs it feeds, so each warp keeps kFineStages-1 blocks in flight with cp.async
-// into its own ring of shared-memory stages (mma_frag.cuh) and reads the fragments from there.
+// Fine stage alone (the pooled stages then run on tcgen05, attn_pooled_tc.cu, and merge into the o / lse written here): one warp per query
+// block.  The selected K / V tiles go through a per-warp ring of three stages, two tiles of one tensor each, filled by TMA two stages
+// ahead (one lane issues; no address arithmetic, no shared-memory store slots).  The blocks are taken GP pairs at a time: the S tiles of a
+// group first, one softmax update, then P.V with V read by ldmatrix.trans.  Four blocks a group (GP = 2) halve the updates against two;
+// GP = 1 is for a top-k that is not a multiple of four.  Bound by the gather from L2, 4 KB per (query block, selected block).
 constexpr int kFineStages = 3;
+constexpr int kFineStageBytes = 2 * kRingTileElems * (int) sizeof(bf16);
+struct FineKvMaps {
+  CUtensorMap k, v;            // [B,H,N,64] 4-D, box 16 rows
+};
 
-template <int NW>
-__global__ void __launch_bounds__(NW * 32, 2) attn_fwd_fine_kernel(AttnP<bf16> a) {
+// One lane requests rows [r0, r0 + 16) and [r1, r1 + 16) of one (head, batch) as neighbouring 2 KB tiles.
+__device__ __forceinline__ void load_two_tiles_w(uint32_t dst, const CUtensorMap* m, uint64_t* bar, int r0, int r1, int h, int b) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t.reg .b32 d;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "add.u32 d, %0, 2048;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], 4096;\n\t"
+      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%7, %3, %5, %6}], [%2];\n\t"
+      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [d], [%1, {%7, %4, %5, %6}], [%2];\n\t"
+      "}" ::"r"(dst), "l"(m), "r"(tc::smem_u32(bar)), "r"(r0), "r"(r1), "r"(h), "r"(b), "r"(0)
+      : "memory");
+}
+
+template <int NW, int GP>
+__global__ void __launch_bounds__(NW * 32, 16 / NW) attn_fwd_fine_kernel(AttnP<bf16> a, const __grid_constant__ FineKvMaps maps) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t s_full[NW][kFineStages];
+  __shared__ tc::WaitCtl s_ctl[NW];             // a warp's own: the warps of a CTA share nothing
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t ring_sa = ((tc::smem_u32(smem_raw) + 1023u) & ~1023u) + warp * kFineStages * kFineStageBytes;
+  volatile tc::WaitCtl* ctl = &s_ctl[warp];
+  if (lane < kFineStages) tc::mbar_init(&s_full[warp][lane], 1);
+  if (lane == 0) {
+    ctl->abort = 0;
+    ctl->limit = a.wait_limit > 0 ? a.wait_limit : tc::kWaitPolls;
+  }
+  tc::fence_mbar_init();
+  __syncwarp();
   pdl_trigger();
   pdl_wait();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  bf16* ring = reinterpret_cast<bf16*>(smem_raw) + warp * (kFineStages * 2 * kRingTileElems);
   const int64_t qb = (int64_t) blockIdx.x * NW + warp, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
-  const int my_fine = lane < a.topk ? (int) fine_block(a, bh, qb, lane) : 0;
-  const float sl2 = a.scale * 1.4426950408889634f;
-  const int n_glob = a.topk;
-  // A lane copies the same four 16-byte chunks of every K tile and of every V tile (chunk = 4 i + lane / 8 -> row, lane % 8 ->
-  // column): their global and shared-memory offsets are computed once, a block costs two base pointers and eight adds.
-  int off_k[4], off_v[4], off_s[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = i * 4 + (lane >> 3), c = lane & 7;
-    off_k[i] = r * (int) a.k.sn + c * 8;
-    off_v[i] = r * (int) a.v.sn + c * 8;
-    off_s[i] = r * 64 + ((c ^ (r & 7)) << 3);
-  }
-  // fragment read offsets inside a ring tile (rows r and r + 8 share r & 7, so the second row is 8 * 64 elements further)
-  const int rd_k[2] = {g * 64 + (((2 * t) ^ (g & 7)) << 3), g * 64 + (((2 * t + 1) ^ (g & 7)) << 3)};
-  const int rd_v[2] = {(2 * t) * 64 + ((g ^ ((2 * t) & 7)) << 3), (2 * t + 1) * 64 + ((g ^ ((2 * t + 1) & 7)) << 3)};
-  const bf16* kb0 = a.k.row(b, h, 0);
-  const bf16* vb0 = a.v.row(b, h, 0);
-  const int64_t kblk = (int64_t) kBS * a.k.sn, vblk = (int64_t) kBS * a.v.sn;
-  auto issue = [&](int i) {
-    const int64_t j = __shfl_sync(0xffffffffu, my_fine, i);
-    bf16* stage = ring + (i % kFineStages) * 2 * kRingTileElems;
-    const bf16* kp = kb0 + j * kblk;
-    const bf16* vp = vb0 + j * vblk;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      cp_async16(stage + off_s[u], kp + off_k[u]);
-      cp_async16(stage + kRingTileElems + off_s[u], vp + off_v[u]);
-    }
+  const int my_row = lane < a.topk ? (int) fine_block(a, bh, qb, lane) * kBS : 0;
+  int rst = 0;
+  auto request = [&](const CUtensorMap* m, int pair) {
+    load_two_tiles_w(ring_sa + rst * kFineStageBytes, m, &s_full[warp][rst], __shfl_sync(0xffffffffu, my_row, 2 * pair),
+                     __shfl_sync(0xffffffffu, my_row, 2 * pair + 1), (int) h, (int) b);
+    rst = rst == kFineStages - 1 ? 0 : rst + 1;
   };
-#pragma unroll
-  for (int s = 0; s < kFineStages - 1; ++s) {
-    if (s < n_glob) issue(s);
-    cp_async_commit();
-  }
-  RowFrag qlo, qhi;
-  load_rowfrag(qlo, a.q.row(b, h, qb * kBS + g), t);
-  load_rowfrag(qhi, a.q.row(b, h, qb * kBS + g + 8), t);
-  FwdState st;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) st.o[j][0] = st.o[j][1] = st.o[j][2] = st.o[j][3] = 0.f;
-  st.m0 = st.m1 = -INFINITY;
-  st.l0 = st.l1 = 0.f;
-  for (int gi = 0; gi < n_glob; ++gi) {
-    cp_async_wait_group<kFineStages - 2>();     // block gi has landed (this lane's chunks) ...
-    __syncwarp();                               // ... and everybody else's; the stage read last time is free
-    if (gi + kFineStages - 1 < n_glob) issue(gi + kFineStages - 1);
-    cp_async_commit();
-    const bf16* tk = ring + (gi % kFineStages) * 2 * kRingTileElems;
-    RowFrag k0, k1;
-    {
-      const uint4 x0 = *reinterpret_cast<const uint4*>(tk + rd_k[0]), x1 = *reinterpret_cast<const uint4*>(tk + rd_k[1]);
-      const uint4 y0 = *reinterpret_cast<const uint4*>(tk + 8 * 64 + rd_k[0]), y1 = *reinterpret_cast<const uint4*>(tk + 8 * 64 + rd_k[1]);
-      k0.r[0] = x0.x; k0.r[1] = x0.y; k0.r[2] = x0.z; k0.r[3] = x0.w; k0.r[4] = x1.x; k0.r[5] = x1.y; k0.r[6] = x1.z; k0.r[7] = x1.w;
-      k1.r[0] = y0.x; k1.r[1] = y0.y; k1.r[2] = y0.z; k1.r[3] = y0.w; k1.r[4] = y1.x; k1.r[5] = y1.y; k1.r[6] = y1.z; k1.r[7] = y1.w;
-    }
-    uint32_t pa[4];
-    fwd_scores(st, qlo, qhi, k0, k1, sl2, 0.f, pa);
-    ColFrag v;
-    v.row[0] = *reinterpret_cast<const uint4*>(tk + kRingTileElems + rd_v[0]);
-    v.row[1] = *reinterpret_cast<const uint4*>(tk + kRingTileElems + rd_v[1]);
-    v.row[2] = *reinterpret_cast<const uint4*>(tk + kRingTileElems + 8 * 64 + rd_v[0]);
-    v.row[3] = *reinterpret_cast<const uint4*>(tk + kRingTileElems + 8 * 64 + rd_v[1]);
-    mma_x_cols(st.o, pa[0], pa[1], pa[2], pa[3], v);
-  }
-  const float l0 = quad_sum(st.l0), l1 = quad_sum(st.l1);
-  store_acc_row<0>(a.o.row(b, h, qb * kBS + g), st.o, t, 1.f / l0);
-  store_acc_row<1>(a.o.row(b, h, qb * kBS + g + 8), st.o, t, 1.f / l1);
-  if (t == 0) {
-    a.lse[bh * a.Nq + qb * kBS + g] = (st.m0 + log2f(l0)) * 0.6931471805599453f;
-    a.lse[bh * a.Nq + qb * kBS + g + 8] = (st.m1 + log2f(l1)) * 0.6931471805599453f;
-  }
-}
-
-// ---- eight fine blocks, second form ----------------------------------------------------------------
-// The kernel above spends most of its issue slots around the MMAs: an online-softmax update (maximum, rescale of the 16x64
-// output) per 16-key block, byte permutes for the V operand, run-time ring addresses.  This form, for top-8, takes the blocks in
-// two halves of four: the four S tiles of a half are computed first, the softmax statistics are updated once per half, and P.V
-// follows with V read by ldmatrix.trans.  The sixteen K / V tiles go through a per-warp ring of six 2 KB stages in the order
-// K0..K3 V0..V3 K4..K7 V4..V7, five tiles ahead; the loop is unrolled over the tiles so that every shared-memory offset is an
-// immediate.  The output leaves through stmatrix into a free stage and 128-bit row stores.
-constexpr int kF8Stages = 6;
-constexpr int kF8TileBytes = kRingTileElems * (int) sizeof(bf16);
-
-template <int I, int N, typename F>
-__device__ __forceinline__ void static_for(F&& f) {
-  if constexpr (I < N) {
-    f(std::integral_constant<int, I>{});
-    static_for<I + 1, N>(f);
-  }
-}
-
-template <int NW>
-__global__ void __launch_bounds__(NW * 32, 2) attn_fwd_fine8_kernel(AttnP<bf16> a) {
-  pdl_trigger();
-  pdl_wait();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  // the swizzle arithmetic works on absolute shared addresses: start at a 128-byte boundary (the launch adds 128 bytes)
-  const uint32_t smem_sa = ((uint32_t) __cvta_generic_to_shared(smem_raw) + 127u) & ~127u;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const uint32_t ring_sa = smem_sa + warp * (kF8Stages * kF8TileBytes);
-  const uint32_t sa_cp0 = ring_sa + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4), sa_cp1 = sa_cp0 ^ 64;
-  const uint32_t sa_f0 = ring_sa + g * 128 + (((2 * t) ^ g) << 4), sa_f1 = sa_f0 ^ 16;
+  // the stages come as the K pairs of a group, then its V pairs; two are requested ahead
+  request(&maps.k, 0);
+  if constexpr (GP == 2) request(&maps.k, 1); else request(&maps.v, 0);
+  // shared addresses of stage 0: chunks 2t, 2t + 1 of row g (sa_f, sa_f ^ 16; row g + 8 is 1024 bytes on), ldmatrix rows of channels 0..15
+  // (sa_m; ^ 32 c: channels 16c..)
+  const uint32_t sa_f = ring_sa + g * 128 + (((2 * t) ^ g) << 4);
   const uint32_t sa_m = ring_sa + ((lane & 7) + ((lane >> 3) & 1) * 8) * 128 + (((lane >> 4) ^ (lane & 7)) << 4);
-  const int64_t qb = (int64_t) blockIdx.x * NW + warp, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
-  const int my_fine = lane < 8 ? (int) fine_block(a, bh, qb, lane) : 0;
-  const float sl2 = a.scale * 1.4426950408889634f;
-  const char* k_lane = reinterpret_cast<const char*>(a.k.row(b, h, lane >> 3) + (lane & 7) * 8);
-  const char* v_lane = reinterpret_cast<const char*>(a.v.row(b, h, lane >> 3) + (lane & 7) * 8);
-  const int kblk = (int) (kBS * a.k.sn * sizeof(bf16)), vblk = (int) (kBS * a.v.sn * sizeof(bf16));
-  // tile s of the sequence K0..K3 V0..V3 K4..K7 V4..V7
-  auto issue = [&](auto s_tag) {
-    constexpr int s = decltype(s_tag)::value, blk = (s / 8) * 4 + s % 4, ST = (s % kF8Stages) * kF8TileBytes;
-    constexpr bool is_v = (s % 8) >= 4;
-    const int j = __shfl_sync(0xffffffffu, my_fine, blk);
-    const int blkb = is_v ? vblk : kblk;
-    const char* p = (is_v ? v_lane : k_lane) + (int64_t) j * blkb;
-    cp_async16_sa<ST>(sa_cp0, p);
-    cp_async16_sa<ST + 512>(sa_cp1, p + (blkb >> 2));
-    cp_async16_sa<ST + 1024>(sa_cp0, p + (blkb >> 1));
-    cp_async16_sa<ST + 1536>(sa_cp1, p + 3 * (blkb >> 2));
-  };
-  static_for<0, kF8Stages - 1>([&](auto s_tag) {
-    issue(s_tag);
-    cp_async_commit();
-  });
   RowFrag qlo, qhi;
   load_rowfrag(qlo, a.q.row(b, h, qb * kBS + g), t);
   load_rowfrag(qhi, a.q.row(b, h, qb * kBS + g + 8), t);
-  float o[8][4], sc[4][2][4];
-  uint32_t pa[4][4];
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-  static_for<0, 16>([&](auto s_tag) {
-    constexpr int s = decltype(s_tag)::value, half = s / 8, i = s % 4, ST = (s % kF8Stages) * kF8TileBytes;
-    constexpr bool is_v = (s % 8) >= 4;
-    cp_async_wait_group<kF8Stages - 2>();       // tile s has landed (this lane's chunks) ...
-    __syncwarp();                               // ... and everybody else's; the stage read last time is free
-    if constexpr (s + kF8Stages - 1 < 16) issue(std::integral_constant<int, s + kF8Stages - 1>{});
-    cp_async_commit();
-    if constexpr (!is_v) {
-      half_rows_x_keys<ST, true>(sc[i][0], sc[i][1], qlo, qhi, sa_f0);
-      half_rows_x_keys<ST, false>(sc[i][0], sc[i][1], qlo, qhi, sa_f1);
-      if constexpr (i == 3) {                   // the half's four S tiles are complete: one softmax update for 64 keys
-        float x0 = -INFINITY, x1 = -INFINITY;
+  const float sl2 = a.scale * 1.4426950408889634f;
+  const F2 sl22 = f2(sl2, sl2);
+  float o[8][4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+  for (int j = 0; j < 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+  float m0 = -INFINITY, m1 = -INFINITY;
+  F2 l0 = f2(0.f, 0.f), l1 = f2(0.f, 0.f);      // per-lane partial sums of rows g, g + 8; reduced over the quad at the end
+  const int n_pairs = a.topk / 2;
+  int st = 0, ph = 0;
+  bool ok = true;
+  auto advance = [&]() {
+    if (st == kFineStages - 1) { st = 0; ph ^= 1; } else { ++st; }
+  };
+  for (int gp = 0; gp < n_pairs; gp += GP) {
+    float sc[2 * GP][2][4];
+    uint32_t pa[2 * GP][4];
 #pragma unroll
-          for (int n = 0; n < 2; ++n) {
-            x0 = fmax3(x0, sc[u][n][0], sc[u][n][1]);
-            x1 = fmax3(x1, sc[u][n][2], sc[u][n][3]);
-          }
-        const float mn0 = fmaxf(m0, quad_max(x0) * sl2), mn1 = fmaxf(m1, quad_max(x1) * sl2);
-        if constexpr (half > 0) {
-          const float al0 = fast_exp2(m0 - mn0), al1 = fast_exp2(m1 - mn1);
-          l0 *= al0; l1 *= al1;
-#pragma unroll
-          for (int u = 0; u < 8; ++u) { o[u][0] *= al0; o[u][1] *= al0; o[u][2] *= al1; o[u][3] *= al1; }
-        }
-        m0 = mn0; m1 = mn1;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-#pragma unroll
-          for (int n = 0; n < 2; ++n) {
-            sc[u][n][0] = fast_exp2(fmaf(sc[u][n][0], sl2, -mn0)); sc[u][n][1] = fast_exp2(fmaf(sc[u][n][1], sl2, -mn0));
-            sc[u][n][2] = fast_exp2(fmaf(sc[u][n][2], sl2, -mn1)); sc[u][n][3] = fast_exp2(fmaf(sc[u][n][3], sl2, -mn1));
-            l0 += sc[u][n][0] + sc[u][n][1];    // per-lane partial sums; reduced over the quad at the end
-            l1 += sc[u][n][2] + sc[u][n][3];
-          }
-          // the two C tiles of S are the k16 halves of the A operand
-          pa[u][0] = pack_bf16(sc[u][0][0], sc[u][0][1]); pa[u][1] = pack_bf16(sc[u][0][2], sc[u][0][3]);
-          pa[u][2] = pack_bf16(sc[u][1][0], sc[u][1][1]); pa[u][3] = pack_bf16(sc[u][1][2], sc[u][1][3]);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r0, r1, r2, r3;
-        ldsm_x4_trans<ST>(r0, r1, r2, r3, sa_m ^ (c << 5));
-        if constexpr (s == 4) {                 // first product: no accumulator input
-          mma_bf16_16816_z(o[2 * c], pa[i][0], pa[i][1], pa[i][2], pa[i][3], r0, r1);
-          mma_bf16_16816_z(o[2 * c + 1], pa[i][0], pa[i][1], pa[i][2], pa[i][3], r2, r3);
-        } else {
-          mma_bf16_16816(o[2 * c], pa[i][0], pa[i][1], pa[i][2], pa[i][3], r0, r1);
-          mma_bf16_16816(o[2 * c + 1], pa[i][0], pa[i][1], pa[i][2], pa[i][3], r2, r3);
-        }
-      }
+    for (int p = 0; p < GP; ++p) {
+      if (!(ok = tc::warp_wait(&s_full[warp][st], ph, ctl))) break;
+      // into the stage read last time: its operands were consumed by products already issued
+      if constexpr (GP == 2) request(&maps.v, gp + p);
+      else if (gp + 1 < n_pairs) request(&maps.k, gp + 1);
+      const uint32_t f0 = sa_f + st * kFineStageBytes, f1 = f0 ^ 16;
+      half_rows_x_keys<0, true>(sc[2 * p][0], sc[2 * p][1], qlo, qhi, f0);
+      half_rows_x_keys<2048, true>(sc[2 * p + 1][0], sc[2 * p + 1][1], qlo, qhi, f0);
+      half_rows_x_keys<0, false>(sc[2 * p][0], sc[2 * p][1], qlo, qhi, f1);
+      half_rows_x_keys<2048, false>(sc[2 * p + 1][0], sc[2 * p + 1][1], qlo, qhi, f1);
+      advance();
     }
-  });
-  l0 = quad_sum(l0); l1 = quad_sum(l1);
-  const float i0 = 1.f / l0, i1 = 1.f / l1;
-  if (t == 0) {
-    a.lse[bh * a.Nq + qb * kBS + g] = (m0 + log2f(l0)) * 0.6931471805599453f;
-    a.lse[bh * a.Nq + qb * kBS + g + 8] = (m1 + log2f(l1)) * 0.6931471805599453f;
+    if (!ok) break;
+    float x0 = -INFINITY, x1 = -INFINITY;
+#pragma unroll
+    for (int u = 0; u < 2 * GP; ++u)
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        x0 = fmax3(x0, sc[u][n][0], sc[u][n][1]);
+        x1 = fmax3(x1, sc[u][n][2], sc[u][n][3]);
+      }
+    const float mn0 = fmaxf(m0, quad_max(x0) * sl2), mn1 = fmaxf(m1, quad_max(x1) * sl2);
+    if (gp > 0) {
+      const float al0 = fast_exp2(m0 - mn0), al1 = fast_exp2(m1 - mn1);
+      l0 = f2_mul(l0, f2(al0, al0)); l1 = f2_mul(l1, f2(al1, al1));
+#pragma unroll
+      for (int u = 0; u < 8; ++u) { o[u][0] *= al0; o[u][1] *= al0; o[u][2] *= al1; o[u][3] *= al1; }
+    }
+    m0 = mn0; m1 = mn1;
+    const F2 nm0 = f2(-mn0, -mn0), nm1 = f2(-mn1, -mn1);
+    auto probs = [&](float y0, float y1, F2 nm, F2& l) {
+      f2_get(f2_fma(f2(y0, y1), sl22, nm), y0, y1);
+      y0 = fast_exp2(y0); y1 = fast_exp2(y1);
+      l = f2_add(l, f2(y0, y1));
+      return pack_bf16(y0, y1);
+    };
+#pragma unroll
+    for (int u = 0; u < 2 * GP; ++u) {          // the two C tiles of S are the k16 halves of the A operand
+      pa[u][0] = probs(sc[u][0][0], sc[u][0][1], nm0, l0); pa[u][1] = probs(sc[u][0][2], sc[u][0][3], nm1, l1);
+      pa[u][2] = probs(sc[u][1][0], sc[u][1][1], nm0, l0); pa[u][3] = probs(sc[u][1][2], sc[u][1][3], nm1, l1);
+    }
+#pragma unroll
+    for (int p = 0; p < GP; ++p) {
+      if (!(ok = tc::warp_wait(&s_full[warp][st], ph, ctl))) break;
+      if (gp + GP < n_pairs) request(GP == 2 ? &maps.k : &maps.v, gp + GP + p);
+      const uint32_t vm = sa_m + st * kFineStageBytes;
+      auto product = [&](auto imm, const uint32_t (&w)[4]) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r0, r1, r2, r3;
+          ldsm_x4_trans<decltype(imm)::value>(r0, r1, r2, r3, vm ^ (c << 5));
+          mma_bf16_16816(o[2 * c], w[0], w[1], w[2], w[3], r0, r1);
+          mma_bf16_16816(o[2 * c + 1], w[0], w[1], w[2], w[3], r2, r3);
+        }
+      };
+      product(std::integral_constant<int, 0>{}, pa[2 * p]);
+      product(std::integral_constant<int, 2048>{}, pa[2 * p + 1]);
+      advance();
+    }
+    if (!ok) break;
   }
-  // accumulator tile u holds channels 8u + 2t, 8u + 2t + 1 of rows g (c0, c1) and g + 8 (c2, c3): through stage 0 to whole rows
+  if (!ok) {
+    tc::abort_drain();
+    if (lane == 0 && a.status) atomicOr(a.status, (int) LLSA_DEV_WAIT_EXPIRED);
+    return;
+  }
+  float y0, y1, z0, z1;
+  f2_get(l0, y0, y1); f2_get(l1, z0, z1);
+  const float s0 = quad_sum(y0 + y1), s1 = quad_sum(z0 + z1), i0 = 1.f / s0, i1 = 1.f / s1;
+  if (t == 0) {
+    a.lse[bh * a.Nq + qb * kBS + g] = (m0 + log2f(s0)) * 0.6931471805599453f;
+    a.lse[bh * a.Nq + qb * kBS + g + 8] = (m1 + log2f(s1)) * 0.6931471805599453f;
+  }
+  // accumulator tile u holds channels 8u + 2t, 8u + 2t + 1 of rows g (c0, c1) and g + 8 (c2, c3): through the idle ring to whole rows
   __syncwarp();
 #pragma unroll
   for (int c = 0; c < 4; ++c)
     stsm_x4<0>(sa_m ^ (c << 5), pack_bf16(o[2 * c][0] * i0, o[2 * c][1] * i0), pack_bf16(o[2 * c][2] * i1, o[2 * c][3] * i1),
                pack_bf16(o[2 * c + 1][0] * i0, o[2 * c + 1][1] * i0), pack_bf16(o[2 * c + 1][2] * i1, o[2 * c + 1][3] * i1));
   __syncwarp();
+  const uint32_t sa_cp = ring_sa + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4);
   bf16* op = a.o.row(b, h, qb * kBS + (lane >> 3)) + (lane & 7) * 8;
   const int64_t os = 4 * a.o.sn;
   uint4 x;
-  lds128<0>(x.x, x.y, x.z, x.w, sa_cp0);    *reinterpret_cast<uint4*>(op) = x;
-  lds128<512>(x.x, x.y, x.z, x.w, sa_cp1);  *reinterpret_cast<uint4*>(op + os) = x;
-  lds128<1024>(x.x, x.y, x.z, x.w, sa_cp0); *reinterpret_cast<uint4*>(op + 2 * os) = x;
-  lds128<1536>(x.x, x.y, x.z, x.w, sa_cp1); *reinterpret_cast<uint4*>(op + 3 * os) = x;
+  lds128<0>(x.x, x.y, x.z, x.w, sa_cp);         *reinterpret_cast<uint4*>(op) = x;
+  lds128<512>(x.x, x.y, x.z, x.w, sa_cp ^ 64);  *reinterpret_cast<uint4*>(op + os) = x;
+  lds128<1024>(x.x, x.y, x.z, x.w, sa_cp);      *reinterpret_cast<uint4*>(op + 2 * os) = x;
+  lds128<1536>(x.x, x.y, x.z, x.w, sa_cp ^ 64); *reinterpret_cast<uint4*>(op + 3 * os) = x;
 }
 
 // A bf16 call whose operands miss the tensor-core kernels' limits still runs, on the scalar kernels and many times
@@ -432,17 +378,22 @@ int launch_attn_fwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
   const bool loop_tc = !pooled_tc_keys(a) && pooled_loop_tc_keys(a) > 0;
   if ((pooled_tc_keys(a) || loop_tc) && !g->no_tcgen05) {
     // fine blocks on mma.sync (o and lse of the fine part alone), pooled keys on tcgen05, merged there
-    if (a.topk == 8) {
-      const size_t ring = (size_t) NW * kF8Stages * kF8TileBytes + 128;
-      LLSA_SMEM_LIMIT((attn_fwd_fine8_kernel<NW>), ring);
-      launch_pdl(attn_fwd_fine8_kernel<NW>, dim3((unsigned) (a.nq1 / NW), (unsigned) BH), NW * 32, ring, st, a);
-      LLSA_LAUNCH_OK("attn_fwd_fine8_kernel");
+    FineKvMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    int rc;
+    if ((rc = tma::make_map_bhnd(&maps.k, g->k, kBS))) return rc;
+    if ((rc = tma::make_map_bhnd(&maps.v, g->v, kBS))) return rc;
+    constexpr int NWF = 4;
+    const size_t ring = (size_t) NWF * kFineStages * kFineStageBytes + 1024;
+    const dim3 fine_grid((unsigned) (a.nq1 / NWF), (unsigned) BH);
+    if (a.topk % 4 == 0) {
+      LLSA_SMEM_LIMIT((attn_fwd_fine_kernel<NWF, 2>), ring);
+      launch_pdl(attn_fwd_fine_kernel<NWF, 2>, fine_grid, NWF * 32, ring, st, a, maps);
     } else {
-      const size_t ring = (size_t) NW * kFineStages * 2 * kRingTileElems * sizeof(bf16);
-      LLSA_SMEM_LIMIT((attn_fwd_fine_kernel<NW>), ring);
-      launch_pdl(attn_fwd_fine_kernel<NW>, dim3((unsigned) (a.nq1 / NW), (unsigned) BH), NW * 32, ring, st, a);
-      LLSA_LAUNCH_OK("attn_fwd_fine_kernel");
+      LLSA_SMEM_LIMIT((attn_fwd_fine_kernel<NWF, 1>), ring);
+      launch_pdl(attn_fwd_fine_kernel<NWF, 1>, fine_grid, NWF * 32, ring, st, a, maps);
     }
+    LLSA_LAUNCH_OK("attn_fwd_fine_kernel");
     return loop_tc ? launch_attn_fwd_pooled_loop_tc(g, a, BH, st) : launch_attn_fwd_pooled_tc(g, a, BH, st);
   }
   const int n_smem = pooled_smem_tiles(a.p1_blocks + a.p2_blocks);

@@ -124,10 +124,6 @@ __device__ __forceinline__ float2 lds64f(uint32_t sa) {
   asm volatile("ld.shared.v2.f32 {%0,%1}, [%2+%3];" : "=f"(v.x), "=f"(v.y) : "r"(sa), "n"(IMM));
   return v;
 }
-template <int IMM>
-__device__ __forceinline__ void cp_async16_sa(uint32_t sa, const void* gsrc) {
-  asm volatile("cp.async.cg.shared.global [%0+%1], [%2], 16;" ::"r"(sa), "n"(IMM), "l"(gsrc) : "memory");
-}
 // RowFrag of tile row (g or g+8: ROWOFF) from a swizzled ring tile: chunks 2t and 2t+1 of the row sit at sa0 / sa1
 template <int IMM>
 __device__ __forceinline__ void rowfrag_sa(RowFrag& f, uint32_t sa0, uint32_t sa1) {

@@ -16,7 +16,7 @@ import json
 import os
 
 GROUPS = {
-    "attn_fwd": ("attn_fwd_fine8_kernel", "attn_fwd_fine_kernel", "attn_fwd_pooled_tc_kernel", "attn_fwd_pooled_loop_tc_kernel", "attn_fwd_mma_kernel"),
+    "attn_fwd": ("attn_fwd_fine_kernel", "attn_fwd_pooled_tc_kernel", "attn_fwd_pooled_loop_tc_kernel", "attn_fwd_mma_kernel"),
     "attn_bwd_dq": ("attn_dq_fine_kernel", "attn_dq_mma_kernel"),
     "attn_bwd_dkv_pooled": ("attn_bwd_pooled_tc_kernel", "attn_dkv_pooled_kernel", "attn_dq_pooled_loop_tc_kernel", "attn_dkv_pooled_loop_tc_kernel"),
     "attn_bwd_dkv_fine": ("attn_dkv_fine_ring_kernel", "attn_dkv_finish_kernel"),
