@@ -255,7 +255,7 @@ typedef struct LlsaAttnArgs {
                                   that walks the pooled key list chunk by chunk (any number of pooled keys
                                   per row but 64, 128 and 192) makes ONE pass over the keys with the fine part's log-sum-exp as the
                                   reference of its exponentials, marks here the rows whose pooled keys
-                                  outweigh the fine ones by more than 1e30, and a second launch redoes
+                                  outweigh the fine ones by more than 1e30, and redoes
                                   exactly those rows with the exact two-pass form.  NULL: two passes for
                                   every row.  Same results either way up to rounding */
 } LlsaAttnArgs;

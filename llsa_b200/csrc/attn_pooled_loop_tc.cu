@@ -15,8 +15,8 @@
 // part through their log-sum-exp, so the fine part's log-sum-exp (already known per row) serves as the reference of the
 // exponentials, P = exp2(S' - lse_fine).  Anything below 2^-126 of the fine part's weight is irrelevant, and bf16 / fp32
 // hold anything up to 2^127 times it; a row whose pooled keys outweigh its fine keys by more than that (its row sum
-// passes 1e30, or is NaN) is left untouched and marked in `redo`, and a second launch of the two-pass form redoes
-// exactly the marked rows (it scans its tiles' marks first and returns at once when there are none).
+// passes 1e30, or is NaN) is left untouched and marked in `redo`; a CTA that has marked a row of its tiles goes over them again
+// with two passes and writes exactly the marked rows.  (A second launch that looked for marks cost every call 1 to 2 us.)
 // Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64):
 //   warp 8, warp 11  : TMA producers: Q per tile (2 stages) and K chunks (ring of 4; every chunk is loaded in both passes); V chunks (ring
 //                      of 4, pass 2 only)
@@ -64,13 +64,34 @@ struct LoopBars {
   uint64_t s_ready[kBufs], wg_done[kBufs], buf_free[kBufs], o_ready[2], o_free[2], sum_ready[2], xchg;
 };
 
+__device__ __forceinline__ void init_bars(LoopBars& bars) {
+  for (int i = 0; i < 2; ++i) {
+    tc::mbar_init(&bars.q_full[i], 1);
+    tc::mbar_init(&bars.q_empty[i], 1);
+  }
+  for (int i = 0; i < kBufs; ++i) {
+    tc::mbar_init(&bars.s_ready[i], 1);
+    tc::mbar_init(&bars.wg_done[i], 4);         // one arrival per warp of the group
+    tc::mbar_init(&bars.buf_free[i], 1);
+  }
+  for (int i = 0; i < kKStages; ++i) { tc::mbar_init(&bars.k_full[i], 1); tc::mbar_init(&bars.k_empty[i], 1); }
+  for (int i = 0; i < kVStages; ++i) { tc::mbar_init(&bars.v_full[i], 1); tc::mbar_init(&bars.v_empty[i], 1); }
+  for (int i = 0; i < 2; ++i) {
+    tc::mbar_init(&bars.o_ready[i], 1);
+    tc::mbar_init(&bars.o_free[i], 4);
+    tc::mbar_init(&bars.sum_ready[i], 8);
+  }
+  tc::mbar_init(&bars.xchg, 8);
+  tc::fence_mbar_init();
+}
+
 // n_chunks: chunks per tile; gathered: how many of them, the first ones, are gathered level-1 blocks (two levels); n_c: rows per
 // head of the contiguous pooled tensor.
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps maps, int n_chunks, int gathered, int64_t n_c, int n_tiles,
-                               int tiles_per_head, int n_pass, unsigned char* redo) {
+                               int tiles_per_head, unsigned char* redo) {
   extern __shared__ unsigned char smem_dyn[];
-  __shared__ LoopBars bars;
+  __shared__ LoopBars bars_of[2];                    // of the first round over the tiles and of the one for marked rows
   __shared__ uint32_t s_tmem;
   __shared__ tc::WaitCtl s_ctl;
   __shared__ float s_max[2][2][kRows];               // [tile parity][group][row]: row maxima after pass 1
@@ -82,36 +103,10 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile tc::WaitCtl* abort_flag = &s_ctl;
   const int n_my = (n_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x;
-  if (n_pass == 2 && redo) {
-    pdl_wait();
-    // the second launch: anything to redo in this CTA's tiles?  (a tile's 128 marks are 32 words)
-    int any = 0;
-    for (int i = warp; i < n_my; i += kThreads / 32)
-      any |= (int) reinterpret_cast<const uint32_t*>(redo)[(int64_t) (blockIdx.x + i * gridDim.x) * (kRows / 4) + lane];
-    if (!__syncthreads_or(any)) return;
-  }
-
   if (tid == 0) {
     s_ctl.abort = 0;
     s_ctl.limit = a.wait_limit > 0 ? a.wait_limit : tc::kWaitPolls;
-    for (int i = 0; i < 2; ++i) {
-      tc::mbar_init(&bars.q_full[i], 1);
-      tc::mbar_init(&bars.q_empty[i], 1);
-    }
-    for (int i = 0; i < kBufs; ++i) {
-      tc::mbar_init(&bars.s_ready[i], 1);
-      tc::mbar_init(&bars.wg_done[i], 4);         // one arrival per warp of the group
-      tc::mbar_init(&bars.buf_free[i], 1);
-    }
-    for (int i = 0; i < kKStages; ++i) { tc::mbar_init(&bars.k_full[i], 1); tc::mbar_init(&bars.k_empty[i], 1); }
-    for (int i = 0; i < kVStages; ++i) { tc::mbar_init(&bars.v_full[i], 1); tc::mbar_init(&bars.v_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) {
-      tc::mbar_init(&bars.o_ready[i], 1);
-      tc::mbar_init(&bars.o_free[i], 4);
-      tc::mbar_init(&bars.sum_ready[i], 8);
-    }
-    tc::mbar_init(&bars.xchg, 8);
-    tc::fence_mbar_init();
+    init_bars(bars_of[0]);
   }
   pdl_wait();
   if (warp == 0) tc::tmem_alloc(&s_tmem, 512);
@@ -120,272 +115,281 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   tc::fence_after_sync();
   pdl_trigger();
   const uint32_t tmem = s_tmem;
-  // jobs per tile; job j of tile i has the CTA-wide number i * jobs + j, which picks the S buffer (mod 3) and the softmax
-  // group (mod 2; with one pass and an odd chunk count the parity of a tile's first job alternates)
-  const int jobs = n_pass * n_chunks, first_p2 = jobs - n_chunks;
-  // keys of chunk c that belong to its list (a multiple of 32)
-  auto keys_of = [&](int c) {
-    const int left = c < gathered ? a.p1_blocks * kBS - c * kChunk : (int) n_c - (c - gathered) * kChunk;
-    return left < kChunk ? left : kChunk;
-  };
-
-  if (warp == 8 || warp == 11) {
-    // ---------------------------------------------------------------- TMA producers: warp 8 Q and keys, warp 11 values
-    const bool vals = warp == 11;
-    uint64_t *full = vals ? bars.v_full : bars.k_full, *empty = vals ? bars.v_empty : bars.k_empty;
-    const CUtensorMap *mg = vals ? &maps.vg : &maps.kg, *mc = vals ? &maps.vc : &maps.kc;
-    bf16* ring = vals ? sV : sK;
-    static_assert(kKStages == kVStages, "one loop for both rings");
-    int st = 0;
-    uint32_t ph = 1;
-    bool ok = true;
-    for (int i = 0; ok && i < n_my; ++i) {
-      const int tile = blockIdx.x + i * gridDim.x, qs = i & 1;
-      const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
-      if (!vals) {
-        if (!(ok = tc::warp_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag))) break;
-        tma::expect_tx_w(&bars.q_full[qs], kTile * 2);
-        tma::load_4d_w(sQ + qs * kTile, &maps.q, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
-      }
-      int krow = 0;                                           // lane j: first row of gathered block j
-      if (gathered) krow = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, min(lane, a.p1_blocks - 1)) * kBS);
-      int crow = (int) ((int64_t) bh * n_c);                  // next contiguous chunk
-      for (int j = vals ? first_p2 : 0; j < jobs; ++j) {
-        const int c = j >= n_chunks ? j - n_chunks : j;
-        if (!(ok = tc::warp_wait(&empty[st], ph, abort_flag))) break;
-        tma::expect_tx_w(&full[st], kTile * 2);
-        if (c < gathered) {
-#pragma unroll
-          for (int b8 = 0; b8 < 8; ++b8) tma::load_2d_w(ring + st * kTile + b8 * kBS * 64, mg, &full[st], 0, __shfl_sync(0xffffffffu, krow, (c * 8 + b8) & 31));
-        } else {
-          if (c == gathered) crow = (int) ((int64_t) bh * n_c);
-          tma::load_2d_w(ring + st * kTile, mc, &full[st], 0, crow);
-          crow += kChunk;
-        }
-        if (++st == kKStages) { st = 0; ph ^= 1; }
-      }
-    }
-  } else if (warp == 9) {
-    // ---------------------------------------------------------------- MMA issuer 1: S of every job
-    {
-      const uint32_t id_s = tc::instr_desc(kRows, kChunk, 0, 0);
-      const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
-      auto lo = [](const void* p, uint32_t lbo_bytes) { return ((tc::smem_u32(p) >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16); };
-      constexpr uint32_t kStage = (uint32_t) (kTile * 2) >> 4;
-      const uint32_t lQ = lo(sQ, 16), lK = lo(sK, 16);
-      int n = 0, ks = 0, buf = 0;                   // jobs issued so far; K ring stage and S buffer of the next one
-      uint32_t kph = 0, bph = 0;                    // their phase parities
-      bool ok = true;
-      for (int i = 0; ok && i < n_my; ++i) {
-        const int qs = i & 1;
-        if (!(ok = tc::warp_wait(&bars.q_full[qs], (i >> 1) & 1, abort_flag))) break;
-        const uint32_t q_ = lQ + qs * kStage;
-        for (int j = 0; j < jobs; ++j, ++n) {
-          // even lanes: the key chunk; odd lanes: the buffer's previous job (three back), whose group has read S and, in pass 2, P.V P
-          const bool b = (lane & 1) && n >= kBufs;
-          if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : &bars.k_full[ks], b ? bph ^ 1 : kph, abort_flag))) break;
-          tc::fence_after_sync();
-          const uint32_t k_ = lK + ks * kStage, d = tmem + buf * kChunk;
-          tc::umma_ss_k64(d, q_, hi, k_, hi, id_s);
-          tc::umma_commit_w(&bars.s_ready[buf]);
-          tc::umma_commit_w(&bars.k_empty[ks]);
-          if (++ks == kKStages) { ks = 0; kph ^= 1; }
-          if (++buf == kBufs) { buf = 0; bph ^= 1; }
-        }
-        if (!ok) break;
-        tc::umma_commit_w(&bars.q_empty[qs]);
-      }
-    }
-  } else if (warp == 10) {
-    // ---------------------------------------------------------------- MMA issuer 2: O (+)= P(job, TMEM) . V chunk
-    {
-      const uint32_t id_o = tc::instr_desc(kRows, 64, 0, 1);
-      const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
-      constexpr uint32_t kStage = (uint32_t) (kTile * 2) >> 4;
-      const uint32_t lV = ((tc::smem_u32(sV) >> 4) & 0x3FFFu) | ((1024u >> 4) << 16);
-      int vs = 0, buf = 0;
-      uint32_t vph = 0, bph = 0;
-      bool ok = true;
-      for (int i = 0; ok && i < n_my; ++i) {
-        for (int j = 0; j < jobs; ++j) {
-          // even lanes: the group's job; odd lanes of a pass-2 job: the value chunk; lane 3: O of the tile before the last has been read
-          const bool pv = j >= first_p2;
-          const int c = j - first_p2;
-          uint64_t* bar = &bars.wg_done[buf];
-          uint32_t par = bph;
-          if (pv && lane == 3 && c == 0 && i > 1) { bar = &bars.o_free[i & 1]; par = ((i - 2) >> 1) & 1; }
-          else if (pv && (lane & 1)) { bar = &bars.v_full[vs]; par = vph; }
-          if (!(ok = tc::warp_wait(bar, par, abort_flag))) break;
-          if (pv) {
-            tc::fence_after_sync();
-            const uint32_t v_ = lV + vs * kStage, p_ = tmem + buf * kChunk, o_ = tmem + kColO + (i & 1) * 64;
-            // P: 16 keys = 8 packed columns per k-step; V: 16 key rows = 2048 bytes
-            const int ksteps = keys_of(c) / 16;
-            const uint32_t acc = c > 0 ? 1u : 0u;
-            if (ksteps >= 4) {
-              if (ksteps == 8) tc::umma_ts_k128(o_, p_, v_, hi, id_o, acc);
-              else tc::umma_ts_k64(o_, p_, v_, hi, id_o, acc);
-            }
-            if (ksteps & 2) tc::umma_ts_k32(o_, p_ + (ksteps == 6 ? 32 : 0), v_ + (ksteps == 6 ? 512 : 0), hi, id_o, ksteps == 6 ? 1u : acc);
-            tc::umma_commit_w(&bars.v_empty[vs]);
-            if (++vs == kVStages) { vs = 0; vph ^= 1; }
-          }
-          tc::umma_commit_w(&bars.buf_free[buf]);
-          if (++buf == kBufs) { buf = 0; bph ^= 1; }
-        }
-        if (!ok) break;
-        tc::umma_commit_w(&bars.o_ready[i & 1]);
-      }
-    }
-  } else if (warp < 8) {
-    // ---------------------------------------------------------------- softmax, thread = query row
-    const int wg = warp >> 2, qd = warp & 3, r = qd * 32 + lane;
-    const float sl2 = a.scale * kLog2eF;
-    const float lw1 = log2f(a.w1), lw2 = log2f(a.w2);
-    const uint32_t t_lane = tmem + ((uint32_t) (qd * 32) << 16);
-    int buf = wg;                          // S buffer of this group's next job (it takes every other job of the CTA) and
-    uint32_t bph = 0;                      // the phase parity of that buffer's barriers
-    float va[32];
-    auto lse_of = [&](int i) {             // the fine part's log-sum-exp of this thread's row of tile i
-      const int tile = blockIdx.x + i * gridDim.x;
-      return a.lse[(int64_t) (tile / tiles_per_head) * a.Nq + (tile % tiles_per_head) * kRows + r];
+  for (int n_pass = redo ? 1 : 2, round = 0;; n_pass = 2, ++round) {
+    LoopBars& bars = bars_of[round];
+    int marked = 0;                           // epilogue: this thread has left a row to the second round
+    // jobs per tile; job j of tile i has the CTA-wide number i * jobs + j, which picks the S buffer (mod 3) and the softmax
+    // group (mod 2; with one pass and an odd chunk count the parity of a tile's first job alternates)
+    const int jobs = n_pass * n_chunks, first_p2 = jobs - n_chunks;
+    // keys of chunk c that belong to its list (a multiple of 32)
+    auto keys_of = [&](int c) {
+      const int left = c < gathered ? a.p1_blocks * kBS - c * kChunk : (int) n_c - (c - gathered) * kChunk;
+      return left < kChunk ? left : kChunk;
     };
-    float lse_next = n_pass == 1 && n_my > 0 ? lse_of(0) : 0.f;
-    bool ok = true;
-    for (int i = 0; ok && i < n_my; ++i) {
-      // one pass: the fine part's log-sum-exp is the reference of the exponentials
-      float mx = n_pass == 1 ? lse_next * kLog2eF : -INFINITY;
-      F2 sum[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};      // four running sums: a chain of adds per element is a third of a job
-      if (n_pass == 1 && i + 1 < n_my) lse_next = lse_of(i + 1);
-      bool exchanged = n_pass == 1;
-      // two passes: the groups exchange their row maxima once per tile, before their first pass-2 job (a group may have none); a copy is
-      // rewritten two exchanges later, after both groups have passed the barrier in between
-      auto exchange_max = [&]() -> bool {
-        exchanged = true;
-        s_max[i & 1][wg][r] = mx;
-        __syncwarp();
-        if (lane == 0) tma::mbar_arrive(&bars.xchg);
-        const bool ok_ = __all_sync(0xffffffffu, tc::bounded_wait(&bars.xchg, (uint32_t) i & 1, abort_flag));
-        mx = fmaxf(s_max[i & 1][0][r], s_max[i & 1][1][r]);
-        return ok_;
-      };
-      for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
-        const bool p2 = j >= first_p2;
-        const int c = j >= n_chunks ? j - n_chunks : j;
-        const float lw = (c < gathered || !a.two_level) ? lw1 : lw2;
-        const int nq = keys_of(c) / 32;
-        if (p2 && !exchanged && !(ok = exchange_max())) break;
-        ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.s_ready[buf], bph, abort_flag));
-        tc::fence_after_sync();
-        if (!ok) break;
-        const uint32_t t_s = t_lane + buf * kChunk;
-        if (!p2) {
-          float m = -INFINITY;
-          for (int q4 = 0; q4 < nq; ++q4) {
-            tc::tmem_ld32_async(t_s + 32 * q4, va);
-            tc::tmem_ld_wait(va);
-#pragma unroll
-            for (int e = 0; e < 32; e += 2) m = fmax3(m, va[e], va[e + 1]);
-          }
-          mx = fmaxf(mx, fmaf(m, sl2, lw));
-        } else {
-          const F2 sl22 = f2(sl2, sl2), off2 = f2(lw - mx, lw - mx);
-#pragma unroll 1          // unrolled, the four quarters' registers overlap and spill (to L2: L1 is 28 KB here)
-          for (int q4 = 0; q4 < nq; ++q4) {
-            tc::tmem_ld32_async(t_s + 32 * q4, va);
-            tc::tmem_ld_wait(va);
-            uint32_t pk[16];
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              float x0, x1;
-              f2_get(f2_fma(f2(va[2 * e], va[2 * e + 1]), sl22, off2), x0, x1);
-              x0 = fast_exp2(x0);
-              x1 = fast_exp2(x1);
-              sum[e & 1] = f2_add(sum[e & 1], f2(x0, x1));
-              pk[e] = pack_bf16(x0, x1);
-            }
-            tc::tmem_st16(t_s + 16 * q4, pk);          // P columns [16 q4, 16 q4 + 16): scores read before
-          }
-          tc::tmem_st_wait();
+
+    if (warp == 8 || warp == 11) {
+      // ---------------------------------------------------------------- TMA producers: warp 8 Q and keys, warp 11 values
+      const bool vals = warp == 11;
+      uint64_t *full = vals ? bars.v_full : bars.k_full, *empty = vals ? bars.v_empty : bars.k_empty;
+      const CUtensorMap *mg = vals ? &maps.vg : &maps.kg, *mc = vals ? &maps.vc : &maps.kc;
+      bf16* ring = vals ? sV : sK;
+      static_assert(kKStages == kVStages, "one loop for both rings");
+      int st = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (int i = 0; ok && i < n_my; ++i) {
+        const int tile = blockIdx.x + i * gridDim.x, qs = i & 1;
+        const int bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
+        if (!vals) {
+          if (!(ok = tc::warp_wait(&bars.q_empty[qs], ((i >> 1) & 1) ^ 1, abort_flag))) break;
+          tma::expect_tx_w(&bars.q_full[qs], kTile * 2);
+          tma::load_4d_w(sQ + qs * kTile, &maps.q, &bars.q_full[qs], 0, row0, bh % a.H, bh / a.H);
         }
-        tc::fence_before_sync();
-        __syncwarp();
-        if (lane == 0) tma::mbar_arrive(&bars.wg_done[buf]);
-        buf += 2;
-        if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
-      }
-      if (ok && !exchanged) ok = exchange_max();
-      // the sums of the tile before the last have been read
-      if (ok && i > 1) ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_free[i & 1], ((uint32_t) (i - 2) >> 1) & 1, abort_flag));
-      if (!ok) break;
-      float l0, l1;
-      f2_get(f2_add(sum[0], sum[1]), l0, l1);
-      s_sum[i & 1][wg][r] = l0 + l1;
-      if (wg == 0) s_ref[i & 1][r] = mx;
-      __syncwarp();
-      if (lane == 0) tma::mbar_arrive(&bars.sum_ready[i & 1]);
-    }
-  } else {
-    // ---------------------------------------------------------------- epilogue, thread = query row
-    const int qd = warp & 3, r = qd * 32 + lane;
-    bool ok = true;
-    for (int i = 0; i < n_my; ++i) {
-      const int tile = blockIdx.x + i * gridDim.x;
-      const int bh = tile / tiles_per_head, row = (tile % tiles_per_head) * kRows + r;
-      bf16* orow = a.o.row(bh / a.H, bh % a.H, row);
-      float* lse_p = a.lse + (int64_t) bh * a.Nq + row;
-      // the fine part of this row, and whether the second launch owns it: requested before the waits
-      uint4 of[8];
+        int krow = 0;                                           // lane j: first row of gathered block j
+        if (gathered) krow = (int) ((int64_t) bh * a.n1 + p1_block(a, bh, row0 / kBS, min(lane, a.p1_blocks - 1)) * kBS);
+        int crow = (int) ((int64_t) bh * n_c);                  // next contiguous chunk
+        for (int j = vals ? first_p2 : 0; j < jobs; ++j) {
+          const int c = j >= n_chunks ? j - n_chunks : j;
+          if (!(ok = tc::warp_wait(&empty[st], ph, abort_flag))) break;
+          tma::expect_tx_w(&full[st], kTile * 2);
+          if (c < gathered) {
 #pragma unroll
-      for (int q8 = 0; q8 < 8; ++q8) of[q8] = *reinterpret_cast<const uint4*>(orow + 8 * q8);
-      const float lse_f = *lse_p;
-      bool mine = true;
-      if (redo && n_pass == 2) mine = redo[(int64_t) bh * a.Nq + row] != 0;
-      ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.sum_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
-      ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
-      tc::fence_after_sync();
-      if (!ok) {
-        if (mine) *lse_p = __int_as_float(0x7fc00000);             // NaN: not completed
-        break;
+            for (int b8 = 0; b8 < 8; ++b8) tma::load_2d_w(ring + st * kTile + b8 * kBS * 64, mg, &full[st], 0, __shfl_sync(0xffffffffu, krow, (c * 8 + b8) & 31));
+          } else {
+            if (c == gathered) crow = (int) ((int64_t) bh * n_c);
+            tma::load_2d_w(ring + st * kTile, mc, &full[st], 0, crow);
+            crow += kChunk;
+          }
+          if (++st == kKStages) { st = 0; ph ^= 1; }
+        }
       }
-      const float lsum = s_sum[i & 1][0][r] + s_sum[i & 1][1][r], mx = s_ref[i & 1][r];
-      // one pass: the row is this launch's unless its sum left the safe range (false for NaN too): the mark hands it to the second
-      if (redo && n_pass == 1) {
-        mine = lsum < 1e30f;
-        redo[(int64_t) bh * a.Nq + row] = mine ? 0 : 1;
+    } else if (warp == 9) {
+      // ---------------------------------------------------------------- MMA issuer 1: S of every job
+      {
+        const uint32_t id_s = tc::instr_desc(kRows, kChunk, 0, 0);
+        const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
+        auto lo = [](const void* p, uint32_t lbo_bytes) { return ((tc::smem_u32(p) >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16); };
+        constexpr uint32_t kStage = (uint32_t) (kTile * 2) >> 4;
+        const uint32_t lQ = lo(sQ, 16), lK = lo(sK, 16);
+        int n = 0, ks = 0, buf = 0;                   // jobs issued so far; K ring stage and S buffer of the next one
+        uint32_t kph = 0, bph = 0;                    // their phase parities
+        bool ok = true;
+        for (int i = 0; ok && i < n_my; ++i) {
+          const int qs = i & 1;
+          if (!(ok = tc::warp_wait(&bars.q_full[qs], (i >> 1) & 1, abort_flag))) break;
+          const uint32_t q_ = lQ + qs * kStage;
+          for (int j = 0; j < jobs; ++j, ++n) {
+            // even lanes: the key chunk; odd lanes: the buffer's previous job (three back), whose group has read S and, in pass 2, P.V P
+            const bool b = (lane & 1) && n >= kBufs;
+            if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : &bars.k_full[ks], b ? bph ^ 1 : kph, abort_flag))) break;
+            tc::fence_after_sync();
+            const uint32_t k_ = lK + ks * kStage, d = tmem + buf * kChunk;
+            tc::umma_ss_k64(d, q_, hi, k_, hi, id_s);
+            tc::umma_commit_w(&bars.s_ready[buf]);
+            tc::umma_commit_w(&bars.k_empty[ks]);
+            if (++ks == kKStages) { ks = 0; kph ^= 1; }
+            if (++buf == kBufs) { buf = 0; bph ^= 1; }
+          }
+          if (!ok) break;
+          tc::umma_commit_w(&bars.q_empty[qs]);
+        }
       }
-      const float Lf = lse_f * kLog2eF;                        // fine part, log2 domain
-      const float Lp = mx + log2f(lsum);
-      const float Lm = fmaxf(Lf, Lp);
-      const float ef = fast_exp2(Lf - Lm), ep = fast_exp2(Lp - Lm);
-      const float inv = 1.f / (ef + ep);
-      const float wf = ef * inv, wp = lsum > 0.f ? ep * inv / lsum : 0.f;      // every exponential may have underflowed
+    } else if (warp == 10) {
+      // ---------------------------------------------------------------- MMA issuer 2: O (+)= P(job, TMEM) . V chunk
+      {
+        const uint32_t id_o = tc::instr_desc(kRows, 64, 0, 1);
+        const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
+        constexpr uint32_t kStage = (uint32_t) (kTile * 2) >> 4;
+        const uint32_t lV = ((tc::smem_u32(sV) >> 4) & 0x3FFFu) | ((1024u >> 4) << 16);
+        int vs = 0, buf = 0;
+        uint32_t vph = 0, bph = 0;
+        bool ok = true;
+        for (int i = 0; ok && i < n_my; ++i) {
+          for (int j = 0; j < jobs; ++j) {
+            // even lanes: the group's job; odd lanes of a pass-2 job: the value chunk; lane 3: O of the tile before the last has been read
+            const bool pv = j >= first_p2;
+            const int c = j - first_p2;
+            uint64_t* bar = &bars.wg_done[buf];
+            uint32_t par = bph;
+            if (pv && lane == 3 && c == 0 && i > 1) { bar = &bars.o_free[i & 1]; par = ((i - 2) >> 1) & 1; }
+            else if (pv && (lane & 1)) { bar = &bars.v_full[vs]; par = vph; }
+            if (!(ok = tc::warp_wait(bar, par, abort_flag))) break;
+            if (pv) {
+              tc::fence_after_sync();
+              const uint32_t v_ = lV + vs * kStage, p_ = tmem + buf * kChunk, o_ = tmem + kColO + (i & 1) * 64;
+              // P: 16 keys = 8 packed columns per k-step; V: 16 key rows = 2048 bytes
+              const int ksteps = keys_of(c) / 16;
+              const uint32_t acc = c > 0 ? 1u : 0u;
+              if (ksteps >= 4) {
+                if (ksteps == 8) tc::umma_ts_k128(o_, p_, v_, hi, id_o, acc);
+                else tc::umma_ts_k64(o_, p_, v_, hi, id_o, acc);
+              }
+              if (ksteps & 2) tc::umma_ts_k32(o_, p_ + (ksteps == 6 ? 32 : 0), v_ + (ksteps == 6 ? 512 : 0), hi, id_o, ksteps == 6 ? 1u : acc);
+              tc::umma_commit_w(&bars.v_empty[vs]);
+              if (++vs == kVStages) { vs = 0; vph ^= 1; }
+            }
+            tc::umma_commit_w(&bars.buf_free[buf]);
+            if (++buf == kBufs) { buf = 0; bph ^= 1; }
+          }
+          if (!ok) break;
+          tc::umma_commit_w(&bars.o_ready[i & 1]);
+        }
+      }
+    } else if (warp < 8) {
+      // ---------------------------------------------------------------- softmax, thread = query row
+      const int wg = warp >> 2, qd = warp & 3, r = qd * 32 + lane;
+      const float sl2 = a.scale * kLog2eF;
+      const float lw1 = log2f(a.w1), lw2 = log2f(a.w2);
+      const uint32_t t_lane = tmem + ((uint32_t) (qd * 32) << 16);
+      int buf = wg;                          // S buffer of this group's next job (it takes every other job of the CTA) and
+      uint32_t bph = 0;                      // the phase parity of that buffer's barriers
+      float va[32];
+      auto lse_of = [&](int i) {             // the fine part's log-sum-exp of this thread's row of tile i
+        const int tile = blockIdx.x + i * gridDim.x;
+        return a.lse[(int64_t) (tile / tiles_per_head) * a.Nq + (tile % tiles_per_head) * kRows + r];
+      };
+      float lse_next = n_pass == 1 && n_my > 0 ? lse_of(0) : 0.f;
+      bool ok = true;
+      for (int i = 0; ok && i < n_my; ++i) {
+        // one pass: the fine part's log-sum-exp is the reference of the exponentials
+        float mx = n_pass == 1 ? lse_next * kLog2eF : -INFINITY;
+        F2 sum[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};      // four running sums: a chain of adds per element is a third of a job
+        if (n_pass == 1 && i + 1 < n_my) lse_next = lse_of(i + 1);
+        bool exchanged = n_pass == 1;
+        // two passes: the groups exchange their row maxima once per tile, before their first pass-2 job (a group may have none); a copy is
+        // rewritten two exchanges later, after both groups have passed the barrier in between
+        auto exchange_max = [&]() -> bool {
+          exchanged = true;
+          s_max[i & 1][wg][r] = mx;
+          __syncwarp();
+          if (lane == 0) tma::mbar_arrive(&bars.xchg);
+          const bool ok_ = __all_sync(0xffffffffu, tc::bounded_wait(&bars.xchg, (uint32_t) i & 1, abort_flag));
+          mx = fmaxf(s_max[i & 1][0][r], s_max[i & 1][1][r]);
+          return ok_;
+        };
+        for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
+          const bool p2 = j >= first_p2;
+          const int c = j >= n_chunks ? j - n_chunks : j;
+          const float lw = (c < gathered || !a.two_level) ? lw1 : lw2;
+          const int nq = keys_of(c) / 32;
+          if (p2 && !exchanged && !(ok = exchange_max())) break;
+          ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.s_ready[buf], bph, abort_flag));
+          tc::fence_after_sync();
+          if (!ok) break;
+          const uint32_t t_s = t_lane + buf * kChunk;
+          if (!p2) {
+            float m = -INFINITY;
+            for (int q4 = 0; q4 < nq; ++q4) {
+              tc::tmem_ld32_async(t_s + 32 * q4, va);
+              tc::tmem_ld_wait(va);
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        float va[32];
-        tc::tmem_ld32_async(tmem + kColO + (i & 1) * 64 + half * 32 + ((uint32_t) (qd * 32) << 16), va);
-        tc::tmem_ld_wait(va);
-        if (half == 1) {                                        // O and the sums are in registers
+              for (int e = 0; e < 32; e += 2) m = fmax3(m, va[e], va[e + 1]);
+            }
+            mx = fmaxf(mx, fmaf(m, sl2, lw));
+          } else {
+            const F2 sl22 = f2(sl2, sl2), off2 = f2(lw - mx, lw - mx);
+#pragma unroll 1          // unrolled, the four quarters' registers overlap and spill (to L2: L1 is 28 KB here)
+            for (int q4 = 0; q4 < nq; ++q4) {
+              tc::tmem_ld32_async(t_s + 32 * q4, va);
+              tc::tmem_ld_wait(va);
+              uint32_t pk[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) {
+                float x0, x1;
+                f2_get(f2_fma(f2(va[2 * e], va[2 * e + 1]), sl22, off2), x0, x1);
+                x0 = fast_exp2(x0);
+                x1 = fast_exp2(x1);
+                sum[e & 1] = f2_add(sum[e & 1], f2(x0, x1));
+                pk[e] = pack_bf16(x0, x1);
+              }
+              tc::tmem_st16(t_s + 16 * q4, pk);          // P columns [16 q4, 16 q4 + 16): scores read before
+            }
+            tc::tmem_st_wait();
+          }
           tc::fence_before_sync();
           __syncwarp();
-          if (lane == 0) tma::mbar_arrive(&bars.o_free[i & 1]);
+          if (lane == 0) tma::mbar_arrive(&bars.wg_done[buf]);
+          buf += 2;
+          if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
         }
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const uint4 f = of[half * 4 + q4];
-          uint4 w;
-          w.x = pack_bf16(bf16_lo(f.x) * wf + va[8 * q4] * wp, bf16_hi(f.x) * wf + va[8 * q4 + 1] * wp);
-          w.y = pack_bf16(bf16_lo(f.y) * wf + va[8 * q4 + 2] * wp, bf16_hi(f.y) * wf + va[8 * q4 + 3] * wp);
-          w.z = pack_bf16(bf16_lo(f.z) * wf + va[8 * q4 + 4] * wp, bf16_hi(f.z) * wf + va[8 * q4 + 5] * wp);
-          w.w = pack_bf16(bf16_lo(f.w) * wf + va[8 * q4 + 6] * wp, bf16_hi(f.w) * wf + va[8 * q4 + 7] * wp);
-          if (mine) *reinterpret_cast<uint4*>(orow + half * 32 + 8 * q4) = w;
-        }
+        if (ok && !exchanged) ok = exchange_max();
+        // the sums of the tile before the last have been read
+        if (ok && i > 1) ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_free[i & 1], ((uint32_t) (i - 2) >> 1) & 1, abort_flag));
+        if (!ok) break;
+        float l0, l1;
+        f2_get(f2_add(sum[0], sum[1]), l0, l1);
+        s_sum[i & 1][wg][r] = l0 + l1;
+        if (wg == 0) s_ref[i & 1][r] = mx;
+        __syncwarp();
+        if (lane == 0) tma::mbar_arrive(&bars.sum_ready[i & 1]);
       }
-      if (mine) *lse_p = (Lm + log2f(ef + ep)) * 0.6931471805599453f;
+    } else {
+      // ---------------------------------------------------------------- epilogue, thread = query row
+      const int qd = warp & 3, r = qd * 32 + lane;
+      bool ok = true;
+      for (int i = 0; i < n_my; ++i) {
+        const int tile = blockIdx.x + i * gridDim.x;
+        const int bh = tile / tiles_per_head, row = (tile % tiles_per_head) * kRows + r;
+        bf16* orow = a.o.row(bh / a.H, bh % a.H, row);
+        float* lse_p = a.lse + (int64_t) bh * a.Nq + row;
+        // the fine part of this row, and whether the second round owns it: requested before the waits
+        uint4 of[8];
+#pragma unroll
+        for (int q8 = 0; q8 < 8; ++q8) of[q8] = *reinterpret_cast<const uint4*>(orow + 8 * q8);
+        const float lse_f = *lse_p;
+        bool mine = true;
+        if (redo && n_pass == 2) mine = redo[(int64_t) bh * a.Nq + row] != 0;
+        ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.sum_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
+        ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
+        tc::fence_after_sync();
+        if (!ok) {
+          if (mine) *lse_p = __int_as_float(0x7fc00000);             // NaN: not completed
+          break;
+        }
+        const float lsum = s_sum[i & 1][0][r] + s_sum[i & 1][1][r], mx = s_ref[i & 1][r];
+        // one pass: the row is this round's unless its sum left the safe range (false for NaN too): the mark hands it to the second
+        if (redo && n_pass == 1) {
+          mine = lsum < 1e30f;
+          redo[(int64_t) bh * a.Nq + row] = mine ? 0 : 1;
+          marked |= !mine;
+        }
+        const float Lf = lse_f * kLog2eF;                        // fine part, log2 domain
+        const float Lp = mx + log2f(lsum);
+        const float Lm = fmaxf(Lf, Lp);
+        const float ef = fast_exp2(Lf - Lm), ep = fast_exp2(Lp - Lm);
+        const float inv = 1.f / (ef + ep);
+        const float wf = ef * inv, wp = lsum > 0.f ? ep * inv / lsum : 0.f;      // every exponential may have underflowed
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          float va[32];
+          tc::tmem_ld32_async(tmem + kColO + (i & 1) * 64 + half * 32 + ((uint32_t) (qd * 32) << 16), va);
+          tc::tmem_ld_wait(va);
+          if (half == 1) {                                        // O and the sums are in registers
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tma::mbar_arrive(&bars.o_free[i & 1]);
+          }
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
+            const uint4 f = of[half * 4 + q4];
+            uint4 w;
+            w.x = pack_bf16(bf16_lo(f.x) * wf + va[8 * q4] * wp, bf16_hi(f.x) * wf + va[8 * q4 + 1] * wp);
+            w.y = pack_bf16(bf16_lo(f.y) * wf + va[8 * q4 + 2] * wp, bf16_hi(f.y) * wf + va[8 * q4 + 3] * wp);
+            w.z = pack_bf16(bf16_lo(f.z) * wf + va[8 * q4 + 4] * wp, bf16_hi(f.z) * wf + va[8 * q4 + 5] * wp);
+            w.w = pack_bf16(bf16_lo(f.w) * wf + va[8 * q4 + 6] * wp, bf16_hi(f.w) * wf + va[8 * q4 + 7] * wp);
+            if (mine) *reinterpret_cast<uint4*>(orow + half * 32 + 8 * q4) = w;
+          }
+        }
+        if (mine) *lse_p = (Lm + log2f(ef + ep)) * 0.6931471805599453f;
+      }
     }
+    tc::fence_before_sync();
+    if (!__syncthreads_or(marked) || abort_flag->abort) break;
+    if (tid == 0) init_bars(bars_of[1]);
+    __syncthreads();
+    tc::fence_after_sync();
   }
   if (abort_flag->abort) tc::abort_drain();
-  tc::fence_before_sync();
   __syncthreads();
   if (threadIdx.x == 0 && abort_flag->abort && a.status) atomicOr(a.status, (int) LLSA_DEV_WAIT_EXPIRED);
   if (warp == 0) tc::tmem_dealloc(tmem, 512);
@@ -426,11 +430,7 @@ int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
   const size_t smem = 1024 + (size_t) (2 + kKStages + kVStages) * kTile * sizeof(bf16);
   LLSA_SMEM_LIMIT((attn_fwd_pooled_loop_tc_kernel), smem);
   unsigned char* redo = g->fwd_redo ? reinterpret_cast<unsigned char*>(g->fwd_redo->ptr) : nullptr;
-  if (redo) {        // one pass with the fine part's log-sum-exp as reference, then the two-pass form for the rows it marked
-    launch_pdl(attn_fwd_pooled_loop_tc_kernel, grid, kThreads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, 1, redo);
-    LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");
-  }
-  launch_pdl(attn_fwd_pooled_loop_tc_kernel, grid, kThreads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, 2, redo);
+  launch_pdl(attn_fwd_pooled_loop_tc_kernel, grid, kThreads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, redo);
   LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");
   return LLSA_OK;
 }

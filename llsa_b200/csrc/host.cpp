@@ -54,7 +54,7 @@ void mark(const char* name) {
   if (g_hook) pybind11::reinterpret_borrow<pybind11::object>(g_hook)(name);
 }
 
-// The marks of the most recent forward (which rows its second launch redid), for whoever wants to look at them.
+// The marks of the most recent forward (which rows its second round redid), for whoever wants to look at them.
 std::mutex g_redo_mutex;
 Tensor& last_redo() {
   static Tensor* t = new Tensor();      // not destroyed at exit: the CUDA context may be gone by then

@@ -124,7 +124,7 @@ def _native():
 
 
 def __getattr__(name):
-    if name == "_last_fwd_redo":      # the marks of the most recent forward over a long pooled list: which rows its second launch redid
+    if name == "_last_fwd_redo":      # the marks of the most recent forward over a long pooled list: which rows its second round redid
         _native()
         return torch.ops.llsa_b200.last_fwd_redo()
     raise AttributeError("module %r has no attribute %r" % (__name__, name))
