@@ -256,7 +256,15 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
 
   const at::cuda::CUDAStream cur = at::cuda::getCurrentCUDAStream(like.device().index());
   const bool hooked = g_has_hook.load(std::memory_order_relaxed);      // a stage hook times every stage on ONE stream
-  const bool overlap = !hooked && !flag(kNoOverlap);
+  // Up to some thousand query blocks the host is the pace of an eager call (110 us of host work; B=1 H=2 N=1024 fp32 forward + backward
+  // 108 us a pass with the side stream, 100 without): two events, four stream operations and a second launch call are worth more there than
+  // the 5 us of the transpose.  In a graph the host's time does not count.
+  auto capturing = [&] {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    C10_CUDA_CHECK(cudaStreamIsCapturing(cur, &s));
+    return s != cudaStreamCaptureStatusNone;
+  };
+  const bool overlap = !hooked && !flag(kNoOverlap) && (BH * d.nq1 > 1024 || capturing());
   auto transpose = [&](cudaStream_t st) {
     mark("transpose_indices");
     ok(tensor_core ? llsa_transpose_indices_pairs(&c.indices, &offsets, &flat, &pairs, &ranges, d.n1, t_scratch ? p + o_ts : nullptr, t_scratch,
