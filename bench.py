@@ -410,9 +410,8 @@ def main():
                            timing="median of %d windows of %d steps (%.2f s timed); min %.4f / max %.4f ms per step" % (
                                len(windows), args.steps, sum(windows) * 1e-3, min(windows) / args.steps, max(windows) / args.steps),
                            overlap="index transpose on a side stream next to the dQ / pooled backward stages (kernel_ms times it alone, on the main stream)",
-                           l2_policy="no flush: a step streams %.0f MB per GPU (q, k, v, do in, o, dq, dk, dv out: 8 x %.1f MB; P / dS scratch %.0f MB), "
-                                     "%s the 126 MB L2" % (8 * units * 2 / 1e6 + nq1 * 8 * 1024 / 1e6, units * 2 / 1e6, nq1 * 8 * 1024 / 1e6,
-                                                           "more than" if 8 * units * 2 + nq1 * 8 * 1024 > 126e6 else "LESS than (reads may hit L2)"),
+                           l2_policy="no flush: a step streams %.0f MB per GPU (q, k, v, do in, o, dq, dk, dv out: 8 x %.1f MB), %s the 126 MB L2" % (
+                               8 * units * 2 / 1e6, units * 2 / 1e6, "more than" if 8 * units * 2 > 126e6 else "LESS than (reads may hit L2)"),
                            parallelism=("%d rank(s): %d group(s) of (b,h) slices x %d rank(s) sharding the sequence (all-gather of k, v and pooled "
                                         "levels, reduce-scatter of dk, dv inside a group)" % (world, world // seq_ranks, seq_ranks))
                            if seq_parallel else "%d rank(s), the %d (batch, head) slices split contiguously%s, no collective"
