@@ -27,7 +27,7 @@
 // warps 0-3 / 4-7 = two softmax warpgroups on alternating jobs, warps 12-15 write a unit's dV and dK, thread = key row.  Every mbarrier
 // wait is bounded (abort flag, TMEM freed).
 // Two levels, B=1 H=6 N=262144 (tensor pipe 768 cycles a job): with one producer lane and results written by the softmax groups 1,010 us
-// dense, 315 gathered; this form DKV_T.
+// dense, 315 gathered; this form needs 916 (856 with packed fp32 pairs) and 268.
 #include <string.h>
 
 #include "attn.cuh"

@@ -27,10 +27,11 @@
 //   warps 0-3 / 4-7  : two softmax warpgroups, group w owns the jobs n = w (mod 2); thread r owns query row r
 //                      (TMEM lane r).  They leave a row's sum (and reference) in shared memory and go on to the next tile.
 //   warps 12-15      : epilogue, thread = row: merges O with the fine part (o, lse written by the fine kernel) and stores both.
-// What bounds it: the 128 exponentials of a row and job on the SM's 16 MUFU lanes (1,024 cycles a job; tensor pipe 640).  A clock trace
+// What bounds it: the chain S -> exponentials -> P.V over three buffers, 1,500 cycles a job (the 128 exponentials of a row take 1,024 on the
+// SM's 16 MUFU lanes, the tensor pipe 640; a quarter of the exponentials moved to the FMA pipe changed nothing).  A clock trace
 // of the form with one producer lane, the epilogue in the softmax groups and one O buffer (785 us at l1, B=2 H=4 N=65536: 1,630 cycles a
 // job) showed the producer needing 1,300 cycles a job for its two waits and two copies, and 5,900 idle cycles at every tile boundary;
-// this form FWD_T.
+// this form needs 712 us (840 -> 625 at two levels, B=1 H=6 N=262144).
 // Every mbarrier wait is bounded; a wait that expires raises a CTA-wide abort flag, every role leaves its loops,
 // lse of the unfinished rows is poisoned with NaN and TMEM is freed.
 #include <string.h>
