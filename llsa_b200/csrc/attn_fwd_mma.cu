@@ -181,7 +181,8 @@ __global__ void __launch_bounds__(NW * 32, 2) attn_fwd_mma_kernel(AttnP<bf16> a,
 // block.  The selected K / V tiles go through a per-warp ring of three stages, two tiles of one tensor each, filled by TMA two stages
 // ahead (one lane issues; no address arithmetic, no shared-memory store slots).  The blocks are taken GP pairs at a time: the S tiles of a
 // group first, one softmax update, then P.V with V read by ldmatrix.trans.  Four blocks a group (GP = 2) halve the updates against two;
-// GP = 1 is for a top-k that is not a multiple of four.  Bound by the gather from L2, 4 KB per (query block, selected block).
+// GP = 1 is for a top-k that is not a multiple of four.  Bound by the gather from L2, 4 KB per (query block, selected block):
+// 127 us at 8 x 6 slices of 16384 tokens, top 8 (143 with cp.async rings of single tiles, every lane copying).
 constexpr int kFineStages = 3;
 constexpr int kFineStageBytes = 2 * kRingTileElems * (int) sizeof(bf16);
 struct FineKvMaps {
