@@ -258,6 +258,11 @@ typedef struct LlsaAttnArgs {
                                   outweigh the fine ones by more than 1e30, and redoes
                                   exactly those rows with the exact two-pass form.  NULL: two passes for
                                   every row.  Same results either way up to rounding */
+  const LlsaTensor* remainder; /* bf16 tensors only, optional: BF16 scratch [B,H,Nq,D], contiguous, wanted where
+                                  llsa_attn_remainder_elems() is not 0 (not read before it is written).  For these pooled
+                                  key lists the fine stage leaves here what rounding its o (backward: stage_mask 1, its
+                                  dq) to bf16 dropped, and the pooled stage (2) adds it, so that results are rounded
+                                  once.  NULL: fine and pooled keys of o / dq in one (slower) kernel for these lists */
 } LlsaAttnArgs;
 
 /* Forward: o, lse.  One level (pk2 == NULL) replaces sparse_indices_attn_res_fwd
@@ -274,6 +279,9 @@ int llsa_attn_bwd(const LlsaAttnArgs* args, void* stream);
  * Nq query rows per (b,h) and `topk` selected blocks per query block (the caller allocates it; any 4-D contiguous
  * shape with at least this many elements is accepted).  The library itself never allocates device memory. */
 int64_t llsa_attn_bwd_partial_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk);
+/* Elements of the scratch LlsaAttnArgs.remainder the forward (backward = 0) or the backward of a problem makes use of, 0 if none.  Read from
+ * `args`: the shapes of q and k, q's type, whether pk2 is given, topk, topk_p and the two switches. */
+int64_t llsa_attn_remainder_elems(const LlsaAttnArgs* args, int backward);
 /* Element count (4-byte elements) LlsaAttnArgs.fine_pds used to need: 1 KB per (query block, selected block) pair.  No scratch of this
  * size is needed any more. */
 int64_t llsa_attn_bwd_pds_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk);

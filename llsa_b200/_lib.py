@@ -36,7 +36,7 @@ class LlsaAttnArgs(C.Structure):
         ("fold_pool_bwd", C.c_int32), ("kv_weight", C.c_float), ("kv_weight_2", C.c_float),
         ("force_generic", C.c_int32), ("stage_mask", C.c_int32), ("dkv_partial", _P),
         ("fine_pds", _P), ("flat_pairs", _P), ("flat_ranges", _P), ("no_tcgen05", C.c_int32), ("wait_limit", C.c_int32), ("status", C.c_void_p),
-        ("fwd_redo", _P),
+        ("fwd_redo", _P), ("remainder", _P),
     ]
 
 
@@ -46,7 +46,7 @@ EXPORTS = [
     "llsa_rms_rope_bwd", "llsa_rms_rope_bwd_partial_elems",
     "llsa_rope_fwd", "llsa_rope_bwd", "llsa_coarse_topk", "llsa_refine_topk", "llsa_select_two_level", "llsa_transpose_scratch_bytes",
     "llsa_transpose_indices", "llsa_transpose_indices_pairs", "llsa_transpose_range_entries", "llsa_transpose_indices_noalloc", "llsa_attn_fwd", "llsa_attn_bwd",
-    "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems", "llsa_status_check",
+    "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems", "llsa_attn_remainder_elems", "llsa_status_check",
 ]
 
 _lib: Optional[C.CDLL] = None
@@ -81,12 +81,15 @@ def _declare(lib: C.CDLL) -> None:
     lib.llsa_transpose_indices_pairs.argtypes = [TP, TP, TP, TP, TP, C.c_int64, C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]
     lib.llsa_attn_bwd_pds_elems.argtypes = [C.c_int64, C.c_int64, C.c_int64, C.c_int32]
     lib.llsa_attn_bwd_pds_elems.restype = C.c_int64
+    lib.llsa_attn_remainder_elems.argtypes = [C.POINTER(LlsaAttnArgs), C.c_int]
+    lib.llsa_attn_remainder_elems.restype = C.c_int64
     lib.llsa_status_check.argtypes = [C.c_int32]
     lib.llsa_attn_fwd.argtypes = [C.POINTER(LlsaAttnArgs), C.c_void_p]
     lib.llsa_attn_bwd.argtypes = [C.POINTER(LlsaAttnArgs), C.c_void_p]
     for name in EXPORTS:
         fn = getattr(lib, name)
-        if name not in ("llsa_last_error_string", "llsa_transpose_scratch_bytes", "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems", "llsa_rms_rope_bwd_partial_elems"):
+        if name not in ("llsa_last_error_string", "llsa_transpose_scratch_bytes", "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems",
+                        "llsa_rms_rope_bwd_partial_elems", "llsa_attn_remainder_elems"):
             fn.restype = C.c_int
 
 

@@ -46,6 +46,10 @@ static int check_attn_args(const LlsaAttnArgs* g, bool bwd) {
   } else {
     LLSA_REQUIRE(n1 < 64 || n1 % 32 == 0, LLSA_ERR_SHAPE, "attn: N/16=%lld must be a multiple of 32", (long long) n1);
   }
+  if (g->remainder && dt == LLSA_BF16) {
+    const int64_t sm[4] = {B, H, Nq, D};
+    if ((rc = check_contig(g->remainder, "remainder", dt, 4, sm))) return rc;
+  }
   if (!bwd && g->fwd_redo) {
     int64_t have = 1;
     for (int i = 0; i < g->fwd_redo->ndim; ++i) have *= g->fwd_redo->shape[i];
@@ -91,9 +95,26 @@ static int check_attn_args(const LlsaAttnArgs* g, bool bwd) {
   return LLSA_OK;
 }
 
+// The key-loop kernels add the pooled part to what the fine stage left in o / dq.  Where one kernel used to do both (attn_fwd_mma_kernel,
+// attn_dq_mma_kernel: every list but those excepted below) the sums stay in fp32 from the first key to the last, and a bf16 o / dq in
+// between, rounded a second time at the end, is a loss: relative error against fp64 at one level, N = 2560 (160 pooled keys) 1.87e-3
+// instead of 1.70e-3 in o and 2.16e-3 instead of 2.00e-3 in dq.  There the fine stage also writes what the rounding left over (bf16, so that value and
+// remainder together hold 16 bits), and the pooled stage adds it: 1.71e-3 and 2.00e-3.  The excepted lists -- more than 192 keys in
+// whole chunks, with eight gathered blocks if two levels -- have always passed bf16 between two kernels, as the single-shot kernels do.
+bool remainder_wanted(const AttnP<__nv_bfloat16>& a, bool bwd) {
+  if (!pooled_loop_tc_keys(a) || (bwd ? pooled_bwd_tc_ok(a) : pooled_tc_keys(a) > 0)) return false;
+  const int64_t np = (int64_t) (a.p1_blocks + a.p2_blocks) * kBS;
+  return np <= 192 || np % 128 || (a.two_level && (a.p1_blocks != 8 || a.p2_blocks == 0));
+}
+
 }  // namespace llsa
 
 using namespace llsa;
+
+extern "C" int64_t llsa_attn_remainder_elems(const LlsaAttnArgs* g, int backward) {
+  if (!g || !g->q || !g->k || g->q->ndim != 4 || g->k->ndim != 4 || g->q->dtype != LLSA_BF16 || g->force_generic || g->no_tcgen05) return 0;
+  return remainder_wanted(attn_dims<__nv_bfloat16>(g), backward != 0) ? g->q->shape[0] * g->q->shape[1] * g->q->shape[2] * kD : 0;
+}
 
 extern "C" int64_t llsa_attn_bwd_partial_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk) {
   if (B <= 0 || H <= 0 || Nq <= 0 || topk <= 0) return 0;

@@ -10,6 +10,8 @@
 // A pooled stage with fewer than 64 keys is skipped, as the reference's forward
 // loops do (res_1.py:85, res_2.py:127).
 #pragma once
+#include <string.h>
+
 #include "common.cuh"
 
 namespace llsa {
@@ -26,6 +28,7 @@ struct AttnP {
   const T* pk2;  // contiguous [BH, n2, D] or nullptr
   const T* pv2;
   IdxView idx, pidx;
+  T* rem;        // [BH, Nq, D] or nullptr: what rounding the fine part's o (forward) or dq (backward) to T left over (remainder_wanted)
   float* lse;    // [BH, Nq]
   float* delta;  // [BH, Nq]
   float* dpk;    // fp32 accumulators [BH, n1, D]
@@ -79,33 +82,24 @@ int pooled_tc_keys(const AttnP<__nv_bfloat16>& a);   // pooled keys per row if t
 int launch_attn_fwd_pooled_tc(const LlsaAttnArgs* g, const AttnP<__nv_bfloat16>& a, int64_t BH, cudaStream_t st);
 int pooled_loop_tc_keys(const AttnP<__nv_bfloat16>& a);   // pooled keys per row if the key-loop tcgen05 forward applies, else 0
 int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<__nv_bfloat16>& a, int64_t BH, cudaStream_t st);
+bool pooled_loop_one_pass(const AttnP<__nv_bfloat16>& a);  // that kernel makes one pass over the keys, given room for its marks
 int pooled_dq_loop_tc_keys(const AttnP<__nv_bfloat16>& a);  // pooled keys per row if the key-loop tcgen05 dQ kernel applies, else 0
 int launch_attn_dq_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<__nv_bfloat16>& a, int64_t BH, cudaStream_t st);
 int launch_attn_dkv_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<__nv_bfloat16>& a, int64_t BH, cudaStream_t st);
 bool pooled_bwd_tc_ok(const AttnP<__nv_bfloat16>& a);  // the tcgen05 pooled backward applies (two levels, 128 + 64 pooled keys)
 int launch_attn_bwd_pooled_tc(const LlsaAttnArgs* g, const AttnP<__nv_bfloat16>& a, int64_t BH, cudaStream_t st);
+bool remainder_wanted(const AttnP<__nv_bfloat16>& a, bool bwd);   // the fine part crosses to the pooled stage with its remainder (attn.cu)
 int launch_attn_fwd_generic(const LlsaAttnArgs* g, cudaStream_t st);
 int launch_attn_bwd_generic(const LlsaAttnArgs* g, cudaStream_t st);
 int launch_attn_fwd_mma(const LlsaAttnArgs* g, cudaStream_t st);
 int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st);
 
+// Sizes and key lists of a problem: what chooses its kernels
 template <typename T>
-inline AttnP<T> build_attn_params(const LlsaAttnArgs* g, bool bwd) {
+inline AttnP<T> attn_dims(const LlsaAttnArgs* g) {
   AttnP<T> a;
   memset(&a, 0, sizeof(a));
-  a.q = make_view<const T>(g->q);
-  a.k = make_view<const T>(g->k);
-  a.v = make_view<const T>(g->v);
-  a.pk = (const T*) g->pk->ptr;
-  a.pv = (const T*) g->pv->ptr;
   a.two_level = g->pk2 != nullptr;
-  if (a.two_level) {
-    a.pk2 = (const T*) g->pk2->ptr;
-    a.pv2 = (const T*) g->pv2->ptr;
-    a.pidx = make_idx(g->p_indices);
-  }
-  a.idx = make_idx(g->indices);
-  a.lse = (float*) g->lse->ptr;
   a.H = (int) g->q->shape[1];
   a.N = g->k->shape[2];
   a.n1 = a.N / kBS;
@@ -115,18 +109,36 @@ inline AttnP<T> build_attn_params(const LlsaAttnArgs* g, bool bwd) {
   a.nq2 = a.nq1 / kBS;
   a.topk = g->topk;
   a.topk_p = g->topk_p;
-  a.w1 = g->token_weight;
-  a.w2 = g->token_weight_2;
-  a.scale = 0.125f;
-  a.status = g->status;
-  a.wait_limit = g->wait_limit;
   if (a.two_level) {
     a.p1_blocks = a.topk_p;
     a.p2_blocks = a.n2 >= 64 ? (int) (a.n2 / kBS) : 0;
   } else {
     a.p1_blocks = a.n1 >= 64 ? (int) (a.n1 / kBS) : 0;
-    a.p2_blocks = 0;
   }
+  return a;
+}
+
+template <typename T>
+inline AttnP<T> build_attn_params(const LlsaAttnArgs* g, bool bwd) {
+  AttnP<T> a = attn_dims<T>(g);
+  a.q = make_view<const T>(g->q);
+  a.k = make_view<const T>(g->k);
+  a.v = make_view<const T>(g->v);
+  a.pk = (const T*) g->pk->ptr;
+  a.pv = (const T*) g->pv->ptr;
+  if (a.two_level) {
+    a.pk2 = (const T*) g->pk2->ptr;
+    a.pv2 = (const T*) g->pv2->ptr;
+    a.pidx = make_idx(g->p_indices);
+  }
+  a.idx = make_idx(g->indices);
+  a.lse = (float*) g->lse->ptr;
+  a.rem = g->remainder ? (T*) g->remainder->ptr : nullptr;
+  a.w1 = g->token_weight;
+  a.w2 = g->token_weight_2;
+  a.scale = 0.125f;
+  a.status = g->status;
+  a.wait_limit = g->wait_limit;
   if (!bwd) {
     a.o = make_view<T>(g->o);
   } else {

@@ -231,7 +231,8 @@ constexpr int kDqStages = 3;
 struct KvMaps {
   CUtensorMap k, v;            // [B,H,N,64] 4-D, box 16 rows
 };
-template <int NW>
+// REM: what rounding dq to bf16 leaves over goes to a.rem, for the pooled stage to add (remainder_wanted).
+template <int NW, bool REM>
 __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps maps) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t s_full[NW][kDqStages];
@@ -324,9 +325,21 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a,
   // the tile leaves through the idle ring (stmatrix, then eight lanes write one whole row)
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
-    stsm_x4<0>(sa_m ^ (c << 5), pack_bf16(dq[2 * c][0] * a.scale, dq[2 * c][1] * a.scale), pack_bf16(dq[2 * c][2] * a.scale, dq[2 * c][3] * a.scale),
-               pack_bf16(dq[2 * c + 1][0] * a.scale, dq[2 * c + 1][1] * a.scale), pack_bf16(dq[2 * c + 1][2] * a.scale, dq[2 * c + 1][3] * a.scale));
+  for (int c = 0; c < 4; ++c) {
+    float x[2][4];
+    uint32_t w[4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[u][e] = dq[2 * c + u][e] * a.scale;
+      w[2 * u] = pack_bf16(x[u][0], x[u][1]);
+      w[2 * u + 1] = pack_bf16(x[u][2], x[u][3]);
+    }
+    stsm_x4<0>(sa_m ^ (c << 5), w[0], w[1], w[2], w[3]);
+    if (REM)
+      stsm_x4<kRingTileBytes>(sa_m ^ (c << 5), pack_rest(x[0][0], x[0][1], w[0]), pack_rest(x[0][2], x[0][3], w[1]),
+                              pack_rest(x[1][0], x[1][1], w[2]), pack_rest(x[1][2], x[1][3], w[3]));
+  }
   __syncwarp();
   const uint32_t sa_cp = ring_sa + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4);
   bf16* out = a.dq.row(b, h, qb * kBS + (lane >> 3)) + (lane & 7) * 8;
@@ -336,6 +349,14 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a,
   lds128<512>(x.x, x.y, x.z, x.w, sa_cp ^ 64);  *reinterpret_cast<uint4*>(out + step) = x;
   lds128<1024>(x.x, x.y, x.z, x.w, sa_cp);      *reinterpret_cast<uint4*>(out + 2 * step) = x;
   lds128<1536>(x.x, x.y, x.z, x.w, sa_cp ^ 64); *reinterpret_cast<uint4*>(out + 3 * step) = x;
+  if (REM) {
+    constexpr int TB = kRingTileBytes;
+    bf16* rp = a.rem + (rbase + (lane >> 3)) * kD + (lane & 7) * 8;
+    lds128<TB>(x.x, x.y, x.z, x.w, sa_cp);             *reinterpret_cast<uint4*>(rp) = x;
+    lds128<TB + 512>(x.x, x.y, x.z, x.w, sa_cp ^ 64);  *reinterpret_cast<uint4*>(rp + 4 * kD) = x;
+    lds128<TB + 1024>(x.x, x.y, x.z, x.w, sa_cp);      *reinterpret_cast<uint4*>(rp + 8 * kD) = x;
+    lds128<TB + 1536>(x.x, x.y, x.z, x.w, sa_cp ^ 64); *reinterpret_cast<uint4*>(rp + 12 * kD) = x;
+  }
 }
 
 // P^T and dS^T (bf16, as A registers) of one (key tile) x (query block) pair from the
@@ -948,8 +969,11 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
   // pooled keys on tcgen05 (attn_pooled_bwd_tc.cu): the dQ kernel then covers the fine blocks only and the
   // tensor-core kernel adds the pooled part of dq and produces the pooled-key gradients
   const bool tc = pooled_bwd_tc_ok(a) && !g->no_tcgen05;
-  // other pooled key lists: the key-loop tcgen05 kernels (dQ, then the key-major dK/dV)
-  const bool loop_dq = !tc && pooled_dq_loop_tc_keys(a) > 0 && !g->no_tcgen05;
+  // other pooled key lists: the key-loop tcgen05 kernels (dQ, then the key-major dK/dV); a list whose fine part of dq has to cross with its
+  // remainder takes dq in one kernel if the caller gave no room for that
+  const bool rem = remainder_wanted(a, true);
+  if (!rem) a.rem = nullptr;
+  const bool loop_dkv = !tc && pooled_dq_loop_tc_keys(a) > 0 && !g->no_tcgen05, loop_dq = loop_dkv && (!rem || a.rem);
   if (mask & 1) {
     if (!(g->stage_mask & 8)) {
       int rc = zero_pooled_acc(g, st);
@@ -968,8 +992,9 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
       if ((rc = tma::make_map_bhnd(&maps.k, g->k, kBS))) return rc;
       if ((rc = tma::make_map_bhnd(&maps.v, g->v, kBS))) return rc;
       const size_t ring = (size_t) NWQ * kDqStages * 2 * kRingTileBytes + 1024;
-      LLSA_SMEM_LIMIT((attn_dq_fine_kernel<NWQ>), ring);
-      launch_pdl(attn_dq_fine_kernel<NWQ>, dim3((unsigned) (a.nq1 / NWQ), BH), NWQ * 32, ring, st, aq, maps);
+      auto fine = loop_dq && a.rem ? attn_dq_fine_kernel<NWQ, true> : attn_dq_fine_kernel<NWQ, false>;
+      LLSA_SMEM_LIMIT(fine, ring);
+      launch_pdl(fine, dim3((unsigned) (a.nq1 / NWQ), BH), NWQ * 32, ring, st, aq, maps);
       LLSA_LAUNCH_OK("attn_dq_fine_kernel");
     } else {
       LLSA_SMEM_LIMIT((attn_dq_mma_kernel<NWQ>), smem);
@@ -985,7 +1010,7 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
       int rc = launch_attn_dq_pooled_loop_tc(g, a, BH, st);
       if (rc) return rc;
     }
-    if (loop_dq) {
+    if (loop_dkv) {
       int rc = launch_attn_dkv_pooled_loop_tc(g, a, BH, st);
       if (rc) return rc;
     } else {

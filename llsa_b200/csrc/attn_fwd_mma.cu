@@ -202,7 +202,8 @@ __device__ __forceinline__ void load_two_tiles_w(uint32_t dst, const CUtensorMap
       : "memory");
 }
 
-template <int NW, int GP>
+// REM: what rounding o to bf16 leaves over goes to a.rem, for the pooled stage to add (remainder_wanted).
+template <int NW, int GP, bool REM>
 __global__ void __launch_bounds__(NW * 32, 16 / NW) attn_fwd_fine_kernel(AttnP<bf16> a, const __grid_constant__ FineKvMaps maps) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t s_full[NW][kFineStages];
@@ -330,9 +331,20 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) attn_fwd_fine_kernel(AttnP<b
   // accumulator tile u holds channels 8u + 2t, 8u + 2t + 1 of rows g (c0, c1) and g + 8 (c2, c3): through the idle ring to whole rows
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
-    stsm_x4<0>(sa_m ^ (c << 5), pack_bf16(o[2 * c][0] * i0, o[2 * c][1] * i0), pack_bf16(o[2 * c][2] * i1, o[2 * c][3] * i1),
-               pack_bf16(o[2 * c + 1][0] * i0, o[2 * c + 1][1] * i0), pack_bf16(o[2 * c + 1][2] * i1, o[2 * c + 1][3] * i1));
+  for (int c = 0; c < 4; ++c) {
+    float x[2][4];
+    uint32_t w[4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      x[u][0] = o[2 * c + u][0] * i0; x[u][1] = o[2 * c + u][1] * i0; x[u][2] = o[2 * c + u][2] * i1; x[u][3] = o[2 * c + u][3] * i1;
+      w[2 * u] = pack_bf16(x[u][0], x[u][1]);
+      w[2 * u + 1] = pack_bf16(x[u][2], x[u][3]);
+    }
+    stsm_x4<0>(sa_m ^ (c << 5), w[0], w[1], w[2], w[3]);
+    if (REM)
+      stsm_x4<2048>(sa_m ^ (c << 5), pack_rest(x[0][0], x[0][1], w[0]), pack_rest(x[0][2], x[0][3], w[1]), pack_rest(x[1][0], x[1][1], w[2]),
+                    pack_rest(x[1][2], x[1][3], w[3]));
+  }
   __syncwarp();
   const uint32_t sa_cp = ring_sa + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4);
   bf16* op = a.o.row(b, h, qb * kBS + (lane >> 3)) + (lane & 7) * 8;
@@ -342,6 +354,13 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) attn_fwd_fine_kernel(AttnP<b
   lds128<512>(x.x, x.y, x.z, x.w, sa_cp ^ 64);  *reinterpret_cast<uint4*>(op + os) = x;
   lds128<1024>(x.x, x.y, x.z, x.w, sa_cp);      *reinterpret_cast<uint4*>(op + 2 * os) = x;
   lds128<1536>(x.x, x.y, x.z, x.w, sa_cp ^ 64); *reinterpret_cast<uint4*>(op + 3 * os) = x;
+  if (REM) {
+    bf16* rp = a.rem + (bh * a.Nq + qb * kBS + (lane >> 3)) * kD + (lane & 7) * 8;
+    lds128<2048>(x.x, x.y, x.z, x.w, sa_cp);             *reinterpret_cast<uint4*>(rp) = x;
+    lds128<2048 + 512>(x.x, x.y, x.z, x.w, sa_cp ^ 64);  *reinterpret_cast<uint4*>(rp + 4 * kD) = x;
+    lds128<2048 + 1024>(x.x, x.y, x.z, x.w, sa_cp);      *reinterpret_cast<uint4*>(rp + 8 * kD) = x;
+    lds128<2048 + 1536>(x.x, x.y, x.z, x.w, sa_cp ^ 64); *reinterpret_cast<uint4*>(rp + 12 * kD) = x;
+  }
 }
 
 // A bf16 call whose operands miss the tensor-core kernels' limits still runs, on the scalar kernels and many times
@@ -375,8 +394,11 @@ int launch_attn_fwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
   AttnP<bf16> a = build_attn_params<bf16>(g, false);
   constexpr int NW = 8;
   const int64_t BH = g->q->shape[0] * a.H;
-  // all pooled keys of a row at once where they fit (64, 128, 192 keys), else chunk by chunk
-  const bool loop_tc = !pooled_tc_keys(a) && pooled_loop_tc_keys(a) > 0;
+  // all pooled keys of a row at once where they fit (64, 128, 192 keys), else chunk by chunk; a list whose fine part has to cross with its
+  // remainder takes the one-kernel form below if the caller gave no room for that
+  const bool rem = remainder_wanted(a, false);
+  if (!rem) a.rem = nullptr;
+  const bool loop_tc = !pooled_tc_keys(a) && pooled_loop_tc_keys(a) > 0 && (!rem || a.rem);
   if ((pooled_tc_keys(a) || loop_tc) && !g->no_tcgen05) {
     // fine blocks on mma.sync (o and lse of the fine part alone), pooled keys on tcgen05, merged there
     FineKvMaps maps;
@@ -387,13 +409,10 @@ int launch_attn_fwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     constexpr int NWF = 4;
     const size_t ring = (size_t) NWF * kFineStages * kFineStageBytes + 1024;
     const dim3 fine_grid((unsigned) (a.nq1 / NWF), (unsigned) BH);
-    if (a.topk % 4 == 0) {
-      LLSA_SMEM_LIMIT((attn_fwd_fine_kernel<NWF, 2>), ring);
-      launch_pdl(attn_fwd_fine_kernel<NWF, 2>, fine_grid, NWF * 32, ring, st, a, maps);
-    } else {
-      LLSA_SMEM_LIMIT((attn_fwd_fine_kernel<NWF, 1>), ring);
-      launch_pdl(attn_fwd_fine_kernel<NWF, 1>, fine_grid, NWF * 32, ring, st, a, maps);
-    }
+    auto fine = a.topk % 4 == 0 ? (a.rem ? attn_fwd_fine_kernel<NWF, 2, true> : attn_fwd_fine_kernel<NWF, 2, false>)
+                                : (a.rem ? attn_fwd_fine_kernel<NWF, 1, true> : attn_fwd_fine_kernel<NWF, 1, false>);
+    LLSA_SMEM_LIMIT(fine, ring);
+    launch_pdl(fine, fine_grid, NWF * 32, ring, st, a, maps);
     LLSA_LAUNCH_OK("attn_fwd_fine_kernel");
     return loop_tc ? launch_attn_fwd_pooled_loop_tc(g, a, BH, st) : launch_attn_fwd_pooled_tc(g, a, BH, st);
   }

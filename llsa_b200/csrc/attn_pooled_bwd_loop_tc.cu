@@ -57,7 +57,8 @@ struct DqBars {
 };
 
 // jobs: 64-key chunks per tile; gathered: number of leading chunks that are gathered level-1 blocks; n_c: rows per head of the
-// contiguous pooled tensor.
+// contiguous pooled tensor.  REM: the fine part of dq is the bf16 value in dq plus its remainder in a.rem.
+template <bool REM>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps, int jobs, int gathered, int64_t n_c, int n_tiles,
                               int tiles_per_head) {
@@ -276,6 +277,12 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         float v[32];
+        uint4 rest[4];
+        if (REM) {
+          const uint4* rp = reinterpret_cast<const uint4*>(a.rem + ((int64_t) bh * a.Nq + row) * kD + half * 32);
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) rest[q4] = rp[q4];
+        }
         tc::tmem_ld32_async(tmem + kColDQ + (i & 1) * 64 + half * 32 + ((uint32_t) (qd * 32) << 16), v);
         tc::tmem_ld_wait(v);
         if (half == 1) {
@@ -286,11 +293,15 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
           const uint4 f = old[half * 4 + q4];
+          auto sum = [&](uint32_t fine, uint32_t left, int e) {
+            const float x = REM ? bf16_lo(fine) + bf16_lo(left) : bf16_lo(fine), y = REM ? bf16_hi(fine) + bf16_hi(left) : bf16_hi(fine);
+            return pack_bf16(fmaf(v[8 * q4 + e], a.scale, x), fmaf(v[8 * q4 + e + 1], a.scale, y));
+          };
           uint4 w;
-          w.x = pack_bf16(fmaf(v[8 * q4], a.scale, bf16_lo(f.x)), fmaf(v[8 * q4 + 1], a.scale, bf16_hi(f.x)));
-          w.y = pack_bf16(fmaf(v[8 * q4 + 2], a.scale, bf16_lo(f.y)), fmaf(v[8 * q4 + 3], a.scale, bf16_hi(f.y)));
-          w.z = pack_bf16(fmaf(v[8 * q4 + 4], a.scale, bf16_lo(f.z)), fmaf(v[8 * q4 + 5], a.scale, bf16_hi(f.z)));
-          w.w = pack_bf16(fmaf(v[8 * q4 + 6], a.scale, bf16_lo(f.w)), fmaf(v[8 * q4 + 7], a.scale, bf16_hi(f.w)));
+          w.x = sum(f.x, rest[q4].x, 0);
+          w.y = sum(f.y, rest[q4].y, 2);
+          w.z = sum(f.z, rest[q4].z, 4);
+          w.w = sum(f.w, rest[q4].w, 6);
           *reinterpret_cast<uint4*>(dqrow + half * 32 + 8 * q4) = w;
         }
       }
@@ -330,8 +341,9 @@ int launch_attn_dq_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, i
   LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) (4 * kTile + 2 * kStages * kChunkElems) * sizeof(bf16);
-  LLSA_SMEM_LIMIT((attn_dq_pooled_loop_tc_kernel), smem);
-  launch_pdl(attn_dq_pooled_loop_tc_kernel, grid, kThreads, smem, st, a, maps, jobs, gathered, n_c, n_tiles, tiles_per_head);
+  auto kernel = a.rem ? attn_dq_pooled_loop_tc_kernel<true> : attn_dq_pooled_loop_tc_kernel<false>;
+  LLSA_SMEM_LIMIT(kernel, smem);
+  launch_pdl(kernel, grid, kThreads, smem, st, a, maps, jobs, gathered, n_c, n_tiles, tiles_per_head);
   LLSA_LAUNCH_OK("attn_dq_pooled_loop_tc_kernel");
   return LLSA_OK;
 }

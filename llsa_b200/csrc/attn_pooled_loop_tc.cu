@@ -13,7 +13,7 @@
 //           the A operand of O += P.V_c; row sums on the side.
 // With a `redo` byte per query row from the caller the first pass is dropped: the pooled part only ever meets the fine
 // part through their log-sum-exp, so the fine part's log-sum-exp (already known per row) serves as the reference of the
-// exponentials, P = exp2(S' - lse_fine).  Anything below 2^-126 of the fine part's weight is irrelevant, and bf16 / fp32
+// exponentials, P = exp2(S' - lse_fine) (up to the next quarter above a power of two: kRefShift).  Anything below 2^-126 of the fine part's weight is irrelevant, and bf16 / fp32
 // hold anything up to 2^127 times it; a row whose pooled keys outweigh its fine keys by more than that (its row sum
 // passes 1e30, or is NaN) is left untouched and marked in `redo`; a CTA that has marked a row of its tiles goes over them again
 // with two passes and writes exactly the marked rows.  (A second launch that looked for marks cost every call 1 to 2 us.)
@@ -53,6 +53,11 @@ constexpr int kThreads = 512;
 constexpr int kBufs = 3;
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr uint32_t kColO = 384;
+// One pass: where in its binade a probability of a logit of 0 lands.  bf16 is finest just below a power of two, which is where a row's
+// maximum as reference puts the largest ones; a reference at no particular place costs up to 12 % of o's error where the keys weigh about alike
+// (against fp64, N(0,1) inputs, two levels, N = 40960, top-16: 2.33e-3; 2.33e-3, 2.11e-3, 2.10e-3, 2.15e-3, 2.22e-3 with the reference at
+// 0, 1/8, 1/4, 3/8, 1/2 above a power of two; 2.09e-3 with two passes).  The weights 16 and 256 are powers of two themselves.
+constexpr float kRefShift = 0.25f;
 
 struct LoopMaps {
   CUtensorMap q;              // [B,H,Nq,64] 4-D, box 128 rows
@@ -87,7 +92,8 @@ __device__ __forceinline__ void init_bars(LoopBars& bars) {
 }
 
 // n_chunks: chunks per tile; gathered: how many of them, the first ones, are gathered level-1 blocks (two levels); n_c: rows per
-// head of the contiguous pooled tensor.
+// head of the contiguous pooled tensor.  REM: the fine part of o is the bf16 value in o plus its remainder in a.rem.
+template <bool REM>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps maps, int n_chunks, int gathered, int64_t n_c, int n_tiles,
                                int tiles_per_head, unsigned char* redo) {
@@ -252,8 +258,8 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       float lse_next = n_pass == 1 && n_my > 0 ? lse_of(0) : 0.f;
       bool ok = true;
       for (int i = 0; ok && i < n_my; ++i) {
-        // one pass: the fine part's log-sum-exp is the reference of the exponentials
-        float mx = n_pass == 1 ? lse_next * kLog2eF : -INFINITY;
+        // one pass: the fine part's log-sum-exp, moved to a fixed place between two powers of two, is the reference of the exponentials
+        float mx = n_pass == 1 ? ceilf(lse_next * kLog2eF) + kRefShift : -INFINITY;
         F2 sum[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};      // four running sums: a chain of adds per element is a third of a job
         if (n_pass == 1 && i + 1 < n_my) lse_next = lse_of(i + 1);
         bool exchanged = n_pass == 1;
@@ -363,6 +369,12 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           float va[32];
+          uint4 rest[4];
+          if (REM) {
+            const uint4* rp = reinterpret_cast<const uint4*>(a.rem + ((int64_t) bh * a.Nq + row) * kD + half * 32);
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) rest[q4] = rp[q4];
+          }
           tc::tmem_ld32_async(tmem + kColO + (i & 1) * 64 + half * 32 + ((uint32_t) (qd * 32) << 16), va);
           tc::tmem_ld_wait(va);
           if (half == 1) {                                        // O and the sums are in registers
@@ -373,11 +385,15 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
             const uint4 f = of[half * 4 + q4];
+            auto merged = [&](uint32_t fine, uint32_t left, int e) {
+              const float x = REM ? bf16_lo(fine) + bf16_lo(left) : bf16_lo(fine), y = REM ? bf16_hi(fine) + bf16_hi(left) : bf16_hi(fine);
+              return pack_bf16(x * wf + va[8 * q4 + e] * wp, y * wf + va[8 * q4 + e + 1] * wp);
+            };
             uint4 w;
-            w.x = pack_bf16(bf16_lo(f.x) * wf + va[8 * q4] * wp, bf16_hi(f.x) * wf + va[8 * q4 + 1] * wp);
-            w.y = pack_bf16(bf16_lo(f.y) * wf + va[8 * q4 + 2] * wp, bf16_hi(f.y) * wf + va[8 * q4 + 3] * wp);
-            w.z = pack_bf16(bf16_lo(f.z) * wf + va[8 * q4 + 4] * wp, bf16_hi(f.z) * wf + va[8 * q4 + 5] * wp);
-            w.w = pack_bf16(bf16_lo(f.w) * wf + va[8 * q4 + 6] * wp, bf16_hi(f.w) * wf + va[8 * q4 + 7] * wp);
+            w.x = merged(f.x, rest[q4].x, 0);
+            w.y = merged(f.y, rest[q4].y, 2);
+            w.z = merged(f.z, rest[q4].z, 4);
+            w.w = merged(f.w, rest[q4].w, 6);
             if (mine) *reinterpret_cast<uint4*>(orow + half * 32 + 8 * q4) = w;
           }
         }
@@ -407,6 +423,14 @@ int pooled_loop_tc_keys(const AttnP<bf16>& a) {
   return (int) np;
 }
 
+// Short lists whose fine part crosses with its remainder take two passes whatever the caller offers: the maximum as reference makes the
+// weightiest probability exact, which one pass does not, and a second pass over two chunks is cheap (o's error against fp64 / time of the whole forward:
+// one level, N = 2560, B=4 H=6, 160 keys 1.714e-3 and 49.3 us, 1.708e-3 and 51.2; two levels, N = 24576, H=6, 224 keys 1.707e-3 and 81.1, 1.696e-3 and 83.8;
+// the one-kernel form 1.706e-3, 1.693e-3).  Beyond that it buys less and costs more: N = 40960, top-16, 416 keys 1.701e-3 and 168 us, 1.694e-3 and 184.
+bool pooled_loop_one_pass(const AttnP<bf16>& a) {
+  return (a.p1_blocks + a.p2_blocks) * kBS > 2 * kChunk || !remainder_wanted(a, false);
+}
+
 int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, int64_t BH, cudaStream_t st) {
   LoopMaps maps;
   memset(&maps, 0, sizeof(maps));
@@ -429,9 +453,10 @@ int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
   LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) (2 + kKStages + kVStages) * kTile * sizeof(bf16);
-  LLSA_SMEM_LIMIT((attn_fwd_pooled_loop_tc_kernel), smem);
-  unsigned char* redo = g->fwd_redo ? reinterpret_cast<unsigned char*>(g->fwd_redo->ptr) : nullptr;
-  launch_pdl(attn_fwd_pooled_loop_tc_kernel, grid, kThreads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, redo);
+  auto kernel = a.rem ? attn_fwd_pooled_loop_tc_kernel<true> : attn_fwd_pooled_loop_tc_kernel<false>;
+  LLSA_SMEM_LIMIT(kernel, smem);
+  unsigned char* redo = g->fwd_redo && pooled_loop_one_pass(a) ? reinterpret_cast<unsigned char*>(g->fwd_redo->ptr) : nullptr;
+  launch_pdl(kernel, grid, kThreads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, redo);
   LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");
   return LLSA_OK;
 }

@@ -207,7 +207,13 @@ struct Core {      // operands common to forward and backward
 void run_fwd(const Core& c, int topk, int topk_p, int bs, double w1, double w2, const Tensor& like, void* redo, int64_t redo_elems,
              const Status& status, cudaStream_t st) {
   LlsaAttnArgs a = c.args(topk, topk_p, bs, w1, w2);
-  LlsaTensor r;
+  LlsaTensor r, rd;
+  Tensor rem;
+  if (llsa_attn_remainder_elems(&a, 0)) {
+    rem = at::empty({c.q.shape[0], c.q.shape[1], c.q.shape[2], c.q.shape[3]}, like.options());
+    rd = desc(rem);
+    a.remainder = &rd;
+  }
   if (redo) {
     r = packed(redo, LLSA_I32, {redo_elems});
     a.fwd_redo = &r;
@@ -239,10 +245,12 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
   const size_t t_scratch = llsa_transpose_scratch_bytes(d.B, d.H, d.nq1, topk, d.n1);
   const int64_t n_partial = tensor_core ? llsa_attn_bwd_partial_elems(d.B, d.H, d.Nq, topk) : 0;
   const int64_t acc1 = BH * d.n1 * D, acc2 = c.two ? BH * d.n2 * D : 0;
+  LlsaAttnArgs a = c.args(topk, topk_p, d.bs, w1, w2);
+  const int64_t n_rem = llsa_attn_remainder_elems(&a, 1);
   Carver cv;
   const int64_t o_off = cv.take(BH * (d.n1 + 1) * 4), o_flat = cv.take(BH * E * 4), o_pairs = cv.take(BH * E * 4), o_ranges = cv.take(BH * R * 8),
                 o_ts = cv.take((int64_t) t_scratch), o_delta = cv.take(BH * d.Nq * 4),
-                o_acc = cv.take(acc ? 0 : (2 * acc1 + 2 * acc2) * 4), o_partial = cv.take(n_partial * 4);
+                o_acc = cv.take(acc ? 0 : (2 * acc1 + 2 * acc2) * 4), o_partial = cv.take(n_partial * 4), o_rem = cv.take(n_rem * 2);
   const Tensor ws = byte_buffer(cv.off, like);
   char* p = (char*) ws.data_ptr();
   if (!acc) acc = (float*) (p + o_acc);
@@ -251,7 +259,8 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
                    delta = packed(p + o_delta, LLSA_F32, {d.B, d.H, d.Nq}), dpk = packed(acc, LLSA_F32, {d.B, d.H, d.n1, D}),
                    dpv = packed(acc + acc1, LLSA_F32, {d.B, d.H, d.n1, D}), dpk2 = packed(acc + 2 * acc1, LLSA_F32, {d.B, d.H, d.n2, D}),
                    dpv2 = packed(acc + 2 * acc1 + acc2, LLSA_F32, {d.B, d.H, d.n2, D}),
-                   partial = packed(p + o_partial, LLSA_F32, {d.B, d.H, BH ? n_partial / (BH * 4096) : 0, 4096});
+                   partial = packed(p + o_partial, LLSA_F32, {d.B, d.H, BH ? n_partial / (BH * 4096) : 0, 4096}),
+                   rem = packed(p + o_rem, LLSA_BF16, {d.B, d.H, d.Nq, D});
   const Status t_status(like), status(like);
 
   const at::cuda::CUDAStream cur = at::cuda::getCurrentCUDAStream(like.device().index());
@@ -272,12 +281,12 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
                    : llsa_transpose_indices(&c.indices, &offsets, &flat, d.n1, t_scratch ? p + o_ts : nullptr, t_scratch, t_status.ptr(), st),
        "transpose_indices");
   };
-  LlsaAttnArgs a = c.args(topk, topk_p, d.bs, w1, w2);
   a.d_o = &d_o; a.dq = &dq; a.dk = &dk; a.dv = &dv;
   a.offsets = &offsets; a.flat = &flat; a.delta = &delta;
   a.dpk_acc = &dpk; a.dpv_acc = &dpv;
   if (c.two) { a.dpk2_acc = &dpk2; a.dpv2_acc = &dpv2; }
   if (tensor_core) { a.dkv_partial = &partial; a.flat_pairs = &pairs; a.flat_ranges = &ranges; }
+  if (n_rem) a.remainder = &rem;
   a.fold_pool_bwd = fold;
   a.kv_weight = (float) kvw1; a.kv_weight_2 = (float) kvw2;
   a.status = status.ptr();

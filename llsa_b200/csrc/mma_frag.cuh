@@ -242,7 +242,13 @@ __device__ __forceinline__ void store_acc_row_t(bf16* row, const float (&acc)[8]
   *reinterpret_cast<uint4*>(row + 16 * t + 8) = y;
 }
 
-// max of three in one instruction (sm_100)
+// What is left of (x, y) after rounding to the bf16 pair `hi`, itself a bf16 pair: hi + rest holds the value to 16 bits.  An infinity
+// leaves nothing.
+__device__ __forceinline__ uint32_t pack_rest(float x, float y, uint32_t hi) {
+  const float a = bf16_lo(hi), b = bf16_hi(hi);
+  return pack_bf16(fabsf(a) == INFINITY ? 0.f : x - a, fabsf(b) == INFINITY ? 0.f : y - b);
+}
+
 // Two fp32 values in a register pair: one issue slot for two of the softmax's multiplies and adds (each rounded as the scalar
 // instruction rounds it).
 struct F2 { uint64_t v; };
@@ -267,6 +273,7 @@ __device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
   return r;
 }
+// max of three in one instruction (sm_100)
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
