@@ -251,10 +251,9 @@ typedef struct LlsaAttnArgs {
   int32_t* status;             /* device int32 or NULL: kernels OR LlsaDeviceStatus bits into it; the
                                   caller zeroes it, and reads it back after synchronising */
   const LlsaTensor* fwd_redo;  /* forward, optional: I32 scratch of at least B*H*N/4 elements (one byte per
-                                  query row; not read before it is written).  With it, a pooled stage
-                                  that walks the pooled key list chunk by chunk (any number of pooled keys
-                                  per row but 64, 128 and 192) makes ONE pass over the keys with the fine part's log-sum-exp as the
-                                  reference of its exponentials, marks here the rows whose pooled keys
+                                  query row; not read before it is written), of use where llsa_attn_fwd_redo_elems() is not 0:
+                                  a pooled stage that walks a long pooled key list chunk by chunk then makes ONE pass over the
+                                  keys with a reference of its exponentials taken from the fine part's log-sum-exp, marks here the rows whose pooled keys
                                   outweigh the fine ones by more than 1e30, and redoes
                                   exactly those rows with the exact two-pass form.  NULL: two passes for
                                   every row.  Same results either way up to rounding */
@@ -279,6 +278,9 @@ int llsa_attn_bwd(const LlsaAttnArgs* args, void* stream);
  * Nq query rows per (b,h) and `topk` selected blocks per query block (the caller allocates it; any 4-D contiguous
  * shape with at least this many elements is accepted).  The library itself never allocates device memory. */
 int64_t llsa_attn_bwd_partial_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk);
+/* Elements of the scratch LlsaAttnArgs.fwd_redo a forward makes use of, 0 if none (its pooled keys all fit at once, or the list is too short
+ * for one pass to pay).  Read from `args` as below. */
+int64_t llsa_attn_fwd_redo_elems(const LlsaAttnArgs* args);
 /* Elements of the scratch LlsaAttnArgs.remainder the forward (backward = 0) or the backward of a problem makes use of, 0 if none.  Read from
  * `args`: the shapes of q and k, q's type, whether pk2 is given, topk, topk_p and the two switches. */
 int64_t llsa_attn_remainder_elems(const LlsaAttnArgs* args, int backward);

@@ -46,7 +46,7 @@ EXPORTS = [
     "llsa_rms_rope_bwd", "llsa_rms_rope_bwd_partial_elems",
     "llsa_rope_fwd", "llsa_rope_bwd", "llsa_coarse_topk", "llsa_refine_topk", "llsa_select_two_level", "llsa_transpose_scratch_bytes",
     "llsa_transpose_indices", "llsa_transpose_indices_pairs", "llsa_transpose_range_entries", "llsa_transpose_indices_noalloc", "llsa_attn_fwd", "llsa_attn_bwd",
-    "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems", "llsa_attn_remainder_elems", "llsa_status_check",
+    "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems", "llsa_attn_remainder_elems", "llsa_attn_fwd_redo_elems", "llsa_status_check",
 ]
 
 _lib: Optional[C.CDLL] = None
@@ -83,13 +83,15 @@ def _declare(lib: C.CDLL) -> None:
     lib.llsa_attn_bwd_pds_elems.restype = C.c_int64
     lib.llsa_attn_remainder_elems.argtypes = [C.POINTER(LlsaAttnArgs), C.c_int]
     lib.llsa_attn_remainder_elems.restype = C.c_int64
+    lib.llsa_attn_fwd_redo_elems.argtypes = [C.POINTER(LlsaAttnArgs)]
+    lib.llsa_attn_fwd_redo_elems.restype = C.c_int64
     lib.llsa_status_check.argtypes = [C.c_int32]
     lib.llsa_attn_fwd.argtypes = [C.POINTER(LlsaAttnArgs), C.c_void_p]
     lib.llsa_attn_bwd.argtypes = [C.POINTER(LlsaAttnArgs), C.c_void_p]
     for name in EXPORTS:
         fn = getattr(lib, name)
         if name not in ("llsa_last_error_string", "llsa_transpose_scratch_bytes", "llsa_attn_bwd_partial_elems", "llsa_attn_bwd_pds_elems",
-                        "llsa_rms_rope_bwd_partial_elems", "llsa_attn_remainder_elems"):
+                        "llsa_rms_rope_bwd_partial_elems", "llsa_attn_remainder_elems", "llsa_attn_fwd_redo_elems"):
             fn.restype = C.c_int
 
 

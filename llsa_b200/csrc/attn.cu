@@ -111,8 +111,18 @@ bool remainder_wanted(const AttnP<__nv_bfloat16>& a, bool bwd) {
 
 using namespace llsa;
 
+static bool on_tcgen05(const LlsaAttnArgs* g) {
+  return g && g->q && g->k && g->q->ndim == 4 && g->k->ndim == 4 && g->q->dtype == LLSA_BF16 && !g->force_generic && !g->no_tcgen05;
+}
+
+extern "C" int64_t llsa_attn_fwd_redo_elems(const LlsaAttnArgs* g) {
+  if (!on_tcgen05(g)) return 0;
+  const AttnP<__nv_bfloat16> a = attn_dims<__nv_bfloat16>(g);
+  return !pooled_tc_keys(a) && pooled_loop_tc_keys(a) && pooled_loop_one_pass(a) ? (g->q->shape[0] * a.H * a.Nq + 3) / 4 : 0;
+}
+
 extern "C" int64_t llsa_attn_remainder_elems(const LlsaAttnArgs* g, int backward) {
-  if (!g || !g->q || !g->k || g->q->ndim != 4 || g->k->ndim != 4 || g->q->dtype != LLSA_BF16 || g->force_generic || g->no_tcgen05) return 0;
+  if (!on_tcgen05(g)) return 0;
   return remainder_wanted(attn_dims<__nv_bfloat16>(g), backward != 0) ? g->q->shape[0] * g->q->shape[1] * g->q->shape[2] * kD : 0;
 }
 

@@ -204,25 +204,32 @@ struct Core {      // operands common to forward and backward
   }
 };
 
-void run_fwd(const Core& c, int topk, int topk_p, int bs, double w1, double w2, const Tensor& like, void* redo, int64_t redo_elems,
-             const Status& status, cudaStream_t st) {
+void keep_redo(const Tensor& t) {
+  std::lock_guard<std::mutex> lock(g_redo_mutex);
+  last_redo() = t;
+}
+
+void run_fwd(const Core& c, int topk, int topk_p, int bs, double w1, double w2, const Tensor& like, const Status& status, cudaStream_t st) {
   LlsaAttnArgs a = c.args(topk, topk_p, bs, w1, w2);
   LlsaTensor r, rd;
-  Tensor rem;
+  Tensor redo, rem;
+  const int64_t n_redo = flag(kTwoPass) ? 0 : llsa_attn_fwd_redo_elems(&a);      // marks of the one-pass form (include/llsa_b200.h: fwd_redo)
+  if (n_redo) {
+    redo = at::empty({n_redo}, like.options().dtype(at::kInt));
+    r = desc(redo);
+    a.fwd_redo = &r;
+  }
   if (llsa_attn_remainder_elems(&a, 0)) {
     rem = at::empty({c.q.shape[0], c.q.shape[1], c.q.shape[2], c.q.shape[3]}, like.options());
     rd = desc(rem);
     a.remainder = &rd;
-  }
-  if (redo) {
-    r = packed(redo, LLSA_I32, {redo_elems});
-    a.fwd_redo = &r;
   }
   a.status = status.ptr();
   mark("attn_fwd");
   ok(llsa_attn_fwd(&a, st), "attn_fwd");
   mark("end");
   status.check("attn_fwd");
+  if (n_redo) keep_redo(redo);
 }
 
 // One side stream per device: the index transpose is needed only by the last stage of the backward and leaves most SMs idle.
@@ -321,17 +328,6 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
   status.check("attn_bwd");
 }
 
-// Marks of the one-pass form of the pooled lists that are walked chunk by chunk (include/llsa_b200.h: fwd_redo): one byte per query
-// row, wanted where a row's pooled keys are not the 64, 128 or 192 the single-shot kernel holds.
-int64_t redo_elems(const Dims& d, bool bf16, bool two, int64_t topk_p) {
-  const int64_t pooled = two ? topk_p * d.bs + (d.n2 >= 64 ? d.n2 : 0) : (d.n1 >= 64 ? d.n1 : 0);
-  return bf16 && !flag(kTwoPass) && (pooled > 192 || pooled % 64) ? (d.B * d.H * d.Nq + 3) / 4 : 0;
-}
-void keep_redo(const Tensor& t) {
-  std::lock_guard<std::mutex> lock(g_redo_mutex);
-  last_redo() = t;
-}
-
 Core make_core(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& pk, const Tensor& pv, const OptTensor& pk2, const OptTensor& pv2,
                const Tensor& indices, const OptTensor& p_indices, const Tensor& o, const Tensor& lse) {
   Core c;
@@ -355,15 +351,10 @@ std::vector<Tensor> attn_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v
     pk2c = cont(*pk2); pv2c = cont(*pv2); pic = cont(*p_indices);
   }
   const Dims d(q, k, block_size);
-  const bool bf16 = q.scalar_type() == at::kBFloat16;
-  Tensor o = at::empty_like(q), lse = at::empty({d.B, d.H, d.Nq}, q.options().dtype(at::kFloat)), redo;
-  const int64_t n_redo = redo_elems(d, bf16, pk2.has_value(), topk_p);
-  if (n_redo) redo = at::empty({n_redo}, q.options().dtype(at::kInt));
+  Tensor o = at::empty_like(q), lse = at::empty({d.B, d.H, d.Nq}, q.options().dtype(at::kFloat));
   const Status status(q);
   const Core c = make_core(q, k, v, pkc, pvc, pk2c, pv2c, ic, pic, o, lse);
-  run_fwd(c, (int) topk, (int) topk_p, (int) block_size, w1, w2, q, n_redo ? redo.data_ptr() : nullptr, n_redo, status,
-          at::cuda::getCurrentCUDAStream(q.device().index()));
-  if (n_redo) keep_redo(redo);
+  run_fwd(c, (int) topk, (int) topk_p, (int) block_size, w1, w2, q, status, at::cuda::getCurrentCUDAStream(q.device().index()));
   return {o, lse};
 }
 
@@ -405,7 +396,7 @@ std::vector<Tensor> layer_fwd(const Tensor& q_, const Tensor& k_, const Tensor& 
   const Dims d(q, k, block_size);
   TORCH_CHECK(k.sizes() == v.sizes() && k.sizes() == q.sizes(), "llsa_b200: q, k, v must have the same shape");
   const at::ScalarType dt = q.scalar_type();
-  const bool bf16 = dt == at::kBFloat16, two = levels == 2, norm = wq.has_value() || wk.has_value();
+  const bool two = levels == 2, norm = wq.has_value() || wk.has_value();
   const int64_t D = q.size(3), es = q.element_size(), BH = d.B * d.H;
   const int code = dtype_code(dt);
   const int topk1 = (int) (two ? topk1_ : std::min<int64_t>(topk1_, d.n1)), topk2 = two ? (int) std::min<int64_t>(topk2_, d.n2) : 0;
@@ -481,12 +472,7 @@ std::vector<Tensor> layer_fwd(const Tensor& q_, const Tensor& k_, const Tensor& 
   Tensor o = at::empty_like(q);
   c.o = desc(o);
   const Status status(q);
-  const int64_t n_redo = redo_elems(d, bf16, two, topk2);
-  Tensor redo;
-  if (n_redo) redo = at::empty({n_redo}, q.options().dtype(at::kInt));
-  run_fwd(c, topk1, topk2, (int) block_size, (double) block_size, two ? (double) (block_size * block_size) : 1.0, q,
-          n_redo ? redo.data_ptr() : nullptr, n_redo, status, st);
-  if (n_redo) keep_redo(redo);
+  run_fwd(c, topk1, topk2, (int) block_size, (double) block_size, two ? (double) (block_size * block_size) : 1.0, q, status, st);
   out[0] = o;
   out[1] = saved;
   return out;

@@ -184,3 +184,24 @@ def test_bwd_partial_scratch_size():
     assert L.llsa_attn_bwd_partial_elems(1, 1, 256, 8) == 2 * 4096
     assert L.llsa_attn_bwd_pds_elems(1, 1, 256, 8) == 16 * 8 * 256                  # 1 KB per (query block, selected block) pair
     assert L.llsa_attn_bwd_partial_elems(0, 6, 16384, 8) == 0
+
+
+@pytest.mark.parametrize("N,topk_p,redo,rest_fwd,rest_bwd", [
+    (1024, 0, 0, 0, 1), (2560, 0, 0, 1, 1), (5632, 0, 1, 1, 1), (4096, 0, 1, 0, 0), (512, 0, 0, 0, 0),      # one level: 64, 160, 352, 256, no pooled keys
+    (16384, 8, 0, 0, 0), (5376, 8, 0, 0, 1), (24576, 2, 0, 1, 1), (40960, 2, 0, 1, 1), (40960, 16, 1, 1, 1), (262144, 8, 1, 0, 0), (8192, 34, 0, 0, 0)])
+def test_forward_scratch_follows_the_kernel_choice(N, topk_p, redo, rest_fwd, rest_bwd):
+    """Marks and remainders are asked for exactly where the kernel that runs makes use of them (two levels: 32 + 96 and 32 + 160 keys are
+    no list of the single-shot kernel, whatever their sum)."""
+    lib, a = _lib.lib(), _lib.LlsaAttnArgs()
+    q = fake((2, 3, N, 64))
+    a.q, a.k, a.topk, a.topk_p, a.block_size = C.pointer(q), C.pointer(q), 8, topk_p, 16
+    pk2 = fake((2, 3, max(N // 256, 1), 64))
+    if topk_p:
+        a.pk2 = C.pointer(pk2)
+    rows = 2 * 3 * N
+    ask = lambda: (lib.llsa_attn_fwd_redo_elems(C.byref(a)), lib.llsa_attn_remainder_elems(C.byref(a), 0), lib.llsa_attn_remainder_elems(C.byref(a), 1))
+    assert ask() == (redo * rows // 4, rest_fwd * rows * 64, rest_bwd * rows * 64)
+    a.no_tcgen05 = 1
+    assert ask() == (0, 0, 0)
+    a.no_tcgen05, q.dtype = 0, _lib.F32
+    assert ask() == (0, 0, 0)
