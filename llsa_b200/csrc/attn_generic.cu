@@ -164,11 +164,13 @@ __global__ void __launch_bounds__(kGw * 32) attn_fwd_generic(AttnP<T> a) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) s[r][j] *= a.scale;
       const float mnew = fmaxf(m[r], quad4_max(fmaxf(fmaxf(s[r][0], s[r][1]), fmaxf(s[r][2], s[r][3]))));
-      const float alpha = expf(m[r] - mnew);
+      // a warp may meet nothing but scores of -inf (keys masked by the type's lowest value): they weigh 0 whatever the reference
+      const float ref = mnew == -INFINITY ? 0.f : mnew;
+      const float alpha = expf(m[r] - ref);
       float sum = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        s[r][j] = expf(s[r][j] - mnew);
+        s[r][j] = expf(s[r][j] - ref);
         sum += s[r][j];
         s[r][j] = round_to<T>(s[r][j]) * w;         // exp_scores.to(v.dtype)
       }

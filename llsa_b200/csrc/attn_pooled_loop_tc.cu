@@ -272,6 +272,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           if (lane == 0) tma::mbar_arrive(&bars.xchg);
           const bool ok_ = __all_sync(0xffffffffu, tc::bounded_wait(&bars.xchg, (uint32_t) i & 1, abort_flag));
           mx = fmaxf(s_max[i & 1][0][r], s_max[i & 1][1][r]);
+          if (mx == -INFINITY) mx = 0.f;       // no score above -inf (masked keys): their weight is 0 whatever the reference
           return ok_;
         };
         for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
