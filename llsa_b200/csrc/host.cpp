@@ -518,7 +518,8 @@ std::vector<Tensor> layer_bwd(const Tensor& d_o_, const Tensor& q_, const Tensor
     LlsaTensor f;
     if (freq_) {
       freq = *freq_;
-      if (freq.scalar_type() != dt && (norm || freq.scalar_type() != at::kFloat)) freq = freq.to(norm ? dt : at::kFloat);
+      // a table wider than the data stays: the backward has always rotated with the table as it was given
+      if (freq.scalar_type() != dt && freq.scalar_type() != at::kFloat) freq = freq.to(at::kFloat);
       if (!table_ok(freq)) freq = freq.contiguous();
       f = desc(freq);
     }

@@ -1,0 +1,45 @@
+"""The layer with the q / k preparation in front, as a caller makes it: table types, absent norms and tables, frozen weights."""
+import pytest
+import torch
+
+import llsa_b200
+from llsa_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+EPS = 1e-5
+
+
+def _inputs(N, seed=3):
+    q, k, v, do = [t.to(DEV) for t in synth.gaussian_qkv(seed, 1, 2, N, 64, dtype=torch.bfloat16)]
+    gen = torch.Generator().manual_seed(seed)
+    ang = torch.rand(N, 32, generator=gen) * 6.3
+    table = torch.stack([ang.sin(), ang.cos()], -1).reshape(N, 64).to(DEV)
+    wq, wk = (1 + 0.2 * torch.randn(2, 64, generator=gen)).to(DEV)
+    return q, k, v, do, table, wq, wk
+
+
+def _norm_backward(x, w, g):
+    x, g = x.double(), g.double()
+    rstd = torch.rsqrt(x.square().mean(-1, keepdim=True) + EPS)
+    xh, gw = x * rstd, g * w.double()
+    return rstd * (gw - xh * (gw * xh).mean(-1, keepdim=True)), (g * xh).sum((0, 1, 2))
+
+
+@pytest.mark.parametrize("table_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,two_level", [(2048, False), (4096, True)])
+def test_norm_and_rotation_backward_with_the_table_as_given(N, two_level, table_dtype):
+    """dq and the norm's weight gradient against the stand-alone rotation with the same table (bf16 data, fp32 table: products rounded to
+    fp32, not with a table cut to bf16) and the norm's gradient in fp64."""
+    q, k, v, do, table, wq, wk = _inputs(N)
+    table = table.to(table_dtype)
+    x, w = [t.detach().clone().requires_grad_(True) for t in (q, k, v)], [t.clone().requires_grad_(True) for t in (wq, wk)]
+    layer = llsa_b200.llsa_l2_rms_rope if two_level else llsa_b200.llsa_l1_rms_rope
+    layer(*x, *w, table, EPS).backward(do)
+    # the operator on q and k prepared beforehand
+    prepared = [llsa_b200.my_rope_fn(ops.rms_norm(t, s, EPS), table.to(q.dtype)).detach().requires_grad_(True) for t, s in ((q, wq), (k, wk))]
+    plain = llsa_b200.llsa_l2 if two_level else llsa_b200.llsa_l1
+    dqr, = torch.autograd.grad(plain(*prepared, v), prepared[:1], do)
+    dq, dw = _norm_backward(q, wq, ops._rope_bwd_op(dqr, table))
+    assert ((x[0].grad.double() - dq).abs() <= 2.0 ** -8 * dq.abs() + 2e-5 * float(dq.abs().max())).all()       # one rounding to bf16
+    assert float((w[0].grad.double() - dw).norm() / dw.norm()) < 1e-5                                           # fp32 sums
