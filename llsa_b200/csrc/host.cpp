@@ -607,7 +607,10 @@ struct LayerFunction : torch::autograd::Function<LayerFunction> {
     const variable_list s = ctx->get_saved_variables();
     const std::vector<int64_t> cfg = ctx->saved_data["cfg"].toIntVector();
     const double eps = ctx->saved_data["eps"].toDouble();
-    const bool want_dw = (s[8].defined() && ctx->needs_input_grad(4)) || (s[9].defined() && ctx->needs_input_grad(5));
+    // needs_input_grad counts the tensors that were given: an absent table or weight has no edge
+    size_t edge = 3 + (s[5].defined() ? 1 : 0);
+    const bool want_wq = s[8].defined() && ctx->needs_input_grad(edge++), want_wk = s[9].defined() && ctx->needs_input_grad(edge);
+    const bool want_dw = want_wq || want_wk;
     std::vector<Tensor> r;
     auto call = [&] {
       r = bwd_op().call(grads[0], s[0], s[1], s[2], s[3], s[4], opt(s[5]), opt(s[6]), opt(s[7]), opt(s[8]), opt(s[9]), eps, cfg[0], cfg[1], cfg[2],

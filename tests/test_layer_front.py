@@ -43,3 +43,34 @@ def test_norm_and_rotation_backward_with_the_table_as_given(N, two_level, table_
     dq, dw = _norm_backward(q, wq, ops._rope_bwd_op(dqr, table))
     assert ((x[0].grad.double() - dq).abs() <= 2.0 ** -8 * dq.abs() + 2e-5 * float(dq.abs().max())).all()       # one rounding to bf16
     assert float((w[0].grad.double() - dw).norm() / dw.norm()) < 1e-5                                           # fp32 sums
+
+
+# which of wq, wk and the table are given; which of the inputs take a gradient; which gradients are asked for
+@pytest.mark.parametrize("given,train,ask", [
+    ("wq wk table", "q k v wq wk", "q k wq wk"), ("wq wk", "q k v wq wk", "q wq wk"), ("wq wk", "q k v", "q k"), ("wq wk", "q k v wq", "q wq"),
+    ("wq wk", "q k v wk", "k wk"), ("wq wk", "wk", "wk"), ("wq table", "q k v wq", "q wq"), ("wk table", "q k v wk", "q k wk"), ("wk table", "q k v", "q"),
+    ("wq wk table", "q k v wk", "q wk"), ("wq wk table", "q k v wq wk", "q")])
+def test_absent_norms_and_tables_frozen_weights(given, train, ask):
+    """Gradients of every form of the call against the operator on q and k prepared beforehand."""
+    given, train, ask = given.split(), train.split(), ask.split()
+    q, k, v, do, table, wq, wk = _inputs(4096)
+    table = table.to(q.dtype)
+    t = dict(q=q, k=k, v=v, wq=wq if "wq" in given else None, wk=wk if "wk" in given else None)
+    x = {n: s.detach().clone().requires_grad_(n in train) if s is not None else None for n, s in t.items()}
+    o = llsa_b200.llsa_l2_rms_rope(x["q"], x["k"], x["v"], x["wq"], x["wk"], table if "table" in given else None, EPS)
+    got = dict(zip(ask, torch.autograd.grad(o, [x[n] for n in ask], do)))
+    prepared = {}
+    for n, w in (("q", t["wq"]), ("k", t["wk"])):
+        y = ops.rms_norm(t[n], w, EPS) if w is not None else t[n]
+        prepared[n] = (llsa_b200.my_rope_fn(y, table) if "table" in given else y).detach().clone().requires_grad_(True)
+    want_o = llsa_b200.llsa_l2(prepared["q"], prepared["k"], v)
+    assert torch.equal(o, want_o)
+    grads = dict(zip("qk", torch.autograd.grad(want_o, [prepared["q"], prepared["k"]], do)))
+    for n, w in (("q", t["wq"]), ("k", t["wk"])):
+        g = ops._rope_bwd_op(grads[n], table) if "table" in given else grads[n]
+        dx, dw = _norm_backward(t[n], w, g) if w is not None else (g.double(), None)
+        # one rounding to bf16 (2^-9 of a value at most) on top of the sums of the pooled-key gradients, whose order differs from call to call
+        if n in got:
+            assert float((got[n].double() - dx).norm() / dx.norm()) < 2.0 ** -8
+        if "w" + n in got:
+            assert float((got["w" + n].double() - dw).norm() / dw.norm()) < 1e-4
