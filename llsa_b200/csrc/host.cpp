@@ -428,7 +428,8 @@ std::vector<Tensor> layer_fwd(const Tensor& q_, const Tensor& k_, const Tensor& 
     ok(llsa_pool_pyramid_fwd(3, x, y1, two ? y2 : nullptr, (int) block_size, st), "pool_pyramid_fwd");
   } else {
     LlsaTensor x[3] = {desc(q), desc(k), desc(v)}, xr[3], f;
-    Tensor qr = at::empty_like(q), kr = at::empty_like(k);
+    // without a table a tensor that has no norm passes unchanged: a copy, since an output of the operator must not be its input
+    Tensor qr = freq.defined() || wq ? at::empty_like(q) : q.clone(), kr = freq.defined() || wk ? at::empty_like(k) : k.clone();
     xr[0] = desc(qr); xr[1] = desc(kr); xr[2] = x[2];
     if (freq.defined()) f = desc(freq);
     if (freq.defined() && freq.scalar_type() != dt) {      // a table wider than the data: rotate first, then pool

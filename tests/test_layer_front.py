@@ -49,7 +49,7 @@ def test_norm_and_rotation_backward_with_the_table_as_given(N, two_level, table_
 @pytest.mark.parametrize("given,train,ask", [
     ("wq wk table", "q k v wq wk", "q k wq wk"), ("wq wk", "q k v wq wk", "q wq wk"), ("wq wk", "q k v", "q k"), ("wq wk", "q k v wq", "q wq"),
     ("wq wk", "q k v wk", "k wk"), ("wq wk", "wk", "wk"), ("wq table", "q k v wq", "q wq"), ("wk table", "q k v wk", "q k wk"), ("wk table", "q k v", "q"),
-    ("wq wk table", "q k v wk", "q wk"), ("wq wk table", "q k v wq wk", "q")])
+    ("wq", "wq", "wq"), ("wk", "q k v wk", "q wk"), ("wq wk table", "q k v wk", "q wk"), ("wq wk table", "q k v wq wk", "q")])
 def test_absent_norms_and_tables_frozen_weights(given, train, ask):
     """Gradients of every form of the call against the operator on q and k prepared beforehand."""
     given, train, ask = given.split(), train.split(), ask.split()
