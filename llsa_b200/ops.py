@@ -123,6 +123,16 @@ def _native():
     return _host
 
 
+def _ready() -> None:
+    """The native host path loaded and up to date, in front of a call of one of its operators."""
+    _native()
+
+
+# A compiled function runs it while it is traced (the loading takes locks and builds descriptors, which cannot be traced) and calls the
+# operator alone afterwards.  This is the mark torch.compiler.assume_constant_result leaves; that function would import the compiler, 4 s.
+_ready._dynamo_marked_constant = True
+
+
 def __getattr__(name):
     if name == "_last_fwd_redo":      # the marks of the most recent forward over a long pooled list: which rows its second round redid
         _native()
@@ -513,7 +523,7 @@ def transpose_indices(q_topk_indices: torch.Tensor, k_ntx: Optional[int] = None,
 
 # ----------------------------------------------------------------------------- attention core
 def _attn_fwd(q, k, v, pk, pv, pk2, pv2, indices, p_indices, topk, topk_p, block_size, w1, w2):
-    _native()
+    _ready()
     return tuple(torch.ops.llsa_b200.attn_fwd(q, k, v, pk, pv, pk2, pv2, indices, p_indices, int(topk), int(topk_p), int(block_size), float(w1),
                                               float(w2)))
 
@@ -543,7 +553,7 @@ def _carve_bytes(specs) -> int:
 
 
 def _attn_bwd(do, q, k, v, pk, pv, pk2, pv2, o, lse, indices, p_indices, topk, topk_p, block_size, w1, w2, kvw1, kvw2, fold):
-    _native()
+    _ready()
     g = torch.ops.llsa_b200.attn_bwd(do, q, k, v, pk, pv, pk2, pv2, o, lse, indices, p_indices, int(topk), int(topk_p), int(block_size), float(w1),
                                      float(w2), float(kvw1), float(kvw2), bool(fold))
     return tuple(g) + (None,) * (7 - len(g))
@@ -626,7 +636,7 @@ flash_sparse_residual_attention_l2_op = _FlashSparseResidualAttentionL2.apply
 
 # ----------------------------------------------------------------------------- fused drop-in operators
 def _layer(q, k, v, freq, wq, wk, eps, topk1, topk2, block_size, levels):
-    _native()
+    _ready()
     return torch.ops.llsa_b200.layer_fwd(q, k, v, freq, wq, wk, eps, topk1, topk2, block_size, levels)
 
 
