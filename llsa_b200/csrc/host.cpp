@@ -242,6 +242,36 @@ at::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
   return *s;
 }
 
+// Work on the side stream between two points of the current one.  The second point is there whatever happens in between: a call that
+// fails half way gives its scratch back to the allocator of the current stream, which may hand it out while the side stream still writes,
+// and a capture cannot end with an open fork.
+struct Fork {
+  const at::cuda::CUDAStream cur, side;
+  at::cuda::CUDAEvent done;
+  bool recorded = false, open = true;
+  Fork(const at::cuda::CUDAStream& c, const at::cuda::CUDAStream& s) : cur(c), side(s) {
+    at::cuda::CUDAEvent start;
+    start.record(cur);
+    start.block(side);
+  }
+  void record() {
+    done.record(side);
+    recorded = true;
+  }
+  void join() {
+    open = false;
+    if (!recorded) record();
+    done.block(cur);
+  }
+  ~Fork() {
+    if (!open) return;
+    try {
+      join();
+    } catch (...) {      // an error of the call itself is on its way out
+    }
+  }
+};
+
 // dq, dk, dv are written; acc holds dpk, dpv(, dpk2, dpv2) back to back in fp32 (nullptr: taken from the call's scratch).
 void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq, const LlsaTensor& dk, const LlsaTensor& dv, int topk,
              int topk_p, double w1, double w2, double kvw1, double kvw2, bool fold, bool bf16, float* acc, const Tensor& like) {
@@ -300,16 +330,14 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
   if (overlap) {
     // the scratch belongs to the current stream; the side stream works between the two events
     const at::cuda::CUDAStream side = side_stream(like.device().index());
-    at::cuda::CUDAEvent fork, join;
-    fork.record(cur);
-    fork.block(side);
+    Fork fork(cur, side);
     // the accumulators are cleared and the lists transposed next to the dQ stage, which needs neither
     if (acc1) C10_CUDA_CHECK(cudaMemsetAsync(acc, 0, (2 * acc1 + 2 * acc2) * 4, side));
     transpose(side);
-    join.record(side);
+    fork.record();
     a.stage_mask = 1 | 8;
     ok(llsa_attn_bwd(&a, cur), "attn_bwd");
-    join.block(cur);
+    fork.join();
     a.stage_mask = 2 | 4;
     ok(llsa_attn_bwd(&a, cur), "attn_bwd");
   } else {

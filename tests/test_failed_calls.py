@@ -1,0 +1,36 @@
+"""Calls of the host path that fail half way, and calls it refuses."""
+import pytest
+import torch
+
+import llsa_b200
+from llsa_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _layer(N, H=2):
+    q, k, v, do = [t.to(DEV) for t in synth.gaussian_qkv(N, 1, H, N, 64, dtype=torch.bfloat16)]
+    o, saved = ops._layer(q, k, v, None, None, None, 0.0, 8, 8, 16, 2)
+    bwd = lambda d_o, q=q, k=k, v=v, o=o, saved=saved: torch.ops.llsa_b200.layer_bwd(d_o, q, k, v, o, saved, None, None, None, None, None, 0.0, 8, 8, 16, 2,
+                                                                                  False)
+    return q, k, v, do, o, saved, bwd
+
+
+def test_a_backward_that_fails_behind_the_fork_joins_the_side_stream():
+    """A gradient of the wrong length is found when the index transpose is already on the side stream.  Were the streams not joined on the
+    way out, the capture around the call could not end."""
+    q, k, v, do, o, saved, bwd = _layer(16384)
+    want = bwd(do)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        with pytest.raises(RuntimeError, match="d_o"):
+            bwd(do[:, :, 256:])
+        got = bwd(do)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], want[0])
+    with pytest.raises(RuntimeError, match="d_o"):
+        bwd(do[:, :, 256:])
+    assert torch.equal(bwd(do)[0], want[0])
