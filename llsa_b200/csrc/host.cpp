@@ -108,6 +108,13 @@ void need_cuda(const Tensor& t) {
   TORCH_CHECK(t.is_cuda(), "llsa_b200 runs on CUDA tensors only (got a ", t.device().type(), " tensor); there is no CPU path");
 }
 
+// Operands the caller may leave out are undefined tensors here.  A host pointer in a descriptor would be read by a kernel.
+void need_cuda(std::initializer_list<Tensor> ts) {
+  for (const Tensor& t : ts)
+    if (t.defined()) need_cuda(t);
+}
+Tensor or_none(const OptTensor& t) { return t.value_or(Tensor()); }
+
 void check_float(std::initializer_list<const Tensor*> ts) {
   const at::ScalarType dt = (*ts.begin())->scalar_type();
   TORCH_CHECK_TYPE(dt == at::kFloat || dt == at::kBFloat16, "llsa_b200 supports float32 and bfloat16 tensors, got ", dt);
@@ -369,7 +376,7 @@ Core make_core(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& 
 std::vector<Tensor> attn_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& pk, const Tensor& pv, const OptTensor& pk2,
                              const OptTensor& pv2, const Tensor& indices, const OptTensor& p_indices, int64_t topk, int64_t topk_p,
                              int64_t block_size, double w1, double w2) {
-  for (const Tensor* t : {&q_, &k_, &v_}) need_cuda(*t);
+  need_cuda({q_, k_, v_, pk, pv, or_none(pk2), or_none(pv2), indices, or_none(p_indices)});
   check_float({&q_, &k_, &v_, &pk, &pv});
   const c10::cuda::CUDAGuard guard(q_.device());
   const Tensor q = prep(q_), k = prep(k_), v = prep(v_), pkc = cont(pk), pvc = cont(pv), ic = cont(indices);
@@ -390,7 +397,7 @@ std::vector<Tensor> attn_bwd(const Tensor& d_o_, const Tensor& q_, const Tensor&
                              const OptTensor& pk2, const OptTensor& pv2, const Tensor& o_, const Tensor& lse, const Tensor& indices,
                              const OptTensor& p_indices, int64_t topk, int64_t topk_p, int64_t block_size, double w1, double w2, double kvw1,
                              double kvw2, bool fold) {
-  for (const Tensor* t : {&d_o_, &q_, &k_, &v_}) need_cuda(*t);
+  need_cuda({d_o_, q_, k_, v_, pk, pv, or_none(pk2), or_none(pv2), o_, lse, indices, or_none(p_indices)});
   const c10::cuda::CUDAGuard guard(q_.device());
   const Tensor d_o = prep(d_o_), q = prep(q_), k = prep(k_), v = prep(v_), o = prep(o_), pkc = cont(pk), pvc = cont(pv), ic = cont(indices),
                lc = cont(lse);
@@ -416,7 +423,7 @@ std::vector<Tensor> attn_bwd(const Tensor& d_o_, const Tensor& q_, const Tensor&
 // ------------------------------------------------------------------ the fused layer
 std::vector<Tensor> layer_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const OptTensor& freq_, const OptTensor& wq, const OptTensor& wk,
                               double eps, int64_t topk1_, int64_t topk2_, int64_t block_size, int64_t levels) {
-  for (const Tensor* t : {&q_, &k_, &v_}) need_cuda(*t);
+  need_cuda({q_, k_, v_, or_none(freq_), or_none(wq), or_none(wk)});
   check_float({&q_, &k_, &v_});
   const c10::cuda::CUDAGuard guard(q_.device());
   const cudaStream_t st = at::cuda::getCurrentCUDAStream(q_.device().index());
@@ -445,7 +452,6 @@ std::vector<Tensor> layer_fwd(const Tensor& q_, const Tensor& k_, const Tensor& 
   Tensor freq;
   if (freq_) {
     freq = *freq_;
-    need_cuda(freq);
     if (norm && freq.scalar_type() != dt) freq = freq.to(dt);
     else if (freq.scalar_type() == at::kDouble || (dt == at::kFloat && freq.scalar_type() == at::kBFloat16)) freq = freq.to(at::kFloat);
     if (!table_ok(freq)) freq = freq.contiguous();
@@ -511,7 +517,7 @@ std::vector<Tensor> layer_fwd(const Tensor& q_, const Tensor& k_, const Tensor& 
 std::vector<Tensor> layer_bwd(const Tensor& d_o_, const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o_, const Tensor& saved,
                               const OptTensor& freq_, const OptTensor& xq, const OptTensor& xk, const OptTensor& wq, const OptTensor& wk, double eps,
                               int64_t topk1_, int64_t topk2_, int64_t block_size, int64_t levels, bool want_dw) {
-  need_cuda(d_o_);
+  need_cuda({d_o_, q_, k_, v_, o_, saved, or_none(freq_), or_none(xq), or_none(xk), or_none(wq), or_none(wk)});
   check_float({&q_, &k_, &v_, &d_o_});
   const c10::cuda::CUDAGuard guard(q_.device());
   const cudaStream_t st = at::cuda::getCurrentCUDAStream(q_.device().index());

@@ -324,7 +324,7 @@ def rms_rope_pool_pyramid(xs: List[torch.Tensor], weights: List[Optional[torch.T
     every pyramid level in ONE pass over HBM: what the attention block does to q and k before llsa_l1 / llsa_l2
     (models/rope_dit_transformer_2d.py:215-238).  Returns (transformed tensors, level-1 list, level-2 list or None); the
     results carry the bits of rms_norm -> my_rope_fn -> mean_pool1d run one after the other."""
-    _need_cuda(*xs)
+    _need_cuda(*xs, freq if any(rope) else None, *[w for w in weights if isinstance(w, torch.Tensor)])
     _check_float(*xs)
     xs = [_prep(x) for x in xs]
     B, H, N, D = xs[0].shape
@@ -361,7 +361,7 @@ def rms_rope_pool_pyramid(xs: List[torch.Tensor], weights: List[Optional[torch.T
 def rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], eps: float = 1e-5) -> torch.Tensor:
     """RMSNorm over the last dimension of [B,H,S,C] with a fixed summation order (the stand-alone form of the
     normalisation fused into rms_rope_pool_pyramid); not differentiable by itself."""
-    _need_cuda(x)
+    _need_cuda(x, weight)
     _check_float(x)
     x = _prep(x)
     y = torch.empty_like(x)

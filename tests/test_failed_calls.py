@@ -34,3 +34,30 @@ def test_a_backward_that_fails_behind_the_fork_joins_the_side_stream():
     with pytest.raises(RuntimeError, match="d_o"):
         bwd(do[:, :, 256:])
     assert torch.equal(bwd(do)[0], want[0])
+
+
+@pytest.mark.parametrize("which", ["q", "k", "v", "o", "saved"])
+def test_backward_refuses_a_host_operand(which):
+    """What a saved-tensor hook that forgets to bring a tensor back would hand over."""
+    q, k, v, do, o, saved, bwd = _layer(4096)
+    x = dict(q=q, k=k, v=v, o=o, saved=saved)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        bwd(do, **{which: x[which].cpu()})
+
+
+def test_operators_refuse_a_host_weight_index_or_table():
+    q, k, v, do, o, saved, bwd = _layer(4096)
+    w, table = torch.ones(64, device=DEV), torch.ones(4096, 64, device=DEV, dtype=q.dtype)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        llsa_b200.llsa_l2_rms_rope(q, k, v, w.cpu(), w, table)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        llsa_b200.llsa_l2_rms_rope(q, k, v, w, w, table.cpu())
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        ops.rms_norm(q, w.cpu())
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        ops.rms_rope_pool_pyramid([q, k, v], [w, w.cpu(), None], 1e-5, table, [True, True, False], 16, 2)
+    dbg = llsa_b200.llsa_l1_debug(q, k, v, 8, 16)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        ops.sparse_indices_attn_res_fwd(q, k, v, dbg["pk"].cpu(), dbg["pv"], dbg["indices"], 8, 16)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        ops.sparse_indices_attn_res_scatter_bwd_v2(do, q, k, v, dbg["pk"], dbg["pv"], dbg["o"], dbg["lse"], dbg["indices"].cpu(), 8, 16, 16)
