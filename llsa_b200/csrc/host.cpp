@@ -406,11 +406,12 @@ std::vector<Tensor> attn_bwd(const Tensor& d_o_, const Tensor& q_, const Tensor&
     TORCH_CHECK(pv2 && p_indices, "llsa_b200: pv2 / p_indices missing for the two-level form");
     pk2c = cont(*pk2); pv2c = cont(*pv2); pic = cont(*p_indices);
   }
+  TORCH_CHECK(ic.dim() == 4 && ic.size(3) == topk, "llsa_b200: indices must be [B,H,N/block,topk=", topk, "], got ", ic.sizes());
   const Dims d(q, k, block_size);
   const int64_t D = q.size(3), a1 = d.B * d.H * d.n1 * D, a2 = pk2 ? d.B * d.H * d.n2 * D : 0;
   Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), acc = at::empty({2 * a1 + 2 * a2}, q.options().dtype(at::kFloat));
   Core c = make_core(q, k, v, pkc, pvc, pk2c, pv2c, ic, pic, o, lc);
-  run_bwd(c, d, desc(d_o), desc(dq), desc(dk), desc(dv), (int) ic.size(3), (int) topk_p, w1, w2, kvw1, kvw2, fold,
+  run_bwd(c, d, desc(d_o), desc(dq), desc(dk), desc(dv), (int) topk, (int) topk_p, w1, w2, kvw1, kvw2, fold,
           q.scalar_type() == at::kBFloat16, (float*) acc.data_ptr(), q);
   std::vector<Tensor> out = {dq, dk, dv, acc.narrow(0, 0, a1).view(pkc.sizes()), acc.narrow(0, a1, a1).view(pvc.sizes())};
   if (pk2) {

@@ -61,3 +61,17 @@ def test_operators_refuse_a_host_weight_index_or_table():
         ops.sparse_indices_attn_res_fwd(q, k, v, dbg["pk"].cpu(), dbg["pv"], dbg["indices"], 8, 16)
     with pytest.raises(RuntimeError, match="CUDA tensors only"):
         ops.sparse_indices_attn_res_scatter_bwd_v2(do, q, k, v, dbg["pk"], dbg["pv"], dbg["o"], dbg["lse"], dbg["indices"].cpu(), 8, 16, 16)
+
+
+def test_core_backward_refuses_lists_of_another_length():
+    q, k, v, do, o, saved, bwd = _layer(4096)
+    one = llsa_b200.llsa_l1_debug(q, k, v, 8, 16)
+    two = llsa_b200.llsa_l2_debug(q, k, v, 8, 8, 16)
+    with pytest.raises(RuntimeError, match="indices"):
+        ops.sparse_indices_attn_res_scatter_bwd_v2(do, q, k, v, one["pk"], one["pv"], one["o"], one["lse"], one["indices"], 4, 16, 16)
+    with pytest.raises(RuntimeError, match="indices"):
+        ops.sparse_indices_attn_res_scatter_2_2_bwd_v2(do, q, k, v, *[two[n] for n in ("pk", "pv", "pk2", "pv2", "o", "lse", "indices", "p_indices")],
+                                                       4, 8, 16, 16, 256)
+    with pytest.raises(RuntimeError, match="p_indices"):
+        ops.sparse_indices_attn_res_scatter_2_2_bwd_v2(do, q, k, v, *[two[n] for n in ("pk", "pv", "pk2", "pv2", "o", "lse", "indices", "p_indices")],
+                                                       8, 4, 16, 16, 256)
