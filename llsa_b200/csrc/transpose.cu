@@ -87,9 +87,9 @@ __global__ void __launch_bounds__(W * 32) transpose_range_kernel(TransposeArgs a
   __shared__ int warp_sums[32];
   __shared__ int s_below[W], s_kept[W];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t bh = blockIdx.y;
-  const int E = (int) a.E, n = (int) a.n_kv, lo = (int) blockIdx.x * keys_per_range, K = min(keys_per_range, n - lo);
-  const bool last = (int) blockIdx.x + 1 == (int) gridDim.x;
+  const int64_t bh = blockIdx.x;                         // any number of heads: the x axis has no 65,535 limit
+  const int E = (int) a.E, n = (int) a.n_kv, lo = (int) blockIdx.y * keys_per_range, K = min(keys_per_range, n - lo);
+  const bool last = (int) blockIdx.y + 1 == (int) gridDim.y;
   int* base = reinterpret_cast<int*>(smraw);             // [K + 1]
   int* tab = base + keys_per_range + 1;                  // [W][K] entries seen, then [W][K] lanes that hold the key right now
   for (int i = threadIdx.x; i < 2 * W * K; i += blockDim.x) tab[i] = 0;
@@ -389,7 +389,7 @@ static int transpose_impl(const LlsaTensor* idx, const LlsaTensor* offsets, cons
   ranges_per_head = ranges_per_head > most ? most : ranges_per_head;
   ranges_per_head = ranges_per_head < fewest ? fewest : ranges_per_head;
   const int keys = (int) ((n_kv + ranges_per_head - 1) / ranges_per_head);
-  const dim3 grid((unsigned) ((n_kv + keys - 1) / keys), (unsigned) (B * H));
+  const dim3 grid((unsigned) (B * H), (unsigned) ((n_kv + keys - 1) / keys));
   const size_t smem = ((size_t) keys * (2 * warps + 1) + 1) * sizeof(int);
   cudaStream_t st = (cudaStream_t) stream;
   if (warps == 32) {

@@ -84,3 +84,14 @@ def test_transpose_ranges(BH, M, T, n, kind):
     assert (pairs.cpu()[0, :, :kept].sort(-1).values.diff(dim=-1) > 0).all()
     cut = ranges.cpu()[0, ..., 0]
     assert int(cut.min()) >= 0 and int(cut.max()) <= kept and (cut.diff(dim=-1) >= 0).all()
+
+
+def test_index_transpose_of_many_heads():
+    """More (batch, head) slices than the y axis of a launch grid holds."""
+    heads, M, T, n = 70000, 2, 2, 8
+    idx = torch.randint(0, n, (heads, 1, M, T), generator=torch.Generator().manual_seed(1), dtype=torch.int32)
+    offsets, flat = [t.cpu() for t in ops.transpose_indices(idx.to(DEV), n)]
+    counts = torch.nn.functional.one_hot(idx.long().view(heads, -1), n).sum(1)
+    assert torch.equal(offsets[:, 0, 1:], counts.cumsum(-1)) and not offsets[..., 0].any()
+    order = idx.view(heads, -1).sort(dim=-1, stable=True).indices          # entry positions by key, in their original order
+    assert torch.equal(flat[:, 0], (order // T).int())
