@@ -671,6 +671,9 @@ struct LayerFunction : torch::autograd::Function<LayerFunction> {
 std::vector<Tensor> layer_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& freq, const OptTensor& wq,
                                        const OptTensor& wk, double eps, int64_t topk1, int64_t topk2, int64_t block_size, int64_t levels) {
   auto wants = [](const Tensor& t) { return t.requires_grad(); };
+  if (wq || wk)      // the tangent would be dropped without a word
+    for (const Tensor& t : {q, k, v, or_none(wq), or_none(wk)})
+      TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(0).defined(), "llsa_b200: no forward-mode derivative of the layer with norms in front");
   if (at::GradMode::is_enabled() && (wants(q) || wants(k) || wants(v) || (wq && wants(*wq)) || (wk && wants(*wk))))
     return LayerFunction::apply(q, k, v, freq, wq, wk, eps, topk1, topk2, block_size, levels);
   at::AutoDispatchBelowADInplaceOrView below;

@@ -74,3 +74,14 @@ def test_absent_norms_and_tables_frozen_weights(given, train, ask):
             assert float((got[n].double() - dx).norm() / dx.norm()) < 2.0 ** -8
         if "w" + n in got:
             assert float((got["w" + n].double() - dw).norm() / dw.norm()) < 1e-4
+
+
+@pytest.mark.parametrize("which", ["q", "v", "wk"])
+def test_forward_mode_is_refused(which):
+    import torch.autograd.forward_ad as fw
+    q, k, v, do, table, wq, wk = _inputs(2048)
+    x = dict(q=q, k=k, v=v, wq=wq, wk=wk)
+    with fw.dual_level():
+        x[which] = fw.make_dual(x[which], torch.ones_like(x[which]))
+        with pytest.raises(NotImplementedError):
+            llsa_b200.llsa_l1_rms_rope(*x.values(), table.to(q.dtype), EPS)
