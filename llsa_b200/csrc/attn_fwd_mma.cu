@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) attn_fwd_fine_kernel(AttnP<b
 // slower: the call succeeds, and the thread's error string says why so that a caller who wonders can find out.
 void note_scalar_path() {
   set_error("note: bf16 operands ran on the scalar kernels (the tensor-core kernels need 32-byte aligned rows, "
-            "batch/head/token strides that are multiples of 16 elements, and top-k <= 32)");
+            "batch/head/token strides that are multiples of 16 elements and at least a row, and top-k <= 32)");
 }
 
 bool mma_path_ok(const LlsaAttnArgs* g, bool bwd) {
@@ -378,7 +378,7 @@ bool mma_path_ok(const LlsaAttnArgs* g, bool bwd) {
     if (!t) continue;
     if ((uintptr_t) t->ptr % 32) return false;
     for (int i = 0; i < 3; ++i)
-      if (t->shape[i] != 1 && t->stride[i] % 16) return false;
+      if (t->shape[i] != 1 && (t->stride[i] % 16 || t->stride[i] < kD)) return false;      // a tensor map's strides reach past a row
   }
   return ((uintptr_t) g->pk->ptr % 32) == 0 && ((uintptr_t) g->pv->ptr % 32) == 0 &&
          (!g->pk2 || (((uintptr_t) g->pk2->ptr % 32) == 0 && ((uintptr_t) g->pv2->ptr % 32) == 0));

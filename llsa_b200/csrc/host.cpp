@@ -121,12 +121,13 @@ void check_float(std::initializer_list<const Tensor*> ts) {
   for (const Tensor* t : ts) TORCH_CHECK_TYPE(t->scalar_type() == dt, "llsa_b200: all floating-point operands must share one dtype");
 }
 
-// Unit channel stride; bf16 rows on 32-byte boundaries (256-bit loads of the tensor-core kernels), fp32 rows on 16-byte ones.
+// Unit channel stride; bf16 rows on 32-byte boundaries (256-bit loads of the tensor-core kernels), fp32 rows on 16-byte ones; no rows that
+// overlap, such as those of an expanded tensor: tensor maps are specified for strides that reach past a row.
 bool rows_ok(const Tensor& t) {
   const int64_t align = t.scalar_type() == at::kBFloat16 ? 32 : 16, per = align / t.element_size();
   if (t.stride(-1) != 1 || (uintptr_t) t.data_ptr() % align) return false;
   for (int64_t i = 0; i + 1 < t.dim(); ++i)
-    if (t.size(i) != 1 && t.stride(i) % per) return false;
+    if (t.size(i) != 1 && (t.stride(i) % per || t.stride(i) < t.size(-1))) return false;
   return true;
 }
 Tensor prep(const Tensor& t) { return rows_ok(t) ? t : t.contiguous(); }
