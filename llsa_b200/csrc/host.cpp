@@ -54,7 +54,9 @@ void mark(const char* name) {
   if (g_hook) pybind11::reinterpret_borrow<pybind11::object>(g_hook)(name);
 }
 
-// The marks of the most recent forward (which rows its second round redid), for whoever wants to look at them.
+// The marks of the most recent forward that was asked to leave them (which rows its second round redid; undefined if it made none): the
+// debug forms of the operators ask, every other call's marks end with the call.
+thread_local bool t_keep_marks = false;
 std::mutex g_redo_mutex;
 Tensor& last_redo() {
   static Tensor* t = new Tensor();      // not destroyed at exit: the CUDA context may be gone by then
@@ -237,7 +239,7 @@ void run_fwd(const Core& c, int topk, int topk_p, int bs, double w1, double w2, 
   ok(llsa_attn_fwd(&a, st), "attn_fwd");
   mark("end");
   status.check("attn_fwd");
-  if (n_redo) keep_redo(redo);
+  if (t_keep_marks) keep_redo(redo);
 }
 
 // One side stream per device: the index transpose is needed only by the last stage of the backward and leaves most SMs idle.
@@ -725,6 +727,7 @@ PYBIND11_MODULE(_host, m) {
     g_flags.store(flags);
     g_wait_limit.store(wait_limit);
   });
+  m.def("keep_marks", [](bool keep) { t_keep_marks = keep; });      // of this thread's forwards
   m.def("set_stage_hook", [](pybind11::object fn) {
     PyObject* old = g_hook;
     g_hook = fn.is_none() ? nullptr : fn.inc_ref().ptr();

@@ -134,7 +134,7 @@ _ready._dynamo_marked_constant = True
 
 
 def __getattr__(name):
-    if name == "_last_fwd_redo":      # the marks of the most recent forward over a long pooled list: which rows its second round redid
+    if name == "_last_fwd_redo":      # the marks of the most recent llsa_*_debug call: which rows its second round redid; None if it made none
         _native()
         return torch.ops.llsa_b200.last_fwd_redo()
     raise AttributeError("module %r has no attribute %r" % (__name__, name))
@@ -680,7 +680,14 @@ def llsa_l2(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, topk1: int = 8, t
 
 
 def _layer_debug(q, k, v, topk1, topk2, block_size, levels):
-    o, saved = _layer(q, k, v, None, None, None, 0.0, topk1, topk2, block_size, levels)
+    host = None if torch.compiler.is_compiling() else _native()
+    if host is not None:
+        host.keep_marks(True)
+    try:
+        o, saved = _layer(q, k, v, None, None, None, 0.0, topk1, topk2, block_size, levels)
+    finally:
+        if host is not None:
+            host.keep_marks(False)
     return dict(o=o, **_carve(saved, _saved_specs(*q.shape, q.dtype, topk1, topk2, block_size, levels)))
 
 

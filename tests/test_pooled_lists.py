@@ -52,3 +52,18 @@ def test_tail_keys_of_the_next_head_do_not_leak():
     assert torch.equal(o[:, :1], o_want) and torch.equal(got[0].grad[:, :1], want[0].grad)
     for i in (1, 2):      # fp32 reductions: the order of the sums may differ
         assert float((got[i].grad[:, :1].float() - want[i].grad.float()).norm() / want[i].grad.float().norm()) < 1e-3
+
+
+def test_marks_are_those_of_the_last_debug_call():
+    """A production call leaves no marks (nor their memory) behind, and a debug call whose list needs none says so."""
+    q, k, v, _ = [t.to(DEV) for t in synth.gaussian_qkv(7, 1, 2, 16384, 64, dtype=torch.bfloat16)]
+    llsa_b200.llsa_l1_debug(q, k, v, 8, 16)                                  # 1024 pooled keys: one pass, marks
+    marks = ops._last_fwd_redo
+    assert marks.numel() * 4 == 2 * 16384 and not marks.any()
+    short = [t[:, :, :5632].contiguous() for t in (q, k, v)]
+    llsa_b200.llsa_l1(*short, 8, 16)
+    assert ops._last_fwd_redo.data_ptr() == marks.data_ptr()
+    llsa_b200.llsa_l1_debug(*short, 8, 16)
+    assert ops._last_fwd_redo.numel() * 4 == 2 * 5632
+    llsa_b200.llsa_l2_debug(q, k, v, 8, 8, 16)                               # 192 pooled keys: all at once
+    assert ops._last_fwd_redo is None
