@@ -155,10 +155,10 @@ int llsa_select_two_level(const LlsaTensor* pq1, const LlsaTensor* pk1, const Ll
 size_t llsa_transpose_scratch_bytes(int64_t B, int64_t H, int64_t M, int64_t T, int64_t n_kv);
 int llsa_transpose_indices(const LlsaTensor* idx, const LlsaTensor* offsets, const LlsaTensor* flat, int64_t n_kv,
                            void* scratch, size_t scratch_bytes, int32_t* status, void* stream);
-/* The same transpose with two more lists for llsa_attn_bwd (the reference has the plain list only,
- * indices_transpose.py:70-78):
+/* The same transpose with two more lists, either of which may be NULL (the reference has the plain list only,
+ * indices_transpose.py:70-78); `scratch` is not used:
  *   pairs  [B,H,M*T] (I32): in the order of `flat`, the position m*T + t of each entry inside its head's idx
- *          (flat = pairs / T); finds what the query-major stage left for each (query block, selected block) pair;
+ *          (flat = pairs / T); llsa_attn_bwd has no use for it;
  *   ranges [B,H,ceil(M*T/S),2] (I32), S = llsa_transpose_range_entries(B,H,M,T) (32, or 16 for problems too small to fill
  *          the GPU with 32; the tensor's length tells the library which): the entry list cut into the work ranges of
  *          the dK/dV kernel, (first entry, bucket of that entry) per range.  Range r nominally starts at entry S r;
@@ -238,10 +238,9 @@ typedef struct LlsaAttnArgs {
                                   blocks whose list of query blocks is split over several CTAs (not
                                   read before it is written; may be NULL for f32 tensors) */
   const LlsaTensor* fine_pds;  /* not used any more (the dK/dV stage recomputes P and dS); may be NULL */
-  const LlsaTensor* flat_pairs;/* backward, bf16 tensors only: I32 [B,H,N/16*topk], the `pairs` list of
-                                  llsa_transpose_indices_pairs for the same CSR as offsets / flat */
+  const LlsaTensor* flat_pairs;/* not used any more; NULL, or the `pairs` list of llsa_transpose_indices_pairs */
   const LlsaTensor* flat_ranges;/* backward, bf16 tensors only: I32 [B,H,ceil(N/16*topk/S),2], the `ranges`
-                                  list of the same call */
+                                  list of llsa_transpose_indices_pairs for the same CSR as offsets / flat */
   int32_t no_tcgen05;          /* 1: keep the pooled-key stages on the mma.sync kernels (the form used
                                   for shapes the tcgen05 kernels do not cover); for cross-checks */
   int32_t wait_limit;          /* 0: default.  Otherwise the number of polls after which a bounded

@@ -79,8 +79,8 @@ static int check_attn_args(const LlsaAttnArgs* g, bool bwd) {
                    LLSA_ERR_WORKSPACE, "attn_bwd: dkv_partial must be a contiguous F32 tensor of at least %lld elements", (long long) need);
     }
     if (dt == LLSA_BF16 && !g->force_generic) {
-      LLSA_REQUIRE(g->flat_pairs && g->flat_ranges, LLSA_ERR_WORKSPACE, "attn_bwd: flat_pairs / flat_ranges missing (llsa_transpose_indices_pairs)");
-      if ((rc = check_contig(g->flat_pairs, "flat_pairs", LLSA_I32, 3, sf))) return rc;
+      LLSA_REQUIRE(g->flat_ranges, LLSA_ERR_WORKSPACE, "attn_bwd: flat_ranges missing (llsa_transpose_indices_pairs)");
+      if (g->flat_pairs && (rc = check_contig(g->flat_pairs, "flat_pairs", LLSA_I32, 3, sf))) return rc;
       LLSA_REQUIRE(g->flat_ranges->ndim == 4 && range_entries_of(nq1 * g->topk, g->flat_ranges->shape[2]) > 0, LLSA_ERR_SHAPE,
                    "attn_bwd: flat_ranges must be the [B,H,R,2] ranges tensor of llsa_transpose_indices_pairs");
       const int64_t sr[4] = {B, H, g->flat_ranges->shape[2], 2};

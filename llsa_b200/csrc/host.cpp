@@ -289,20 +289,18 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
   const bool tensor_core = bf16 && !flag(kForceGeneric);
   const int S = llsa_transpose_range_entries(d.B, d.H, d.nq1, topk);
   const int64_t R = (E + S - 1) / S;
-  const size_t t_scratch = llsa_transpose_scratch_bytes(d.B, d.H, d.nq1, topk, d.n1);
   const int64_t n_partial = tensor_core ? llsa_attn_bwd_partial_elems(d.B, d.H, d.Nq, topk) : 0;
   const int64_t acc1 = BH * d.n1 * D, acc2 = c.two ? BH * d.n2 * D : 0;
   LlsaAttnArgs a = c.args(topk, topk_p, d.bs, w1, w2);
   const int64_t n_rem = llsa_attn_remainder_elems(&a, 1);
   Carver cv;
-  const int64_t o_off = cv.take(BH * (d.n1 + 1) * 4), o_flat = cv.take(BH * E * 4), o_pairs = cv.take(BH * E * 4), o_ranges = cv.take(BH * R * 8),
-                o_ts = cv.take((int64_t) t_scratch), o_delta = cv.take(BH * d.Nq * 4),
+  const int64_t o_off = cv.take(BH * (d.n1 + 1) * 4), o_flat = cv.take(BH * E * 4), o_ranges = cv.take(BH * R * 8), o_delta = cv.take(BH * d.Nq * 4),
                 o_acc = cv.take(acc ? 0 : (2 * acc1 + 2 * acc2) * 4), o_partial = cv.take(n_partial * 4), o_rem = cv.take(n_rem * 2);
   const Tensor ws = byte_buffer(cv.off, like);
   char* p = (char*) ws.data_ptr();
   if (!acc) acc = (float*) (p + o_acc);
   const LlsaTensor offsets = packed(p + o_off, LLSA_I32, {d.B, d.H, d.n1 + 1}), flat = packed(p + o_flat, LLSA_I32, {d.B, d.H, E}),
-                   pairs = packed(p + o_pairs, LLSA_I32, {d.B, d.H, E}), ranges = packed(p + o_ranges, LLSA_I32, {d.B, d.H, R, 2}),
+                   ranges = packed(p + o_ranges, LLSA_I32, {d.B, d.H, R, 2}),
                    delta = packed(p + o_delta, LLSA_F32, {d.B, d.H, d.Nq}), dpk = packed(acc, LLSA_F32, {d.B, d.H, d.n1, D}),
                    dpv = packed(acc + acc1, LLSA_F32, {d.B, d.H, d.n1, D}), dpk2 = packed(acc + 2 * acc1, LLSA_F32, {d.B, d.H, d.n2, D}),
                    dpv2 = packed(acc + 2 * acc1 + acc2, LLSA_F32, {d.B, d.H, d.n2, D}),
@@ -323,16 +321,14 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
   const bool overlap = !hooked && !flag(kNoOverlap) && (BH * d.nq1 > 1024 || capturing());
   auto transpose = [&](cudaStream_t st) {
     mark("transpose_indices");
-    ok(tensor_core ? llsa_transpose_indices_pairs(&c.indices, &offsets, &flat, &pairs, &ranges, d.n1, t_scratch ? p + o_ts : nullptr, t_scratch,
-                                                  t_status.ptr(), st)
-                   : llsa_transpose_indices(&c.indices, &offsets, &flat, d.n1, t_scratch ? p + o_ts : nullptr, t_scratch, t_status.ptr(), st),
+    ok(llsa_transpose_indices_pairs(&c.indices, &offsets, &flat, nullptr, tensor_core ? &ranges : nullptr, d.n1, nullptr, 0, t_status.ptr(), st),
        "transpose_indices");
   };
   a.d_o = &d_o; a.dq = &dq; a.dk = &dk; a.dv = &dv;
   a.offsets = &offsets; a.flat = &flat; a.delta = &delta;
   a.dpk_acc = &dpk; a.dpv_acc = &dpv;
   if (c.two) { a.dpk2_acc = &dpk2; a.dpv2_acc = &dpv2; }
-  if (tensor_core) { a.dkv_partial = &partial; a.flat_pairs = &pairs; a.flat_ranges = &ranges; }
+  if (tensor_core) { a.dkv_partial = &partial; a.flat_ranges = &ranges; }
   if (n_rem) a.remainder = &rem;
   a.fold_pool_bwd = fold;
   a.kv_weight = (float) kvw1; a.kv_weight_2 = (float) kvw2;

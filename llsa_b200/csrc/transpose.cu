@@ -333,7 +333,7 @@ extern "C" size_t llsa_transpose_scratch_bytes(int64_t B, int64_t H, int64_t M, 
 }
 
 static int transpose_impl(const LlsaTensor* idx, const LlsaTensor* offsets, const LlsaTensor* flat, const LlsaTensor* pairs,
-                          const LlsaTensor* ranges, int64_t n_kv, void* scratch, size_t scratch_bytes, int32_t* status, void* stream) {
+                          const LlsaTensor* ranges, int64_t n_kv, int32_t* status, void* stream) {
   LLSA_REQUIRE(idx && offsets && flat && idx->ptr && offsets->ptr && flat->ptr, LLSA_ERR_NULL, "transpose_indices: null tensor");
   LLSA_REQUIRE(idx->ndim == 4, LLSA_ERR_SHAPE, "transpose_indices: idx must be [B,H,M,T]");
   const int64_t B = idx->shape[0], H = idx->shape[1], M = idx->shape[2], T = idx->shape[3];
@@ -360,8 +360,6 @@ static int transpose_impl(const LlsaTensor* idx, const LlsaTensor* offsets, cons
   // the per-key prefixes over the segments are 16-bit: with distinct keys inside a row a key occurs at most M times per head
   LLSA_REQUIRE(M <= 65535, LLSA_ERR_SHAPE, "transpose_indices: M=%lld query blocks per head exceed the supported 65535", (long long) M);
   LLSA_REQUIRE((int64_t) n_kv * 4 <= 200 * 1024, LLSA_ERR_SHAPE, "transpose_indices: n_kv=%lld too large", (long long) n_kv);
-  const size_t need = llsa_transpose_scratch_bytes(B, H, M, T, n_kv);
-  LLSA_REQUIRE(need == 0 || (scratch && scratch_bytes >= need), LLSA_ERR_WORKSPACE, "transpose_indices: needs %zu bytes of scratch", need);
   if (B * H == 0) return LLSA_OK;
   TransposeArgs a;
   a.idx = make_idx(idx);
@@ -405,14 +403,19 @@ static int transpose_impl(const LlsaTensor* idx, const LlsaTensor* offsets, cons
 
 extern "C" int llsa_transpose_indices(const LlsaTensor* idx, const LlsaTensor* offsets, const LlsaTensor* flat, int64_t n_kv,
                                       void* scratch, size_t scratch_bytes, int32_t* status, void* stream) {
-  return transpose_impl(idx, offsets, flat, nullptr, nullptr, n_kv, scratch, scratch_bytes, status, stream);
+  if (idx && idx->ndim == 4 && n_kv >= 1) {      // what this entry point asks for by contract, although no table lives there any more
+    const size_t need = llsa_transpose_scratch_bytes(idx->shape[0], idx->shape[1], idx->shape[2], idx->shape[3], n_kv);
+    LLSA_REQUIRE(need == 0 || (scratch && scratch_bytes >= need), LLSA_ERR_WORKSPACE, "transpose_indices: needs %zu bytes of scratch", need);
+  }
+  return transpose_impl(idx, offsets, flat, nullptr, nullptr, n_kv, status, stream);
 }
 
 extern "C" int llsa_transpose_indices_pairs(const LlsaTensor* idx, const LlsaTensor* offsets, const LlsaTensor* flat, const LlsaTensor* pairs,
                                             const LlsaTensor* ranges, int64_t n_kv, void* scratch, size_t scratch_bytes, int32_t* status,
                                             void* stream) {
-  LLSA_REQUIRE(pairs && pairs->ptr && ranges && ranges->ptr, LLSA_ERR_NULL, "transpose_indices_pairs: null pairs / ranges tensor");
-  return transpose_impl(idx, offsets, flat, pairs, ranges, n_kv, scratch, scratch_bytes, status, stream);
+  (void) scratch;
+  (void) scratch_bytes;
+  return transpose_impl(idx, offsets, flat, pairs, ranges, n_kv, status, stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -95,3 +95,20 @@ def test_index_transpose_of_many_heads():
     assert torch.equal(offsets[:, 0, 1:], counts.cumsum(-1)) and not offsets[..., 0].any()
     order = idx.view(heads, -1).sort(dim=-1, stable=True).indices          # entry positions by key, in their original order
     assert torch.equal(flat[:, 0], (order // T).int())
+
+
+@pytest.mark.parametrize("n_kv", [64, 16384])
+def test_index_transpose_without_the_pairs_list_and_scratch(n_kv):
+    import ctypes as C
+
+    from llsa_b200 import _lib
+    B, H, M, T = 1, 2, 300, 8
+    idx = torch.randint(0, n_kv, (B, H, M, T), generator=torch.Generator().manual_seed(n_kv), dtype=torch.int32).to(DEV)
+    offsets, flat, (pairs, ranges), _ = ops._transpose(idx, n_kv, torch.int32, True)
+    got = [torch.full_like(t, -7) for t in (offsets, flat, ranges)]
+    d = [_lib.desc(t) for t in (idx, *got)]
+    lib = _lib.lib()
+    _lib.check(lib.llsa_transpose_indices_pairs(*[_lib.ref(t) for t in d[:3]], None, _lib.ref(d[3]), n_kv, None, 0, None, _lib.stream_ptr(torch.device(DEV))),
+               "transpose_indices_pairs")
+    assert all(torch.equal(a, b) for a, b in zip(got, (offsets, flat, ranges)))
+    assert torch.equal(flat.long(), pairs.long() // T)
