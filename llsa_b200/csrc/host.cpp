@@ -282,9 +282,9 @@ struct Fork {
   }
 };
 
-// dq, dk, dv are written; acc holds dpk, dpv(, dpk2, dpv2) back to back in fp32 (nullptr: taken from the call's scratch).
+// dq, dk, dv are written, and dpk, dpv(, dpk2, dpv2) in fp32 at acc (nullptr: in the call's scratch).
 void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq, const LlsaTensor& dk, const LlsaTensor& dv, int topk,
-             int topk_p, double w1, double w2, double kvw1, double kvw2, bool fold, bool bf16, float* acc, const Tensor& like) {
+             int topk_p, double w1, double w2, double kvw1, double kvw2, bool fold, bool bf16, float* const* acc, const Tensor& like) {
   const int64_t BH = d.B * d.H, E = d.nq1 * topk, D = d.B * d.H ? c.q.shape[3] : 0;
   const bool tensor_core = bf16 && !flag(kForceGeneric);
   const int S = llsa_transpose_range_entries(d.B, d.H, d.nq1, topk);
@@ -298,12 +298,14 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
                 o_acc = cv.take(acc ? 0 : (2 * acc1 + 2 * acc2) * 4), o_partial = cv.take(n_partial * 4), o_rem = cv.take(n_rem * 2);
   const Tensor ws = byte_buffer(cv.off, like);
   char* p = (char*) ws.data_ptr();
-  if (!acc) acc = (float*) (p + o_acc);
+  float* const scratch = (float*) (p + o_acc);
+  float* const inside[4] = {scratch, scratch + acc1, scratch + 2 * acc1, scratch + 2 * acc1 + acc2};
+  float* const* const at = acc ? acc : inside;
   const LlsaTensor offsets = packed(p + o_off, LLSA_I32, {d.B, d.H, d.n1 + 1}), flat = packed(p + o_flat, LLSA_I32, {d.B, d.H, E}),
                    ranges = packed(p + o_ranges, LLSA_I32, {d.B, d.H, R, 2}),
-                   delta = packed(p + o_delta, LLSA_F32, {d.B, d.H, d.Nq}), dpk = packed(acc, LLSA_F32, {d.B, d.H, d.n1, D}),
-                   dpv = packed(acc + acc1, LLSA_F32, {d.B, d.H, d.n1, D}), dpk2 = packed(acc + 2 * acc1, LLSA_F32, {d.B, d.H, d.n2, D}),
-                   dpv2 = packed(acc + 2 * acc1 + acc2, LLSA_F32, {d.B, d.H, d.n2, D}),
+                   delta = packed(p + o_delta, LLSA_F32, {d.B, d.H, d.Nq}), dpk = packed(at[0], LLSA_F32, {d.B, d.H, d.n1, D}),
+                   dpv = packed(at[1], LLSA_F32, {d.B, d.H, d.n1, D}), dpk2 = packed(at[2], LLSA_F32, {d.B, d.H, d.n2, D}),
+                   dpv2 = packed(at[3], LLSA_F32, {d.B, d.H, d.n2, D}),
                    partial = packed(p + o_partial, LLSA_F32, {d.B, d.H, BH ? n_partial / (BH * 4096) : 0, 4096}),
                    rem = packed(p + o_rem, LLSA_BF16, {d.B, d.H, d.Nq, D});
   const Status t_status(like), status(like);
@@ -338,7 +340,11 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
     const at::cuda::CUDAStream side = side_stream(like.device().index());
     Fork fork(cur, side);
     // the accumulators are cleared and the lists transposed next to the dQ stage, which needs neither
-    if (acc1) C10_CUDA_CHECK(cudaMemsetAsync(acc, 0, (2 * acc1 + 2 * acc2) * 4, side));
+    if (!acc) {
+      if (acc1) C10_CUDA_CHECK(cudaMemsetAsync(scratch, 0, (2 * acc1 + 2 * acc2) * 4, side));
+    } else {
+      for (int i = 0; i < (c.two ? 4 : 2); ++i) C10_CUDA_CHECK(cudaMemsetAsync(acc[i], 0, (i < 2 ? acc1 : acc2) * 4, side));
+    }
     transpose(side);
     fork.record();
     a.stage_mask = 1 | 8;
@@ -407,16 +413,16 @@ std::vector<Tensor> attn_bwd(const Tensor& d_o_, const Tensor& q_, const Tensor&
   }
   TORCH_CHECK(ic.dim() == 4 && ic.size(3) == topk, "llsa_b200: indices must be [B,H,N/block,topk=", topk, "], got ", ic.sizes());
   const Dims d(q, k, block_size);
-  const int64_t D = q.size(3), a1 = d.B * d.H * d.n1 * D, a2 = pk2 ? d.B * d.H * d.n2 * D : 0;
-  Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), acc = at::empty({2 * a1 + 2 * a2}, q.options().dtype(at::kFloat));
-  Core c = make_core(q, k, v, pkc, pvc, pk2c, pv2c, ic, pic, o, lc);
-  run_bwd(c, d, desc(d_o), desc(dq), desc(dk), desc(dv), (int) topk, (int) topk_p, w1, w2, kvw1, kvw2, fold,
-          q.scalar_type() == at::kBFloat16, (float*) acc.data_ptr(), q);
-  std::vector<Tensor> out = {dq, dk, dv, acc.narrow(0, 0, a1).view(pkc.sizes()), acc.narrow(0, a1, a1).view(pvc.sizes())};
-  if (pk2) {
-    out.push_back(acc.narrow(0, 2 * a1, a2).view(pk2c->sizes()));
-    out.push_back(acc.narrow(0, 2 * a1 + a2, a2).view(pv2c->sizes()));
+  // tensors of their own, not views of one: outputs of an operator must not share memory
+  std::vector<Tensor> out = {at::empty_like(q), at::empty_like(k), at::empty_like(v)};
+  float* acc[4] = {nullptr, nullptr, nullptr, nullptr};
+  for (int i = 0; i < (pk2 ? 4 : 2); ++i) {
+    out.push_back(at::empty({d.B, d.H, i < 2 ? d.n1 : d.n2, q.size(3)}, q.options().dtype(at::kFloat)));
+    acc[i] = (float*) out.back().data_ptr();
   }
+  Core c = make_core(q, k, v, pkc, pvc, pk2c, pv2c, ic, pic, o, lc);
+  run_bwd(c, d, desc(d_o), desc(out[0]), desc(out[1]), desc(out[2]), (int) topk, (int) topk_p, w1, w2, kvw1, kvw2, fold,
+          q.scalar_type() == at::kBFloat16, acc, q);
   return out;
 }
 
