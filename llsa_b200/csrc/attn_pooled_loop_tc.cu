@@ -13,7 +13,7 @@
 //           the A operand of O += P.V_c; row sums on the side.
 // With a `redo` byte per query row from the caller the first pass is dropped: the pooled part only ever meets the fine
 // part through their log-sum-exp, so the fine part's log-sum-exp (already known per row) serves as the reference of the
-// exponentials, P = exp2(S' - lse_fine) (up to the next quarter above a power of two: kRefShift).  Anything below 2^-126 of the fine part's weight is irrelevant, and bf16 / fp32
+// exponentials, P = exp2(S' - lse_fine) (REM: moved up to a quarter above a power of two, kRefShift).  Anything below 2^-126 of the fine part's weight is irrelevant, and bf16 / fp32
 // hold anything up to 2^127 times it; a row whose pooled keys outweigh its fine keys by more than that (its row sum
 // passes 1e30, or is NaN) is left untouched and marked in `redo`; a CTA that has marked a row of its tiles goes over them again
 // with two passes and writes exactly the marked rows.  (A second launch that looked for marks cost every call 1 to 2 us.)
@@ -53,10 +53,10 @@ constexpr int kThreads = 512;
 constexpr int kBufs = 3;
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr uint32_t kColO = 384;
-// One pass: where in its binade a probability of a logit of 0 lands.  bf16 is finest just below a power of two, which is where a row's
+// One pass over a list that one kernel used to take with running maxima (REM): where in its binade a probability of a logit of 0 lands.  bf16 is finest just below a power of two, which is where a row's
 // maximum as reference puts the largest ones; a reference at no particular place costs up to 12 % of o's error where the keys weigh about alike
 // (against fp64, N(0,1) inputs, two levels, N = 40960, top-16: 2.33e-3; 2.33e-3, 2.11e-3, 2.10e-3, 2.15e-3, 2.22e-3 with the reference at
-// 0, 1/8, 1/4, 3/8, 1/2 above a power of two; 2.09e-3 with two passes).  The weights 16 and 256 are powers of two themselves.
+// 0, 1/8, 1/4, 3/8, 1/2 above a power of two; 2.09e-3 with two passes, 2.07e-3 in one kernel).  The weights 16 and 256 are powers of two.
 constexpr float kRefShift = 0.25f;
 
 struct LoopMaps {
@@ -258,8 +258,8 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       float lse_next = n_pass == 1 && n_my > 0 ? lse_of(0) : 0.f;
       bool ok = true;
       for (int i = 0; ok && i < n_my; ++i) {
-        // one pass: the fine part's log-sum-exp, moved to a fixed place between two powers of two, is the reference of the exponentials
-        float mx = n_pass == 1 ? ceilf(lse_next * kLog2eF) + kRefShift : -INFINITY;
+        // one pass: the fine part's log-sum-exp is the reference of the exponentials
+        float mx = n_pass == 1 ? (REM ? ceilf(lse_next * kLog2eF) + kRefShift : lse_next * kLog2eF) : -INFINITY;
         F2 sum[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};      // four running sums: a chain of adds per element is a third of a job
         if (n_pass == 1 && i + 1 < n_my) lse_next = lse_of(i + 1);
         bool exchanged = n_pass == 1;
