@@ -501,8 +501,9 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 //     window of four ranges, every range on a warp at once; a warp parks the tile of a bucket it shares with EARLIER warps in its
 //     shared-memory slot, the tile it shares with later ones stays in its accumulators until the CTA has synchronised.
 //     Pieces of buckets that straddle windows go to the `partial` scratch and attn_dkv_finish_kernel adds them in window order.
-// What bounds it: issue slots (0.42 instructions per scheduler and cycle with three warps on each; some 290 instructions per entry), then
-// the raggedness of the last ranges.  With P and dS handed over by the dQ stage instead of recomputed this kernel issued half as much,
+// What bounds it: latency.  0.42 instructions per scheduler and cycle: 58 % of the issue slots stay empty with three warps on a scheduler, each on
+// one serial chain (wait, S and dP, exponentials, the two products: some 290 instructions per entry); then the raggedness of the last ranges.
+// 168 registers in the persistent form, 4 bytes of them spilled.  With P and dS handed over by the dQ stage instead of recomputed this kernel issued half as much,
 // but 1 KB per entry went out to HBM and came back: at 8 x 6 slices of 16384 tokens, top 8, dQ stage 205 -> 158 us and this one 192 -> 255
 // on random inputs, 207 -> 164 and 284 -> 255 on correlated ones; at 6 of 262144 421 -> 315 and 563 -> 460 (the first figures of the
 // correlated pairs with eight warps per SM in groups of four that waited for the longest of their ranges: 322 and 645 on random inputs).

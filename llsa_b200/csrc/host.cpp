@@ -312,9 +312,11 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
 
   const at::cuda::CUDAStream cur = at::cuda::getCurrentCUDAStream(like.device().index());
   const bool hooked = g_has_hook.load(std::memory_order_relaxed);      // a stage hook times every stage on ONE stream
-  // Up to some thousand query blocks the host is the pace of an eager call (110 us of host work; B=1 H=2 N=1024 fp32 forward + backward
-  // 108 us a pass with the side stream, 100 without): two events, four stream operations and a second launch call are worth more there than
-  // the 5 us of the transpose.  In a graph the host's time does not count.
+  // Up to some thousand query blocks the host is the pace of an eager call: two events, four stream operations and a second launch call are
+  // worth more there than the 5 us of the transpose.  Forward + backward, us a pass with the side stream / on one stream: one level, N = 1024,
+  // 128 query blocks fp32 108 / 97, bf16 117 / 108, 1,024 blocks 118 / 108; two levels, 512 blocks (N = 4096) 119 / 113, 1,024 blocks
+  // (N = 16384) 114 / 111; from 2,048 blocks on the GPU is the pace and the two are equal (119 / 119 at one level, 150 / 150 at 4,096 blocks of
+  // two).  In a graph the host's time does not count.
   auto capturing = [&] {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     C10_CUDA_CHECK(cudaStreamIsCapturing(cur, &s));

@@ -100,9 +100,6 @@ __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.w
 // makes 128-bit ld.shared of row fragments and ldmatrix bank-conflict free.
 constexpr int kRingTileElems = 16 * 64;          // one tile, in bf16 elements
 
-
-
-
 // Shared-memory accesses as [32-bit shared address + compile-time offset]: the per-lane part of every address is computed
 // once per kernel, the stage / tile / row part is an immediate, and the entry loop spends no integer instruction on them.
 template <int IMM>

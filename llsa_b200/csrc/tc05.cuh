@@ -95,7 +95,6 @@ __device__ __forceinline__ void abort_drain() {
   for (int i = 0; i < 64; ++i) __nanosleep(1000);
 }
 
-
 // ---- fences ----
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
