@@ -3,9 +3,9 @@
 single-shot pooled backward with its two MMA-issuing threads (attn_pooled_bwd_tc.cu).
 
 Test infrastructure: nothing in the package imports it.  Every role of a CTA
-(TMA producer, the threads that issue MMAs, the eight softmax warps) is a Python
-generator that waits on barriers, spends random time and arrives, exactly in the
-order the kernel's role does.  The model keeps the hardware's semantics where
+(the two TMA producers, the warps that issue MMAs, the eight softmax warps, the
+four epilogue warps) is a Python generator that waits on barriers, spends random
+time and arrives, exactly in the order the kernel's role does.  The model keeps the hardware's semantics where
 they matter for correctness:
 
 * a barrier has an arrival count and a phase; a wait names a PARITY and passes
@@ -45,7 +45,7 @@ class Sim:
     def __init__(self, seed):
         self.t, self.queue, self.serial = 0, [], 0
         self.rng = random.Random(seed)
-        self.waiting = []                 # (role, barrier, parity)
+        self.waiting = []                 # (role, [(barrier, parity)])
         self.roles = {}
         self.pipe_free = 0                # the tensor pipe executes in issue order
         self.last_mma_done = {}           # per issuing thread
@@ -69,20 +69,20 @@ class Sim:
             return
         if op[0] == "delay":
             self.at(self.t + op[1], lambda: self.step(name))
-        else:                             # ("wait", barrier, parity)
-            _, bar, par = op
-            if bar.parity() != par:
+        else:                             # ("wait", barrier, parity[, barrier, parity ...]): all of them in one look
+            conds = list(zip(op[1::2], op[2::2]))
+            if all(b.parity() != par for b, par in conds):
                 self.at(self.t + self.rng.randint(20, 120), lambda: self.step(name))
             else:
-                self.waiting.append((name, bar, par))
+                self.waiting.append((name, conds))
 
     def wake(self, bar):
         still = []
-        for name, b, par in self.waiting:
-            if b is bar and b.parity() != par:
+        for name, conds in self.waiting:
+            if any(b is bar for b, _ in conds) and all(b.parity() != par for b, par in conds):
                 self.at(self.t + self.rng.randint(20, 150), (lambda nm: (lambda: self.step(nm)))(name))
             else:
-                still.append((name, b, par))
+                still.append((name, conds))
         self.waiting = still
 
     def run(self):
@@ -112,344 +112,6 @@ class Sim:
         return self.rng.randint(a, b)
 
 
-def key_major_kernel(seed, units, score_threads=1, score_barriers=3, stages=8, buffers=3):
-    """attn_dkv_pooled_loop_tc_kernel.  `units`: job counts of the (head, chunk) units of one CTA's piece.
-    score_threads: threads that issue S^T / dP^T (1 = the kernel; 2 = even and odd jobs on two threads).
-    score_barriers: sdp_ready / buf_free barriers (3 = one per buffer, the kernel; 6 = one per job number mod 6)."""
-    sim = Sim(seed)
-    nb = score_barriers
-    kv_full, kv_empty = Barrier("kv_full", 1), Barrier("kv_empty", score_threads)
-    q_full = [Barrier("q_full%d" % i, 1) for i in range(stages)]
-    q_empty = [Barrier("q_empty%d" % i, 1) for i in range(stages)]
-    sdp = [Barrier("sdp_ready%d" % i, 1) for i in range(nb)]
-    pds = [Barrier("pds_ready%d" % i, 4) for i in range(buffers)]
-    free = [Barrier("buf_free%d" % i, 1) for i in range(nb)]
-    acc_ready, acc_free = Barrier("acc_ready", 1), Barrier("acc_free", 8)
-    owner = [None] * buffers              # None: free; ("s", job): scores; ("p", job): probabilities
-
-    def producer():
-        job = 0
-        for i, n in enumerate(units):
-            yield ("wait", kv_empty, (i & 1) ^ 1)
-            sim.tma(kv_full)
-            for _ in range(n):
-                st = job % stages
-                yield ("wait", q_empty[st], ((job // stages) & 1) ^ 1)
-                yield ("delay", sim.r(20, 80))
-                sim.tma(q_full[st])
-                job += 1
-
-    def score_issuer(mine):
-        job, first = mine, 0
-        for i, n in enumerate(units):
-            yield ("wait", kv_full, i & 1)
-            while job < first + n:
-                st, buf = job % stages, job % buffers
-                if job >= buffers:
-                    prev = job - buffers
-                    yield ("wait", free[prev % nb], (prev // nb) & 1)
-                yield ("wait", q_full[st], (job // stages) & 1)
-                if sim.rng.random() < 0.15:
-                    yield ("delay", sim.r(500, 4000))          # one thread falls behind the other
-                assert owner[buf] is None, ("scores written over a live buffer", buf, owner[buf], job)
-                start, done = sim.mma(("score", mine), 384)
-                sim.at(done, (lambda b=buf, j=job: owner.__setitem__(b, ("s", j))))
-                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
-                sim.commit(("score", mine), sdp[job % nb])
-                yield ("delay", sim.r(30, 80))
-                job += score_threads
-            first += n
-            sim.commit(("score", mine), kv_empty)
-            yield ("delay", sim.r(30, 80))
-
-    def out_issuer():
-        job = 0
-        for i, n in enumerate(units):
-            for j in range(n):
-                st, buf = job % stages, job % buffers
-                yield ("wait", pds[buf], (job // buffers) & 1)
-                if j == 0 and i > 0:
-                    yield ("wait", acc_free, (i - 1) & 1)
-                assert owner[buf] == ("p", job), ("dV / dK read", buf, owner[buf], job)
-                start, done = sim.mma("out", 384)
-                sim.at(done, (lambda b=buf: owner.__setitem__(b, None)))
-                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
-                sim.commit("out", q_empty[st])
-                sim.commit("out", free[job % nb])
-                yield ("delay", sim.r(60, 160))
-                job += 1
-            sim.commit("out", acc_ready)
-            yield ("delay", sim.r(30, 80))
-
-    def softmax(group, warp):
-        job, first = group, 0
-        for i, n in enumerate(units):
-            while job < first + n:
-                buf = job % buffers
-                yield ("wait", sdp[job % nb], (job // nb) & 1)
-                assert owner[buf] is not None and owner[buf][1] == job, ("softmax read", buf, owner[buf], job)
-                yield ("delay", sim.r(500, 1200))
-                if warp == 0:
-                    owner[buf] = ("p", job)
-                pds[buf].arrive(sim)
-                job += 2
-            first += n
-            yield ("wait", acc_ready, i & 1)
-            yield ("delay", sim.r(200, 600))
-            acc_free.arrive(sim)
-
-    sim.spawn("producer", producer())
-    for t in range(score_threads):
-        sim.spawn("score%d" % t, score_issuer(t))
-    sim.spawn("out", out_issuer())
-    for g in range(2):
-        for w in range(4):
-            sim.spawn("softmax%d%d" % (g, w), softmax(g, w))
-    return sim.run()
-
-
-def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=3, stages=8, buffers=3):
-    """attn_dq_pooled_loop_tc_kernel: `tiles` query tiles of `jobs` key chunks (even); Q / dO in two stages, K and V
-    chunks in rings, S / dP into three buffers, dQ accumulated per tile."""
-    sim = Sim(seed)
-    nb = score_barriers
-    q_full = [Barrier("q_full%d" % i, 1) for i in range(2)]
-    q_empty = [Barrier("q_empty%d" % i, score_threads) for i in range(2)]
-    k_full = [Barrier("k_full%d" % i, 1) for i in range(stages)]
-    k_empty = [Barrier("k_empty%d" % i, 1) for i in range(stages)]
-    v_full = [Barrier("v_full%d" % i, 1) for i in range(stages)]
-    v_empty = [Barrier("v_empty%d" % i, 1) for i in range(stages)]
-    sdp = [Barrier("sdp_ready%d" % i, 1) for i in range(nb)]
-    ds = [Barrier("ds_ready%d" % i, 4) for i in range(buffers)]
-    free = [Barrier("buf_free%d" % i, 1) for i in range(nb)]
-    dq_ready, dq_free = Barrier("dq_ready", 1), Barrier("dq_free", 8)
-    owner = [None] * buffers
-    held = [None] * stages                # chunk number a K ring stage holds
-
-    def producer():
-        job = 0
-        for i in range(tiles):
-            yield ("wait", q_empty[i & 1], ((i >> 1) & 1) ^ 1)
-            sim.tma(q_full[i & 1])
-            for _ in range(jobs):
-                st, par = job % stages, ((job // stages) & 1) ^ 1
-                yield ("wait", k_empty[st], par)
-                assert held[st] is None, ("keys loaded over a live stage", st, held[st], job)
-                sim.tma(k_full[st], (lambda s=st, j=job: held.__setitem__(s, j)))
-                yield ("wait", v_empty[st], par)
-                sim.tma(v_full[st])
-                job += 1
-
-    def score_issuer(mine):
-        job = mine
-        for i in range(tiles):
-            yield ("wait", q_full[i & 1], (i >> 1) & 1)
-            for _ in range(mine, jobs, score_threads):
-                st, par, buf = job % stages, (job // stages) & 1, job % buffers
-                if job >= buffers:
-                    prev = job - buffers
-                    yield ("wait", free[prev % nb], (prev // nb) & 1)
-                yield ("wait", k_full[st], par)
-                yield ("wait", v_full[st], par)
-                if sim.rng.random() < 0.15:
-                    yield ("delay", sim.r(500, 4000))
-                assert owner[buf] is None, ("scores written over a live buffer", buf, owner[buf], job)
-                assert held[st] == job, ("S read the wrong keys", st, held[st], job)
-                start, done = sim.mma(("score", mine), 384)
-                sim.at(done, (lambda b=buf, j=job: owner.__setitem__(b, ("s", j))))
-                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
-                sim.commit(("score", mine), sdp[job % nb])
-                sim.commit(("score", mine), v_empty[st])
-                yield ("delay", sim.r(30, 80))
-                job += score_threads
-            sim.commit(("score", mine), q_empty[i & 1])
-            yield ("delay", sim.r(30, 80))
-
-    def dq_issuer():
-        job = 0
-        for i in range(tiles):
-            for j in range(jobs):
-                st, buf = job % stages, job % buffers
-                yield ("wait", ds[buf], (job // buffers) & 1)
-                if j == 0 and i > 0:
-                    yield ("wait", dq_free, (i - 1) & 1)
-                assert owner[buf] == ("p", job), ("dQ read", buf, owner[buf], job)
-                assert held[st] == job, ("dQ read the wrong keys", st, held[st], job)
-                start, done = sim.mma("dq", 192)
-
-                def release(b=buf, s=st):
-                    owner[b] = None
-                    held[s] = None
-                sim.at(done, release)
-                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
-                sim.commit("dq", k_empty[st])
-                sim.commit("dq", free[job % nb])
-                yield ("delay", sim.r(60, 160))
-                job += 1
-            sim.commit("dq", dq_ready)
-            yield ("delay", sim.r(30, 80))
-
-    def softmax(group, warp):
-        job = group
-        for i in range(tiles):
-            for _ in range(group, jobs, 2):
-                buf = job % buffers
-                yield ("wait", sdp[job % nb], (job // nb) & 1)
-                assert owner[buf] is not None and owner[buf][1] == job, ("softmax read", buf, owner[buf], job)
-                yield ("delay", sim.r(400, 1000))
-                if warp == 0:
-                    owner[buf] = ("p", job)
-                ds[buf].arrive(sim)
-                job += 2
-            yield ("wait", dq_ready, i & 1)
-            yield ("delay", sim.r(200, 600))
-            dq_free.arrive(sim)
-
-    sim.spawn("producer", producer())
-    for t in range(score_threads):
-        sim.spawn("score%d" % t, score_issuer(t))
-    sim.spawn("dq", dq_issuer())
-    for g in range(2):
-        for w in range(4):
-            sim.spawn("softmax%d%d" % (g, w), softmax(g, w))
-    return sim.run()
-
-
-def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=3):
-    """attn_fwd_pooled_loop_tc_kernel: `tiles` query tiles of `chunks` key chunks; one pass (jobs = chunks, every job
-    feeds P.V) or two (jobs = 2 * chunks: row maxima first, then the exponentials; the two groups exchange their maxima
-    before their first second-pass job).  One thread issues S, one issues P.V and hands every job's buffer back; the two
-    softmax groups take the jobs of one parity of the CTA-wide job number each (with an odd job count the parity of a
-    tile's first job alternates) and exchange their row sums at the end of a tile."""
-    sim = Sim(seed)
-    jobs, first_p2 = passes * chunks, (passes - 1) * chunks
-    q_full = [Barrier("q_full%d" % i, 1) for i in range(2)]
-    q_empty = [Barrier("q_empty%d" % i, 1) for i in range(2)]
-    k_full = [Barrier("k_full%d" % i, 1) for i in range(k_stages)]
-    k_empty = [Barrier("k_empty%d" % i, 1) for i in range(k_stages)]
-    v_full = [Barrier("v_full%d" % i, 1) for i in range(v_stages)]
-    v_empty = [Barrier("v_empty%d" % i, 1) for i in range(v_stages)]
-    s_ready = [Barrier("s_ready%d" % i, 1) for i in range(buffers)]
-    wg_done = [Barrier("wg_done%d" % i, 4) for i in range(buffers)]
-    free = [Barrier("buf_free%d" % i, 1) for i in range(buffers)]
-    o_ready, o_free, xchg = Barrier("o_ready", 1), Barrier("o_free", 8), Barrier("xchg", 8)
-    owner = [None] * buffers
-    v_held = [None] * v_stages
-    o_busy = [False]                      # the O accumulator holds a finished tile that has not been read yet
-
-    def producer():
-        kjob = vjob = 0
-        for i in range(tiles):
-            yield ("wait", q_empty[i & 1], ((i >> 1) & 1) ^ 1)
-            sim.tma(q_full[i & 1])
-            for j in range(jobs):
-                ks = kjob % k_stages
-                yield ("wait", k_empty[ks], ((kjob // k_stages) & 1) ^ 1)
-                sim.tma(k_full[ks])
-                kjob += 1
-                if j >= first_p2:
-                    vs = vjob % v_stages
-                    yield ("wait", v_empty[vs], ((vjob // v_stages) & 1) ^ 1)
-                    assert v_held[vs] is None, ("values loaded over a live stage", vs, v_held[vs], vjob)
-                    sim.tma(v_full[vs], (lambda s=vs, j=vjob: v_held.__setitem__(s, j)))
-                    vjob += 1
-
-    def s_issuer():
-        n = 0
-        for i in range(tiles):
-            yield ("wait", q_full[i & 1], (i >> 1) & 1)
-            for _ in range(jobs):
-                buf, ks = n % buffers, n % k_stages
-                if n >= buffers:
-                    yield ("wait", free[buf], ((n // buffers) & 1) ^ 1)
-                yield ("wait", k_full[ks], (n // k_stages) & 1)
-                assert owner[buf] is None, ("scores written over a live buffer", buf, owner[buf], n)
-                start, done = sim.mma("s", 256)
-                sim.at(done, (lambda b=buf, j=n: owner.__setitem__(b, ("s", j))))
-                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
-                sim.commit("s", s_ready[buf])
-                sim.commit("s", k_empty[ks])
-                yield ("delay", sim.r(30, 80))
-                n += 1
-            sim.commit("s", q_empty[i & 1])
-            yield ("delay", sim.r(30, 80))
-
-    def pv_issuer():
-        n = vjob = 0
-        for i in range(tiles):
-            for j in range(jobs):
-                buf = n % buffers
-                yield ("wait", wg_done[buf], (n // buffers) & 1)
-                if j >= first_p2:
-                    vs = vjob % v_stages
-                    yield ("wait", v_full[vs], (vjob // v_stages) & 1)
-                    if j == first_p2 and i > 0:
-                        yield ("wait", o_free, (i - 1) & 1)
-                    if j == first_p2:
-                        assert not o_busy[0], ("O overwritten before it was read", i)
-                    assert owner[buf] == ("p", n), ("P.V read", buf, owner[buf], n)
-                    assert v_held[vs] == vjob, ("P.V read the wrong values", vs, v_held[vs], vjob)
-                    start, done = sim.mma("pv", 384)
-
-                    def release(b=buf, s=vs):
-                        owner[b] = None
-                        v_held[s] = None
-                    sim.at(done, release)
-                    yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
-                    sim.commit("pv", v_empty[vs])
-                    vjob += 1
-                else:
-                    assert owner[buf] == ("m", n), ("first-pass buffer handed back early", buf, owner[buf], n)
-                    owner[buf] = None
-                sim.commit("pv", free[buf])
-                yield ("delay", sim.r(30, 80))
-                n += 1
-            last = max(sim.last_mma_done.get("pv", 0), sim.t)
-            sim.at(last, (lambda: o_busy.__setitem__(0, True)))
-            sim.commit("pv", o_ready)
-            yield ("delay", sim.r(30, 80))
-
-    def softmax(group, warp):
-        n_x = 0
-        state = {"n": group}              # this group's next job, numbered over the CTA
-
-        def exchange():
-            nonlocal n_x
-            xchg.arrive(sim)
-            yield ("wait", xchg, n_x & 1)
-            n_x += 1
-
-        for i in range(tiles):
-            j = (group - i * jobs) & 1
-            assert i * jobs + j == state["n"], ("job numbering", i, j, state["n"])
-            while j < jobs:
-                n, buf = state["n"], state["n"] % buffers
-                if passes == 2 and j >= first_p2 and j - 2 < first_p2:
-                    yield from exchange()                  # row maxima of the two groups
-                yield ("wait", s_ready[buf], (n // buffers) & 1)
-                assert owner[buf] is not None and owner[buf][1] == n, ("softmax read", buf, owner[buf], n)
-                yield ("delay", sim.r(400, 1400))
-                if warp == 0:
-                    owner[buf] = ("p" if j >= first_p2 else "m", n)
-                wg_done[buf].arrive(sim)
-                state["n"] += 2
-                j += 2
-            yield from exchange()                          # row sums
-            yield ("wait", o_ready, i & 1)
-            yield ("delay", sim.r(200, 600))
-            if group == 0 and warp == 0:
-                o_busy[0] = False
-            o_free.arrive(sim)
-
-    sim.spawn("producer", producer())
-    sim.spawn("s", s_issuer())
-    sim.spawn("pv", pv_issuer())
-    for g in range(2):
-        for w in range(4):
-            sim.spawn("softmax%d%d" % (g, w), softmax(g, w))
-    return sim.run()
-
-
 class Resource:
     """A buffer with one content tag; reads must see the expected tag, and an overwrite must come after the last read
     (an MMA reads until it completes) has ended."""
@@ -467,6 +129,406 @@ class Resource:
         else:
             self.tag = ("in flight", tag)
             sim.at(at, (lambda: setattr(self, "tag", tag)))
+
+
+def _bars(name, n, count):
+    return [Barrier("%s%d" % (name, i), count) for i in range(n)]
+
+
+def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8, buffers=3, accs=1, full_count=2):
+    """attn_dkv_pooled_loop_tc_kernel.  `units`: job counts of the units of one CTA's piece: (head, chunk) units in the dense form
+    (three S^T / dP^T buffers, one pair of accumulators), units of four jobs and fewer in the gathered one (buffers=2, accs=2).
+    score_threads: threads that issue S^T / dP^T (1 = the kernel; 2 = even and odd jobs on two threads).
+    score_barriers: sdp_ready / buf_free barriers (None = one per buffer, the kernel; 6 = one per job number mod 6).
+    full_count: producers a query stage waits for (2 = the kernel: Q, and dO with lse and delta; 1 breaks the protocol on purpose)."""
+    sim = Sim(seed)
+    nb = score_barriers or buffers
+    kv_full, kv_empty = _bars("kv_full", 2, 1), _bars("kv_empty", 2, score_threads)
+    q_full, q_empty = _bars("q_full", stages, full_count), _bars("q_empty", stages, 1)
+    sdp, pds, free = _bars("sdp_ready", nb, 1), _bars("pds_ready", buffers, 4), _bars("buf_free", nb, 1)
+    acc_ready, acc_free = _bars("acc_ready", accs, 1), _bars("acc_free", accs, 4)
+    owner = [None] * buffers              # None: free; ("s", job): scores; ("p", job): probabilities
+    keys = [Resource("key stage %d" % i) for i in range(2)]
+    tiles = {n: [Resource("%s stage %d" % (n, i)) for i in range(stages)] for n in ("Q", "dO")}
+    acc = [Resource("accumulator %d" % i) for i in range(accs)]
+
+    def producer(which):
+        job = 0
+        for i, n in enumerate(units):
+            if which == "Q":              # this producer also loads the unit's keys and values
+                yield ("wait", kv_empty[i & 1], ((i >> 1) & 1) ^ 1)
+                land = sim.t + sim.r(500, 1500)
+                keys[i & 1].write(sim, i, at=land)
+                sim.at(land, (lambda b=kv_full[i & 1]: b.arrive(sim)))
+            for _ in range(n):
+                st = job % stages
+                yield ("wait", q_empty[st], ((job // stages) & 1) ^ 1)
+                yield ("delay", sim.r(20, 80))
+                land = sim.t + sim.r(500, 1500)
+                tiles[which][st].write(sim, job, at=land)
+                if which == "Q" or full_count == 2:
+                    sim.at(land, (lambda b=q_full[st]: b.arrive(sim)))
+                job += 1
+
+    def score_issuer(mine):
+        job, first = mine, 0
+        for i, n in enumerate(units):
+            yield ("wait", kv_full[i & 1], (i >> 1) & 1)
+            while job < first + n:
+                st, buf = job % stages, job % buffers
+                wait = ["wait", q_full[st], (job // stages) & 1]
+                if job >= buffers:
+                    prev = job - buffers
+                    wait += [free[prev % nb], (prev // nb) & 1]
+                yield tuple(wait)
+                if sim.rng.random() < 0.15:
+                    yield ("delay", sim.r(500, 4000))          # one thread falls behind the other
+                assert owner[buf] is None, ("scores written over a live buffer", buf, owner[buf], job)
+                start, done = sim.mma(("score", mine), 384)
+                keys[i & 1].read(sim, i, done)
+                for t in tiles.values():
+                    t[st].read(sim, job, done)
+                sim.at(done, (lambda b=buf, j=job: owner.__setitem__(b, ("s", j))))
+                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+                sim.commit(("score", mine), sdp[job % nb])
+                yield ("delay", sim.r(30, 80))
+                job += score_threads
+            first += n
+            sim.commit(("score", mine), kv_empty[i & 1])
+            yield ("delay", sim.r(30, 80))
+
+    def out_issuer():
+        job = 0
+        for i, n in enumerate(units):
+            for j in range(n):
+                st, buf = job % stages, job % buffers
+                wait = ["wait", pds[buf], (job // buffers) & 1]
+                if j == 0 and i >= accs:
+                    wait += [acc_free[i % accs], (i // accs - 1) & 1]
+                yield tuple(wait)
+                assert owner[buf] == ("p", job), ("dV / dK read", buf, owner[buf], job)
+                start, done = sim.mma("out", 384)
+                for t in tiles.values():
+                    t[st].read(sim, job, done)
+                if j == 0:
+                    acc[i % accs].write(sim, i)
+                sim.at(done, (lambda b=buf: owner.__setitem__(b, None)))
+                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+                sim.commit("out", q_empty[st])
+                sim.commit("out", free[job % nb])
+                yield ("delay", sim.r(60, 160))
+                job += 1
+            sim.commit("out", acc_ready[i % accs])
+            yield ("delay", sim.r(30, 80))
+
+    def softmax(group, warp):
+        for job in range(group, sum(units), 2):
+            buf = job % buffers
+            yield ("wait", sdp[job % nb], (job // nb) & 1)
+            assert owner[buf] is not None and owner[buf][1] == job, ("softmax read", buf, owner[buf], job)
+            yield ("delay", sim.r(500, 1200))
+            if warp == 0:
+                owner[buf] = ("p", job)
+            pds[buf].arrive(sim)
+
+    def epilogue(warp):
+        for i in range(len(units)):
+            a = i % accs
+            yield ("wait", acc_ready[a], (i // accs) & 1)
+            acc[a].read(sim, i)
+            yield ("delay", sim.r(200, 1500))
+            acc[a].read(sim, i)
+            acc_free[a].arrive(sim)
+
+    for which in ("Q", "dO"):
+        sim.spawn("producer " + which, producer(which))
+    for t in range(score_threads):
+        sim.spawn("score%d" % t, score_issuer(t))
+    sim.spawn("out", out_issuer())
+    for w in range(4):
+        for g in range(2):
+            sim.spawn("softmax%d%d" % (g, w), softmax(g, w))
+        sim.spawn("epilogue%d" % w, epilogue(w))
+    return sim.run()
+
+
+def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=3, stages=8, buffers=3, free_count=4):
+    """attn_dq_pooled_loop_tc_kernel: `tiles` query tiles of `jobs` key chunks; Q / dO in two stages, K and V chunks (two
+    producers) in one ring of pairs, S / dP into three buffers, dQ of a tile into one of two accumulators, read by epilogue warps.
+    free_count: epilogue warps an accumulator waits for (4 = the kernel; 1 breaks the protocol on purpose)."""
+    sim = Sim(seed)
+    nb = score_barriers
+    q_full, q_empty = _bars("q_full", 2, 1), _bars("q_empty", 2, score_threads)
+    kv_full, kv_empty = _bars("kv_full", stages, 2), _bars("kv_empty", stages, 1)
+    sdp, ds, free = _bars("sdp_ready", nb, 1), _bars("ds_ready", buffers, 4), _bars("buf_free", nb, 1)
+    dq_ready, dq_free = _bars("dq_ready", 2, 1), _bars("dq_free", 2, free_count)
+    owner = [None] * buffers
+    ring = {n: [Resource("%s stage %d" % (n, i)) for i in range(stages)] for n in ("K", "V")}
+    q_tile = [Resource("Q / dO stage %d" % i) for i in range(2)]
+    acc = [Resource("dQ accumulator %d" % i) for i in range(2)]
+
+    def producer(which):
+        job = 0
+        for i in range(tiles):
+            if which == "K":              # this producer also loads Q and dO
+                yield ("wait", q_empty[i & 1], ((i >> 1) & 1) ^ 1)
+                land = sim.t + sim.r(500, 1500)
+                q_tile[i & 1].write(sim, i, at=land)
+                sim.at(land, (lambda b=q_full[i & 1]: b.arrive(sim)))
+            for _ in range(jobs):
+                st = job % stages
+                yield ("wait", kv_empty[st], ((job // stages) & 1) ^ 1)
+                land = sim.t + sim.r(500, 1500)
+                ring[which][st].write(sim, job, at=land)
+                sim.at(land, (lambda b=kv_full[st]: b.arrive(sim)))
+                job += 1
+
+    def score_issuer(mine):
+        job = mine
+        for i in range(tiles):
+            yield ("wait", q_full[i & 1], (i >> 1) & 1)
+            while job < (i + 1) * jobs:
+                st, buf = job % stages, job % buffers
+                wait = ["wait", kv_full[st], (job // stages) & 1]
+                if job >= buffers:
+                    prev = job - buffers
+                    wait += [free[prev % nb], (prev // nb) & 1]
+                yield tuple(wait)
+                if sim.rng.random() < 0.15:
+                    yield ("delay", sim.r(500, 4000))
+                assert owner[buf] is None, ("scores written over a live buffer", buf, owner[buf], job)
+                start, done = sim.mma(("score", mine), 384)
+                q_tile[i & 1].read(sim, i, done)
+                for r in ring.values():
+                    r[st].read(sim, job, done)
+                sim.at(done, (lambda b=buf, j=job: owner.__setitem__(b, ("s", j))))
+                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+                sim.commit(("score", mine), sdp[job % nb])
+                yield ("delay", sim.r(30, 80))
+                job += score_threads
+            sim.commit(("score", mine), q_empty[i & 1])
+            yield ("delay", sim.r(30, 80))
+
+    def dq_issuer():
+        job = 0
+        for i in range(tiles):
+            for j in range(jobs):
+                st, buf = job % stages, job % buffers
+                wait = ["wait", ds[buf], (job // buffers) & 1]
+                if j == 0 and i > 1:
+                    wait += [dq_free[i & 1], ((i - 2) >> 1) & 1]
+                yield tuple(wait)
+                assert owner[buf] == ("p", job), ("dQ read", buf, owner[buf], job)
+                start, done = sim.mma("dq", 192)
+                ring["K"][st].read(sim, job, done)
+                if j == 0:
+                    acc[i & 1].write(sim, i)
+                sim.at(done, (lambda b=buf: owner.__setitem__(b, None)))
+                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+                sim.commit("dq", kv_empty[st])
+                sim.commit("dq", free[job % nb])
+                yield ("delay", sim.r(60, 160))
+                job += 1
+            sim.commit("dq", dq_ready[i & 1])
+            yield ("delay", sim.r(30, 80))
+
+    def softmax(group, warp):
+        for job in range(group, tiles * jobs, 2):
+            buf = job % buffers
+            yield ("wait", sdp[job % nb], (job // nb) & 1)
+            assert owner[buf] is not None and owner[buf][1] == job, ("softmax read", buf, owner[buf], job)
+            yield ("delay", sim.r(400, 1000))
+            if warp == 0:
+                owner[buf] = ("p", job)
+            ds[buf].arrive(sim)
+
+    def epilogue(warp):
+        for i in range(tiles):
+            yield ("wait", dq_ready[i & 1], (i >> 1) & 1)
+            acc[i & 1].read(sim, i)
+            yield ("delay", sim.r(200, 3000))
+            acc[i & 1].read(sim, i)
+            if warp < free_count:
+                dq_free[i & 1].arrive(sim)
+
+    for which in ("K", "V"):
+        sim.spawn("producer " + which, producer(which))
+    for t in range(score_threads):
+        sim.spawn("score%d" % t, score_issuer(t))
+    sim.spawn("dq", dq_issuer())
+    for w in range(4):
+        for g in range(2):
+            sim.spawn("softmax%d%d" % (g, w), softmax(g, w))
+        sim.spawn("epilogue%d" % w, epilogue(w))
+    return sim.run()
+
+
+def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=3, second_round=False, softmax_waits_for_sums=True):
+    """attn_fwd_pooled_loop_tc_kernel: `tiles` query tiles of `chunks` key chunks; one pass (jobs = chunks, every job
+    feeds P.V) or two (jobs = 2 * chunks: row maxima first, then the exponentials; the two groups exchange their maxima
+    once per tile, a group without a second-pass job at its end).  Producers of keys (with Q) and of values; one warp issues S, one P.V
+    and hands every job's buffer back; the two softmax groups take the jobs of one parity of the CTA-wide job number each (with an
+    odd job count the parity of a tile's first job alternates) and leave their row sums to four epilogue warps, as O in one of
+    two accumulators.
+    second_round: the CTA has marked a row and goes over its tiles again with two passes, on barriers of its own, behind a CTA-wide
+    synchronisation.  softmax_waits_for_sums=False breaks the protocol on purpose (row sums overwritten before they are read)."""
+    sim = Sim(seed)
+    owner = [None] * buffers
+    k_ring = [Resource("K stage %d" % i) for i in range(k_stages)]
+    v_ring = [Resource("V stage %d" % i) for i in range(v_stages)]
+    q_tile = [Resource("Q stage %d" % i) for i in range(2)]
+    acc = [Resource("O accumulator %d" % i) for i in range(2)]
+    sums = [[Resource("row sums %d of group %d" % (i, g)) for g in range(2)] for i in range(2)]
+    maxima = [[Resource("row maxima %d of group %d" % (i, g)) for g in range(2)] for i in range(2)]
+    n_roles = 2 + 2 + 8 + 4
+    sync = Barrier("__syncthreads", n_roles)
+
+    class Round:
+        def __init__(self, number, passes):
+            self.number, self.passes = number, passes
+            self.jobs, self.first_p2 = passes * chunks, (passes - 1) * chunks
+            self.q_full, self.q_empty = _bars("q_full", 2, 1), _bars("q_empty", 2, 1)
+            self.k_full, self.k_empty = _bars("k_full", k_stages, 1), _bars("k_empty", k_stages, 1)
+            self.v_full, self.v_empty = _bars("v_full", v_stages, 1), _bars("v_empty", v_stages, 1)
+            self.s_ready, self.wg_done, self.free = _bars("s_ready", buffers, 1), _bars("wg_done", buffers, 4), _bars("buf_free", buffers, 1)
+            self.o_ready, self.o_free, self.sum_ready = _bars("o_ready", 2, 1), _bars("o_free", 2, 4), _bars("sum_ready", 2, 8)
+            self.xchg = Barrier("xchg", 8)
+
+    rounds = [Round(0, passes)] + ([Round(1, 2)] if second_round else [])
+
+    def producer(x, which):
+        stages, full, empty, ring = ((k_stages, x.k_full, x.k_empty, k_ring) if which == "K" else (v_stages, x.v_full, x.v_empty, v_ring))
+        n = 0
+        for i in range(tiles):
+            if which == "K":
+                yield ("wait", x.q_empty[i & 1], ((i >> 1) & 1) ^ 1)
+                land = sim.t + sim.r(500, 1500)
+                q_tile[i & 1].write(sim, (x.number, i), at=land)
+                sim.at(land, (lambda b=x.q_full[i & 1]: b.arrive(sim)))
+            for _ in range(x.jobs if which == "K" else chunks):
+                st = n % stages
+                yield ("wait", empty[st], ((n // stages) & 1) ^ 1)
+                land = sim.t + sim.r(500, 1500)
+                ring[st].write(sim, (x.number, n), at=land)
+                sim.at(land, (lambda b=full[st]: b.arrive(sim)))
+                n += 1
+
+    def s_issuer(x):
+        n = 0
+        for i in range(tiles):
+            yield ("wait", x.q_full[i & 1], (i >> 1) & 1)
+            for _ in range(x.jobs):
+                buf, ks = n % buffers, n % k_stages
+                wait = ["wait", x.k_full[ks], (n // k_stages) & 1]
+                if n >= buffers:
+                    wait += [x.free[buf], ((n // buffers) & 1) ^ 1]
+                yield tuple(wait)
+                assert owner[buf] is None, ("scores written over a live buffer", buf, owner[buf], n)
+                start, done = sim.mma("s", 256)
+                q_tile[i & 1].read(sim, (x.number, i), done)
+                k_ring[ks].read(sim, (x.number, n), done)
+                sim.at(done, (lambda b=buf, j=n: owner.__setitem__(b, ("s", j))))
+                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+                sim.commit("s", x.s_ready[buf])
+                sim.commit("s", x.k_empty[ks])
+                yield ("delay", sim.r(30, 80))
+                n += 1
+            sim.commit("s", x.q_empty[i & 1])
+            yield ("delay", sim.r(30, 80))
+
+    def pv_issuer(x):
+        n = vjob = 0
+        for i in range(tiles):
+            for j in range(x.jobs):
+                buf, vs, pv = n % buffers, vjob % v_stages, j >= x.first_p2
+                wait = ["wait", x.wg_done[buf], (n // buffers) & 1]
+                if pv:
+                    wait += [x.v_full[vs], (vjob // v_stages) & 1]
+                    if j == x.first_p2 and i > 1:
+                        wait += [x.o_free[i & 1], ((i - 2) >> 1) & 1]
+                yield tuple(wait)
+                if pv:
+                    assert owner[buf] == ("p", n), ("P.V read", buf, owner[buf], n)
+                    start, done = sim.mma("pv", 384)
+                    v_ring[vs].read(sim, (x.number, vjob), done)
+                    if j == x.first_p2:
+                        acc[i & 1].write(sim, (x.number, i))
+                    sim.at(done, (lambda b=buf: owner.__setitem__(b, None)))
+                    yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+                    sim.commit("pv", x.v_empty[vs])
+                    vjob += 1
+                else:
+                    assert owner[buf] == ("m", n), ("first-pass buffer handed back early", buf, owner[buf], n)
+                    owner[buf] = None
+                sim.commit("pv", x.free[buf])
+                yield ("delay", sim.r(30, 80))
+                n += 1
+            sim.commit("pv", x.o_ready[i & 1])
+            yield ("delay", sim.r(30, 80))
+
+    def softmax(x, group, warp):
+        n = group                         # this group's next job, numbered over the CTA
+
+        def exchange(i):
+            slot = maxima[i & 1][group]
+            if warp == 0:
+                slot.write(sim, (x.number, i))
+            x.xchg.arrive(sim)
+            yield ("wait", x.xchg, i & 1)
+            for g in range(2):
+                maxima[i & 1][g].read(sim, (x.number, i))
+
+        for i in range(tiles):
+            j = (group - i * x.jobs) & 1
+            assert j >= x.jobs or i * x.jobs + j == n, ("job numbering", i, j, n)
+            exchanged = x.passes == 1
+            while j < x.jobs:
+                buf = n % buffers
+                if j >= x.first_p2 and not exchanged:
+                    exchanged = True
+                    yield from exchange(i)
+                yield ("wait", x.s_ready[buf], (n // buffers) & 1)
+                assert owner[buf] is not None and owner[buf][1] == n, ("softmax read", buf, owner[buf], n)
+                yield ("delay", sim.r(400, 1400))
+                if warp == 0:
+                    owner[buf] = ("p" if j >= x.first_p2 else "m", n)
+                x.wg_done[buf].arrive(sim)
+                n += 2
+                j += 2
+            if not exchanged:
+                yield from exchange(i)
+            if i > 1 and softmax_waits_for_sums:
+                yield ("wait", x.o_free[i & 1], ((i - 2) >> 1) & 1)
+            if warp == 0:
+                sums[i & 1][group].write(sim, (x.number, i))
+            x.sum_ready[i & 1].arrive(sim)
+
+    def epilogue(x, warp):
+        for i in range(tiles):
+            yield ("wait", x.sum_ready[i & 1], (i >> 1) & 1)
+            yield ("wait", x.o_ready[i & 1], (i >> 1) & 1)
+            for _ in range(2):
+                for r in (acc[i & 1], *sums[i & 1]):
+                    r.read(sim, (x.number, i))
+                yield ("delay", sim.r(100, 2500))
+            acc[i & 1].read(sim, (x.number, i))
+            x.o_free[i & 1].arrive(sim)
+
+    def all_rounds(role, *args):
+        for x in rounds:
+            yield from role(x, *args)
+            sync.arrive(sim)
+            yield ("wait", sync, x.number & 1)
+
+    for which in ("K", "V"):
+        sim.spawn("producer " + which, all_rounds(producer, which))
+    sim.spawn("s", all_rounds(s_issuer))
+    sim.spawn("pv", all_rounds(pv_issuer))
+    for w in range(4):
+        for g in range(2):
+            sim.spawn("softmax%d%d" % (g, w), all_rounds(softmax, g, w))
+        sim.spawn("epilogue%d" % w, all_rounds(epilogue, w))
+    return sim.run()
 
 
 def single_shot_backward_kernel(seed, t_begin, n_tiles, tiles_per_head, mma_done_count=2, softmax_waits_for_products=True):

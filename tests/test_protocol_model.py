@@ -17,13 +17,14 @@ def _pieces(seed):
 
 
 def test_key_major_kernel_protocol_has_no_hazard_or_deadlock():
-    """attn_dkv_pooled_loop_tc_kernel as built: one S^T / dP^T thread, one dV / dK thread, three buffers, barriers per buffer."""
+    """attn_dkv_pooled_loop_tc_kernel, dense form: two producers, one S^T / dP^T warp, one dV / dK warp, three buffers, barriers per
+    buffer, epilogue warps."""
     for seed in range(RUNS):
         assert outcome(key_major_kernel, seed, _pieces(seed)) == "ok", seed
 
 
 def test_query_major_kernel_protocol_has_no_hazard_or_deadlock():
-    """attn_dq_pooled_loop_tc_kernel as built: one S / dP thread, one dQ thread."""
+    """attn_dq_pooled_loop_tc_kernel: two producers, one S / dP warp, one dQ warp, two accumulators, epilogue warps."""
     for seed in range(RUNS):
         rng = random.Random(seed)
         assert outcome(query_major_kernel, seed, rng.randint(1, 7), rng.choice([4, 6, 18])) == "ok", seed
@@ -31,8 +32,8 @@ def test_query_major_kernel_protocol_has_no_hazard_or_deadlock():
 
 @pytest.mark.parametrize("passes", [1, 2])
 def test_forward_kernel_protocol_has_no_hazard_or_deadlock(passes):
-    """attn_fwd_pooled_loop_tc_kernel as built, in its one-pass form (odd and even chunk counts: with 9 chunks the groups
-    swap the parity of their first job from tile to tile) and in the two-pass form that redoes marked rows."""
+    """attn_fwd_pooled_loop_tc_kernel in its one-pass form (odd and even chunk counts: with 9 chunks the groups
+    swap the parity of their first job from tile to tile) and in the two-pass form."""
     for seed in range(RUNS):
         rng = random.Random(seed)
         assert outcome(forward_kernel, seed, rng.randint(1, 6), rng.choice([2, 3, 8, 9]), passes) == "ok", seed
@@ -82,3 +83,37 @@ def test_model_catches_a_stage_freed_by_one_issuer_only_and_an_unguarded_overwri
     one = sum(outcome(single_shot_backward_kernel, s, *_single_shot_case(s), mma_done_count=1) != "ok" for s in range(80))
     two = sum(outcome(single_shot_backward_kernel, s, *_single_shot_case(s), softmax_waits_for_products=False) != "ok" for s in range(80))
     assert one > 0 and two > 0
+
+
+def test_gathered_key_major_form_has_no_hazard_or_deadlock():
+    """attn_dkv_pooled_loop_tc_kernel, gathered form: units of four query tiles (pieces begin and end inside one), two buffers -- a group
+    meets its own buffer again with its next job -- and two accumulators."""
+    for seed in range(RUNS):
+        rng = random.Random(seed)
+        units = [rng.randint(1, 4)] + [4] * rng.randint(0, 9) + [rng.randint(1, 4)]
+        assert outcome(key_major_kernel, seed, units, buffers=2, accs=2) == "ok", seed
+
+
+def test_one_chunk_tiles_leave_a_group_without_work():
+    """A list of one chunk: every other tile has no job for a group, which still takes part in the exchange of maxima and row sums."""
+    for seed in range(RUNS):
+        rng = random.Random(seed)
+        assert outcome(forward_kernel, seed, rng.randint(1, 7), 1, 1 + seed % 2) == "ok", seed
+        assert outcome(query_major_kernel, seed, rng.randint(1, 7), rng.choice([1, 3])) == "ok", seed
+
+
+@pytest.mark.parametrize("chunks", [1, 3, 8])
+def test_second_round_on_fresh_barriers_has_no_hazard_or_deadlock(chunks):
+    """A CTA that marked a row walks its tiles again, in two passes, over the same shared and tensor memory; commits of the first round may
+    still land on that round's own barriers."""
+    for seed in range(RUNS // 2):
+        assert outcome(forward_kernel, seed, random.Random(seed).randint(1, 5), chunks, 1, second_round=True) == "ok", seed
+
+
+def test_model_catches_a_producer_an_epilogue_warp_and_a_reader_left_out_of_the_count():
+    """Three mutations of today's protocols: a query stage that counts one of its two producers, an accumulator handed back by the first of four
+    epilogue warps, row sums overwritten without waiting for the epilogue."""
+    producer = sum(outcome(key_major_kernel, s, _pieces(s), full_count=1) != "ok" for s in range(60))
+    warp = sum(outcome(query_major_kernel, s, 7, 1, free_count=1) != "ok" for s in range(60))
+    sums = sum(outcome(forward_kernel, s, 6, 1, 1, softmax_waits_for_sums=False) != "ok" for s in range(60))
+    assert producer > 0 and warp > 0 and sums > 0
