@@ -241,8 +241,8 @@ typedef struct LlsaAttnArgs {
   const LlsaTensor* flat_pairs;/* not used any more; NULL, or the `pairs` list of llsa_transpose_indices_pairs */
   const LlsaTensor* flat_ranges;/* backward, bf16 tensors only: I32 [B,H,ceil(N/16*topk/S),2], the `ranges`
                                   list of llsa_transpose_indices_pairs for the same CSR as offsets / flat */
-  int32_t no_tcgen05;          /* 1: keep the pooled-key stages on the mma.sync kernels (the form used
-                                  for shapes the tcgen05 kernels do not cover); for cross-checks */
+  int32_t no_tcgen05;          /* 1: keep the pooled-key stages on the mma.sync kernels, which sum fine and pooled keys in one
+                                  kernel (otherwise used where a list wants `remainder` and has none); for cross-checks */
   int32_t wait_limit;          /* 0: default.  Otherwise the number of polls after which a bounded
                                   mbarrier wait inside the tcgen05 kernels gives up (tests use a tiny
                                   value to exercise the give-up path; the kernel then returns

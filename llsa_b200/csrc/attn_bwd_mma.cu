@@ -2,7 +2,8 @@
 // Reference: sparse_indices_attn_res_scatter_bwd_v2 (sparse_attention_res_1.py:403-471)
 // and sparse_indices_attn_res_scatter_2_2_bwd_v2 (sparse_attention_res_2.py:578-681).
 //
-// Three kernels on mma.sync.m16n8k16 with the operand fragments of mma_frag.cuh:
+// Kernels on mma.sync.m16n8k16 with the operand fragments of mma_frag.cuh.  The first two hold fine and pooled keys together; they run where
+// the tcgen05 kernels do not take the pooled ones: switched off (no_tcgen05), or a list that wants `remainder` and has none (dQ only).
 //   attn_dq_mma_kernel     one warp per query block: delta = rowsum(o*do) (the
 //                          reference's separate _attn_bwd_preprocess pass), then
 //                          S, dP and dQ over the fine, pooled-1 and pooled-2 keys.

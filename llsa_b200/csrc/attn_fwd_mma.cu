@@ -2,6 +2,9 @@
 // Reference: _sparse_indices_attn_res_fwd (sparse_attention_res_1.py:9-120) and
 // _sparse_indices_attn_res_2_2_fwd (sparse_attention_res_2.py:9-163).
 //
+// attn_fwd_fine_kernel (below) takes the fine blocks where tcgen05 kernels take the pooled keys.  Otherwise -- no pooled keys at all, the
+// tcgen05 kernels switched off, or a list that wants `remainder` and has none -- attn_fwd_mma_kernel takes both:
+//
 // One warp owns one 16-row query block (the m16 of mma.sync.m16n8k16); a CTA of
 // NW warps owns NW consecutive query blocks, which always share their parent
 // block and therefore the same pooled keys.

@@ -21,7 +21,7 @@ GROUPS = {
     "attn_bwd_dkv_pooled": ("attn_bwd_pooled_tc_kernel", "attn_dkv_pooled_kernel", "attn_dq_pooled_loop_tc_kernel", "attn_dkv_pooled_loop_tc_kernel"),
     "attn_bwd_dkv_fine": ("attn_dkv_fine_ring_kernel", "attn_dkv_finish_kernel"),
     "pool_pyramid": ("pool_pyramid_kernel", "pool_pyramid_bf16_kernel"),
-    "coarse_topk": ("coarse_topk_mma_kernel", "coarse_topk_kernel"),
+    "coarse_topk": ("coarse_topk_mma_kernel", "coarse_topk_tile_kernel", "coarse_topk_kernel"),
     "refine_topk": ("refine_topk_kernel",),
     "transpose_indices": ("transpose_range_kernel",),
 }

@@ -48,7 +48,7 @@ _exact_pooled_grad = os.environ.get("LLSA_B200_EXACT_POOLED_GRAD", "0") == "1"
 
 _stage_hook = None
 _overlap_transpose = os.environ.get("LLSA_B200_OVERLAP_TRANSPOSE", "1") != "0"
-# Cross-check switch: keep the pooled-key stages on the mma.sync kernels (the form other shapes use).
+# Cross-check switch: keep the pooled-key stages on the mma.sync kernels (fine and pooled keys of o / dq in one kernel).
 _no_tcgen05 = False
 # Cross-check switch: False = long pooled key lists take two passes over the keys for every row (no `fwd_redo` scratch).
 _one_pass_pooled = True

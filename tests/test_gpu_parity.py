@@ -458,7 +458,7 @@ def _pooled_fwd_both_forms(L, q, k, v, monkeypatch):
         monkeypatch.setattr(ops, "_one_pass_pooled", one_pass)
         dbg = L.llsa_l2_debug(q.to(DEV), k.to(DEV), v.to(DEV), 8, 8, 16)
         out.append({n: dbg[n].detach().cpu() for n in ("o", "lse", "indices", "p_indices", "pk", "pv", "pk2", "pv2")})
-        if one_pass:      # one byte per query row: 1 = left to the second launch
+        if one_pass:      # one byte per query row: 1 = left to the second round
             out[-1]["redone"] = int(ops._last_fwd_redo.view(torch.uint8)[:q.shape[0] * q.shape[1] * q.shape[2]].sum())
     return out
 
@@ -477,7 +477,7 @@ def test_long_pooled_list_one_pass_matches_two_passes(monkeypatch):
 
 def test_long_pooled_list_rows_beyond_the_one_pass_range_are_redone(monkeypatch):
     """Logits in the hundreds: in many rows a pooled key outweighs all fine keys by more than 1e30, the one-pass form
-    marks those rows and the second launch redoes them exactly.  Both forms against the oracle's fp32 evaluation."""
+    marks those rows and its second round redoes them exactly.  Both forms against the oracle's fp32 evaluation."""
     L = _ops()
     q, k, v, _ = synth.correlated_qkv(51, 1, 1, 65536, 64, dtype=torch.bfloat16)
     q, k = (q.float() * 12).to(torch.bfloat16), (k.float() * 12).to(torch.bfloat16)
@@ -784,7 +784,7 @@ def test_host_pipeline_matches_direct_call(chunk_heads, graphs):
 
 # ------------------------------------------------------------------ full-size properties (BASELINE config 3 shape)
 def test_batch_of_288_slices_matches_its_own_slices():
-    """288 (b,h) slices (B=48, H=6, N=16384: 8 GB on the device, the P / dS hand-over alone 2.4 GB -- byte offsets past 2^31):
+    """288 (b,h) slices (B=48, H=6, N=16384: 8 GB on the device: byte offsets of a tensor past 2^29, of the layer past 2^31):
     every slice is independent, so the first and the last two batch elements computed alone must give the same o and dq bit
     for bit and the same dk, dv up to the order of their fp32 sums (the work ranges depend on the size of the launch)."""
     L = _ops()
