@@ -193,6 +193,7 @@ int llsa_transpose_indices_noalloc(const LlsaTensor* idx, const LlsaTensor* offs
                                    int32_t* status, void* stream);
 
 /* ---- attention ------------------------------------------------------------ */
+/* Zero-initialise it, and build against the header of the library in use: fields are appended (`remainder` with llsa_version() 102). */
 typedef struct LlsaAttnArgs {
   /* forward operands */
   const LlsaTensor* q;   /* [B,H,N,D] */

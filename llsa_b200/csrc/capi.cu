@@ -65,7 +65,7 @@ int raise_smem_limit(const void* kernel, size_t bytes) {
 
 }  // namespace llsa
 
-extern "C" int llsa_version(void) { return 101; }
+extern "C" int llsa_version(void) { return 102; }
 extern "C" int llsa_status_check(int32_t w) {
   LLSA_REQUIRE(w == 0, LLSA_ERR_DEVICE_CHECK, "device status 0x%x:%s%s", (unsigned) w,
                (w & LLSA_DEV_BAD_INDEX) ? " a block index outside its range was met;" : "",

@@ -1,7 +1,7 @@
 """Turns an ncu report of the benchmark's kernels into the figures the repository keeps.
 
     ncu -i REPORT.ncu-rep --page raw --csv > raw.csv
-    python -m llsa_b200.ncu_summary raw.csv --slices 12 [--json profiles/ncu_dram_bytes.json] [--table]
+    python -m llsa_b200.ncu_summary raw.csv [raw2.csv ...] --slices 24 [--json profiles/ncu_dram_bytes.json] [--table]
 
 --json writes, per kernel group of bench.py (attn_fwd, attn_bwd_dq, attn_bwd_dkv_pooled, attn_bwd_dkv_fine, ...),
 the DRAM bytes of one launch (dram__bytes_read.sum + dram__bytes_write.sum, mean over the captured launches) at the
@@ -63,12 +63,12 @@ def read_raw(path):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("raw_csv")
+    ap.add_argument("raw_csv", nargs="+", help="one file per report: units differ from report to report")
     ap.add_argument("--slices", type=int, required=True, help="(b,h) slices of the captured launch")
     ap.add_argument("--json", default=None)
     ap.add_argument("--table", action="store_true")
     args = ap.parse_args()
-    launches = read_raw(args.raw_csv)
+    launches = [k for path in args.raw_csv for k in read_raw(path)]
     per = {}
     for k in launches:
         per.setdefault(k["name"], []).append(k)
