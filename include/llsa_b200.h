@@ -261,7 +261,8 @@ typedef struct LlsaAttnArgs {
                                   llsa_attn_remainder_elems() is not 0 (not read before it is written).  For these pooled
                                   key lists the fine stage leaves here what rounding its o (backward: stage_mask 1, its
                                   dq) to bf16 dropped, and the pooled stage (2) adds it, so that results are rounded
-                                  once.  NULL: fine and pooled keys of o / dq in one (slower) kernel for these lists */
+                                  once.  NULL: fine and pooled keys of o / dq in one (slower) kernel for these lists.  Calls that
+                                  issue the stages of one backward separately pass the same scratch to 1 and 2 */
 } LlsaAttnArgs;
 
 /* Forward: o, lse.  One level (pk2 == NULL) replaces sparse_indices_attn_res_fwd
