@@ -17,21 +17,23 @@
 // hold anything up to 2^127 times it; a row whose pooled keys outweigh its fine keys by more than that (its row sum
 // passes 1e30, or is NaN) is left untouched and marked in `redo`; a CTA that has marked a row of its tiles goes over them again
 // with two passes and writes exactly the marked rows.  (A second launch that looked for marks cost every call 1 to 2 us.)
-// Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64):
+// Roles (one persistent CTA per SM, 20 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64):
 //   warp 8, warp 11  : TMA producers: Q per tile (2 stages) and K chunks (ring of 4; every chunk is loaded in both passes); V chunks (ring
 //                      of 4, pass 2 only)
 //   warp 9           : issues S of every "job" (a chunk of a pass).  Job number n, counted over all tiles of the CTA,
 //                      uses S buffer n mod 3 (TMEM columns [128 b, 128 b + 128)); O of tile i lives in [384 + 64 (i mod 2), + 64).
 //   warp 10          : issues O += P.V of the pass-2 jobs and hands every job's buffer back to warp 9 (buf_free,
 //                      committed behind the instructions that read P)
-//   warps 0-3 / 4-7  : two softmax warpgroups, group w owns the jobs n = w (mod 2); thread r owns query row r
-//                      (TMEM lane r).  They leave a row's sum (and reference) in shared memory and go on to the next tile.
+//   warps 0-3 / 4-7 / 16-19 : three softmax warpgroups, group w owns the jobs n = w (mod 3) and with them S buffer w; thread r owns query
+//                      row r (TMEM lane r).  They leave a row's sum (and reference) in shared memory and go on to the next tile.
 //   warps 12-15      : epilogue, thread = row: merges O with the fine part (o, lse written by the fine kernel) and stores both.
-// What bounds it: the chain S -> exponentials -> P.V over three buffers, 1,500 cycles a job (the 128 exponentials of a row take 1,024 on the
-// SM's 16 MUFU lanes, the tensor pipe 640; a quarter of the exponentials moved to the FMA pipe changed nothing).  A clock trace
-// of the form with one producer lane, the epilogue in the softmax groups and one O buffer (785 us at l1, B=2 H=4 N=65536: 1,630 cycles a
-// job) showed the producer needing 1,300 cycles a job for its two waits and two copies, and 5,900 idle cycles at every tile boundary;
-// this form needs 712 us (840 -> 625 at two levels, B=1 H=6 N=262144).
+// What bounds it: the chain S -> exponentials -> P.V over three buffers, 1,430 cycles a job: with the softmax left out the copies, products and
+// hand-overs of a job take 900, with its exponentials alone left out 1,070; the 128 exponentials of a row take 1,024 on the SM's 16 MUFU lanes.
+// l1, B=2 H=4 N=65536: 692 us with two groups (their warps spend two thirds of a job in waits and loads), 669 with three; two levels, H=6
+// N=262144: 620 -> 590; B=2 H=4 N=65536: 90 -> 85.  No gain from: two groups that load a whole row of scores at once and hand the S buffer back
+// before the exponentials (732: fewer warps for the MUFU), eight warps a job (657 long lists, 56 -> 58 short ones), a
+// quarter or a third of the exponentials as a degree-5 polynomial on the FMA pipe (669 and 676; 85 -> 95 and 98 at N=65536 two levels).  In the form with one producer lane, the epilogue in the softmax groups and one O buffer
+// (785 us) the producer needed 1,300 cycles a job for its two waits and two copies, and every tile boundary cost 5,900 idle cycles.
 // Every mbarrier wait is bounded; a wait that expires raises a CTA-wide abort flag, every role leaves its loops,
 // lse of the unfinished rows is poisoned with NaN and TMEM is freed.
 #include <string.h>
@@ -49,8 +51,10 @@ constexpr int kRows = 128;
 constexpr int kChunk = 128;                 // keys per chunk
 constexpr int kTile = kRows * 64;           // elements of a [128 x 64] bf16 tile (16 KB)
 constexpr int kKStages = 4, kVStages = 4;
-constexpr int kThreads = 512;
-constexpr int kBufs = 3;
+constexpr int kThreads = 640;
+constexpr int kLaunchRegs = 96, kIssueRegs = 40, kEpilogueRegs = 104, kSoftmaxRegs = 112;     // a thread's, per role: 40 + 104 + 3 x 112 = 5 x 96
+static_assert(kIssueRegs + kEpilogueRegs + 3 * kSoftmaxRegs <= 5 * kLaunchRegs, "the takers would wait for good");
+constexpr int kBufs = 3, kGroups = 3;       // softmax group w owns S buffer w
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr uint32_t kColO = 384;
 // One pass over a list that one kernel used to take with running maxima (REM): where in its binade a probability of a logit of 0 lands.  bf16 is finest just below a power of two, which is where a row's
@@ -85,9 +89,9 @@ __device__ __forceinline__ void init_bars(LoopBars& bars) {
   for (int i = 0; i < 2; ++i) {
     tc::mbar_init(&bars.o_ready[i], 1);
     tc::mbar_init(&bars.o_free[i], 4);
-    tc::mbar_init(&bars.sum_ready[i], 8);
+    tc::mbar_init(&bars.sum_ready[i], 4 * kGroups);
   }
-  tc::mbar_init(&bars.xchg, 8);
+  tc::mbar_init(&bars.xchg, 4 * kGroups);
   tc::fence_mbar_init();
 }
 
@@ -101,8 +105,8 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   __shared__ LoopBars bars_of[2];                    // of the first round over the tiles and of the one for marked rows
   __shared__ uint32_t s_tmem;
   __shared__ tc::WaitCtl s_ctl;
-  __shared__ float s_max[2][2][kRows];               // [tile parity][group][row]: row maxima after pass 1
-  __shared__ float s_sum[2][2][kRows], s_ref[2][kRows];      // [tile parity][group][row] row sums; [tile parity][row] their reference
+  __shared__ float s_max[2][kGroups][kRows];             // [tile parity][group][row]: row maxima after pass 1
+  __shared__ float s_sum[2][kGroups][kRows], s_ref[2][kRows];      // [tile parity][group][row] row sums; [tile parity][row] their reference
   bf16* base = reinterpret_cast<bf16*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   bf16* sQ = base;                          // [2][128][64]
   bf16* sK = sQ + 2 * kTile;                // [kKStages][128][64]
@@ -122,21 +126,34 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   tc::fence_after_sync();
   pdl_trigger();
   const uint32_t tmem = s_tmem;
-  for (int n_pass = redo ? 1 : 2, round = 0;; n_pass = 2, ++round) {
-    LoopBars& bars = bars_of[round];
-    int marked = 0;                           // epilogue: this thread has left a row to the second round
-    // jobs per tile; job j of tile i has the CTA-wide number i * jobs + j, which picks the S buffer (mod 3) and the softmax
-    // group (mod 2; with one pass and an odd chunk count the parity of a tile's first job alternates)
-    const int jobs = n_pass * n_chunks, first_p2 = jobs - n_chunks;
-    // keys of chunk c that belong to its list (a multiple of 32)
-    auto keys_of = [&](int c) {
-      const int left = c < gathered ? a.p1_blocks * kBS - c * kChunk : (int) n_c - (c - gathered) * kChunk;
-      return left < kChunk ? left : kChunk;
-    };
+  // One round over the CTA's tiles, and another for marked rows.  body(round's barriers, passes, jobs per tile): job j of tile i has the CTA-wide
+  // number i * jobs + j, which picks the S buffer and the softmax group (mod 3).  Every role calls this with its own body; the roles meet at
+  // the end of a round.
+  int marked = 0;                             // epilogue: this thread has left a row to the second round
+  auto rounds = [&](auto body) {
+    for (int round = 0, n_pass = redo ? 1 : 2;; ++round, n_pass = 2) {
+      marked = 0;
+      body(bars_of[round], n_pass, n_pass * n_chunks);
+      tc::fence_before_sync();
+      if (!__syncthreads_or(marked) || abort_flag->abort) break;
+      if (tid == 0) init_bars(bars_of[1]);
+      __syncthreads();
+      tc::fence_after_sync();
+    }
+  };
+  // keys of chunk c that belong to its list (a multiple of 32)
+  auto keys_of = [&](int c) {
+    const int left = c < gathered ? a.p1_blocks * kBS - c * kChunk : (int) n_c - (c - gathered) * kChunk;
+    return left < kChunk ? left : kChunk;
+  };
 
-    if (warp == 8 || warp == 11) {
+  // 640 threads launch with 96 registers each; the warps that issue copies and products leave most of theirs to the others
+  if (warp >= 8 && warp < 12) tc::regs_set<kIssueRegs, kLaunchRegs>();
+  if (warp == 8 || warp == 11) {
+    rounds([&](LoopBars& bars, int, int jobs) {
       // ---------------------------------------------------------------- TMA producers: warp 8 Q and keys, warp 11 values
       const bool vals = warp == 11;
+      const int first_p2 = jobs - n_chunks;
       uint64_t *full = vals ? bars.v_full : bars.k_full, *empty = vals ? bars.v_empty : bars.k_empty;
       const CUtensorMap *mg = vals ? &maps.vg : &maps.kg, *mc = vals ? &maps.vc : &maps.kc;
       bf16* ring = vals ? sV : sK;
@@ -170,7 +187,9 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           if (++st == kKStages) { st = 0; ph ^= 1; }
         }
       }
-    } else if (warp == 9) {
+    });
+  } else if (warp == 9) {
+    rounds([&](LoopBars& bars, int, int jobs) {
       // ---------------------------------------------------------------- MMA issuer 1: S of every job
       {
         const uint32_t id_s = tc::instr_desc(kRows, kChunk, 0, 0);
@@ -201,10 +220,13 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           tc::umma_commit_w(&bars.q_empty[qs]);
         }
       }
-    } else if (warp == 10) {
+    });
+  } else if (warp == 10) {
+    rounds([&](LoopBars& bars, int, int jobs) {
       // ---------------------------------------------------------------- MMA issuer 2: O (+)= P(job, TMEM) . V chunk
       {
         const uint32_t id_o = tc::instr_desc(kRows, 64, 0, 1);
+        const int first_p2 = jobs - n_chunks;
         const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
         constexpr uint32_t kStage = (uint32_t) (kTile * 2) >> 4;
         const uint32_t lV = ((tc::smem_u32(sV) >> 4) & 0x3FFFu) | ((1024u >> 4) << 16);
@@ -242,14 +264,19 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           tc::umma_commit_w(&bars.o_ready[i & 1]);
         }
       }
-    } else if (warp < 8) {
+    });
+  } else if (warp < 8 || warp >= 16) {
+    tc::regs_set<kSoftmaxRegs, kLaunchRegs>();
+    rounds([&](LoopBars& bars, int n_pass, int jobs) {
       // ---------------------------------------------------------------- softmax, thread = query row
-      const int wg = warp >> 2, qd = warp & 3, r = qd * 32 + lane;
+      const int wg = warp < 8 ? warp >> 2 : 2, qd = warp & 3, r = qd * 32 + lane;
+      const int first_p2 = jobs - n_chunks;
       const float sl2 = a.scale * kLog2eF;
       const float lw1 = log2f(a.w1), lw2 = log2f(a.w2);
       const uint32_t t_lane = tmem + ((uint32_t) (qd * 32) << 16);
-      int buf = wg;                          // S buffer of this group's next job (it takes every other job of the CTA) and
-      uint32_t bph = 0;                      // the phase parity of that buffer's barriers
+      const int buf = wg;                    // this group takes every third job of the CTA: always the same S buffer; the phase parity of
+      uint32_t bph = 0;                      // that buffer's barriers
+      int first = wg;                        // its first job of the tile at hand
       float va[32];
       auto lse_of = [&](int i) {             // the fine part's log-sum-exp of this thread's row of tile i
         const int tile = blockIdx.x + i * gridDim.x;
@@ -271,11 +298,12 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           __syncwarp();
           if (lane == 0) tma::mbar_arrive(&bars.xchg);
           const bool ok_ = __all_sync(0xffffffffu, tc::bounded_wait(&bars.xchg, (uint32_t) i & 1, abort_flag));
-          mx = fmaxf(s_max[i & 1][0][r], s_max[i & 1][1][r]);
+          mx = fmax3(s_max[i & 1][0][r], s_max[i & 1][1][r], s_max[i & 1][2][r]);
           if (mx == -INFINITY) mx = 0.f;       // no score above -inf (masked keys): their weight is 0 whatever the reference
           return ok_;
         };
-        for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
+        int j = first;
+        for (; j < jobs; j += kGroups) {
           const bool p2 = j >= first_p2;
           const int c = j >= n_chunks ? j - n_chunks : j;
           const float lw = (c < gathered || !a.two_level) ? lw1 : lw2;
@@ -317,9 +345,9 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tma::mbar_arrive(&bars.wg_done[buf]);
-          buf += 2;
-          if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
+          bph ^= 1;
         }
+        first = j - jobs;
         if (ok && !exchanged) ok = exchange_max();
         // the sums of the tile before the last have been read
         if (ok && i > 1) ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_free[i & 1], ((uint32_t) (i - 2) >> 1) & 1, abort_flag));
@@ -331,7 +359,10 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         __syncwarp();
         if (lane == 0) tma::mbar_arrive(&bars.sum_ready[i & 1]);
       }
-    } else {
+    });
+  } else {
+    tc::regs_set<kEpilogueRegs, kLaunchRegs>();
+    rounds([&](LoopBars& bars, int n_pass, int) {
       // ---------------------------------------------------------------- epilogue, thread = query row
       const int qd = warp & 3, r = qd * 32 + lane;
       bool ok = true;
@@ -354,7 +385,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           if (mine) *lse_p = __int_as_float(0x7fc00000);             // NaN: not completed
           break;
         }
-        const float lsum = s_sum[i & 1][0][r] + s_sum[i & 1][1][r], mx = s_ref[i & 1][r];
+        const float lsum = s_sum[i & 1][0][r] + s_sum[i & 1][1][r] + s_sum[i & 1][2][r], mx = s_ref[i & 1][r];
         // one pass: the row is this round's unless its sum left the safe range (false for NaN too): the mark hands it to the second
         if (redo && n_pass == 1) {
           mine = lsum < 1e30f;
@@ -400,12 +431,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         }
         if (mine) *lse_p = (Lm + log2f(ef + ep)) * 0.6931471805599453f;
       }
-    }
-    tc::fence_before_sync();
-    if (!__syncthreads_or(marked) || abort_flag->abort) break;
-    if (tid == 0) init_bars(bars_of[1]);
-    __syncthreads();
-    tc::fence_after_sync();
+    });
   }
   if (abort_flag->abort) tc::abort_drain();
   __syncthreads();
@@ -455,7 +481,7 @@ int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) (2 + kKStages + kVStages) * kTile * sizeof(bf16);
   auto kernel = a.rem ? attn_fwd_pooled_loop_tc_kernel<true> : attn_fwd_pooled_loop_tc_kernel<false>;
-  LLSA_SMEM_LIMIT(kernel, smem);
+  LLSA_SMEM_LIMIT_REGS(kernel, smem, kLaunchRegs);
   unsigned char* redo = g->fwd_redo && pooled_loop_one_pass(a) ? reinterpret_cast<unsigned char*>(g->fwd_redo->ptr) : nullptr;
   launch_pdl(kernel, grid, kThreads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, redo);
   LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");

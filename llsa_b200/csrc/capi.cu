@@ -49,7 +49,7 @@ int check_contig(const LlsaTensor* t, const char* name, int dtype, int ndim, con
 // The dynamic shared-memory limit is an attribute of the kernel, not of a launch: it is only ever raised, under a lock,
 // and remembered per (kernel, device), so launches of different sizes from different host threads cannot lower each
 // other's limit between the attribute call and the launch.
-int raise_smem_limit(const void* kernel, size_t bytes) {
+int raise_smem_limit(const void* kernel, size_t bytes, int launch_regs) {
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, size_t> limit;
   int dev = 0;
@@ -57,6 +57,11 @@ int raise_smem_limit(const void* kernel, size_t bytes) {
   std::lock_guard<std::mutex> lock(mu);
   size_t& cur = limit[std::make_pair(kernel, dev)];
   if (bytes > cur) {
+    if (launch_regs) {
+      cudaFuncAttributes at;
+      LLSA_CUDA_OK(cudaFuncGetAttributes(&at, kernel));
+      LLSA_REQUIRE(at.numRegs == launch_regs, LLSA_ERR_CUDA, "kernel built with %d registers a thread, its split needs %d", at.numRegs, launch_regs);
+    }
     LLSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes));
     cur = bytes;
   }

@@ -64,12 +64,18 @@ inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);      // LLSA_LAUNCH_OK picks the error up
 }
 
-// Raises (never lowers) a kernel's dynamic shared-memory limit on the current device; thread-safe.
-int raise_smem_limit(const void* kernel, size_t bytes);
+// Raises (never lowers) a kernel's dynamic shared-memory limit on the current device; thread-safe.  launch_regs: the registers per thread that
+// a kernel which redistributes them (tc05.cuh: regs_set) must have been built with; a launch with fewer would wait for good, so it is refused.
+int raise_smem_limit(const void* kernel, size_t bytes, int launch_regs = 0);
 #define LLSA_SMEM_LIMIT(kernel, bytes)                                              \
   do {                                                                              \
     int rc__ = ::llsa::raise_smem_limit((const void*) (kernel), (size_t) (bytes));  \
     if (rc__) return rc__;                                                          \
+  } while (0)
+#define LLSA_SMEM_LIMIT_REGS(kernel, bytes, regs)                                           \
+  do {                                                                                      \
+    int rc__ = ::llsa::raise_smem_limit((const void*) (kernel), (size_t) (bytes), (regs));  \
+    if (rc__) return rc__;                                                                  \
   } while (0)
 
 // Nominal entries per work range of the fine dK/dV kernel: the index transpose cuts the CSR entry list into ranges of this

@@ -95,6 +95,16 @@ __device__ __forceinline__ void abort_drain() {
   for (int i = 0; i < 64; ++i) __nanosleep(1000);
 }
 
+// ---- register split of a warp-specialised kernel: a warpgroup (all of it, once) gives back registers or takes more than the LAUNCH it was
+// launched with.  All the warpgroups' shares together stay within threads x LAUNCH, or the takers wait for good; an increase to fewer
+// registers than a warp has, or a decrease to more, is an illegal instruction.
+template <int N, int LAUNCH>
+__device__ __forceinline__ void regs_set() {
+  static_assert(N % 8 == 0 && N >= 24 && N <= 256, "what setmaxnreg takes");
+  if constexpr (N < LAUNCH) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+  else if constexpr (N > LAUNCH) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 // ---- fences ----
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }

@@ -363,12 +363,12 @@ def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=3, sta
     return sim.run()
 
 
-def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=3, second_round=False, softmax_waits_for_sums=True):
+def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=3, groups=3, second_round=False, softmax_waits_for_sums=True):
     """attn_fwd_pooled_loop_tc_kernel: `tiles` query tiles of `chunks` key chunks; one pass (jobs = chunks, every job
-    feeds P.V) or two (jobs = 2 * chunks: row maxima first, then the exponentials; the two groups exchange their maxima
+    feeds P.V) or two (jobs = 2 * chunks: row maxima first, then the exponentials; the groups exchange their maxima
     once per tile, a group without a second-pass job at its end).  Producers of keys (with Q) and of values; one warp issues S, one P.V
-    and hands every job's buffer back; the two softmax groups take the jobs of one parity of the CTA-wide job number each (with an
-    odd job count the parity of a tile's first job alternates) and leave their row sums to four epilogue warps, as O in one of
+    and hands every job's buffer back; softmax group g of three takes the jobs whose CTA-wide number is g mod 3 (always the same buffer;
+    a tile's first job goes round the groups) and leave their row sums to four epilogue warps, as O in one of
     two accumulators.
     second_round: the CTA has marked a row and goes over its tiles again with two passes, on barriers of its own, behind a CTA-wide
     synchronisation.  softmax_waits_for_sums=False breaks the protocol on purpose (row sums overwritten before they are read)."""
@@ -378,9 +378,9 @@ def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=
     v_ring = [Resource("V stage %d" % i) for i in range(v_stages)]
     q_tile = [Resource("Q stage %d" % i) for i in range(2)]
     acc = [Resource("O accumulator %d" % i) for i in range(2)]
-    sums = [[Resource("row sums %d of group %d" % (i, g)) for g in range(2)] for i in range(2)]
-    maxima = [[Resource("row maxima %d of group %d" % (i, g)) for g in range(2)] for i in range(2)]
-    n_roles = 2 + 2 + 8 + 4
+    sums = [[Resource("row sums %d of group %d" % (i, g)) for g in range(groups)] for i in range(2)]
+    maxima = [[Resource("row maxima %d of group %d" % (i, g)) for g in range(groups)] for i in range(2)]
+    n_roles = 2 + 2 + 4 * groups + 4
     sync = Barrier("__syncthreads", n_roles)
 
     class Round:
@@ -391,8 +391,8 @@ def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=
             self.k_full, self.k_empty = _bars("k_full", k_stages, 1), _bars("k_empty", k_stages, 1)
             self.v_full, self.v_empty = _bars("v_full", v_stages, 1), _bars("v_empty", v_stages, 1)
             self.s_ready, self.wg_done, self.free = _bars("s_ready", buffers, 1), _bars("wg_done", buffers, 4), _bars("buf_free", buffers, 1)
-            self.o_ready, self.o_free, self.sum_ready = _bars("o_ready", 2, 1), _bars("o_free", 2, 4), _bars("sum_ready", 2, 8)
-            self.xchg = Barrier("xchg", 8)
+            self.o_ready, self.o_free, self.sum_ready = _bars("o_ready", 2, 1), _bars("o_free", 2, 4), _bars("sum_ready", 2, 4 * groups)
+            self.xchg = Barrier("xchg", 4 * groups)
 
     rounds = [Round(0, passes)] + ([Round(1, 2)] if second_round else [])
 
@@ -475,11 +475,11 @@ def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=
                 slot.write(sim, (x.number, i))
             x.xchg.arrive(sim)
             yield ("wait", x.xchg, i & 1)
-            for g in range(2):
+            for g in range(groups):
                 maxima[i & 1][g].read(sim, (x.number, i))
 
         for i in range(tiles):
-            j = (group - i * x.jobs) & 1
+            j = (group - i * x.jobs) % groups
             assert j >= x.jobs or i * x.jobs + j == n, ("job numbering", i, j, n)
             exchanged = x.passes == 1
             while j < x.jobs:
@@ -493,8 +493,8 @@ def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=
                 if warp == 0:
                     owner[buf] = ("p" if j >= x.first_p2 else "m", n)
                 x.wg_done[buf].arrive(sim)
-                n += 2
-                j += 2
+                n += groups
+                j += groups
             if not exchanged:
                 yield from exchange(i)
             if i > 1 and softmax_waits_for_sums:
@@ -525,7 +525,7 @@ def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=
     sim.spawn("s", all_rounds(s_issuer))
     sim.spawn("pv", all_rounds(pv_issuer))
     for w in range(4):
-        for g in range(2):
+        for g in range(groups):
             sim.spawn("softmax%d%d" % (g, w), all_rounds(softmax, g, w))
         sim.spawn("epilogue%d" % w, all_rounds(epilogue, w))
     return sim.run()
