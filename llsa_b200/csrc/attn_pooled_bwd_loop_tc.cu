@@ -12,17 +12,20 @@
 // what is loaded behind its end is neither exponentiated nor multiplied.
 // The final log-sum-exp is known in the backward, so one pass over the chunks suffices.  dQ accumulates in TMEM over
 // all chunks of the tile and is then added to the fine part already in dq.
-// TMEM columns: three buffers, chunk number n of the CTA (counted over all its tiles) uses buffer n mod 3: S at 128 b,
-// dP at 128 b + 64.
-// TMEM columns: dQ of tile i at [384 + 64 (i mod 2), + 64).
+// TMEM columns, chunk number n of the CTA (counted over all its tiles): S, and dS over it, at 64 (n mod 4); dP at [256 + 64 (n mod 2), + 64); dQ of
+// tile i at [384 + 64 (i mod 2), + 64).
 // Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64): warps 8 and 11 = TMA producers (Q, dO per
 // tile, 2 stages, and K chunks; V chunks; one ring of 8 pairs), warp 9 issues S and dP, warp 10 dQ, warps 0-3 / 4-7 = two softmax
-// warpgroups on alternating chunks, warps 12-15 = epilogue, thread = row: adds dQ to the row.  The two issuing warps run
-// independently (S / dP of the next tile start while dQ of this one is still being issued); a buffer goes back to the
-// S / dP warp through buf_free, committed behind the dQ instructions that read its dS.
-// A clock trace of the form with one producer lane, the epilogue in the softmax groups and one dQ accumulator (1,050 us at two levels,
-// B=1 H=6 N=262144: 1,350 cycles a chunk, tensor pipe 576) showed the producer needing 1,130 cycles a chunk for two waits and two copies
-// and an idle tensor pipe at every tile boundary; this form needs 787 us, 757 with packed fp32 pairs.
+// warpgroups on alternating chunks, warps 12-15 = epilogue, thread = row: adds dQ to the row.  A softmax thread takes its whole row of S and
+// dP into registers at once (which is what the register split is for) and hands the dP buffer back before it begins, so that two dP buffers
+// do and S gets four.  The two issuing warps run independently (S / dP of the next tile start while dQ of this one is still being issued); an
+// S buffer goes back to the S / dP warp through buf_free, committed behind the dQ instructions that read its dS.
+// What bounds it: the loop S, dP -> dS -> dQ, 850 cycles a chunk; the tensor pipe takes 576, copies, products and hand-overs without the softmax
+// 680.  Two levels, B=1 H=6 N=262144: 757 us with three buffers for S and dP together and 32 columns loaded at a time, 680 now; l1, B=2 H=4
+// N=16384: 64.5 -> 58.5.  On the old form nothing came of three softmax groups (751), of eight warps a chunk (787), of dP handed over apart
+// from S (814); four S buffers and two of dP without the early hand-back made it 825.
+// The form with one producer lane, the epilogue in the softmax groups and one dQ accumulator (1,050 us) needed 1,130 cycles a chunk for the
+// producer's two waits and two copies and left the tensor pipe idle at every tile boundary.
 // Every mbarrier wait is bounded (abort flag; the kernel then ends early and frees its TMEM; dq is left partial).
 #include <string.h>
 
@@ -41,9 +44,11 @@ constexpr int kTile = kRows * 64;            // elements of a [128 x 64] bf16 ti
 constexpr int kChunkElems = kCk * 64;        // elements of a key chunk (8 KB)
 constexpr int kStages = 8;
 constexpr int kThreads = 512;
+constexpr int kLaunchRegs = 128, kIssueRegs = 40, kEpilogueRegs = 88, kSoftmaxRegs = 192;     // a thread's, per role: 40 + 88 + 2 x 192 = 4 x 128
+static_assert(kIssueRegs + kEpilogueRegs + 2 * kSoftmaxRegs <= 4 * kLaunchRegs, "the takers would wait for good");
 constexpr float kLog2eF = 1.4426950408889634f;
-constexpr int kBufs = 3;
-constexpr uint32_t kColDQ = 384;
+constexpr int kBufs = 4;                     // S buffers (dS over them)
+constexpr uint32_t kColDP = 256, kColDQ = 384;
 
 struct DqMaps {
   CUtensorMap q, d_o;         // [B,H,Nq,64] 4-D, box 128 rows
@@ -53,7 +58,7 @@ struct DqMaps {
 
 struct DqBars {
   uint64_t q_full[2], q_empty[2], kv_full[kStages], kv_empty[kStages];
-  uint64_t sdp_ready[kBufs], ds_ready[kBufs], buf_free[kBufs], dq_ready[2], dq_free[2];
+  uint64_t sdp_ready[kBufs], ds_ready[kBufs], buf_free[kBufs], dp_free[2], dq_ready[2], dq_free[2];
 };
 
 // jobs: 64-key chunks per tile; gathered: number of leading chunks that are gathered level-1 blocks; n_c: rows per head of the
@@ -93,6 +98,7 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&bars.dq_ready[i], 1);
       tc::mbar_init(&bars.dq_free[i], 4);
+      tc::mbar_init(&bars.dp_free[i], 4);
     }
     tc::fence_mbar_init();
   }
@@ -110,6 +116,8 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
     return left < kCk ? left : kCk;
   };
 
+  // the warps that issue copies and products leave most of their registers to the others
+  if (warp >= 8 && warp < 12) tc::regs_set<kIssueRegs, kLaunchRegs>();
   if (warp == 8 || warp == 11) {
     // ---------------------------------------------------------------- TMA producers: warp 8 Q, dO and keys, warp 11 values
     const bool vals = warp == 11;
@@ -160,14 +168,16 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
         if (!(ok = tc::warp_wait(&bars.q_full[qs], (i >> 1) & 1, abort_flag))) break;
         const uint32_t q_ = lQ + qs * kQStage, o_ = lDO + qs * kQStage;
         for (int j = 0; j < jobs; ++j) {
-          // even lanes: the chunk; odd lanes: the buffer's previous chunk (three back), whose dQ instructions have read dS
-          const bool b = (lane & 1) && cj >= kBufs;
-          if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : &bars.kv_full[st], b ? bph ^ 1 : par, abort_flag))) break;
+          // even lanes: the chunk; lanes 1, 5, ..: the S buffer's previous chunk (four back), whose dQ instructions have read dS; lanes 3, 7, ..:
+          // the dP buffer's (two back), which its group has loaded
+          const bool b = (lane & 3) == 1 && cj >= kBufs, p = (lane & 3) == 3 && cj >= 2;
+          if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : p ? &bars.dp_free[cj & 1] : &bars.kv_full[st],
+                                   b ? bph ^ 1 : p ? (uint32_t) ((cj >> 1) - 1) & 1 : par, abort_flag))) break;
           tc::fence_after_sync();
-          const uint32_t d = tmem + buf * 128;
+          const uint32_t d = tmem + buf * 64, dp = tmem + kColDP + (cj & 1) * 64;
           const uint32_t k_ = lK + st * kCStage, v_ = lV + st * kCStage;
           tc::umma_ss_k64(d, q_, hi, k_, hi, id_s);
-          tc::umma_ss_k64(d + 64, o_, hi, v_, hi, id_s);
+          tc::umma_ss_k64(dp, o_, hi, v_, hi, id_s);
           tc::umma_commit_w(&bars.sdp_ready[buf]);
           ++cj;
           if (++st == kStages) { st = 0; par ^= 1; }
@@ -193,7 +203,7 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
           const bool f = (lane & 1) && j == 0 && i > 1;
           if (!(ok = tc::warp_wait(f ? &bars.dq_free[i & 1] : &bars.ds_ready[buf], f ? ((uint32_t) (i - 2) >> 1) & 1 : bph, abort_flag))) break;
           tc::fence_after_sync();
-          const uint32_t k_ = lKm + st * kCStage, d_ = tmem + buf * 128;       // 16 key rows = 2048 bytes per k-step
+          const uint32_t k_ = lKm + st * kCStage, d_ = tmem + buf * 64;       // 16 key rows = 2048 bytes per k-step
           if (keys_of(j) == kCk) tc::umma_ts_k64(tmem + kColDQ + (i & 1) * 64, d_, k_, hi, id_dq, j > 0 ? 1u : 0u);
           else tc::umma_ts_k32(tmem + kColDQ + (i & 1) * 64, d_, k_, hi, id_dq, j > 0 ? 1u : 0u);
           tc::umma_commit_w(&bars.kv_empty[st]);
@@ -206,6 +216,7 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
       }
     }
   } else if (warp < 8) {
+    tc::regs_set<kSoftmaxRegs, kLaunchRegs>();
     // ---------------------------------------------------------------- dS; thread = query row
     const int wg = warp >> 2, qd = warp & 3, r = qd * 32 + lane;
     const float sl2 = a.scale * kLog2eF;
@@ -213,7 +224,7 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
     const uint32_t t_lane = tmem + ((uint32_t) (qd * 32) << 16);
     int buf = wg;                          // this group takes every other chunk: buffer and phase parity of its next one
     uint32_t bph = 0;
-    float vs[32], vd[32];
+    float vs[32], vs2[32], vd[32], vd2[32];
     float lse_next = 0.f, delta_next = 0.f;
     auto fetch = [&](int i) {              // this thread's row of tile i
       const int tile = blockIdx.x + i * gridDim.x;
@@ -230,28 +241,34 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
       for (int j = (int) ((wg - (int64_t) i * jobs) & 1); j < jobs; j += 2) {
         const float off = ((j < gathered || !a.two_level) ? lw1 : lw2) - L;
         const F2 off2 = f2(off, off);
-        const int halves = keys_of(j) / 32;
         ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.sdp_ready[buf], bph, abort_flag));
         tc::fence_after_sync();
         if (!ok) break;
-        const uint32_t t_b = t_lane + buf * 128;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          if (half == halves) break;
-          tc::tmem_ld32_async(t_b + 32 * half, vs);
-          tc::tmem_ld32_async(t_b + 64 + 32 * half, vd);
-          tc::tmem_ld_wait(vs);
-          tc::tmem_ld_wait(vd);
+        const uint32_t t_b = t_lane + buf * 64, t_p = t_lane + kColDP + wg * 64;
+        tc::tmem_ld32_async(t_p, vd);
+        tc::tmem_ld32_async(t_p + 32, vd2);
+        tc::tmem_ld32_async(t_b, vs);
+        tc::tmem_ld32_async(t_b + 32, vs2);
+        tc::tmem_ld_wait(vd);
+        tc::tmem_ld_wait(vd2);
+        tc::tmem_ld_wait(vs);
+        tc::tmem_ld_wait(vs2);
+        tc::fence_before_sync();                     // dP is in registers: the next but one chunk's may come
+        __syncwarp();
+        if (lane == 0) tma::mbar_arrive(&bars.dp_free[wg]);
+        auto ds_of = [&](uint32_t at, const float (&s)[32], const float (&d)[32]) {
           uint32_t pk[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             float x0, x1;
-            f2_get(f2_fma(f2(vs[2 * e], vs[2 * e + 1]), sl22, off2), x0, x1);
-            f2_get(f2_mul(f2(fast_exp2(x0), fast_exp2(x1)), f2_add(f2(vd[2 * e], vd[2 * e + 1]), nd2)), x0, x1);
+            f2_get(f2_fma(f2(s[2 * e], s[2 * e + 1]), sl22, off2), x0, x1);
+            f2_get(f2_mul(f2(fast_exp2(x0), fast_exp2(x1)), f2_add(f2(d[2 * e], d[2 * e + 1]), nd2)), x0, x1);
             pk[e] = pack_bf16(x0, x1);
           }
-          tc::tmem_st16(t_b + 16 * half, pk);          // dS columns [16 half, 16 half + 16) over S columns read before
-        }
+          tc::tmem_st16(at, pk);
+        };
+        ds_of(t_b, vs, vd);                          // dS over S; where the list ends after 32 keys, the products stop there
+        ds_of(t_b + 16, vs2, vd2);
         tc::tmem_st_wait();
         tc::fence_before_sync();
         __syncwarp();
@@ -261,6 +278,7 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
       }
     }
   } else {
+    tc::regs_set<kEpilogueRegs, kLaunchRegs>();
     // ---------------------------------------------------------------- dq += dQ; thread = query row
     const int qd = warp & 3, r = qd * 32 + lane;
     bool ok = true;
@@ -275,34 +293,33 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
       tc::fence_after_sync();
       if (!ok) break;
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        float v[32];
-        uint4 rest[4];
+      for (int part = 0; part < 4; ++part) {
+        float v[16];
+        uint4 rest[2];
         if (REM) {
-          const uint4* rp = reinterpret_cast<const uint4*>(a.rem + ((int64_t) bh * a.Nq + row) * kD + half * 32);
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) rest[q4] = rp[q4];
+          const uint4* rp = reinterpret_cast<const uint4*>(a.rem + ((int64_t) bh * a.Nq + row) * kD + part * 16);
+          rest[0] = rp[0];
+          rest[1] = rp[1];
         }
-        tc::tmem_ld32_async(tmem + kColDQ + (i & 1) * 64 + half * 32 + ((uint32_t) (qd * 32) << 16), v);
-        tc::tmem_ld_wait(v);
-        if (half == 1) {
+        tc::tmem_ld16(tmem + kColDQ + (i & 1) * 64 + part * 16 + ((uint32_t) (qd * 32) << 16), v);
+        if (part == 3) {
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tma::mbar_arrive(&bars.dq_free[i & 1]);
         }
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const uint4 f = old[half * 4 + q4];
+        for (int q2 = 0; q2 < 2; ++q2) {
+          const uint4 f = old[part * 2 + q2];
           auto sum = [&](uint32_t fine, uint32_t left, int e) {
             const float x = REM ? bf16_lo(fine) + bf16_lo(left) : bf16_lo(fine), y = REM ? bf16_hi(fine) + bf16_hi(left) : bf16_hi(fine);
-            return pack_bf16(fmaf(v[8 * q4 + e], a.scale, x), fmaf(v[8 * q4 + e + 1], a.scale, y));
+            return pack_bf16(fmaf(v[8 * q2 + e], a.scale, x), fmaf(v[8 * q2 + e + 1], a.scale, y));
           };
           uint4 w;
-          w.x = sum(f.x, rest[q4].x, 0);
-          w.y = sum(f.y, rest[q4].y, 2);
-          w.z = sum(f.z, rest[q4].z, 4);
-          w.w = sum(f.w, rest[q4].w, 6);
-          *reinterpret_cast<uint4*>(dqrow + half * 32 + 8 * q4) = w;
+          w.x = sum(f.x, rest[q2].x, 0);
+          w.y = sum(f.y, rest[q2].y, 2);
+          w.z = sum(f.z, rest[q2].z, 4);
+          w.w = sum(f.w, rest[q2].w, 6);
+          *reinterpret_cast<uint4*>(dqrow + part * 16 + 8 * q2) = w;
         }
       }
     }
@@ -342,7 +359,7 @@ int launch_attn_dq_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, i
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) (4 * kTile + 2 * kStages * kChunkElems) * sizeof(bf16);
   auto kernel = a.rem ? attn_dq_pooled_loop_tc_kernel<true> : attn_dq_pooled_loop_tc_kernel<false>;
-  LLSA_SMEM_LIMIT(kernel, smem);
+  LLSA_SMEM_LIMIT_REGS(kernel, smem, kLaunchRegs);
   launch_pdl(kernel, grid, kThreads, smem, st, a, maps, jobs, gathered, n_c, n_tiles, tiles_per_head);
   LLSA_LAUNCH_OK("attn_dq_pooled_loop_tc_kernel");
   return LLSA_OK;

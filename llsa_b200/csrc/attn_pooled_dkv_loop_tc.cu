@@ -19,15 +19,19 @@
 // multiple of 32 keys) hold a repeated block or the rows that follow in memory; their results stay in their own rows and are dropped.
 // Work split: all (head, chunk, job) triples in that order form one flat list that is cut into gridDim.x equal pieces,
 // one per CTA; a piece is one to a few units (it changes unit where it crosses a chunk boundary).
-// TMEM columns: NB buffers, job number n of the CTA uses buffer n mod NB: S^T at 128 b, dP^T at 128 b + 64; then NA accumulators, unit number
-// i of the CTA uses i mod NA: dV, dK (64 columns each).  Dense units are hundreds of jobs long: NB = 3, NA = 1.  Gathered units are
-// four jobs long: NB = 2, NA = 2, so that a unit's first products do not wait for the last one's results to be read.
+// TMEM columns, job number n and unit number i of the CTA.  Dense units are hundreds of jobs long: S^T, and P^T and dS^T over it (queries 0..31
+// at 0 and 16, 32..63 at 32 and 48), at 64 (n mod 4); dP^T at 256 + 64 (n mod 2), handed back as soon as its group has it in registers; one pair of
+// accumulators dV, dK at 384.  Gathered units are four jobs long: two buffers of S^T and dP^T (overwritten by P^T and dS^T) at 128 (n mod 2), two
+// pairs of accumulators at 256 + 128 (i mod 2), so that a unit's first products do not wait for the last one's results to be read.
 // Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64): warps 8 and 11 = TMA producers (K_c, V_c
 // per unit in two stages, Q_t per job; dO_t, lse, delta per job; a ring of 8), warp 9 issues S^T and dP^T, warp 10 dV and dK,
 // warps 0-3 / 4-7 = two softmax warpgroups on alternating jobs, warps 12-15 write a unit's dV and dK, thread = key row.  Every mbarrier
 // wait is bounded (abort flag, TMEM freed).
-// Two levels, B=1 H=6 N=262144 (tensor pipe 768 cycles a job): with one producer lane and results written by the softmax groups 1,010 us
-// dense, 315 gathered; this form needs 916 (856 with packed fp32 pairs) and 268.
+// What bounds them.  Dense, tensor pipe 768 cycles a job: the loop S^T, dP^T -> P^T, dS^T -> dV, dK, 1,170 cycles; copies, products and hand-overs
+// without the softmax 930.  Two levels, B=1 H=6 N=262144: 870 us with three buffers for both and 32 columns loaded at a time, 830 now; l1, B=2 H=4
+// N=16384: 85 -> 79.5.  Three softmax groups change nothing (866), eight warps a job spill (1,165).  Gathered: the fp32 reductions, 100 M at
+// the same size; 263 us with results read from tensor memory 32 columns at a time, 241 with 16 (top-16, H=5 N=40960: 71 -> 65); in the dense
+// form's layout 254 to 270.
 #include <string.h>
 
 #include "attn.cuh"
@@ -45,6 +49,8 @@ constexpr int kKeyTile = kKeys * 64;         // elements of the K / V chunk (16 
 constexpr int kQTile = kQ * 64;              // elements of a Q / dO job tile (8 KB)
 constexpr int kStages = 8;
 constexpr int kThreads = 512;
+constexpr int kLaunchRegs = 128, kIssueRegs = 56, kEpilogueRegs = 88, kSoftmaxRegs = 184;     // a thread's, per role: 56 + 88 + 2 x 184 = 4 x 128
+static_assert(kIssueRegs + kEpilogueRegs + 2 * kSoftmaxRegs <= 4 * kLaunchRegs, "the takers would wait for good");
 constexpr float kLog2eF = 1.4426950408889634f;
 
 struct KvMaps {
@@ -53,7 +59,7 @@ struct KvMaps {
 };
 
 struct KvBars {
-  uint64_t kv_full[2], kv_empty[2], q_full[kStages], q_empty[kStages], sdp_ready[3], pds_ready[3], buf_free[3], acc_ready[2], acc_free[2];
+  uint64_t kv_full[2], kv_empty[2], q_full[kStages], q_empty[kStages], sdp_ready[4], pds_ready[4], buf_free[4], dp_free[2], acc_ready[2], acc_free[2];
 };
 
 // A CTA's piece of the flat job list, walked unit by unit.
@@ -92,8 +98,8 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
   bf16* sV = sK + 2 * kKeyTile;              // [2][128][64]
   bf16* sQ = sV + 2 * kKeyTile;              // [kStages][64][64]
   bf16* sDO = sQ + kStages * kQTile;         // [kStages][64][64]
-  constexpr int kBufs = GATHER ? 2 : 3, kAccs = GATHER ? 2 : 1;
-  constexpr uint32_t kColAcc = kBufs * 128;
+  constexpr int kBufs = GATHER ? 2 : 4, kAccs = GATHER ? 2 : 1;
+  constexpr uint32_t kBufCols = GATHER ? 128 : 64, kColDP = 256, kColAcc = GATHER ? 256 : 384;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile tc::WaitCtl* abort_flag = &s_ctl;
 
@@ -107,6 +113,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       tc::mbar_init(&bars.pds_ready[i], 4);
       tc::mbar_init(&bars.buf_free[i], 1);
     }
+    for (int i = 0; i < 2; ++i) tc::mbar_init(&bars.dp_free[i], 4);
     for (int i = 0; i < kAccs; ++i) { tc::mbar_init(&bars.acc_ready[i], 1); tc::mbar_init(&bars.acc_free[i], 4); }
     tc::fence_mbar_init();
   }
@@ -120,6 +127,8 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
   const int units_per_head = GATHER ? chunks * (int) a.nq2 : chunks;
   Piece pc((int64_t) n_base * jobs_all, jobs_all);
 
+  // the warps that issue copies and products leave most of their registers to the others
+  if (!GATHER && warp >= 8 && warp < 12) tc::regs_set<kIssueRegs, kLaunchRegs>();
   if (warp == 8 || warp == 11) {
     // ---------------------------------------------------------------- TMA producers: warp 8 the unit's keys and Q, warp 11 dO, lse, delta
     const bool second = warp == 11;
@@ -179,13 +188,15 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
         const uint32_t k_ = lK + ks * kKeyStage, v_ = lV + ks * kKeyStage;
         for (int j = 0; j < pc.n; ++j, ++cj) {
           const int st = cj & (kStages - 1);
-          // even lanes: the query tile; odd lanes: the buffer's previous job (kBufs back), whose P^T / dS^T have been read
-          const bool b = (lane & 1) && cj >= kBufs;
-          if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : &bars.q_full[st], b ? bph ^ 1 : (uint32_t) (cj / kStages) & 1, abort_flag))) break;
+          // even lanes: the query tile; lanes 1, 5, ..: the S^T buffer's previous job (kBufs back), whose P^T / dS^T have been read; lanes 3,
+          // 7, ..: the dP^T buffer's (two back), which its group has loaded
+          const bool b = (lane & 3) == 1 && cj >= kBufs, p = !GATHER && (lane & 3) == 3 && cj >= 2;
+          if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : p ? &bars.dp_free[cj & 1] : &bars.q_full[st],
+                                   b ? bph ^ 1 : p ? (uint32_t) ((cj >> 1) - 1) & 1 : (uint32_t) (cj / kStages) & 1, abort_flag))) break;
           tc::fence_after_sync();
-          const uint32_t d = tmem + buf * 128, q_ = lQ + st * kQStage, o_ = lDO + st * kQStage;
+          const uint32_t d = tmem + buf * kBufCols, dp = GATHER ? d + 64 : tmem + kColDP + (cj & 1) * 64, q_ = lQ + st * kQStage, o_ = lDO + st * kQStage;
           tc::umma_ss_k64(d, k_, hi, q_, hi, id_s);
-          tc::umma_ss_k64(d + 64, v_, hi, o_, hi, id_s);
+          tc::umma_ss_k64(dp, v_, hi, o_, hi, id_s);
           tc::umma_commit_w(&bars.sdp_ready[buf]);
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
         }
@@ -212,9 +223,16 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
           if (!(ok = tc::warp_wait(f ? &bars.acc_free[i % kAccs] : &bars.pds_ready[buf], f ? (uint32_t) (i / kAccs - 1) & 1 : bph, abort_flag))) break;
           tc::fence_after_sync();
           // 4 k-steps of 16 query rows (2048 bytes of the MN-major dO / Q tile)
-          const uint32_t o_ = lDOm + st * kQStage, q_ = lQm + st * kQStage, b = tmem + buf * 128, acc = tmem + kColAcc + (i % kAccs) * 128;
-          tc::umma_ts_k64(acc, b, o_, hi, id_o, j > 0 ? 1u : 0u);
-          tc::umma_ts_k64(acc + 64, b + 64, q_, hi, id_o, j > 0 ? 1u : 0u);
+          const uint32_t o_ = lDOm + st * kQStage, q_ = lQm + st * kQStage, b = tmem + buf * kBufCols, acc = tmem + kColAcc + (i % kAccs) * 128;
+          if (GATHER) {
+            tc::umma_ts_k64(acc, b, o_, hi, id_o, j > 0 ? 1u : 0u);
+            tc::umma_ts_k64(acc + 64, b + 64, q_, hi, id_o, j > 0 ? 1u : 0u);
+          } else {                             // the first 32 queries' P^T, dS^T lie in the buffer's columns 0 and 16, the others' in 32 and 48
+            tc::umma_ts_k32(acc, b, o_, hi, id_o, j > 0 ? 1u : 0u);
+            tc::umma_ts_k32(acc, b + 32, o_ + 256, hi, id_o, 1u);
+            tc::umma_ts_k32(acc + 64, b + 16, q_, hi, id_o, j > 0 ? 1u : 0u);
+            tc::umma_ts_k32(acc + 64, b + 48, q_ + 256, hi, id_o, 1u);
+          }
           tc::umma_commit_w(&bars.q_empty[st]);
           tc::umma_commit_w(&bars.buf_free[buf]);
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
@@ -224,6 +242,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       }
     }
   } else if (warp < 8) {
+    if (!GATHER) tc::regs_set<kSoftmaxRegs, kLaunchRegs>();
     // ---------------------------------------------------------------- P^T / dS^T; thread = key row
     const int wg = warp >> 2, qd = warp & 3;
     const float sl2 = a.scale * kLog2eF;
@@ -238,16 +257,12 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       const bool ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.sdp_ready[buf], bph, abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
-      const uint32_t t_b = t_lane + buf * 128;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        tc::tmem_ld32_async(t_b + 32 * half, vs);
-        tc::tmem_ld32_async(t_b + 64 + 32 * half, vd);
-        tc::tmem_ld_wait(vs);
-        tc::tmem_ld_wait(vd);
+      const uint32_t t_b = t_lane + buf * kBufCols, t_p = GATHER ? t_b + 64 : t_lane + kColDP + wg * 64;
+      // P^T and dS^T of 32 query columns
+      auto half_of = [&](int half, const float (&s)[32], const float (&d)[32], uint32_t to_p, uint32_t to_ds) {
         uint32_t pp[16], pd[16];
 #pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) {           // 4 query columns at a time: their lse / delta are broadcast reads
+        for (int q4 = 0; q4 < 8; ++q4) {             // 4 query columns at a time: their lse / delta are broadcast reads
           const float4 l4 = *reinterpret_cast<const float4*>(&s_lse[st][32 * half + 4 * q4]);
           const float4 d4 = *reinterpret_cast<const float4*>(&s_delta[st][32 * half + 4 * q4]);
 #pragma unroll
@@ -255,16 +270,41 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
             const F2 l2 = e ? f2(l4.z, l4.w) : f2(l4.x, l4.y), d2 = e ? f2(d4.z, d4.w) : f2(d4.x, d4.y);
             const int k = 4 * q4 + 2 * e;
             float x0, x1;
-            f2_get(f2_fma(f2(vs[k], vs[k + 1]), sl22, f2_fma(l2, nlog2e2, lw2)), x0, x1);
+            f2_get(f2_fma(f2(s[k], s[k + 1]), sl22, f2_fma(l2, nlog2e2, lw2)), x0, x1);
             x0 = fast_exp2(x0);
             x1 = fast_exp2(x1);
             pp[2 * q4 + e] = pack_bf16(x0, x1);
-            f2_get(f2_mul(f2(x0, x1), f2_fma(d2, minus1, f2(vd[k], vd[k + 1]))), x0, x1);
+            f2_get(f2_mul(f2(x0, x1), f2_fma(d2, minus1, f2(d[k], d[k + 1]))), x0, x1);
             pd[2 * q4 + e] = pack_bf16(x0, x1);
           }
         }
-        tc::tmem_st16(t_b + 16 * half, pp);            // P^T over S^T columns read before
-        tc::tmem_st16(t_b + 64 + 16 * half, pd);       // dS^T over dP^T columns read before
+        tc::tmem_st16(to_p, pp);                     // over columns read before
+        tc::tmem_st16(to_ds, pd);
+      };
+      if constexpr (GATHER) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          tc::tmem_ld32_async(t_b + 32 * half, vs);
+          tc::tmem_ld32_async(t_p + 32 * half, vd);
+          tc::tmem_ld_wait(vs);
+          tc::tmem_ld_wait(vd);
+          half_of(half, vs, vd, t_b + 16 * half, t_p + 16 * half);
+        }
+      } else {
+        float vs2[32], vd2[32];
+        tc::tmem_ld32_async(t_p, vd);
+        tc::tmem_ld32_async(t_p + 32, vd2);
+        tc::tmem_ld32_async(t_b, vs);
+        tc::tmem_ld32_async(t_b + 32, vs2);
+        tc::tmem_ld_wait(vd);
+        tc::tmem_ld_wait(vd2);
+        tc::tmem_ld_wait(vs);
+        tc::tmem_ld_wait(vs2);
+        tc::fence_before_sync();                     // dP^T is in registers: the next but one job's may come
+        __syncwarp();
+        if (lane == 0) tma::mbar_arrive(&bars.dp_free[wg]);
+        half_of(0, vs, vd, t_b, t_b + 16);
+        half_of(1, vs2, vd2, t_b + 32, t_b + 48);
       }
       tc::tmem_st_wait();
       tc::fence_before_sync();
@@ -278,6 +318,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       }
     }
   } else {
+    if (!GATHER) tc::regs_set<kEpilogueRegs, kLaunchRegs>();
     // ---------------------------------------------------------------- results of a unit; thread = key row
     const int qd = warp & 3, r = qd * 32 + lane;
     for (int i = 0; pc.next(); ++i) {
@@ -297,25 +338,24 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       tc::fence_after_sync();
       if (!ok) break;
 #pragma unroll
-      for (int part = 0; part < 4; ++part) {
-        float v[32];
-        tc::tmem_ld32_async(tmem + kColAcc + (i % kAccs) * 128 + part * 32 + ((uint32_t) (qd * 32) << 16), v);
-        tc::tmem_ld_wait(v);
-        if (part == 3) {
+      for (int part = 0; part < 8; ++part) {
+        float v[16];
+        tc::tmem_ld16(tmem + kColAcc + (i % kAccs) * 128 + part * 16 + ((uint32_t) (qd * 32) << 16), v);
+        if (part == 7) {
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tma::mbar_arrive(&bars.acc_free[i % kAccs]);
         }
-        const float mul = part < 2 ? out_mul : out_mul * a.scale;
-        float* dst = (part < 2 ? dpv : dpk) + ((int64_t) bh * n_keys + key) * kD + (part & 1) * 32;
+        const float mul = part < 4 ? out_mul : out_mul * a.scale;
+        float* dst = (part < 4 ? dpv : dpk) + ((int64_t) bh * n_keys + key) * kD + (part & 3) * 16;
         if (!live) {
         } else if (whole) {
 #pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4)
+          for (int q4 = 0; q4 < 4; ++q4)
             *reinterpret_cast<float4*>(dst + 4 * q4) = make_float4(v[4 * q4] * mul, v[4 * q4 + 1] * mul, v[4 * q4 + 2] * mul, v[4 * q4 + 3] * mul);
         } else {
 #pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4) red_add_v4(dst + 4 * q4, v[4 * q4] * mul, v[4 * q4 + 1] * mul, v[4 * q4 + 2] * mul, v[4 * q4 + 3] * mul);
+          for (int q4 = 0; q4 < 4; ++q4) red_add_v4(dst + 4 * q4, v[4 * q4] * mul, v[4 * q4 + 1] * mul, v[4 * q4 + 2] * mul, v[4 * q4 + 3] * mul);
         }
       }
     }
@@ -349,7 +389,7 @@ int launch_attn_dkv_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
     if ((rc = tma::make_map_rows(&maps.v, a.two_level ? a.pv2 : a.pv, (uint64_t) BH * n_dense, kKeys))) return rc;
     const int chunks = (int) ((n_dense + kKeys - 1) / kKeys), jobs = (int) (a.Nq / kQ), units = (int) BH * chunks;
     const float w = a.two_level ? a.w2 : a.w1, kvw = a.two_level ? a.kvw2 : a.kvw1;
-    LLSA_SMEM_LIMIT((attn_dkv_pooled_loop_tc_kernel<false>), smem);
+    LLSA_SMEM_LIMIT_REGS((attn_dkv_pooled_loop_tc_kernel<false>), smem, kLaunchRegs);
     launch_pdl(attn_dkv_pooled_loop_tc_kernel<false>, grid_of((int64_t) units * jobs), kThreads, smem, st, 
         a, maps, a.two_level ? a.dpk2 : a.dpk, a.two_level ? a.dpv2 : a.dpv, n_dense, jobs, units, chunks, log2f(w), kvw / w);
     LLSA_LAUNCH_OK("attn_dkv_pooled_loop_tc_kernel");

@@ -135,14 +135,18 @@ def _bars(name, n, count):
     return [Barrier("%s%d" % (name, i), count) for i in range(n)]
 
 
-def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8, buffers=3, accs=1, full_count=2):
+def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8, buffers=None, accs=1, full_count=2):
     """attn_dkv_pooled_loop_tc_kernel.  `units`: job counts of the units of one CTA's piece: (head, chunk) units in the dense form
-    (three S^T / dP^T buffers, one pair of accumulators), units of four jobs and fewer in the gathered one (buffers=2, accs=2).
+    (four S^T buffers, which P^T and dS^T overwrite, one pair of accumulators), units of four jobs and fewer in the gathered one (buffers=2,
+    accs=2); two dP^T buffers, handed back as soon as their group has loaded them.  Two score threads share three S^T buffers.
     score_threads: threads that issue S^T / dP^T (1 = the kernel; 2 = even and odd jobs on two threads).
     score_barriers: sdp_ready / buf_free barriers (None = one per buffer, the kernel; 6 = one per job number mod 6).
     full_count: producers a query stage waits for (2 = the kernel: Q, and dO with lse and delta; 1 breaks the protocol on purpose)."""
     sim = Sim(seed)
+    buffers = buffers or (4 if score_threads == 1 else 3)
     nb = score_barriers or buffers
+    dp = [Resource("dP^T buffer %d" % i) for i in range(2)]
+    dp_free = _bars("dp_free", 2, 4)
     kv_full, kv_empty = _bars("kv_full", 2, 1), _bars("kv_empty", 2, score_threads)
     q_full, q_empty = _bars("q_full", stages, full_count), _bars("q_empty", stages, 1)
     sdp, pds, free = _bars("sdp_ready", nb, 1), _bars("pds_ready", buffers, 4), _bars("buf_free", nb, 1)
@@ -180,6 +184,8 @@ def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8
                 if job >= buffers:
                     prev = job - buffers
                     wait += [free[prev % nb], (prev // nb) & 1]
+                if job >= 2:
+                    wait += [dp_free[job & 1], ((job >> 1) - 1) & 1]
                 yield tuple(wait)
                 if sim.rng.random() < 0.15:
                     yield ("delay", sim.r(500, 4000))          # one thread falls behind the other
@@ -189,6 +195,7 @@ def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8
                 for t in tiles.values():
                     t[st].read(sim, job, done)
                 sim.at(done, (lambda b=buf, j=job: owner.__setitem__(b, ("s", j))))
+                dp[job & 1].write(sim, job, at=done)
                 yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
                 sim.commit(("score", mine), sdp[job % nb])
                 yield ("delay", sim.r(30, 80))
@@ -226,6 +233,9 @@ def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8
             buf = job % buffers
             yield ("wait", sdp[job % nb], (job // nb) & 1)
             assert owner[buf] is not None and owner[buf][1] == job, ("softmax read", buf, owner[buf], job)
+            yield ("delay", sim.r(100, 400))
+            dp[job & 1].read(sim, job)
+            dp_free[job & 1].arrive(sim)
             yield ("delay", sim.r(500, 1200))
             if warp == 0:
                 owner[buf] = ("p", job)
@@ -252,12 +262,16 @@ def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8
     return sim.run()
 
 
-def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=3, stages=8, buffers=3, free_count=4):
+def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=None, stages=8, buffers=None, free_count=4):
     """attn_dq_pooled_loop_tc_kernel: `tiles` query tiles of `jobs` key chunks; Q / dO in two stages, K and V chunks (two
-    producers) in one ring of pairs, S / dP into three buffers, dQ of a tile into one of two accumulators, read by epilogue warps.
+    producers) in one ring of pairs, S into four buffers (three with two score threads), which dS overwrites, dP into two, handed back as soon
+    as their group has loaded them, dQ of a tile into one of two accumulators, read by epilogue warps.
     free_count: epilogue warps an accumulator waits for (4 = the kernel; 1 breaks the protocol on purpose)."""
     sim = Sim(seed)
-    nb = score_barriers
+    buffers = buffers or (4 if score_threads == 1 else 3)
+    nb = score_barriers or buffers
+    dp = [Resource("dP buffer %d" % i) for i in range(2)]
+    dp_free = _bars("dp_free", 2, 4)
     q_full, q_empty = _bars("q_full", 2, 1), _bars("q_empty", 2, score_threads)
     kv_full, kv_empty = _bars("kv_full", stages, 2), _bars("kv_empty", stages, 1)
     sdp, ds, free = _bars("sdp_ready", nb, 1), _bars("ds_ready", buffers, 4), _bars("buf_free", nb, 1)
@@ -293,6 +307,8 @@ def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=3, sta
                 if job >= buffers:
                     prev = job - buffers
                     wait += [free[prev % nb], (prev // nb) & 1]
+                if job >= 2:
+                    wait += [dp_free[job & 1], ((job >> 1) - 1) & 1]
                 yield tuple(wait)
                 if sim.rng.random() < 0.15:
                     yield ("delay", sim.r(500, 4000))
@@ -302,6 +318,7 @@ def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=3, sta
                 for r in ring.values():
                     r[st].read(sim, job, done)
                 sim.at(done, (lambda b=buf, j=job: owner.__setitem__(b, ("s", j))))
+                dp[job & 1].write(sim, job, at=done)
                 yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
                 sim.commit(("score", mine), sdp[job % nb])
                 yield ("delay", sim.r(30, 80))
@@ -337,6 +354,9 @@ def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=3, sta
             buf = job % buffers
             yield ("wait", sdp[job % nb], (job // nb) & 1)
             assert owner[buf] is not None and owner[buf][1] == job, ("softmax read", buf, owner[buf], job)
+            yield ("delay", sim.r(100, 400))
+            dp[job & 1].read(sim, job)
+            dp_free[job & 1].arrive(sim)
             yield ("delay", sim.r(400, 1000))
             if warp == 0:
                 owner[buf] = ("p", job)
