@@ -34,8 +34,8 @@
 // before the exponentials (732: fewer warps for the MUFU), eight warps a job (657 long lists, 56 -> 58 short ones), a
 // quarter or a third of the exponentials as a degree-5 polynomial on the FMA pipe (669 and 676; 85 -> 95 and 98 at N=65536 two levels).  In the form with one producer lane, the epilogue in the softmax groups and one O buffer
 // (785 us) the producer needed 1,300 cycles a job for its two waits and two copies, and every tile boundary cost 5,900 idle cycles.
-// Every mbarrier wait is bounded; a wait that expires raises a CTA-wide abort flag, every role leaves its loops, lse of every row of the CTA
-// that is not finished (or was marked: a second round may have been cut short) becomes NaN and TMEM is freed.
+// Every mbarrier wait is bounded; a wait that expires raises a CTA-wide abort flag, every role leaves its loops, the epilogue puts NaN into lse of
+// every row of the CTA (poison_lse) and TMEM is freed.
 #include <string.h>
 
 #include "attn.cuh"
@@ -381,10 +381,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.sum_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
         ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
         tc::fence_after_sync();
-        if (!ok) {
-          if (mine) *lse_p = __int_as_float(0x7fc00000);             // NaN: not completed, nor will the tiles behind it be
-          continue;
-        }
+        if (!ok) break;
         const float lsum = s_sum[i & 1][0][r] + s_sum[i & 1][1][r] + s_sum[i & 1][2][r], mx = s_ref[i & 1][r];
         // one pass: the row is this round's unless its sum left the safe range (false for NaN too): the mark hands it to the second
         if (redo && n_pass == 1) {
@@ -432,16 +429,11 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         if (mine) *lse_p = (Lm + log2f(ef + ep)) * 0.6931471805599453f;
       }
     });
-    // after an abort no second round comes, or not all of it: the rows left to it still hold the fine part
-    if (redo && abort_flag->abort) {
-      for (int i = 0; i < n_my; ++i) {
-        const int tile = blockIdx.x + i * gridDim.x;
-        const int64_t at = (int64_t) (tile / tiles_per_head) * a.Nq + (tile % tiles_per_head) * kRows + (warp & 3) * 32 + lane;
-        if (redo[at]) a.lse[at] = __int_as_float(0x7fc00000);
-      }
-    }
   }
-  if (abort_flag->abort) tc::abort_drain();
+  if (abort_flag->abort) {
+    tc::abort_drain();
+    if (warp >= 12 && warp < 16) poison_lse(a.lse, blockIdx.x, gridDim.x, n_tiles);
+  }
   __syncthreads();
   if (threadIdx.x == 0 && abort_flag->abort && a.status) atomicOr(a.status, (int) LLSA_DEV_WAIT_EXPIRED);
   if (warp == 0) tc::tmem_dealloc(tmem, 512);

@@ -26,7 +26,7 @@
 // tcgen05.mma operations of one thread execute in issue order, which is what lets S of tile i+2
 // reuse the buffer of tile i right behind P.PV of tile i without a barrier.
 // All mbarrier waits are bounded; a wait that expires raises a CTA-wide abort flag, every
-// role leaves its loop, lse of the unfinished rows is poisoned with NaN and TMEM is freed.
+// role leaves its loop, lse of every row of the CTA becomes NaN (poison_lse) and TMEM is freed.
 #include <string.h>
 
 #include "attn.cuh"
@@ -167,7 +167,6 @@ attn_fwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ TcMaps maps, in
     const float sl2 = a.scale * 1.4426950408889634f;
     const float lw1 = log2f(a.w1), lw2 = log2f(a.w2);
     const uint32_t t_s = tmem + wg * 256 + ((uint32_t) ((warp & 3) * 32) << 16), t_o = t_s + np;
-    bool ok = true;                              // stays false: the tiles behind an unfinished one are not finished either
     for (int i = wg; i < n_my; i += 2) {
       const int tile = blockIdx.x + i * gridDim.x, u = i >> 1;
       const int64_t bh = tile / tiles_per_head, row = (int64_t) (tile % tiles_per_head) * kTcRows + r_tile;
@@ -179,7 +178,7 @@ attn_fwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ TcMaps maps, in
       for (int q = 0; q < 8; ++q) of[q] = *reinterpret_cast<const uint4*>(orow + 8 * q);
       const float lse_f = a.lse[bh * a.Nq + row];
       // `ok` is kept warp-uniform: the TMEM accesses below are warp-wide instructions
-      ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.s_ready[wg], u & 1, abort_flag));
+      bool ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.s_ready[wg], u & 1, abort_flag));
       tc::fence_after_sync();
       float mx = 0.f, lsum = 0.f;
       float va[32], vb[32];
@@ -265,9 +264,13 @@ attn_fwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ TcMaps maps, in
         merge(vb, 32);
       }
       a.lse[bh * a.Nq + row] = lse_out;
+      if (!ok) break;
     }
   }
-  if (abort_flag->abort) tc::abort_drain();
+  if (abort_flag->abort) {
+    tc::abort_drain();
+    if (warp < 8) poison_lse(a.lse, blockIdx.x + (warp >> 2) * gridDim.x, 2 * gridDim.x, n_tiles);
+  }
   tc::fence_before_sync();
   __syncthreads();
   if (threadIdx.x == 0 && abort_flag->abort && a.status) atomicOr(a.status, (int) LLSA_DEV_WAIT_EXPIRED);
