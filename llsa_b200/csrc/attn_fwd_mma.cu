@@ -320,6 +320,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) attn_fwd_fine_kernel(AttnP<b
     if (!ok) break;
   }
   if (!ok) {
+    if (lane < kBS) a.lse[bh * a.Nq + qb * kBS + lane] = __int_as_float(0x7fc00000);      // NaN: not completed; the pooled stage passes it on
     tc::abort_drain();
     if (lane == 0 && a.status) atomicOr(a.status, (int) LLSA_DEV_WAIT_EXPIRED);
     return;

@@ -1,6 +1,6 @@
 """What a forward leaves behind whose bounded mbarrier waits run out (forced here by a poll limit of a few looks): with device checks off, a NaN in
-lse is the only sign of it, so every row must hold its final value or NaN.  The fine part's own lse, which the pooled stage finds there, looks
-plausible and is neither."""
+lse is the only sign of it, so every row must hold its final value or NaN.  The fine part's own lse, which the pooled stage finds there, and what
+an earlier call left in that memory look plausible and are neither."""
 import pytest
 import torch
 
@@ -50,3 +50,9 @@ def test_rows_marked_for_a_round_that_an_expired_wait_cuts_short_are_nan(limit, 
     x = [(q.float() * 12).to(DEV, torch.bfloat16), (k.float() * 12).to(DEV, torch.bfloat16), v.to(DEV)]
     _check(2, x, limit, monkeypatch)
     assert int(ops._last_fwd_redo.view(torch.uint8)[:2 * 65536].sum()) > 0
+
+
+@pytest.mark.parametrize("levels,B,H,N", [(1, 2, 4, 16384), (2, 1, 2, 65536), (2, 2, 6, 16384)])
+def test_every_row_behind_an_expired_wait_of_the_fine_forward_is_nan(levels, B, H, N, monkeypatch):
+    """A limit of one: most of the fine forward's copies have not landed at the first look, and nothing writes those rows."""
+    assert _check(levels, _inputs(levels, B, H, N), 1, monkeypatch) > 0
