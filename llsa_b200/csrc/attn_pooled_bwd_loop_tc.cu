@@ -49,6 +49,11 @@ static_assert(kIssueRegs + kEpilogueRegs + 2 * kSoftmaxRegs <= 4 * kLaunchRegs, 
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr int kBufs = 4;                     // S buffers (dS over them)
 constexpr uint32_t kColDP = 256, kColDQ = 384;
+// Up to this many chunks a tile the epilogue is the pace, and the first half of a row's remainder is requested with the fine part, ahead of the
+// wait; beyond, the softmax is, and the remainder is better left until it is needed, a quarter of a row at a time.  Backward in us, ahead / a
+// quarter at a time: 1 chunk (one level, B=2 H=6 N=1024) 45.4 / 46.4, 4 (two levels, top-8 parents, H=6 N=24576) 211 / 214, 5 (H=5 N=40960)
+// 287 / 290, 6 (top-16 parents, H=6 N=24576) 242 / 239, 7 (H=5 N=40960) 391 / 384, 17 (one level, B=2 H=6 N=16896) 383 / 375.
+constexpr int kAheadJobs = 5;
 
 struct DqMaps {
   CUtensorMap q, d_o;         // [B,H,Nq,64] 4-D, box 128 rows
@@ -62,8 +67,8 @@ struct DqBars {
 };
 
 // jobs: 64-key chunks per tile; gathered: number of leading chunks that are gathered level-1 blocks; n_c: rows per head of the
-// contiguous pooled tensor.  REM: the fine part of dq is the bf16 value in dq plus its remainder in a.rem.
-template <bool REM>
+// contiguous pooled tensor.  REM: the fine part of dq is the bf16 value in dq plus its remainder in a.rem.  AHEAD: jobs <= kAheadJobs.
+template <bool REM, bool AHEAD>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps, int jobs, int gathered, int64_t n_c, int n_tiles,
                               int tiles_per_head) {
@@ -286,20 +291,23 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
       const int tile = blockIdx.x + i * gridDim.x;
       const int bh = tile / tiles_per_head, row = (tile % tiles_per_head) * kRows + r;
       bf16* dqrow = a.dq.row(bh / a.H, bh % a.H, row);
-      uint4 old[8];                        // the fine part: requested before the wait
+      uint4 old[8], rest[4];               // the fine part, requested before the wait, and half a row of its remainder
+      const uint4* rp = REM ? reinterpret_cast<const uint4*>(a.rem + ((int64_t) bh * a.Nq + row) * kD) : nullptr;
 #pragma unroll
       for (int q8 = 0; q8 < 8; ++q8) old[q8] = *reinterpret_cast<const uint4*>(dqrow + 8 * q8);
+      if (REM && AHEAD) {
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4) rest[q4] = rp[q4];
+      }
       ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.dq_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
 #pragma unroll
       for (int part = 0; part < 4; ++part) {
         float v[16];
-        uint4 rest[2];
-        if (REM) {
-          const uint4* rp = reinterpret_cast<const uint4*>(a.rem + ((int64_t) bh * a.Nq + row) * kD + part * 16);
-          rest[0] = rp[0];
-          rest[1] = rp[1];
+        if (REM && !AHEAD) {
+          rest[(part & 1) * 2] = rp[part * 2];
+          rest[(part & 1) * 2 + 1] = rp[part * 2 + 1];
         }
         tc::tmem_ld16(tmem + kColDQ + (i & 1) * 64 + part * 16 + ((uint32_t) (qd * 32) << 16), v);
         if (part == 3) {
@@ -315,10 +323,12 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
             return pack_bf16(fmaf(v[8 * q2 + e], a.scale, x), fmaf(v[8 * q2 + e + 1], a.scale, y));
           };
           uint4 w;
-          w.x = sum(f.x, rest[q2].x, 0);
-          w.y = sum(f.y, rest[q2].y, 2);
-          w.z = sum(f.z, rest[q2].z, 4);
-          w.w = sum(f.w, rest[q2].w, 6);
+          const uint4 left = rest[(part & 1) * 2 + q2];
+          if (REM && AHEAD && part < 2) rest[(part & 1) * 2 + q2] = rp[(part + 2) * 2 + q2];      // the second half's, two parts ahead
+          w.x = sum(f.x, left.x, 0);
+          w.y = sum(f.y, left.y, 2);
+          w.z = sum(f.z, left.z, 4);
+          w.w = sum(f.w, left.w, 6);
           *reinterpret_cast<uint4*>(dqrow + part * 16 + 8 * q2) = w;
         }
       }
@@ -358,7 +368,8 @@ int launch_attn_dq_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, i
   LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) (4 * kTile + 2 * kStages * kChunkElems) * sizeof(bf16);
-  auto kernel = a.rem ? attn_dq_pooled_loop_tc_kernel<true> : attn_dq_pooled_loop_tc_kernel<false>;
+  auto kernel = !a.rem ? attn_dq_pooled_loop_tc_kernel<false, false>
+                : jobs <= kAheadJobs ? attn_dq_pooled_loop_tc_kernel<true, true> : attn_dq_pooled_loop_tc_kernel<true, false>;
   LLSA_SMEM_LIMIT_REGS(kernel, smem, kLaunchRegs);
   launch_pdl(kernel, grid, kThreads, smem, st, a, maps, jobs, gathered, n_c, n_tiles, tiles_per_head);
   LLSA_LAUNCH_OK("attn_dq_pooled_loop_tc_kernel");

@@ -38,6 +38,34 @@ def test_one_level_lists_vs_oracle(B, H, N, one_pass, monkeypatch):
     assert_bf16_close(vg.grad, dv + O.mean_pool1d_bwd(dpv, 16), "dv")
 
 
+# the two sides of the line up to which the dQ epilogue requests its remainder ahead: 288 and 320 keys are five jobs, 352 and two levels' 256 + 96 six
+LINE = [(4608, 8, 0), (5120, 8, 0), (5632, 8, 0), (24576, 8, 16)]
+
+
+@pytest.mark.parametrize("N,topk,topk2", LINE)
+def test_remainder_of_dq_at_the_line(N, topk, topk2, monkeypatch):
+    """The one-kernel form's error is the measure, as for the other lists: a remainder left out or in the wrong place is beyond it."""
+    from test_rounding import test_rounded_once as check
+    check(N, topk, topk2, ("dq",), monkeypatch)
+
+
+@pytest.mark.parametrize("N,topk,topk2", LINE[1:])
+def test_dq_of_a_head_does_not_depend_on_its_tiles_neighbours(N, topk, topk2):
+    """Three and more tiles per CTA against the same head alone (one tile, or two): what is requested ahead belongs to the next tile."""
+    H = max(2, 148 * 128 * 3 // N + 1)
+    x = [t.to(DEV) for t in synth.gaussian_qkv(N + topk2, 1, H, N, 64, dtype=torch.bfloat16)]
+
+    def dq(h0, h1):
+        q, k, v, do = [t[:, h0:h1].detach().clone() for t in x]
+        q.requires_grad_(True)
+        o = llsa_b200.llsa_l2(q, k, v, topk, topk2, 16) if topk2 else llsa_b200.llsa_l1(q, k, v, topk, 16)
+        return torch.autograd.grad(o, q, do)[0]
+
+    every = dq(0, H)
+    for h in (0, H - 1):
+        assert torch.equal(every[:, h:h + 1], dq(h, h + 1)), h
+
+
 def test_tail_keys_of_the_next_head_do_not_leak():
     """A chunk's rows behind the end of a head's list belong to the next head: NaN and infinities there must stay there."""
     q, k, v, do = [t.to(DEV) for t in synth.gaussian_qkv(5, 1, 2, 2560, 64, dtype=torch.bfloat16)]
