@@ -17,23 +17,25 @@
 // hold anything up to 2^127 times it; a row whose pooled keys outweigh its fine keys by more than that (its row sum
 // passes 1e30, or is NaN) is left untouched and marked in `redo`; a CTA that has marked a row of its tiles goes over them again
 // with two passes and writes exactly the marked rows.  (A second launch that looked for marks cost every call 1 to 2 us.)
-// Roles (one persistent CTA per SM, 20 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64):
+// Roles (one persistent CTA per SM, 16 or 20 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64):
 //   warp 8, warp 11  : TMA producers: Q per tile (2 stages) and K chunks (ring of 4; every chunk is loaded in both passes); V chunks (ring
 //                      of 4, pass 2 only)
 //   warp 9           : issues S of every "job" (a chunk of a pass).  Job number n, counted over all tiles of the CTA,
 //                      uses S buffer n mod 3 (TMEM columns [128 b, 128 b + 128)); O of tile i lives in [384 + 64 (i mod 2), + 64).
 //   warp 10          : issues O += P.V of the pass-2 jobs and hands every job's buffer back to warp 9 (buf_free,
 //                      committed behind the instructions that read P)
-//   warps 0-3 / 4-7 / 16-19 : three softmax warpgroups, group w owns the jobs n = w (mod 3) and with them S buffer w; thread r owns query
-//                      row r (TMEM lane r).  They leave a row's sum (and reference) in shared memory and go on to the next tile.
+//   warps 0-3 / 4-7 (/ 16-19) : two or three softmax warpgroups (GROUPS), group w owns the jobs n = w (mod GROUPS); thread r owns query row r (TMEM
+//                      lane r).  They leave a row's sum (and reference) in shared memory and go on to the next tile.
 //   warps 12-15      : epilogue, thread = row: merges O with the fine part (o, lse written by the fine kernel) and stores both.
 // What bounds it: the chain S -> exponentials -> P.V over three buffers, 1,430 cycles a job: with the softmax left out the copies, products and
 // hand-overs of a job take 900, with its exponentials alone left out 1,070; the 128 exponentials of a row take 1,024 on the SM's 16 MUFU lanes.
-// l1, B=2 H=4 N=65536: 692 us with two groups (their warps spend two thirds of a job in waits and loads), 669 with three; two levels, H=6
-// N=262144: 620 -> 590; B=2 H=4 N=65536: 90 -> 85.  No gain from: two groups that load a whole row of scores at once and hand the S buffer back
-// before the exponentials (732: fewer warps for the MUFU), eight warps a job (657 long lists, 56 -> 58 short ones), a
-// quarter or a third of the exponentials as a degree-5 polynomial on the FMA pipe (669 and 676; 85 -> 95 and 98 at N=65536 two levels).  In the form with one producer lane, the epilogue in the softmax groups and one O buffer
-// (785 us) the producer needed 1,300 cycles a job for its two waits and two copies, and every tile boundary cost 5,900 idle cycles.
+// Two groups' warps spend two thirds of a job in waits and loads; a third one takes turns with them where tiles are long enough (kThreeGroupKeys):
+// l1, B=2 H=4 N=65536: 692 us with two, 669 with three; two levels, H=6 N=262144: 620 -> 590; B=2 H=4 N=65536: 90 -> 85.  No gain from: two
+// groups that load a whole row of scores at once and hand the S buffer back before the exponentials (732: fewer warps for the MUFU); a quarter
+// or a third of the exponentials as a degree-5 polynomial on the FMA pipe (669 and 676; 85 -> 95 and 98 at N=65536 two levels).  Eight warps a job
+// were 2 % faster on long lists (657) and 4 % slower on short ones (56 -> 58).  In the form with one producer lane, the epilogue in the softmax
+// groups and one O buffer (785 us) the producer needed 1,300 cycles a job for its two waits and two copies, and every tile boundary cost 5,900
+// idle cycles.
 // Every mbarrier wait is bounded; a wait that expires raises a CTA-wide abort flag, every role leaves its loops, the epilogue puts NaN into lse of
 // every row of the CTA (poison_lse) and TMEM is freed.
 #include <string.h>
@@ -51,10 +53,15 @@ constexpr int kRows = 128;
 constexpr int kChunk = 128;                 // keys per chunk
 constexpr int kTile = kRows * 64;           // elements of a [128 x 64] bf16 tile (16 KB)
 constexpr int kKStages = 4, kVStages = 4;
-constexpr int kThreads = 640;
-constexpr int kLaunchRegs = 96, kIssueRegs = 40, kEpilogueRegs = 104, kSoftmaxRegs = 112;     // a thread's, per role: 40 + 104 + 3 x 112 = 5 x 96
-static_assert(kIssueRegs + kEpilogueRegs + 3 * kSoftmaxRegs <= 5 * kLaunchRegs, "the takers would wait for good");
-constexpr int kBufs = 3, kGroups = 3;       // softmax group w owns S buffer w
+constexpr int kBufs = 3;                    // S buffers
+// Registers of a thread, per role.  Three softmax groups share what 640 threads launch with: 40 + 104 + 3 x 112 = 5 x 96; with two every thread keeps
+// the 128 of the launch.
+template <int GROUPS>
+struct Split {
+  static constexpr int kThreads = GROUPS == 3 ? 640 : 512, kLaunch = GROUPS == 3 ? 96 : 128;
+  static constexpr int kIssue = GROUPS == 3 ? 40 : kLaunch, kEpilogue = GROUPS == 3 ? 104 : kLaunch, kSoftmax = GROUPS == 3 ? 112 : kLaunch;
+  static_assert(kIssue + kEpilogue + GROUPS * kSoftmax <= (2 + GROUPS) * kLaunch, "the takers would wait for good");
+};
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr uint32_t kColO = 384;
 // One pass over a list that one kernel used to take with running maxima (REM): where in its binade a probability of a logit of 0 lands.  bf16 is finest just below a power of two, which is where a row's
@@ -62,6 +69,13 @@ constexpr uint32_t kColO = 384;
 // (against fp64, N(0,1) inputs, two levels, N = 40960, top-16: 2.33e-3; 2.33e-3, 2.11e-3, 2.10e-3, 2.15e-3, 2.22e-3 with the reference at
 // 0, 1/8, 1/4, 3/8, 1/2 above a power of two; 2.09e-3 with two passes, 2.07e-3 in one kernel).  The weights 16 and 256 are powers of two.
 constexpr float kRefShift = 0.25f;
+
+// Pooled keys of a row from which three softmax groups are the better split; below, a tile is a few jobs, and every group of it costs the tile a
+// round of hand-overs (sums, maxima, the next tile's reference).  Lists whose fine part comes with a remainder gain later: their epilogue is longer.
+// Whole forward in us, two groups / three: one level, B=2 H=6, 256 keys 30.9 / 31.5, 512 57.5 / 56.5, 608 (remainder) 126.6 / 125.1; two levels, B=3
+// H=6 N=32768, 256 keys 238 / 242; H=6 N=24576, 256 (160 + 96) 93 / 96, remainder; H=6 N=16384, 320 and 384, remainder, 69 / 70 and 99 / 100; H=6
+// N=65536, 384 keys 178 / 174, 448 with remainder 254 / 263; H=5 N=40960, 480 with remainder 184.5 / 184.1.
+constexpr int kThreeGroupKeys = 384, kThreeGroupKeysRem = 480;
 
 struct LoopMaps {
   CUtensorMap q;              // [B,H,Nq,64] 4-D, box 128 rows
@@ -74,6 +88,7 @@ struct LoopBars {
   uint64_t s_ready[kBufs], wg_done[kBufs], buf_free[kBufs], o_ready[2], o_free[2], sum_ready[2], xchg;
 };
 
+template <int GROUPS>
 __device__ __forceinline__ void init_bars(LoopBars& bars) {
   for (int i = 0; i < 2; ++i) {
     tc::mbar_init(&bars.q_full[i], 1);
@@ -89,24 +104,24 @@ __device__ __forceinline__ void init_bars(LoopBars& bars) {
   for (int i = 0; i < 2; ++i) {
     tc::mbar_init(&bars.o_ready[i], 1);
     tc::mbar_init(&bars.o_free[i], 4);
-    tc::mbar_init(&bars.sum_ready[i], 4 * kGroups);
+    tc::mbar_init(&bars.sum_ready[i], 4 * GROUPS);
   }
-  tc::mbar_init(&bars.xchg, 4 * kGroups);
+  tc::mbar_init(&bars.xchg, 4 * GROUPS);
   tc::fence_mbar_init();
 }
 
 // n_chunks: chunks per tile; gathered: how many of them, the first ones, are gathered level-1 blocks (two levels); n_c: rows per
 // head of the contiguous pooled tensor.  REM: the fine part of o is the bf16 value in o plus its remainder in a.rem.
-template <bool REM>
-__global__ void __launch_bounds__(kThreads, 1)
+template <bool REM, int GROUPS>
+__global__ void __launch_bounds__(Split<GROUPS>::kThreads, 1)
 attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps maps, int n_chunks, int gathered, int64_t n_c, int n_tiles,
                                int tiles_per_head, unsigned char* redo) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ LoopBars bars_of[2];                    // of the first round over the tiles and of the one for marked rows
   __shared__ uint32_t s_tmem;
   __shared__ tc::WaitCtl s_ctl;
-  __shared__ float s_max[2][kGroups][kRows];             // [tile parity][group][row]: row maxima after pass 1
-  __shared__ float s_sum[2][kGroups][kRows], s_ref[2][kRows];      // [tile parity][group][row] row sums; [tile parity][row] their reference
+  __shared__ float s_max[2][GROUPS][kRows];             // [tile parity][group][row]: row maxima after pass 1
+  __shared__ float s_sum[2][GROUPS][kRows], s_ref[2][kRows];      // [tile parity][group][row] row sums; [tile parity][row] their reference
   bf16* base = reinterpret_cast<bf16*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   bf16* sQ = base;                          // [2][128][64]
   bf16* sK = sQ + 2 * kTile;                // [kKStages][128][64]
@@ -117,7 +132,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   if (tid == 0) {
     s_ctl.abort = 0;
     s_ctl.limit = a.wait_limit > 0 ? a.wait_limit : tc::kWaitPolls;
-    init_bars(bars_of[0]);
+    init_bars<GROUPS>(bars_of[0]);
   }
   pdl_wait();
   if (warp == 0) tc::tmem_alloc(&s_tmem, 512);
@@ -136,7 +151,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       body(bars_of[round], n_pass, n_pass * n_chunks);
       tc::fence_before_sync();
       if (!__syncthreads_or(marked) || abort_flag->abort) break;
-      if (tid == 0) init_bars(bars_of[1]);
+      if (tid == 0) init_bars<GROUPS>(bars_of[1]);
       __syncthreads();
       tc::fence_after_sync();
     }
@@ -148,7 +163,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   };
 
   // 640 threads launch with 96 registers each; the warps that issue copies and products leave most of theirs to the others
-  if (warp >= 8 && warp < 12) tc::regs_set<kIssueRegs, kLaunchRegs>();
+  if (warp >= 8 && warp < 12) tc::regs_set<Split<GROUPS>::kIssue, Split<GROUPS>::kLaunch>();
   if (warp == 8 || warp == 11) {
     rounds([&](LoopBars& bars, int, int jobs) {
       // ---------------------------------------------------------------- TMA producers: warp 8 Q and keys, warp 11 values
@@ -266,7 +281,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       }
     });
   } else if (warp < 8 || warp >= 16) {
-    tc::regs_set<kSoftmaxRegs, kLaunchRegs>();
+    tc::regs_set<Split<GROUPS>::kSoftmax, Split<GROUPS>::kLaunch>();
     rounds([&](LoopBars& bars, int n_pass, int jobs) {
       // ---------------------------------------------------------------- softmax, thread = query row
       const int wg = warp < 8 ? warp >> 2 : 2, qd = warp & 3, r = qd * 32 + lane;
@@ -274,8 +289,8 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       const float sl2 = a.scale * kLog2eF;
       const float lw1 = log2f(a.w1), lw2 = log2f(a.w2);
       const uint32_t t_lane = tmem + ((uint32_t) (qd * 32) << 16);
-      const int buf = wg;                    // this group takes every third job of the CTA: always the same S buffer; the phase parity of
-      uint32_t bph = 0;                      // that buffer's barriers
+      int buf = wg;                          // S buffer of this group's next job: it takes every GROUPS-th of the CTA (one of three always meets
+      uint32_t bph = 0;                      // the same buffer); the phase parity of that buffer's barriers
       int first = wg;                        // its first job of the tile at hand
       float va[32];
       auto lse_of = [&](int i) {             // the fine part's log-sum-exp of this thread's row of tile i
@@ -291,19 +306,19 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         if (n_pass == 1 && i + 1 < n_my) lse_next = lse_of(i + 1);
         bool exchanged = n_pass == 1;
         // two passes: the groups exchange their row maxima once per tile, before their first pass-2 job (a group may have none); a copy is
-        // rewritten two exchanges later, after both groups have passed the barrier in between
+        // rewritten two exchanges later, after every group has passed the barrier in between
         auto exchange_max = [&]() -> bool {
           exchanged = true;
           s_max[i & 1][wg][r] = mx;
           __syncwarp();
           if (lane == 0) tma::mbar_arrive(&bars.xchg);
           const bool ok_ = __all_sync(0xffffffffu, tc::bounded_wait(&bars.xchg, (uint32_t) i & 1, abort_flag));
-          mx = fmax3(s_max[i & 1][0][r], s_max[i & 1][1][r], s_max[i & 1][2][r]);
+          mx = fmax3(s_max[i & 1][0][r], s_max[i & 1][1][r], s_max[i & 1][GROUPS - 1][r]);
           if (mx == -INFINITY) mx = 0.f;       // no score above -inf (masked keys): their weight is 0 whatever the reference
           return ok_;
         };
         int j = first;
-        for (; j < jobs; j += kGroups) {
+        for (; j < jobs; j += GROUPS) {
           const bool p2 = j >= first_p2;
           const int c = j >= n_chunks ? j - n_chunks : j;
           const float lw = (c < gathered || !a.two_level) ? lw1 : lw2;
@@ -345,7 +360,12 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tma::mbar_arrive(&bars.wg_done[buf]);
-          bph ^= 1;
+          if (GROUPS == kBufs) {
+            bph ^= 1;
+          } else {
+            buf += GROUPS;
+            if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
+          }
         }
         first = j - jobs;
         if (ok && !exchanged) ok = exchange_max();
@@ -361,7 +381,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
       }
     });
   } else {
-    tc::regs_set<kEpilogueRegs, kLaunchRegs>();
+    tc::regs_set<Split<GROUPS>::kEpilogue, Split<GROUPS>::kLaunch>();
     rounds([&](LoopBars& bars, int n_pass, int) {
       // ---------------------------------------------------------------- epilogue, thread = query row
       const int qd = warp & 3, r = qd * 32 + lane;
@@ -382,7 +402,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
         tc::fence_after_sync();
         if (!ok) break;
-        const float lsum = s_sum[i & 1][0][r] + s_sum[i & 1][1][r] + s_sum[i & 1][2][r], mx = s_ref[i & 1][r];
+        const float two = s_sum[i & 1][0][r] + s_sum[i & 1][1][r], lsum = GROUPS == 3 ? two + s_sum[i & 1][GROUPS - 1][r] : two, mx = s_ref[i & 1][r];
         // one pass: the row is this round's unless its sum left the safe range (false for NaN too): the mark hands it to the second
         if (redo && n_pass == 1) {
           mine = lsum < 1e30f;
@@ -480,10 +500,13 @@ int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
   LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) (2 + kKStages + kVStages) * kTile * sizeof(bf16);
-  auto kernel = a.rem ? attn_fwd_pooled_loop_tc_kernel<true> : attn_fwd_pooled_loop_tc_kernel<false>;
-  LLSA_SMEM_LIMIT_REGS(kernel, smem, kLaunchRegs);
+  const bool three = (a.p1_blocks + a.p2_blocks) * kBS >= (a.rem ? kThreeGroupKeysRem : kThreeGroupKeys);
+  auto kernel = three ? (a.rem ? attn_fwd_pooled_loop_tc_kernel<true, 3> : attn_fwd_pooled_loop_tc_kernel<false, 3>)
+                      : (a.rem ? attn_fwd_pooled_loop_tc_kernel<true, 2> : attn_fwd_pooled_loop_tc_kernel<false, 2>);
+  const int threads = three ? Split<3>::kThreads : Split<2>::kThreads;
+  LLSA_SMEM_LIMIT_REGS(kernel, smem, three ? Split<3>::kLaunch : 0);
   unsigned char* redo = g->fwd_redo && pooled_loop_one_pass(a) ? reinterpret_cast<unsigned char*>(g->fwd_redo->ptr) : nullptr;
-  launch_pdl(kernel, grid, kThreads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, redo);
+  launch_pdl(kernel, grid, threads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, redo);
   LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");
   return LLSA_OK;
 }

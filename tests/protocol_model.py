@@ -387,9 +387,9 @@ def forward_kernel(seed, tiles, chunks, passes, k_stages=4, v_stages=4, buffers=
     """attn_fwd_pooled_loop_tc_kernel: `tiles` query tiles of `chunks` key chunks; one pass (jobs = chunks, every job
     feeds P.V) or two (jobs = 2 * chunks: row maxima first, then the exponentials; the groups exchange their maxima
     once per tile, a group without a second-pass job at its end).  Producers of keys (with Q) and of values; one warp issues S, one P.V
-    and hands every job's buffer back; softmax group g of three takes the jobs whose CTA-wide number is g mod 3 (always the same buffer;
-    a tile's first job goes round the groups) and leave their row sums to four epilogue warps, as O in one of
-    two accumulators.
+    and hands every job's buffer back; softmax group g of `groups` (three, or two for short lists) takes the jobs whose CTA-wide number is g mod
+    groups (of three always the same buffer; a tile's first job goes round the groups) and leaves its row sums to four epilogue warps, as O in
+    one of two accumulators.
     second_round: the CTA has marked a row and goes over its tiles again with two passes, on barriers of its own, behind a CTA-wide
     synchronisation.  softmax_waits_for_sums=False breaks the protocol on purpose (row sums overwritten before they are read)."""
     sim = Sim(seed)

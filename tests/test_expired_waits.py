@@ -33,8 +33,8 @@ def _check(levels, x, limit, monkeypatch):
     return int(lse.isnan().sum())
 
 
-# key-loop pooled forward, one and two levels, one pass and two, three to seven tiles per CTA; the single-shot one, ten tiles per CTA
-@pytest.mark.parametrize("levels,B,H,N,one_pass", [(1, 2, 4, 16384, True), (1, 2, 4, 16384, False), (2, 1, 2, 65536, True), (2, 2, 6, 16384, True)])
+# key-loop pooled forward, one and two levels, one pass and two, two and three softmax groups, three to seven tiles per CTA; the single-shot one, ten
+@pytest.mark.parametrize("levels,B,H,N,one_pass", [(1, 2, 8, 4096, True), (1, 2, 4, 16384, True), (1, 2, 4, 16384, False), (2, 1, 2, 65536, True), (2, 2, 6, 16384, True)])
 def test_every_row_behind_an_expired_wait_of_the_pooled_forward_is_nan(levels, B, H, N, one_pass, monkeypatch):
     """A limit that the fine forward's waits keep and the pooled one's do not: the tiles behind a CTA's first unfinished one included."""
     from llsa_b200 import ops

@@ -66,6 +66,23 @@ def test_dq_of_a_head_does_not_depend_on_its_tiles_neighbours(N, topk, topk2):
         assert torch.equal(every[:, h:h + 1], dq(h, h + 1)), h
 
 
+# the lines between two and three softmax groups of the forward: 256 and 384 keys without a remainder, 448 and 480 with one
+@pytest.mark.parametrize("one_pass", [True, False])
+@pytest.mark.parametrize("N", [4096, 6144, 7168, 7680])
+def test_forward_on_both_sides_of_the_group_line(N, one_pass, monkeypatch):
+    """Against the oracle, and with three and more tiles per CTA what the first and last head give alone.  Which group takes a tile's first job
+    depends on the tile's place, and with it the order of the fp32 sum of a row's three or two partial sums: 2^-23 of it, which moves one o in
+    2^-23 / 2^-8 = 2^-15 over a rounding boundary of bf16, by 2^-8 at most: 2^-15.5 in the 2-norm.  A row or a tile mixed up is of order one."""
+    test_one_level_lists_vs_oracle(1, 1, N, one_pass, monkeypatch)
+    H = 148 * 128 * 3 // N + 1
+    q, k, v, _ = [t.to(DEV) for t in synth.gaussian_qkv(N + 1, 1, H, N, 64, dtype=torch.bfloat16)]
+    with torch.no_grad():
+        every = llsa_b200.llsa_l1(q, k, v, 8, 16)
+        for h in (0, H - 1):
+            alone = llsa_b200.llsa_l1(*[t[:, h:h + 1].contiguous() for t in (q, k, v)], 8, 16).float()
+            assert float((every[:, h:h + 1].float() - alone).norm() / alone.norm()) < 2 ** -13, h
+
+
 def test_tail_keys_of_the_next_head_do_not_leak():
     """A chunk's rows behind the end of a head's list belong to the next head: NaN and infinities there must stay there."""
     q, k, v, do = [t.to(DEV) for t in synth.gaussian_qkv(5, 1, 2, 2560, 64, dtype=torch.bfloat16)]

@@ -117,3 +117,13 @@ def test_model_catches_a_producer_an_epilogue_warp_and_a_reader_left_out_of_the_
     warp = sum(outcome(query_major_kernel, s, 7, 1, free_count=1) != "ok" for s in range(60))
     sums = sum(outcome(forward_kernel, s, 6, 1, 1, softmax_waits_for_sums=False) != "ok" for s in range(60))
     assert producer > 0 and warp > 0 and sums > 0
+
+
+def test_two_softmax_groups_have_no_hazard_or_deadlock():
+    """attn_fwd_pooled_loop_tc_kernel as short lists get it: two groups on three S buffers, so that a group's buffer changes from job to job; one
+    to four chunks, one pass and two, and a second round."""
+    for seed in range(RUNS):
+        rng = random.Random(seed)
+        tiles, chunks = rng.randint(1, 7), rng.randint(1, 4)
+        assert outcome(forward_kernel, seed, tiles, chunks, 1 + seed % 2, groups=2) == "ok", seed
+        assert outcome(forward_kernel, seed, tiles, chunks, 1, groups=2, second_round=True) == "ok", seed
