@@ -3,7 +3,7 @@
 single-shot pooled backward with its two MMA-issuing threads (attn_pooled_bwd_tc.cu).
 
 Test infrastructure: nothing in the package imports it.  Every role of a CTA
-(the two TMA producers, the warps that issue MMAs, the eight softmax warps, the
+(the two TMA producers, the warps that issue MMAs, the softmax warps, the
 four epilogue warps) is a Python generator that waits on barriers, spends random
 time and arrives, exactly in the order the kernel's role does.  The model keeps the hardware's semantics where
 they matter for correctness:
@@ -135,18 +135,24 @@ def _bars(name, n, count):
     return [Barrier("%s%d" % (name, i), count) for i in range(n)]
 
 
-def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8, buffers=None, accs=1, full_count=2):
-    """attn_dkv_pooled_loop_tc_kernel.  `units`: job counts of the units of one CTA's piece: (head, chunk) units in the dense form
-    (four S^T buffers, which P^T and dS^T overwrite, one pair of accumulators), units of four jobs and fewer in the gathered one (buffers=2,
-    accs=2); two dP^T buffers, handed back as soon as their group has loaded them.  Two score threads share three S^T buffers.
+def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8, buffers=None, accs=1, full_count=2, gathered=False, dp_count=4,
+                     dp_back_first=False):
+    """attn_dkv_pooled_loop_tc_kernel.  `units`: job counts of the units of one CTA's piece.  Dense form: (head, chunk) units; four S^T buffers,
+    which P^T and dS^T overwrite, one pair of accumulators, and two dP^T buffers, handed back as soon as their group has loaded them.  Gathered
+    form: units of four jobs and fewer; two buffers of S^T and dP^T together, which go back with the products that read P^T and dS^T, and two
+    pairs of accumulators.  Two score threads share three S^T buffers.
+    dp_count: warps whose arrivals hand a dP^T buffer back (4 = the kernel; fewer break the protocol on purpose), dp_back_first: a warp
+    arrives before it has loaded its part (the same).
     score_threads: threads that issue S^T / dP^T (1 = the kernel; 2 = even and odd jobs on two threads).
     score_barriers: sdp_ready / buf_free barriers (None = one per buffer, the kernel; 6 = one per job number mod 6).
     full_count: producers a query stage waits for (2 = the kernel: Q, and dO with lse and delta; 1 breaks the protocol on purpose)."""
     sim = Sim(seed)
+    if gathered:
+        buffers, accs = 2, 2
     buffers = buffers or (4 if score_threads == 1 else 3)
     nb = score_barriers or buffers
     dp = [Resource("dP^T buffer %d" % i) for i in range(2)]
-    dp_free = _bars("dp_free", 2, 4)
+    dp_free = None if gathered else _bars("dp_free", 2, dp_count)
     kv_full, kv_empty = _bars("kv_full", 2, 1), _bars("kv_empty", 2, score_threads)
     q_full, q_empty = _bars("q_full", stages, full_count), _bars("q_empty", stages, 1)
     sdp, pds, free = _bars("sdp_ready", nb, 1), _bars("pds_ready", buffers, 4), _bars("buf_free", nb, 1)
@@ -184,7 +190,7 @@ def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8
                 if job >= buffers:
                     prev = job - buffers
                     wait += [free[prev % nb], (prev // nb) & 1]
-                if job >= 2:
+                if job >= 2 and not gathered:
                     wait += [dp_free[job & 1], ((job >> 1) - 1) & 1]
                 yield tuple(wait)
                 if sim.rng.random() < 0.15:
@@ -233,10 +239,15 @@ def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8
             buf = job % buffers
             yield ("wait", sdp[job % nb], (job // nb) & 1)
             assert owner[buf] is not None and owner[buf][1] == job, ("softmax read", buf, owner[buf], job)
+            if dp_back_first:
+                dp_free[job & 1].arrive(sim)
             yield ("delay", sim.r(100, 400))
             dp[job & 1].read(sim, job)
-            dp_free[job & 1].arrive(sim)
+            if not gathered and not dp_back_first:
+                dp_free[job & 1].arrive(sim)
             yield ("delay", sim.r(500, 1200))
+            if gathered:                  # dP^T is loaded half by half and overwritten by dS^T: it is the job's up to here
+                dp[job & 1].read(sim, job)
             if warp == 0:
                 owner[buf] = ("p", job)
             pds[buf].arrive(sim)
@@ -262,16 +273,17 @@ def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8
     return sim.run()
 
 
-def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=None, stages=8, buffers=None, free_count=4):
+def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=None, stages=8, buffers=None, free_count=4, dp_count=4, dp_back_first=False):
     """attn_dq_pooled_loop_tc_kernel: `tiles` query tiles of `jobs` key chunks; Q / dO in two stages, K and V chunks (two
     producers) in one ring of pairs, S into four buffers (three with two score threads), which dS overwrites, dP into two, handed back as soon
     as their group has loaded them, dQ of a tile into one of two accumulators, read by epilogue warps.
-    free_count: epilogue warps an accumulator waits for (4 = the kernel; 1 breaks the protocol on purpose)."""
+    free_count: epilogue warps an accumulator waits for (4 = the kernel; 1 breaks the protocol on purpose); dp_count, dp_back_first: as in
+    key_major_kernel."""
     sim = Sim(seed)
     buffers = buffers or (4 if score_threads == 1 else 3)
     nb = score_barriers or buffers
     dp = [Resource("dP buffer %d" % i) for i in range(2)]
-    dp_free = _bars("dp_free", 2, 4)
+    dp_free = _bars("dp_free", 2, dp_count)
     q_full, q_empty = _bars("q_full", 2, 1), _bars("q_empty", 2, score_threads)
     kv_full, kv_empty = _bars("kv_full", stages, 2), _bars("kv_empty", stages, 1)
     sdp, ds, free = _bars("sdp_ready", nb, 1), _bars("ds_ready", buffers, 4), _bars("buf_free", nb, 1)
@@ -354,9 +366,12 @@ def query_major_kernel(seed, tiles, jobs, score_threads=1, score_barriers=None, 
             buf = job % buffers
             yield ("wait", sdp[job % nb], (job // nb) & 1)
             assert owner[buf] is not None and owner[buf][1] == job, ("softmax read", buf, owner[buf], job)
+            if dp_back_first:
+                dp_free[job & 1].arrive(sim)
             yield ("delay", sim.r(100, 400))
             dp[job & 1].read(sim, job)
-            dp_free[job & 1].arrive(sim)
+            if not dp_back_first:
+                dp_free[job & 1].arrive(sim)
             yield ("delay", sim.r(400, 1000))
             if warp == 0:
                 owner[buf] = ("p", job)

@@ -17,8 +17,8 @@ def _pieces(seed):
 
 
 def test_key_major_kernel_protocol_has_no_hazard_or_deadlock():
-    """attn_dkv_pooled_loop_tc_kernel, dense form: two producers, one S^T / dP^T warp, one dV / dK warp, three buffers, barriers per
-    buffer, epilogue warps."""
+    """attn_dkv_pooled_loop_tc_kernel, dense form: two producers, one S^T / dP^T warp, one dV / dK warp, four S^T and two dP^T buffers,
+    barriers per buffer, epilogue warps."""
     for seed in range(RUNS):
         assert outcome(key_major_kernel, seed, _pieces(seed)) == "ok", seed
 
@@ -32,8 +32,8 @@ def test_query_major_kernel_protocol_has_no_hazard_or_deadlock():
 
 @pytest.mark.parametrize("passes", [1, 2])
 def test_forward_kernel_protocol_has_no_hazard_or_deadlock(passes):
-    """attn_fwd_pooled_loop_tc_kernel in its one-pass form (odd and even chunk counts: with 9 chunks the groups
-    swap the parity of their first job from tile to tile) and in the two-pass form."""
+    """attn_fwd_pooled_loop_tc_kernel with three softmax groups in its one-pass form (with 2 and 8 chunks a tile's first job goes round the groups,
+    with 3 and 9 it is always the same group's) and in the two-pass form."""
     for seed in range(RUNS):
         rng = random.Random(seed)
         assert outcome(forward_kernel, seed, rng.randint(1, 6), rng.choice([2, 3, 8, 9]), passes) == "ok", seed
@@ -86,16 +86,17 @@ def test_model_catches_a_stage_freed_by_one_issuer_only_and_an_unguarded_overwri
 
 
 def test_gathered_key_major_form_has_no_hazard_or_deadlock():
-    """attn_dkv_pooled_loop_tc_kernel, gathered form: units of four query tiles (pieces begin and end inside one), two buffers -- a group
-    meets its own buffer again with its next job -- and two accumulators."""
+    """attn_dkv_pooled_loop_tc_kernel, gathered form: units of four query tiles (pieces begin and end inside one), two buffers of S^T and dP^T --
+    a group meets its own buffer again with its next job, and nothing but the products behind it hands it back -- and two accumulators."""
     for seed in range(RUNS):
         rng = random.Random(seed)
         units = [rng.randint(1, 4)] + [4] * rng.randint(0, 9) + [rng.randint(1, 4)]
-        assert outcome(key_major_kernel, seed, units, buffers=2, accs=2) == "ok", seed
+        assert outcome(key_major_kernel, seed, units, gathered=True) == "ok", seed
 
 
 def test_one_chunk_tiles_leave_a_group_without_work():
-    """A list of one chunk: every other tile has no job for a group, which still takes part in the exchange of maxima and row sums."""
+    """A list of one chunk: in one pass two of three tiles have no job for a group, in two passes one of three; it still takes part in the exchange of
+    maxima and row sums."""
     for seed in range(RUNS):
         rng = random.Random(seed)
         assert outcome(forward_kernel, seed, rng.randint(1, 7), 1, 1 + seed % 2) == "ok", seed
@@ -117,6 +118,15 @@ def test_model_catches_a_producer_an_epilogue_warp_and_a_reader_left_out_of_the_
     warp = sum(outcome(query_major_kernel, s, 7, 1, free_count=1) != "ok" for s in range(60))
     sums = sum(outcome(forward_kernel, s, 6, 1, 1, softmax_waits_for_sums=False) != "ok" for s in range(60))
     assert producer > 0 and warp > 0 and sums > 0
+
+
+def test_model_catches_a_dp_buffer_handed_back_too_early():
+    """Two mutations of the hand-back of dP (dQ and dense dK/dV kernels): the first of a group's four warps to have loaded its rows gives the whole
+    buffer back, and warps give it back before they have loaded.  The next but one job's product then overwrites what is being read."""
+    for broken in ({"dp_count": 1}, {"dp_back_first": True}):
+        bad_kv = sum(outcome(key_major_kernel, s, _pieces(s), **broken) != "ok" for s in range(60))
+        bad_q = sum(outcome(query_major_kernel, s, 4, 6, **broken) != "ok" for s in range(60))
+        assert bad_kv > 0 and bad_q > 0, (broken, bad_kv, bad_q)
 
 
 def test_two_softmax_groups_have_no_hazard_or_deadlock():
