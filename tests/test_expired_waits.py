@@ -56,3 +56,37 @@ def test_rows_marked_for_a_round_that_an_expired_wait_cuts_short_are_nan(limit, 
 def test_every_row_behind_an_expired_wait_of_the_fine_forward_is_nan(levels, B, H, N, monkeypatch):
     """A limit of one: most of the fine forward's copies have not landed at the first look, and nothing writes those rows."""
     assert _check(levels, _inputs(levels, B, H, N), 1, monkeypatch) > 0
+
+
+# key-loop dQ and dense dK/dV at one level, with the gathered dK/dV at two, lists that come with a remainder; the single-shot backward.  A limit of
+# four: the fine stages' waits mostly keep it, those of a tile of many jobs do not
+@pytest.mark.parametrize("levels,B,H,N,limits", [(1, 2, 6, 1024, (1,)), (1, 1, 4, 16384, (1, 4)), (2, 1, 3, 40960, (1, 4)), (2, 1, 2, 65536, (1, 4)),
+                                                 (2, 1, 6, 16384, (1,))])
+def test_expired_waits_of_the_backward_are_reported(levels, B, H, N, limits, monkeypatch):
+    """The kernels leave their loops, give their tensor memory back and report it; the next backward is right again."""
+    import llsa_b200 as L
+    from llsa_b200 import ops
+    q, k, v = _inputs(levels, B, H, N)
+    do = torch.ones_like(q)
+    q.requires_grad_(True)
+
+    def forward():
+        return L.llsa_l1(q, k, v, 8, 16) if levels == 1 else L.llsa_l2(q, k, v, 8, 8, 16)
+
+    want, = torch.autograd.grad(forward(), q, do)
+    for limit in limits:
+        o = forward()
+        torch.cuda.synchronize()
+        monkeypatch.setattr(ops, "_wait_limit", limit)
+        L.set_device_checks(True)
+        ops._native()                # hands the settings over: the backward runs without a call of this module's
+        try:
+            with pytest.raises(RuntimeError, match="bounded wait"):
+                torch.autograd.grad(o, q, do)
+        finally:
+            monkeypatch.setattr(ops, "_wait_limit", 0)
+            L.set_device_checks(False)
+            ops._native()
+        torch.cuda.synchronize()
+        again, = torch.autograd.grad(forward(), q, do)
+        assert torch.equal(again, want)
