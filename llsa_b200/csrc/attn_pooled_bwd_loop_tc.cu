@@ -9,7 +9,8 @@
 //                                                                         is applied to dQ
 //     dQ += dS . K_c    [128 x 64]  (K = 64 keys)             dS read from TENSOR MEMORY (packed bf16 over S), K_c MN-major
 // Two levels: first the gathered level-1 blocks (four to a chunk), then the level-2 keys.  Either list may end inside a chunk (at 32 keys):
-// what is loaded behind its end is neither exponentiated nor multiplied.
+// what is loaded behind its end (a repeated block, or another head's rows, infinities and NaN included) goes through the softmax with the rest
+// of the row, and the dQ products stop in front of it.
 // The final log-sum-exp is known in the backward, so one pass over the chunks suffices.  dQ accumulates in TMEM over
 // all chunks of the tile and is then added to the fine part already in dq.
 // TMEM columns, chunk number n of the CTA (counted over all its tiles): S, and dS over it, at 64 (n mod 4); dP at [256 + 64 (n mod 2), + 64); dQ of
@@ -21,7 +22,7 @@
 // do and S gets four.  The two issuing warps run independently (S / dP of the next tile start while dQ of this one is still being issued); an
 // S buffer goes back to the S / dP warp through buf_free, committed behind the dQ instructions that read its dS.
 // What bounds it: the loop S, dP -> dS -> dQ, 850 cycles a chunk; the tensor pipe takes 576, copies, products and hand-overs without the softmax
-// 680.  Two levels, B=1 H=6 N=262144: 757 us with three buffers for S and dP together and 32 columns loaded at a time, 680 now; l1, B=2 H=4
+// 745, with its exponentials alone left out 810.  Two levels, B=1 H=6 N=262144: 757 us with three buffers for S and dP together and 32 columns loaded at a time, 680 now; l1, B=2 H=4
 // N=16384: 64.5 -> 58.5.  On the old form nothing came of three softmax groups (751), of eight warps a chunk (787), of dP handed over apart
 // from S (814); four S buffers and two of dP without the early hand-back made it 825.
 // The form with one producer lane, the epilogue in the softmax groups and one dQ accumulator (1,050 us) needed 1,130 cycles a chunk for the
@@ -46,6 +47,8 @@ constexpr int kStages = 8;
 constexpr int kThreads = 512;
 constexpr int kLaunchRegs = 128, kIssueRegs = 40, kEpilogueRegs = 88, kSoftmaxRegs = 192;     // a thread's, per role: 40 + 88 + 2 x 192 = 4 x 128
 static_assert(kIssueRegs + kEpilogueRegs + 2 * kSoftmaxRegs <= 4 * kLaunchRegs, "the takers would wait for good");
+// The split is that of the form with a remainder (46.7 us at H=5 N=40960, 416 keys, against 50.4 with 56 / 88 / 184); the form without spills one
+// word with it, which 48 / 88 / 184 and 56 / 72 / 192 do not (71 us against 72 at H=6 N=65536).
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr int kBufs = 4;                     // S buffers (dS over them)
 constexpr uint32_t kColDP = 256, kColDQ = 384;

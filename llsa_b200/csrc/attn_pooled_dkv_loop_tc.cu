@@ -11,8 +11,8 @@
 //     P^T  = exp2(S^T*scale*log2e + log2 w - lse[q]),  dS^T = P^T * (dP^T - delta[q])     thread = key row; the scale
 //            (a power of two) is applied to dK;
 //            lse and delta of the 64 query columns sit in shared memory next to the Q / dO tile
-//     dV_c += P^T  . dO_t  [128 x 64]  (K = 64 queries)   P^T, dS^T read from TENSOR MEMORY (packed bf16, written over
-//     dK_c += dS^T . Q_t                                   S^T / dP^T), dO_t / Q_t as MN-major operands (the same tiles)
+//     dV_c += P^T  . dO_t  [128 x 64]  (K = 64 queries)   P^T, dS^T read from TENSOR MEMORY (packed bf16, written over S^T;
+//     dK_c += dS^T . Q_t                                   gathered: dS^T over dP^T), dO_t / Q_t as MN-major operands (the same tiles)
 // dK_c, dV_c accumulate in TMEM over the unit's query range and are then written to the fp32 pooled-gradient
 // accumulators (scaled by kv_weight / token_weight, the reference's weighting of the pooled dK/dV side): plain stores if
 // the unit covers all queries of its head, reductions otherwise.  Rows of a chunk behind the end of its list (which may end at any
@@ -28,9 +28,9 @@
 // warps 0-3 / 4-7 = two softmax warpgroups on alternating jobs, warps 12-15 write a unit's dV and dK, thread = key row.  Every mbarrier
 // wait is bounded (abort flag, TMEM freed).
 // What bounds them.  Dense, tensor pipe 768 cycles a job: the loop S^T, dP^T -> P^T, dS^T -> dV, dK, 1,170 cycles; copies, products and hand-overs
-// without the softmax 930.  Two levels, B=1 H=6 N=262144: 870 us with three buffers for both and 32 columns loaded at a time, 830 now; l1, B=2 H=4
-// N=16384: 85 -> 79.5.  Three softmax groups change nothing (866), eight warps a job spill (1,165).  Gathered: the fp32 reductions, 100 M at
-// the same size; 263 us with results read from tensor memory 32 columns at a time, 241 with 16 (top-16, H=5 N=40960: 71 -> 65); in the dense
+// without the softmax 915, with its exponentials alone left out 1,090.  Two levels, B=1 H=6 N=262144: 870 us with three buffers for both and 32
+// columns loaded at a time, 835 now; l1, B=2 H=4 N=16384: 85 -> 79.  Three softmax groups change nothing (866), eight warps a job spill (1,165).  Gathered: the fp32 reductions, 100 M at
+// the same size; 263 us with results read from tensor memory 32 columns at a time, 245 with 16 (top-16, H=5 N=40960: 71 -> 65); in the dense
 // form's layout 254 to 270.
 #include <string.h>
 

@@ -28,7 +28,7 @@
 //                      lane r).  They leave a row's sum (and reference) in shared memory and go on to the next tile.
 //   warps 12-15      : epilogue, thread = row: merges O with the fine part (o, lse written by the fine kernel) and stores both.
 // What bounds it: the chain S -> exponentials -> P.V over three buffers, 1,430 cycles a job: with the softmax left out the copies, products and
-// hand-overs of a job take 900, with its exponentials alone left out 1,070; the 128 exponentials of a row take 1,024 on the SM's 16 MUFU lanes.
+// hand-overs of a job take 900, with its exponentials alone left out 1,090; the 128 exponentials of a row take 1,024 on the SM's 16 MUFU lanes.
 // Two groups' warps spend two thirds of a job in waits and loads; a third one takes turns with them where tiles are long enough (kThreeGroupKeys):
 // l1, B=2 H=4 N=65536: 692 us with two, 669 with three; two levels, H=6 N=262144: 620 -> 590; B=2 H=4 N=65536: 90 -> 85.  No gain from: two
 // groups that load a whole row of scores at once and hand the S buffer back before the exponentials (732: fewer warps for the MUFU); a quarter
