@@ -111,8 +111,8 @@ __device__ __forceinline__ void init_bars(LoopBars& bars) {
 }
 
 // n_chunks: chunks per tile; gathered: how many of them, the first ones, are gathered level-1 blocks (two levels); n_c: rows per
-// head of the contiguous pooled tensor.  REM: the fine part of o is the bf16 value in o plus its remainder in a.rem.
-template <bool REM, int GROUPS>
+// head of the contiguous pooled tensor.  REM: the fine part of o is the bf16 value in o plus its remainder in a.rem; AHEAD: the launch.
+template <bool REM, int GROUPS, bool AHEAD = false>
 __global__ void __launch_bounds__(Split<GROUPS>::kThreads, 1)
 attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps maps, int n_chunks, int gathered, int64_t n_c, int n_tiles,
                                int tiles_per_head, unsigned char* redo) {
@@ -392,9 +392,14 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         bf16* orow = a.o.row(bh / a.H, bh % a.H, row);
         float* lse_p = a.lse + (int64_t) bh * a.Nq + row;
         // the fine part of this row, and whether the second round owns it: requested before the waits
-        uint4 of[8];
+        uint4 of[8], rest[4];                // rest: half a row of the remainder
+        const uint4* rp = REM ? reinterpret_cast<const uint4*>(a.rem + ((int64_t) bh * a.Nq + row) * kD) : nullptr;
 #pragma unroll
         for (int q8 = 0; q8 < 8; ++q8) of[q8] = *reinterpret_cast<const uint4*>(orow + 8 * q8);
+        if (REM && AHEAD) {
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) rest[q4] = rp[q4];
+        }
         const float lse_f = *lse_p;
         bool mine = true;
         if (redo && n_pass == 2) mine = redo[(int64_t) bh * a.Nq + row] != 0;
@@ -418,11 +423,9 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           float va[32];
-          uint4 rest[4];
-          if (REM) {
-            const uint4* rp = reinterpret_cast<const uint4*>(a.rem + ((int64_t) bh * a.Nq + row) * kD + half * 32);
+          if (REM && !AHEAD) {
 #pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) rest[q4] = rp[q4];
+            for (int q4 = 0; q4 < 4; ++q4) rest[q4] = rp[half * 4 + q4];
           }
           tc::tmem_ld32_async(tmem + kColO + (i & 1) * 64 + half * 32 + ((uint32_t) (qd * 32) << 16), va);
           tc::tmem_ld_wait(va);
@@ -438,11 +441,13 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
               const float x = REM ? bf16_lo(fine) + bf16_lo(left) : bf16_lo(fine), y = REM ? bf16_hi(fine) + bf16_hi(left) : bf16_hi(fine);
               return pack_bf16(x * wf + va[8 * q4 + e] * wp, y * wf + va[8 * q4 + e + 1] * wp);
             };
+            const uint4 left = rest[q4];
+            if (REM && AHEAD && half == 0) rest[q4] = rp[4 + q4];      // the second half's, a half ahead
             uint4 w;
-            w.x = merged(f.x, rest[q4].x, 0);
-            w.y = merged(f.y, rest[q4].y, 2);
-            w.z = merged(f.z, rest[q4].z, 4);
-            w.w = merged(f.w, rest[q4].w, 6);
+            w.x = merged(f.x, left.x, 0);
+            w.y = merged(f.y, left.y, 2);
+            w.z = merged(f.z, left.z, 4);
+            w.w = merged(f.w, left.w, 6);
             if (mine) *reinterpret_cast<uint4*>(orow + half * 32 + 8 * q4) = w;
           }
         }
@@ -500,12 +505,17 @@ int launch_attn_fwd_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
   LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int grid = n_tiles < sms ? n_tiles : sms;
   const size_t smem = 1024 + (size_t) (2 + kKStages + kVStages) * kTile * sizeof(bf16);
+  // AHEAD, for lists with a remainder in one pass on two groups: the epilogue is the pace there, and the remainder's first half row requested with the
+  // fine part, ahead of the waits, takes one memory latency out of every tile.  Whole forward in us, without / with: two levels, B=2 H=6 N=49152 288 /
+  // 277 (284 before there was a third group), N=40960, 288 keys, 274 / 265, 416 keys, H=5, 167.9 / 168.4.  In two passes it costs: H=5 N=40960, 224 and
+  // 256 keys, 126 / 128 and 128 / 131.
   const bool three = (a.p1_blocks + a.p2_blocks) * kBS >= (a.rem ? kThreeGroupKeysRem : kThreeGroupKeys);
+  unsigned char* redo = g->fwd_redo && pooled_loop_one_pass(a) ? reinterpret_cast<unsigned char*>(g->fwd_redo->ptr) : nullptr;
   auto kernel = three ? (a.rem ? attn_fwd_pooled_loop_tc_kernel<true, 3> : attn_fwd_pooled_loop_tc_kernel<false, 3>)
-                      : (a.rem ? attn_fwd_pooled_loop_tc_kernel<true, 2> : attn_fwd_pooled_loop_tc_kernel<false, 2>);
+                : !a.rem ? attn_fwd_pooled_loop_tc_kernel<false, 2>
+                : redo ? attn_fwd_pooled_loop_tc_kernel<true, 2, true> : attn_fwd_pooled_loop_tc_kernel<true, 2>;
   const int threads = three ? Split<3>::kThreads : Split<2>::kThreads;
   LLSA_SMEM_LIMIT_REGS(kernel, smem, three ? Split<3>::kLaunch : 0);
-  unsigned char* redo = g->fwd_redo && pooled_loop_one_pass(a) ? reinterpret_cast<unsigned char*>(g->fwd_redo->ptr) : nullptr;
   launch_pdl(kernel, grid, threads, smem, st, a, maps, n_chunks, gathered, n_c, n_tiles, tiles_per_head, redo);
   LLSA_LAUNCH_OK("attn_fwd_pooled_loop_tc_kernel");
   return LLSA_OK;
