@@ -1,6 +1,8 @@
 // Argument validation and dispatch of the attention entry points.
 #include <string.h>
 
+#include <algorithm>
+
 #include "attn.cuh"
 
 namespace llsa {
@@ -129,7 +131,10 @@ extern "C" int64_t llsa_attn_remainder_elems(const LlsaAttnArgs* g, int backward
 extern "C" int64_t llsa_attn_bwd_partial_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk) {
   if (B <= 0 || H <= 0 || Nq <= 0 || topk <= 0) return 0;
   const int64_t ranges = (Nq / kBS * topk + kRangeEntriesSmall - 1) / kRangeEntriesSmall;     // sized for the smaller of the two range sizes
-  return B * H * ((ranges + 3) / 4) * 4096;          // a head and a tail tile (2048 floats each) per CTA of four ranges
+  // a head and a tail tile (2048 floats each) per window of four small ranges, or per span (problems of fewer than 256 entries: long spans)
+  const int64_t windows = B * H * ((ranges + 3) / 4), total = B * H * (Nq / kBS) * topk;
+  const int64_t spans = total < 256 ? 0 : std::min<int64_t>((total + kSpanEntries - 1) / kSpanEntries, kMaxSpans);
+  return std::max(windows, (spans + B * H - 1) / (B * H) * (B * H)) * 4096;      // a multiple of B H tiles: the tensor is [B,H,.,4096]
 }
 
 extern "C" int64_t llsa_attn_bwd_pds_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk) {

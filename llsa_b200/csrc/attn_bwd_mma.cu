@@ -29,6 +29,7 @@
 // here scale rides in the exp2 argument and in the epilogues.
 #include <string.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "attn.cuh"
@@ -454,8 +455,8 @@ __global__ void __launch_bounds__(NW * 32, 1) attn_dkv_pooled_kernel(AttnP<bf16>
 // block.  Fan-in is very uneven (0 ... >150 on correlated inputs), so the work is cut by ENTRIES, not by buckets: the
 // index transpose cuts the list into ranges of nominally kRangeEntries entries, one per warp, moving a cut that would
 // fall inside a bucket of at most kRangeEntries entries to that bucket's start.  Most buckets are therefore finished
-// by one warp; longer ones are cut at multiples of kRangeEntries and their pieces meet in shared memory (same CTA) or
-// in the `partial` scratch (summed in window order by the finish kernel).  No atomics: bit-reproducible.
+// by one warp; longer ones are cut at multiples of kRangeEntries and their pieces meet in the `partial` scratch (summed in window order by the
+// finish kernel).  Small problems are cut into equal spans instead.  No atomics: bit-reproducible.
 constexpr int kTileFloats = 64 * 32;            // a parked dK + dV tile pair: 64 accumulators x 32 lanes (8 KB)
 
 __device__ __forceinline__ int64_t csr_off(const AttnP<bf16>& a, int64_t bh, int64_t j) {
@@ -496,12 +497,14 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 //   * The Q / dO tiles of an entry come through a per-warp ring of kRingFineStages stages, two entries ahead, as two TMA copies issued
 //     by one lane (plus one 4-byte copy per lane: lse and delta); K, V and the pooled-gradient rows of the next bucket through a buffer
 //     of their own, requested as soon as those of the bucket at hand sit in registers.
-//   * Two forms.  PERSISTENT (ranges of kRangeEntries, i.e. problems of some 4,700 ranges and more): one CTA of twelve warps per SM; a
-//     window is two ranges, a warp draws one range after another from a counter in shared memory, and where a long bucket crosses from
-//     the first range of a window into the second one warp takes both.  Otherwise (ranges of half that size): one CTA of four warps per
-//     window of four ranges, every range on a warp at once; a warp parks the tile of a bucket it shares with EARLIER warps in its
-//     shared-memory slot, the tile it shares with later ones stays in its accumulators until the CTA has synchronised.
-//     Pieces of buckets that straddle windows go to the `partial` scratch and attn_dkv_finish_kernel adds them in window order.
+//   * One CTA of twelve warps per SM, in two forms.  Windows (ranges of kRangeEntries, i.e. problems of some 4,700 ranges and more): a window is two
+//     ranges, a warp draws one range after another from a counter in shared memory, and where a long bucket crosses from the first range of a
+//     window into the second one warp takes both.  All SMs work on neighbouring entries at any time, so that the tiles stay in L2.  Spans (smaller
+//     problems, whose tensors L2 holds anyway): the entries of all heads, one head behind the other, are cut into equal spans, one per warp, wherever
+//     the cut falls: every warp begins once, and all end together.  As CTAs of four warps, each with a range of 16 entries and its own start, two CTAs
+//     an SM, these problems took 63 us instead of 48 (one level, B=4 H=6 N=4096), 55 / 44 (two levels, B=3 H=5 N=5376), 78 / 60 (one level, B=2 H=4
+//     N=16384).
+//     Pieces of buckets that straddle windows or spans go to the `partial` scratch and attn_dkv_finish_kernel adds them in order.
 // What bounds it: latency.  0.42 instructions per scheduler and cycle: 58 % of the issue slots stay empty with three warps on a scheduler, each on
 // one serial chain (wait, S and dP, exponentials, the two products: some 290 instructions per entry); then the raggedness of the last ranges.
 // 168 registers in the persistent form, 4 bytes of them spilled.  With P and dS handed over by the dQ stage instead of recomputed this kernel issued half as much,
@@ -509,8 +512,7 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 // on random inputs, 207 -> 164 and 284 -> 255 on correlated ones; at 6 of 262144 421 -> 315 and 563 -> 460 (the first figures of the
 // correlated pairs with eight warps per SM in groups of four that waited for the longest of their ranges: 322 and 645 on random inputs).
 // Accumulator layout (ldmatrix): tile u holds channels 8u + 2t, 8u + 2t + 1 of keys g (c0, c1) and g + 8 (c2, c3).
-constexpr int kRingWarps = 4;                   // warps per CTA, one window per CTA
-constexpr int kRingWarpsP = 12;                 // warps per CTA, one persistent CTA per SM
+constexpr int kRingWarps = 12;                  // warps per CTA, one CTA per SM
 constexpr int kRingFineStages = 3;
 constexpr int kRingFineStageBytes = 2 * kRingTileBytes;                                // Q tile, dO tile
 constexpr int kRingTilesBytes = (kRingFineStages + 1) * kRingFineStageBytes;           // per warp: the ring, then K and V tile of the next bucket
@@ -522,6 +524,10 @@ constexpr int kRingWindow = 64;                 // nominal entries per window: t
 struct FineMaps {
   CUtensorMap q, d_o, k, v;    // [B,H,N,64] 4-D, box 16 rows
 };
+
+// SPANS: the entries of all heads, one head behind the other, in n equal pieces; the piece that holds entry p.
+__host__ __device__ __forceinline__ int64_t span_begin(int64_t i, int64_t n, int64_t total) { return total * i / n; }
+__device__ __forceinline__ int span_of(int64_t p, int64_t n, int64_t total) { return (int) (((p + 1) * n + total - 1) / total - 1); }
 
 // Pooling-backward fold and scale for the ldmatrix accumulator layout: afterwards dk / dv hold the final fp32 values.  The gradient rows
 // [dpk | dpv | dpk2 | dpv2] x 64 fp32 of the bucket lie at `fold`; a lane first combines four channels of one tensor in place.
@@ -591,18 +597,17 @@ __device__ __forceinline__ void dkv_fine_store_staged(const AttnP<bf16>& a, int6
   tc::fence_async_smem();                 // the stage is refilled by the asynchronous proxy
 }
 
-template <bool PERSISTENT>
-__global__ void __launch_bounds__((PERSISTENT ? kRingWarpsP : kRingWarps) * 32, PERSISTENT ? 1 : 2)
-attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, float* __restrict__ partial, int n_windows, int64_t n_total) {
-  constexpr int NW = PERSISTENT ? kRingWarpsP : kRingWarps;
+// SPANS: n_pieces = spans, n_total = entries of all heads; otherwise n_pieces = windows per head, n_total = windows of all heads.
+template <bool SPANS>
+__global__ void __launch_bounds__(kRingWarps * 32, 1)
+attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, float* __restrict__ partial, int n_pieces, int64_t n_total) {
+  constexpr int NW = kRingWarps;
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t s_full[NW][kRingFineStages + 1];       // the ring's stages, then the next bucket's K / V
   __shared__ tc::WaitCtl s_ctl;
-  __shared__ int s_head_bucket[NW];
   __shared__ int s_next;
   // swizzled tiles: 1024-byte aligned
   unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
-  float* slots = reinterpret_cast<float*>(smem + NW * kRingWarpBytes);   // !PERSISTENT: [kRingWarps][kTileFloats], tile of the bucket a warp shares with earlier warps
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   volatile tc::WaitCtl* ctl = &s_ctl;
   if (threadIdx.x == 0) {
@@ -610,7 +615,6 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
     s_ctl.limit = a.wait_limit > 0 ? a.wait_limit : tc::kWaitPolls;
     s_next = 0;
   }
-  if (threadIdx.x < NW) s_head_bucket[threadIdx.x] = -1;
   if (threadIdx.x < NW * (kRingFineStages + 1)) tc::mbar_init(&s_full[0][0] + threadIdx.x, 1);
   tc::fence_mbar_init();
   pdl_trigger();
@@ -633,52 +637,58 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
   const float sl2 = a.scale * kLog2e;
   float dk[8][4], dv[8][4];
   RowFrag klo, khi, vlo, vhi;               // K and V of the bucket at hand, as A operands
-  int tail_j = -1;                          // !PERSISTENT: bucket whose tile is still in dk / dv after the loop
   int st = 0, ph = 0;                       // ring stage of the entry at hand, parity of its fill
   int kvph = 0, fold_buf = 0;               // parity of the next K / V fill, fold buffer of the bucket at hand
-  int64_t bh = blockIdx.y;
-  int ce = 0;
   // entries the CSR really holds: fewer than E when the transpose dropped out-of-range indices; ranges and offsets handed in
   // by a caller are not trusted further than these clamps and the bounds on the bucket walk below
-  auto cut = [&](int r, int used) { return r < R ? min(max(__ldcg(&a.ranges[bh * R + r].x), 0), used) : used; };
-  // A span of the entry list.  !PERSISTENT: one range per warp, one window per CTA.  PERSISTENT: the warps of a CTA draw one range after
-  // another; a range that begins inside a bucket is left to the warp that has the range in front of it, unless it opens a window.
+  auto cut = [&](int64_t bh, int r, int used) { return r < R ? min(max(__ldcg(&a.ranges[bh * R + r].x), 0), used) : used; };
+  // SPANS: the warp's own, a head at a time.  Otherwise the warps of a CTA draw one range after another; a range that begins inside a bucket is
+  // left to the warp that has the range in front of it, unless it opens a window.
+  const int span = warp * (int) gridDim.x + (int) blockIdx.x;
+  int bh = 0, rb = 0, left = 0;              // SPANS: head and first entry of the next piece, entries left of the span
+  if (SPANS && span < n_pieces) {
+    const int64_t f = span_begin(span, n_pieces, n_total);
+    left = (int) (span_begin(span + 1, n_pieces, n_total) - f);
+    bh = (int) (f / E) - 1;
+    rb = (int) (f - (int64_t) (bh + 1) * E);
+  }
   bool ok = true;
-  for (bool more = true; ok && more; more = PERSISTENT) {
-    int r0, rb, re;
-    if (PERSISTENT) {
+  while (ok) {
+    int re, r0;                              // entries [rb, re) of head bh; the range that rb is looked up by
+    if constexpr (SPANS) {
+      if (left <= 0) break;
+      ++bh;
+      re = min(E, rb + left);
+      left -= re - rb;
+      re = min(re, (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1))));
+      r0 = rb / a.range_entries;
+    } else {
       int k = 0;
       if (lane == 0) k = atomicAdd(&s_next, 1);
       k = __shfl_sync(0xffffffffu, k, 0);
       const int64_t u = blockIdx.x + (int64_t) (k >> 1) * gridDim.x;        // both ranges of a window: a left-over range is work for its neighbour
       if (u >= n_total) break;
-      bh = u / n_windows;
-      r0 = (int) (u % n_windows) * 2 + (k & 1);
+      bh = (int) (u / n_pieces);
+      r0 = (int) (u % n_pieces) * 2 + (k & 1);
       if (r0 >= R) continue;
-    } else {
-      r0 = blockIdx.x * kRingWarps + warp;
-    }
-    const int E_used = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1)));
-    if (PERSISTENT) {
+      const int E_used = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1)));
       auto begins_inside = [&](int r) {
         const int2 x = __ldcg(&a.ranges[bh * R + r]);
         return (int) csr_off(a, bh, min(max(x.y, 0), n1 - 1)) < x.x;
       };
       const bool odd = r0 & 1, both = (odd || r0 + 1 < R) && begins_inside(r0 | 1);
       if (odd && both) continue;
-      rb = cut(r0, E_used);
-      re = max(cut(r0 + (both ? 2 : 1), E_used), rb);
-    } else {
-      const int cb = cut(blockIdx.x * kRingWarps, E_used);
-      ce = max(cut((blockIdx.x + 1) * kRingWarps, E_used), cb);
-      rb = min(max(cut(r0, E_used), cb), ce);
-      re = min(max(cut(r0 + 1, E_used), rb), ce);
+      rb = cut(bh, r0, E_used);
+      re = max(cut(bh, r0 + (both ? 2 : 1), E_used), rb);
     }
-    const int win = PERSISTENT ? r0 / (kRingWindow / kRangeEntries) : (int) blockIdx.x;
-    if (rb >= re) continue;
-    const int64_t b = bh / a.H, h = bh % a.H;
-    float* const pieces = partial + (bh * n_windows + win) * 2 * (int64_t) kTileFloats;     // the window's head and tail slots
-    const int32_t* fl = a.flat + bh * (int64_t) E;
+    if (rb >= re) {
+      if (SPANS) rb = 0;
+      continue;
+    }
+    const int b = bh / (int) a.H, h = bh % (int) a.H;
+    // the span's or the window's head and tail slots
+    float* const pieces = partial + (SPANS ? (int64_t) span : (int64_t) bh * n_pieces + r0 / (kRingWindow / kRangeEntries)) * 2 * (int64_t) kTileFloats;
+    const int32_t* fl = a.flat + (int64_t) bh * E;
     const int n = re - rb;
     // lane i: query block of entry 32 c + i of the chunk c being requested and of the one after it (clamped: nothing is read outside the
     // tensors)
@@ -752,8 +762,7 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
           if (!began_before) {
             dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, rst * kRingFineStageBytes, fold_sa + fold_buf * kRingFoldBytes, lane);
           } else {                                    // began in an earlier span
-            tile_to_mem(PERSISTENT ? pieces : slots + warp * kTileFloats, dk, dv, lane);
-            if (!PERSISTENT && lane == 0) s_head_bucket[warp] = j;
+            tile_to_mem(pieces, dk, dv, lane);
           }
           began_before = false;
         }
@@ -819,35 +828,13 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
     // the last bucket of the span; the ring is idle by now
     if (!began_before && nxt <= re) {
       dkv_fine_store_staged(a, b, h, j, dk, dv, sa_m, sa_cp, 0, fold_sa + fold_buf * kRingFoldBytes, lane);
-    } else if (PERSISTENT) {
-      tile_to_mem(pieces + (began_before ? 0 : kTileFloats), dk, dv, lane);     // lies across the whole window or ends here, or continues in the next
-    } else if (began_before) {
-      tile_to_mem(slots + warp * kTileFloats, dk, dv, lane);
-      if (lane == 0) s_head_bucket[warp] = j;
     } else {
-      tail_j = j;                           // continues in later warps (or windows): completed below
+      tile_to_mem(pieces + (began_before ? 0 : kTileFloats), dk, dv, lane);     // reaches back or across, or continues in the next
     }
+    if (SPANS) rb = 0;                       // what is left is the next head's
   }
   if (!ok) tc::abort_drain();
   __syncthreads();
-  if (!PERSISTENT) {
-    const int64_t b = bh / a.H, h = bh % a.H;
-    float* const pieces = partial + (bh * n_windows + blockIdx.x) * 2 * (int64_t) kTileFloats;
-    if (tail_j >= 0) {
-      for (int w = warp + 1; w < kRingWarps && s_head_bucket[w] == tail_j; ++w) tile_add_mem(slots + w * kTileFloats, dk, dv, lane);
-      if ((int) csr_off(a, bh, tail_j + 1) <= ce) {
-        dkv_fine_store_staged(a, b, h, tail_j, dk, dv, sa_m, sa_cp, 0, fold_sa + fold_buf * kRingFoldBytes, lane);
-      } else {                                // runs on into the next window: this window's tail slot
-        tile_to_mem(pieces + kTileFloats, dk, dv, lane);
-      }
-    }
-    if (warp == 0 && s_head_bucket[0] >= 0) { // began in an earlier window: this window's head slot
-      const int j0 = s_head_bucket[0];
-      tile_zero(dk, dv);
-      for (int w = 0; w < kRingWarps && s_head_bucket[w] == j0; ++w) tile_add_mem(slots + w * kTileFloats, dk, dv, lane);
-      tile_to_mem(pieces, dk, dv, lane);
-    }
-  }
   if (threadIdx.x == 0 && s_ctl.abort && a.status) atomicOr(a.status, (int) LLSA_DEV_WAIT_EXPIRED);
 }
 
@@ -896,39 +883,62 @@ __device__ __forceinline__ void dkv_store_unselected(const AttnP<bf16>& a, int64
   }
 }
 
-// Buckets whose pieces lie in several windows of the kernel above.  Each of them crosses a window boundary, and a boundary lies in one
-// bucket: one CTA per boundary looks up that bucket (the transpose kernel left it beside the range that starts there), leaves unless
-// this is the first boundary the bucket crosses, and adds the pieces in window order: the tail of the window the bucket begins in, then
+// Buckets whose pieces lie in several windows (spans) of the kernel above.  Each of them crosses a boundary, and a boundary lies in one
+// bucket: one CTA per boundary looks up that bucket (the transpose kernel left it beside the range that starts there, or in front), leaves unless
+// this is the first boundary the bucket crosses, and adds the pieces in order: the tail of the window the bucket begins in, then
 // the heads.  A warp owns 32 channels of one tensor, so a piece is four 128-bit loads per lane, four pieces in flight.
-// blockIdx.x >= n_windows - 1: the unselected blocks, 16 per CTA -- stores at the memory's rate next to the latency of the lookups (as extra
+// The first n_plain * BH CTAs: the unselected blocks, 16 per CTA -- stores at the memory's rate next to the latency of the lookups (as extra
 // CTAs or extra work of the kernel above they cost twice as much: two CTAs of it fill an SM).
 // One warp for eight buckets, looking for both kinds, took 46 us at 48 slices of 16384 tokens and 160 us at 6 of 262144; this kernel 31
 // and 81.
-__global__ void __launch_bounds__(128) attn_dkv_finish_kernel(AttnP<bf16> a, const float* __restrict__ partial, int n_windows) {
-  if ((int) blockIdx.x >= n_windows - 1) {
-    const int first = (((int) blockIdx.x - (n_windows - 1)) * 4 + (int) (threadIdx.x >> 5)) * kPlainPerWarp;
-    dkv_store_unselected(a, blockIdx.y / a.H, blockIdx.y % a.H, blockIdx.y, first, threadIdx.x & 31);
+__global__ void __launch_bounds__(128) attn_dkv_finish_kernel(AttnP<bf16> a, const float* __restrict__ partial, unsigned n_plain, unsigned BH, int n_spans) {
+  if (blockIdx.x < n_plain * BH) {
+    const int bh = (int) (blockIdx.x / n_plain), first = ((int) (blockIdx.x % n_plain) * 4 + (int) (threadIdx.x >> 5)) * kPlainPerWarp;
+    dkv_store_unselected(a, bh / a.H, bh % a.H, bh, first, threadIdx.x & 31);
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n1 = (int) a.n1;
-  const int64_t bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
-  const int E = (int) (a.nq1 * a.topk), range = a.range_entries, window = kRingWindow;
-  const int R = (E + range - 1) / range, edge = ((int) blockIdx.x + 1) * window;
+  const int E = (int) (a.nq1 * a.topk), range = a.range_entries, R = (E + range - 1) / range;
+  const unsigned boundary = blockIdx.x - n_plain * BH;
   // offsets are clamped to [0, E] and to each other: a malformed CSR cannot send the arithmetic below outside `partial`
-  const int j = min(max(__ldcg(&a.ranges[bh * R + edge / range].y), 0), n1 - 1);
-  const int bo = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, j))), be = (int) min((int64_t) E, max((int64_t) bo, csr_off(a, bh, j + 1)));
-  if (be - bo <= range || bo >= edge || be <= edge || bo / window != (int) blockIdx.x) return;
-  const int c_first = bo / window, c_last = min((be - 1) / window, n_windows - 1);
+  int64_t bh;
+  int j, c_first, c_last;
+  if (n_spans > 0) {
+    const int64_t total = (int64_t) BH * E, f = span_begin(boundary + 1, n_spans, total);
+    bh = f / E;
+    const int e = (int) (f - bh * E);
+    if (e == 0) return;
+    int j0 = min(max(__ldcg(&a.ranges[bh * R + e / range].y), 0), n1 - 1), c;      // its bucket begins at or in front of e
+    while ((c = __popc(__ballot_sync(0xffffffffu, j0 + 1 + lane <= n1 && (int) csr_off(a, bh, j0 + 1 + lane) <= e))) == 32) j0 += 32;
+    j = min(j0 + c, n1 - 1);
+    const int bo = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, j))), be = (int) min((int64_t) E, max((int64_t) bo, csr_off(a, bh, j + 1)));
+    if (bo >= e || be <= e) return;
+    c_first = span_of(bh * E + bo, n_spans, total);
+    if (c_first != (int) boundary) return;
+    c_last = min(span_of(bh * E + be - 1, n_spans, total), n_spans - 1);
+    partial += (int64_t) c_first * 2 * kTileFloats;
+  } else {
+    const int window = kRingWindow, n_windows = (E + window - 1) / window, at = (int) (boundary % (n_windows - 1)), edge = (at + 1) * window;
+    bh = boundary / (n_windows - 1);
+    j = min(max(__ldcg(&a.ranges[bh * R + edge / range].y), 0), n1 - 1);
+    const int bo = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, j))), be = (int) min((int64_t) E, max((int64_t) bo, csr_off(a, bh, j + 1)));
+    if (be - bo <= range || bo >= edge || be <= edge || bo / window != at) return;
+    c_first = bo / window;
+    c_last = min((be - 1) / window, n_windows - 1);
+    partial += (bh * n_windows + c_first) * 2 * (int64_t) kTileFloats;
+  }
+  const int64_t b = bh / a.H, h = bh % a.H;
+  c_last -= c_first;                                                   // pieces behind the first one
   const int ten = warp >> 1, u0 = (warp & 1) * 4;                      // tiles u0 .. u0 + 3 of dk / dv: tile u holds channels 8u + 2t, +1 of rows g, g + 8
   float acc[4][4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.f;
-  for (int c0 = c_first; c0 <= c_last; c0 += 4) {
+  for (int c0 = 0; c0 <= c_last; c0 += 4) {
     float4 x[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int c = min(c0 + i, c_last);
-      const float4* p = reinterpret_cast<const float4*>(partial + ((bh * n_windows + c) * 2 + (c == c_first ? 1 : 0)) * (int64_t) kTileFloats) + (8 * ten + u0) * 32 + lane;
+      const float4* p = reinterpret_cast<const float4*>(partial + (c * 2 + (c == 0 ? 1 : 0)) * (int64_t) kTileFloats) + (8 * ten + u0) * 32 + lane;
 #pragma unroll
       for (int u = 0; u < 4; ++u) x[i][u] = __ldcg(p + u * 32);
     }
@@ -1034,23 +1044,25 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     if ((rc = tma::make_map_bhnd(&maps.d_o, g->d_o, kBS))) return rc;
     if ((rc = tma::make_map_bhnd(&maps.k, g->k, kBS))) return rc;
     if ((rc = tma::make_map_bhnd(&maps.v, g->v, kBS))) return rc;
+    int dev = 0, sms = 148;
+    LLSA_CUDA_OK(cudaGetDevice(&dev));
+    LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const size_t ring = (size_t) kRingWarps * kRingWarpBytes + 1024;
+    int n_spans = 0;
     if (a.range_entries == kRangeEntries) {
-      int dev = 0, sms = 148;
-      LLSA_CUDA_OK(cudaGetDevice(&dev));
-      LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      static_assert(kRingWindow == 2 * kRangeEntries, "a window of the persistent form is two ranges");
+      static_assert(kRingWindow == 2 * kRangeEntries, "a window is two ranges");
       const int64_t total = (int64_t) n_windows * BH;
-      const size_t ring = (size_t) kRingWarpsP * kRingWarpBytes + 1024;
-      LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel<true>), ring);
-      launch_pdl(attn_dkv_fine_ring_kernel<true>, dim3((unsigned) (total < sms ? total : sms)), kRingWarpsP * 32, ring, st, a, maps, partial, n_windows, total);
+      LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel<false>), ring);
+      launch_pdl(attn_dkv_fine_ring_kernel<false>, dim3((unsigned) (total < sms ? total : sms)), kRingWarps * 32, ring, st, a, maps, partial, n_windows, total);
     } else {
-      const size_t smem = 1024 + (size_t) kRingWarps * (kRingWarpBytes + kTileFloats * sizeof(float));
-      LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel<false>), smem);
-      launch_pdl(attn_dkv_fine_ring_kernel<false>, dim3((unsigned) n_windows, BH), kRingWarps * 32, smem, st, a, maps, partial, n_windows, (int64_t) 0);
+      const int64_t total = E * BH, room = g->dkv_partial->shape[0] * g->dkv_partial->shape[1] * g->dkv_partial->shape[2] * g->dkv_partial->shape[3] / (2 * kTileFloats);
+      n_spans = (int) std::min({(total + kSpanEntries - 1) / kSpanEntries, (int64_t) sms * kRingWarps, room});
+      LLSA_SMEM_LIMIT((attn_dkv_fine_ring_kernel<true>), ring);
+      launch_pdl(attn_dkv_fine_ring_kernel<true>, dim3((unsigned) std::min(n_spans, sms)), kRingWarps * 32, ring, st, a, maps, partial, n_spans, total);
     }
     LLSA_LAUNCH_OK("attn_dkv_fine_ring_kernel");
-    const int n_plain = (int) ((a.n1 + 4 * kPlainPerWarp - 1) / (4 * kPlainPerWarp));
-    attn_dkv_finish_kernel<<<dim3((unsigned) (n_windows - 1 + n_plain), BH), 128, 0, st>>>(a, partial, n_windows);
+    const unsigned n_plain = (unsigned) ((a.n1 + 4 * kPlainPerWarp - 1) / (4 * kPlainPerWarp)), boundaries = n_spans ? (unsigned) n_spans - 1 : (unsigned) (n_windows - 1) * BH;
+    attn_dkv_finish_kernel<<<dim3(n_plain * BH + boundaries), 128, 0, st>>>(a, partial, n_plain, BH, n_spans);
     LLSA_LAUNCH_OK("attn_dkv_finish_kernel");
   }
   return LLSA_OK;

@@ -81,9 +81,11 @@ int raise_smem_limit(const void* kernel, size_t bytes, int launch_regs = 0);
 // Nominal entries per work range of the fine dK/dV kernel: the index transpose cuts the CSR entry list into ranges of this
 // many entries (transpose.cu), one warp of attn_dkv_fine_ring_kernel walks one range (attn_bwd_mma.cu).
 constexpr int kRangeEntries = 32;
-// Small problems are cut into ranges of half that size, so that the dK/dV kernel still fills the SMs (llsa_transpose_range_entries draws
-// the line): the range size travels with the `ranges` tensor, whose length names it.
+// Small problems are cut into ranges of half that size (llsa_transpose_range_entries draws the line): the range size travels with the `ranges`
+// tensor, whose length names it.  The dK/dV kernel takes their entries in equal spans, one per warp, of at least kSpanEntries entries, and looks the
+// bucket of a cut up in the ranges.  kMaxSpans: twelve warps on each of 148 SMs.
 constexpr int kRangeEntriesSmall = 16;
+constexpr int kSpanEntries = 16, kMaxSpans = 148 * 12;
 // Range size S that a ranges tensor of R ranges over E entries was cut with (0: neither size fits)
 inline int range_entries_of(int64_t E, int64_t R) {
   if ((E + kRangeEntries - 1) / kRangeEntries == R) return kRangeEntries;

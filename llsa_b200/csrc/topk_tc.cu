@@ -1,0 +1,301 @@
+// Coarse selection of long lists on tcgen05 (bf16, D = 64, top-k <= 8): gen_sparse_indices (topk.py:6-9), scores rounded to bf16.
+//
+// A CTA owns 128 query rows and walks the head's keys twice, 128 at a time (a job):  S = Q.K_c^T  [128 x 128] into tensor memory, thread = query row.
+//   * Pass 1 keeps the maxima of 16 interleaved groups of columns per thread, 32 per row; the eighth largest bounds the row's eighth score from
+//     below, and some nine scores of a row reach it, whatever its length.
+//   * Pass 2 computes the same scores again and looks, eight columns at a time, only at what reaches the bound: candidates as words (topk_words.cuh)
+//     are set aside in shared memory and sorted at the end (inserted at once, with the warp's other rows waiting, they are half of the kernel's time).
+// Two warpgroups take alternate jobs (odd and even), each with two score buffers of its own, half a job each, so that the products of one half run while
+// the other is looked at; they share a row's bound and merge its two lists through
+// shared memory.  Roles: warps 0-3 / 4-7 the two groups, warp 8 TMA producer (queries once, a ring of 4 key chunks), warp 9 issues the products.
+// What bounds it: the comparisons, 64 maxima a thread and job in either pass next to 256 cycles of tensor pipe; two CTAs share an SM, so that one's hand-overs
+// are hidden by the other's work.
+// Every mbarrier wait is bounded.  A CTA whose wait expires computes its rows with scalar arithmetic instead (slowly, and with another order of the
+// sums): a selection that went missing would not show in anything downstream.
+#include <string.h>
+
+#include "mma_frag.cuh"
+#include "tc05.cuh"
+#include "tma.cuh"
+#include "topk_words.cuh"
+
+namespace llsa {
+
+namespace {
+
+constexpr int kRows = 128, kChunk = 128;
+constexpr int kTile = kRows * 64;            // elements of a [128 x 64] bf16 tile (16 KB)
+constexpr int kStages = 3;
+constexpr int kThreads = 320;
+constexpr int kGroups = 16;                  // column groups of a thread in pass 1
+constexpr int kHits = 24;                    // scores of a row and group that pass 2 sets aside before it takes them one by one
+
+struct CoarseMaps {
+  CUtensorMap q, k;           // contiguous [BH*M, 64], [BH*n, 64], box 128 rows
+};
+
+struct CoarseBars {
+  uint64_t q_full, k_full[kStages], k_empty[kStages], s_ready[4], s_free[4];      // scores: by group and half of a job
+};
+
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {      // NaN if one of them is
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+__device__ __forceinline__ void store_list(void* idx_out, int idx64, int64_t at, int topk, const uint32_t (&list)[kCmTop]) {
+#pragma unroll
+  for (int u = 0; u < kCmTop; ++u)
+    if (u < topk) {
+      const uint32_t col = 65535u - (list[u] & 0xFFFFu);
+      if (idx64) reinterpret_cast<int64_t*>(idx_out)[at + u] = (int64_t) col;
+      else reinterpret_cast<int32_t*>(idx_out)[at + u] = (int32_t) col;
+    }
+}
+
+// n: a multiple of 64, at most 65536, at least kGroups * 32
+__global__ void __launch_bounds__(kThreads, 2)
+coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __restrict__ pq, const bf16* __restrict__ pk, void* __restrict__ idx_out,
+                      int idx64, int64_t M, int64_t n, int topk, int wait_limit) {
+  extern __shared__ unsigned char smem_dyn[];
+  __shared__ CoarseBars bars;
+  __shared__ uint32_t s_tmem;
+  __shared__ tc::WaitCtl s_ctl;
+  __shared__ uint32_t s_list[2][kRows][kHits + 1];       // + 1: a row's words walk the banks.  The groups' best maxima, what reaches the bound, their lists
+  bf16* sQ = reinterpret_cast<bf16*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));      // [128][64]
+  bf16* sK = sQ + kTile;                                 // [kStages][128][64]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  volatile tc::WaitCtl* abort_flag = &s_ctl;
+  const int64_t bh = blockIdx.y, row0 = (int64_t) blockIdx.x * kRows;
+  const int chunks = (int) ((n + kChunk - 1) / kChunk), jobs = 2 * chunks;
+  if (tid == 0) {
+    s_ctl.abort = 0;
+    s_ctl.limit = wait_limit > 0 ? wait_limit : tc::kWaitPolls;
+    tc::mbar_init(&bars.q_full, 1);
+    for (int i = 0; i < kStages; ++i) { tc::mbar_init(&bars.k_full[i], 1); tc::mbar_init(&bars.k_empty[i], 1); }
+    for (int i = 0; i < 4; ++i) { tc::mbar_init(&bars.s_ready[i], 1); tc::mbar_init(&bars.s_free[i], 4); }
+    tc::fence_mbar_init();
+  }
+  pdl_wait();
+  if (warp == 0) tc::tmem_alloc(&s_tmem, 256);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  pdl_trigger();
+  const uint32_t tmem = s_tmem;
+
+  if (warp == 8) {
+    // ---------------------------------------------------------------- TMA producer
+    tma::expect_tx_w(&bars.q_full, kTile * 2);
+    tma::load_2d_w(sQ, &maps.q, &bars.q_full, 0, (int) (bh * M + row0));      // rows past M: the next head's, or zeros; dropped
+    int st = 0, c = 0;
+    uint32_t ph = 1;
+    for (int j = 0; j < jobs; ++j) {
+      if (!tc::warp_wait(&bars.k_empty[st], ph, abort_flag)) break;
+      tma::expect_tx_w(&bars.k_full[st], kTile * 2);
+      tma::load_2d_w(sK + st * kTile, &maps.k, &bars.k_full[st], 0, (int) (bh * n) + c * kChunk);
+      if (++st == kStages) { st = 0; ph ^= 1; }
+      if (++c == chunks) c = 0;
+    }
+  } else if (warp == 9) {
+    // ---------------------------------------------------------------- products
+    const uint32_t id_s = tc::instr_desc(kRows, kChunk / 2, 0, 0);
+    const uint32_t hi = (uint32_t) (tc::smem_desc(0, 0, 1024) >> 32);
+    auto lo = [](const void* p) { return ((tc::smem_u32(p) >> 4) & 0x3FFFu) | ((16u >> 4) << 16); };
+    constexpr uint32_t kStage = (uint32_t) (kTile * 2) >> 4;
+    const uint32_t lQ = lo(sQ), lK = lo(sK);
+    if (tc::warp_wait(&bars.q_full, 0, abort_flag)) {
+      int st = 0;
+      uint32_t ph = 0;
+      for (int j = 0; j < jobs; ++j) {
+        int half = 0;
+        for (; half < 2; ++half) {
+          const int buf = (j & 1) * 2 + half;
+          // even lanes: the key chunk; odd lanes: the buffer's previous scores have been read
+          const bool b = (lane & 1) && j >= 2;
+          if (!tc::warp_wait(b ? &bars.s_free[buf] : &bars.k_full[st], b ? (uint32_t) ((j >> 1) - 1) & 1 : ph, abort_flag)) break;
+          tc::fence_after_sync();
+          tc::umma_ss_k64(tmem + buf * (kChunk / 2), lQ, hi, lK + st * kStage + half * (kStage / 2), hi, id_s);
+          tc::umma_commit_w(&bars.s_ready[buf]);
+        }
+        if (half < 2) break;
+        tc::umma_commit_w(&bars.k_empty[st]);
+        if (++st == kStages) { st = 0; ph ^= 1; }
+      }
+    }
+  } else {
+    // ---------------------------------------------------------------- comparisons; thread = query row
+    const int wg = warp >> 2, r = (warp & 3) * 32 + lane;
+    const uint32_t t_s = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + wg * kChunk;
+    auto group_sync = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
+    bool ok = true;
+    float v[32];
+    auto ready = [&](int j, int half) {                      // half the scores of job j are there
+      ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.s_ready[wg * 2 + half], (uint32_t) (j >> 1) & 1, abort_flag));
+      tc::fence_after_sync();
+      return ok;
+    };
+    auto quarter = [&](int q4) {                             // 32 columns of them
+      tc::tmem_ld32_async(t_s + 32 * q4, v);
+      tc::tmem_ld_wait(v);
+    };
+    auto give_back = [&](int half) {                         // they have been read
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tma::mbar_arrive(&bars.s_free[wg * 2 + half]);
+    };
+    auto halves = [&](int c) { return (int64_t) (c + 1) * kChunk <= n ? 2 : 1; };      // the last chunk may be half a chunk
+    int j = wg;
+    float m[kGroups];
+#pragma unroll
+    for (int u = 0; u < kGroups; ++u) m[u] = -CUDART_INF_F;
+    for (; ok && j < chunks; j += 2) {
+      const int nh = halves(j);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (!ready(j, half)) break;
+        if (half < nh) {
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            quarter(half * 2 + q);
+            if (q == 1) give_back(half);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+              for (int e = 0; e < 8; e += 2) m[half * 8 + q * 4 + u] = fmax3(m[half * 8 + q * 4 + u], v[8 * u + e], v[8 * u + e + 1]);
+          }
+        } else {
+          give_back(half);
+        }
+      }
+    }
+    // the eight largest of this thread's maxima, descending, then of the row's
+    float best[kCmTop];
+#pragma unroll
+    for (int u = 0; u < kCmTop; ++u) best[u] = -CUDART_INF_F;
+#pragma unroll
+    for (int i = 0; i < kGroups; ++i) {
+      best[kCmTop - 1] = fmaxf(best[kCmTop - 1], m[i]);
+#pragma unroll
+      for (int u = kCmTop - 1; u > 0; --u) {
+        const float x = fmaxf(best[u - 1], best[u]), y = fminf(best[u - 1], best[u]);
+        best[u - 1] = x;
+        best[u] = y;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kCmTop; ++u) s_list[wg][r][u] = __float_as_uint(best[u]);
+    group_sync();
+    float eighth = CUDART_INF_F;
+#pragma unroll
+    for (int u = 0; u < kCmTop; ++u) eighth = fminf(eighth, fmaxf(best[u], __uint_as_float(s_list[wg ^ 1][r][kCmTop - 1 - u])));
+    group_sync();                                            // both groups have read the maxima
+    uint32_t list[kCmTop], thr, w, none;
+    float low;
+    int hits = 0;
+    candidate_words(eighth, 0.f, 0u, w, none);
+    bound_limits(eighth > -CUDART_INF_F ? w & 0xFFFF0000u : 0u, thr, low);      // fewer than eight groups above -inf: no bound
+#pragma unroll
+    for (int u = 0; u < kCmTop; ++u) list[u] = 0u;
+    for (; ok && j < jobs; j += 2) {
+      const int c = j - chunks, nq = 2 * halves(c);
+#pragma unroll 1
+      for (int q4 = 0; q4 < 4; ++q4) {
+        __syncwarp();                                        // rows went different ways
+        if (!(q4 & 1) && !ready(j, q4 >> 1)) break;
+        if (q4 < nq) quarter(q4);
+        if (q4 & 1) give_back(q4 >> 1);
+        if (q4 >= nq) continue;
+        const uint32_t c0 = (uint32_t) (c * kChunk + q4 * 32);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float x = max3_nan(v[8 * u], v[8 * u + 1], v[8 * u + 2]);
+          x = max3_nan(x, v[8 * u + 3], v[8 * u + 4]);
+          x = max3_nan(x, v[8 * u + 5], v[8 * u + 6]);
+          if (max_nan(x, v[8 * u + 7]) < low) continue;      // false for NaN
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (!(v[8 * u + e] < low)) {
+              candidate_words(v[8 * u + e], 0.f, 65535u - (c0 + 8 * u + e), w, none);
+              if (hits < kHits) {
+                s_list[wg][r][hits++] = w;
+              } else if (w > thr) {                          // many equal scores
+                list_insert(list, w);
+                thr = umax(thr, list[kCmTop - 1]);
+              }
+            }
+        }
+      }
+    }
+    __syncwarp();
+    for (int u = 0; __any_sync(0xffffffffu, u < hits); ++u) {
+      w = u < hits ? s_list[wg][r][u] : 0u;
+      if (w > thr) {
+        list_insert(list, w);
+        thr = umax(thr, list[kCmTop - 1]);
+      }
+    }
+    __syncwarp();
+    if (wg == 1) {
+#pragma unroll
+      for (int u = 0; u < kCmTop; ++u) s_list[1][r][u] = list[u];
+    }
+    group_sync();
+    if (wg == 0 && row0 + r < M && !abort_flag->abort) {
+      // the eight largest of two descending lists, sorted: the larger of the ends that meet, which is a bitonic sequence
+#pragma unroll
+      for (int u = 0; u < kCmTop; ++u) list[u] = umax(list[u], s_list[1][r][kCmTop - 1 - u]);
+#pragma unroll
+      for (int d = kCmTop / 2; d > 0; d >>= 1)
+#pragma unroll
+        for (int u = 0; u < kCmTop; ++u)
+          if ((u & d) == 0) {
+            const uint32_t x = umax(list[u], list[u + d]), y = umin(list[u], list[u + d]);
+            list[u] = x;
+            list[u + d] = y;
+          }
+      store_list(idx_out, idx64, (bh * M + row0 + r) * topk, topk, list);
+    }
+  }
+  if (abort_flag->abort) tc::abort_drain();
+  tc::fence_before_sync();
+  __syncthreads();
+  if (abort_flag->abort && tid < kRows && row0 + tid < M) {
+    const bf16* q = pq + (bh * M + row0 + tid) * 64;
+    uint32_t list[kCmTop];
+#pragma unroll
+    for (int u = 0; u < kCmTop; ++u) list[u] = 0u;
+#pragma unroll 1
+    for (int c = 0; c < (int) n; ++c) {
+      const bf16* k = pk + (bh * n + c) * 64;
+      float acc = 0.f;
+#pragma unroll 1
+      for (int d = 0; d < 64; ++d) acc = fmaf(__bfloat162float(q[d]), __bfloat162float(k[d]), acc);
+      uint32_t w, none;
+      candidate_words(acc, 0.f, 65535u - (uint32_t) c, w, none);
+      if (w > list[kCmTop - 1]) list_insert(list, w);
+    }
+    store_list(idx_out, idx64, (bh * M + row0 + tid) * topk, topk, list);
+  }
+  if (warp == 0) tc::tmem_dealloc(tmem, 256);
+}
+
+}  // namespace
+
+int launch_coarse_topk_tc(const LlsaTensor* pq, const LlsaTensor* pk, const LlsaTensor* idx, int topk, int wait_limit, cudaStream_t st) {
+  const int64_t BH = pq->shape[0] * pq->shape[1], M = pq->shape[2], n = pk->shape[2];
+  CoarseMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  int rc;
+  if ((rc = tma::make_map_rows(&maps.q, pq->ptr, (uint64_t) (BH * M), kRows))) return rc;
+  if ((rc = tma::make_map_rows(&maps.k, pk->ptr, (uint64_t) (BH * n), kChunk))) return rc;
+  const size_t smem = 1024 + (size_t) (1 + kStages) * kTile * sizeof(bf16);
+  LLSA_SMEM_LIMIT(coarse_topk_tc_kernel, smem);
+  launch_pdl(coarse_topk_tc_kernel, dim3((unsigned) ((M + kRows - 1) / kRows), (unsigned) BH), kThreads, smem, st, maps, (const bf16*) pq->ptr,
+             (const bf16*) pk->ptr, idx->ptr, idx->dtype == LLSA_I64 ? 1 : 0, M, n, topk, wait_limit);
+  LLSA_LAUNCH_OK("coarse_topk_tc_kernel");
+  return LLSA_OK;
+}
+
+}  // namespace llsa

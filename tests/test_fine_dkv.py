@@ -1,4 +1,5 @@
-"""Fine dK/dV kernel in its persistent form (lists of 4,736 ranges and more) against the oracle."""
+"""Fine dK/dV kernel against the oracle: windows drawn by the warps of a CTA (lists of 4,736 ranges and more), equal spans of the entries (shorter
+ones)."""
 import pytest
 import torch
 
@@ -45,3 +46,11 @@ def test_persistent_form_vs_oracle(B, H, N, topk, hot):
         _close(Q.grad[sl], dq[:n], "dq")
         _close(K.grad[sl], (dk + O.mean_pool1d_bwd(dpk, 16))[:n], "dk")
         _close(V.grad[sl], (dv + O.mean_pool1d_bwd(dpv, 16))[:n], "dv")
+
+
+# spans: of 64 entries (a problem of fewer than 256), the shortest spans on some of the SMs, spans of two lengths on all of them, which begin and end
+# inside buckets and inside heads; hot: a bucket that reaches over many spans, of one head and of every head
+@pytest.mark.parametrize("B,H,N,topk,hot", [(2, 1, 256, 2, ()), (2, 1, 256, 8, ()), (3, 2, 768, 6, ()), (3, 2, 768, 6, (3,)), (2, 2, 1024, 8, (0, 63)),
+                                            (9, 7, 2048, 8, ()), (9, 7, 2048, 8, (0, 1, 127)), (21, 11, 1024, 8, (5,))])
+def test_spans_vs_oracle(B, H, N, topk, hot):
+    test_persistent_form_vs_oracle(B, H, N, topk, hot)
