@@ -617,8 +617,8 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
   }
   if (threadIdx.x < NW * (kRingFineStages + 1)) tc::mbar_init(&s_full[0][0] + threadIdx.x, 1);
   tc::fence_mbar_init();
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();            // behind the wait: the finish kernel's first CTAs rely on the kernels in front of this one
   __syncthreads();
 
   const int E = (int) (a.nq1 * a.topk), n1 = (int) a.n1;
@@ -891,10 +891,15 @@ __device__ __forceinline__ void dkv_store_unselected(const AttnP<bf16>& a, int64
 // CTAs or extra work of the kernel above they cost twice as much: two CTAs of it fill an SM).
 // One warp for eight buckets, looking for both kinds, took 46 us at 48 slices of 16384 tokens and 160 us at 6 of 262144; this kernel 31
 // and 81.
+// It is launched while the kernel above ends: the unselected blocks and the lookups need nothing of it (its CTAs let this launch begin once they have
+// waited for the kernels in front of them) and take the SMs that its ragged end leaves idle; what adds pieces waits.  Whole layer, launched behind / into
+// the end: one level, B=4 H=6 N=4096 189.2 / 186.5 us, B=2 H=4 N=16384 334 / 329; two levels, B=3 H=5 N=5376 164.9 / 160.1, H=5 N=40960 top-16
+// 548 / 542, B=4 H=6 N=16384 641 / 634.
 __global__ void __launch_bounds__(128) attn_dkv_finish_kernel(AttnP<bf16> a, const float* __restrict__ partial, unsigned n_plain, unsigned BH, int n_spans) {
   if (blockIdx.x < n_plain * BH) {
     const int bh = (int) (blockIdx.x / n_plain), first = ((int) (blockIdx.x % n_plain) * 4 + (int) (threadIdx.x >> 5)) * kPlainPerWarp;
     dkv_store_unselected(a, bh / a.H, bh % a.H, bh, first, threadIdx.x & 31);
+    if (blockIdx.x == n_plain * BH - 1) pdl_wait();      // whatever else there is, this kernel does not end before the one in front of it
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n1 = (int) a.n1;
@@ -929,6 +934,7 @@ __global__ void __launch_bounds__(128) attn_dkv_finish_kernel(AttnP<bf16> a, con
   }
   const int64_t b = bh / a.H, h = bh % a.H;
   c_last -= c_first;                                                   // pieces behind the first one
+  pdl_wait();                                                          // for the pieces
   const int ten = warp >> 1, u0 = (warp & 1) * 4;                      // tiles u0 .. u0 + 3 of dk / dv: tile u holds channels 8u + 2t, +1 of rows g, g + 8
   float acc[4][4];
 #pragma unroll
@@ -1062,7 +1068,7 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
     }
     LLSA_LAUNCH_OK("attn_dkv_fine_ring_kernel");
     const unsigned n_plain = (unsigned) ((a.n1 + 4 * kPlainPerWarp - 1) / (4 * kPlainPerWarp)), boundaries = n_spans ? (unsigned) n_spans - 1 : (unsigned) (n_windows - 1) * BH;
-    attn_dkv_finish_kernel<<<dim3(n_plain * BH + boundaries), 128, 0, st>>>(a, partial, n_plain, BH, n_spans);
+    launch_pdl(attn_dkv_finish_kernel, dim3(n_plain * BH + boundaries), 128, 0, st, a, (const float*) partial, n_plain, BH, n_spans);
     LLSA_LAUNCH_OK("attn_dkv_finish_kernel");
   }
   return LLSA_OK;

@@ -44,8 +44,9 @@ void set_error(const char* fmt, ...);
 // passed pdl_trigger() (or exited), and starts its own work after pdl_wait(), which returns when that kernel has completed and its
 // writes are visible.  A layer is a chain of some ten kernels of 4 to 300 us; without this every one of them begins with an idle GPU for
 // the 2 us between the last CTA of a kernel and the first instruction of the next.  Every kernel launched this way waits before its first
-// access to global memory, so completion stays transitive along the chain.
-// Not for the streaming kernels (pooling pass, rotation / norm backward, unselected dK/dV blocks): a CTA that arrives while the kernel in
+// access to global memory, so completion stays transitive along the chain; attn_dkv_finish_kernel alone works ahead of its wait, on what the kernels
+// in front of its predecessor left, and one of its CTAs waits in any case.
+// Not for the streaming kernels (pooling pass, rotation / norm backward): a CTA that arrives while the kernel in
 // front still runs finds the SM divided for that kernel's shared memory, and with 28 KB of L1 to land its loads in it streams at two thirds
 // of its rate (B=4 H=6 N=16384 with norm and rotation, whole layer: 709 us with the three launched plainly, 757 with all chained, 720 with
 // none; l1_rope B=4 H=6 N=4096 243, 243 and 259).
