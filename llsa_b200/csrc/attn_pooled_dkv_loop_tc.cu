@@ -24,15 +24,18 @@
 // accumulators dV, dK at 384.  Gathered units are four jobs long: two buffers of S^T and dP^T (overwritten by P^T and dS^T) at 128 (n mod 2), two
 // pairs of accumulators at 256 + 128 (i mod 2), so that a unit's first products do not wait for the last one's results to be read.
 // Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64): warps 8 and 11 = TMA producers (K_c, V_c
-// per unit in two stages, Q_t per job; dO_t, lse, delta per job; a ring of 8), warp 9 issues S^T and dP^T, warp 10 dV and dK,
+// per unit in two stages, Q_t per job; dO_t, lse, delta per job; a ring of 8, gathered 4), warp 9 issues S^T and dP^T, warp 10 dV and dK,
 // warps 0-3 / 4-7 = two softmax warpgroups on alternating jobs, warps 12-15 write a unit's dV and dK, thread = key row.  Every mbarrier
 // wait is bounded (abort flag, TMEM freed).
 // What bounds them.  Dense, tensor pipe 768 cycles a job: the loop S^T, dP^T -> P^T, dS^T -> dV, dK, 1,170 cycles; copies, products and hand-overs
 // without the softmax 915, with its exponentials alone left out 1,090.  Two levels, B=1 H=6 N=262144: 870 us with three buffers for both and 32
-// columns loaded at a time, 835 now; l1, B=2 H=4 N=16384: 85 -> 79.  Three softmax groups change nothing (866), eight warps a job spill (1,165).  Gathered: the fp32 reductions, 100 M at
-// the same size; 263 us with results read from tensor memory 32 columns at a time, 245 with 16 (top-16, H=5 N=40960: 71 -> 65); in the dense
-// form's layout 254 to 270.
+// columns loaded at a time, 835 now; l1, B=2 H=4 N=16384: 85 -> 79.  Three softmax groups change nothing (866), eight warps a job spill (1,165).
+// Gathered: the fp32 reductions, 100 M at the same size.  A unit's results go through shared memory and are added by bulk reductions of whole lines (blocks of 16 keys
+// lie together in the accumulators): 251 -> 198 us; top-16, H=5 N=40960 65 -> 51.5; B=3 H=5 N=5376 23.7 -> 20.  As reductions of 16 bytes a lane they
+// were the pace of the kernel.
 #include <string.h>
+
+#include <type_traits>
 
 #include "attn.cuh"
 #include "mma_frag.cuh"
@@ -47,7 +50,8 @@ constexpr int kKeys = 128;                   // keys per unit (MMA M)
 constexpr int kQ = 64;                       // query rows per job (MMA N)
 constexpr int kKeyTile = kKeys * 64;         // elements of the K / V chunk (16 KB)
 constexpr int kQTile = kQ * 64;              // elements of a Q / dO job tile (8 KB)
-constexpr int kStages = 8;
+template <bool GATHER>
+constexpr int kRing = GATHER ? 4 : 8;        // stages of the Q / dO ring
 constexpr int kThreads = 512;
 constexpr int kLaunchRegs = 128, kIssueRegs = 56, kEpilogueRegs = 88, kSoftmaxRegs = 184;     // a thread's, per role: 56 + 88 + 2 x 184 = 4 x 128
 static_assert(kIssueRegs + kEpilogueRegs + 2 * kSoftmaxRegs <= 4 * kLaunchRegs, "the takers would wait for good");
@@ -56,10 +60,11 @@ constexpr float kLog2eF = 1.4426950408889634f;
 struct KvMaps {
   CUtensorMap q, d_o;         // [B,H,Nq,64] 4-D, box 64 rows
   CUtensorMap k, v;           // contiguous pooled keys / values [BH*n, 64], box 128 rows (gathered: 16 rows)
+  CUtensorMap dpk, dpv;       // gathered: the fp32 accumulators [BH*n, 64], box 16 rows x 32 columns
 };
 
 struct KvBars {
-  uint64_t kv_full[2], kv_empty[2], q_full[kStages], q_empty[kStages], sdp_ready[4], pds_ready[4], buf_free[4], dp_free[2], acc_ready[2], acc_free[2];
+  uint64_t kv_full[2], kv_empty[2], q_full[8], q_empty[8], sdp_ready[4], pds_ready[4], buf_free[4], dp_free[2], acc_ready[2], acc_free[2];
 };
 
 // A CTA's piece of the flat job list, walked unit by unit.
@@ -88,6 +93,7 @@ template <bool GATHER>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps maps, float* __restrict__ dpk, float* __restrict__ dpv,
                                int64_t n_keys, int jobs_all, int n_base, int chunks, float lw_log2, float out_mul) {
+  constexpr int kStages = kRing<GATHER>;
   extern __shared__ unsigned char smem_dyn[];
   __shared__ KvBars bars;
   __shared__ uint32_t s_tmem;
@@ -98,6 +104,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
   bf16* sV = sK + 2 * kKeyTile;              // [2][128][64]
   bf16* sQ = sV + 2 * kKeyTile;              // [kStages][64][64]
   bf16* sDO = sQ + kStages * kQTile;         // [kStages][64][64]
+  float* sOut = reinterpret_cast<float*>(sDO + kStages * kQTile);      // GATHER: [dV, dK][columns 0..31, 32..63][128 keys][32], swizzled
   constexpr int kBufs = GATHER ? 2 : 4, kAccs = GATHER ? 2 : 1;
   constexpr uint32_t kBufCols = GATHER ? 128 : 64, kColDP = 256, kColAcc = GATHER ? 256 : 384;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -323,42 +330,76 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
     const int qd = warp & 3, r = qd * 32 + lane;
     for (int i = 0; pc.next(); ++i) {
       const int bh = pc.unit / units_per_head, u = pc.unit - bh * units_per_head, c = GATHER ? u % chunks : u;
-      // this thread's key: its row in the pooled tensor, or none
-      bool live = true;
-      int64_t key = (int64_t) c * kKeys + r;
+      // gathered: row in the pooled tensor where this thread's block of keys begins, -1: no block; dense: this thread's key
+      int key_row = -1;
+      const int64_t key = (int64_t) c * kKeys + r;
       if (GATHER) {
         const int blk = c * 8 + (r >> 4);
-        live = blk < a.p1_blocks;
-        key = p1_block(a, bh, u / chunks * kBS, live ? blk : 0) * kBS + (r & 15);
-      } else {
-        live = key < n_keys;
+        if (blk < a.p1_blocks) key_row = (int) ((int64_t) bh * n_keys + p1_block(a, bh, u / chunks * kBS, blk) * kBS);
       }
-      const bool whole = !GATHER && pc.n == jobs_all;           // the unit saw every query of its head: nobody else adds to these rows
+      const bool live = key < n_keys, whole = pc.n == jobs_all;      // dense; whole: the unit saw every query of its head, nobody else adds to these rows
       const bool ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.acc_ready[i % kAccs], (uint32_t) (i / kAccs) & 1, abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
+      const uint32_t t_acc = tmem + kColAcc + (i % kAccs) * 128 + ((uint32_t) (qd * 32) << 16);
+      if constexpr (GATHER) {
+        // Through shared memory: a warp's 32 rows are two blocks, whose 16 x 64 sums are contiguous in the accumulators.
+        const int rows[2] = {__shfl_sync(0xffffffffu, key_row, 0), __shfl_sync(0xffffffffu, key_row, 16)};      // below 0: no such block
+        tma::reduce_wait_read();                     // the last unit's results have been read
+        __syncwarp();
 #pragma unroll
-      for (int part = 0; part < 8; ++part) {
-        float v[16];
-        tc::tmem_ld16(tmem + kColAcc + (i % kAccs) * 128 + part * 16 + ((uint32_t) (qd * 32) << 16), v);
-        if (part == 7) {
-          tc::fence_before_sync();
+        for (int part = 0; part < 4; ++part) {       // dV's columns 0..31 and 32..63, dK's
+          float v[32];
+          tc::tmem_ld32_async(t_acc + part * 32, v);
+          tc::tmem_ld_wait(v);
+          if (part == 3) {
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tma::mbar_arrive(&bars.acc_free[i % kAccs]);
+          }
+          const float mul = part < 2 ? out_mul : out_mul * a.scale;
+          const uint32_t at = tc::smem_u32(sOut + part * kKeys * 32 + r * 32) + ((r & 7) << 4);
+          auto put = [&](auto tag) {
+            constexpr int C = decltype(tag)::value;
+            tc::sts128_xor<16 * C>(at, __float_as_uint(v[4 * C] * mul), __float_as_uint(v[4 * C + 1] * mul), __float_as_uint(v[4 * C + 2] * mul),
+                                   __float_as_uint(v[4 * C + 3] * mul));
+          };
+          put(std::integral_constant<int, 0>{}); put(std::integral_constant<int, 1>{}); put(std::integral_constant<int, 2>{});
+          put(std::integral_constant<int, 3>{}); put(std::integral_constant<int, 4>{}); put(std::integral_constant<int, 5>{});
+          put(std::integral_constant<int, 6>{}); put(std::integral_constant<int, 7>{});
+          tc::fence_async_smem();
           __syncwarp();
-          if (lane == 0) tma::mbar_arrive(&bars.acc_free[i % kAccs]);
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+            if (rows[b] >= 0)
+              tma::reduce_add_2d_w(part < 2 ? &maps.dpv : &maps.dpk, (part & 1) * 32, rows[b], tc::smem_u32(sOut + part * kKeys * 32 + (qd * 32 + b * kBS) * 32));
         }
-        const float mul = part < 4 ? out_mul : out_mul * a.scale;
-        float* dst = (part < 4 ? dpv : dpk) + ((int64_t) bh * n_keys + key) * kD + (part & 3) * 16;
-        if (!live) {
-        } else if (whole) {
+        tma::reduce_commit_w();
+      } else {
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4)
-            *reinterpret_cast<float4*>(dst + 4 * q4) = make_float4(v[4 * q4] * mul, v[4 * q4 + 1] * mul, v[4 * q4 + 2] * mul, v[4 * q4 + 3] * mul);
-        } else {
+        for (int part = 0; part < 8; ++part) {
+          float v[16];
+          tc::tmem_ld16(t_acc + part * 16, v);
+          if (part == 7) {
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tma::mbar_arrive(&bars.acc_free[i % kAccs]);
+          }
+          const float mul = part < 4 ? out_mul : out_mul * a.scale;
+          float* dst = (part < 4 ? dpv : dpk) + ((int64_t) bh * n_keys + key) * kD + (part & 3) * 16;
+          if (!live) {
+          } else if (whole) {
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) red_add_v4(dst + 4 * q4, v[4 * q4] * mul, v[4 * q4 + 1] * mul, v[4 * q4 + 2] * mul, v[4 * q4 + 3] * mul);
+            for (int q4 = 0; q4 < 4; ++q4)
+              *reinterpret_cast<float4*>(dst + 4 * q4) = make_float4(v[4 * q4] * mul, v[4 * q4 + 1] * mul, v[4 * q4 + 2] * mul, v[4 * q4 + 3] * mul);
+          } else {
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) red_add_v4(dst + 4 * q4, v[4 * q4] * mul, v[4 * q4 + 1] * mul, v[4 * q4 + 2] * mul, v[4 * q4 + 3] * mul);
+          }
         }
       }
     }
+    if (GATHER) tma::reduce_wait_all();              // the sums are in memory, and shared memory is no longer read, before the kernel ends
   }
   if (abort_flag->abort) tc::abort_drain();
   tc::fence_before_sync();
@@ -380,7 +421,7 @@ int launch_attn_dkv_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
   int dev = 0, sms = 148;
   LLSA_CUDA_OK(cudaGetDevice(&dev));
   LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const size_t smem = 1024 + (size_t) (4 * kKeyTile + 2 * kStages * kQTile) * sizeof(bf16);
+  const size_t smem = 1024 + (size_t) (4 * kKeyTile + 2 * kRing<false> * kQTile) * sizeof(bf16);
   // one CTA per SM, each with an equal piece of the flat (unit, job) list
   auto grid_of = [&](int64_t total) { return total < sms ? (int) total : sms; };
   const int64_t n_dense = a.two_level ? (int64_t) a.p2_blocks * kBS : a.n1;
@@ -398,8 +439,11 @@ int launch_attn_dkv_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
     if ((rc = tma::make_map_rows(&maps.k, a.pk, (uint64_t) BH * a.n1, kBS))) return rc;
     if ((rc = tma::make_map_rows(&maps.v, a.pv, (uint64_t) BH * a.n1, kBS))) return rc;
     const int chunks = (a.p1_blocks + 7) / 8, jobs = kBS * kBS / kQ, units = (int) (BH * a.nq2) * chunks;
-    LLSA_SMEM_LIMIT((attn_dkv_pooled_loop_tc_kernel<true>), smem);
-    launch_pdl(attn_dkv_pooled_loop_tc_kernel<true>, grid_of((int64_t) units * jobs), kThreads, smem, st, a, maps, a.dpk, a.dpv, a.n1, jobs, units, chunks,
+    if ((rc = tma::make_map_acc(&maps.dpk, a.dpk, (uint64_t) BH * a.n1, kBS))) return rc;
+    if ((rc = tma::make_map_acc(&maps.dpv, a.dpv, (uint64_t) BH * a.n1, kBS))) return rc;
+    const size_t smem_g = 1024 + (size_t) (4 * kKeyTile + 2 * kRing<true> * kQTile) * sizeof(bf16) + (size_t) 4 * kKeys * 32 * sizeof(float);
+    LLSA_SMEM_LIMIT((attn_dkv_pooled_loop_tc_kernel<true>), smem_g);
+    launch_pdl(attn_dkv_pooled_loop_tc_kernel<true>, grid_of((int64_t) units * jobs), kThreads, smem_g, st, a, maps, a.dpk, a.dpv, a.n1, jobs, units, chunks,
                                                                                                  log2f(a.w1), a.kvw1 / a.w1);
     LLSA_LAUNCH_OK("attn_dkv_pooled_loop_tc_kernel<gathered>");
   }

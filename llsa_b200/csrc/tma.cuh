@@ -63,6 +63,19 @@ inline int make_map_rows(CUtensorMap* m, const void* base, uint64_t rows, uint32
   return make_map(m, base, 2, dims, strides, box_rows);
 }
 
+// Contiguous fp32 [rows, 64] matrix as the target of reductions from shared memory: boxes of box_rows rows x 32 columns (the 128 bytes that a
+// swizzled row holds).
+inline int make_map_acc(CUtensorMap* m, void* base, uint64_t rows, uint32_t box_rows) {
+  EncodeFn fn = encode_fn();
+  LLSA_REQUIRE(fn != nullptr, LLSA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint64_t gd[2] = {64, rows}, gs[1] = {256};
+  const cuuint32_t box[2] = {32, box_rows}, es[2] = {1, 1};
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  LLSA_REQUIRE(r == CUDA_SUCCESS, LLSA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int) r);
+  return LLSA_OK;
+}
+
 #ifdef __CUDACC__
 __device__ __forceinline__ void load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* mbar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
@@ -99,6 +112,20 @@ __device__ __forceinline__ void load_bulk_w(void* smem_dst, const void* gsrc, ui
                "l"(gsrc), "r"(bytes), "r"((uint32_t) __cvta_generic_to_shared(mbar))
                : "memory");
 }
+// Shared memory tile += into a matrix of make_map_acc, issued by one lane of a warp in step; reduce_commit_w closes a group of them, the waits
+// are for all groups: until shared memory may be written again, or until the sums are in memory.
+__device__ __forceinline__ void reduce_add_2d_w(const CUtensorMap* map, int c0, int c1, uint32_t smem_src) {
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+               "@e cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];\n\t}" ::"l"(map), "r"(c0), "r"(c1),
+               "r"(smem_src)
+               : "memory");
+}
+__device__ __forceinline__ void reduce_commit_w() {
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t@e cp.async.bulk.commit_group;\n\t}" ::: "memory");
+}
+// Every lane may execute the waits: a lane that has committed nothing passes
+__device__ __forceinline__ void reduce_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void reduce_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void expect_tx_w(uint64_t* mbar, uint32_t bytes) {
   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
                "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"((uint32_t) __cvta_generic_to_shared(mbar)), "r"(bytes) : "memory");

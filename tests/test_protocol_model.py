@@ -91,7 +91,7 @@ def test_gathered_key_major_form_has_no_hazard_or_deadlock():
     for seed in range(RUNS):
         rng = random.Random(seed)
         units = [rng.randint(1, 4)] + [4] * rng.randint(0, 9) + [rng.randint(1, 4)]
-        assert outcome(key_major_kernel, seed, units, gathered=True) == "ok", seed
+        assert outcome(key_major_kernel, seed, units, gathered=True, stages=4) == "ok", seed
 
 
 def test_one_chunk_tiles_leave_a_group_without_work():
