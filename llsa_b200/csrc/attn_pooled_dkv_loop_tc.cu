@@ -11,18 +11,16 @@
 //     P^T  = exp2(S^T*scale*log2e + log2 w - lse[q]),  dS^T = P^T * (dP^T - delta[q])     thread = key row; the scale
 //            (a power of two) is applied to dK;
 //            lse and delta of the 64 query columns sit in shared memory next to the Q / dO tile
-//     dV_c += P^T  . dO_t  [128 x 64]  (K = 64 queries)   P^T, dS^T read from TENSOR MEMORY (packed bf16, written over S^T;
-//     dK_c += dS^T . Q_t                                   gathered: dS^T over dP^T), dO_t / Q_t as MN-major operands (the same tiles)
+//     dV_c += P^T  . dO_t  [128 x 64]  (K = 64 queries)   P^T, dS^T read from TENSOR MEMORY (packed bf16, written over S^T),
+//     dK_c += dS^T . Q_t                                   dO_t / Q_t as MN-major operands (the same tiles)
 // dK_c, dV_c accumulate in TMEM over the unit's query range and are then written to the fp32 pooled-gradient
 // accumulators (scaled by kv_weight / token_weight, the reference's weighting of the pooled dK/dV side): plain stores if
 // the unit covers all queries of its head, reductions otherwise.  Rows of a chunk behind the end of its list (which may end at any
 // multiple of 32 keys) hold a repeated block or the rows that follow in memory; their results stay in their own rows and are dropped.
 // Work split: all (head, chunk, job) triples in that order form one flat list that is cut into gridDim.x equal pieces,
 // one per CTA; a piece is one to a few units (it changes unit where it crosses a chunk boundary).
-// TMEM columns, job number n and unit number i of the CTA.  Dense units are hundreds of jobs long: S^T, and P^T and dS^T over it (queries 0..31
-// at 0 and 16, 32..63 at 32 and 48), at 64 (n mod 4); dP^T at 256 + 64 (n mod 2), handed back as soon as its group has it in registers; one pair of
-// accumulators dV, dK at 384.  Gathered units are four jobs long: two buffers of S^T and dP^T (overwritten by P^T and dS^T) at 128 (n mod 2), two
-// pairs of accumulators at 256 + 128 (i mod 2), so that a unit's first products do not wait for the last one's results to be read.
+// TMEM columns, job number n of the CTA: S^T, and P^T and dS^T over it (queries 0..31 at 0 and 16, 32..63 at 32 and 48), at 64 (n mod 4); dP^T at
+// 256 + 64 (n mod 2), handed back as soon as its group has it in registers; one pair of accumulators dV, dK at 384.
 // Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64): warps 8 and 11 = TMA producers (K_c, V_c
 // per unit in two stages, Q_t per job; dO_t, lse, delta per job; a ring of 8, gathered 4), warp 9 issues S^T and dP^T, warp 10 dV and dK,
 // warps 0-3 / 4-7 = two softmax warpgroups on alternating jobs, warps 12-15 write a unit's dV and dK, thread = key row.  Every mbarrier
@@ -30,9 +28,9 @@
 // What bounds them.  Dense, tensor pipe 768 cycles a job: the loop S^T, dP^T -> P^T, dS^T -> dV, dK, 1,170 cycles; copies, products and hand-overs
 // without the softmax 915, with its exponentials alone left out 1,090.  Two levels, B=1 H=6 N=262144: 870 us with three buffers for both and 32
 // columns loaded at a time, 835 now; l1, B=2 H=4 N=16384: 85 -> 79.  Three softmax groups change nothing (866), eight warps a job spill (1,165).
-// Gathered: the fp32 reductions, 100 M at the same size.  A unit's results go through shared memory and are added by bulk reductions of whole lines (blocks of 16 keys
-// lie together in the accumulators): 251 -> 198 us; top-16, H=5 N=40960 65 -> 51.5; B=3 H=5 N=5376 23.7 -> 20.  As reductions of 16 bytes a lane they
-// were the pace of the kernel.
+// Gathered: the fp32 reductions, 100 M at the same size, and a unit's few jobs.  A unit's results go through shared memory and are added by bulk reductions of
+// whole lines (blocks of 16 keys lie together in the accumulators): 251 -> 198 us; top-16, H=5 N=40960 65 -> 51.5; as reductions of 16 bytes a lane they were
+// the pace.  With one pair of accumulators and the dense form's four buffers instead of two pairs and two buffers 198 -> 182, 51.5 -> 47.6.
 #include <string.h>
 
 #include <type_traits>
@@ -53,6 +51,8 @@ constexpr int kQTile = kQ * 64;              // elements of a Q / dO job tile (8
 template <bool GATHER>
 constexpr int kRing = GATHER ? 4 : 8;        // stages of the Q / dO ring
 constexpr int kThreads = 512;
+constexpr int kBufs = 4;                     // S^T buffers (P^T and dS^T over them)
+constexpr uint32_t kColDP = 256, kColAcc = 384;
 constexpr int kLaunchRegs = 128, kIssueRegs = 56, kEpilogueRegs = 88, kSoftmaxRegs = 184;     // a thread's, per role: 56 + 88 + 2 x 184 = 4 x 128
 static_assert(kIssueRegs + kEpilogueRegs + 2 * kSoftmaxRegs <= 4 * kLaunchRegs, "the takers would wait for good");
 constexpr float kLog2eF = 1.4426950408889634f;
@@ -64,7 +64,7 @@ struct KvMaps {
 };
 
 struct KvBars {
-  uint64_t kv_full[2], kv_empty[2], q_full[8], q_empty[8], sdp_ready[4], pds_ready[4], buf_free[4], dp_free[2], acc_ready[2], acc_free[2];
+  uint64_t kv_full[2], kv_empty[2], q_full[8], q_empty[8], sdp_ready[4], pds_ready[4], buf_free[4], dp_free[2], acc_ready, acc_free;
 };
 
 // A CTA's piece of the flat job list, walked unit by unit.
@@ -105,8 +105,6 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
   bf16* sQ = sV + 2 * kKeyTile;              // [kStages][64][64]
   bf16* sDO = sQ + kStages * kQTile;         // [kStages][64][64]
   float* sOut = reinterpret_cast<float*>(sDO + kStages * kQTile);      // GATHER: [dV, dK][columns 0..31, 32..63][128 keys][32], swizzled
-  constexpr int kBufs = GATHER ? 2 : 4, kAccs = GATHER ? 2 : 1;
-  constexpr uint32_t kBufCols = GATHER ? 128 : 64, kColDP = 256, kColAcc = GATHER ? 256 : 384;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile tc::WaitCtl* abort_flag = &s_ctl;
 
@@ -121,7 +119,8 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       tc::mbar_init(&bars.buf_free[i], 1);
     }
     for (int i = 0; i < 2; ++i) tc::mbar_init(&bars.dp_free[i], 4);
-    for (int i = 0; i < kAccs; ++i) { tc::mbar_init(&bars.acc_ready[i], 1); tc::mbar_init(&bars.acc_free[i], 4); }
+    tc::mbar_init(&bars.acc_ready, 1);
+    tc::mbar_init(&bars.acc_free, 4);
     tc::fence_mbar_init();
   }
   pdl_wait();
@@ -135,7 +134,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
   Piece pc((int64_t) n_base * jobs_all, jobs_all);
 
   // the warps that issue copies and products leave most of their registers to the others
-  if (!GATHER && warp >= 8 && warp < 12) tc::regs_set<kIssueRegs, kLaunchRegs>();
+  if (warp >= 8 && warp < 12) tc::regs_set<kIssueRegs, kLaunchRegs>();
   if (warp == 8 || warp == 11) {
     // ---------------------------------------------------------------- TMA producers: warp 8 the unit's keys and Q, warp 11 dO, lse, delta
     const bool second = warp == 11;
@@ -197,11 +196,11 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
           const int st = cj & (kStages - 1);
           // even lanes: the query tile; lanes 1, 5, ..: the S^T buffer's previous job (kBufs back), whose P^T / dS^T have been read; lanes 3,
           // 7, ..: the dP^T buffer's (two back), which its group has loaded
-          const bool b = (lane & 3) == 1 && cj >= kBufs, p = !GATHER && (lane & 3) == 3 && cj >= 2;
+          const bool b = (lane & 3) == 1 && cj >= kBufs, p = (lane & 3) == 3 && cj >= 2;
           if (!(ok = tc::warp_wait(b ? &bars.buf_free[buf] : p ? &bars.dp_free[cj & 1] : &bars.q_full[st],
                                    b ? bph ^ 1 : p ? (uint32_t) ((cj >> 1) - 1) & 1 : (uint32_t) (cj / kStages) & 1, abort_flag))) break;
           tc::fence_after_sync();
-          const uint32_t d = tmem + buf * kBufCols, dp = GATHER ? d + 64 : tmem + kColDP + (cj & 1) * 64, q_ = lQ + st * kQStage, o_ = lDO + st * kQStage;
+          const uint32_t d = tmem + buf * 64, dp = tmem + kColDP + (cj & 1) * 64, q_ = lQ + st * kQStage, o_ = lDO + st * kQStage;
           tc::umma_ss_k64(d, k_, hi, q_, hi, id_s);
           tc::umma_ss_k64(dp, v_, hi, o_, hi, id_s);
           tc::umma_commit_w(&bars.sdp_ready[buf]);
@@ -226,30 +225,26 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
         for (int j = 0; j < pc.n; ++j, ++cj) {
           const int st = cj & (kStages - 1);
           // odd lanes, first job of a unit: the results this accumulator held last have been read
-          const bool f = (lane & 1) && j == 0 && i >= kAccs;
-          if (!(ok = tc::warp_wait(f ? &bars.acc_free[i % kAccs] : &bars.pds_ready[buf], f ? (uint32_t) (i / kAccs - 1) & 1 : bph, abort_flag))) break;
+          const bool f = (lane & 1) && j == 0 && i >= 1;
+          if (!(ok = tc::warp_wait(f ? &bars.acc_free : &bars.pds_ready[buf], f ? (uint32_t) (i - 1) & 1 : bph, abort_flag))) break;
           tc::fence_after_sync();
           // 4 k-steps of 16 query rows (2048 bytes of the MN-major dO / Q tile)
-          const uint32_t o_ = lDOm + st * kQStage, q_ = lQm + st * kQStage, b = tmem + buf * kBufCols, acc = tmem + kColAcc + (i % kAccs) * 128;
-          if (GATHER) {
-            tc::umma_ts_k64(acc, b, o_, hi, id_o, j > 0 ? 1u : 0u);
-            tc::umma_ts_k64(acc + 64, b + 64, q_, hi, id_o, j > 0 ? 1u : 0u);
-          } else {                             // the first 32 queries' P^T, dS^T lie in the buffer's columns 0 and 16, the others' in 32 and 48
-            tc::umma_ts_k32(acc, b, o_, hi, id_o, j > 0 ? 1u : 0u);
-            tc::umma_ts_k32(acc, b + 32, o_ + 256, hi, id_o, 1u);
-            tc::umma_ts_k32(acc + 64, b + 16, q_, hi, id_o, j > 0 ? 1u : 0u);
-            tc::umma_ts_k32(acc + 64, b + 48, q_ + 256, hi, id_o, 1u);
-          }
+          const uint32_t o_ = lDOm + st * kQStage, q_ = lQm + st * kQStage, b = tmem + buf * 64, acc = tmem + kColAcc;
+          // the first 32 queries' P^T, dS^T lie in the buffer's columns 0 and 16, the others' in 32 and 48
+          tc::umma_ts_k32(acc, b, o_, hi, id_o, j > 0 ? 1u : 0u);
+          tc::umma_ts_k32(acc, b + 32, o_ + 256, hi, id_o, 1u);
+          tc::umma_ts_k32(acc + 64, b + 16, q_, hi, id_o, j > 0 ? 1u : 0u);
+          tc::umma_ts_k32(acc + 64, b + 48, q_ + 256, hi, id_o, 1u);
           tc::umma_commit_w(&bars.q_empty[st]);
           tc::umma_commit_w(&bars.buf_free[buf]);
           if (++buf == kBufs) { buf = 0; bph ^= 1; }
         }
         if (!ok) break;
-        tc::umma_commit_w(&bars.acc_ready[i % kAccs]);
+        tc::umma_commit_w(&bars.acc_ready);
       }
     }
   } else if (warp < 8) {
-    if (!GATHER) tc::regs_set<kSoftmaxRegs, kLaunchRegs>();
+    tc::regs_set<kSoftmaxRegs, kLaunchRegs>();
     // ---------------------------------------------------------------- P^T / dS^T; thread = key row
     const int wg = warp >> 2, qd = warp & 3;
     const float sl2 = a.scale * kLog2eF;
@@ -264,7 +259,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
       const bool ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.sdp_ready[buf], bph, abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
-      const uint32_t t_b = t_lane + buf * kBufCols, t_p = GATHER ? t_b + 64 : t_lane + kColDP + wg * 64;
+      const uint32_t t_b = t_lane + buf * 64, t_p = t_lane + kColDP + wg * 64;
       // P^T and dS^T of 32 query columns
       auto half_of = [&](int half, const float (&s)[32], const float (&d)[32], uint32_t to_p, uint32_t to_ds) {
         uint32_t pp[16], pd[16];
@@ -288,44 +283,29 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
         tc::tmem_st16(to_p, pp);                     // over columns read before
         tc::tmem_st16(to_ds, pd);
       };
-      if constexpr (GATHER) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          tc::tmem_ld32_async(t_b + 32 * half, vs);
-          tc::tmem_ld32_async(t_p + 32 * half, vd);
-          tc::tmem_ld_wait(vs);
-          tc::tmem_ld_wait(vd);
-          half_of(half, vs, vd, t_b + 16 * half, t_p + 16 * half);
-        }
-      } else {
-        float vs2[32], vd2[32];
-        tc::tmem_ld32_async(t_p, vd);
-        tc::tmem_ld32_async(t_p + 32, vd2);
-        tc::tmem_ld32_async(t_b, vs);
-        tc::tmem_ld32_async(t_b + 32, vs2);
-        tc::tmem_ld_wait(vd);
-        tc::tmem_ld_wait(vd2);
-        tc::tmem_ld_wait(vs);
-        tc::tmem_ld_wait(vs2);
-        tc::fence_before_sync();                     // dP^T is in registers: the next but one job's may come
-        __syncwarp();
-        if (lane == 0) tma::mbar_arrive(&bars.dp_free[wg]);
-        half_of(0, vs, vd, t_b, t_b + 16);
-        half_of(1, vs2, vd2, t_b + 32, t_b + 48);
-      }
+      float vs2[32], vd2[32];
+      tc::tmem_ld32_async(t_p, vd);
+      tc::tmem_ld32_async(t_p + 32, vd2);
+      tc::tmem_ld32_async(t_b, vs);
+      tc::tmem_ld32_async(t_b + 32, vs2);
+      tc::tmem_ld_wait(vd);
+      tc::tmem_ld_wait(vd2);
+      tc::tmem_ld_wait(vs);
+      tc::tmem_ld_wait(vs2);
+      tc::fence_before_sync();                     // dP^T is in registers: the next but one job's may come
+      __syncwarp();
+      if (lane == 0) tma::mbar_arrive(&bars.dp_free[wg]);
+      half_of(0, vs, vd, t_b, t_b + 16);
+      half_of(1, vs2, vd2, t_b + 32, t_b + 48);
       tc::tmem_st_wait();
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) tma::mbar_arrive(&bars.pds_ready[buf]);
-      if (kBufs == 2) {                              // the group's own buffer again
-        bph ^= 1;
-      } else {
-        buf += 2;
-        if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
-      }
+      buf += 2;
+      if (buf >= kBufs) { buf -= kBufs; bph ^= 1; }
     }
   } else {
-    if (!GATHER) tc::regs_set<kEpilogueRegs, kLaunchRegs>();
+    tc::regs_set<kEpilogueRegs, kLaunchRegs>();
     // ---------------------------------------------------------------- results of a unit; thread = key row
     const int qd = warp & 3, r = qd * 32 + lane;
     for (int i = 0; pc.next(); ++i) {
@@ -338,10 +318,10 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
         if (blk < a.p1_blocks) key_row = (int) ((int64_t) bh * n_keys + p1_block(a, bh, u / chunks * kBS, blk) * kBS);
       }
       const bool live = key < n_keys, whole = pc.n == jobs_all;      // dense; whole: the unit saw every query of its head, nobody else adds to these rows
-      const bool ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.acc_ready[i % kAccs], (uint32_t) (i / kAccs) & 1, abort_flag));
+      const bool ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.acc_ready, (uint32_t) i & 1, abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
-      const uint32_t t_acc = tmem + kColAcc + (i % kAccs) * 128 + ((uint32_t) (qd * 32) << 16);
+      const uint32_t t_acc = tmem + kColAcc + ((uint32_t) (qd * 32) << 16);
       if constexpr (GATHER) {
         // Through shared memory: a warp's 32 rows are two blocks, whose 16 x 64 sums are contiguous in the accumulators.
         const int rows[2] = {__shfl_sync(0xffffffffu, key_row, 0), __shfl_sync(0xffffffffu, key_row, 16)};      // below 0: no such block
@@ -355,7 +335,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
           if (part == 3) {
             tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0) tma::mbar_arrive(&bars.acc_free[i % kAccs]);
+            if (lane == 0) tma::mbar_arrive(&bars.acc_free);
           }
           const float mul = part < 2 ? out_mul : out_mul * a.scale;
           const uint32_t at = tc::smem_u32(sOut + part * kKeys * 32 + r * 32) + ((r & 7) << 4);
@@ -383,7 +363,7 @@ attn_dkv_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps map
           if (part == 7) {
             tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0) tma::mbar_arrive(&bars.acc_free[i % kAccs]);
+            if (lane == 0) tma::mbar_arrive(&bars.acc_free);
           }
           const float mul = part < 4 ? out_mul : out_mul * a.scale;
           float* dst = (part < 4 ? dpv : dpk) + ((int64_t) bh * n_keys + key) * kD + (part & 3) * 16;
@@ -442,7 +422,7 @@ int launch_attn_dkv_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, 
     if ((rc = tma::make_map_acc(&maps.dpk, a.dpk, (uint64_t) BH * a.n1, kBS))) return rc;
     if ((rc = tma::make_map_acc(&maps.dpv, a.dpv, (uint64_t) BH * a.n1, kBS))) return rc;
     const size_t smem_g = 1024 + (size_t) (4 * kKeyTile + 2 * kRing<true> * kQTile) * sizeof(bf16) + (size_t) 4 * kKeys * 32 * sizeof(float);
-    LLSA_SMEM_LIMIT((attn_dkv_pooled_loop_tc_kernel<true>), smem_g);
+    LLSA_SMEM_LIMIT_REGS((attn_dkv_pooled_loop_tc_kernel<true>), smem_g, kLaunchRegs);
     launch_pdl(attn_dkv_pooled_loop_tc_kernel<true>, grid_of((int64_t) units * jobs), kThreads, smem_g, st, a, maps, a.dpk, a.dpv, a.n1, jobs, units, chunks,
                                                                                                  log2f(a.w1), a.kvw1 / a.w1);
     LLSA_LAUNCH_OK("attn_dkv_pooled_loop_tc_kernel<gathered>");

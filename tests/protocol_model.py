@@ -135,24 +135,22 @@ def _bars(name, n, count):
     return [Barrier("%s%d" % (name, i), count) for i in range(n)]
 
 
-def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8, buffers=None, accs=1, full_count=2, gathered=False, dp_count=4,
+def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8, buffers=None, full_count=2, dp_count=4,
                      dp_back_first=False):
-    """attn_dkv_pooled_loop_tc_kernel.  `units`: job counts of the units of one CTA's piece.  Dense form: (head, chunk) units; four S^T buffers,
-    which P^T and dS^T overwrite, one pair of accumulators, and two dP^T buffers, handed back as soon as their group has loaded them.  Gathered
-    form: units of four jobs and fewer; two buffers of S^T and dP^T together, which go back with the products that read P^T and dS^T, and two
-    pairs of accumulators.  Two score threads share three S^T buffers.
+    """attn_dkv_pooled_loop_tc_kernel.  `units`: job counts of the units of one CTA's piece: long (head, chunk) units, or, gathered, units of four
+    jobs and fewer.  Four S^T buffers, which P^T and dS^T overwrite, one pair of accumulators, and two dP^T buffers, handed back as soon as their
+    group has loaded them.  stages: of the Q / dO ring (8; gathered 4).  Two score threads share three S^T buffers.
     dp_count: warps whose arrivals hand a dP^T buffer back (4 = the kernel; fewer break the protocol on purpose), dp_back_first: a warp
     arrives before it has loaded its part (the same).
     score_threads: threads that issue S^T / dP^T (1 = the kernel; 2 = even and odd jobs on two threads).
     score_barriers: sdp_ready / buf_free barriers (None = one per buffer, the kernel; 6 = one per job number mod 6).
     full_count: producers a query stage waits for (2 = the kernel: Q, and dO with lse and delta; 1 breaks the protocol on purpose)."""
     sim = Sim(seed)
-    if gathered:
-        buffers, accs = 2, 2
+    accs = 1
     buffers = buffers or (4 if score_threads == 1 else 3)
     nb = score_barriers or buffers
     dp = [Resource("dP^T buffer %d" % i) for i in range(2)]
-    dp_free = None if gathered else _bars("dp_free", 2, dp_count)
+    dp_free = _bars("dp_free", 2, dp_count)
     kv_full, kv_empty = _bars("kv_full", 2, 1), _bars("kv_empty", 2, score_threads)
     q_full, q_empty = _bars("q_full", stages, full_count), _bars("q_empty", stages, 1)
     sdp, pds, free = _bars("sdp_ready", nb, 1), _bars("pds_ready", buffers, 4), _bars("buf_free", nb, 1)
@@ -190,7 +188,7 @@ def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8
                 if job >= buffers:
                     prev = job - buffers
                     wait += [free[prev % nb], (prev // nb) & 1]
-                if job >= 2 and not gathered:
+                if job >= 2:
                     wait += [dp_free[job & 1], ((job >> 1) - 1) & 1]
                 yield tuple(wait)
                 if sim.rng.random() < 0.15:
@@ -243,11 +241,9 @@ def key_major_kernel(seed, units, score_threads=1, score_barriers=None, stages=8
                 dp_free[job & 1].arrive(sim)
             yield ("delay", sim.r(100, 400))
             dp[job & 1].read(sim, job)
-            if not gathered and not dp_back_first:
+            if not dp_back_first:
                 dp_free[job & 1].arrive(sim)
             yield ("delay", sim.r(500, 1200))
-            if gathered:                  # dP^T is loaded half by half and overwritten by dS^T: it is the job's up to here
-                dp[job & 1].read(sim, job)
             if warp == 0:
                 owner[buf] = ("p", job)
             pds[buf].arrive(sim)

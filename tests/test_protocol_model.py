@@ -86,12 +86,11 @@ def test_model_catches_a_stage_freed_by_one_issuer_only_and_an_unguarded_overwri
 
 
 def test_gathered_key_major_form_has_no_hazard_or_deadlock():
-    """attn_dkv_pooled_loop_tc_kernel, gathered form: units of four query tiles (pieces begin and end inside one), two buffers of S^T and dP^T --
-    a group meets its own buffer again with its next job, and nothing but the products behind it hands it back -- and two accumulators."""
+    """attn_dkv_pooled_loop_tc_kernel, gathered form: units of four query tiles (pieces begin and end inside one) and a ring of four stages."""
     for seed in range(RUNS):
         rng = random.Random(seed)
         units = [rng.randint(1, 4)] + [4] * rng.randint(0, 9) + [rng.randint(1, 4)]
-        assert outcome(key_major_kernel, seed, units, gathered=True, stages=4) == "ok", seed
+        assert outcome(key_major_kernel, seed, units, stages=4) == "ok", seed
 
 
 def test_one_chunk_tiles_leave_a_group_without_work():
