@@ -641,7 +641,6 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
   int kvph = 0, fold_buf = 0;               // parity of the next K / V fill, fold buffer of the bucket at hand
   // entries the CSR really holds: fewer than E when the transpose dropped out-of-range indices; ranges and offsets handed in
   // by a caller are not trusted further than these clamps and the bounds on the bucket walk below
-  auto cut = [&](int64_t bh, int r, int used) { return r < R ? min(max(__ldcg(&a.ranges[bh * R + r].x), 0), used) : used; };
   // SPANS: the warp's own, a head at a time.  Otherwise the warps of a CTA draw one range after another; a range that begins inside a bucket is
   // left to the warp that has the range in front of it, unless it opens a window.
   const int span = warp * (int) gridDim.x + (int) blockIdx.x;
@@ -660,7 +659,6 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
       ++bh;
       re = min(E, rb + left);
       left -= re - rb;
-      re = min(re, (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1))));
       r0 = rb / a.range_entries;
     } else {
       int k = 0;
@@ -671,15 +669,34 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
       bh = (int) (u / n_pieces);
       r0 = (int) (u % n_pieces) * 2 + (k & 1);
       if (r0 >= R) continue;
-      const int E_used = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1)));
-      auto begins_inside = [&](int r) {
-        const int2 x = __ldcg(&a.ranges[bh * R + r]);
-        return (int) csr_off(a, bh, min(max(x.y, 0), n1 - 1)) < x.x;
-      };
-      const bool odd = r0 & 1, both = (odd || r0 + 1 < R) && begins_inside(r0 | 1);
+    }
+    // What the walk starts from is two rounds of loads away, each in flight at once: the ranges from r0 on and the entries in use; then the bucket
+    // ends from the range's bucket on, the query blocks of the first entries, and where the bucket of the window's second range begins.  (One after the
+    // other, seven rounds: l1, B=2 H=4 N=16384 60.3 us instead of 59.2, l2, B=3 H=5 N=5376 43.7 / 43.0, B=4 H=6 N=16384 152.6 / 151.5.)
+    const int32_t* fl = a.flat + (int64_t) bh * E;
+    int cur_qb = 0, nx_qb = 0;               // lane i: query block of entry 32 c + i of the chunk c being requested and of the one after it
+    auto first_entries = [&] { if (rb + lane < E) nx_qb = __ldcg(fl + rb + lane); };
+    if (SPANS) first_entries();
+    const int2 rr = __ldcg(&a.ranges[(int64_t) bh * R + min(r0 + min(lane, 2), R - 1)]);
+    const int E_used = (int) min((int64_t) E, max((int64_t) 0, csr_off(a, bh, n1)));
+    auto bucket_of = [&](int i) { return min(max(__shfl_sync(0xffffffffu, rr.y, i), 0), n1 - 1); };
+    // Bucket walk: lane l holds the end of bucket jb + l, so the bucket of an entry is the number of ends at or below it, and the next
+    // non-empty bucket is known without a load while the one at hand is being worked on.
+    auto bucket_end = [&](int j0) { return j0 + 1 + lane <= n1 ? (int) csr_off(a, bh, j0 + 1 + lane) : 0x7fffffff; };
+    int jb = bucket_of(0), ends = bucket_end(jb), ends2 = bucket_end(jb + 32);
+    const int begin_jb = (int) csr_off(a, bh, jb);
+    if constexpr (SPANS) {
+      re = min(re, E_used);
+    } else {
+      // a cut: the range's entry, or the entries' end
+      auto cut = [&](int i) { return r0 + i < R ? min(max(__shfl_sync(0xffffffffu, rr.x, i), 0), E_used) : E_used; };
+      const int odd = r0 & 1, x1 = __shfl_sync(0xffffffffu, rr.x, 1 - odd), begin1 = (int) csr_off(a, bh, bucket_of(1 - odd));
+      rb = cut(0);
+      first_entries();
+      const int re1 = cut(1), re2 = cut(2);
+      const bool both = (odd || r0 + 1 < R) && begin1 < x1;      // the window's second range begins inside a bucket
       if (odd && both) continue;
-      rb = cut(bh, r0, E_used);
-      re = max(cut(bh, r0 + (both ? 2 : 1), E_used), rb);
+      re = max(both ? re2 : re1, rb);
     }
     if (rb >= re) {
       if (SPANS) rb = 0;
@@ -688,21 +705,16 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
     const int b = bh / (int) a.H, h = bh % (int) a.H;
     // the span's or the window's head and tail slots
     float* const pieces = partial + (SPANS ? (int64_t) span : (int64_t) bh * n_pieces + r0 / (kRingWindow / kRangeEntries)) * 2 * (int64_t) kTileFloats;
-    const int32_t* fl = a.flat + (int64_t) bh * E;
     const int n = re - rb;
-    // lane i: query block of entry 32 c + i of the chunk c being requested and of the one after it (clamped: nothing is read outside the
-    // tensors)
-    int cur_qb = 0, nx_qb = 0;
     auto fetch = [&](int i0) {
-      if (i0 + lane < n) nx_qb = min(max(__ldcg(fl + rb + i0 + lane), 0), (int) a.nq1 - 1);
+      if (i0 + lane < n) nx_qb = __ldcg(fl + rb + i0 + lane);
     };
-    fetch(0);
     int rst = st;                            // ring stage of the next request
     const float* stat = (lane < 16 ? a.lse : a.delta) + bh * a.Nq + (lane & 15);
     auto request = [&](int i) {              // Q and dO tile by TMA, lse and delta by one 4-byte copy per lane
       if (i < n) {
         if ((i & 31) == 0) {
-          cur_qb = nx_qb;
+          cur_qb = min(max(nx_qb, 0), (int) a.nq1 - 1);      // nothing is read outside the tensors
           fetch(i + 32);
         }
         const int qb = __shfl_sync(0xffffffffu, cur_qb, i & 31);
@@ -714,11 +726,6 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
     };
     request(0);
     request(1);
-    // Bucket walk: lane l holds the end of bucket jb + l, so the bucket of an entry is the number of ends at or below it, and the next
-    // non-empty bucket is known without a load while the one at hand is being worked on.
-    auto bucket_end = [&](int j0) { return j0 + 1 + lane <= n1 ? (int) csr_off(a, bh, j0 + 1 + lane) : 0x7fffffff; };
-    int jb = min(max(__ldcg(&a.ranges[bh * R + r0].y), 0), n1 - 1);
-    int ends = bucket_end(jb), ends2 = bucket_end(jb + 32);
     int j = -1, nxt = rb, j2 = 0, nxt2 = 0;  // the bucket at hand and its end, the one after it and its end
     auto find_bucket = [&](int e) {          // j2, nxt2: the bucket of entry e
       int c = __popc(__ballot_sync(0xffffffffu, ends <= e));
@@ -747,8 +754,9 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
         }
       }
     };
+    const int c0 = __popc(__ballot_sync(0xffffffffu, ends <= rb)), end_c0 = __shfl_sync(0xffffffffu, ends, (c0 - 1) & 31);
     find_bucket(rb);
-    bool began_before = (int) csr_off(a, bh, j2) < rb;
+    bool began_before = (c0 == 0 ? begin_jb : c0 < 32 ? end_c0 : (int) csr_off(a, bh, j2)) < rb;      // the first bucket's begin lies in front of rb
     request_bucket();
     for (int i = 0; i < n; ++i) {
       const int e = rb + i;
