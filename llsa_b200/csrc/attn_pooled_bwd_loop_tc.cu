@@ -16,7 +16,7 @@
 // TMEM columns, chunk number n of the CTA (counted over all its tiles): S, and dS over it, at 64 (n mod 4); dP at [256 + 64 (n mod 2), + 64); dQ of
 // tile i at [384 + 64 (i mod 2), + 64).
 // Roles (one persistent CTA per SM, 16 warps; warps 8 to 11 run in step, tc05.cuh: umma_ss_k64): warps 8 and 11 = TMA producers (Q, dO per
-// tile, 2 stages, and K chunks; V chunks; one ring of 8 pairs), warp 9 issues S and dP, warp 10 dQ, warps 0-3 / 4-7 = two softmax
+// tile, 2 stages, and K chunks; V chunks; one ring of 8 pairs, 7 with a remainder), warp 9 issues S and dP, warp 10 dQ, warps 0-3 / 4-7 = two softmax
 // warpgroups on alternating chunks, warps 12-15 = epilogue, thread = row: adds dQ to the row.  A softmax thread takes its whole row of S and
 // dP into registers at once (which is what the register split is for) and hands the dP buffer back before it begins, so that two dP buffers
 // do and S gets four.  The two issuing warps run independently (S / dP of the next tile start while dQ of this one is still being issued); an
@@ -29,6 +29,8 @@
 // producer's two waits and two copies and left the tensor pipe idle at every tile boundary.
 // Every mbarrier wait is bounded (abort flag; the kernel then ends early and frees its TMEM; dq is left partial).
 #include <string.h>
+
+#include <type_traits>
 
 #include "attn.cuh"
 #include "mma_frag.cuh"
@@ -43,7 +45,8 @@ constexpr int kRows = 128;
 constexpr int kCk = 64;                      // keys per chunk
 constexpr int kTile = kRows * 64;            // elements of a [128 x 64] bf16 tile (16 KB)
 constexpr int kChunkElems = kCk * 64;        // elements of a key chunk (8 KB)
-constexpr int kStages = 8;
+template <bool REM>
+constexpr int kRing = REM ? 7 : 8;            // key and value chunks; the remainder's tile takes the place of one pair
 constexpr int kThreads = 512;
 constexpr int kLaunchRegs = 128, kIssueRegs = 40, kEpilogueRegs = 88, kSoftmaxRegs = 192;     // a thread's, per role: 40 + 88 + 2 x 192 = 4 x 128
 static_assert(kIssueRegs + kEpilogueRegs + 2 * kSoftmaxRegs <= 4 * kLaunchRegs, "the takers would wait for good");
@@ -52,29 +55,25 @@ static_assert(kIssueRegs + kEpilogueRegs + 2 * kSoftmaxRegs <= 4 * kLaunchRegs, 
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr int kBufs = 4;                     // S buffers (dS over them)
 constexpr uint32_t kColDP = 256, kColDQ = 384;
-// Up to this many chunks a tile the epilogue is the pace, and the first half of a row's remainder is requested with the fine part, ahead of the
-// wait; beyond, the softmax is, and the remainder is better left until it is needed, a quarter of a row at a time.  Backward in us, ahead / a
-// quarter at a time: 1 chunk (one level, B=2 H=6 N=1024) 45.4 / 46.4, 4 (two levels, top-8 parents, H=6 N=24576) 211 / 214, 5 (H=5 N=40960)
-// 287 / 290, 6 (top-16 parents, H=6 N=24576) 242 / 239, 7 (H=5 N=40960) 391 / 384, 17 (one level, B=2 H=6 N=16896) 383 / 375.
-constexpr int kAheadJobs = 5;
-
 struct DqMaps {
   CUtensorMap q, d_o;         // [B,H,Nq,64] 4-D, box 128 rows
+  CUtensorMap dq, rem;        // [B,H,Nq,64] 4-D; [BH*Nq, 64]; box 32 rows
   CUtensorMap kg, vg;         // gathered level-1 keys / values (two levels): [BH*n1, 64], box 16 rows
   CUtensorMap kc, vc;         // contiguous pooled keys / values: [BH*n, 64], box 64 rows
 };
 
 struct DqBars {
-  uint64_t q_full[2], q_empty[2], kv_full[kStages], kv_empty[kStages];
+  uint64_t q_full[2], q_empty[2], kv_full[8], kv_empty[8], out_full[4][2], rem_full[4];
   uint64_t sdp_ready[kBufs], ds_ready[kBufs], buf_free[kBufs], dp_free[2], dq_ready[2], dq_free[2];
 };
 
 // jobs: 64-key chunks per tile; gathered: number of leading chunks that are gathered level-1 blocks; n_c: rows per head of the
-// contiguous pooled tensor.  REM: the fine part of dq is the bf16 value in dq plus its remainder in a.rem.  AHEAD: jobs <= kAheadJobs.
-template <bool REM, bool AHEAD>
+// contiguous pooled tensor.  REM: the fine part of dq is the bf16 value in dq plus its remainder in a.rem.
+template <bool REM>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps, int jobs, int gathered, int64_t n_c, int n_tiles,
                               int tiles_per_head) {
+  constexpr int kStages = kRing<REM>;
   extern __shared__ unsigned char smem_dyn[];
   __shared__ DqBars bars;
   __shared__ uint32_t s_tmem;
@@ -84,6 +83,8 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
   bf16* sDO = sQ + 2 * kTile;               // [2][128][64]
   bf16* sK = sDO + 2 * kTile;               // [kStages][64][64]
   bf16* sV = sK + kStages * kChunkElems;    // [kStages][64][64]
+  bf16* sOut = sV + kStages * kChunkElems;  // [2][128][64]: dq
+  bf16* sRem = sOut + 2 * kTile;            // REM: [128][64]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile tc::WaitCtl* abort_flag = &s_ctl;
 
@@ -107,6 +108,11 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
       tc::mbar_init(&bars.dq_ready[i], 1);
       tc::mbar_init(&bars.dq_free[i], 4);
       tc::mbar_init(&bars.dp_free[i], 4);
+    }
+    for (int i = 0; i < 4; ++i) {
+      tc::mbar_init(&bars.out_full[i][0], 1);
+      tc::mbar_init(&bars.out_full[i][1], 1);
+      tc::mbar_init(&bars.rem_full[i], 1);
     }
     tc::fence_mbar_init();
   }
@@ -288,54 +294,69 @@ attn_dq_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ DqMaps maps
   } else {
     tc::regs_set<kEpilogueRegs, kLaunchRegs>();
     // ---------------------------------------------------------------- dq += dQ; thread = query row
-    const int qd = warp & 3, r = qd * 32 + lane;
+    // A warp's 32 rows of dq (and of the remainder) come by TMA a tile ahead and leave by TMA from the same memory.  As loads and stores of 16 bytes a
+    // lane, 128 bytes apart, they took the epilogue longer than a tile of a few chunks lasts: kernel at three chunks with a remainder (two levels, B=3 H=5
+    // N=5376) 21.4 us, now 17.5, at seven (H=5 N=40960, top-16) 47.2 / 45.9, at four without (one level, B=4 H=6 N=4096) 22.6 / 21.4; long lists 668 / 666.
+    const int w = warp & 3, r = w * 32 + lane;
+    const uint32_t out_row = tc::smem_u32(sOut) + (uint32_t) r * 128 + ((r & 7) << 4), rem_row = out_row + 2 * kTile * 2;      // the row's first chunk, swizzled
+    auto request = [&](int i) {              // dq of tile i into stage i & 1
+      const int tile = blockIdx.x + i * gridDim.x, bh = tile / tiles_per_head;
+      tma::expect_tx_w(&bars.out_full[w][i & 1], 32 * 128);
+      tma::load_4d_w(sOut + (i & 1) * kTile + w * 32 * 64, &maps.dq, &bars.out_full[w][i & 1], 0, (tile % tiles_per_head) * kRows + w * 32, bh % a.H, bh / a.H);
+    };
+    auto request_rem = [&](int i) {
+      const int tile = blockIdx.x + i * gridDim.x;
+      tma::expect_tx_w(&bars.rem_full[w], 32 * 128);
+      tma::load_2d_w(sRem + w * 32 * 64, &maps.rem, &bars.rem_full[w], 0, tile * kRows + w * 32);
+    };
+    if (n_my > 0) {
+      request(0);
+      if (REM) request_rem(0);
+    }
     bool ok = true;
     for (int i = 0; ok && i < n_my; ++i) {
-      const int tile = blockIdx.x + i * gridDim.x;
-      const int bh = tile / tiles_per_head, row = (tile % tiles_per_head) * kRows + r;
-      bf16* dqrow = a.dq.row(bh / a.H, bh % a.H, row);
-      uint4 old[8], rest[4];               // the fine part, requested before the wait, and half a row of its remainder
-      const uint4* rp = REM ? reinterpret_cast<const uint4*>(a.rem + ((int64_t) bh * a.Nq + row) * kD) : nullptr;
-#pragma unroll
-      for (int q8 = 0; q8 < 8; ++q8) old[q8] = *reinterpret_cast<const uint4*>(dqrow + 8 * q8);
-      if (REM && AHEAD) {
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) rest[q4] = rp[q4];
-      }
-      ok = __all_sync(0xffffffffu, tc::bounded_wait(&bars.dq_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
+      const int tile = blockIdx.x + i * gridDim.x, bh = tile / tiles_per_head, row0 = (tile % tiles_per_head) * kRows;
+      const uint32_t out = out_row + (i & 1) * (kTile * 2), t_q = tmem + kColDQ + (i & 1) * 64 + ((uint32_t) (w * 32) << 16);
+      ok = tc::warp_wait(lane & 1 ? &bars.out_full[w][i & 1] : &bars.dq_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag);
+      ok = ok && (!REM || tc::warp_wait(&bars.rem_full[w], (uint32_t) i & 1, abort_flag));
       tc::fence_after_sync();
       if (!ok) break;
-#pragma unroll
-      for (int part = 0; part < 4; ++part) {
-        float v[16];
-        if (REM && !AHEAD) {
-          rest[(part & 1) * 2] = rp[part * 2];
-          rest[(part & 1) * 2 + 1] = rp[part * 2 + 1];
-        }
-        tc::tmem_ld16(tmem + kColDQ + (i & 1) * 64 + part * 16 + ((uint32_t) (qd * 32) << 16), v);
-        if (part == 3) {
-          tc::fence_before_sync();
-          __syncwarp();
-          if (lane == 0) tma::mbar_arrive(&bars.dq_free[i & 1]);
-        }
-#pragma unroll
-        for (int q2 = 0; q2 < 2; ++q2) {
-          const uint4 f = old[part * 2 + q2];
-          auto sum = [&](uint32_t fine, uint32_t left, int e) {
-            const float x = REM ? bf16_lo(fine) + bf16_lo(left) : bf16_lo(fine), y = REM ? bf16_hi(fine) + bf16_hi(left) : bf16_hi(fine);
-            return pack_bf16(fmaf(v[8 * q2 + e], a.scale, x), fmaf(v[8 * q2 + e + 1], a.scale, y));
-          };
-          uint4 w;
-          const uint4 left = rest[(part & 1) * 2 + q2];
-          if (REM && AHEAD && part < 2) rest[(part & 1) * 2 + q2] = rp[(part + 2) * 2 + q2];      // the second half's, two parts ahead
-          w.x = sum(f.x, left.x, 0);
-          w.y = sum(f.y, left.y, 2);
-          w.z = sum(f.z, left.z, 4);
-          w.w = sum(f.w, left.w, 6);
-          *reinterpret_cast<uint4*>(dqrow + part * 16 + 8 * q2) = w;
-        }
+      if (i + 1 < n_my) {
+        tma::reduce_wait_read();             // the last tile has left the other stage
+        __syncwarp();
+        request(i + 1);
       }
+      float v[16];
+      auto sum = [&](auto tag, int e) {      // chunk C of the row, eight channels: v[e ..]
+        constexpr int C = decltype(tag)::value;
+        uint32_t f[4], l[4] = {0u, 0u, 0u, 0u};
+        lds128<0>(f[0], f[1], f[2], f[3], out ^ (16 * C));
+        if (REM) lds128<0>(l[0], l[1], l[2], l[3], rem_row ^ (16 * C));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float x = REM ? bf16_lo(f[k]) + bf16_lo(l[k]) : bf16_lo(f[k]), y = REM ? bf16_hi(f[k]) + bf16_hi(l[k]) : bf16_hi(f[k]);
+          f[k] = pack_bf16(fmaf(v[e + 2 * k], a.scale, x), fmaf(v[e + 2 * k + 1], a.scale, y));
+        }
+        tc::sts128_xor<16 * C>(out, f[0], f[1], f[2], f[3]);
+      };
+      tc::tmem_ld16(t_q, v);
+      sum(std::integral_constant<int, 0>{}, 0); sum(std::integral_constant<int, 1>{}, 8);
+      tc::tmem_ld16(t_q + 16, v);
+      sum(std::integral_constant<int, 2>{}, 0); sum(std::integral_constant<int, 3>{}, 8);
+      tc::tmem_ld16(t_q + 32, v);
+      sum(std::integral_constant<int, 4>{}, 0); sum(std::integral_constant<int, 5>{}, 8);
+      tc::tmem_ld16(t_q + 48, v);
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tma::mbar_arrive(&bars.dq_free[i & 1]);
+      sum(std::integral_constant<int, 6>{}, 0); sum(std::integral_constant<int, 7>{}, 8);
+      tc::fence_async_smem();
+      __syncwarp();
+      tma::store_4d_w(&maps.dq, 0, row0 + w * 32, bh % a.H, bh / a.H, tc::smem_u32(sOut + (i & 1) * kTile + w * 32 * 64));
+      tma::reduce_commit_w();
+      if (REM && i + 1 < n_my) request_rem(i + 1);
     }
+    tma::reduce_wait_all();                  // dq is in memory before the kernel ends
   }
   if (abort_flag->abort) tc::abort_drain();
   tc::fence_before_sync();
@@ -355,6 +376,8 @@ int launch_attn_dq_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, i
   int rc;
   if ((rc = tma::make_map_bhnd(&maps.q, g->q, kRows))) return rc;
   if ((rc = tma::make_map_bhnd(&maps.d_o, g->d_o, kRows))) return rc;
+  if ((rc = tma::make_map_bhnd(&maps.dq, g->dq, 32))) return rc;
+  if (a.rem && (rc = tma::make_map_rows(&maps.rem, a.rem, (uint64_t) BH * a.Nq, 32))) return rc;
   const int64_t n_c = a.two_level ? (int64_t) a.p2_blocks * kBS : a.n1;
   const int gathered = a.two_level ? (a.p1_blocks + 3) / 4 : 0, jobs = gathered + (int) ((n_c + kCk - 1) / kCk);
   if (gathered) {
@@ -370,9 +393,8 @@ int launch_attn_dq_pooled_loop_tc(const LlsaAttnArgs* g, const AttnP<bf16>& a, i
   LLSA_CUDA_OK(cudaGetDevice(&dev));
   LLSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int grid = n_tiles < sms ? n_tiles : sms;
-  const size_t smem = 1024 + (size_t) (4 * kTile + 2 * kStages * kChunkElems) * sizeof(bf16);
-  auto kernel = !a.rem ? attn_dq_pooled_loop_tc_kernel<false, false>
-                : jobs <= kAheadJobs ? attn_dq_pooled_loop_tc_kernel<true, true> : attn_dq_pooled_loop_tc_kernel<true, false>;
+  const size_t smem = 1024 + (size_t) (6 * kTile + 2 * (a.rem ? kRing<true> : kRing<false>) * kChunkElems + (a.rem ? kTile : 0)) * sizeof(bf16);
+  auto kernel = a.rem ? attn_dq_pooled_loop_tc_kernel<true> : attn_dq_pooled_loop_tc_kernel<false>;
   LLSA_SMEM_LIMIT_REGS(kernel, smem, kLaunchRegs);
   launch_pdl(kernel, grid, kThreads, smem, st, a, maps, jobs, gathered, n_c, n_tiles, tiles_per_head);
   LLSA_LAUNCH_OK("attn_dq_pooled_loop_tc_kernel");

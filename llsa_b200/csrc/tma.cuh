@@ -120,11 +120,19 @@ __device__ __forceinline__ void reduce_add_2d_w(const CUtensorMap* map, int c0, 
                "r"(smem_src)
                : "memory");
 }
+// Shared memory tile -> global memory, in the same groups
+__device__ __forceinline__ void store_4d_w(const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t smem_src) {
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+               "@e cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];\n\t}" ::"l"(map), "r"(c0), "r"(c1), "r"(c2),
+               "r"(c3), "r"(smem_src)
+               : "memory");
+}
 __device__ __forceinline__ void reduce_commit_w() {
   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t@e cp.async.bulk.commit_group;\n\t}" ::: "memory");
 }
 // Every lane may execute the waits: a lane that has committed nothing passes
-__device__ __forceinline__ void reduce_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+template <int PENDING = 0>
+__device__ __forceinline__ void reduce_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory"); }
 __device__ __forceinline__ void reduce_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void expect_tx_w(uint64_t* mbar, uint32_t bytes) {
   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"

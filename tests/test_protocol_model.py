@@ -136,3 +136,10 @@ def test_two_softmax_groups_have_no_hazard_or_deadlock():
         tiles, chunks = rng.randint(1, 7), rng.randint(1, 4)
         assert outcome(forward_kernel, seed, tiles, chunks, 1 + seed % 2, groups=2) == "ok", seed
         assert outcome(forward_kernel, seed, tiles, chunks, 1, groups=2, second_round=True) == "ok", seed
+
+
+def test_query_major_ring_of_seven_has_no_hazard_or_deadlock():
+    """attn_dq_pooled_loop_tc_kernel with a remainder: seven ring stages, which no count of chunks or buffers divides."""
+    for seed in range(RUNS):
+        rng = random.Random(seed)
+        assert outcome(query_major_kernel, seed, rng.randint(1, 7), rng.randint(1, 9), stages=7) == "ok", seed
