@@ -222,9 +222,10 @@ static int front_bwd_typed(int n, const LlsaTensor* dy, const LlsaTensor* x, con
   const int64_t chunks = BH * a.chunks_per_head;
   LLSA_REQUIRE(chunks < (1ll << 31), LLSA_ERR_SHAPE, "rms_rope_bwd: too many rows");
   a.n_chunks = (int) chunks;
-  // One wave of four CTAs per SM over all tensors, and as many rows of partial weight gradients for the kernel behind it to add: two waves
-  // took the layer with norms and rotation, B=4 H=6 N=16384, 634 us instead of 630
-  const int64_t resident = kFbMaxCtas / n;
+  // With norms one wave of four CTAs per SM over all tensors, and as many rows of partial weight gradients for the kernel behind it to add: two waves
+  // took the layer with norms and rotation, B=4 H=6 N=16384, 634 us instead of 630.  Without, more and shorter CTAs even out better (rotation, B=4 H=6
+  // N=4096: 186.5 us, 187.6 with half as many).
+  const int64_t resident = norm_mask ? kFbMaxCtas / n : kFbMaxCtas;
   const int grid = (int) (chunks < resident ? chunks : resident);
   const bool want_dw = norm_mask && dw && (dw[0] || (n > 1 && dw[1]));
   a.dw_partial = want_dw ? (float*) dw_partial->ptr : nullptr;
