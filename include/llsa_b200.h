@@ -128,6 +128,9 @@ int llsa_rms_rope_bwd(int n_tensors, const LlsaTensor* dy, const LlsaTensor* x, 
  * descending, ties -> smallest index.  idx is I32 or I64 [B,H,M,topk].  Replaces
  * gen_sparse_indices (topk.py:6-9: torch.matmul + torch.topk). */
 int llsa_coarse_topk(const LlsaTensor* pq, const LlsaTensor* pk, const LlsaTensor* idx, int topk, void* stream);
+/* The same with a poll limit for the waits of the long-list tensor-core kernel (0: its own).  A CTA whose wait expires computes its rows with scalar
+ * arithmetic: the result is a selection either way. */
+int llsa_coarse_topk_bounded(const LlsaTensor* pq, const LlsaTensor* pk, const LlsaTensor* idx, int topk, int wait_limit, void* stream);
 /* Refine: for level-1 query block i with parent P = i / bs the candidates are
  * the children p*bs .. p*bs+bs-1 of p in p_idx[b,h,P,:]; fp32 scores, top-`topk`,
  * descending, ties -> smallest block index.  Replaces compute_topk_indices_sparse

@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "mma_frag.cuh"
+#include "topk_words.cuh"
 
 namespace llsa {
 
@@ -156,44 +157,8 @@ coarse_topk_kernel(const T* __restrict__ pq, const T* __restrict__ pk, void* __r
 // Large problems are bound by the latency of a warp's product and comparison chains (four warps per scheduler, tensor pipe 41 % busy);
 // keys through a cp.async ring or 24 warps per SM of one row tile each changed nothing.  n = M = 4096, 8 slices: 243 us with one pass
 // and lists of (value, column) pairs in four-warp CTAs of 64 rows, 139 now; n = M = 1024, 8 slices: 59 -> 20; n = M = 256, 24
-// slices: 24 -> 6.7; n = M = 64, 6 slices: 14.9 -> 3.7.
-constexpr int kCmTop = 8, kCmWarps = 8, kCmBoundFrom = 1024;
-
-__device__ __forceinline__ uint32_t umax(uint32_t a, uint32_t b) { return a > b ? a : b; }
-__device__ __forceinline__ uint32_t umin(uint32_t a, uint32_t b) { return a < b ? a : b; }
-
-template <uint32_t SEL>
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b) {      // selector bit 3 of a byte: its sign, replicated (__byte_perm drops that bit)
-  uint32_t d;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "n"(SEL));
-  return d;
-}
-
-// Candidate words of two neighbouring columns: cinv holds 65535 - c (low half) and 65535 - (c + 1) (high half).
-// NaN (0x7FFF after the conversion) ranks above everything as in torch.topk, -0 ties with +0.
-__device__ __forceinline__ void candidate_words(float s0, float s1, uint32_t cinv, uint32_t& k0, uint32_t& k1) {
-  __nv_bfloat162 p = __hadd2(__floats2bfloat162_rn(s0, s1), __float2bfloat162_rn(0.f));      // -0 + 0 = +0
-  const uint32_t u = *reinterpret_cast<uint32_t*>(&p);
-  const uint32_t o = u ^ (prmt<0xBB99>(u, 0u) | 0x80008000u);      // negative: all bits flipped, else the sign bit set
-  k0 = prmt<0x1054>(o, cinv);
-  k1 = prmt<0x3276>(o, cinv);
-}
-
-__device__ __forceinline__ float max_nan(float a, float b) {      // NaN if either is
-  float d;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
-  return d;
-}
-
-__device__ __forceinline__ void list_insert(uint32_t (&list)[kCmTop], uint32_t k) {
-  list[kCmTop - 1] = umax(list[kCmTop - 1], k);
-#pragma unroll
-  for (int u = kCmTop - 1; u > 0; --u) {
-    const uint32_t hi = umax(list[u - 1], list[u]), lo = umin(list[u - 1], list[u]);
-    list[u - 1] = hi;
-    list[u] = lo;
-  }
-}
+// slices: 24 -> 6.7; n = M = 64, 6 slices: 14.9 -> 3.7.  Long lists of many rows are topk_tc.cu's.
+constexpr int kCmWarps = 8, kCmBoundFrom = 1024;
 
 // ROWT row tiles per warp, KW warps share a CTA's keys, the other kCmWarps / KW are further row tiles.
 template <int ROWT, int KW>
@@ -275,10 +240,7 @@ coarse_topk_mma_kernel(const bf16* __restrict__ pq, const bf16* __restrict__ pk,
   for (int r = 0; r < ROWT; ++r)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const uint32_t w = bounded ? bound[wrow + r * 16 + g + 8 * e] : 0u;
-      thr[r][e] = w > 0u ? w - 1u : 0u;
-      const uint32_t below = (w >> 16) - ((w >> 16) == 0x8000u ? 2u : 1u);            // image of the bf16 value one step down (-0 is no step)
-      low[r][e] = w > 0x00800000u ? __uint_as_float((below & 0x8000u ? below ^ 0x8000u : ~below & 0xFFFFu) << 16) : -CUDART_INF_F;
+      bound_limits(bounded ? bound[wrow + r * 16 + g + 8 * e] : 0u, thr[r][e], low[r][e]);
 #pragma unroll
       for (int u = 0; u < kCmTop; ++u) list[r][e][u] = 0u;
     }
@@ -760,9 +722,16 @@ refine_topk_kernel(const T* __restrict__ pq1, const T* __restrict__ pk1, IdxView
   }
 }
 
+int launch_coarse_topk_tc(const LlsaTensor* pq, const LlsaTensor* pk, const LlsaTensor* idx, int topk, int wait_limit, cudaStream_t st);      // topk_tc.cu
+
 }  // namespace llsa
 
 using namespace llsa;
+
+// The tcgen05 kernel walks a list twice with one CTA per 128 rows; it takes lists of at least kCoarseTcFrom keys where that fills the SMs.  us, here / there:
+// 8 slices of n = M = 4096 (256 tiles) smooth 131 / 69, random 139 / 74; 3968, top-4 116 / 71; 2048 (128 tiles) 43.6 / 41.6 and 45.8 / 39; 144 slices of 1024
+// (1,152 tiles) 213 / 121 and 254 / 105; fewer tiles: 2 slices of 4096 (64) 46 / 48, 6 of 1024 (48) 12 / 23, 24 of 512 (96) 16.3 / 16.0, 6 of 512 (24) 7.4 / 16.7.
+constexpr int64_t kCoarseTcFrom = 512, kCoarseTcTiles = 128;
 
 // The tensor-core kernel's range: its accumulation order differs from the scalar kernels' in the last bit of a score, so the line
 // between the two decides which bits a caller gets and stays where it was (whole 64-key tiles, top-k <= 8).
@@ -773,6 +742,10 @@ static bool coarse_on_mma(const LlsaTensor* pq, const LlsaTensor* pk, int topk) 
 }
 
 extern "C" int llsa_coarse_topk(const LlsaTensor* pq, const LlsaTensor* pk, const LlsaTensor* idx, int topk, void* stream) {
+  return llsa_coarse_topk_bounded(pq, pk, idx, topk, 0, stream);
+}
+
+extern "C" int llsa_coarse_topk_bounded(const LlsaTensor* pq, const LlsaTensor* pk, const LlsaTensor* idx, int topk, int wait_limit, void* stream) {
   LLSA_REQUIRE(pq && pk && idx && pq->ptr && pk->ptr && idx->ptr, LLSA_ERR_NULL, "coarse_topk: null tensor");
   LLSA_REQUIRE(pq->ndim == 4 && pk->ndim == 4, LLSA_ERR_SHAPE, "coarse_topk: pq, pk must be [B,H,M,D]");
   const int64_t B = pq->shape[0], H = pq->shape[1], M = pq->shape[2], D = pq->shape[3], n = pk->shape[2];
@@ -791,6 +764,7 @@ extern "C" int llsa_coarse_topk(const LlsaTensor* pq, const LlsaTensor* pk, cons
   const int idx64 = idx->dtype == LLSA_I64;
   const bool bf = pq->dtype == LLSA_BF16;
   auto blocks = [&](int rows) { return dim3((unsigned) ((M + rows - 1) / rows), BH); };
+  if (coarse_on_mma(pq, pk, topk) && n >= kCoarseTcFrom && B * H * ((M + 127) / 128) >= kCoarseTcTiles) return launch_coarse_topk_tc(pq, pk, idx, topk, wait_limit, st);
   if (coarse_on_mma(pq, pk, topk)) {
     const bf16 *q = (const bf16*) pq->ptr, *k = (const bf16*) pk->ptr;
     // 64 rows per CTA (each key read from L2 once per 64 rows) where that still gives every SM two CTAs, else 16 rows, the keys

@@ -3,13 +3,16 @@
 // A CTA owns 128 query rows and walks the head's keys twice, 128 at a time (a job):  S = Q.K_c^T  [128 x 128] into tensor memory, thread = query row.
 //   * Pass 1 keeps the maxima of 16 interleaved groups of columns per thread, 32 per row; the eighth largest bounds the row's eighth score from
 //     below, and some nine scores of a row reach it, whatever its length.
-//   * Pass 2 computes the same scores again and looks, eight columns at a time, only at what reaches the bound: candidates as words (topk_words.cuh)
-//     are set aside in shared memory and sorted at the end (inserted at once, with the warp's other rows waiting, they are half of the kernel's time).
+//   * Pass 2 computes the same scores again and looks, eight columns at a time, for what reaches the bound.  Eight such scores are set aside in shared
+//     memory as they are; they become candidates (topk_words.cuh) and go into the thread's sorted list when a warp's rows have several of them.  (Taken
+//     at once, with the warp's other rows waiting, one such group cost some 500 cycles: 65 and 87 us at n = M = 4096, 8 slices, smooth and random.)
 // Two warpgroups take alternate jobs (odd and even), each with two score buffers of its own, half a job each, so that the products of one half run while
 // the other is looked at; they share a row's bound and merge its two lists through
 // shared memory.  Roles: warps 0-3 / 4-7 the two groups, warp 8 TMA producer (queries once, a ring of 4 key chunks), warp 9 issues the products.
-// What bounds it: the comparisons, 64 maxima a thread and job in either pass next to 256 cycles of tensor pipe; two CTAs share an SM, so that one's hand-overs
-// are hidden by the other's work.
+// What bounds it: instructions of pass 2 where some row of a warp has something to set aside (nearly half of the groups of eight), two thirds of all; the
+// comparisons are 64 maxima a thread and job in either pass, the tensor pipe takes 384 cycles a job.  Two CTAs share an SM, so that one's hand-overs are hidden
+// by the other's work.  n = M = 4096, 8 slices: 69 us smooth, 74 random, 131 and 139 with mma.sync (topk.cu); whole layer, l1, B=2 H=4 N=65536 923 -> 856.
+// Same scores as there, bit for bit, in all but some 2 of 100,000 rows.
 // Every mbarrier wait is bounded.  A CTA whose wait expires computes its rows with scalar arithmetic instead (slowly, and with another order of the
 // sums): a selection that went missing would not show in anything downstream.
 #include <string.h>
@@ -25,10 +28,10 @@ namespace {
 
 constexpr int kRows = 128, kChunk = 128;
 constexpr int kTile = kRows * 64;            // elements of a [128 x 64] bf16 tile (16 KB)
-constexpr int kStages = 3;
+constexpr int kStages = 2;
 constexpr int kThreads = 320;
 constexpr int kGroups = 16;                  // column groups of a thread in pass 1
-constexpr int kHits = 24;                    // scores of a row and group that pass 2 sets aside before it takes them one by one
+constexpr int kSlots = 12;                   // groups of eight scores that a thread sets aside in pass 2
 
 struct CoarseMaps {
   CUtensorMap q, k;           // contiguous [BH*M, 64], [BH*n, 64], box 128 rows
@@ -62,9 +65,14 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
   __shared__ CoarseBars bars;
   __shared__ uint32_t s_tmem;
   __shared__ tc::WaitCtl s_ctl;
-  __shared__ uint32_t s_list[2][kRows][kHits + 1];       // + 1: a row's words walk the banks.  The groups' best maxima, what reaches the bound, their lists
   bf16* sQ = reinterpret_cast<bf16*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));      // [128][64]
   bf16* sK = sQ + kTile;                                 // [kStages][128][64]
+  // Pass 2: [slot][thread] eight scores as bf16, and their group; before and behind it the lists of maxima and of candidates, [group][row], a row's
+  // words walking the banks
+  uint4(*s_slot)[2 * kRows] = reinterpret_cast<uint4(*)[2 * kRows]>(sK + kStages * kTile);
+  uint16_t(*s_at)[2 * kRows] = reinterpret_cast<uint16_t(*)[2 * kRows]>(s_slot + kSlots);
+  uint32_t(*s_list)[kRows][kCmTop + 1] = reinterpret_cast<uint32_t(*)[kRows][kCmTop + 1]>(s_slot);
+  static_assert(kSlots * 16 >= (kCmTop + 1) * 4, "room for the lists");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile tc::WaitCtl* abort_flag = &s_ctl;
   const int64_t bh = blockIdx.y, row0 = (int64_t) blockIdx.x * kRows;
@@ -193,50 +201,64 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
     group_sync();                                            // both groups have read the maxima
     uint32_t list[kCmTop], thr, w, none;
     float low;
-    int hits = 0;
     candidate_words(eighth, 0.f, 0u, w, none);
     bound_limits(eighth > -CUDART_INF_F ? w & 0xFFFF0000u : 0u, thr, low);      // fewer than eight groups above -inf: no bound
 #pragma unroll
     for (int u = 0; u < kCmTop; ++u) list[u] = 0u;
+    int held = 0;                                            // slots in use
+    auto flush = [&] {                                       // what was set aside -> the list
+#pragma unroll 1
+      for (int u = 0; __any_sync(0xffffffffu, u < held); ++u) {
+        if (u < held) {
+          const uint4 x = s_slot[u][tid];
+          const uint32_t p[4] = {x.x, x.y, x.z, x.w}, c = 8u * s_at[u][tid];
+#pragma unroll 1
+          for (int e = 0; e < 4; ++e) {
+            uint32_t k[2];
+            const uint32_t pe = e == 0 ? p[0] : e == 1 ? p[1] : e == 2 ? p[2] : p[3];
+            candidate_words(__uint_as_float(pe << 16), __uint_as_float(pe & 0xFFFF0000u), (65535u - c - 2 * e) | ((65534u - c - 2 * e) << 16), k[0], k[1]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              if (k[i] > thr) {
+                list_insert(list, k[i]);
+                thr = umax(thr, list[kCmTop - 1]);
+              }
+          }
+        }
+      }
+      __syncwarp();
+      held = 0;
+      // A full list leaves out what rounds to its last score as well: the columns that follow are larger
+      if (list[kCmTop - 1]) {
+        const uint32_t image = list[kCmTop - 1] >> 16, last = (image & 0x8000u ? image ^ 0x8000u : ~image & 0xFFFFu) << 16;
+        low = fmaxf(low, __uint_as_float(last & 0x80000000u ? last - 1u : last + 1u));
+      }
+    };
     for (; ok && j < jobs; j += 2) {
       const int c = j - chunks, nq = 2 * halves(c);
 #pragma unroll 1
       for (int q4 = 0; q4 < 4; ++q4) {
-        __syncwarp();                                        // rows went different ways
         if (!(q4 & 1) && !ready(j, q4 >> 1)) break;
         if (q4 < nq) quarter(q4);
         if (q4 & 1) give_back(q4 >> 1);
         if (q4 >= nq) continue;
-        const uint32_t c0 = (uint32_t) (c * kChunk + q4 * 32);
+        if (__any_sync(0xffffffffu, held > kSlots - 4)) flush();
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           float x = max3_nan(v[8 * u], v[8 * u + 1], v[8 * u + 2]);
           x = max3_nan(x, v[8 * u + 3], v[8 * u + 4]);
           x = max3_nan(x, v[8 * u + 5], v[8 * u + 6]);
-          if (max_nan(x, v[8 * u + 7]) < low) continue;      // false for NaN
-#pragma unroll
-          for (int e = 0; e < 8; ++e)
-            if (!(v[8 * u + e] < low)) {
-              candidate_words(v[8 * u + e], 0.f, 65535u - (c0 + 8 * u + e), w, none);
-              if (hits < kHits) {
-                s_list[wg][r][hits++] = w;
-              } else if (w > thr) {                          // many equal scores
-                list_insert(list, w);
-                thr = umax(thr, list[kCmTop - 1]);
-              }
-            }
+          if (!(max_nan(x, v[8 * u + 7]) < low)) {           // true for NaN
+            s_slot[held][tid] = make_uint4(pack_bf16(v[8 * u], v[8 * u + 1]), pack_bf16(v[8 * u + 2], v[8 * u + 3]), pack_bf16(v[8 * u + 4], v[8 * u + 5]),
+                                           pack_bf16(v[8 * u + 6], v[8 * u + 7]));
+            s_at[held++][tid] = (uint16_t) (c * (kChunk / 8) + q4 * 4 + u);
+          }
         }
+        __syncwarp();                                        // rows went different ways
       }
     }
-    __syncwarp();
-    for (int u = 0; __any_sync(0xffffffffu, u < hits); ++u) {
-      w = u < hits ? s_list[wg][r][u] : 0u;
-      if (w > thr) {
-        list_insert(list, w);
-        thr = umax(thr, list[kCmTop - 1]);
-      }
-    }
-    __syncwarp();
+    flush();
+    group_sync();                                            // both groups are through with their slots
     if (wg == 1) {
 #pragma unroll
       for (int u = 0; u < kCmTop; ++u) s_list[1][r][u] = list[u];
@@ -290,7 +312,7 @@ int launch_coarse_topk_tc(const LlsaTensor* pq, const LlsaTensor* pk, const Llsa
   int rc;
   if ((rc = tma::make_map_rows(&maps.q, pq->ptr, (uint64_t) (BH * M), kRows))) return rc;
   if ((rc = tma::make_map_rows(&maps.k, pk->ptr, (uint64_t) (BH * n), kChunk))) return rc;
-  const size_t smem = 1024 + (size_t) (1 + kStages) * kTile * sizeof(bf16);
+  const size_t smem = 1024 + (size_t) (1 + kStages) * kTile * sizeof(bf16) + (size_t) kSlots * 2 * kRows * (sizeof(uint4) + sizeof(uint16_t));
   LLSA_SMEM_LIMIT(coarse_topk_tc_kernel, smem);
   launch_pdl(coarse_topk_tc_kernel, dim3((unsigned) ((M + kRows - 1) / kRows), (unsigned) BH), kThreads, smem, st, maps, (const bf16*) pq->ptr,
              (const bf16*) pk->ptr, idx->ptr, idx->dtype == LLSA_I64 ? 1 : 0, M, n, topk, wait_limit);

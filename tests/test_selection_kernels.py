@@ -29,6 +29,42 @@ def test_coarse_topk_shapes(BH, M, n, dtype, topk):
     assert topk == 1 or (got.sort(-1).values.diff(dim=-1) > 0).all(), "duplicate block in a row"
 
 
+# the long-list kernel (128 tiles of 128 rows and more): its shortest list, a list that ends half way through a 128-key chunk (an odd and an even number of chunks), rows that do not
+# fill a tile
+@pytest.mark.parametrize("BH,M,n,topk", [(128, 40, 512, 8), (64, 130, 576, 8), (130, 40, 704, 5), (16, 1024, 1024, 4), (43, 300, 4160, 1), (129, 4, 8192, 8)])
+def test_coarse_topk_of_long_lists(BH, M, n, topk):
+    test_coarse_topk_shapes(BH, M, n, torch.bfloat16, topk)
+
+
+@pytest.mark.parametrize("wait_limit", [0, 1])
+@pytest.mark.parametrize("kind", ["ties", "equal", "nan", "-inf", "masked"])
+@pytest.mark.parametrize("n", [512, 1088])
+def test_coarse_topk_of_long_lists_orders_exact_scores(n, kind, wait_limit):
+    """Small whole numbers: sums are exact in any order, so the order of a row is known, ties to the smaller column and NaN first.  A limit of one
+    look makes the kernel's waits run out: its CTAs then select with scalar arithmetic."""
+    from llsa_b200 import _lib
+    gen = torch.Generator().manual_seed(n)
+    pq, pk = torch.randint(-2, 3, (1, 64, 200, 64), generator=gen).bfloat16(), torch.randint(-2, 3, (1, 64, n, 64), generator=gen).bfloat16()
+    pq[..., 0] = 1
+    if kind == "equal":
+        pk[:] = pk[:, :, :1]
+    elif kind == "nan":
+        pk[:, :, ::97, 3] = float("nan")
+        pq[:, :, 5, 7] = float("nan")
+    elif kind == "-inf":
+        pk[:, :, 40:n - 5, 0] = float("-inf")
+    elif kind == "masked":
+        pk[:, :, ::2] = 0
+        pk[:, :, ::2, 0] = -3e38
+    score = (pq.float() @ pk.float().transpose(-1, -2)).bfloat16().float()
+    rank = torch.where(score.isnan(), torch.full_like(score, float("inf")), score)
+    want = rank.sort(dim=-1, descending=True, stable=True).indices[..., :8].int()
+    q, k, got = pq.to(DEV), pk.to(DEV), torch.full((1, 64, 200, 8), -1, dtype=torch.int32, device=DEV)
+    d = [_lib.desc(t) for t in (q, k, got)]
+    _lib.check(_lib.lib().llsa_coarse_topk_bounded(*[_lib.ref(t) for t in d], 8, wait_limit, _lib.stream_ptr(torch.device(DEV))), "coarse_topk_bounded")
+    assert torch.equal(got.cpu(), want)
+
+
 def test_coarse_topk_zero_and_negative_scores_tie_and_order():
     """Scores of exactly zero of either sign tie, so the smaller column wins; all-negative rows come out in order."""
     pq, pk = torch.zeros(1, 1, 64, 64, dtype=torch.bfloat16), torch.zeros(1, 1, 128, 64, dtype=torch.bfloat16)
