@@ -408,60 +408,69 @@ __device__ __forceinline__ uint32_t orderable(float v) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// Refine selection with the candidates of a row in registers: lane l keeps candidates l, l + 32, ... (eight of them) as 64-bit words,
-// the order-preserving image of the score above the complemented block index, sorted once, so that its best is always slot 0.  A round is
-// one warp maximum over the score images and a ballot (a second maximum, over the complemented blocks, only where scores tie); the winner's
-// lane shifts its list up by one, and winner t stays in lane t until one store writes the row's list (top-k <= 32; a store by each winner
-// is 20 % slower).  A warp takes
-// two rows at a time: the rounds are chains of warp-wide instructions, and two chains hide each other's latency.
+// The best `topk` (at most 32) of up to 256 candidates of each of ROWS rows, lane l holding candidates l, l + 32, ... (eight of them) as 64-bit words: the
+// order-preserving image of the score above the complemented index; 0: none.  A lane sorts its words once, so that its best is always slot 0.  A
+// round is one warp maximum over the score images and a ballot (a second maximum, over the complemented indices, only where scores tie); the winner's
+// lane shifts its list up by one, and winner t stays in lane t of `mine`, complemented.  Two rows at a time: the rounds are chains of warp-wide
+// instructions, and two chains hide each other's latency.
+template <int ROWS>
+__device__ __forceinline__ void select_sorted8(uint64_t (&w)[ROWS][8], uint32_t (&mine)[ROWS], int topk, int lane) {
+  constexpr int SLOTS = 8;
+#pragma unroll
+  for (int e = 0; e < ROWS; ++e) {
+    mine[e] = 0u;
+#pragma unroll
+    for (int k = 2; k <= SLOTS; k <<= 1)                          // bitonic, descending
+#pragma unroll
+      for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+        for (int i = 0; i < SLOTS; ++i)
+          if ((i ^ j) > i) {
+            const bool desc = (i & k) == 0;
+            const uint64_t x = w[e][i], y = w[e][i ^ j];
+            const bool sw = desc ? y > x : x > y;
+            w[e][i] = sw ? y : x;
+            w[e][i ^ j] = sw ? x : y;
+          }
+  }
+  for (int t = 0; t < topk; ++t) {
+#pragma unroll
+    for (int e = 0; e < ROWS; ++e) {
+      const uint32_t hi = (uint32_t) (w[e][0] >> 32), lo = (uint32_t) w[e][0];
+      const uint32_t m = __reduce_max_sync(0xffffffffu, hi);
+      unsigned who = __ballot_sync(0xffffffffu, hi == m);
+      if (who & (who - 1)) {                                      // equal scores: the smallest index
+        const uint32_t ml = __reduce_max_sync(0xffffffffu, hi == m ? lo : 0u);
+        who = __ballot_sync(0xffffffffu, hi == m && lo == ml);
+      }
+      const int src = __ffs((int) who) - 1;
+      const uint32_t win = __shfl_sync(0xffffffffu, lo, src);
+      if (lane == t) mine[e] = win;
+      if (lane == src) {                                          // candidates are distinct: one owner
+#pragma unroll
+        for (int u = 0; u + 1 < SLOTS; ++u) w[e][u] = w[e][u + 1];
+        w[e][SLOTS - 1] = 0;
+      }
+    }
+  }
+}
+
+// Refine selection of lists of up to 256 candidates; one store writes a row's list (a store by each winner is 20 % slower).
 __device__ __forceinline__ void refine_select_sorted8(const float* sc, const int* cand, int C, int bs, int topk, void* idx_out, int idx64,
                                                       int64_t out_row0, int warp, int lane, int nwarps) {
-  constexpr int SLOTS = 8;
   for (int r0 = warp; r0 < bs; r0 += 2 * nwarps) {
-    uint64_t w[2][SLOTS];
-    uint32_t mine[2] = {0u, 0u};
+    uint64_t w[2][8];
+    uint32_t mine[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const float* s = sc + min(r0 + e * nwarps, bs - 1) * C;      // past the last row: computed on it and dropped
 #pragma unroll
-      for (int u = 0; u < SLOTS; ++u) {
+      for (int u = 0; u < 8; ++u) {
         const int j = lane + 32 * u;
         w[e][u] = (j < C && cand[j] >= 0) ? ((uint64_t) orderable(s[j]) << 32) | (0xFFFFFFFFu - (uint32_t) cand[j]) : 0;      // 0 is below every real candidate
       }
-#pragma unroll
-      for (int k = 2; k <= SLOTS; k <<= 1)                          // bitonic, descending
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1)
-#pragma unroll
-          for (int i = 0; i < SLOTS; ++i)
-            if ((i ^ j) > i) {
-              const bool desc = (i & k) == 0;
-              const uint64_t x = w[e][i], y = w[e][i ^ j];
-              const bool sw = desc ? y > x : x > y;
-              w[e][i] = sw ? y : x;
-              w[e][i ^ j] = sw ? x : y;
-            }
     }
-    for (int t = 0; t < topk; ++t) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const uint32_t hi = (uint32_t) (w[e][0] >> 32), lo = (uint32_t) w[e][0];
-        const uint32_t m = __reduce_max_sync(0xffffffffu, hi);
-        unsigned who = __ballot_sync(0xffffffffu, hi == m);
-        if (who & (who - 1)) {                                      // equal scores: the smallest block
-          const uint32_t ml = __reduce_max_sync(0xffffffffu, hi == m ? lo : 0u);
-          who = __ballot_sync(0xffffffffu, hi == m && lo == ml);
-        }
-        const int src = __ffs((int) who) - 1;
-        const uint32_t win = __shfl_sync(0xffffffffu, lo, src);
-        if (lane == t) mine[e] = win;
-        if (lane == src) {                                          // candidates are distinct blocks: one owner
-#pragma unroll
-          for (int u = 0; u + 1 < SLOTS; ++u) w[e][u] = w[e][u + 1];
-          w[e][SLOTS - 1] = 0;
-        }
-      }
-    }
+    select_sorted8<2>(w, mine, topk, lane);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int r = r0 + e * nwarps;
@@ -580,7 +589,7 @@ __device__ __forceinline__ void coarse_row_scalar(const FusedCoarse& f, int64_t 
   for (int j = threadIdx.x; j < n2; j += blockDim.x) {
     const T* k = reinterpret_cast<const T*>(f.pk2) + (bh * n2 + j) * 64;
     float acc = 0.f;
-#pragma unroll
+#pragma unroll 8
     for (int d = 0; d < 64; d += 4) {
       const float4 a = load4<T>(q + d), x = load4<T>(k + d);
       acc = fmaf(a.x, x.x, acc); acc = fmaf(a.y, x.y, acc); acc = fmaf(a.z, x.z, acc); acc = fmaf(a.w, x.w, acc);
@@ -589,11 +598,16 @@ __device__ __forceinline__ void coarse_row_scalar(const FusedCoarse& f, int64_t 
   }
   __syncthreads();
   if (warp == 0) {
-    uint64_t list = 0, thr = 0;
-    for (int j = lane; j - lane < n2; j += 32)
-      warp_list_insert(list, thr, j < n2 ? ((uint64_t) sc2[j] << 32) | (0xFFFFFFFFu - (uint32_t) j) : 0, p_topk, lane);
+    uint64_t w[1][8];
+    uint32_t mine[1];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int j = lane + 32 * u;
+      w[0][u] = j < n2 ? ((uint64_t) sc2[j] << 32) | (0xFFFFFFFFu - (uint32_t) j) : 0;
+    }
+    select_sorted8<1>(w, mine, p_topk, lane);
     if (lane < p_topk) {
-      const uint32_t col = 0xFFFFFFFFu - (uint32_t) list;
+      const uint32_t col = 0xFFFFFFFFu - mine[0];
       s_pidx[lane] = (int) col;
       const int64_t o = (bh * n2q + P) * p_topk + lane;
       if (f.pidx64) reinterpret_cast<int64_t*>(f.pidx_out)[o] = (int64_t) col;
@@ -603,9 +617,13 @@ __device__ __forceinline__ void coarse_row_scalar(const FusedCoarse& f, int64_t 
   __syncthreads();
 }
 
-// FUSED: 0 parents given, 1 selected here by coarse_row_64, 2 by coarse_row_scalar
+// FUSED: 0 parents given, 1 selected here by coarse_row_64, 2 by coarse_row_scalar.
+// A CTA is a chain of short steps (parents, keys, scores, rounds of the selection), so what counts is how many of them an SM holds, and that they are few
+// waves: 9 CTAs (8 with the scalar step, 6 in fp32) where the compiler's choice of registers allowed 8 and 5.  H=5 N=40960, top-16: 49 us with five an SM,
+// where 800 CTAs are 740 and a second wave of 60, parents inserted into a list one by one and keys loaded when they are needed; 32.8 now.  Lists of eight
+// parents: B=8 H=6 N=16384 31.8 -> 29.9, B=4 19.7 -> 18.6, B=1 8.8 -> 8.2, B=3 H=5 N=5376 10.0 -> 8.9.
 template <typename T, bool MMA, int FUSED = 0>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, FUSED < 2 ? 9 : sizeof(T) == 2 ? 8 : 6)
 refine_topk_kernel(const T* __restrict__ pq1, const T* __restrict__ pk1, IdxView p_idx, void* __restrict__ idx_out, int idx64, int64_t M,
                    int64_t Mk, int D_, int topk, int p_topk, int bs_, FusedCoarse fused) {
   pdl_trigger();
@@ -646,12 +664,16 @@ refine_topk_kernel(const T* __restrict__ pq1, const T* __restrict__ pk1, IdxView
       RowFrag qlo, qhi;
       load_rowfrag(qlo, reinterpret_cast<const bf16*>(q0) + g * D, t);
       load_rowfrag(qhi, reinterpret_cast<const bf16*>(q0) + (g + 8) * D, t);
-      for (int tile = warp_ * 2; tile < C / 8; tile += 8) {      // two 8-candidate n-tiles per step and warp
-        RowFrag ka, kb;
+      RowFrag ka, kb;
+      auto keys = [&](int tile) {
         load_rowfrag(ka, reinterpret_cast<const bf16*>(k0) + (int64_t) max(cand[tile * 8 + g], 0) * D, t);
         load_rowfrag(kb, reinterpret_cast<const bf16*>(k0) + (int64_t) max(cand[tile * 8 + 8 + g], 0) * D, t);
-        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_rows_x_keys(s0, s1, qlo, qhi, ka, kb);
+      };
+      if (warp_ * 2 < C / 8) keys(warp_ * 2);
+      for (int tile = warp_ * 2; tile < C / 8; tile += 8) {      // two 8-candidate n-tiles per step and warp; the next step's keys on their way
+        float s0[4], s1[4];
+        mma_rows_x_keys_z(s0, s1, qlo, qhi, ka, kb);
+        if (tile + 8 < C / 8) keys(tile + 8);
         // C fragment: rows g / g+8, candidates tile*8 + 2t, +1 (and +8 for the second tile)
         sc[g * C + tile * 8 + 2 * t] = s0[0];       sc[g * C + tile * 8 + 2 * t + 1] = s0[1];
         sc[(g + 8) * C + tile * 8 + 2 * t] = s0[2]; sc[(g + 8) * C + tile * 8 + 2 * t + 1] = s0[3];
