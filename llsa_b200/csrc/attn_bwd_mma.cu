@@ -233,9 +233,10 @@ constexpr int kDqStages = 3;
 struct KvMaps {
   CUtensorMap k, v;            // [B,H,N,64] 4-D, box 16 rows
 };
-// REM: what rounding dq to bf16 leaves over goes to a.rem, for the pooled stage to add (remainder_wanted).
+// REM: what rounding dq to bf16 leaves over goes to a.rem, for the pooled stage to add (remainder_wanted).  zero: clear the pooled-gradient
+// accumulators on the way, a few rows a warp.
 template <int NW, bool REM>
-__global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps maps) {
+__global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a, const __grid_constant__ KvMaps maps, bool zero) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t s_full[NW][kDqStages];
   __shared__ tc::WaitCtl s_ctl[NW];             // a warp's own: the warps of a CTA share nothing
@@ -263,6 +264,12 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a,
 #pragma unroll
   for (int s = 0; s < kDqStages - 1; ++s)
     if (s < n_glob) request(s);
+  if (zero) {      // lanes 0..15 a row of dpk, 16..31 of dpv
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int64_t r = qb; r < a.n1; r += a.nq1) reinterpret_cast<float4*>((lane < 16 ? a.dpk : a.dpv) + (bh * a.n1 + r) * kD)[lane & 15] = none;
+    if (a.two_level)
+      for (int64_t r = qb; r < a.n2; r += a.nq1) reinterpret_cast<float4*>((lane < 16 ? a.dpk2 : a.dpv2) + (bh * a.n2 + r) * kD)[lane & 15] = none;
+  }
   // shared addresses of stage 0: chunks 2t, 2t + 1 of row g (sa_f, sa_f ^ 16; row g + 8 is 1024 bytes on), ldmatrix rows of channels 0..15
   // (sa_m; ^ 32 c: channels 16c..)
   const uint32_t sa_f = ring_sa + g * 128 + (((2 * t) ^ g) << 4);
@@ -1001,14 +1008,17 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
   if (!rem) a.rem = nullptr;
   const bool loop_dkv = !tc && pooled_dq_loop_tc_keys(a) > 0 && !g->no_tcgen05, loop_dq = loop_dkv && (!rem || a.rem);
   if (mask & 1) {
-    if (!(g->stage_mask & 8)) {
-      int rc = zero_pooled_acc(g, st);
-      if (rc) return rc;
-    }
     constexpr int NWQ = 4;
     AttnP<bf16> aq = a;
     if (tc || loop_dq) aq.p1_blocks = aq.p2_blocks = 0;
     const int n_all = aq.p1_blocks + aq.p2_blocks;
+    // The fine kernel clears the pooled-gradient accumulators itself: a memset beside it (on another stream) finds no room until its last wave and holds up
+    // the stage that follows
+    const bool zero = !(g->stage_mask & 8);
+    if (zero && n_all) {
+      int rc = zero_pooled_acc(g, st);
+      if (rc) return rc;
+    }
     const int n_smem = n_all < 12 ? n_all : 12;   // 12 tiles = 54 KB of K+V, three CTAs per SM
     const size_t smem = (size_t) n_smem * kBS * kSmemPitch * sizeof(bf16) * 2;
     if (n_all == 0) {
@@ -1020,7 +1030,7 @@ int launch_attn_bwd_mma(const LlsaAttnArgs* g, cudaStream_t st) {
       const size_t ring = (size_t) NWQ * kDqStages * 2 * kRingTileBytes + 1024;
       auto fine = loop_dq && a.rem ? attn_dq_fine_kernel<NWQ, true> : attn_dq_fine_kernel<NWQ, false>;
       LLSA_SMEM_LIMIT(fine, ring);
-      launch_pdl(fine, dim3((unsigned) (a.nq1 / NWQ), BH), NWQ * 32, ring, st, aq, maps);
+      launch_pdl(fine, dim3((unsigned) (a.nq1 / NWQ), BH), NWQ * 32, ring, st, aq, maps, zero);
       LLSA_LAUNCH_OK("attn_dq_fine_kernel");
     } else {
       LLSA_SMEM_LIMIT((attn_dq_mma_kernel<NWQ>), smem);

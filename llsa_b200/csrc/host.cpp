@@ -242,13 +242,14 @@ void run_fwd(const Core& c, int topk, int topk_p, int bs, double w1, double w2, 
   if (t_keep_marks) keep_redo(redo);
 }
 
-// One side stream per device: the index transpose is needed only by the last stage of the backward and leaves most SMs idle.
+// One side stream per device: the index transpose is needed only by the last stage of the backward and leaves most SMs idle.  Of high priority: its
+// CTAs take the place of the first ones of the dQ stage that end, not of the last.
 at::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
   static std::mutex mu;
   static std::array<std::optional<at::cuda::CUDAStream>, C10_COMPILE_TIME_MAX_GPUS> streams;
   std::lock_guard<std::mutex> lock(mu);
   auto& s = streams[dev];
-  if (!s) s = at::cuda::getStreamFromPool(false, dev);
+  if (!s) s = at::cuda::getStreamFromPool(true, dev);
   return *s;
 }
 
@@ -341,15 +342,16 @@ void run_bwd(Core& c, const Dims& d, const LlsaTensor& d_o, const LlsaTensor& dq
     // the scratch belongs to the current stream; the side stream works between the two events
     const at::cuda::CUDAStream side = side_stream(like.device().index());
     Fork fork(cur, side);
-    // the accumulators are cleared and the lists transposed next to the dQ stage, which needs neither
-    if (!acc) {
+    // The lists are transposed next to the dQ stage, which does not need them.  The transpose is first in line: its CTAs find no room once those of
+    // the dQ stage have filled the SMs.  The scalar dQ stage has the accumulators cleared here too.
+    transpose(side);
+    if (!tensor_core && !acc) {
       if (acc1) C10_CUDA_CHECK(cudaMemsetAsync(scratch, 0, (2 * acc1 + 2 * acc2) * 4, side));
-    } else {
+    } else if (!tensor_core) {
       for (int i = 0; i < (c.two ? 4 : 2); ++i) C10_CUDA_CHECK(cudaMemsetAsync(acc[i], 0, (i < 2 ? acc1 : acc2) * 4, side));
     }
-    transpose(side);
     fork.record();
-    a.stage_mask = 1 | 8;
+    a.stage_mask = tensor_core ? 1 : 1 | 8;
     ok(llsa_attn_bwd(&a, cur), "attn_bwd");
     fork.join();
     a.stage_mask = 2 | 4;

@@ -7,8 +7,7 @@
 //     memory as they are; they become candidates (topk_words.cuh) and go into the thread's sorted list when a warp's rows have several of them.  (Taken
 //     at once, with the warp's other rows waiting, one such group cost some 500 cycles: 65 and 87 us at n = M = 4096, 8 slices, smooth and random.)
 // Two warpgroups take alternate jobs (odd and even), each with two score buffers of its own, half a job each, so that the products of one half run while
-// the other is looked at; they share a row's bound and merge its two lists through
-// shared memory.  Roles: warps 0-3 / 4-7 the two groups, warp 8 TMA producer (queries once, a ring of 4 key chunks), warp 9 issues the products.
+// the other is looked at; they share a row's bound and merge its two lists through shared memory.  Roles: warps 0-3 / 4-7 the two groups, warp 8 TMA producer (queries once, a ring of two key chunks), warp 9 issues the products.
 // What bounds it: instructions of pass 2 where some row of a warp has something to set aside (nearly half of the groups of eight), two thirds of all; the
 // comparisons are 64 maxima a thread and job in either pass, the tensor pipe takes 384 cycles a job.  Two CTAs share an SM, so that one's hand-overs are hidden
 // by the other's work.  n = M = 4096, 8 slices: 69 us smooth, 74 random, 131 and 139 with mma.sync (topk.cu); whole layer, l1, B=2 H=4 N=65536 923 -> 856.

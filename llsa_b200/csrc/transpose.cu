@@ -79,8 +79,9 @@ __device__ __forceinline__ void place_range(const TransposeArgs& a, int64_t bh, 
 }
 
 // ---- one CTA per (b,h) and key range ----------------------------------------------------------------
+// 32 registers a thread: 16 warps then take the room of one CTA of the dQ stage it runs beside (48 to 54 registers took that of two).
 template <int W>
-__global__ void __launch_bounds__(W * 32) transpose_range_kernel(TransposeArgs a, int keys_per_range, uint32_t t_magic) {
+__global__ void __launch_bounds__(W * 32, 64 / W) transpose_range_kernel(TransposeArgs a, int keys_per_range, uint32_t t_magic) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
