@@ -81,6 +81,11 @@ int llsa_mean_pool_bwd(const LlsaTensor* dy, const LlsaTensor* dx, int k, void* 
  * torch_op/flash_sparse_attention_res_1.py:42-44 and ..._res_2.py:49-55. */
 int llsa_pool_pyramid_fwd(int n_tensors, const LlsaTensor* x, const LlsaTensor* y1, const LlsaTensor* y2,
                           int block_size, void* stream);
+/* The same, beside the work of this library in front of it on the stream: it may begin before that has ended, and ends after it.  The calls in front, back
+ * to the last pooling call of another kind, must neither write x nor touch y1 / y2.  For the values of a layer, which its selection does not need: pool q
+ * and k, select, pool v beside, attend.  (bf16, 64 channels, blocks of 16; other forms run in order.) */
+int llsa_pool_pyramid_beside_fwd(int n_tensors, const LlsaTensor* x, const LlsaTensor* y1, const LlsaTensor* y2, int block_size, void* stream);
+
 /* The same pass with the 2-D RoPE apply fused in front (north-star item "fused 2D RoPE apply on Q/K ahead of
  * pooling"): tensors whose bit is set in rope_mask (bit i = x[i]) are rotated by the [N,C] table `freq` (even
  * columns sin, odd columns cos; same dtype as x) exactly as llsa_rope_fwd does, the rotated rows are written to

@@ -42,6 +42,7 @@ class LlsaAttnArgs(C.Structure):
 
 EXPORTS = [
     "llsa_version", "llsa_last_error_string", "llsa_mean_pool_fwd", "llsa_mean_pool_bwd", "llsa_pool_pyramid_fwd",
+    "llsa_pool_pyramid_beside_fwd",
     "llsa_rope_pool_pyramid_fwd", "llsa_rms_rope_pool_pyramid_fwd", "llsa_rms_norm_fwd",
     "llsa_rms_rope_bwd", "llsa_rms_rope_bwd_partial_elems",
     "llsa_rope_fwd", "llsa_rope_bwd", "llsa_coarse_topk", "llsa_coarse_topk_bounded", "llsa_refine_topk", "llsa_select_two_level", "llsa_transpose_scratch_bytes",
@@ -60,6 +61,7 @@ def _declare(lib: C.CDLL) -> None:
     lib.llsa_mean_pool_fwd.argtypes = [TP, TP, C.c_int, C.c_void_p]
     lib.llsa_mean_pool_bwd.argtypes = [TP, TP, C.c_int, C.c_void_p]
     lib.llsa_pool_pyramid_fwd.argtypes = [C.c_int, TP, TP, TP, C.c_int, C.c_void_p]
+    lib.llsa_pool_pyramid_beside_fwd.argtypes = [C.c_int, TP, TP, TP, C.c_int, C.c_void_p]
     lib.llsa_rope_pool_pyramid_fwd.argtypes = [C.c_int, TP, TP, C.c_int, TP, TP, TP, C.c_int, C.c_void_p]
     lib.llsa_rms_rope_pool_pyramid_fwd.argtypes = [C.c_int, TP, C.POINTER(TP), C.c_int, C.c_float, TP, C.c_int, TP, TP, TP, C.c_int, C.c_void_p]
     lib.llsa_rms_norm_fwd.argtypes = [TP, TP, C.c_float, TP, C.c_void_p]

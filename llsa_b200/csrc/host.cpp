@@ -242,6 +242,20 @@ void run_fwd(const Core& c, int topk, int topk_p, int bs, double w1, double w2, 
   if (t_keep_marks) keep_redo(redo);
 }
 
+// The values' share of the pooling pass runs beside the two-level selection, which reads little and leaves SMs idle, instead of in front of it: one launch
+// more.  Below the first line the host is the pace of a call; above the second the refinement fills the SMs one and a half times and more, and only
+// its end is left for the values.  Whole pass in us, in front / beside: B=1 H=6 N=4096 (1,536 query blocks) forward + backward 117 / 120; B=3 H=5 N=5376
+// (5,040) 148 / 144; B=1 H=6 N=16384 (6,144) 171 / 167, forward alone 46.8 / 47.2; B=2 H=6 N=16384 (12,288) 290 / 280, forward 82.0 / 77.9; B=1 H=5
+// N=40960, top-16 (12,800) 507 / 498; B=4 H=6 N=16384 (24,576) 506 / 505; B=2 H=4 N=65536 (32,768) forward 228 / 227; B=8 H=6 N=16384 (49,152)
+// 951 / 960; B=1 H=6 N=262144 (98,304) forward 1034 / 1045.
+// One level: no gain (B=2 H=4 N=16384 323 / 325).  With a norm or a rotation the values are a fifth of the pass: B=1 H=6 N=16384 57.9 / 59.1.
+constexpr int64_t kValuesBesideFrom = 4096, kValuesBesideTo = 24576;
+bool values_beside(const Dims& d, int64_t D, at::ScalarType dt, bool two, bool transformed) {
+  const int64_t blocks = d.B * d.H * d.nq1;
+  return two && !transformed && dt == at::kBFloat16 && D == 64 && d.bs == 16 && blocks >= kValuesBesideFrom && blocks <= kValuesBesideTo &&
+         !g_has_hook.load(std::memory_order_relaxed);      // a stage hook's stages do not overlap
+}
+
 // One side stream per device: the index transpose is needed only by the last stage of the backward and leaves most SMs idle.  Of high priority: its
 // CTAs take the place of the first ones of the dQ stage that end, not of the last.
 at::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
@@ -466,10 +480,11 @@ std::vector<Tensor> layer_fwd(const Tensor& q_, const Tensor& k_, const Tensor& 
     else if (freq.scalar_type() == at::kDouble || (dt == at::kFloat && freq.scalar_type() == at::kBFloat16)) freq = freq.to(at::kFloat);
     if (!table_ok(freq)) freq = freq.contiguous();
   }
+  const bool v_beside = values_beside(d, D, dt, two, freq.defined() || norm);
   mark("pool_pyramid");
   if (!freq.defined() && !norm) {
     const LlsaTensor x[3] = {desc(q), desc(k), desc(v)};
-    ok(llsa_pool_pyramid_fwd(3, x, y1, two ? y2 : nullptr, (int) block_size, st), "pool_pyramid_fwd");
+    ok(llsa_pool_pyramid_fwd(v_beside ? 2 : 3, x, y1, two ? y2 : nullptr, (int) block_size, st), "pool_pyramid_fwd");
   } else {
     LlsaTensor x[3] = {desc(q), desc(k), desc(v)}, xr[3], f;
     // without a table a tensor that has no norm passes unchanged: a copy, since an output of the operator must not be its input
@@ -513,6 +528,7 @@ std::vector<Tensor> layer_fwd(const Tensor& q_, const Tensor& k_, const Tensor& 
     mark("coarse_topk");
     ok(llsa_coarse_topk(&y1[0], &y1[1], &c.indices, topk1, st), "coarse_topk");
   }
+  if (v_beside) ok(llsa_pool_pyramid_beside_fwd(1, &c.v, &y1[2], two ? &y2[2] : nullptr, (int) block_size, st), "pool_pyramid_beside_fwd");
   // ---- attention
   Tensor o = at::empty_like(q);
   c.o = desc(o);

@@ -63,6 +63,7 @@ struct PyramidArgs {
   const float* norm_w[3];
   float eps;
   int norm_mask;
+  bool beside;     // launched to run beside the kernel in front of it (llsa_pool_pyramid_beside_fwd)
 };
 
 // RMSNorm of one token row held by `lanes` neighbouring threads (VEC consecutive channels each; lanes a power of two, the
@@ -279,6 +280,8 @@ __global__ void __launch_bounds__(128) pool_pyramid_bf16_kernel(PyramidArgs<__nv
       reinterpret_cast<uint32_t*>(a.y2[ti] + ((int64_t) bh * groups_per_head + grp) * C)[threadIdx.x] = mul2(s, kSixteenth);
     }
   }
+  // one CTA is enough for the kernel not to end before the one in front of it; the others make room for the next
+  if (a.beside && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1) pdl_wait();
 }
 
 // One output row chunk per thread, any k; VEC = 1 handles channel counts that are not a multiple of 16 bytes.
@@ -408,6 +411,7 @@ static void launch_pyramid_bf16(const PyramidArgs<__nv_bfloat16>& a, dim3 grid, 
   if (a.rope_mask && a.norm_mask) pool_pyramid_bf16_kernel<LEVELS, true, true><<<grid, 128, 0, st>>>(a, groups);
   else if (a.rope_mask) pool_pyramid_bf16_kernel<LEVELS, true, false><<<grid, 128, 0, st>>>(a, groups);
   else if (a.norm_mask) pool_pyramid_bf16_kernel<LEVELS, false, true><<<grid, 128, 0, st>>>(a, groups);
+  else if (a.beside) launch_pdl(pool_pyramid_bf16_kernel<LEVELS, false, false>, grid, 128, 0, st, a, groups);
   else pool_pyramid_bf16_kernel<LEVELS, false, false><<<grid, 128, 0, st>>>(a, groups);
 }
 
@@ -421,10 +425,12 @@ static void launch_pyramid_variant(const PyramidArgs<T>& a, dim3 grid, int threa
 
 template <typename T>
 static int launch_pyramid(int n, const LlsaTensor* x, const LlsaTensor* y1, const LlsaTensor* y2, int bs, cudaStream_t st,
-                          const LlsaTensor* freq = nullptr, int rope_mask = 0, const LlsaTensor* xr = nullptr, const NormSpec* norm = nullptr) {
+                          const LlsaTensor* freq = nullptr, int rope_mask = 0, const LlsaTensor* xr = nullptr, const NormSpec* norm = nullptr,
+                          bool beside = false) {
   constexpr int VEC = Vec16<T>::N;
   PyramidArgs<T> a;
   memset(&a, 0, sizeof(a));
+  a.beside = beside;
   a.rope_mask = freq ? rope_mask : 0;
   a.norm_mask = norm ? norm->mask : 0;
   if (a.rope_mask) {
@@ -472,7 +478,7 @@ static int launch_pyramid(int n, const LlsaTensor* x, const LlsaTensor* y1, cons
 
 static int pyramid_entry(int n_tensors, const LlsaTensor* x, const LlsaTensor* y1, const LlsaTensor* y2, int block_size, void* stream,
                          const LlsaTensor* freq, int rope_mask, const LlsaTensor* xr, const LlsaTensor* const* norm_w = nullptr, int norm_mask = 0,
-                         float eps = 0.f) {
+                         float eps = 0.f, bool beside = false) {
   LLSA_REQUIRE(x && y1, LLSA_ERR_NULL, "pool_pyramid: null tensor list");
   LLSA_REQUIRE(n_tensors >= 1 && n_tensors <= 3, LLSA_ERR_ARG, "pool_pyramid: n_tensors must be 1..3");
   const int bs = block_size;
@@ -538,14 +544,19 @@ static int pyramid_entry(int n_tensors, const LlsaTensor* x, const LlsaTensor* y
   }
   if (B * H * N * C == 0) return LLSA_OK;
   cudaStream_t st = (cudaStream_t) stream;
-  const int rc = dt == LLSA_F32 ? launch_pyramid<float>(n_tensors, x, y1, y2, bs, st, freq, rope_mask, xr, norm_mask ? &ns : nullptr)
-                                : launch_pyramid<__nv_bfloat16>(n_tensors, x, y1, y2, bs, st, freq, rope_mask, xr, norm_mask ? &ns : nullptr);
+  const int rc = dt == LLSA_F32 ? launch_pyramid<float>(n_tensors, x, y1, y2, bs, st, freq, rope_mask, xr, norm_mask ? &ns : nullptr, beside)
+                                : launch_pyramid<__nv_bfloat16>(n_tensors, x, y1, y2, bs, st, freq, rope_mask, xr, norm_mask ? &ns : nullptr, beside);
   return rc;
 }
 
 extern "C" int llsa_pool_pyramid_fwd(int n_tensors, const LlsaTensor* x, const LlsaTensor* y1, const LlsaTensor* y2,
                                      int block_size, void* stream) {
   return pyramid_entry(n_tensors, x, y1, y2, block_size, stream, nullptr, 0, nullptr);
+}
+
+extern "C" int llsa_pool_pyramid_beside_fwd(int n_tensors, const LlsaTensor* x, const LlsaTensor* y1, const LlsaTensor* y2, int block_size,
+                                            void* stream) {
+  return pyramid_entry(n_tensors, x, y1, y2, block_size, stream, nullptr, 0, nullptr, nullptr, 0, 0.f, true);
 }
 
 extern "C" int llsa_rope_pool_pyramid_fwd(int n_tensors, const LlsaTensor* x, const LlsaTensor* freq, int rope_mask, const LlsaTensor* xr,

@@ -85,3 +85,39 @@ def test_forward_mode_is_refused(which):
         x[which] = fw.make_dual(x[which], torch.ones_like(x[which]))
         with pytest.raises(NotImplementedError):
             llsa_b200.llsa_l1_rms_rope(*x.values(), table.to(q.dtype), EPS)
+
+
+# 4,032, 4,096, 24,576 and 25,600 query blocks: on both sides of the lines between which the values are pooled beside the selection
+@pytest.mark.parametrize("B,H,N", [(2, 6, 5376), (1, 8, 8192), (3, 8, 16384), (5, 5, 16384)])
+def test_values_pooled_beside_the_selection(B, H, N):
+    """Pooled values and output of the layer are those of its parts called one by one, bit for bit, on new values at every call and in a graph."""
+    gen = torch.Generator(device=DEV).manual_seed(N + B)
+    q, k, v = [torch.randn(B, H, N, 64, device=DEV, generator=gen).bfloat16() for _ in range(3)]
+
+    def parts():
+        (pq, pk, pv), (pq2, pk2, pv2) = ops.pool_pyramid([q, k, v], 16, 2)
+        idx, _ = ops._select_two_level(pq, pk, pq2, pk2, 8, 8, 16)
+        return idx, pv, pv2
+
+    for _ in range(3):
+        got, (idx, pv, pv2) = llsa_b200.llsa_l2_debug(q, k, v), parts()
+        assert torch.equal(got["indices"], idx.to(got["indices"].dtype)) and torch.equal(got["pv"], pv) and torch.equal(got["pv2"], pv2)
+        v.normal_(generator=gen)
+    want = llsa_b200.llsa_l2(q, k, v)
+    x = [t.detach().clone() for t in (q, k, v)]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side), torch.no_grad():
+        llsa_b200.llsa_l2(*x)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            o = llsa_b200.llsa_l2(*x)
+    for t in x:
+        t.zero_()
+    graph.replay()
+    for t, s in zip(x, (q, k, v)):
+        t.copy_(s)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(o, want)
