@@ -509,12 +509,12 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 //     window into the second one warp takes both.  All SMs work on neighbouring entries at any time, so that the tiles stay in L2.  Spans (smaller
 //     problems, whose tensors L2 holds anyway): the entries of all heads, one head behind the other, are cut into equal spans, one per warp, wherever
 //     the cut falls: every warp begins once, and all end together.  As CTAs of four warps, each with a range of 16 entries and its own start, two CTAs
-//     an SM, these problems took 63 us instead of 48 (one level, B=4 H=6 N=4096), 55 / 44 (two levels, B=3 H=5 N=5376), 78 / 60 (one level, B=2 H=4
-//     N=16384).
+//     an SM, these problems took 63 us instead of 48 (45 now; one level, B=4 H=6 N=4096), 55 / 44 (two levels, B=3 H=5 N=5376), 78 / 60 (one level, B=2
+//     H=4 N=16384).
 //     Pieces of buckets that straddle windows or spans go to the `partial` scratch and attn_dkv_finish_kernel adds them in order.
 // What bounds it: latency.  0.42 instructions per scheduler and cycle: 58 % of the issue slots stay empty with three warps on a scheduler, each on
 // one serial chain (wait, S and dP, exponentials, the two products: some 290 instructions per entry); then the raggedness of the last ranges.
-// 168 registers in the persistent form, 4 bytes of them spilled.  With P and dS handed over by the dQ stage instead of recomputed this kernel issued half as much,
+// 168 registers, nothing spilled.  With P and dS handed over by the dQ stage instead of recomputed this kernel issued half as much,
 // but 1 KB per entry went out to HBM and came back: at 8 x 6 slices of 16384 tokens, top 8, dQ stage 205 -> 158 us and this one 192 -> 255
 // on random inputs, 207 -> 164 and 284 -> 255 on correlated ones; at 6 of 262144 421 -> 315 and 563 -> 460 (the first figures of the
 // correlated pairs with eight warps per SM in groups of four that waited for the longest of their ranges: 322 and 645 on random inputs).
@@ -792,8 +792,6 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
         rowfrag_sa<KV + TB + 1024>(vhi, sa_f, sa_f ^ 16);
         tile_zero(dk, dv);
       }
-      // the stage read an entry ago is free: its operands were consumed by products already issued
-      request(i + kRingFineStages - 1);
       // S^T = K.Q^T and dP^T = V.dO^T: rows = keys g, g + 8, columns = queries 2t, 2t + 1 (s0, e0) and 8 more (s1, e1)
       float s0[4], s1[4], e0[4], e1[4];
       const uint32_t f0 = sa_f + so, f1 = f0 ^ 16, m0 = sa_m + so;
@@ -801,6 +799,11 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
       half_rows_x_keys<kRingTileBytes, true>(e0, e1, vlo, vhi, f0);
       half_rows_x_keys<0, false>(s0, s1, klo, khi, f1);
       half_rows_x_keys<kRingTileBytes, false>(e0, e1, vlo, vhi, f1);
+      // The stage read an entry ago is free: its operands were consumed by products already issued.  A request keeps its warp some 270 cycles, which
+      // pass beside the products above; spans, whose tiles come from L2, can wait until the exponentials are on their way too.  us, in front of the products
+      // / here / behind the exponentials: spans at one level, B=4 H=6 N=4096 47.9 / 47.4 / 45.4; windows at two levels, B=1 H=5 N=40960, top-16
+      // 132.8 / 130.5 / 132.0, B=8 H=6 N=16384 245.3 / 244.0 / 245.5.
+      if constexpr (!SPANS) request(i + kRingFineStages - 1);
       const uint32_t sa_s = stat_sa + st * kRingStatBytes + 8 * t;
       auto half = [&](const float2 l, const float2 d, const float (&s)[4], const float (&p)[4], uint32_t& P0, uint32_t& P1, uint32_t& D0, uint32_t& D1) {
         const F2 nl = f2_mul(f2(l.x, l.y), f2(-kLog2e, -kLog2e)), nd = f2(-d.x, -d.y), sc = f2(sl2, sl2);
@@ -818,6 +821,7 @@ attn_dkv_fine_ring_kernel(AttnP<bf16> a, const __grid_constant__ FineMaps maps, 
       uint4 P, D;                                     // P^T and dS^T / scale as A operands
       half(lds64f<0>(sa_s), lds64f<64>(sa_s), s0, e0, P.x, P.y, D.x, D.y);
       half(lds64f<32>(sa_s), lds64f<96>(sa_s), s1, e1, P.z, P.w, D.z, D.w);
+      if constexpr (SPANS) request(i + kRingFineStages - 1);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t bd[4];
