@@ -227,8 +227,8 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_mma_kernel(AttnP<bf16> a, 
 
 // Fine blocks only (the pooled keys are on the tcgen05 kernels): one warp per query block; the selected K / V blocks go through a per-warp
 // ring in shared memory, filled by TMA two blocks ahead, and K is read a second time, transposed, by ldmatrix.  Bound by the gather from
-// L2: 4 KB per (query block, selected block), 9.9 TB/s at 8 x 6 slices of 16384 tokens (158 us; 205 with P and dS, 1 KB per pair, written
-// out for the dK/dV stage).
+// L2: 4 KB per (query block, selected block), 9.6 TB/s at 8 x 6 slices of 16384 tokens (167 us with the lists transposed beside it, 158 without; 205
+// with P and dS, 1 KB per pair, written out for the dK/dV stage).
 constexpr int kDqStages = 3;
 struct KvMaps {
   CUtensorMap k, v;            // [B,H,N,64] 4-D, box 16 rows
@@ -299,11 +299,14 @@ __global__ void __launch_bounds__(NW * 32, 4) attn_dq_fine_kernel(AttnP<bf16> a,
   bool ok = true;
   for (int gi = 0; gi < n_glob; ++gi) {
     if (!(ok = tc::warp_wait(&s_full[warp][st], ph, ctl))) break;
-    if (gi + kDqStages - 1 < n_glob) request(gi + kDqStages - 1);      // into the stage read last time: its operands were consumed by products already issued
     const uint32_t so = st * kStageBytes, f0 = sa_f + so, f1 = f0 ^ 16, m0 = sa_m + so;
     float s0[4], s1[4], p0[4], p1[4];
     half_rows_x_keys<0, true>(s0, s1, qlo, qhi, f0);
     half_rows_x_keys<kRingTileBytes, true>(p0, p1, dlo, dhi, f0);
+    // Into the stage read last time: its operands were consumed by products already issued.  The time a request keeps its warp passes beside the
+    // first half of the score products: B=8 H=6 N=16384 171.8 us in front of them, 167.5 here, 187 behind all of them; B=4 H=6 N=4096 24.4 / 23.6 /
+    // 25.2; B=1 H=5 N=40960, top-16 90.5 / 88.5 / 87.6.
+    if (gi + kDqStages - 1 < n_glob) request(gi + kDqStages - 1);
     half_rows_x_keys<0, false>(s0, s1, qlo, qhi, f1);
     half_rows_x_keys<kRingTileBytes, false>(p0, p1, dlo, dhi, f1);
     // P = exp2(s * scale * log2(e) - lse), dS / scale = P * (dP - delta)
