@@ -167,9 +167,9 @@ int llsa_transpose_indices(const LlsaTensor* idx, const LlsaTensor* offsets, con
  * indices_transpose.py:70-78); `scratch` is not used:
  *   pairs  [B,H,M*T] (I32): in the order of `flat`, the position m*T + t of each entry inside its head's idx
  *          (flat = pairs / T); llsa_attn_bwd has no use for it;
- *   ranges [B,H,ceil(M*T/S),2] (I32), S = llsa_transpose_range_entries(B,H,M,T) (32, or 16 for problems too small to fill
- *          the GPU with 32; the tensor's length tells the library which): the entry list cut into the work ranges of
- *          the dK/dV kernel, (first entry, bucket of that entry) per range.  Range r nominally starts at entry S r;
+ *   ranges [B,H,ceil(M*T/S),2] (I32), S = llsa_transpose_range_entries(B,H,M,T) (32, or 16 for smaller problems; the
+ *          tensor's length tells the library which form of the dK/dV kernel to run): the entry list cut into ranges,
+ *          (first entry, bucket of that entry) per range: work for a warp (32), or where to look up a place in the list (16).  Range r nominally starts at entry S r;
  *          where that entry lies inside a bucket of at most S entries the range starts at the bucket's first entry
  *          instead, so that only longer buckets are ever split (at multiples of S).  Range r ends where r+1 starts. */
 int llsa_transpose_range_entries(int64_t B, int64_t H, int64_t M, int64_t T);
@@ -244,7 +244,7 @@ typedef struct LlsaAttnArgs {
                                   on another stream while 1 and 2 run) */
   const LlsaTensor* dkv_partial; /* backward, bf16 tensors only: F32 scratch
                                   of llsa_attn_bwd_partial_elems() elements for dK/dV tiles of KV
-                                  blocks whose list of query blocks is split over several CTAs (not
+                                  blocks whose list of query blocks is split over several warps (not
                                   read before it is written; may be NULL for f32 tensors) */
   const LlsaTensor* fine_pds;  /* not used any more (the dK/dV stage recomputes P and dS); may be NULL */
   const LlsaTensor* flat_pairs;/* not used any more; NULL, or the `pairs` list of llsa_transpose_indices_pairs */

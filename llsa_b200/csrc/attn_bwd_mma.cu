@@ -19,8 +19,9 @@
 //   attn_dq_fine_kernel    the same for the fine blocks alone (the pooled keys then run on
 //                          tcgen05)
 //   attn_dkv_fine_ring_kernel  the CSR of a head is cut into ranges of equal length (32
-//                          entries, buckets of up to that many kept whole), one warp each,
-//                          however skewed the fan-in is; an entry is S^T, dP^T, then
+//                          entries, buckets of up to that many kept whole), or the lists
+//                          of all heads into one span per warp, however skewed the fan-in
+//                          is; an entry is S^T, dP^T, then
 //                          dV += P^T.dO, dK += dS^T.Q; pieces of longer buckets meet in
 //                          a global partial tensor (no atomics), and
 //   attn_dkv_finish_kernel sums the pieces; every store folds in the pooling
@@ -917,6 +918,10 @@ __device__ __forceinline__ void dkv_store_unselected(const AttnP<bf16>& a, int64
 // waited for the kernels in front of them) and take the SMs that its ragged end leaves idle; what adds pieces waits.  Whole layer, launched behind / into
 // the end: one level, B=4 H=6 N=4096 189.2 / 186.5 us, B=2 H=4 N=16384 334 / 329; two levels, B=3 H=5 N=5376 164.9 / 160.1, H=5 N=40960 top-16
 // 548 / 542, B=4 H=6 N=16384 641 / 634.
+// What it still takes behind the end (24 us at 48 slices of 16384 tokens, 55 % of whose blocks are unselected, 90 at 6 of 262144, 87 %) is the memory's time
+// for 4 KB a block.  No gain from: the unselected blocks written by warps of the kernel above that have run out of ranges (that kernel grows by what this one
+// loses: 506 and 516 us for both at 262144); one wave of CTAs that go from boundary to boundary with the next lookups under way (50 instead of 42 us at B=1 H=5
+// N=40960 top-16); eight to thirty-two blocks a warp.
 __global__ void __launch_bounds__(128) attn_dkv_finish_kernel(AttnP<bf16> a, const float* __restrict__ partial, unsigned n_plain, unsigned BH, int n_spans) {
   if (blockIdx.x < n_plain * BH) {
     const int bh = (int) (blockIdx.x / n_plain), first = ((int) (blockIdx.x % n_plain) * 4 + (int) (threadIdx.x >> 5)) * kPlainPerWarp;

@@ -322,11 +322,10 @@ static int plan_transpose(int64_t n_kv, int64_t E, size_t* smem, bool* global) {
 using namespace llsa;
 
 extern "C" int llsa_transpose_range_entries(int64_t B, int64_t H, int64_t M, int64_t T) {
-  // The size also picks the dK/dV kernel's form (attn_bwd_mma.cu).  The line, two rounds of eight warps per SM, is older than the persistent
-  // form with its twelve.  Whole backward in us, ranges of 16 / of 32 entries: one level, N = 4096: 1,024 ranges (of 32) 98 / 116, 2,048
-  // 167 / 163, 3,072 227 / 220, 4,096 287 / 263, 6,144 408 / 358; two levels, N = 16384: 1,024 102 / 123, 2,048 165 / 165, 4,096 286 / 269;
-  // N = 40960: 1,280 154 / 166, 2,560 247 / 235, 5,120 423 / 398.  The two cross near 2,000 ranges: from there to the line the small form
-  // costs up to 9 %.
+  // The size also picks the dK/dV kernel's form (attn_bwd_mma.cu): spans, one per warp, for ranges of 16, windows for ranges of 32.  Forward + backward
+  // in a graph, us, spans / windows: one level, N = 16384: 2,048 ranges (of 32) 311 / 320, 3,072 464 / 458, 4,096 590 / 604, 4,608 690 / 691, N = 4096:
+  // 4,608 402 / 399; two levels, N = 16384: 3,072 268 / 271, 3,840 322 / 324, 4,608 385 / 382, N = 40960: 3,200 338 / 343, 3,840 397 / 402, N = 65536:
+  // 4,096 403 / 419.  Above, spans fall behind (6,144 ranges 642 / 616, 6,400 547 / 536): warps far apart in the list no longer meet in L2.
   const int64_t ranges = B * H * ((M * T + kRangeEntries - 1) / kRangeEntries);
   return ranges < 2 * 148 * 8 * 2 ? kRangeEntriesSmall : kRangeEntries;
 }
