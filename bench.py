@@ -38,7 +38,8 @@ sys.path.insert(0, ROOT)
 
 METRIC = "llsa_l2 fwd+bwd tokens/sec @N=16384,B*H=48,D=64"
 
-# this library's kernels launched by one llsa_l2 forward + backward (torch's own zero fills are not counted)
+# this library's kernels launched by one llsa_l2 forward + backward at 48 slices (torch's own zero fills are not counted; between 4,096 and 24,576 query
+# blocks, i.e. 4 to 24 slices, the pooling pass is two launches)
 KERNELS_PER_STEP = ("pool_pyramid_bf16_kernel", "refine_topk_kernel", "attn_fwd_fine_kernel", "attn_fwd_pooled_tc_kernel",
                     "transpose_range_kernel", "attn_bwd_pooled_tc_kernel",
                     "attn_dq_fine_kernel", "attn_dkv_fine_ring_kernel", "attn_dkv_finish_kernel")
