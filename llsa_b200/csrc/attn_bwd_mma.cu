@@ -516,7 +516,7 @@ __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) 
 //     an SM, these problems took 63 us instead of 48 (45 now; one level, B=4 H=6 N=4096), 55 / 44 (two levels, B=3 H=5 N=5376), 78 / 60 (one level, B=2
 //     H=4 N=16384).
 //     Pieces of buckets that straddle windows or spans go to the `partial` scratch and attn_dkv_finish_kernel adds them in order.
-// What bounds it: latency.  0.42 instructions per scheduler and cycle: 58 % of the issue slots stay empty with three warps on a scheduler, each on
+// What bounds it: latency.  0.46 instructions per scheduler and cycle: 54 % of the issue slots stay empty with three warps on a scheduler, each on
 // one serial chain (wait, S and dP, exponentials, the two products: some 290 instructions per entry); then the raggedness of the last ranges.
 // 168 registers, nothing spilled.  With P and dS handed over by the dQ stage instead of recomputed this kernel issued half as much,
 // but 1 KB per entry went out to HBM and came back: at 8 x 6 slices of 16384 tokens, top 8, dQ stage 205 -> 158 us and this one 192 -> 255

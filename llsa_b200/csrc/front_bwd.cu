@@ -8,13 +8,16 @@
 // neighbouring tokens of one (b,h) slice, so the slice is found once per chunk and every thread has all its loads (row of dy, of x,
 // of the table) in flight before it uses one.  The weight gradient is kept in registers over all chunks of a CTA, reduced through
 // shared memory, and leaves as one [C] row per CTA; a one-CTA-per-tensor kernel adds the rows in order (bit-reproducible).
-// B=4 H=6 N=16384, [B,N,H,D] storage, both tensors: 302 MB in 65 us = 4.6 TB/s; the rotation's two launches and the eager fp32 formula it
-// replaces took 2050 us.
+// B=4 H=6 N=16384, [B,N,H,D] storage, both tensors: 302 MB in 63 us = 4.8 TB/s; the rotation's two launches and the eager fp32 formula it
+// replaces took 2050 us.  Instructions come next after the memory (0.6 a scheduler and cycle): channels are taken in pairs (66 us one by one); the next
+// chunk's rows in flight early, in registers at three CTAs per SM or by cp.async at four, cost more instructions than they hide time (79 and 77 us), and five
+// CTAs per SM spill or leave the loads too few registers (65.5).
 #include <string.h>
 
 #include <type_traits>
 
 #include "common.cuh"
+#include "mma_frag.cuh"
 
 namespace llsa {
 
@@ -96,11 +99,11 @@ __global__ void __launch_bounds__(kFbThreads, NORM ? 4 : 1) front_bwd_kernel(Fro
   const int ti = blockIdx.y, r0 = threadIdx.x / LANES, c = (threadIdx.x % LANES) * VEC;
   const bool norm = NORM && ((a.norm_mask >> ti) & 1);
   const TF* freq = reinterpret_cast<const TF*>(a.freq);
-  float w[VEC], dw[VEC];
+  F2 w[VEC / 2], dw2[VEC / 2];          // channels in pairs: one instruction for two
 #pragma unroll
-  for (int i = 0; i < VEC; ++i) {
-    w[i] = norm && a.w[ti] ? a.w[ti][c + i] : 1.f;
-    dw[i] = 0.f;
+  for (int i = 0; i < VEC / 2; ++i) {
+    w[i] = norm && a.w[ti] ? f2(a.w[ti][c + 2 * i], a.w[ti][c + 2 * i + 1]) : f2(1.f, 1.f);
+    dw2[i] = f2(0.f, 0.f);
   }
   for (int ch = blockIdx.x; ch < a.n_chunks; ch += gridDim.x) {
     const int bh = ch / a.chunks_per_head, s0 = (ch - bh * a.chunks_per_head) * (STEP * ROWS) + r0;
@@ -124,21 +127,32 @@ __global__ void __launch_bounds__(kFbThreads, NORM ? 4 : 1) front_bwd_kernel(Fro
           float gv[VEC], xv[VEC];
           unpack16<T>(g[u], gv);
           unpack16<T>(x[u], xv);
-          float ss = 0.f, dot = 0.f;
+          F2 gw[VEC / 2], ss2 = f2(0.f, 0.f), dot2 = ss2;
 #pragma unroll
-          for (int i = 0; i < VEC; ++i) { ss = fmaf(xv[i], xv[i], ss); dot = fmaf(gv[i] * w[i], xv[i], dot); }
+          for (int i = 0; i < VEC / 2; ++i) {
+            const F2 xi = f2(xv[2 * i], xv[2 * i + 1]);
+            gw[i] = f2_mul(f2(gv[2 * i], gv[2 * i + 1]), w[i]);
+            ss2 = f2_fma(xi, xi, ss2);
+            dot2 = f2_fma(gw[i], xi, dot2);
+          }
+          float ss, dot, ss1, dot1;
+          f2_get(ss2, ss, ss1);
+          f2_get(dot2, dot, dot1);
+          ss += ss1;
+          dot += dot1;
 #pragma unroll
           for (int o = 1; o < LANES; o <<= 1) {
             ss += __shfl_xor_sync(0xffffffffu, ss, o);
             dot += __shfl_xor_sync(0xffffffffu, dot, o);
           }
           const float rstd = rsqrtf(ss / (float) kFbC + a.eps), k = dot * rstd / (float) kFbC;      // k = mean(g w xh)
-          const float live = s < a.S ? 1.f : 0.f;
+          const float live = s < a.S ? rstd : 0.f, back = -(rstd * k) * rstd;
+          const F2 r2 = f2(rstd, rstd), l2 = f2(live, live), b2 = f2(back, back);
 #pragma unroll
-          for (int i = 0; i < VEC; ++i) {
-            const float xh = xv[i] * rstd;
-            dw[i] = fmaf(gv[i] * live, xh, dw[i]);
-            gv[i] = rstd * (gv[i] * w[i] - xh * k);
+          for (int i = 0; i < VEC / 2; ++i) {
+            const F2 xi = f2(xv[2 * i], xv[2 * i + 1]);
+            dw2[i] = f2_fma(f2(gv[2 * i], gv[2 * i + 1]), f2_mul(xi, l2), dw2[i]);
+            f2_get(f2_fma(xi, b2, f2_mul(gw[i], r2)), gv[2 * i], gv[2 * i + 1]);
           }
           g[u] = pack16<T>(gv);
         }
@@ -149,6 +163,9 @@ __global__ void __launch_bounds__(kFbThreads, NORM ? 4 : 1) front_bwd_kernel(Fro
   if (NORM && a.dw_partial) {
     __shared__ float sw[kFbThreads / 32][kFbC];
     const int warp = threadIdx.x >> 5;
+    float dw[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC / 2; ++i) f2_get(dw2[i], dw[2 * i], dw[2 * i + 1]);
 #pragma unroll
     for (int i = 0; i < VEC; ++i)
 #pragma unroll
