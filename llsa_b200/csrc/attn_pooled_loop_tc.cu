@@ -139,7 +139,7 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  pdl_trigger();
+  // no pdl_trigger: what follows, often the pooling pass of the next layer, would take the SMs that this kernel's CTAs leave first and run unevenly
   const uint32_t tmem = s_tmem;
   // One round over the CTA's tiles, and another for marked rows.  body(round's barriers, passes, jobs per tile): job j of tile i has the CTA-wide
   // number i * jobs + j, which picks the S buffer and the softmax group (mod 3).  Every role calls this with its own body; the roles meet at

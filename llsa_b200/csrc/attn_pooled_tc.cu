@@ -91,7 +91,7 @@ attn_fwd_pooled_tc_kernel(AttnP<bf16> a, const __grid_constant__ TcMaps maps, in
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  pdl_trigger();
+  // no pdl_trigger: what follows, often the pooling pass of the next layer, would take the SMs that this kernel's CTAs leave first and run unevenly
   const uint32_t tmem = s_tmem;
   const int n_my = (n_tiles - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x;
 

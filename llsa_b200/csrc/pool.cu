@@ -107,6 +107,7 @@ template <typename T, int LEVELS, bool ROPE = false, bool NORM = false>
 __global__ void pool_pyramid_kernel(PyramidArgs<T> a, int rows_per_cta, int64_t ctas_per_head) {
   constexpr int VEC = Vec16<T>::N;
   extern __shared__ float smem[];  // LEVELS==2: [rows][C] level-1 results as fp32 images of T
+  pdl_wait();
   const int ti = blockIdx.y;
   const int64_t bh = blockIdx.x / ctas_per_head;
   const int64_t grp = blockIdx.x % ctas_per_head;
@@ -216,6 +217,7 @@ template <int LEVELS, bool ROPE, bool NORM>
 __global__ void __launch_bounds__(128) pool_pyramid_bf16_kernel(PyramidArgs<__nv_bfloat16> a, int groups_per_head) {
   constexpr int BS = 16, C = 64;
   __shared__ __align__(16) uint4 s_row[LEVELS == 2 ? BS * 8 : 1];
+  if (!a.beside) pdl_wait();
   const int ti = blockIdx.y, bh = blockIdx.x / groups_per_head, grp = blockIdx.x - bh * groups_per_head;
   const int b = bh / a.H, h = bh - b * a.H, r = threadIdx.x >> 3, c = (threadIdx.x & 7) * 8;
   const int row1 = grp * BS + r;                           // level-1 row inside (b,h)
@@ -406,21 +408,23 @@ struct NormSpec {
   float eps;
 };
 
+// The launch is made ready while the kernel in front of it, the caller's or the end of the layer before, still runs.  Forward + backward in us, launched plainly
+// / so: one level, B=4 H=6 N=4096 178.9 / 176.5, B=2 H=4 N=16384 322.5 / 314.6, two levels, B=3 H=5 N=5376 140.1 / 138.2; forward alone, B=1 H=6 N=16384
+// with norm and rotation 57.4 / 56.0.  (The pooled forward does not let it begin early: its CTAs would settle unevenly on the SMs that become free first, 61.1.)
 template <int LEVELS>
 static void launch_pyramid_bf16(const PyramidArgs<__nv_bfloat16>& a, dim3 grid, int groups, cudaStream_t st) {
-  if (a.rope_mask && a.norm_mask) pool_pyramid_bf16_kernel<LEVELS, true, true><<<grid, 128, 0, st>>>(a, groups);
-  else if (a.rope_mask) pool_pyramid_bf16_kernel<LEVELS, true, false><<<grid, 128, 0, st>>>(a, groups);
-  else if (a.norm_mask) pool_pyramid_bf16_kernel<LEVELS, false, true><<<grid, 128, 0, st>>>(a, groups);
-  else if (a.beside) launch_pdl(pool_pyramid_bf16_kernel<LEVELS, false, false>, grid, 128, 0, st, a, groups);
-  else pool_pyramid_bf16_kernel<LEVELS, false, false><<<grid, 128, 0, st>>>(a, groups);
+  if (a.rope_mask && a.norm_mask) launch_pdl(pool_pyramid_bf16_kernel<LEVELS, true, true>, grid, 128, 0, st, a, groups);
+  else if (a.rope_mask) launch_pdl(pool_pyramid_bf16_kernel<LEVELS, true, false>, grid, 128, 0, st, a, groups);
+  else if (a.norm_mask) launch_pdl(pool_pyramid_bf16_kernel<LEVELS, false, true>, grid, 128, 0, st, a, groups);
+  else launch_pdl(pool_pyramid_bf16_kernel<LEVELS, false, false>, grid, 128, 0, st, a, groups);
 }
 
 template <typename T, int LEVELS>
 static void launch_pyramid_variant(const PyramidArgs<T>& a, dim3 grid, int threads, size_t smem, int rows, int64_t per_head, cudaStream_t st) {
-  if (a.rope_mask && a.norm_mask) pool_pyramid_kernel<T, LEVELS, true, true><<<grid, threads, smem, st>>>(a, rows, per_head);
-  else if (a.rope_mask) pool_pyramid_kernel<T, LEVELS, true, false><<<grid, threads, smem, st>>>(a, rows, per_head);
-  else if (a.norm_mask) pool_pyramid_kernel<T, LEVELS, false, true><<<grid, threads, smem, st>>>(a, rows, per_head);
-  else pool_pyramid_kernel<T, LEVELS, false, false><<<grid, threads, smem, st>>>(a, rows, per_head);
+  if (a.rope_mask && a.norm_mask) launch_pdl(pool_pyramid_kernel<T, LEVELS, true, true>, grid, threads, smem, st, a, rows, per_head);
+  else if (a.rope_mask) launch_pdl(pool_pyramid_kernel<T, LEVELS, true, false>, grid, threads, smem, st, a, rows, per_head);
+  else if (a.norm_mask) launch_pdl(pool_pyramid_kernel<T, LEVELS, false, true>, grid, threads, smem, st, a, rows, per_head);
+  else launch_pdl(pool_pyramid_kernel<T, LEVELS, false, false>, grid, threads, smem, st, a, rows, per_head);
 }
 
 template <typename T>
