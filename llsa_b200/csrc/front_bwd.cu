@@ -147,13 +147,14 @@ __global__ void __launch_bounds__(kFbThreads, NORM ? 4 : 1) front_bwd_kernel(Fro
             dot += __shfl_xor_sync(0xffffffffu, dot, o);
           }
           const float rstd = rsqrtf(ss / (float) kFbC + a.eps), k = dot * rstd / (float) kFbC;      // k = mean(g w xh)
-          const float live = s < a.S ? rstd : 0.f, back = -(rstd * k) * rstd;
-          const F2 r2 = f2(rstd, rstd), l2 = f2(live, live), b2 = f2(back, back);
+          // rstd meets x before it meets k and itself again: without an eps the square of it leaves the range of a float long before dx does
+          const float live = s < a.S ? rstd : 0.f;
+          const F2 l2 = f2(live, live), k2 = f2(-k, -k);
 #pragma unroll
           for (int i = 0; i < VEC / 2; ++i) {
-            const F2 xi = f2(xv[2 * i], xv[2 * i + 1]);
-            dw2[i] = f2_fma(f2(gv[2 * i], gv[2 * i + 1]), f2_mul(xi, l2), dw2[i]);
-            f2_get(f2_fma(xi, b2, f2_mul(gw[i], r2)), gv[2 * i], gv[2 * i + 1]);
+            const F2 xh = f2_mul(f2(xv[2 * i], xv[2 * i + 1]), l2);
+            dw2[i] = f2_fma(f2(gv[2 * i], gv[2 * i + 1]), xh, dw2[i]);
+            f2_get(f2_mul(f2_fma(xh, k2, gw[i]), l2), gv[2 * i], gv[2 * i + 1]);
           }
           g[u] = pack16<T>(gv);
         }

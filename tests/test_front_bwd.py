@@ -13,14 +13,14 @@ DEV = "cuda:0"
 EPS = 1e-5
 
 
-def _reference(dy, x, w, table):
+def _reference(dy, x, w, table, eps=EPS):
     """(dx in fp64, dw in fp64): g is the rotation's backward rounded to the data's type, as the stand-alone kernel leaves it."""
     # evaluated in the wider of the two types, as the kernel does (the oracle itself narrows the table to its tensor's type)
     g = (O.rope_bwd(dy.to(torch.promote_types(dy.dtype, table.dtype)), table).to(dy.dtype) if table is not None else dy).double()
     if w is None:
         return g, None
     xd = x.double()
-    rstd = torch.rsqrt(xd.square().mean(-1, keepdim=True) + EPS)
+    rstd = torch.rsqrt(xd.square().mean(-1, keepdim=True) + eps)
     xh, gw = xd * rstd, g * w.double()
     return rstd * (gw - xh * (gw * xh).mean(-1, keepdim=True)), (g * xh).sum((0, 1, 2))
 
@@ -59,3 +59,24 @@ def test_rms_rope_bwd(S, dtype, table, norm, view):
         assert ((got - dx).abs() <= ulp * dx.abs() + noise).all(), float((got - dx).abs().max())
         if norm:      # a sum of B H S terms in fp32: sqrt(n) 2^-24 per unit of size, with an order of magnitude to spare
             assert float((dw[i].cpu().double() - dwr).norm() / dwr.norm()) < 1e-5
+
+
+# Without an eps: rows whose reciprocal root mean square, squared and times dy, is beyond a float's largest value, or below its smallest, while
+# dx is well inside.  Bounds as above, in units of |rstd g|.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("size_x,size_dy", [(1e-18, 1e4), (1e18, 1e-8)])
+def test_norm_of_very_small_and_very_large_rows_without_eps(size_x, size_dy, dtype):
+    gen = torch.Generator().manual_seed(5)
+    dy, x = [(size * torch.randn(1, 2, 300, 64, generator=gen)).to(dtype) for size in (size_dy, size_x)]
+    w = 1 + 0.2 * torch.randn(64, generator=gen)
+    lib, TP = _lib.lib(), C.POINTER(_lib.LlsaTensor)
+    got, dw, part = dy.to(DEV), torch.empty(64, device=DEV), torch.empty(lib.llsa_rms_rope_bwd_partial_elems(1), device=DEV)
+    xd, wd = x.to(DEV), w.to(DEV)
+    one = lambda t: (TP * 1)(C.pointer(t))
+    dyt, xt, wt, dwt, pt = [_lib.desc(t) for t in (got, xd, wd, dw, part)]
+    _lib.check(lib.llsa_rms_rope_bwd(1, _lib.ref(dyt), _lib.ref(xt), one(wt), 1, 0.0, None, _lib.ref(dyt), _lib.ref(pt), one(dwt),
+                                     _lib.stream_ptr(torch.device(DEV))), "rms_rope_bwd")
+    dx, dwr = _reference(dy, x, w, None, 0.0)
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
+    assert ((got.cpu().double() - dx).abs() <= ulp * dx.abs() + 2e-5 * size_dy / size_x).all()
+    assert float((dw.cpu().double() - dwr).norm() / dwr.norm()) < 1e-5
