@@ -382,10 +382,11 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
     });
   } else {
     tc::regs_set<Split<GROUPS>::kEpilogue, Split<GROUPS>::kLaunch>();
-    rounds([&](LoopBars& bars, int n_pass, int) {
+    rounds([&](LoopBars& bars, int n_pass, int jobs) {
       // ---------------------------------------------------------------- epilogue, thread = query row
       const int qd = warp & 3, r = qd * 32 + lane;
       bool ok = true;
+      int g0 = 0;                            // the group that takes the tile's first job
       for (int i = 0; i < n_my; ++i) {
         const int tile = blockIdx.x + i * gridDim.x;
         const int bh = tile / tiles_per_head, row = (tile % tiles_per_head) * kRows + r;
@@ -407,7 +408,14 @@ attn_fwd_pooled_loop_tc_kernel(AttnP<bf16> a, const __grid_constant__ LoopMaps m
         ok = ok && __all_sync(0xffffffffu, tc::bounded_wait(&bars.o_ready[i & 1], (uint32_t) (i >> 1) & 1, abort_flag));
         tc::fence_after_sync();
         if (!ok) break;
-        const float two = s_sum[i & 1][0][r] + s_sum[i & 1][1][r], lsum = GROUPS == 3 ? two + s_sum[i & 1][GROUPS - 1][r] : two, mx = s_ref[i & 1][r];
+        // Three sums in the order of the tile's jobs, not of the groups: a row's bits do not depend on where in the CTA's list its tile stands
+        float lsum = s_sum[i & 1][0][r] + s_sum[i & 1][1][r];
+        if constexpr (GROUPS == 3) {
+          const int g1 = g0 == 2 ? 0 : g0 + 1, g2 = g1 == 2 ? 0 : g1 + 1;
+          lsum = s_sum[i & 1][g0][r] + s_sum[i & 1][g1][r] + s_sum[i & 1][g2][r];
+          g0 = (g0 + jobs) % 3;
+        }
+        const float mx = s_ref[i & 1][r];
         // one pass: the row is this round's unless its sum left the safe range (false for NaN too): the mark hands it to the second
         if (redo && n_pass == 1) {
           mine = lsum < 1e30f;

@@ -806,6 +806,24 @@ def test_batch_of_288_slices_matches_its_own_slices():
         assert rel_l2(K.grad[sl], ks.grad) < 2e-3 and rel_l2(V.grad[sl], vs.grad) < 2e-3
 
 
+@pytest.mark.parametrize("B,H,N", [(16, 4, 8192), (8, 4, 16384), (2, 4, 65536)])
+def test_llsa_l1_of_long_lists_does_not_depend_on_the_batch(B, H, N):
+    """Lists of 512, 1024 and 4096 pooled keys, where a slice's rows stand at other places of their CTAs' lists when it is alone: its o and dq are
+    the same, bit for bit."""
+    L = _ops()
+    gen = torch.Generator(device=DEV).manual_seed(N)
+    Q, K, V, DO = [torch.randn(B, H, N, 64, device=DEV, generator=gen).bfloat16() for _ in range(4)]
+    Q, K, V = [t.requires_grad_(True) for t in (Q, K, V)]
+    o = L.llsa_l1(Q, K, V, 8, 16)
+    o.backward(DO)
+    for b in range(B):
+        qs, ks, vs = [t[b:b + 1].detach().clone().requires_grad_(True) for t in (Q, K, V)]
+        os_ = L.llsa_l1(qs, ks, vs, 8, 16)
+        os_.backward(DO[b:b + 1])
+        assert torch.equal(o[b:b + 1], os_) and torch.equal(Q.grad[b:b + 1], qs.grad), b
+        assert rel_l2(K.grad[b:b + 1], ks.grad) < 2e-3 and rel_l2(V.grad[b:b + 1], vs.grad) < 2e-3
+
+
 def test_llsa_l1_288_slices_whole_and_partial_key_units():
     """llsa_l1, 288 (b,h) slices of 4096 tokens: the key-major pooled dK/dV kernel cuts its flat (head, chunk, job) list
     into one piece per SM, and with 576 (head, chunk) pairs a piece holds whole units (plain stores) between two partial

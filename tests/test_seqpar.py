@@ -88,12 +88,12 @@ def test_two_gloo_ranks_sequence_sharded_matches_unsharded_oracle(tmp_path, leve
 
 
 # ------------------------------------------------------------------ GPU
-def _rank_by_rank(levels, world, dtype):
+def _rank_by_rank(levels, world, dtype, H=2, N=None):
     """Every rank's local forward + backward on ONE device, in turn; the exchange is a plain sum."""
     import llsa_b200 as L
     dev = "cuda:0"
-    N = 16384 if levels == 2 else 4096
-    q, k, v, do = [t.to(dev) for t in synth.correlated_qkv(11, 1, 2, N, 64, dtype=dtype)]
+    N = N or (16384 if levels == 2 else 4096)
+    q, k, v, do = [t.to(dev) for t in synth.correlated_qkv(11, 1, H, N, 64, dtype=dtype)]
     be = seqpar.CudaBackend()
     pyr = be.pool_pyramid([q, k, v], 16, levels)
     pk, pv = pyr[0][1], pyr[0][2]
@@ -124,6 +124,16 @@ def test_rectangular_kernels_rank_by_rank_match_unsharded(levels, world, dtype):
     assert torch.equal(dq, dq_ref)
     tol = 4e-3 if dtype == torch.bfloat16 else 1e-5      # W partials, each rounded to the dtype, against one rounding
     assert rel_l2(dk, dk_ref) < tol and rel_l2(dv, dv_ref) < tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,N,world", [(8, 16384, 2), (4, 65536, 2), (8, 65536, 4)])
+def test_one_level_ranks_of_long_lists_match_unsharded(H, N, world):
+    """Lists of 1024 and 4096 pooled keys: the same blocks, o and dq, whichever rows a rank has (and so whichever kernels, tiles and CTAs they meet)."""
+    from helpers import rel_l2
+    o, dq, dk, dv, o_ref, dq_ref, dk_ref, dv_ref = _rank_by_rank(1, world, torch.bfloat16, H, N)
+    assert torch.equal(o, o_ref) and torch.equal(dq, dq_ref)
+    assert rel_l2(dk, dk_ref) < 4e-3 and rel_l2(dv, dv_ref) < 4e-3      # as above
 
 
 def _nccl_worker(rank, world, port, out):
