@@ -50,19 +50,27 @@ void set_error(const char* fmt, ...);
 // front still runs finds the SM divided for that kernel's shared memory, and with 28 KB of L1 to land its loads in it streams at two thirds
 // of its rate (B=4 H=6 N=16384 with norm and rotation, whole layer: 709 us with the three launched plainly, 757 with all chained, 720 with
 // none; l1_rope B=4 H=6 N=4096 243, 243 and 259).
+// cluster: neighbouring CTAs along x that form a cluster (the grid's x is a multiple of it).
 template <typename... P, typename... A>
-inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline void launch_pdl_cluster(void (*kernel)(P...), dim3 grid, dim3 block, unsigned cluster, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);      // LLSA_LAUNCH_OK picks the error up
+}
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  launch_pdl_cluster(kernel, grid, block, 1, smem, st, std::forward<A>(args)...);
 }
 
 // Raises (never lowers) a kernel's dynamic shared-memory limit on the current device; thread-safe.  launch_regs: the registers per thread that

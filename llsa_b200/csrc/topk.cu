@@ -157,7 +157,7 @@ coarse_topk_kernel(const T* __restrict__ pq, const T* __restrict__ pk, void* __r
 // Large problems are bound by the latency of a warp's product and comparison chains (four warps per scheduler, tensor pipe 41 % busy);
 // keys through a cp.async ring or 24 warps per SM of one row tile each changed nothing.  n = M = 4096, 8 slices: 243 us with one pass
 // and lists of (value, column) pairs in four-warp CTAs of 64 rows, 139 now; n = M = 1024, 8 slices: 59 -> 20; n = M = 256, 24
-// slices: 24 -> 6.7; n = M = 64, 6 slices: 14.9 -> 3.7.  Long lists of many rows are topk_tc.cu's.
+// slices: 24 -> 6.7; n = M = 64, 6 slices: 14.9 -> 3.7.  Long lists are topk_tc.cu's.
 constexpr int kCmWarps = 8, kCmBoundFrom = 1024;
 
 // ROWT row tiles per warp, KW warps share a CTA's keys, the other kCmWarps / KW are further row tiles.
@@ -750,10 +750,13 @@ int launch_coarse_topk_tc(const LlsaTensor* pq, const LlsaTensor* pk, const Llsa
 
 using namespace llsa;
 
-// The tcgen05 kernel walks a list twice with one CTA per 128 rows; it takes lists of at least kCoarseTcFrom keys where that fills the SMs.  us, here / there:
-// 8 slices of n = M = 4096 (256 tiles) smooth 131 / 69, random 139 / 74; 3968, top-4 116 / 71; 2048 (128 tiles) 43.6 / 41.6 and 45.8 / 39; 144 slices of 1024
-// (1,152 tiles) 213 / 121 and 254 / 105; fewer tiles: 2 slices of 4096 (64) 46 / 48, 6 of 1024 (48) 12 / 23, 24 of 512 (96) 16.3 / 16.0, 6 of 512 (24) 7.4 / 16.7.
-constexpr int64_t kCoarseTcFrom = 512, kCoarseTcTiles = 128;
+// The tcgen05 kernel (topk_tc.cu) sums a score in another order, so the length of the list alone may choose between the two: a row's blocks must not depend
+// on the batch or on how many of the sequence's rows a call holds.  The line lies where that kernel, its keys shared by a cluster where there are few rows,
+// is at least about equal for any number of square slices (n = M).  us in a graph, smooth inputs, here / there: n = 4096: 1 slice 27.3 / 24.4, 2 45.7 / 34.9,
+// 4 70 / 48, 8 131 / 69, 128 rows 20.0 / 18.6, but 3 slices of 2048 rows 28.3 / 36.4; 3584: 1 24.2 / 25.6, 2 38.0 / 35.9, 3 42.4 / 44.2; 3072: 1 20.9 / 24.6,
+// 2 22.2 / 28.3, 6 58 / 49; 2048: 1 15.3 / 18.3, 2 (n = 2112) 17.5 / 23.6, 8 42.1 / 36.0; 1024: 1 8.8 / 18, 6 11.8 / 20.3, 24 50.6 / 34.7, 144 211 / 119;
+// 512: 6 7.5 / 17, 48 33.9 / 23.6.
+constexpr int64_t kCoarseTcFrom = 3584;
 
 // The tensor-core kernel's range: its accumulation order differs from the scalar kernels' in the last bit of a score, so the line
 // between the two decides which bits a caller gets and stays where it was (whole 64-key tiles, top-k <= 8).
@@ -786,7 +789,7 @@ extern "C" int llsa_coarse_topk_bounded(const LlsaTensor* pq, const LlsaTensor* 
   const int idx64 = idx->dtype == LLSA_I64;
   const bool bf = pq->dtype == LLSA_BF16;
   auto blocks = [&](int rows) { return dim3((unsigned) ((M + rows - 1) / rows), BH); };
-  if (coarse_on_mma(pq, pk, topk) && n >= kCoarseTcFrom && B * H * ((M + 127) / 128) >= kCoarseTcTiles) return launch_coarse_topk_tc(pq, pk, idx, topk, wait_limit, st);
+  if (coarse_on_mma(pq, pk, topk) && n >= kCoarseTcFrom) return launch_coarse_topk_tc(pq, pk, idx, topk, wait_limit, st);
   if (coarse_on_mma(pq, pk, topk)) {
     const bf16 *q = (const bf16*) pq->ptr, *k = (const bf16*) pk->ptr;
     // 64 rows per CTA (each key read from L2 once per 64 rows) where that still gives every SM two CTAs, else 16 rows, the keys

@@ -7,13 +7,18 @@
 //     memory as they are; they become candidates (topk_words.cuh) and go into the thread's sorted list when a warp's rows have several of them.  (Taken
 //     at once, with the warp's other rows waiting, one such group cost some 500 cycles: 65 and 87 us at n = M = 4096, 8 slices, smooth and random.)
 // Two warpgroups take alternate jobs (odd and even), each with two score buffers of its own, half a job each, so that the products of one half run while
-// the other is looked at; they share a row's bound and merge its two lists through shared memory.  Roles: warps 0-3 / 4-7 the two groups, warp 8 TMA producer (queries once, a ring of two key chunks), warp 9 issues the products.
+// the other is looked at; they share a row's bound and merge its two lists through shared memory.  Roles: warps 0-3 / 4-7 the two groups, warp 8 TMA
+// producer (queries once, a ring of two key chunks), warp 9 issues the products.
+// Where there are few rows (up to 128 tiles) a cluster of two, four or eight CTAs shares a tile, each with its part of the keys.  They share their bounds
+// after pass 1 and merge their lists at the end.  A score does not depend on who computes it and the candidates of a row are distinct words, so the result is the
+// same for any split.  At most 256 CTAs, 32 clusters of eight: 33 and more do not run at once (n = M = 4096, 32 tiles 51 / 40 / 31 / 24 us with one, two, four and
+// eight CTAs a tile, 48 tiles 56 / 47 / 36 / 44, 64 tiles 56 / 39 / 35 / 48, 96 tiles 60 / 45 / 59 / 70, 160 tiles 65 / 69).
 // What bounds it: instructions of pass 2 where some row of a warp has something to set aside (nearly half of the groups of eight), two thirds of all; the
 // comparisons are 64 maxima a thread and job in either pass, the tensor pipe takes 384 cycles a job.  Two CTAs share an SM, so that one's hand-overs are hidden
-// by the other's work.  n = M = 4096, 8 slices: 69 us smooth, 74 random, 131 and 139 with mma.sync (topk.cu); whole layer, l1, B=2 H=4 N=65536 923 -> 856.
-// Same scores as there, bit for bit, in all but some 2 of 100,000 rows.
-// Every mbarrier wait is bounded.  A CTA whose wait expires computes its rows with scalar arithmetic instead (slowly, and with another order of the
-// sums): a selection that went missing would not show in anything downstream.
+// by the other's work.  n = M = 4096, 8 slices: 69 us smooth, 72 random, 131 and 138 with mma.sync (topk.cu); whole layer, l1, B=2 H=4 N=65536 923 -> 856.
+// The same blocks as there in all but some 2 of 100,000 rows: the sums are taken in another order.
+// Every mbarrier wait is bounded.  A CTA whose wait expires computes its rows against its keys with scalar arithmetic instead (slowly, and with
+// another order of the sums): a selection that went missing would not show in anything downstream.  Every CTA of a cluster comes to its meetings either way.
 #include <string.h>
 
 #include "mma_frag.cuh"
@@ -56,14 +61,46 @@ __device__ __forceinline__ void store_list(void* idx_out, int idx64, int64_t at,
     }
 }
 
-// n: a multiple of 64, at most 65536, at least kGroups * 32
+// ---- clusters: the CTAs that share a tile of rows, each with a part of the keys
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t ld_cluster(const void* smem, uint32_t rank) {      // the word at this place of CTA `rank`'s shared memory
+  uint32_t at, d;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(tc::smem_u32(smem)), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(d) : "r"(at) : "memory");
+  return d;
+}
+
+// The larger half of two descending lists, descending: the larger of the ends that meet, which is a bitonic sequence
+template <typename F>
+__device__ __forceinline__ void list_merge(uint32_t (&list)[kCmTop], F&& other) {      // other(u): word u of the second list
+  uint32_t o[kCmTop];
+#pragma unroll
+  for (int u = 0; u < kCmTop; ++u) o[u] = other(u);
+#pragma unroll
+  for (int u = 0; u < kCmTop; ++u) list[u] = umax(list[u], o[kCmTop - 1 - u]);
+#pragma unroll
+  for (int d = kCmTop / 2; d > 0; d >>= 1)
+#pragma unroll
+    for (int u = 0; u < kCmTop; ++u)
+      if ((u & d) == 0) {
+        const uint32_t x = umax(list[u], list[u + d]), y = umin(list[u], list[u + d]);
+        list[u] = x;
+        list[u + d] = y;
+      }
+}
+
+// n: a multiple of 64, at most 65536.  SHARED: clusters of 1 << log_split CTAs, at most 8 and at most as many as there are chunks, share a tile of rows.
+template <bool SHARED>
 __global__ void __launch_bounds__(kThreads, 2)
 coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __restrict__ pq, const bf16* __restrict__ pk, void* __restrict__ idx_out,
-                      int idx64, int64_t M, int64_t n, int topk, int wait_limit) {
+                      int idx64, int64_t M, int64_t n, int topk, int log_split, int wait_limit) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ CoarseBars bars;
   __shared__ uint32_t s_tmem;
   __shared__ tc::WaitCtl s_ctl;
+  __shared__ float s_bound[SHARED ? kRows : 1];
+  __shared__ int s_part[2];                              // SHARED: this CTA's first key, and how many it has
   bf16* sQ = reinterpret_cast<bf16*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));      // [128][64]
   bf16* sK = sQ + kTile;                                 // [kStages][128][64]
   // Pass 2: [slot][thread] eight scores as bf16, and their group; before and behind it the lists of maxima and of candidates, [group][row], a row's
@@ -74,9 +111,17 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
   static_assert(kSlots * 16 >= (kCmTop + 1) * 4, "room for the lists");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile tc::WaitCtl* abort_flag = &s_ctl;
-  const int64_t bh = blockIdx.y, row0 = (int64_t) blockIdx.x * kRows;
-  const int chunks = (int) ((n + kChunk - 1) / kChunk), jobs = 2 * chunks;
+  if (!SHARED) log_split = 0;
+  const int rank = SHARED ? (int) blockIdx.x & ((1 << log_split) - 1) : 0;
+  const int64_t bh = blockIdx.y, row0 = (int64_t) (blockIdx.x >> log_split) * kRows;
+  const int chunks_all = (int) ((n + kChunk - 1) / kChunk), chunk0 = (chunks_all * rank) >> log_split;
+  const int chunks = ((chunks_all * (rank + 1)) >> log_split) - chunk0, jobs = 2 * chunks;
+  const volatile int* part = s_part;                     // in shared memory: a register less in the loops below
+  auto key0 = [&] { return SHARED ? part[0] : 0; };
+  auto keys = [&] { return SHARED ? part[1] : (int) n; };
   if (tid == 0) {
+    s_part[0] = chunk0 * kChunk;
+    s_part[1] = min((int) n - chunk0 * kChunk, chunks * kChunk);
     s_ctl.abort = 0;
     s_ctl.limit = wait_limit > 0 ? wait_limit : tc::kWaitPolls;
     tc::mbar_init(&bars.q_full, 1);
@@ -92,6 +137,7 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
   pdl_trigger();
   const uint32_t tmem = s_tmem;
 
+  if (SHARED && warp >= 8) cluster_arrive();                 // the bounds of pass 2 need nothing of these
   if (warp == 8) {
     // ---------------------------------------------------------------- TMA producer
     tma::expect_tx_w(&bars.q_full, kTile * 2);
@@ -101,7 +147,7 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
     for (int j = 0; j < jobs; ++j) {
       if (!tc::warp_wait(&bars.k_empty[st], ph, abort_flag)) break;
       tma::expect_tx_w(&bars.k_full[st], kTile * 2);
-      tma::load_2d_w(sK + st * kTile, &maps.k, &bars.k_full[st], 0, (int) (bh * n) + c * kChunk);
+      tma::load_2d_w(sK + st * kTile, &maps.k, &bars.k_full[st], 0, (int) (bh * n) + key0() + c * kChunk);
       if (++st == kStages) { st = 0; ph ^= 1; }
       if (++c == chunks) c = 0;
     }
@@ -152,7 +198,7 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
       __syncwarp();
       if (lane == 0) tma::mbar_arrive(&bars.s_free[wg * 2 + half]);
     };
-    auto halves = [&](int c) { return (int64_t) (c + 1) * kChunk <= n ? 2 : 1; };      // the last chunk may be half a chunk
+    auto halves = [&](int c) { return (c + 1) * kChunk <= keys() ? 2 : 1; };      // the last chunk may be half a chunk
     int j = wg;
     float m[kGroups];
 #pragma unroll
@@ -197,7 +243,16 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
     float eighth = CUDART_INF_F;
 #pragma unroll
     for (int u = 0; u < kCmTop; ++u) eighth = fminf(eighth, fmaxf(best[u], __uint_as_float(s_list[wg ^ 1][r][kCmTop - 1 - u])));
-    group_sync();                                            // both groups have read the maxima
+    if constexpr (SHARED) {                                  // eight scores of this CTA's keys reach that; the largest of the cluster's is the better bound
+      if (wg == 0) s_bound[r] = eighth;
+      __syncwarp();
+      cluster_arrive();                                      // both groups have read the maxima, and the bounds are there
+      cluster_wait();
+#pragma unroll 1
+      for (int o = 1; o < 1 << log_split; ++o) eighth = fmaxf(eighth, __uint_as_float(ld_cluster(&s_bound[r], (uint32_t) (rank ^ o))));
+    } else {
+      group_sync();                                          // both groups have read the maxima
+    }
     uint32_t list[kCmTop], thr, w, none;
     float low;
     candidate_words(eighth, 0.f, 0u, w, none);
@@ -210,7 +265,7 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
       for (int u = 0; __any_sync(0xffffffffu, u < held); ++u) {
         if (u < held) {
           const uint4 x = s_slot[u][tid];
-          const uint32_t p[4] = {x.x, x.y, x.z, x.w}, c = 8u * s_at[u][tid];
+          const uint32_t p[4] = {x.x, x.y, x.z, x.w}, c = key0() + 8u * s_at[u][tid];
 #pragma unroll 1
           for (int e = 0; e < 4; ++e) {
             uint32_t k[2];
@@ -263,22 +318,17 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
       for (int u = 0; u < kCmTop; ++u) s_list[1][r][u] = list[u];
     }
     group_sync();
-    if (wg == 0 && row0 + r < M && !abort_flag->abort) {
-      // the eight largest of two descending lists, sorted: the larger of the ends that meet, which is a bitonic sequence
+    if (wg == 0) {
+      list_merge(list, [&](int u) { return s_list[1][r][u]; });
+      if (SHARED) {
 #pragma unroll
-      for (int u = 0; u < kCmTop; ++u) list[u] = umax(list[u], s_list[1][r][kCmTop - 1 - u]);
-#pragma unroll
-      for (int d = kCmTop / 2; d > 0; d >>= 1)
-#pragma unroll
-        for (int u = 0; u < kCmTop; ++u)
-          if ((u & d) == 0) {
-            const uint32_t x = umax(list[u], list[u + d]), y = umin(list[u], list[u + d]);
-            list[u] = x;
-            list[u + d] = y;
-          }
-      store_list(idx_out, idx64, (bh * M + row0 + r) * topk, topk, list);
+        for (int u = 0; u < kCmTop; ++u) s_list[0][r][u] = list[u];
+      } else if (row0 + r < M && !abort_flag->abort) {
+        store_list(idx_out, idx64, (bh * M + row0 + r) * topk, topk, list);
+      }
     }
   }
+  if (SHARED && warp >= 8) cluster_wait();
   if (abort_flag->abort) tc::abort_drain();
   tc::fence_before_sync();
   __syncthreads();
@@ -288,7 +338,7 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
 #pragma unroll
     for (int u = 0; u < kCmTop; ++u) list[u] = 0u;
 #pragma unroll 1
-    for (int c = 0; c < (int) n; ++c) {
+    for (int c = key0(); c < key0() + keys(); ++c) {
       const bf16* k = pk + (bh * n + c) * 64;
       float acc = 0.f;
 #pragma unroll 1
@@ -297,7 +347,30 @@ coarse_topk_tc_kernel(const __grid_constant__ CoarseMaps maps, const bf16* __res
       candidate_words(acc, 0.f, 65535u - (uint32_t) c, w, none);
       if (w > list[kCmTop - 1]) list_insert(list, w);
     }
-    store_list(idx_out, idx64, (bh * M + row0 + tid) * topk, topk, list);
+    if (SHARED) {
+#pragma unroll
+      for (int u = 0; u < kCmTop; ++u) s_list[0][tid][u] = list[u];
+    } else {
+      store_list(idx_out, idx64, (bh * M + row0 + tid) * topk, topk, list);
+    }
+  }
+  if constexpr (SHARED) {
+    // Every CTA merges the lists of an equal share of the rows: 1 << log_split neighbouring threads read a row's list each and meet in steps.
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (warp < 4) {
+      const int row = (kRows * rank + tid) >> log_split, others = (1 << log_split) - 1;
+      uint32_t list[kCmTop];
+#pragma unroll
+      for (int u = 0; u < kCmTop; ++u) list[u] = ld_cluster(&s_list[0][row][u], (uint32_t) (tid & others));
+#pragma unroll 1
+      for (int d = 1; d <= others; d <<= 1) list_merge(list, [&](int u) { return __shfl_xor_sync(0xffffffffu, list[u], d); });
+      if ((tid & others) == 0 && row0 + row < M) store_list(idx_out, idx64, (bh * M + row0 + row) * topk, topk, list);
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();                                          // nobody leaves while its lists are being read
   }
   if (warp == 0) tc::tmem_dealloc(tmem, 256);
 }
@@ -312,9 +385,13 @@ int launch_coarse_topk_tc(const LlsaTensor* pq, const LlsaTensor* pk, const Llsa
   if ((rc = tma::make_map_rows(&maps.q, pq->ptr, (uint64_t) (BH * M), kRows))) return rc;
   if ((rc = tma::make_map_rows(&maps.k, pk->ptr, (uint64_t) (BH * n), kChunk))) return rc;
   const size_t smem = 1024 + (size_t) (1 + kStages) * kTile * sizeof(bf16) + (size_t) kSlots * 2 * kRows * (sizeof(uint4) + sizeof(uint16_t));
-  LLSA_SMEM_LIMIT(coarse_topk_tc_kernel, smem);
-  launch_pdl(coarse_topk_tc_kernel, dim3((unsigned) ((M + kRows - 1) / kRows), (unsigned) BH), kThreads, smem, st, maps, (const bf16*) pq->ptr,
-             (const bf16*) pk->ptr, idx->ptr, idx->dtype == LLSA_I64 ? 1 : 0, M, n, topk, wait_limit);
+  const int64_t tiles = (M + kRows - 1) / kRows;
+  int log_split = 0;                         // of how many CTAs share a tile; no influence on the result
+  while (log_split < 3 && (BH * tiles) << (log_split + 1) <= 256 && n >= (int64_t) kChunk << (log_split + 1)) ++log_split;
+  auto kernel = log_split ? coarse_topk_tc_kernel<true> : coarse_topk_tc_kernel<false>;
+  LLSA_SMEM_LIMIT(kernel, smem);
+  launch_pdl_cluster(kernel, dim3((unsigned) (tiles << log_split), (unsigned) BH), kThreads, 1u << log_split, smem, st, maps, (const bf16*) pq->ptr,
+                     (const bf16*) pk->ptr, idx->ptr, idx->dtype == LLSA_I64 ? 1 : 0, M, n, topk, log_split, wait_limit);
   LLSA_LAUNCH_OK("coarse_topk_tc_kernel");
   return LLSA_OK;
 }

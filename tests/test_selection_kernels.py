@@ -29,8 +29,7 @@ def test_coarse_topk_shapes(BH, M, n, dtype, topk):
     assert topk == 1 or (got.sort(-1).values.diff(dim=-1) > 0).all(), "duplicate block in a row"
 
 
-# the long-list kernel (128 tiles of 128 rows and more): its shortest list, a list that ends half way through a 128-key chunk (an odd and an even number of chunks), rows that do not
-# fill a tile
+# long lists and many rows: lists that end half way through a 128-key chunk (an odd and an even number of chunks), rows that do not fill a tile
 @pytest.mark.parametrize("BH,M,n,topk", [(128, 40, 512, 8), (64, 130, 576, 8), (130, 40, 704, 5), (16, 1024, 1024, 4), (43, 300, 4160, 1), (129, 4, 8192, 8)])
 def test_coarse_topk_of_long_lists(BH, M, n, topk):
     test_coarse_topk_shapes(BH, M, n, torch.bfloat16, topk)
@@ -40,11 +39,15 @@ def test_coarse_topk_of_long_lists(BH, M, n, topk):
 @pytest.mark.parametrize("kind", ["ties", "equal", "nan", "-inf", "masked"])
 @pytest.mark.parametrize("n", [512, 1088])
 def test_coarse_topk_of_long_lists_orders_exact_scores(n, kind, wait_limit):
+    _exact_scores(64, 200, n, kind, wait_limit)
+
+
+def _exact_scores(BH, M, n, kind, wait_limit):
     """Small whole numbers: sums are exact in any order, so the order of a row is known, ties to the smaller column and NaN first.  A limit of one
-    look makes the kernel's waits run out: its CTAs then select with scalar arithmetic."""
+    look makes the tcgen05 kernel's waits run out: its CTAs then select with scalar arithmetic."""
     from llsa_b200 import _lib
     gen = torch.Generator().manual_seed(n)
-    pq, pk = torch.randint(-2, 3, (1, 64, 200, 64), generator=gen).bfloat16(), torch.randint(-2, 3, (1, 64, n, 64), generator=gen).bfloat16()
+    pq, pk = torch.randint(-2, 3, (1, BH, M, 64), generator=gen).bfloat16(), torch.randint(-2, 3, (1, BH, n, 64), generator=gen).bfloat16()
     pq[..., 0] = 1
     if kind == "equal":
         pk[:] = pk[:, :, :1]
@@ -59,10 +62,40 @@ def test_coarse_topk_of_long_lists_orders_exact_scores(n, kind, wait_limit):
     score = (pq.float() @ pk.float().transpose(-1, -2)).bfloat16().float()
     rank = torch.where(score.isnan(), torch.full_like(score, float("inf")), score)
     want = rank.sort(dim=-1, descending=True, stable=True).indices[..., :8].int()
-    q, k, got = pq.to(DEV), pk.to(DEV), torch.full((1, 64, 200, 8), -1, dtype=torch.int32, device=DEV)
+    q, k, got = pq.to(DEV), pk.to(DEV), torch.full((1, BH, M, 8), -1, dtype=torch.int32, device=DEV)
     d = [_lib.desc(t) for t in (q, k, got)]
     _lib.check(_lib.lib().llsa_coarse_topk_bounded(*[_lib.ref(t) for t in d], 8, wait_limit, _lib.stream_ptr(torch.device(DEV))), "coarse_topk_bounded")
     assert torch.equal(got.cpu(), want)
+
+
+# the tcgen05 kernel: its shortest list and the longest, lists that end half way through a 128-key chunk; few tiles, whose keys a cluster of eight, four or two
+# CTAs shares (up to 32, 64 and 128), with shares of unlike length, and more than that
+@pytest.mark.parametrize("BH,M,n,topk", [(1, 40, 3584, 8), (1, 300, 3648, 8), (2, 128, 4160, 5), (8, 500, 3584, 8), (9, 500, 3648, 8), (17, 512, 3712, 4),
+                                         (129, 4, 3584, 8), (43, 300, 3648, 1), (1, 16, 65536, 8)])
+def test_coarse_topk_on_tcgen05(BH, M, n, topk):
+    test_coarse_topk_shapes(BH, M, n, torch.bfloat16, topk)
+
+
+# tiles: a cluster of eight, four, two, none
+@pytest.mark.parametrize("wait_limit", [0, 1])
+@pytest.mark.parametrize("kind", ["ties", "equal", "nan", "-inf", "masked"])
+@pytest.mark.parametrize("BH,n", [(2, 3584), (2, 3648), (40, 3648), (100, 3584), (129, 3648)])
+def test_coarse_topk_on_tcgen05_orders_exact_scores(BH, n, kind, wait_limit):
+    _exact_scores(BH, 8, n, kind, wait_limit)
+
+
+# 512 tiles of 128 rows together; 32, 4 and 1 alone.  At these sizes a kernel that sums in another order chooses other blocks for one row or more.
+@pytest.mark.parametrize("n,seed", [(512, 0), (1024, 1), (2048, 2), (4096, 3)])
+def test_coarse_selection_of_a_row_depends_on_its_keys_alone(n, seed):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    pq, pk = [(torch.randn(1, 16, m, 64, device=DEV, generator=gen) * 0.25).bfloat16() for m in (4096, n)]
+    whole = ops._coarse_topk(pq, pk, 8)
+    for h in range(16):
+        assert torch.equal(whole[:, h:h + 1], ops._coarse_topk(pq[:, h:h + 1].contiguous(), pk[:, h:h + 1].contiguous(), 8)), h
+    for r in (0, 16, 1024, 3984):
+        for rows in (112, 512):
+            part = pq[:, :2, r:r + rows].contiguous()
+            assert torch.equal(whole[:, :2, r:r + rows], ops._coarse_topk(part, pk[:, :2].contiguous(), 8)), (r, rows)
 
 
 def test_coarse_topk_zero_and_negative_scores_tie_and_order():
