@@ -283,9 +283,10 @@ int llsa_attn_fwd(const LlsaAttnArgs* args, void* stream);
  * (sparse_attention_res_2.py:578-681) and, with fold_pool_bwd, the
  * MeanPool1dFunction_BHSC.backward calls autograd runs after them. */
 int llsa_attn_bwd(const LlsaAttnArgs* args, void* stream);
-/* Element count of the F32 scratch tensor LlsaAttnArgs.dkv_partial that llsa_attn_bwd needs for bf16 tensors with
- * Nq query rows per (b,h) and `topk` selected blocks per query block (the caller allocates it; any 4-D contiguous
- * shape with at least this many elements is accepted).  The library itself never allocates device memory. */
+/* Element count of the F32 scratch tensor LlsaAttnArgs.dkv_partial that llsa_attn_bwd makes use of for bf16 tensors with
+ * Nq query rows per (b,h) and `topk` selected blocks per query block (the caller allocates it, 4-D and contiguous).  Any size from
+ * B*H*ceil(Nq/16*topk/64)*4096 on is accepted; with less than this function names, small problems are spread over fewer warps.  The
+ * library itself never allocates device memory. */
 int64_t llsa_attn_bwd_partial_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk);
 /* Elements of the scratch LlsaAttnArgs.fwd_redo a forward makes use of, 0 if none (its pooled keys all fit at once, or the list is too short
  * for one pass to pay).  Read from `args` as below. */

@@ -7,6 +7,13 @@
 
 namespace llsa {
 
+// Windows of four small ranges of the entry lists, each with a head and a tail tile of 2048 floats in dkv_partial: the least that the fine dK/dV stage
+// needs.  With more it cuts small problems into more spans.
+static int64_t partial_windows(int64_t B, int64_t H, int64_t Nq, int32_t topk) {
+  const int64_t ranges = (Nq / kBS * topk + kRangeEntriesSmall - 1) / kRangeEntriesSmall;
+  return B * H * ((ranges + 3) / 4);
+}
+
 static int check_attn_args(const LlsaAttnArgs* g, bool bwd) {
   LLSA_REQUIRE(g, LLSA_ERR_NULL, "attn: null argument block");
   LLSA_REQUIRE(g->q && g->k && g->v && g->pk && g->pv && g->indices && g->o && g->lse, LLSA_ERR_NULL, "attn: a required tensor is null");
@@ -75,7 +82,7 @@ static int check_attn_args(const LlsaAttnArgs* g, bool bwd) {
     if ((rc = check_contig(g->dpv_acc, "dpv_acc", LLSA_F32, 4, s1))) return rc;
     if (dt == LLSA_BF16 && !g->force_generic) {
       LLSA_REQUIRE(g->dkv_partial, LLSA_ERR_WORKSPACE, "attn_bwd: dkv_partial scratch missing");
-      const int64_t need = llsa_attn_bwd_partial_elems(B, H, Nq, g->topk);
+      const int64_t need = partial_windows(B, H, Nq, g->topk) * 4096;
       LLSA_REQUIRE(g->dkv_partial->ptr && g->dkv_partial->dtype == LLSA_F32 && g->dkv_partial->ndim == 4 && is_contiguous(g->dkv_partial) &&
                        g->dkv_partial->shape[0] * g->dkv_partial->shape[1] * g->dkv_partial->shape[2] * g->dkv_partial->shape[3] >= need,
                    LLSA_ERR_WORKSPACE, "attn_bwd: dkv_partial must be a contiguous F32 tensor of at least %lld elements", (long long) need);
@@ -130,9 +137,8 @@ extern "C" int64_t llsa_attn_remainder_elems(const LlsaAttnArgs* g, int backward
 
 extern "C" int64_t llsa_attn_bwd_partial_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk) {
   if (B <= 0 || H <= 0 || Nq <= 0 || topk <= 0) return 0;
-  const int64_t ranges = (Nq / kBS * topk + kRangeEntriesSmall - 1) / kRangeEntriesSmall;     // sized for the smaller of the two range sizes
-  // a head and a tail tile (2048 floats each) per window of four small ranges, or per span (problems of fewer than 256 entries: long spans)
-  const int64_t windows = B * H * ((ranges + 3) / 4), total = B * H * (Nq / kBS) * topk;
+  // a head and a tail tile per window, or per span (problems of fewer than 256 entries: long spans)
+  const int64_t windows = partial_windows(B, H, Nq, topk), total = B * H * (Nq / kBS) * topk;
   const int64_t spans = total < 256 ? 0 : std::min<int64_t>((total + kSpanEntries - 1) / kSpanEntries, kMaxSpans);
   return std::max(windows, (spans + B * H - 1) / (B * H) * (B * H)) * 4096;      // a multiple of B H tiles: the tensor is [B,H,.,4096]
 }

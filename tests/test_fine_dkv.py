@@ -1,5 +1,7 @@
 """Fine dK/dV kernel against the oracle: windows drawn by the warps of a CTA (lists of 4,736 ranges and more), equal spans of the entries (shorter
 ones)."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -54,3 +56,38 @@ def test_persistent_form_vs_oracle(B, H, N, topk, hot):
                                             (9, 7, 2048, 8, ()), (9, 7, 2048, 8, (0, 1, 127)), (21, 11, 1024, 8, (5,))])
 def test_spans_vs_oracle(B, H, N, topk, hot):
     test_persistent_form_vs_oracle(B, H, N, topk, hot)
+
+
+@pytest.mark.parametrize("B,H,N", [(1, 2, 1024), (4, 6, 4096)])
+def test_scratch_of_one_window_per_64_entries_is_enough(B, H, N):
+    """llsa_attn_bwd with the least dkv_partial it accepts, through the C interface: fewer and longer spans, the same gradients."""
+    from llsa_b200 import _lib
+    L, dev = _lib.lib(), torch.device(DEV)
+    gen = torch.Generator(device=DEV).manual_seed(N)
+    q, k, v, do = [torch.randn(B, H, N, 64, device=DEV, generator=gen).bfloat16() for _ in range(4)]
+    dbg = llsa_b200.llsa_l1_debug(q, k, v, 8, 16)
+    idx, n1, E, S = dbg["indices"].int().contiguous(), N // 16, N // 16 * 8, L.llsa_transpose_range_entries(B, H, N // 16, 8)
+    assert S == 16
+    i32, f32 = dict(dtype=torch.int32, device=DEV), dict(device=DEV)
+    t = dict(q=q, k=k, v=v, pk=dbg["pk"], pv=dbg["pv"], indices=idx, o=dbg["o"], lse=dbg["lse"], d_o=do, delta=torch.empty(B, H, N, **f32),
+             offsets=torch.empty(B, H, n1 + 1, **i32), flat=torch.empty(B, H, E, **i32), flat_ranges=torch.empty(B, H, -(-E // S), 2, **i32),
+             dpk_acc=torch.empty(B, H, n1, 64, **f32), dpv_acc=torch.empty(B, H, n1, 64, **f32), remainder=torch.empty_like(q))
+    d = {n: _lib.desc(x) for n, x in t.items()}
+    _lib.check(L.llsa_transpose_indices_pairs(*[_lib.ref(d[n]) for n in ("indices", "offsets", "flat")], None, _lib.ref(d["flat_ranges"]), n1, None, 0, None,
+                                              _lib.stream_ptr(dev)), "transpose")
+    least, full, got = B * H * -(-E // 64) * 4096, L.llsa_attn_bwd_partial_elems(B, H, N, 8), {}
+    assert least < full
+    for n in (least, full, least - 4096):
+        out = [torch.full_like(q, float("nan")) for _ in range(3)]
+        partial = torch.empty(1, 1, n // 4096, 4096, **f32)
+        od, pd = [_lib.desc(x) for x in out], _lib.desc(partial)
+        a = _lib.LlsaAttnArgs()
+        for name, x in list(d.items()) + list(zip(("dq", "dk", "dv"), od)) + [("dkv_partial", pd)]:
+            setattr(a, name, _lib.ptr(x))
+        a.topk, a.block_size, a.token_weight, a.kv_weight, a.fold_pool_bwd = 8, 16, 16.0, 16.0, 1
+        rc = L.llsa_attn_bwd(C.byref(a), _lib.stream_ptr(dev))
+        torch.cuda.synchronize()
+        assert (rc == 0) == (n >= least), (n, rc)
+        got[n] = [x.float() for x in out]
+    for x, y in zip(got[least], got[full]):      # fp32 sums meet in another order, then one rounding to bf16
+        assert float((x - y).norm() / y.norm()) < 2e-3
