@@ -619,11 +619,11 @@ __device__ __forceinline__ void coarse_row_scalar(const FusedCoarse& f, int64_t 
 
 // FUSED: 0 parents given, 1 selected here by coarse_row_64, 2 by coarse_row_scalar.
 // A CTA is a chain of short steps (parents, keys, scores, rounds of the selection), so what counts is how many of them an SM holds, and that they are few
-// waves: 9 CTAs (8 with the scalar step, 6 in fp32) where the compiler's choice of registers allowed 8 and 5.  H=5 N=40960, top-16: 49 us with five an SM,
+// waves: PER_SM of them, 9 (8 with the scalar step) where the compiler's choice of registers allowed 8 and 5.  H=5 N=40960, top-16: 49 us with five an SM,
 // where 800 CTAs are 740 and a second wave of 60, parents inserted into a list one by one and keys loaded when they are needed; 32.8 now.  Lists of eight
 // parents: B=8 H=6 N=16384 31.8 -> 29.9, B=4 19.7 -> 18.6, B=1 8.8 -> 8.2, B=3 H=5 N=5376 10.0 -> 8.9.
-template <typename T, bool MMA, int FUSED = 0>
-__global__ void __launch_bounds__(128, FUSED < 2 ? 9 : sizeof(T) == 2 ? 8 : 6)
+template <typename T, bool MMA, int FUSED = 0, int PER_SM = FUSED < 2 ? 9 : 8>
+__global__ void __launch_bounds__(128, PER_SM)
 refine_topk_kernel(const T* __restrict__ pq1, const T* __restrict__ pk1, IdxView p_idx, void* __restrict__ idx_out, int idx64, int64_t M,
                    int64_t Mk, int D_, int topk, int p_topk, int bs_, FusedCoarse fused) {
   pdl_trigger();
@@ -905,9 +905,12 @@ extern "C" int llsa_select_two_level(const LlsaTensor* pq1, const LlsaTensor* pk
   const int idx64 = idx->dtype == LLSA_I64;
   const IdxView none{nullptr, 0};
   if (dt == LLSA_F32) {
-    LLSA_SMEM_LIMIT((refine_topk_kernel<float, false, 2>), smem);
-    launch_pdl(refine_topk_kernel<float, false, 2>, grid, 128, smem, st, (const float*) pq1->ptr, (const float*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D,
-                                                                 topk, p_topk, bs, f);
+    // Six CTAs per SM cost 48 bytes of spilled registers, five 8: five where they are one wave anyway.  Forward in us, five / six: B=1 H=2 N=4096 (32 CTAs)
+    // 45.5 / 46.2, B=3 H=5 N=5376 (315) 290.7 / 292.6, B=1 H=6 N=16384 (384) 425.4 / 426.7; B=2 H=6 N=16384 (768) 855.6 / 851.3, B=1 H=5 N=40960 top-16
+    // (800) 1707 / 1702, B=1 H=6 N=65536 (1536) 2458 / 2454.
+    auto kernel = B * H * (M / bs) <= 5 * 148 ? refine_topk_kernel<float, false, 2, 5> : refine_topk_kernel<float, false, 2, 6>;
+    LLSA_SMEM_LIMIT(kernel, smem);
+    launch_pdl(kernel, grid, 128, smem, st, (const float*) pq1->ptr, (const float*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D, topk, p_topk, bs, f);
   } else if (on_mma) {
     LLSA_SMEM_LIMIT((refine_topk_kernel<bf16, true, 1>), smem);
     launch_pdl(refine_topk_kernel<bf16, true, 1>, grid, 128, smem, st, (const bf16*) pq1->ptr, (const bf16*) pk1->ptr, none, idx->ptr, idx64, M, Mk, (int) D, topk,

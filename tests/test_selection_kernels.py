@@ -127,6 +127,19 @@ def test_select_two_level_is_its_two_steps(N, topk, p_topk, dtype):
     assert bad == 0
 
 
+@pytest.mark.parametrize("H,N", [(4, 47360), (5, 40960)])
+def test_fp32_selection_of_one_wave_of_five_ctas_per_sm_and_of_more(H, N):
+    """740 CTAs and 800: the lists of its two steps, and what every head has alone."""
+    gen = torch.Generator(device=DEV).manual_seed(N)
+    pq, pk = [torch.randn(1, H, N // 16, 64, device=DEV, generator=gen) for _ in range(2)]
+    pq2, pk2 = ops.mean_pool1d(pq, 16), ops.mean_pool1d(pk, 16)
+    idx, pidx = ops._select_two_level(pq, pk, pq2, pk2, 16, 16, 16)
+    assert torch.equal(pidx, ops._coarse_topk(pq2, pk2, 16)) and torch.equal(idx, ops._refine_topk(pq, pk, pidx, 16, 16, 16))
+    for h in range(H):
+        alone = ops._select_two_level(*[t[:, h:h + 1].contiguous() for t in (pq, pk, pq2, pk2)], 16, 16, 16)
+        assert torch.equal(alone[0], idx[:, h:h + 1]) and torch.equal(alone[1], pidx[:, h:h + 1])
+
+
 # lists with repeats inside a row, every entry in one bucket, keys outside their range; one and several key ranges, 16 and 32 warps, T = 1
 @pytest.mark.parametrize("BH,M,T,n,kind", [(1, 16, 8, 16, "uniform"), (3, 130, 6, 129, "uniform"), (2, 3000, 8, 3000, "one"), (1, 5000, 16, 5000, "hot"),
                                            (2, 300, 1, 1000, "uniform"), (60, 64, 8, 64, "hot"), (1, 16384, 8, 16384, "hot")])
