@@ -96,11 +96,12 @@ def test_values_pooled_beside_the_selection(B, H, N):
 
     def parts():
         (pq, pk, pv), (pq2, pk2, pv2) = ops.pool_pyramid([q, k, v], 16, 2)
-        idx, _ = ops._select_two_level(pq, pk, pq2, pk2, 8, 8, 16)
-        return idx, pv, pv2
+        idx, pidx = ops._select_two_level(pq, pk, pq2, pk2, 8, 8, 16)
+        return idx, pv, pv2, ops._attn_fwd(q, k, v, pk, pv, pk2, pv2, idx, pidx, 8, 8, 16, 16.0, 256.0)[0]
 
     for _ in range(3):
-        got, (idx, pv, pv2) = llsa_b200.llsa_l2_debug(q, k, v), parts()
+        got, (idx, pv, pv2, o) = llsa_b200.llsa_l2_debug(q, k, v), parts()
+        assert torch.equal(got["o"], o)      # an attention stage that ran ahead of the values' pooling would have read the last call's
         assert torch.equal(got["indices"], idx.to(got["indices"].dtype)) and torch.equal(got["pv"], pv) and torch.equal(got["pv2"], pv2)
         v.normal_(generator=gen)
     want = llsa_b200.llsa_l2(q, k, v)
