@@ -1,6 +1,6 @@
 """Discrete-event model of the mbarrier protocol of the key-loop tcgen05 kernels
-(llsa_b200/csrc/attn_pooled_loop_tc.cu, attn_pooled_bwd_loop_tc.cu, attn_pooled_dkv_loop_tc.cu) and of the
-single-shot pooled backward with its two MMA-issuing threads (attn_pooled_bwd_tc.cu).
+(llsa_b200/csrc/attn_pooled_loop_tc.cu, attn_pooled_bwd_loop_tc.cu, attn_pooled_dkv_loop_tc.cu) of the
+single-shot pooled forward and backward (attn_pooled_tc.cu, attn_pooled_bwd_tc.cu) and of the coarse selection (topk_tc.cu).
 
 Test infrastructure: nothing in the package imports it.  Every role of a CTA
 (the two TMA producers, the warps that issue MMAs, the softmax warps, the
@@ -721,6 +721,269 @@ def single_shot_backward_kernel(seed, t_begin, n_tiles, tiles_per_head, mma_done
         sim.spawn("drain%d" % w, drain(w))
     for w in range(12):
         sim.spawn("softmax%d" % w, softmax(w))
+    return sim.run()
+
+def single_shot_forward_kernel(seed, tiles, head=True, sums_wait_for_epilogue=True, products_wait_for_epilogue=True, o_ring=3):
+    """attn_fwd_pooled_tc_kernel: `tiles` query tiles of one CTA, two score buffers (P over S, O behind them).  Two producers (Q and keys, three
+    stages; values, two), one warp issues S, one O = P.V, two softmax groups on alternate tiles, four epilogue warps, each with its own rows of o:
+    loaded a tile ahead into a ring of three, merged in place and stored from there.
+    head: P of all but the last 64 keys is handed over first (more than 64 keys).  The last three arguments break the protocol on purpose:
+    maxima and sums written before the tile before last's have been read, O written before it has been read, an o ring that is too short for
+    the store that may still read it."""
+    sim = Sim(seed)
+    key_stages, value_stages = 3, 2
+    owner = [None, None]
+    keys = [Resource("Q / key stage %d" % i) for i in range(key_stages)]
+    values = [Resource("value stage %d" % i) for i in range(value_stages)]
+    acc = [Resource("O of buffer %d" % i) for i in range(2)]
+    stats = [Resource("maxima and sums %d" % i) for i in range(2)]
+    full_k, empty_k = _bars("full_k", key_stages, 1), _bars("empty_k", key_stages, 1)
+    full_v, empty_v = _bars("full_v", value_stages, 1), _bars("empty_v", value_stages, 1)
+    s_ready, p_head, p_ready = _bars("s_ready", 2, 1), _bars("p_head", 2, 4), _bars("p_ready", 2, 4)
+    buf_free, o_ready, o_free = _bars("buf_free", 2, 1), _bars("o_ready", 2, 1), _bars("o_free", 2, 4)
+
+    def producer(ring, full, empty, stages):
+        for i in range(tiles):
+            st = i % stages
+            yield ("wait", empty[st], ((i // stages) & 1) ^ 1)
+            land = sim.t + sim.r(500, 1500)
+            ring[st].write(sim, i, at=land)
+            sim.at(land, (lambda b=full[st]: b.arrive(sim)))
+
+    def s_issuer():
+        for i in range(tiles):
+            st, b = i % key_stages, i & 1
+            wait = ["wait", full_k[st], (i // key_stages) & 1]
+            if i >= 2:
+                wait += [buf_free[b], ((i >> 1) - 1) & 1]
+            yield tuple(wait)
+            assert owner[b] is None, ("scores written over a live buffer", b, owner[b], i)
+            start, done = sim.mma("s", 384)
+            keys[st].read(sim, i, done)
+            sim.at(done, (lambda b=b, i=i: owner.__setitem__(b, ("s", i))))
+            yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+            sim.commit("s", s_ready[b])
+            sim.commit("s", empty_k[st])
+            yield ("delay", sim.r(30, 80))
+
+    def o_issuer():
+        for i in range(tiles):
+            st, b, par = i % value_stages, i & 1, (i >> 1) & 1
+            wait = ["wait", full_v[st], (i // value_stages) & 1, (p_head if head else p_ready)[b], par]
+            if i >= 2 and products_wait_for_epilogue:
+                wait += [o_free[b], par ^ 1]
+            yield tuple(wait)
+            acc[b].write(sim, i)
+            if head:
+                assert owner[b] in (("h", i), ("p", i)), ("first part of P.V read", b, owner[b], i)
+                start, done = sim.mma("o", 384)
+                values[st].read(sim, i, done)
+                yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+                yield ("wait", p_ready[b], par)
+            assert owner[b] == ("p", i), ("P.V read", b, owner[b], i)
+            start, done = sim.mma("o", 192)
+            values[st].read(sim, i, done)
+            sim.at(done, (lambda b=b: owner.__setitem__(b, None)))
+            yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+            for bar in (o_ready[b], empty_v[st], buf_free[b]):
+                sim.commit("o", bar)
+            yield ("delay", sim.r(30, 80))
+
+    def softmax(group, warp):
+        for i in range(group, tiles, 2):
+            par = (i >> 1) & 1
+            yield ("wait", s_ready[group], par)
+            assert owner[group] is not None and owner[group][1] == i, ("softmax read", group, owner[group], i)
+            yield ("delay", sim.r(600, 2000))
+            if head:
+                if warp == 0:
+                    owner[group] = ("h", i)
+                p_head[group].arrive(sim)
+                yield ("delay", sim.r(200, 600))
+            if i >= 2 and sums_wait_for_epilogue:
+                yield ("wait", o_free[group], par ^ 1)
+            if warp == 0:
+                stats[group].write(sim, ("being written", i))
+                owner[group] = ("p", i)
+            yield ("delay", sim.r(5, 30))
+            if warp == 0:
+                stats[group].tag = i
+            p_ready[group].arrive(sim)
+
+    def epilogue(warp):
+        ring = [Resource("o stage %d of warp %d" % (i, warp)) for i in range(o_ring)]
+        full = _bars("out_full", o_ring, 1)
+        stored = []                       # when the stores issued so far have read their stage
+
+        def request(i):
+            land = sim.t + sim.r(500, 1500)
+            ring[i % o_ring].write(sim, i, at=land)
+            sim.at(land, (lambda b=full[i % o_ring]: b.arrive(sim)))
+
+        if tiles:
+            request(0)
+        for i in range(tiles):
+            b, par = i & 1, (i >> 1) & 1
+            if i + 1 < tiles:
+                if len(stored) >= 2:      # all but the newest store have read their stage
+                    yield ("delay", max(0, stored[-2] - sim.t))
+                request(i + 1)
+            yield ("wait", full[i % o_ring], (i // o_ring) & 1)
+            yield ("wait", p_ready[b], par)
+            yield ("wait", o_ready[b], par)
+            for _ in range(2):
+                for r in (acc[b], stats[b]):
+                    r.read(sim, i)
+                yield ("delay", sim.r(100, 2500))
+            acc[b].read(sim, i)
+            stats[b].read(sim, i)
+            o_free[b].arrive(sim)
+            yield ("delay", sim.r(50, 300))
+            at = max([sim.t] + stored[-1:]) + sim.r(100, 3000)      # stores read in order
+            ring[i % o_ring].read(sim, i, at)
+            stored.append(at)
+
+    sim.spawn("producer K", producer(keys, full_k, empty_k, key_stages))
+    sim.spawn("producer V", producer(values, full_v, empty_v, value_stages))
+    sim.spawn("s", s_issuer())
+    sim.spawn("o", o_issuer())
+    for w in range(4):
+        for g in range(2):
+            sim.spawn("softmax%d%d" % (g, w), softmax(g, w))
+        sim.spawn("epilogue%d" % w, epilogue(w))
+    return sim.run()
+
+
+def coarse_selection_kernel(seed, shares, free_count=4, groups_meet=True, lists_wait=True):
+    """coarse_topk_tc_kernel: a cluster whose CTA k walks shares[k] key chunks twice (a job each time).  One producer (two key stages), one warp issues
+    the products, half a job at a time, two groups of four warps on alternate jobs, each with a score buffer per half of its job.  The groups of a CTA share
+    the maxima of the first pass, the CTAs the bounds, then (pass 2 sets scores aside where the maxima were) the groups and in the end the CTAs
+    their lists.
+    free_count: warps whose arrivals hand a score buffer back (4 = the kernel); groups_meet=False: maxima read without the meeting that
+    says they are written; lists_wait=False: a CTA leaves without waiting for the ones that read its lists.  Each breaks the protocol on purpose."""
+    sim = Sim(seed)
+    meet_count = 10 * len(shares)         # every warp of the cluster
+    meet = [Barrier("cluster meeting %d" % i, meet_count) for i in range(3)]
+    bound = [Resource("bound of CTA %d" % k) for k in range(len(shares))]
+    lists = [Resource("lists of CTA %d" % k) for k in range(len(shares))]
+
+    def cta(k, chunks):
+        jobs = 2 * chunks
+        stage = [Resource("key stage %d of CTA %d" % (i, k)) for i in range(2)]
+        owner = {}
+        place = [Resource("maxima / slots of group %d, CTA %d" % (g, k)) for g in range(2)]
+        k_full, k_empty = _bars("k_full", 2, 1), _bars("k_empty", 2, 1)
+        s_ready, s_free = _bars("s_ready", 4, 1), _bars("s_free", 4, free_count)
+        pair = [Barrier("group_sync %d" % i, 8) for i in range(3)]
+        sync = Barrier("__syncthreads", 10)
+
+        def end(warp):
+            sync.arrive(sim)
+            yield ("wait", sync, 0)
+            if warp == 0:
+                lists[k].tag = "lists"
+            meet[1].arrive(sim)
+            yield ("wait", meet[1], 0)
+            if warp < 4:
+                for o in range(len(shares)):
+                    lists[o].read(sim, "lists")
+                yield ("delay", sim.r(50, 800))
+                for o in range(len(shares)):
+                    lists[o].read(sim, "lists")
+            meet[2].arrive(sim)
+            if lists_wait:
+                yield ("wait", meet[2], 0)
+            if warp == 0:
+                lists[k].write(sim, "gone with the CTA")
+
+        def producer():
+            meet[0].arrive(sim)
+            for j in range(jobs):
+                yield ("wait", k_empty[j & 1], ((j >> 1) & 1) ^ 1)
+                land = sim.t + sim.r(500, 1500)
+                stage[j & 1].write(sim, j, at=land)
+                sim.at(land, (lambda b=k_full[j & 1]: b.arrive(sim)))
+            yield ("wait", meet[0], 0)
+            yield from end(8)
+
+        def issuer():
+            meet[0].arrive(sim)
+            for j in range(jobs):
+                for half in range(2):
+                    buf = (j & 1) * 2 + half
+                    wait = ["wait", k_full[j & 1], (j >> 1) & 1]
+                    if j >= 2:
+                        wait += [s_free[buf], ((j >> 1) - 1) & 1]
+                    yield tuple(wait)
+                    assert owner.get(buf) is None, ("scores written over a live buffer", buf, owner[buf], j)
+                    start, done = sim.mma(("s", k), 192)
+                    stage[j & 1].read(sim, j, done)
+                    owner[buf] = ("in flight", j)
+                    sim.at(done, (lambda b=buf, j=j: owner.__setitem__(b, (j, 4))))
+                    yield ("delay", max(0, start - sim.t) + sim.r(50, 200))
+                    sim.commit(("s", k), s_ready[buf])
+                sim.commit(("s", k), k_empty[j & 1])
+                yield ("delay", sim.r(30, 80))
+            yield ("wait", meet[0], 0)
+            yield from end(9)
+
+        def group(g, warp):
+            def look(j, first):
+                for half in range(2):
+                    buf = g * 2 + half
+                    yield ("wait", s_ready[buf], (j >> 1) & 1)
+                    assert owner[buf] is not None and owner[buf][0] == j, ("scores read", buf, owner[buf], j)
+                    yield ("delay", sim.r(100, 900))
+                    assert owner[buf] is not None and owner[buf][0] == j, ("scores gone while they are read", buf, owner[buf], j)
+                    left = owner[buf][1] - 1
+                    owner[buf] = (j, left) if left else None
+                    if warp < free_count:
+                        s_free[buf].arrive(sim)
+                    if not first and sim.rng.random() < 0.3:
+                        yield ("delay", sim.r(200, 3000))
+
+            for j in range(g, chunks, 2):
+                yield from look(j, True)
+            if warp == 0:
+                place[g].tag = "maxima"
+            pair[0].arrive(sim)
+            if groups_meet:
+                yield ("wait", pair[0], 0)
+            for o in range(2):
+                place[o].read(sim, "maxima", sim.t + 40)
+            yield ("delay", sim.r(40, 200))
+            if g == 0 and warp == 0:
+                bound[k].tag = "bound"
+            meet[0].arrive(sim)
+            yield ("wait", meet[0], 0)
+            for o in range(len(shares)):
+                bound[o].read(sim, "bound")
+            if warp == 0:
+                place[g].write(sim, "slots")
+            first2 = chunks + ((chunks & 1) ^ g)
+            for j in range(first2, jobs, 2):
+                yield from look(j, False)
+            if warp == 0:                 # every warp has slots of its own; the model follows the first one's
+                place[g].read(sim, "slots")
+            pair[1].arrive(sim)
+            yield ("wait", pair[1], 0)
+            if g == 1 and warp == 0:
+                place[1].write(sim, "list")
+            pair[2].arrive(sim)
+            yield ("wait", pair[2], 0)
+            if g == 0:
+                place[1].read(sim, "list")
+            yield ("delay", sim.r(20, 100))
+            yield from end(4 * g + warp)
+
+        sim.spawn("producer %d" % k, producer())
+        sim.spawn("s %d" % k, issuer())
+        for w in range(4):
+            for g in range(2):
+                sim.spawn("group %d%d of %d" % (g, w, k), group(g, w))
+
+    for k, chunks in enumerate(shares):
+        cta(k, chunks)
     return sim.run()
 
 

@@ -6,7 +6,8 @@ import random
 
 import pytest
 
-from protocol_model import forward_kernel, key_major_kernel, outcome, query_major_kernel, single_shot_backward_kernel
+from protocol_model import (coarse_selection_kernel, forward_kernel, key_major_kernel, outcome, query_major_kernel, single_shot_backward_kernel,
+                            single_shot_forward_kernel)
 
 RUNS = 250
 
@@ -143,3 +144,29 @@ def test_query_major_ring_of_seven_has_no_hazard_or_deadlock():
     for seed in range(RUNS):
         rng = random.Random(seed)
         assert outcome(query_major_kernel, seed, rng.randint(1, 7), rng.randint(1, 9), stages=7) == "ok", seed
+
+
+@pytest.mark.parametrize("head", [False, True])
+def test_single_shot_forward_has_no_hazard_or_deadlock(head):
+    """attn_fwd_pooled_tc_kernel with 64 keys a row (P in one part) and with 128 and 192; one tile, two, and more than the rings have stages."""
+    for seed in range(RUNS):
+        assert outcome(single_shot_forward_kernel, seed, 1 + seed % 9, head) == "ok", seed
+
+
+@pytest.mark.parametrize("broken", [dict(sums_wait_for_epilogue=False), dict(products_wait_for_epilogue=False), dict(o_ring=2)])
+def test_model_catches_a_single_shot_forward_that_does_not_wait_for_its_epilogue(broken):
+    assert any(outcome(single_shot_forward_kernel, seed, 8, True, **broken) != "ok" for seed in range(60))
+
+
+def test_coarse_selection_has_no_hazard_or_deadlock():
+    """coarse_topk_tc_kernel alone and in clusters of two to eight; shares of one chunk, where a group is without work in either pass, odd and even ones,
+    of unlike length."""
+    for seed in range(RUNS):
+        rng = random.Random(seed)
+        low = rng.choice([1, 1, 2, 3, 8])
+        assert outcome(coarse_selection_kernel, seed, [low + rng.randint(0, 1) for _ in range(rng.choice([1, 1, 2, 4, 8]))]) == "ok", seed
+
+
+@pytest.mark.parametrize("broken", [dict(free_count=3), dict(groups_meet=False), dict(lists_wait=False)])
+def test_model_catches_broken_coarse_selections(broken):
+    assert any(outcome(coarse_selection_kernel, seed, [5, 4], **broken) != "ok" for seed in range(60))
