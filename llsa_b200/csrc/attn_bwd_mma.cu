@@ -486,15 +486,6 @@ __device__ __forceinline__ void tile_to_mem(float* s, const float (&dk)[8][4], c
     s4[(8 + u) * 32] = make_float4(dv[u][0], dv[u][1], dv[u][2], dv[u][3]);
   }
 }
-__device__ __forceinline__ void tile_add_mem(const float* s, float (&dk)[8][4], float (&dv)[8][4], int lane) {
-  const float4* s4 = reinterpret_cast<const float4*>(s) + lane;
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const float4 x = s4[u * 32], y = s4[(8 + u) * 32];
-    dk[u][0] += x.x; dk[u][1] += x.y; dk[u][2] += x.z; dk[u][3] += x.w;
-    dv[u][0] += y.x; dv[u][1] += y.y; dv[u][2] += y.z; dv[u][3] += y.w;
-  }
-}
 __device__ __forceinline__ void tile_zero(float (&dk)[8][4], float (&dv)[8][4]) {
 #pragma unroll
   for (int u = 0; u < 8; ++u) dk[u][0] = dk[u][1] = dk[u][2] = dk[u][3] = dv[u][0] = dv[u][1] = dv[u][2] = dv[u][3] = 0.f;

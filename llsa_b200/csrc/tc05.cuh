@@ -127,16 +127,6 @@ __host__ __device__ constexpr uint32_t instr_desc(int M, int N, int a_mn, int b_
          ((uint32_t) (M >> 4) << 24);
 }
 
-// D(tmem) (+)= A(smem) . B(smem); one thread issues.
-__device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      :
-      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
 // ---- issue by a warp in step: every lane executes the statement, elect.sync picks the lane that issues.  tcgen05.mma takes its
 // descriptors from uniform registers and is issued once per executing thread; where the compiler sees an elected thread in uniform control
 // flow the descriptors stay there, where it sees `if (lane == 0)` every instruction costs some 98 cycles of moves, whatever its size, and
@@ -247,21 +237,6 @@ __device__ __forceinline__ void umma_commit_w(uint64_t* bar) {
   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
                "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
 }
-// D(tmem) (+)= A(tmem) . B(smem): A is M x K with row r in TMEM lane r and the K values packed two per 32-bit column.
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      :
-      : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-// The mbarrier gets one arrival when every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // ---- TMEM -> registers: lane (32 * (warp % 4) + lane id) gets 32 consecutive fp32 columns ----
 // Asynchronous: the registers may be read only after tmem_ld_wait(v) (which ties them to the wait).
 __device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, float (&v)[32]) {

@@ -77,19 +77,7 @@ inline int make_map_acc(CUtensorMap* m, void* base, uint64_t rows, uint32_t box_
 }
 
 #ifdef __CUDACC__
-__device__ __forceinline__ void load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* mbar, int c0, int c1) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-                   (uint32_t) __cvta_generic_to_shared(smem_dst)),
-               "l"(map), "r"((uint32_t) __cvta_generic_to_shared(mbar)), "r"(c0), "r"(c1)
-               : "memory");
-}
-__device__ __forceinline__ void load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* mbar, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(
-                   (uint32_t) __cvta_generic_to_shared(smem_dst)),
-               "l"(map), "r"((uint32_t) __cvta_generic_to_shared(mbar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-               : "memory");
-}
-// The same issued by one lane of a warp in step (tc05.cuh: umma_ss_k64): inside `if (lane == 0)` a copy costs its warp some 300 cycles, and
+// Copies issued by one lane of a warp in step (tc05.cuh: umma_ss_k64): inside `if (lane == 0)` a copy costs its warp some 300 cycles, and
 // two of them per job were the pace of the key-loop kernels.
 __device__ __forceinline__ void load_2d_w(void* smem_dst, const CUtensorMap* map, uint64_t* mbar, int c0, int c1) {
   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
@@ -137,9 +125,6 @@ __device__ __forceinline__ void reduce_wait_all() { asm volatile("cp.async.bulk.
 __device__ __forceinline__ void expect_tx_w(uint64_t* mbar, uint32_t bytes) {
   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
                "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"((uint32_t) __cvta_generic_to_shared(mbar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void expect_tx(uint64_t* mbar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"((uint32_t) __cvta_generic_to_shared(mbar)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t) __cvta_generic_to_shared(mbar)) : "memory");
