@@ -902,14 +902,14 @@ __device__ __forceinline__ void dkv_store_unselected(const AttnP<bf16>& a, int64
 // this is the first boundary the bucket crosses, and adds the pieces in order: the tail of the window the bucket begins in, then
 // the heads.  A warp owns 32 channels of one tensor, so a piece is four 128-bit loads per lane, four pieces in flight.
 // The first n_plain * BH CTAs: the unselected blocks, 16 per CTA -- stores at the memory's rate next to the latency of the lookups (as extra
-// CTAs or extra work of the kernel above they cost twice as much: two CTAs of it fill an SM).
-// One warp for eight buckets, looking for both kinds, took 46 us at 48 slices of 16384 tokens and 160 us at 6 of 262144; this kernel 31
-// and 81.
+// CTAs or extra work of the kernel above they cost twice as much: one CTA of it fills an SM).
+// Launched behind the kernel above it takes 42 us at 48 slices of 16384 tokens and 114 at 6 of 262144 (ncu, cold cache); one warp for eight buckets, looking for
+// both kinds, took half as long again and twice as long.
 // It is launched while the kernel above ends: the unselected blocks and the lookups need nothing of it (its CTAs let this launch begin once they have
 // waited for the kernels in front of them) and take the SMs that its ragged end leaves idle; what adds pieces waits.  Whole layer, launched behind / into
 // the end: one level, B=4 H=6 N=4096 189.2 / 186.5 us, B=2 H=4 N=16384 334 / 329; two levels, B=3 H=5 N=5376 164.9 / 160.1, H=5 N=40960 top-16
 // 548 / 542, B=4 H=6 N=16384 641 / 634.
-// What it still takes behind the end (24 us at 48 slices of 16384 tokens, 55 % of whose blocks are unselected, 90 at 6 of 262144, 87 %) is the memory's time
+// What it still takes behind the end (in a graph, 24 us at 48 slices of 16384 tokens, 55 % of whose blocks are unselected, 90 at 6 of 262144, 87 %) is the memory's time
 // for 4 KB a block.  No gain from: the unselected blocks written by warps of the kernel above that have run out of ranges (that kernel grows by what this one
 // loses: 506 and 516 us for both at 262144); one wave of CTAs that go from boundary to boundary with the next lookups under way (50 instead of 42 us at B=1 H=5
 // N=40960 top-16); eight to thirty-two blocks a warp.

@@ -50,8 +50,8 @@ constexpr int kRing = REM ? 7 : 8;            // key and value chunks; the remai
 constexpr int kThreads = 512;
 constexpr int kLaunchRegs = 128, kIssueRegs = 40, kEpilogueRegs = 88, kSoftmaxRegs = 192;     // a thread's, per role: 40 + 88 + 2 x 192 = 4 x 128
 static_assert(kIssueRegs + kEpilogueRegs + 2 * kSoftmaxRegs <= 4 * kLaunchRegs, "the takers would wait for good");
-// The split is that of the form with a remainder (46.7 us at H=5 N=40960, 416 keys, against 50.4 with 56 / 88 / 184); the form without spills one
-// word with it, which 48 / 88 / 184 and 56 / 72 / 192 do not (71 us against 72 at H=6 N=65536).
+// Nothing spills with 56 / 88 / 184 or 48 / 88 / 184 either.  Forward + backward in a graph, us, as it is / 56 / 48: two levels, B=3 H=5 N=5376 138.2 / 138.9 / 139.6,
+// H=5 N=40960 top-16 492.2 / 492.2 / 492.2, H=6 N=65536 588.7 / 590.5 / 590.7; one level, B=2 H=4 N=16384 313.6 / 314.0 / 315.4, B=4 H=6 N=4096 162.2 / 162.4 / 161.6.
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr int kBufs = 4;                     // S buffers (dS over them)
 constexpr uint32_t kColDP = 256, kColDQ = 384;

@@ -44,12 +44,14 @@ void set_error(const char* fmt, ...);
 // passed pdl_trigger() (or exited), and starts its own work after pdl_wait(), which returns when that kernel has completed and its
 // writes are visible.  A layer is a chain of some ten kernels of 4 to 300 us; without this every one of them begins with an idle GPU for
 // the 2 us between the last CTA of a kernel and the first instruction of the next.  Every kernel launched this way waits before its first
-// access to global memory, so completion stays transitive along the chain; attn_dkv_finish_kernel alone works ahead of its wait, on what the kernels
-// in front of its predecessor left, and one of its CTAs waits in any case.
-// Not for the streaming kernels (pooling pass, rotation / norm backward): a CTA that arrives while the kernel in
-// front still runs finds the SM divided for that kernel's shared memory, and with 28 KB of L1 to land its loads in it streams at two thirds
-// of its rate (B=4 H=6 N=16384 with norm and rotation, whole layer: 709 us with the three launched plainly, 757 with all chained, 720 with
-// none; l1_rope B=4 H=6 N=4096 243, 243 and 259).
+// access to global memory, so completion stays transitive along the chain.  Two work ahead of their wait, and keep one CTA that waits in any case:
+//   * attn_dkv_finish_kernel reads what the kernels in front of its predecessor left: attn_dkv_fine_ring_kernel lets it begin behind its own wait, so
+//     these have completed;
+//   * pool_pyramid_bf16_kernel, launched to run beside the selection, reads the values and writes their pooled levels.  The pooling launch of q and k in
+//     front of the selection waits in every CTA and has no pdl_trigger(): the selection's CTAs, and so this launch, begin when it has ended, and all
+//     in front of it has completed.
+// A kernel in front of a streaming one (pooling pass, rotation / norm backward) has no pdl_trigger(): that one's CTAs would settle unevenly on the SMs that
+// become free first (figures at its launch).
 // cluster: neighbouring CTAs along x that form a cluster (the grid's x is a multiple of it).
 template <typename... P, typename... A>
 inline void launch_pdl_cluster(void (*kernel)(P...), dim3 grid, dim3 block, unsigned cluster, size_t smem, cudaStream_t st, A&&... args) {

@@ -147,7 +147,8 @@ __global__ void __launch_bounds__(kFbThreads, NORM ? 4 : 1) front_bwd_kernel(Fro
             dot += __shfl_xor_sync(0xffffffffu, dot, o);
           }
           const float rstd = rsqrtf(ss / (float) kFbC + a.eps), k = dot * rstd / (float) kFbC;      // k = mean(g w xh)
-          // rstd meets x before it meets k and itself again: without an eps the square of it leaves the range of a float long before dx does
+          // rstd meets x before it meets k and itself again: without an eps the square of it leaves the range of a float long before dx does.  (Kernel alone, in a
+          // graph, B=4 H=6 N=16384: with the square 65.5 us, so 65.9, with k rstd beside x rstd 66.7.)
           const float live = s < a.S ? rstd : 0.f;
           const F2 l2 = f2(live, live), k2 = f2(-k, -k);
 #pragma unroll

@@ -243,11 +243,11 @@ void run_fwd(const Core& c, int topk, int topk_p, int bs, double w1, double w2, 
 }
 
 // The values' share of the pooling pass runs beside the two-level selection, which reads little and leaves SMs idle, instead of in front of it: one launch
-// more.  Below the first line the host is the pace of a call; above the second the refinement fills the SMs one and a half times and more, and only
-// its end is left for the values.  Whole pass in us, in front / beside: B=1 H=6 N=4096 (1,536 query blocks) forward + backward 117 / 120; B=3 H=5 N=5376
-// (5,040) 148 / 144; B=1 H=6 N=16384 (6,144) 171 / 167, forward alone 46.8 / 47.2; B=2 H=6 N=16384 (12,288) 290 / 280, forward 82.0 / 77.9; B=1 H=5
-// N=40960, top-16 (12,800) 507 / 498; B=4 H=6 N=16384 (24,576) 506 / 505; B=2 H=4 N=65536 (32,768) forward 228 / 227; B=8 H=6 N=16384 (49,152)
-// 951 / 960; B=1 H=6 N=262144 (98,304) forward 1034 / 1045.
+// more.  Below the first line the host is the pace of an eager forward + backward; above the second the refinement fills the SMs one and a half times and
+// more, and only its end is left for the values.  us, in front / beside, forward + backward, the same in a graph, forward alone: B=1 H=6 N=4096 (1,536
+// query blocks) 112.7 / 115.8, 80.0 / 78.7, 25.2 / 24.5; B=3 H=5 N=5376 (5,040) 142.8 / 138.5, 140.3 / 138.8, 39.3 / 39.4; B=1 H=6 N=16384 (6,144) 165.3 / 160.1, 164.3 /
+// 160.2, 45.3 / 44.9; B=2 H=6 N=16384 (12,288) 278.0 / 270.1, 275.7 / 271.0, 78.9 / 75.4; B=4 H=6 N=16384 (24,576) 505 / 499, 507 / 501, 153 / 146; B=2 H=4 N=65536
+// (32,768) 791 / 795, 781 / 781, 228.8 / 225.5; B=8 H=6 N=16384 (49,152) 951 / 960 eager; B=1 H=6 N=262144 (98,304) forward 1034 / 1045.
 // One level: no gain (B=2 H=4 N=16384 323 / 325).  With a norm or a rotation the values are a fifth of the pass: B=1 H=6 N=16384 57.9 / 59.1.
 constexpr int64_t kValuesBesideFrom = 4096, kValuesBesideTo = 24576;
 bool values_beside(const Dims& d, int64_t D, at::ScalarType dt, bool two, bool transformed) {

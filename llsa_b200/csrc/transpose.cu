@@ -79,7 +79,10 @@ __device__ __forceinline__ void place_range(const TransposeArgs& a, int64_t bh, 
 }
 
 // ---- one CTA per (b,h) and key range ----------------------------------------------------------------
-// 32 registers a thread: 16 warps then take the room of one CTA of the dQ stage it runs beside (48 to 54 registers took that of two).
+// 32 registers a thread: 16 warps then take the room of one CTA of the dQ stage it runs beside (64 registers, as the compiler would have them, that of
+// two), 32 warps that of two (62 registers: a whole SM; the limit spills 20 bytes there).  Forward + backward in us, without the limit / with it: 16 warps, two
+// levels, B=3 H=5 N=5376 138.6 / 137.3, B=4 H=6 N=16384 with norms 608.9 / 606.4, one level, B=4 H=6 N=4096 175.3 / 176.1; 32 warps, B=1 H=5 N=40960 top-16
+// 499.7 / 493.9 (in a graph 489.3 / 491.8), B=1 H=6 N=65536 601.0 / 602.6; alone on its stream, fp32, B=1 H=2 N=1024, 96.3 / 96.4.
 template <int W>
 __global__ void __launch_bounds__(W * 32, 64 / W) transpose_range_kernel(TransposeArgs a, int keys_per_range, uint32_t t_magic) {
   pdl_trigger();
