@@ -70,8 +70,8 @@ def _exact_scores(BH, M, n, kind, wait_limit):
 
 # the tcgen05 kernel: its shortest list and the longest, lists that end half way through a 128-key chunk; few tiles, whose keys a cluster of eight, four or two
 # CTAs shares (up to 32, 64 and 128), with shares of unlike length, and more than that
-@pytest.mark.parametrize("BH,M,n,topk", [(1, 40, 3584, 8), (1, 300, 3648, 8), (2, 128, 4160, 5), (8, 500, 3584, 8), (9, 500, 3648, 8), (17, 512, 3712, 4),
-                                         (129, 4, 3584, 8), (43, 300, 3648, 1), (1, 16, 65536, 8)])
+@pytest.mark.parametrize("BH,M,n,topk", [(1, 40, 2048, 8), (1, 300, 2112, 8), (2, 128, 4160, 5), (8, 500, 2048, 8), (9, 500, 2112, 8), (17, 512, 2176, 4),
+                                         (129, 4, 2048, 8), (43, 300, 2112, 1), (1, 16, 65536, 8)])
 def test_coarse_topk_on_tcgen05(BH, M, n, topk):
     test_coarse_topk_shapes(BH, M, n, torch.bfloat16, topk)
 
@@ -79,7 +79,7 @@ def test_coarse_topk_on_tcgen05(BH, M, n, topk):
 # tiles: a cluster of eight, four, two, none
 @pytest.mark.parametrize("wait_limit", [0, 1])
 @pytest.mark.parametrize("kind", ["ties", "equal", "nan", "-inf", "masked"])
-@pytest.mark.parametrize("BH,n", [(2, 3584), (2, 3648), (40, 3648), (100, 3584), (129, 3648)])
+@pytest.mark.parametrize("BH,n", [(2, 2048), (2, 2112), (40, 2112), (100, 2048), (129, 2112)])
 def test_coarse_topk_on_tcgen05_orders_exact_scores(BH, n, kind, wait_limit):
     _exact_scores(BH, 8, n, kind, wait_limit)
 
