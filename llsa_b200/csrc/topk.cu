@@ -752,7 +752,7 @@ using namespace llsa;
 
 // The tcgen05 kernel (topk_tc.cu) sums a score in another order, so the length of the list alone may choose between the two: a row's blocks must not depend
 // on the batch or on how many of the sequence's rows a call holds.  So the line weighs few rows against many: below it mma.sync is ahead up to eight or twelve
-// square slices (n = M), above it tcgen05, its keys shared by a cluster where there are few rows, from three or four on.  us in a graph, smooth inputs,
+// square slices (n = M), above it tcgen05, its keys shared by a cluster where there are few rows, from three to six on.  us in a graph, smooth inputs,
 // here / there: n = 1024: 1 slice 8.8 / 18.4, 6 11.7 / 20.5, 12 21.5 / 25.2, 24 50 / 35, 48 81 / 57; 1536: 1 11.8 / 17.3, 4 14.6 / 24.8, 8 26.5 / 30.2, 16 60 / 42;
 // 2048: 1 15.3 / 18.1, 3 17.4 / 24.3, 4 27.4 / 25.1, 8 42.0 / 36.0, 12 72 / 47, 48 217 / 112; 2560: 1 18.3 / 20.6, 2 20.0 / 28.9, 4 33.1 / 36.6, 6 48.7 / 39.2, 12 94 / 48;
 // 3072: 2 22.2 / 28.3, 3 36.8 / 37.0, 12 107 / 59; 4096: 1 27.3 / 24.4, 2 45.7 / 34.9, 8 131 / 69, 128 rows 20.0 / 18.6.
