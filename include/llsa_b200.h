@@ -284,7 +284,7 @@ int llsa_attn_fwd(const LlsaAttnArgs* args, void* stream);
  * MeanPool1dFunction_BHSC.backward calls autograd runs after them. */
 int llsa_attn_bwd(const LlsaAttnArgs* args, void* stream);
 /* Element count of the F32 scratch tensor LlsaAttnArgs.dkv_partial that llsa_attn_bwd makes use of for bf16 tensors with
- * Nq query rows per (b,h) and `topk` selected blocks per query block (the caller allocates it, 4-D and contiguous).  Any size from
+ * Nq query rows per (b,h) and `topk` selected blocks per query block (the caller allocates it, 4-D, contiguous and 16-byte aligned).  Any size from
  * B*H*ceil(Nq/16*topk/64)*4096 on is accepted; with less than this function names, small problems are spread over fewer warps.  The
  * library itself never allocates device memory. */
 int64_t llsa_attn_bwd_partial_elems(int64_t B, int64_t H, int64_t Nq, int32_t topk);

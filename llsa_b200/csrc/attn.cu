@@ -83,9 +83,10 @@ static int check_attn_args(const LlsaAttnArgs* g, bool bwd) {
     if (dt == LLSA_BF16 && !g->force_generic) {
       LLSA_REQUIRE(g->dkv_partial, LLSA_ERR_WORKSPACE, "attn_bwd: dkv_partial scratch missing");
       const int64_t need = partial_windows(B, H, Nq, g->topk) * 4096;
-      LLSA_REQUIRE(g->dkv_partial->ptr && g->dkv_partial->dtype == LLSA_F32 && g->dkv_partial->ndim == 4 && is_contiguous(g->dkv_partial) &&
+      LLSA_REQUIRE(g->dkv_partial->ptr && ((uintptr_t) g->dkv_partial->ptr % 16) == 0 && g->dkv_partial->dtype == LLSA_F32 &&
+                       g->dkv_partial->ndim == 4 && is_contiguous(g->dkv_partial) &&
                        g->dkv_partial->shape[0] * g->dkv_partial->shape[1] * g->dkv_partial->shape[2] * g->dkv_partial->shape[3] >= need,
-                   LLSA_ERR_WORKSPACE, "attn_bwd: dkv_partial must be a contiguous F32 tensor of at least %lld elements", (long long) need);
+                   LLSA_ERR_WORKSPACE, "attn_bwd: dkv_partial must be a contiguous, 16-byte aligned F32 tensor of at least %lld elements", (long long) need);
     }
     if (dt == LLSA_BF16 && !g->force_generic) {
       LLSA_REQUIRE(g->flat_ranges, LLSA_ERR_WORKSPACE, "attn_bwd: flat_ranges missing (llsa_transpose_indices_pairs)");

@@ -148,6 +148,24 @@ def test_attention_argument_errors():
     assert lib.llsa_attn_fwd(C.byref(args(pk2=fake((B, H, N // 256, D)))), None) == ERR_NULL
 
 
+@pytest.mark.parametrize("ptr,elems,want", [(0x10004, 2 * 8 * 4096, ERR_WORKSPACE), (0x10000, 2 * 8 * 4096 - 4096, ERR_WORKSPACE),
+                                            (0x10000, 2 * 8 * 4096, ERR_SHAPE)])
+def test_backward_scratch_is_checked_for_size_and_alignment(ptr, elems, want):
+    """dkv_partial is read and written 16 bytes at a time.  The work ranges behind it are of a wrong shape, so that no form of the call launches."""
+    lib, f32, i32 = _lib.lib(), torch.float32, torch.int32
+    B, H, N, D = 1, 2, 1024, 64
+    row, pooled = (B, H, N, D), (B, H, N // 16, D)
+    t = dict(q=fake(row), k=fake(row), v=fake(row), o=fake(row), d_o=fake(row), dq=fake(row), dk=fake(row), dv=fake(row), pk=fake(pooled), pv=fake(pooled),
+             dpk_acc=fake(pooled, f32), dpv_acc=fake(pooled, f32), lse=fake((B, H, N), f32), delta=fake((B, H, N), f32), indices=fake((B, H, 64, 8), i32),
+             offsets=fake((B, H, 65), i32), flat=fake((B, H, 512), i32), flat_ranges=fake((B, H, 5, 2), i32),
+             dkv_partial=fake((1, 1, elems // 4096, 4096), f32, ptr=ptr))
+    a = _lib.LlsaAttnArgs()
+    for name, d in t.items():
+        setattr(a, name, _lib.ptr(d))
+    a.topk, a.block_size, a.token_weight, a.kv_weight = 8, 16, 16.0, 16.0
+    assert lib.llsa_attn_bwd(C.byref(a), None) == want
+
+
 def test_ops_refuse_cpu_tensors():
     import llsa_b200
     x = torch.randn(1, 1, 1024, 64)
