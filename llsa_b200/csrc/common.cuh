@@ -50,8 +50,8 @@ void set_error(const char* fmt, ...);
 //   * pool_pyramid_bf16_kernel, launched to run beside the selection, reads the values and writes their pooled levels.  The pooling launch of q and k in
 //     front of the selection waits in every CTA and has no pdl_trigger(): the selection's CTAs, and so this launch, begin when it has ended, and all
 //     in front of it has completed.
-// A kernel in front of a streaming one (pooling pass, rotation / norm backward) has no pdl_trigger(): that one's CTAs would settle unevenly on the SMs that
-// become free first (figures at its launch).
+// The tcgen05 forwards, with which a layer's forward ends, and the finish kernel, with which its dK/dV stage does, have no pdl_trigger(): what comes next, the
+// pooling pass or the rotation / norm backward, streams, and its CTAs would settle unevenly on the SMs that become free first (figures at its launch).
 // cluster: neighbouring CTAs along x that form a cluster (the grid's x is a multiple of it).
 template <typename... P, typename... A>
 inline void launch_pdl_cluster(void (*kernel)(P...), dim3 grid, dim3 block, unsigned cluster, size_t smem, cudaStream_t st, A&&... args) {
